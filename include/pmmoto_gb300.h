@@ -349,30 +349,21 @@ int pmg_set_iteration_cap(int32_t cap);
 
 /*
  * Tunable launch parameters (no counterpart in the reference): results never
- * depend on them, only speed.  Names: "edt.pair_seg" (positions per thread
- * of the strided line-pair envelope pass, default 256), "edt.pair_ctas" and
- * "edt.rows_ctas" (CTAs per SM of the strided and contiguous line-pair
- * passes, defaults 32 and 16), "cc.cross_fused" (block labelling's
+ * depend on them, only speed.  Names: "cc.cross_fused" (block labelling's
  * cross-tile phase as one fused pass, 1, or as a classification pass and a
- * union pass, 0; default 0), "edt.path" (envelope passes with power-of-two
- * voxels: windowed with the probed fallback, 0, the exact integer stream, 1,
- * or the float envelope, 2; default 0), "edt.fallback" and
- * "edt.fallback_rows" (probe samples, of 8192, that the +-12 window does not
- * finish, from which a strided or a contiguous windowed pass hands the whole
- * pass to the float envelope; 0 always, 8193 never; defaults 96 and 2048),
- * "edt.narrow" and "edt.narrow_rows" (probe samples the +-8 window does not
- * finish, below which the pass runs the +-8 window instead of the +-12 one;
- * 0 never; defaults 64 and 32), "edt.wide" (probe samples the +-24 window
- * does not finish, below which a strided pass of at least 131,072 lines that
- * the +-12 window would hand to the float envelope runs the +-24 window;
- * 0 never, 8193 always and for any line count; default 1024),
- * "cc.seam_batched" (periodic merge: the
- * seams of all periodic features deduplicated in one sort, 1, or one
- * feature at a time, 0; default 1; one at a time is also taken when labels
- * need more than 29 bits).  A negative value restores the default, and so
- * does 0 for the knobs whose smallest value is 1; values are process-wide
- * and apply to launches that follow.  pmmoto_gb300.tune sets them from its
- * cached measurements.
+ * union pass, 0; default 0), "edt.path" (envelope passes: the integer lattice
+ * and the outward scan, 0, the exact integer stream, 1, or the float envelope,
+ * 2; default 0), "cc.seam_batched" (periodic merge: the seams of all periodic
+ * features deduplicated in one sort, 1, or one feature at a time, 0; default
+ * 1; one at a time is also taken when labels need more than 29 bits).
+ * "edt.pair_seg", "edt.pair_ctas", "edt.rows_ctas", "edt.fallback",
+ * "edt.fallback_rows", "edt.narrow", "edt.narrow_rows" and "edt.wide" belonged
+ * to a windowed pass that the lattice passes replaced; they are still
+ * accepted, in the same ranges, so that saved settings keep loading, and have
+ * no effect.  A negative value restores the default, and so does 0 for the
+ * knobs whose smallest value is 1; values are process-wide and apply to
+ * launches that follow.  pmmoto_gb300.tune sets them from its cached
+ * measurements.
  */
 int pmg_tune_set(const char *name, int32_t value);
 int pmg_tune_get(const char *name, int32_t *value);

@@ -27,8 +27,6 @@
 #include <cfloat>
 #include <cmath>
 #include <algorithm>
-#include <cstring>
-#include <cooperative_groups.h>
 
 #include "edt_internal.cuh"
 
@@ -106,105 +104,6 @@ __global__ void k_pass0(const uint8_t *__restrict__ img, float *__restrict__ out
     }
 }
 
-// k_pass0 on four adjacent strided lines per thread (their voxels are
-// adjacent along the contiguous axis): uchar4 loads of the image and float4
-// loads and stores of the distances, each of the four lines with the same
-// state and the same float operations as k_pass0.
-__global__ void __launch_bounds__(256) k_pass0_x4(const uint8_t *__restrict__ img, float *__restrict__ out, Lines Ls,
-                                                  float res, pmg_axis_cfg cfg)
-{
-    const long long nquads = Ls.count() >> 2;
-    for (long long qi = blockIdx.x * (long long)blockDim.x + threadIdx.x; qi < nquads;
-         qi += (long long)gridDim.x * blockDim.x) {
-        const LineGeo g = line_addr(Ls, qi * 4);
-        const uint8_t *in = img + g.base;
-        float *d = out + g.base;
-        const long long st = g.stride;
-        const int n = g.n;
-        float lc[4] = {INFINITY, INFINITY, INFINITY, INFINITY}, uc[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
-        if (cfg.periodic) {
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                int F = -1, L = -1;
-                for (int i = cfg.f_lo; i < n; i++)
-                    if (in[i * st + q] == 0) {
-                        F = i;
-                        break;
-                    }
-                for (int i = n - cfg.l_hi - 1; i >= cfg.l_lo; i--)
-                    if (in[i * st + q] == 0) {
-                        L = i;
-                        break;
-                    }
-                if (F != -1)
-                    uc[q] = (float)(F + cfg.a_u);
-                if (L != -1)
-                    lc[q] = (float)(n - L + cfg.a_l);
-            }
-        }
-        // forward sweep (reset at zeros, restart at a change of nonzero value)
-        const uchar4 v0 = *reinterpret_cast<const uchar4 *>(in);
-        uint8_t seg[4] = {v0.x, v0.y, v0.z, v0.w};
-        uint8_t prev_v[4] = {v0.x, v0.y, v0.z, v0.w};
-        float prev[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-            prev[q] = seg[q] == 0 ? 0.0f : fmul(lc[q], res);
-        *reinterpret_cast<float4 *>(d) = make_float4(prev[0], prev[1], prev[2], prev[3]);
-#pragma unroll 4
-        for (int i = 1; i < n; i++) {
-            const uchar4 vv = *reinterpret_cast<const uchar4 *>(in + i * st);
-            const uint8_t v[4] = {vv.x, vv.y, vv.z, vv.w};
-            float cur[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                if (v[q] == 0) {
-                    cur[q] = 0.0f;
-                } else if (v[q] == seg[q]) {
-                    cur[q] = fadd(prev[q], res);
-                } else {
-                    cur[q] = res;
-                    d[(i - 1) * st + q] = prev_v[q] != 0 ? res : 0.0f;
-                    seg[q] = v[q];
-                }
-                prev[q] = cur[q];
-                prev_v[q] = v[q];
-            }
-            *reinterpret_cast<float4 *>(d + i * st) = make_float4(cur[0], cur[1], cur[2], cur[3]);
-        }
-        // clamp the last voxel, backward sweep, square, inf -> FLT_MAX
-        float b[4];
-        {
-            const float4 t = *reinterpret_cast<const float4 *>(d + (n - 1) * st);
-            const float tv[4] = {t.x, t.y, t.z, t.w};
-            float q4[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                b[q] = tv[q];
-                const float ucr = fmul(uc[q], res);
-                if (b[q] > ucr)
-                    b[q] = ucr;
-                const float sq = fmul(b[q], b[q]);
-                q4[q] = sq == INFINITY ? FLT_MAX : sq;
-            }
-            *reinterpret_cast<float4 *>(d + (n - 1) * st) = make_float4(q4[0], q4[1], q4[2], q4[3]);
-        }
-#pragma unroll 4
-        for (int i = n - 2; i >= 0; i--) {
-            const float4 t = *reinterpret_cast<const float4 *>(d + i * st);
-            const float tv[4] = {t.x, t.y, t.z, t.w};
-            float q4[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                b[q] = fminf(tv[q], fadd(b[q], res));
-                const float sq = fmul(b[q], b[q]);
-                q4[q] = sq == INFINITY ? FLT_MAX : sq;
-            }
-            *reinterpret_cast<float4 *>(d + i * st) = make_float4(q4[0], q4[1], q4[2], q4[3]);
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
 // envelope stack kept as a bitmask in shared memory
 // ---------------------------------------------------------------------------
@@ -269,16 +168,59 @@ struct Stack {
     }
 };
 
-// Height of a native vertex (re-read from the input line).
-__device__ __forceinline__ float vh(const float *line, long long st, int v) { return line[v * st]; }
+// Heights of a line by vertex: read from the line in global memory ...
+struct LineGlobal {
+    const float *p;
+    long long st;
+    __device__ __forceinline__ float operator()(int v) const { return p[v * st]; }
+    __device__ __forceinline__ LineGlobal from(int v) const { return {p + v * st, st}; }
+};
+
+// ... or with both line ends staged in shared memory (the first and last
+// kEndWin positions, slot v of this thread's line at s[v * sst]; global
+// memory in between, as floats or as counts of voxels).
+constexpr int kEndWin = 32;
+
+__device__ __forceinline__ float height_of(const float *p, float) { return __ldg(p); }
+__device__ __forceinline__ float height_of(const uint16_t *p, float res)
+{
+    const uint32_t c = __ldg(p);
+    const float d = fmul((float)c, res);
+    return c >= 0x4000u ? FLT_MAX : fmul(d, d);
+}
+
+template <class T>
+struct LineEnds {
+    const T *p;
+    long long st;
+    const float *s;
+    int sst, n, off;
+    float res;
+    __device__ __forceinline__ float operator()(int v) const
+    {
+        v += off;
+        if (v < kEndWin)
+            return s[v * sst];
+        if (v >= n - kEndWin)
+            return s[(v - n + 2 * kEndWin) * sst];
+        return height_of(p + v * st, res);
+    }
+    __device__ __forceinline__ LineEnds from(int v) const
+    {
+        LineEnds l = *this;
+        l.off += v;
+        return l;
+    }
+};
 
 // Range of the native vertex `v` = intersection with the entry below it.
-__device__ __forceinline__ float native_range(Stack &S, const float *line, long long st, int v,
-                                              float h, float aniso, int below_native_count)
+template <class L>
+__device__ __forceinline__ float native_range(Stack &S, const L &line, int v, float h, float aniso,
+                                              int below_native_count)
 {
     if (below_native_count > 0) {
         int pv = S.prev_bit(v);
-        return isect(h, (float)v, vh(line, st, pv), (float)pv, aniso);
+        return isect(h, (float)v, line(pv), (float)pv, aniso);
     }
     if (S.nl > 0)
         return isect(h, (float)v, S.lh[S.nl - 1], (float)S.lv[S.nl - 1], aniso);
@@ -286,7 +228,8 @@ __device__ __forceinline__ float native_range(Stack &S, const float *line, long 
 }
 
 // Pop the top entry and reload the cache with the new top.
-__device__ __forceinline__ void pop_top(Stack &S, const float *line, long long st, float aniso)
+template <class L>
+__device__ __forceinline__ void pop_top(Stack &S, const L &line, float aniso)
 {
     if (S.nu > 0) {
         --S.nu;
@@ -305,8 +248,8 @@ __device__ __forceinline__ void pop_top(Stack &S, const float *line, long long s
     }
     if (S.nn > 0) {
         S.tv = S.ntv;
-        S.th = vh(line, st, S.ntv);
-        S.tr = native_range(S, line, st, S.ntv, S.th, aniso, S.nn - 1);
+        S.th = line(S.ntv);
+        S.tr = native_range(S, line, S.ntv, S.th, aniso, S.nn - 1);
     } else {
         S.tv = S.lv[S.nl - 1];
         S.th = S.lh[S.nl - 1];
@@ -316,12 +259,12 @@ __device__ __forceinline__ void pop_top(Stack &S, const float *line, long long s
 
 // update_hull (_distance.hpp:89-112) for vertex i with height f; `kind`
 // 0 = native vertex (a bit), 1 = imported upper hull.
-__device__ __forceinline__ void insert(Stack &S, const float *line, long long st, int i, float f,
-                                       float aniso, int kind)
+template <class L>
+__device__ __forceinline__ void insert(Stack &S, const L &line, int i, float f, float aniso, int kind)
 {
     float s = isect(f, (float)i, S.th, (float)S.tv, aniso);
     while (S.nl + S.nn + S.nu > 1 && s <= S.tr) {
-        pop_top(S, line, st, aniso);
+        pop_top(S, line, aniso);
         s = isect(f, (float)i, S.th, (float)S.tv, aniso);
     }
     if (kind == 0) {
@@ -341,8 +284,8 @@ __device__ __forceinline__ void insert(Stack &S, const float *line, long long st
 
 // Build the envelope of a line segment [0, n) of `line` with no imports:
 // entry (0, f(0)) at the bottom, then vertices 1..n-1.
-__device__ __forceinline__ void build_plain(Stack &S, const float *line, long long st, int n,
-                                            float aniso)
+template <class L>
+__device__ __forceinline__ void build_plain(Stack &S, const L &line, int n, float aniso)
 {
     S.nl = 0;
     S.nu = 0;
@@ -350,10 +293,10 @@ __device__ __forceinline__ void build_plain(Stack &S, const float *line, long lo
     S.nn = 1;
     S.ntv = 0;
     S.tv = 0;
-    S.th = vh(line, st, 0);
+    S.th = line(0);
     S.tr = -INFINITY;
     for (int i = 1; i < n; i++)
-        insert(S, line, st, i, vh(line, st, i), aniso, 0);
+        insert(S, line, i, line(i), aniso, 0);
 }
 
 // Iterator over the final stack, bottom to top.
@@ -362,8 +305,9 @@ struct Iter {
     int idx;   // lower/upper index or native vertex
 };
 
-__device__ __forceinline__ bool iter_next(Stack &S, Iter &it, const float *line, long long st,
-                                          int nwords, Entry &e, int &is_lower, float &given_r)
+template <class L>
+__device__ __forceinline__ bool iter_next(Stack &S, Iter &it, const L &line, int nwords, Entry &e, int &is_lower,
+                                          float &given_r)
 {
     for (;;) {
         if (it.phase == 0) {
@@ -383,7 +327,7 @@ __device__ __forceinline__ bool iter_next(Stack &S, Iter &it, const float *line,
             if (nb >= 0) {
                 it.idx = nb;
                 e.v = nb;
-                e.h = vh(line, st, nb);
+                e.h = line(nb);
                 is_lower = 0;
                 return true;
             }
@@ -408,15 +352,15 @@ __device__ __forceinline__ bool iter_next(Stack &S, Iter &it, const float *line,
 // of the line: keep up to num_hull+1 finite parabolas from the chosen end,
 // vertices and ranges shifted by `corr`.  Returns the count; the bitmask is
 // left cleared.
-__device__ int boundary_hull(Stack &S, const float *line, long long st, int start, int nv,
-                             float aniso, int num_hull, int corr, bool forward, int *ov,
-                             float *oh, float *orr)
+template <class L>
+__device__ int boundary_hull(Stack &S, const L &line, int start, int nv, float aniso, int num_hull, int corr,
+                             bool forward, int *ov, float *oh, float *orr)
 {
-    const float *seg = line + (long long)start * st;
+    const L seg = line.from(start);
     if (nv <= 0)
         return 0;
     if (nv == 1) {
-        const float f0 = seg[0];
+        const float f0 = seg(0);
         if (f0 < FLT_MAX) {
             ov[0] = corr;
             oh[0] = f0;
@@ -430,7 +374,7 @@ __device__ int boundary_hull(Stack &S, const float *line, long long st, int star
         return 1;
     }
     const int nwords = (nv + 31) >> 5;
-    build_plain(S, seg, st, nv, aniso);
+    build_plain(S, seg, nv, aniso);
     const int top = S.nn - 1; // stack index of the top entry
     const int keep = num_hull < top ? num_hull : top;
     int cnt = 0;
@@ -440,7 +384,7 @@ __device__ int boundary_hull(Stack &S, const float *line, long long st, int star
         int prev_v = 0;
         for (int k = 0; k <= top && cnt <= keep; k++) {
             v = S.next_bit(v, nwords);
-            const float h = vh(seg, st, v);
+            const float h = seg(v);
             const float r = k == 0 ? -INFINITY : isect(h, (float)v, prev_h, (float)prev_v, aniso);
             if (h < FLT_MAX) {
                 ov[cnt] = v + corr;
@@ -455,13 +399,13 @@ __device__ int boundary_hull(Stack &S, const float *line, long long st, int star
         }
     } else {
         int v = S.ntv;
-        float h = vh(seg, st, v);
+        float h = seg(v);
         for (int k = top; k >= 0 && cnt <= keep; k--) {
             int pv = 0;
             float ph = 0.0f, r;
             if (k > 0) {
                 pv = S.prev_bit(v);
-                ph = vh(seg, st, pv);
+                ph = seg(pv);
                 r = isect(h, (float)v, ph, (float)pv, aniso);
             } else {
                 r = -INFINITY;
@@ -489,21 +433,21 @@ __device__ int boundary_hull(Stack &S, const float *line, long long st, int star
 // The imported boundary hulls of a periodic line (return_boundary_hull on the
 // segment before the first zero and after the last zero, the far end's hull
 // becoming the lower imports): lower imports into S, upper ones into up_*.
-__device__ __forceinline__ void load_imports(Stack &S, const float *line, long long st, int n, float aniso,
-                                             const pmg_axis_cfg &cfg, int num_hull, int *up_v, float *up_h,
-                                             float *up_r, int &n_up)
+template <class L>
+__device__ __forceinline__ void load_imports(Stack &S, const L &line, int n, float aniso, const pmg_axis_cfg &cfg,
+                                             int num_hull, int *up_v, float *up_h, float *up_r, int &n_up)
 {
     // first / last zero (a zero height is exactly a zero voxel of the
     // original image: pass 0 gives 0 only there and every later pass keeps
     // it, all other values being >= res^2 > 0)
     int bf = -1, bb = -1;
     for (int i = cfg.hf_lo; i < n; i++)
-        if (line[i * st] == 0.0f) {
+        if (line(i) == 0.0f) {
             bf = i;
             break;
         }
     for (int i = n - cfg.hb_hi - 1; i >= 0; i--)
-        if (line[i * st] == 0.0f) {
+        if (line(i) == 0.0f) {
             bb = i;
             break;
         }
@@ -517,7 +461,7 @@ __device__ __forceinline__ void load_imports(Stack &S, const float *line, long l
         nv = bf - cfg.hf_lo + 1;
     }
     corr = 0;
-    n_up = boundary_hull(S, line, st, start, nv, aniso, num_hull, corr, true, up_v, up_h, up_r);
+    n_up = boundary_hull(S, line, start, nv, aniso, num_hull, corr, true, up_v, up_h, up_r);
     // far end (backward) -> lower imports, given in top-down order
     int lo_v[kMaxHull];
     float lo_h[kMaxHull], lo_r[kMaxHull];
@@ -529,7 +473,7 @@ __device__ __forceinline__ void load_imports(Stack &S, const float *line, long l
         nv = n - bb - cfg.hb_hi;
     }
     corr = -nv;
-    const int n_lo = boundary_hull(S, line, st, start, nv, aniso, num_hull, corr, false, lo_v, lo_h, lo_r);
+    const int n_lo = boundary_hull(S, line, start, nv, aniso, num_hull, corr, false, lo_v, lo_h, lo_r);
     // the reference pushes the lower list in reverse (rbegin..rend)
     for (int j = 0; j < n_lo; j++) {
         S.lv[j] = lo_v[n_lo - 1 - j];
@@ -541,22 +485,22 @@ __device__ __forceinline__ void load_imports(Stack &S, const float *line, long l
 
 // Evaluation sweep over the final stack (bottom to top), written for
 // positions [i_lo, i_hi) of the line.
-__device__ __forceinline__ void evaluate(Stack &S, const float *line, long long st, int nwords, float aniso,
-                                         int form, const MorphEpi &me, const LineGeo &g, float *o, int i_lo,
-                                         int i_hi)
+template <class L>
+__device__ __forceinline__ void evaluate(Stack &S, const L &line, int nwords, float aniso, int form,
+                                         const MorphEpi &me, const LineGeo &g, float *o, int i_lo, int i_hi)
 {
     Iter it{0, 0};
     Entry cur, nxt;
     int is_lower;
     float given_r;
-    iter_next(S, it, line, st, nwords, cur, is_lower, given_r);
-    bool has_next = iter_next(S, it, line, st, nwords, nxt, is_lower, given_r);
+    iter_next(S, it, line, nwords, cur, is_lower, given_r);
+    bool has_next = iter_next(S, it, line, nwords, nxt, is_lower, given_r);
     float nr = has_next ? (is_lower ? given_r : isect(nxt.h, (float)nxt.v, cur.h, (float)cur.v, aniso)) : INFINITY;
     for (int i = i_lo; i < i_hi; i++) {
         const float fi = (float)i;
         while (nr < fi) {
             cur = nxt;
-            has_next = iter_next(S, it, line, st, nwords, nxt, is_lower, given_r);
+            has_next = iter_next(S, it, line, nwords, nxt, is_lower, given_r);
             nr = has_next ? (is_lower ? given_r : isect(nxt.h, (float)nxt.v, cur.h, (float)cur.v, aniso))
                           : INFINITY;
         }
@@ -568,46 +512,13 @@ __device__ __forceinline__ void evaluate(Stack &S, const float *line, long long 
         }
         if (form == PMG_EDT_DIST)
             val = __fsqrt_rn(val);
-        o[i * st] = val;
+        o[i * g.stride] = val;
     }
-}
-
-// The choice a windowed pass makes from its probe (k_env_probe, below):
-// count[0] and count[1] are the samples the +-8 and the +-12 windows do not
-// finish.  Choice 0 runs the +-8 line-pair kernels, 1 the +-12 ones, 2 the
-// float envelope on every line; the kernels of the other choices return at
-// once.  Without a probe the +-12 window runs.
-// count[2] counts those the +-24 window does not finish: below thr24 (the
-// strided passes only) the +-24 kernel takes a pass the +-12 one would
-// leave to the envelope (choice 3).
-struct Probe {
-    const int *count;
-    int thr8, thr12, thr24;
-    __device__ __forceinline__ int choice() const
-    {
-        if (!count)
-            return 1;
-        if (count[0] < thr8)
-            return 0;
-        if (count[1] < thr12)
-            return 1;
-        return count[2] < thr24 ? 3 : 2;
-    }
-};
-
-template <int W>
-__host__ __device__ constexpr int window_choice()
-{
-    static_assert(W == 8 || W == 12 || W == 24, "windows of +-8, +-12 and +-24");
-    return W == 8 ? 0 : W == 12 ? 1 : 3;
 }
 
 __global__ void k_envelope(const float *__restrict__ fin, float *__restrict__ fout, Lines Ls, float res,
-                           pmg_axis_cfg cfg, int num_hull, int form, MorphEpi me, int redo, Probe probe)
+                           pmg_axis_cfg cfg, int num_hull, int form, MorphEpi me, int redo)
 {
-    // behind the windowed kernels: every line, when the probe chose the envelope
-    if (probe.count && probe.choice() != 2)
-        return;
     const long long nlines = Ls.count();
     extern __shared__ uint32_t smem_bm[];
     const float aniso = fmul(res, res);
@@ -620,8 +531,7 @@ __global__ void k_envelope(const float *__restrict__ fin, float *__restrict__ fo
         // second chance for lines the exact streaming kernel handed back
         if (redo && !line_marked(fout, me, g, form))
             continue;
-        const float *line = fin + g.base;
-        const long long st = g.stride;
+        const LineGlobal line{fin + g.base, g.stride};
         const int n = g.n;
         const int nwords = (n + 31) >> 5;
         S.clear(nwords);
@@ -631,7 +541,7 @@ __global__ void k_envelope(const float *__restrict__ fin, float *__restrict__ fo
         float up_h[kMaxHull], up_r[kMaxHull];
         int n_up = 0;
         if (cfg.periodic)
-            load_imports(S, line, st, n, aniso, cfg, num_hull, up_v, up_h, up_r, n_up);
+            load_imports(S, line, n, aniso, cfg, num_hull, up_v, up_h, up_r, n_up);
         // main build
         int loop_start;
         if (S.nl > 0) {
@@ -647,811 +557,360 @@ __global__ void k_envelope(const float *__restrict__ fin, float *__restrict__ fo
             S.nn = 1;
             S.ntv = 0;
             S.tv = 0;
-            S.th = vh(line, st, 0);
+            S.th = line(0);
             S.tr = -INFINITY;
         }
         for (int i = loop_start; i < n; i++)
-            insert(S, line, st, i, vh(line, st, i), aniso, 0);
+            insert(S, line, i, line(i), aniso, 0);
         for (int j = 0; j < n_up; j++)
-            insert(S, line, st, up_v[j] + n, up_h[j], aniso, 1);
-        evaluate(S, line, st, nwords, aniso, form, me, g, fout + g.base, 0, n);
+            insert(S, line, up_v[j] + n, up_h[j], aniso, 1);
+        evaluate(S, line, nwords, aniso, form, me, g, fout + g.base, 0, n);
     }
 }
 
 // ---------------------------------------------------------------------------
-// periodic lines with power-of-two voxels: windowed exact minimum + end
-// segments
+// flagged lines
 // ---------------------------------------------------------------------------
-// Every height is an exact integer multiple K * res^2, and a zero height (a
-// solid voxel) shields everything beyond it: at x, a parabola beyond the
-// nearest zero on either side is above that zero's value.  So the result at x
-// is the exact minimum of K_v + (x - v)^2 over the voxels v that the scan
-// outward from x reaches before (x - v)^2 exceeds the best value, and the
-// reference's float32 envelope returns exactly that minimum there (the
-// rounding argument of edt_exact.cu) -- unless the scan runs off the end of
-// a periodic line, where the imported boundary hulls (a truncated set) come
-// into play.  k_env_window computes every voxel whose scan stays inside the
-// line and flags the lines with one that does not; k_envelope_ends then
-// replays the reference's float envelope on those lines' end segments only:
-// the lower imports with the voxels up to the first zero, and the voxels from
-// the last zero with the upper imports.  No parabola can pop a zero off the
-// stack, so these partial stacks and sweeps make the same float decisions as
-// the whole line's.  A line without a zero, with a height that is not an
-// exact integer, or with a scan longer than kWinMax is flagged for the whole
-// float envelope.
+// Lines the lattice and scan passes flag (edt_lattice.cu, edt_scan.cu) depend
+// on the imported hulls at their ends, or need the reference's float envelope
+// as a whole.
 
-constexpr int kWinMax = 64;
-
-// One voxel: the exact windowed minimum (returns true and the value), or
-// false with the flag bits its line needs (2: the whole float envelope, 1: its
-// end segments).  Heights are exact multiples of res^2 here (the passes
-// before only ever produce such values, or FLT_MAX for a line without a
-// solid voxel), so K = f / res^2 and every sum below are exact in float32.
-__device__ __forceinline__ bool window_voxel(const float *line, long long st, int n, int x, float inv_a, float kmax,
-                                             int periodic, float &best, int &need)
+// One line replayed with the float envelope: the whole line (`whole`, or a line
+// without a zero height), or its end segments only -- the lower imports with
+// the voxels up to the first zero, and the voxels from the last zero with the
+// upper imports.  No parabola can pop a zero off the stack, so these partial
+// stacks and sweeps make the same float decisions as the whole line's.
+// bm: this thread's envelope bits, nthr threads apart.
+template <class L>
+__device__ __noinline__ void replay_line(uint32_t *bm, int nthr, const L &line, const LineGeo &g, float aniso,
+                                         const pmg_axis_cfg &cfg, int num_hull, bool whole, int form,
+                                         const MorphEpi &me, float *fout)
 {
-    const float f = line[x * st];
-    if (f == 0.0f) {
-        best = 0.0f;
-        return true;
-    }
-    best = fmul(f, inv_a);
-    if (best >= kmax) {
-        need = 2;
-        return false;
-    }
-    bool ldone = false, rdone = false;
-    for (int t = 1; (float)(t * t) < best; t++) {
-        if (t > kWinMax) {
-            need = 2;
-            return false;
-        }
-        const float tt = (float)(t * t);
-        if (!ldone) {
-            const int v = x - t;
-            if (v < 0) {
-                if (periodic) {
-                    need = 1;
-                    return false;
-                }
-                ldone = true;
-            } else {
-                const float kv = fmul(line[v * st], inv_a);
-                if (kv >= kmax) {
-                    need = 2;
-                    return false;
-                }
-                best = fminf(best, fadd(kv, tt));
-                ldone = kv == 0.0f;
-            }
-        }
-        if (!rdone) {
-            const int v = x + t;
-            if (v >= n) {
-                if (periodic) {
-                    need = 1;
-                    return false;
-                }
-                rdone = true;
-            } else {
-                const float kv = fmul(line[v * st], inv_a);
-                if (kv >= kmax) {
-                    need = 2;
-                    return false;
-                }
-                best = fminf(best, fadd(kv, tt));
-                rdone = kv == 0.0f;
-            }
-        }
-        if (ldone && rdone)
-            break;
-    }
-    return true;
-}
-
-// Strided lines: one thread per chunk of kWinChunk voxels of a line,
-// neighbouring lines in neighbouring lanes; contiguous lines: one warp per
-// line, lanes 32 voxels apart.
-constexpr int kWinChunk = 64;
-
-__global__ void k_env_window(const float *__restrict__ fin, float *__restrict__ fout, Lines Ls, float a,
-                             float inv_a, int periodic, int form, int *__restrict__ flag,
-                             Probe probe)
-{
-    if (probe.choice() == 2)
-        return;
-    const long long nlines = Ls.count();
-    const LineGeo g0 = line_addr(Ls, 0);
-    const int n = g0.n;
-    const bool contiguous = g0.stride == 1;
-    const int nchunk = contiguous ? 1 : (n + kWinChunk - 1) / kWinChunk;
-    const float kmax = 16777216.0f - (float)(3 * n) * (float)(3 * n);
-    const int lane = threadIdx.x & 31;
-    const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const long long nthreads = (long long)gridDim.x * blockDim.x;
-    const long long items = nlines * nchunk;
-    const long long first = contiguous ? tid >> 5 : tid, step = contiguous ? nthreads >> 5 : nthreads;
-    for (long long it = first; it < items; it += step) {
-        const int chunk = (int)(it / nlines);
-        const long long li = it - (long long)chunk * nlines;
-        const LineGeo g = line_addr(Ls, li);
-        const float *line = fin + g.base;
-        float *o = fout + g.base;
-        const long long st = g.stride;
-        int need = 0;
-        const int x0 = contiguous ? lane : chunk * kWinChunk, dx = contiguous ? 32 : 1;
-        const int x1 = contiguous ? n : min(n, x0 + kWinChunk);
-        for (int x = x0; x < x1; x += dx) {
-            float best = 0.0f;
-            int nd = 0;
-            if (!window_voxel(line, st, n, x, inv_a, kmax, periodic, best, nd)) {
-                need |= nd;
-                continue;
-            }
-            float val = fmul(best, a);
-            if (form == PMG_EDT_DIST)
-                val = __fsqrt_rn(val);
-            o[x * st] = val;
-        }
-        // bit 1: the whole line needs the float envelope; bit 0: its ends
-        if (need)
-            atomicOr(flag + li, need);
-    }
-}
-
-// The line-pair kernels' slow path, out of line: window_voxel from the start
-// (t0 = 1), or continued past a window of +-W = t0 - 1 whose exact minimum m0
-// (units of res^2, every height in the window an exact integer) is above
-// (W + 1)^2.  In the second case no solid voxel lies within the window (one
-// would give at most W^2), so the scan from the start would cover the whole
-// window: it runs off a periodic line end there (flag 1), or closes the side
-// of a non-periodic end there, and otherwise continues at distance W + 1 with
-// the best value m0.  Either way the result and the flags are those of
-// window_voxel.  Four distances are loaded per side at a time so that the
-// loads overlap.
-__device__ __forceinline__ bool window_voxel_from(const float *line, long long st, int n, int x, float inv_a,
-                                               float kmax, int periodic, int t0, float m0, float *best_out,
-                                               int *need)
-{
-    float best;
-    bool ldone, rdone;
-    if (t0 <= 1) {
-        const float f = line[x * st];
-        if (f == 0.0f) {
-            *best_out = 0.0f;
-            return true;
-        }
-        best = fmul(f, inv_a);
-        if (best >= kmax) {
-            *need = 2;
-            return false;
-        }
-        t0 = 1;
-        ldone = rdone = false;
-    } else {
-        const int W = t0 - 1;
-        if (periodic && (x + 1 <= W || n - x <= W)) {
-            *need = 1;
-            return false;
-        }
-        best = m0;
-        ldone = !periodic && x + 1 <= W;
-        rdone = !periodic && n - x <= W;
-    }
-    for (int t = t0; (float)(t * t) < best && !(ldone && rdone); t += 4) {
-        float kl[4], kr[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int vl = x - t - q, vr = x + t + q;
-            kl[q] = (!ldone && vl >= 0) ? __ldg(line + vl * st) : 0.0f;
-            kr[q] = (!rdone && vr < n) ? __ldg(line + vr * st) : 0.0f;
-        }
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int tq = t + q;
-            const float tt = (float)(tq * tq);
-            if (tt >= best)
-                break;
-            if (tq > kWinMax) {
-                *need = 2;
-                return false;
-            }
-            if (!ldone) {
-                if (x - tq < 0) {
-                    if (periodic) {
-                        *need = 1;
-                        return false;
-                    }
-                    ldone = true;
-                } else {
-                    const float kv = fmul(kl[q], inv_a);
-                    if (kv >= kmax) {
-                        *need = 2;
-                        return false;
-                    }
-                    best = fminf(best, fadd(kv, tt));
-                    ldone = kv == 0.0f;
-                }
-            }
-            if (!rdone) {
-                if (x + tq >= n) {
-                    if (periodic) {
-                        *need = 1;
-                        return false;
-                    }
-                    rdone = true;
-                } else {
-                    const float kv = fmul(kr[q], inv_a);
-                    if (kv >= kmax) {
-                        *need = 2;
-                        return false;
-                    }
-                    best = fminf(best, fadd(kv, tt));
-                    rdone = kv == 0.0f;
-                }
-            }
-            if (ldone && rdone)
-                break;
-        }
-    }
-    *best_out = best;
-    return true;
-}
-
-// Voxels the line-pair kernels do not finish in their window are deferred to
-// k_env_slow: one 64-bit entry each, the line index (<< 32), the position
-// (<< 17), whether the scan continues past the window (<< 16) and the window
-// minimum (low 16 bits).  Appends are aggregated over the lanes that defer at
-// the same step; when the list is full the line is flagged for the whole float
-// envelope instead (a correct, slower result).
-__device__ __forceinline__ unsigned long long slow_entry(long long li, int x, bool resume, unsigned m)
-{
-    return ((unsigned long long)li << 32) | ((unsigned long long)(unsigned)x << 17) |
-           ((unsigned long long)(resume ? 1u : 0u) << 16) | (unsigned long long)(resume ? (m & 0xFFFFu) : 0u);
-}
-
-__device__ __forceinline__ bool slow_push(unsigned long long *list, int *count, int cap, unsigned long long e)
-{
-    namespace cg = cooperative_groups;
-    const cg::coalesced_group g = cg::coalesced_threads();
-    int base = 0;
-    if (g.thread_rank() == 0)
-        base = atomicAdd(count, (int)g.size());
-    base = g.shfl(base, 0);
-    const int pos = base + (int)g.thread_rank();
-    if (pos >= cap)
-        return false;
-    list[pos] = e;
-    return true;
-}
-
-// The deferred voxels, one thread each: window_voxel_from, then the output or
-// the line's flags (before the flagged lines are listed and replayed).
-__global__ void __launch_bounds__(256) k_env_slow(const float *__restrict__ fin, float *__restrict__ fout, Lines Ls,
-                                                  float a, float inv_a, int periodic, int form,
-                                                  int *__restrict__ flag, const unsigned long long *__restrict__ list,
-                                                  const int *__restrict__ count, int cap, Probe probe)
-{
-    // the window of the kernel that deferred the voxels
-    const int ch = probe.choice();
-    const int W = ch == 0 ? 8 : ch == 3 ? 24 : 12;
-    const int cnt = min(*count, cap);
-    const int n = line_addr(Ls, 0).n;
-    const float kmax = 16777216.0f - (float)(3 * n) * (float)(3 * n);
-    for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < cnt; it += gridDim.x * blockDim.x) {
-        const unsigned long long e = list[it];
-        const long long li = (long long)(e >> 32);
-        const int x = (int)((e >> 17) & 0x7FFFu);
-        const bool resume = (e >> 16) & 1u;
-        const LineGeo g = line_addr(Ls, li);
-        float best = 0.0f;
-        int nd = 0;
-        if (!window_voxel_from(fin + g.base, g.stride, n, x, inv_a, kmax, periodic, resume ? W + 1 : 1,
-                               (float)(unsigned)(e & 0xFFFFu), &best, &nd)) {
-            atomicOr(flag + li, nd);
-            continue;
-        }
-        float val = fmul(best, a);
-        if (form == PMG_EDT_DIST)
-            val = __fsqrt_rn(val);
-        fout[g.base + (long long)x * g.stride] = val;
-    }
-}
-
-// How often the windowed passes would fall back, sampled before a pass:
-// kProbe (line, position) samples spread over the lines; a sample counts for a
-// window of +-W when its minimum there is above (W + 1)^2 (not final: the
-// per-voxel scan would take it) or the window holds a height that is not an
-// integer below 2^16, for W = 8 and W = 12.  Media with wide pores (sphere packs) fall back at most voxels,
-// and the per-voxel scans cost several times the float envelope's sweep; so
-// when the count reaches the threshold the windowed kernels return at once
-// and the float envelope takes every line of the pass.  The choice is made on
-// the device (no host round trip) and changes no output: both give the
-// reference's values.
-constexpr int kProbe = 8192;
-
-__global__ void __launch_bounds__(256) k_env_probe(const float *__restrict__ fin, Lines Ls, float inv_a,
-                                                   int *__restrict__ count)
-{
-    const long long nl = Ls.count();
-    if (nl <= 0)
-        return;
-    const int n = line_addr(Ls, 0).n;
-    int c8 = 0, c12 = 0, c24 = 0;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < kProbe; s += gridDim.x * blockDim.x) {
-        const long long li = (long long)(((unsigned long long)s * (unsigned long long)nl) / kProbe);
-        const int x = (int)(((unsigned)s * 2654435761u) % (unsigned)n);
-        const LineGeo g = line_addr(Ls, li);
-        const float *line = fin + g.base;
-        const long long st = g.stride;
-        float best = fmul(line[x * st], inv_a);
-        bool bad = !(best < 65000.0f && best == truncf(best));
-#pragma unroll
-        for (int d = 1; d <= 24; d++) {
-            const float dd = (float)(d * d);
-            if (x - d >= 0) {
-                const float k = fmul(line[(x - d) * st], inv_a);
-                bad |= !(k < 65000.0f && k == truncf(k));
-                best = fminf(best, fadd(k, dd));
-            }
-            if (x + d < n) {
-                const float k = fmul(line[(x + d) * st], inv_a);
-                bad |= !(k < 65000.0f && k == truncf(k));
-                best = fminf(best, fadd(k, dd));
-            }
-            if (d == 8)
-                c8 += (bad || best > 81.0f) ? 1 : 0;
-            if (d == 12)
-                c12 += (bad || best > 169.0f) ? 1 : 0;
-        }
-        c24 += (bad || best > 625.0f) ? 1 : 0;
-    }
-    c8 = __reduce_add_sync(0xffffffffu, c8);
-    c12 = __reduce_add_sync(0xffffffffu, c12);
-    c24 = __reduce_add_sync(0xffffffffu, c24);
-    if ((threadIdx.x & 31) == 0) {
-        if (c8)
-            atomicAdd(count, c8);
-        if (c12)
-            atomicAdd(count + 1, c12);
-        if (c24)
-            atomicAdd(count + 2, c24);
-    }
-}
-
-// Strided lines, two at a time (adjacent along the contiguous axis, packed
-// as the halves of 32-bit words of integer heights K = f / res^2): the exact
-// minimum of K(x + d) + d^2 over |d| <= W by packed add-min, walking each
-// line segment with a register ring of 2W + 1 words.  A minimum m <= (W+1)^2
-// is final (every position beyond the window adds at least (W+1)^2); a
-// larger one, a window holding a height that is not an integer below 2^16
-// (clamped, so no sum wraps) or a periodic line end within reach ((x+1)^2 or
-// (n-x)^2 <= m: the per-voxel scan would run off the line there) falls back
-// to window_voxel for that voxel, which sets the same line flags as
-// k_env_window.  Outputs are those of k_env_window, with far fewer
-// divergent loops.
-template <int W, int A>
-__global__ void __launch_bounds__(256) k_env_pair(const float *__restrict__ fin, float *__restrict__ fout, Lines Ls,
-                                                  float a, float inv_a, int periodic, int form, int *__restrict__ flag,
-                                                  int seglen, Probe probe,
-                                                  unsigned long long *__restrict__ slow, int *__restrict__ slow_count,
-                                                  int slow_cap)
-{
-    if (probe.choice() != window_choice<W>())
-        return;
-    constexpr int R = 2 * W + 1; // the window of packed heights
-    constexpr unsigned kClamp = 65535u - (unsigned)(W * W) - 1u;
-    constexpr unsigned kFinal = (unsigned)((W + 1) * (W + 1));
-    const long long nlines = Ls.count();
-    const long long npairs = nlines >> 1;
-    const LineGeo g0 = line_addr(Ls, 0);
-    const int n = g0.n;
-    const long long st = g0.stride;
-    const int nseg = (n + seglen - 1) / seglen;
-    const uint32_t big = kClamp * 0x10001u;
-    const float2 kOut = make_float2(-1.0f, -1.0f); // marks a position outside the line
-    for (long long it = blockIdx.x * (long long)blockDim.x + threadIdx.x; it < npairs * nseg;
-         it += (long long)gridDim.x * blockDim.x) {
-        const int seg = (int)(it / npairs);
-        const long long li = (it - (long long)seg * npairs) * 2;
-        const LineGeo g = line_addr(Ls, li);
-        const float *line = fin + g.base;
-        float *o = fout + g.base;
-        const int x0 = seg * seglen, x1 = min(n, x0 + seglen);
-        // big_until*: the last output position whose window holds a height
-        // that is not an integer below 2^16 (clamped); those outputs take the scan
-        int big_until0 = -1, big_until1 = -1;
-        auto raw = [&](int y) -> float2 {
-            return (y < 0 || y >= n) ? kOut : __ldg(reinterpret_cast<const float2 *>(line + y * st));
-        };
-        // packing happens when a position enters the window, A positions
-        // after its load was issued, so the warp does not wait on the load
-        auto pack = [&](float2 f, int y) -> uint32_t {
-            if (f.x < 0.0f)
-                return big;
-            // heights are integers K res^2 when every axis has the same
-            // power-of-two voxel size; any other height takes the scan
-            const float k0 = fmul(f.x, inv_a), k1 = fmul(f.y, inv_a);
-            unsigned u0 = kClamp, u1 = kClamp;
-            if (k0 < (float)kClamp && k0 == truncf(k0))
-                u0 = (unsigned)k0;
-            else
-                big_until0 = y + W;
-            if (k1 < (float)kClamp && k1 == truncf(k1))
-                u1 = (unsigned)k1;
-            else
-                big_until1 = y + W;
-            return u0 | (u1 << 16);
-        };
-        // win[s] holds position x - W + s; ahead[q] the raw load of position
-        // x + W + 1 + q.  The loop is rolled and the window shifts by register
-        // moves, so the loop body stays small enough for the instruction cache.
-        uint32_t win[R];
-        float2 ahead[A];
-#pragma unroll
-        for (int s2 = 0; s2 < R; s2++)
-            win[s2] = pack(raw(x0 - W + s2), x0 - W + s2);
-#pragma unroll
-        for (int q = 0; q < A; q++)
-            ahead[q] = raw(x0 + W + 1 + q);
-        int need0 = 0, need1 = 0;
-#pragma unroll 1
-        for (int x = x0; x < x1; x++) {
-            uint32_t m = win[W];
-#pragma unroll
-            for (int d = 1; d <= W; d++) {
-                const uint32_t dd = (uint32_t)(d * d) * 0x10001u;
-                m = __viaddmin_u16x2(win[W - d], dd, m);
-                m = __viaddmin_u16x2(win[W + d], dd, m);
-            }
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const unsigned mh = h ? (m >> 16) : (m & 0xFFFFu);
-                // clean: every height in the window is an exact integer below the clamp
-                const bool clean = x > (h ? big_until1 : big_until0);
-                bool fin_ok = mh <= kFinal && clean;
-                const bool resume = mh > kFinal && clean;
-                if (fin_ok && periodic) {
-                    const unsigned el = (unsigned)((x + 1) * (x + 1)), er = (unsigned)((n - x) * (n - x));
-                    if (el < mh || er < mh) {
-                        // no solid voxel between x and that line end (it would
-                        // bound the minimum below): the scan runs off the line
-                        if (h)
-                            need1 |= 1;
-                        else
-                            need0 |= 1;
-                        continue;
-                    }
-                    if (el == mh || er == mh)
-                        fin_ok = false;
-                }
-                if (!fin_ok) {
-                    // deferred to k_env_slow
-                    if (!slow_push(slow, slow_count, slow_cap, slow_entry(li + h, x, resume, mh))) {
-                        if (h)
-                            need1 |= 2;
-                        else
-                            need0 |= 2;
-                    }
-                    continue;
-                }
-                float val = fmul((float)mh, a);
-                if (form == PMG_EDT_DIST)
-                    val = __fsqrt_rn(val);
-                o[x * st + h] = val;
-            }
-#pragma unroll
-            for (int s2 = 0; s2 < R - 1; s2++)
-                win[s2] = win[s2 + 1];
-            win[R - 1] = pack(ahead[0], x + W + 1);
-#pragma unroll
-            for (int q = 0; q < A - 1; q++)
-                ahead[q] = ahead[q + 1];
-            ahead[A - 1] = raw(x + W + 1 + A);
-        }
-        if (need0)
-            atomicOr(flag + li, need0);
-        if (need1)
-            atomicOr(flag + li + 1, need1);
-    }
-}
-
-// Contiguous lines (the last axis), 64 rows at a time: the rows' heights over
-// kRowsTX columns plus a W halo on each side are staged in shared memory as
-// packed 16-bit pairs (rows 2p, 2p + 1 in one word; a padded row stride keeps
-// the column walk free of bank conflicts), each thread walks 16 columns of
-// one row pair with the same register ring as k_env_pair, results go through
-// a shared tile to coalesced stores.  A row with a clamped height anywhere in
-// its staged span, an inconclusive minimum or a periodic end within reach
-// takes window_voxel on the row in global memory, as k_env_window does.
-constexpr int kRowsTX = 128;
-
-template <int W>
-constexpr size_t rows_smem_bytes()
-{
-    return sizeof(uint32_t) * 32 * (kRowsTX + 2 * W + 1) + sizeof(float) * 64 * (kRowsTX + 1) + sizeof(int) * 64;
-}
-
-template <int W>
-__global__ void __launch_bounds__(256) k_env_pair_rows(const float *__restrict__ fin, float *__restrict__ fout,
-                                                       Lines Ls, float a, float inv_a, int periodic, int form,
-                                                       int *__restrict__ flag, Probe probe,
-                                                       unsigned long long *__restrict__ slow,
-                                                       int *__restrict__ slow_count, int slow_cap)
-{
-    if (probe.choice() != window_choice<W>())
-        return;
-    constexpr int R = 2 * W + 1;
-    constexpr int SPAN = kRowsTX + 2 * W;
-    constexpr int SROW = SPAN + 1; // padded word stride of a pair row
-    constexpr unsigned kClamp = 65535u - (unsigned)(W * W) - 1u;
-    constexpr unsigned kFinal = (unsigned)((W + 1) * (W + 1));
-    constexpr float kSkip = -1.0f; // "left to k_env_slow or the end-segment replay"
-    extern __shared__ uint32_t rows_smem[];
-    uint32_t *sin = rows_smem;                                // [32][SROW]
-    float *sout = reinterpret_cast<float *>(sin + 32 * SROW); // [64][kRowsTX + 1]
-    int *sbig = reinterpret_cast<int *>(sout + 64 * (kRowsTX + 1));
-    __shared__ long long sbase[64]; // first element of each staged row
-    const long long nlines = Ls.count();
-    const int n = (int)Ls.s2;
-    const int ntx = (n + kRowsTX - 1) / kRowsTX;
-    const long long ntiles = ((nlines + 63) / 64) * ntx;
-    const uint32_t big = kClamp * 0x10001u;
-    const int tid = threadIdx.x;
-    // rows start on 16-byte boundaries when the row length is a multiple of 4
-    // (and the volume starts on one)
-    const bool vec4 = !(n & 3) && !(reinterpret_cast<uintptr_t>(fin) & 15);
-    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const long long li0 = (tile / ntx) * 64;
-        const int c0 = (int)(tile % ntx) * kRowsTX;
-        const int rows = (int)min(64LL, nlines - li0);
-        if (tid < 64) {
-            sbig[tid] = 0;
-            sbase[tid] = tid < rows ? line_addr(Ls, li0 + tid).base : 0;
-        }
-        __syncthreads();
-        // stage: (pair, 4-column group) items, columns fastest (coalesced
-        // rows); 16-byte loads where the rows allow them
-        auto pack = [&](int pr, float f0, float f1) -> uint32_t {
-            const float k0 = fmul(f0, inv_a), k1 = fmul(f1, inv_a);
-            unsigned u0 = kClamp, u1 = kClamp;
-            if (k0 < (float)kClamp && k0 == truncf(k0))
-                u0 = (unsigned)k0;
-            else
-                sbig[2 * pr] = 1;
-            if (k1 < (float)kClamp && k1 == truncf(k1))
-                u1 = (unsigned)k1;
-            else
-                sbig[2 * pr + 1] = 1;
-            return u0 | (u1 << 16);
-        };
-        static_assert(SPAN % 4 == 0 && W % 4 == 0, "4-column groups");
-        for (int it = tid; it < 32 * (SPAN / 4); it += blockDim.x) {
-            const int pr = it / (SPAN / 4), cc = (it - pr * (SPAN / 4)) * 4;
-            const int c = c0 - W + cc;
-            uint32_t wv[4] = {big, big, big, big};
-            if (2 * pr < rows) {
-                const long long b0 = sbase[2 * pr];
-                if (vec4 && c >= 0 && c + 3 < n) {
-                    const float4 f0 = __ldg(reinterpret_cast<const float4 *>(fin + b0 + c));
-                    const float4 f1 = __ldg(reinterpret_cast<const float4 *>(fin + b0 + (long long)n + c));
-                    wv[0] = pack(pr, f0.x, f1.x);
-                    wv[1] = pack(pr, f0.y, f1.y);
-                    wv[2] = pack(pr, f0.z, f1.z);
-                    wv[3] = pack(pr, f0.w, f1.w);
-                } else {
-#pragma unroll
-                    for (int q = 0; q < 4; q++)
-                        if (c + q >= 0 && c + q < n)
-                            wv[q] = pack(pr, fin[b0 + c + q], fin[b0 + (long long)n + c + q]);
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-                sin[pr * SROW + cc + q] = wv[q];
-        }
-        __syncthreads();
-        {
-            const int pr = tid & 31, seg = tid >> 5; // 8 segments of 16 columns
-            const uint32_t *row = sin + pr * SROW;
-            const int xs = c0 + seg * 16, xe = min(n, xs + 16);
-            int need0 = 0, need1 = 0;
-            const long long lia = li0 + 2 * pr;
-            if (2 * pr < rows && xs < xe) {
-                uint32_t win[R];
-#pragma unroll
-                for (int s2 = 0; s2 < R; s2++)
-                    win[s2] = row[seg * 16 + s2];
-#pragma unroll
-                for (int u = 0; u < 16; u++) {
-                    const int x = xs + u;
-                    if (x < xe) {
-                        uint32_t m = win[(u + W) % R];
-#pragma unroll
-                        for (int d = 1; d <= W; d++) {
-                            const uint32_t dd = (uint32_t)(d * d) * 0x10001u;
-                            m = __viaddmin_u16x2(win[(u + W - d) % R], dd, m);
-                            m = __viaddmin_u16x2(win[(u + W + d) % R], dd, m);
-                        }
-#pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            const unsigned mh = h ? (m >> 16) : (m & 0xFFFFu);
-                            const bool clean = !sbig[2 * pr + h];
-                            bool fin_ok = mh <= kFinal && clean;
-                            const bool resume = mh > kFinal && clean;
-                            if (fin_ok && periodic) {
-                                const unsigned el = (unsigned)((x + 1) * (x + 1)),
-                                               er = (unsigned)((n - x) * (n - x));
-                                if (el < mh || er < mh) {
-                                    // the scan would run off the line: flag it directly
-                                    if (h)
-                                        need1 |= 1;
-                                    else
-                                        need0 |= 1;
-                                    sout[(2 * pr + h) * (kRowsTX + 1) + (x - c0)] = kSkip;
-                                    continue;
-                                }
-                                if (el == mh || er == mh)
-                                    fin_ok = false;
-                            }
-                            if (!fin_ok) {
-                                // deferred to k_env_slow
-                                if (!slow_push(slow, slow_count, slow_cap, slow_entry(lia + h, x, resume, mh))) {
-                                    if (h)
-                                        need1 |= 2;
-                                    else
-                                        need0 |= 2;
-                                }
-                                sout[(2 * pr + h) * (kRowsTX + 1) + (x - c0)] = kSkip;
-                                continue;
-                            }
-                            float val = fmul((float)mh, a);
-                            if (form == PMG_EDT_DIST)
-                                val = __fsqrt_rn(val);
-                            sout[(2 * pr + h) * (kRowsTX + 1) + (x - c0)] = val;
-                        }
-                    }
-                    win[u % R] = row[seg * 16 + u + R < SPAN ? seg * 16 + u + R : SPAN - 1];
-                }
-            }
-            if (need0)
-                atomicOr(flag + lia, need0);
-            if (need1)
-                atomicOr(flag + lia + 1, need1);
-        }
-        __syncthreads();
-        // coalesced stores of the tile
-        const int tw = min(kRowsTX, n - c0);
-        for (int it = tid; it < rows * kRowsTX; it += blockDim.x) {
-            const int r = it / kRowsTX, c = it - r * kRowsTX;
-            if (c >= tw)
-                continue;
-            const float v = sout[r * (kRowsTX + 1) + c];
-            if (v != kSkip)
-                fout[sbase[r] + c0 + c] = v;
-        }
-        __syncthreads();
-    }
-}
-
-// Flagged lines, compacted: list[0 .. *count) gets the indices of the lines
-// whose flag is set (in no particular order), so the replay's warps only hold
-// lines with work.
-__global__ void k_flag_list(const int *__restrict__ flag, long long nlines, int *__restrict__ list,
-                            int *__restrict__ count)
-{
-    const int lane = threadIdx.x & 31;
-    for (long long base = (blockIdx.x * (long long)blockDim.x + threadIdx.x) - lane; base < nlines;
-         base += (long long)gridDim.x * blockDim.x) {
-        const long long li = base + lane;
-        const bool f = li < nlines && flag[li] != 0;
-        const unsigned bal = __ballot_sync(0xffffffffu, f);
-        if (!bal)
-            continue;
-        int pos = 0;
-        if (lane == 0)
-            pos = atomicAdd(count, __popc(bal));
-        pos = __shfl_sync(0xffffffffu, pos, 0);
-        if (f)
-            list[pos + __popc(bal & ((1u << lane) - 1u))] = (int)li;
-    }
-}
-
-// list (optional): the flagged lines' indices and their number (*count);
-// without it every line is visited and unflagged ones are skipped.
-__global__ void k_envelope_ends(const float *__restrict__ fin, float *__restrict__ fout, Lines Ls, float res,
-                                pmg_axis_cfg cfg, int num_hull, int form, const int *__restrict__ flag,
-                                const int *__restrict__ list, const int *__restrict__ count)
-{
-    const long long nlines = list ? (long long)*count : Ls.count();
-    extern __shared__ uint32_t smem_bm[];
-    const float aniso = fmul(res, res);
-    const MorphEpi none{};
     Stack S;
-    S.bm = smem_bm + threadIdx.x;
-    S.nthr = blockDim.x;
-    for (long long it = blockIdx.x * (long long)blockDim.x + threadIdx.x; it < nlines;
-         it += (long long)gridDim.x * blockDim.x) {
-        const long long li = list ? (long long)list[it] : it;
-        const int fl = flag[li];
-        if (!fl)
-            continue;
-        const LineGeo g = line_addr(Ls, li);
-        const float *line = fin + g.base;
-        const long long st = g.stride;
-        const int n = g.n;
-        const int nwords = (n + 31) >> 5;
-        int z1 = -1, z2 = -1;
-        for (int i = 0; i < n; i++)
-            if (line[i * st] == 0.0f) {
-                z1 = i;
-                break;
-            }
-        for (int i = n - 1; i >= 0; i--)
-            if (line[i * st] == 0.0f) {
-                z2 = i;
-                break;
-            }
+    S.bm = bm;
+    S.nthr = nthr;
+    const int n = g.n;
+    const int nwords = (n + 31) >> 5;
+    int z1 = -1, z2 = -1;
+    for (int i = 0; i < n; i++)
+        if (line(i) == 0.0f) {
+            z1 = i;
+            break;
+        }
+    for (int i = n - 1; i >= 0; i--)
+        if (line(i) == 0.0f) {
+            z2 = i;
+            break;
+        }
+    S.clear(nwords);
+    S.nl = 0;
+    S.nu = 0;
+    int up_v[kMaxHull];
+    float up_h[kMaxHull], up_r[kMaxHull];
+    int n_up = 0;
+    if (cfg.periodic)
+        load_imports(S, line, n, aniso, cfg, num_hull, up_v, up_h, up_r, n_up);
+    whole = whole || z1 < 0;
+    const int lo_end = whole ? n - 1 : z1; // last native of the lower stack
+    // lower part: the imports below, natives up to lo_end
+    if (whole || z1 > 0) {
+        int loop_start;
+        if (S.nl > 0) {
+            loop_start = 0;
+            S.nn = 0;
+            S.ntv = -1;
+            S.tv = S.lv[S.nl - 1];
+            S.th = S.lh[S.nl - 1];
+            S.tr = S.lr[S.nl - 1];
+        } else {
+            loop_start = 1;
+            S.setbit(0);
+            S.nn = 1;
+            S.ntv = 0;
+            S.tv = 0;
+            S.th = line(0);
+            S.tr = -INFINITY;
+        }
+        for (int i = loop_start; i <= lo_end; i++)
+            insert(S, line, i, line(i), aniso, 0);
+        if (whole) {
+            for (int j = 0; j < n_up; j++)
+                insert(S, line, up_v[j] + n, up_h[j], aniso, 1);
+            evaluate(S, line, nwords, aniso, form, me, g, fout + g.base, 0, n);
+            return;
+        }
+        evaluate(S, line, nwords, aniso, form, me, g, fout + g.base, 0, z1);
         S.clear(nwords);
+    }
+    // upper part: the zero at z2 at the bottom, natives above it, the upper
+    // imports on top
+    if (z2 < n - 1) {
         S.nl = 0;
         S.nu = 0;
-        int up_v[kMaxHull];
-        float up_h[kMaxHull], up_r[kMaxHull];
-        int n_up = 0;
-        if (cfg.periodic)
-            load_imports(S, line, st, n, aniso, cfg, num_hull, up_v, up_h, up_r, n_up);
-        const bool whole = (fl & 2) || z1 < 0;
-        const int lo_end = whole ? n - 1 : z1; // last native of the lower stack
-        // lower part: the imports below, natives up to lo_end
-        if (whole || z1 > 0) {
-            int loop_start;
-            if (S.nl > 0) {
-                loop_start = 0;
-                S.nn = 0;
-                S.ntv = -1;
-                S.tv = S.lv[S.nl - 1];
-                S.th = S.lh[S.nl - 1];
-                S.tr = S.lr[S.nl - 1];
-            } else {
-                loop_start = 1;
-                S.setbit(0);
-                S.nn = 1;
-                S.ntv = 0;
-                S.tv = 0;
-                S.th = vh(line, st, 0);
-                S.tr = -INFINITY;
-            }
-            for (int i = loop_start; i <= lo_end; i++)
-                insert(S, line, st, i, vh(line, st, i), aniso, 0);
-            if (whole) {
-                for (int j = 0; j < n_up; j++)
-                    insert(S, line, st, up_v[j] + n, up_h[j], aniso, 1);
-                evaluate(S, line, st, nwords, aniso, form, none, g, fout + g.base, 0, n);
-                S.clear(nwords);
-                continue;
-            }
-            evaluate(S, line, st, nwords, aniso, form, none, g, fout + g.base, 0, z1);
-            S.clear(nwords);
+        S.setbit(z2);
+        S.nn = 1;
+        S.ntv = z2;
+        S.tv = z2;
+        S.th = 0.0f;
+        S.tr = -INFINITY;
+        for (int i = z2 + 1; i < n; i++)
+            insert(S, line, i, line(i), aniso, 0);
+        for (int j = 0; j < n_up; j++)
+            insert(S, line, up_v[j] + n, up_h[j], aniso, 1);
+        evaluate(S, line, nwords, aniso, form, me, g, fout + g.base, z2 + 1, n);
+    }
+}
+
+// The first and last kEndWin heights of 32 adjacent lines (l0, l0 + 1, ...; g:
+// this lane's), staged by `parts` warps, this one being `part`.
+template <class T>
+__device__ __forceinline__ void stage_ends(float *se, const T *__restrict__ fin, const Lines &Ls, long long l0,
+                                           int lines, const LineGeo &g, float res, int part, int parts)
+{
+    const int lane = threadIdx.x & 31, n = g.n;
+    if (Ls.ax == 2) {
+        // rows: lanes along the row, transposed on the way in
+        const T *p0 = fin + line_addr(Ls, l0).base;
+#pragma unroll 4
+        for (int r = part; r < lines; r += parts) {
+            const T *p = p0 + (long long)r * Ls.s2;
+            const int u = n - kEndWin + lane;
+            if (lane < n)
+                se[lane * 33 + r] = height_of(p + lane, res);
+            if (u >= 0)
+                se[(kEndWin + lane) * 33 + r] = height_of(p + u, res);
         }
-        // upper part: the zero at z2 at the bottom, natives above it, the
-        // upper imports on top
-        if (z2 < n - 1) {
-            S.nl = 0;
-            S.nu = 0;
-            S.setbit(z2);
-            S.nn = 1;
-            S.ntv = z2;
-            S.tv = z2;
-            S.th = 0.0f;
-            S.tr = -INFINITY;
-            for (int i = z2 + 1; i < n; i++)
-                insert(S, line, st, i, vh(line, st, i), aniso, 0);
-            for (int j = 0; j < n_up; j++)
-                insert(S, line, st, up_v[j] + n, up_h[j], aniso, 1);
-            evaluate(S, line, st, nwords, aniso, form, none, g, fout + g.base, z2 + 1, n);
-            S.clear(nwords);
+    } else {
+        const T *p = fin + g.base;
+#pragma unroll 8
+        for (int v = part; v < kEndWin; v += parts) {
+            const int u = n - kEndWin + v;
+            if (v < n)
+                se[v * 33 + lane] = height_of(p + v * g.stride, res);
+            if (u >= 0)
+                se[(kEndWin + v) * 33 + lane] = height_of(p + u * g.stride, res);
         }
     }
+}
+
+// Flagged lines of any voxel size (flag bit 1: the whole line): one lane per
+// line, 32 adjacent lines per warp (unflagged ones idle); both ends of the
+// lines are staged in shared memory first, because the zero searches, hulls,
+// pushes and the sweep read them again and again in dependent steps.
+constexpr int kEndBlock = 64;
+
+__global__ void __launch_bounds__(kEndBlock) k_envelope_ends(const float *__restrict__ fin, float *__restrict__ fout,
+                                                             Lines Ls, float res, pmg_axis_cfg cfg, int num_hull,
+                                                             int form, MorphEpi me, const uint8_t *__restrict__ flag)
+{
+    extern __shared__ uint32_t smem_bm[];
+    __shared__ float s_ends[kEndBlock / 32][2 * kEndWin * 33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float *se = s_ends[w];
+    // tiles of 32 lines that are adjacent in memory (along the second axis)
+    const int tiles = (Ls.nb2 + 31) / 32;
+    const long long ntiles = (long long)Ls.nb1 * tiles;
+    for (long long t = blockIdx.x * (long long)(kEndBlock / 32) + w; t < ntiles;
+         t += (long long)gridDim.x * (kEndBlock / 32)) {
+        const int ra = (int)(t / tiles), kb = (int)(t - (long long)ra * tiles) * 32;
+        const int lines = min(32, Ls.nb2 - kb);
+        const long long l0 = (long long)ra * Ls.nb2 + kb;
+        const int fl = lane < lines ? flag[l0 + lane] : 0;
+        if (!__any_sync(0xffffffffu, fl))
+            continue;
+        const LineGeo g = line_addr(Ls, l0 + min(lane, lines - 1));
+        __syncwarp();
+        stage_ends(se, fin, Ls, l0, lines, g, res, 0, 1);
+        __syncwarp();
+        if (!fl)
+            continue;
+        const LineEnds<float> line{fin + g.base, g.stride, se + lane, 33, g.n, 0, res};
+        replay_line(smem_bm + threadIdx.x, kEndBlock, line, g, fmul(res, res), cfg, num_hull, (fl & 2) != 0, form, me,
+                    fout);
+    }
+}
+
+// Flagged lines of the lattice passes (flag bits 0 and 2: the low and the high
+// end, bit 1: the whole line).  Heights are integer multiples K of res^2, so a
+// voxel before the first zero (after the last one) is the smaller of the value
+// the pass left there and the imported parabolas, and only the imports have to
+// be found: the last (first) num_hull + 1 finite entries of the hull of the
+// far (near) segment.  They are wrapped one by one from the line's end -- the
+// entry next to e is the vertex whose intersection with e lies closest, of
+// equal ones the farthest (the reference pops on equality) -- by
+// cross-multiplied integer comparisons.  The reference compares rounded
+// quotients: a comparison closer than their rounding (kept in `hard`) leaves
+// the line to the float replay, and so do lines flagged as a whole, segments
+// too long for 32-bit products, and longer lines without a zero (there the
+// rounding of intersections across the whole line could reach the distance to
+// an integer).  A block takes 32 adjacent lines, warp 0 their low ends and
+// warp 1 their high ones, so that the two independent chains overlap.
+// Building the reference's hull stacks instead kept a warp in divergent
+// pops and divisions: 1024^3 field 1.8 ms over both passes, 128^3 pack 0.54 ms.
+constexpr int kWrapMax = 255;   // longest segment (products below 2^31)
+constexpr int kWrapLine = 320;  // longest line without a zero
+
+template <class T>
+__global__ void __launch_bounds__(64) k_lattice_ends(const T *__restrict__ fin, float *__restrict__ fout, Lines Ls,
+                                                     float res, pmg_axis_cfg cfg, int num_hull, int form,
+                                                     const uint8_t *__restrict__ flag)
+{
+    extern __shared__ uint32_t smem_bm[]; // envelope bits of the replays: [nwords][32]
+    __shared__ float s_ends[2 * kEndWin * 33];
+    __shared__ int s_hard[32];
+    const float aniso = fmul(res, res), inv_a = 1.0f / aniso;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int tiles = (Ls.nb2 + 31) / 32;
+    const long long ntiles = (long long)Ls.nb1 * tiles;
+    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const int ra = (int)(t / tiles), kb = (int)(t - (long long)ra * tiles) * 32;
+        const int lines = min(32, Ls.nb2 - kb);
+        const long long l0 = (long long)ra * Ls.nb2 + kb;
+        const int fl = lane < lines ? flag[l0 + lane] : 0;
+        if (!__any_sync(0xffffffffu, fl)) // the same for both warps
+            continue;
+        const LineGeo g = line_addr(Ls, l0 + min(lane, lines - 1));
+        const int n = g.n;
+        __syncthreads(); // (the previous tile's readers)
+        if (w == 0)
+            s_hard[lane] = fl & 2;
+        stage_ends(s_ends, fin, Ls, l0, lines, g, res, w, 2);
+        __syncthreads();
+        const LineEnds<T> line{fin + g.base, g.stride, s_ends + lane, 33, n, 0, res};
+        if (!(fl & 2) && (fl & (w == 0 ? 1 : 4))) {
+            // positions of the segment from its end that faces the line: q = 0
+            // is that end, q = nv - 1 the zero that bounds it
+            const int p0 = w == 0 ? n - cfg.hb_hi - 1 : cfg.hf_lo, dir = w == 0 ? -1 : 1;
+            const int most = w == 0 ? n - cfg.hb_hi : n - cfg.hf_lo;
+            int nv = 0;
+            bool zero = false;
+            while (nv < most && !zero)
+                zero = line(p0 + dir * nv++) == 0.0f;
+            bool hard = nv < 1 || nv > kWrapMax || (!zero && (n > kWrapLine || nv < 2));
+            // entries (position q, height K); q = -1: none
+            int eq[kMaxHull], ek[kMaxHull];
+#pragma unroll
+            for (int c = 0; c < kMaxHull; c++) {
+                eq[c] = -1;
+                ek[c] = 0;
+            }
+            if (!hard) {
+                auto height = [&](int q) -> int {
+                    const float f = line(p0 + dir * q);
+                    return f >= FLT_MAX ? -1 : (int)fmul(f, inv_a);
+                };
+                int e = 0, ke = height(0);
+                while (ke < 0 && ++e < nv)
+                    ke = height(e);
+                if (e < nv) {
+                    eq[0] = e;
+                    ek[0] = ke;
+                }
+#pragma unroll
+                for (int c = 1; c < kMaxHull; c++) {
+                    if (c > num_hull || e >= nv)
+                        continue;
+                    // distance from e of the intersection with q: N / D, smallest
+                    int b = nv, kb2 = 0, nb = 0, db = 1;
+                    bool near = false; // another one within the rounding of the best
+                    for (int q = e + 1; q < nv; q++) {
+                        const int k = height(q);
+                        if (k < 0)
+                            continue;
+                        const int d = q - e, N = k - ke + d * d;
+                        const int diff = N * db - nb * d;
+                        const float tol = 2.4e-7f * (float)(2 * max(k, max(ke, kb2)) + 6 * nv) * (float)(d * db);
+                        if (b < nv && diff != 0 && (float)abs(diff) < tol)
+                            near = true;
+                        else if (b == nv || diff < 0)
+                            near = false;
+                        if (b == nv || diff <= 0) {
+                            b = q;
+                            kb2 = k;
+                            nb = N;
+                            db = d;
+                        }
+                    }
+                    hard = hard || near;
+                    e = b;
+                    ke = kb2;
+                    if (e < nv) {
+                        eq[c] = e;
+                        ek[c] = ke;
+                    }
+                }
+            }
+            if (hard) {
+                s_hard[lane] = 1;
+            } else {
+                // import c lies eq[c] + 1 beyond the line's end
+                for (int i = 0; i < n; i++) {
+                    const int x = w == 0 ? i : n - 1 - i;
+                    if (line(x) == 0.0f)
+                        break;
+                    int best = 1 << 30;
+#pragma unroll
+                    for (int c = 0; c < kMaxHull; c++)
+                        if (eq[c] >= 0) {
+                            const int d = i + 1 + eq[c];
+                            best = min(best, ek[c] + d * d);
+                        }
+                    if (best == 1 << 30)
+                        break;
+                    float val = fmul((float)best, aniso);
+                    if (form == PMG_EDT_DIST)
+                        val = __fsqrt_rn(val);
+                    // (both ends of a line without a zero meet here; values are >= 0)
+                    float *o = fout + g.base + x * g.stride;
+                    if (val < *o)
+                        atomicMin(reinterpret_cast<int *>(o), __float_as_int(val));
+                }
+            }
+        }
+        __syncthreads();
+        if (w == 0 && s_hard[lane])
+            replay_line(smem_bm + lane, 32, line, g, aniso, cfg, num_hull, (fl & 2) != 0, form, MorphEpi{}, fout);
+    }
+}
+
+template <class T>
+static int launch_lattice_ends(const T *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
+                               int num_hull, int form, const uint8_t *flag, cudaStream_t st)
+{
+    const int n = (int)(Ls.ax == 0 ? Ls.s0 : Ls.ax == 1 ? Ls.s1 : Ls.s2);
+    const size_t smem = (size_t)((n + 31) / 32) * 32 * 4;
+    const long long tiles = (long long)Ls.nb1 * ((Ls.nb2 + 31) / 32);
+    const int ps__ = prof_begin("k_lattice_ends", st);
+    k_lattice_ends<T><<<grid_for(tiles, 1, 152LL * 64), 64, smem, st>>>(fin, fout, Ls, res, cfg, num_hull, form, flag);
+    prof_end(ps__, 0.0, st);
+    PMG_CHECK_LAUNCH();
+    return PMG_OK;
+}
+
+int launch_ends_counts(const uint16_t *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
+                       int num_hull, const uint8_t *flag, cudaStream_t st)
+{
+    return launch_lattice_ends(fin, fout, Ls, res, cfg, num_hull, PMG_EDT_SQUARED, flag, st);
+}
+
+int launch_ends_heights(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
+                        int num_hull, int form, const uint8_t *flag, cudaStream_t st)
+{
+    return launch_lattice_ends(fin, fout, Ls, res, cfg, num_hull, form, flag, st);
+}
+
+int launch_ends_float(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
+                      int num_hull, int form, const MorphEpi &me, const uint8_t *flag, cudaStream_t st)
+{
+    const int n = (int)(Ls.ax == 0 ? Ls.s0 : Ls.ax == 1 ? Ls.s1 : Ls.s2);
+    const size_t smem = (size_t)((n + 31) / 32) * kEndBlock * 4;
+    const long long tiles = (long long)Ls.nb1 * ((Ls.nb2 + 31) / 32);
+    const int ps__ = prof_begin("k_envelope_ends", st);
+    k_envelope_ends<<<grid_for(tiles, kEndBlock / 32, 152LL * 64), kEndBlock, smem, st>>>(
+        fin, fout, Ls, res, cfg, num_hull, form, me, flag);
+    prof_end(ps__, 0.0, st);
+    PMG_CHECK_LAUNCH();
+    return PMG_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -1463,14 +922,7 @@ int launch_pass0(const uint8_t *img, float *out, const Lines &Ls, float res,
     const int block = 256;
     {
         const int ps__ = prof_begin("k_pass0", st);
-        // four adjacent strided lines per thread where the quads align to 16
-        // bytes (float4) and 4 bytes (uchar4)
-        const bool quads = Ls.ax != 2 && !(Ls.nb2 & 3) && !(Ls.b2lo & 3) && !(Ls.s2 & 3) &&
-                           !(reinterpret_cast<uintptr_t>(out) & 15) && !(reinterpret_cast<uintptr_t>(img) & 3);
-        if (quads)
-            k_pass0_x4<<<grid_for(Ls.count() >> 2, block, 1LL << 30), block, 0, st>>>(img, out, Ls, res, cfg);
-        else
-            k_pass0<<<grid_for(Ls.count(), block, 1LL << 30), block, 0, st>>>(img, out, Ls, res, cfg);
+        k_pass0<<<grid_for(Ls.count(), block, 1LL << 30), block, 0, st>>>(img, out, Ls, res, cfg);
         prof_end(ps__, (double)Ls.count() * (Ls.ax == 0 ? Ls.s0 : Ls.ax == 1 ? Ls.s1 : Ls.s2) * 5, st);
     }
     PMG_CHECK_LAUNCH();
@@ -1490,9 +942,9 @@ static int envelope_block(int n)
 // power-of-two voxel size and lines of at most 1024 voxels (imported hull
 // vertices then stay within the exact float range of the reference's
 // intersection arithmetic)
-static bool window_path_ok(float res, int n)
+bool window_path_ok(float res, int n)
 {
-    if (n > 1024 || !(res > 0.0f))
+    if (n > kScanMaxLine || !(res > 0.0f))
         return false;
     int ex = 0;
     const float m = frexpf(res, &ex);
@@ -1501,7 +953,7 @@ static bool window_path_ok(float res, int n)
 
 int launch_envelope(const float *fin, float *fout, const Lines &Ls, float res,
                     const pmg_axis_cfg &cfg, int num_hull, int form, const MorphEpi &me,
-                    cudaStream_t st, int cap, int *flag_buf, long long flag_cap)
+                    cudaStream_t st, int cap, int *flag_buf, long long flag_cap, float vcap)
 {
     const int n = (int)(Ls.ax == 0 ? Ls.s0 : Ls.ax == 1 ? Ls.s1 : Ls.s2);
     int block = envelope_block(n);
@@ -1510,150 +962,15 @@ int launch_envelope(const float *fin, float *fout, const Lines &Ls, float res,
         PMG_CUDA(cudaFuncSetAttribute(k_envelope, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
     const int path = tune_value(kTuneEdtPath);
-    if (form != PMG_EDT_MORPH && window_path_ok(res, n) && path == 0) {
-        // windowed exact minimum everywhere, the float envelope on the end
-        // segments of periodic lines (or whole lines) the window kernel flags
-        const long long nl = Ls.count();
-        // The library's own buffer (ints): flags [0, nl) | the flagged-line
-        // list [nl, 2nl) | its count | the probe's count | the deferred count |
-        // the deferred voxels (8-byte entries).  A caller's buffer of flag_cap
-        // ints: flags in its first half (one block of rows at a time), then
-        // the two counts and the deferred voxels; no flagged-line list.
-        int *flag = flag_buf, *probe = nullptr, *slow_cnt = nullptr;
-        unsigned long long *slow = nullptr;
-        long long fcap = nl, slow_cap = 0;
-        if (!flag_buf) {
-            slow_cap = std::min<long long>(nl * n / 16 + 1024, 1LL << 27);
-            const size_t head = ((sizeof(int) * (size_t)(2 * nl + 5)) + 15) & ~(size_t)15;
-            void *mem = nullptr;
-            PMG_TRY(scratch_alloc(&mem, head + sizeof(unsigned long long) * (size_t)slow_cap, st));
-            flag = (int *)mem;
-            probe = flag + 2 * nl + 1;
-            slow = (unsigned long long *)((char *)mem + head);
-        } else {
-            fcap = flag_cap / 2;
-            probe = flag_buf + fcap;
-            const uintptr_t lo = ((uintptr_t)(probe + 4) + 15) & ~(uintptr_t)15, hi = (uintptr_t)(flag_buf + flag_cap);
-            slow = (unsigned long long *)lo;
-            slow_cap = hi > lo ? (long long)((hi - lo) / sizeof(unsigned long long)) : 0;
-        }
-        slow_cnt = probe + 3;
-        const bool rows_pass = Ls.ax == 2;
-        // the +-24 window only for strided passes of many lines (on small
-        // volumes its 106-register grid runs too few warps and the envelope
-        // is faster), unless its threshold is 8193 (always)
-        const int wide = tune_value(kTuneEdtWide);
-        const Probe pr{probe, tune_value(rows_pass ? kTuneEdtNarrowRows : kTuneEdtNarrow),
-                       tune_value(rows_pass ? kTuneEdtFallbackRows : kTuneEdtFallback),
-                       rows_pass || (nl < (1LL << 17) && wide < 8193) ? 0 : wide};
-        // a caller-supplied flag buffer smaller than the line count is used
-        // for one block of rows (lines along the first other axis) at a time
-        const int rows = flag_buf ? (int)std::min<long long>(Ls.nb1, std::max<long long>(1, fcap / Ls.nb2))
-                                  : Ls.nb1;
-        int s = PMG_OK;
-        if (flag_buf && (long long)Ls.nb2 > fcap) {
-            set_error("envelope: flag buffer of %lld lines holds less than one row of %d lines", fcap, Ls.nb2);
-            s = PMG_EINVAL;
-        }
-        for (int r0 = 0; s == PMG_OK && r0 < Ls.nb1; r0 += rows) {
-            Lines C = Ls;
-            C.b1lo = Ls.b1lo + r0;
-            C.nb1 = std::min(rows, Ls.nb1 - r0);
-            const long long nc = C.count();
-            s = cudaMemsetAsync(flag, 0, sizeof(int) * (size_t)nc, st) == cudaSuccess ? PMG_OK : PMG_ECUDA;
-            if (s == PMG_OK) // the probe's three counts and the deferred count
-                s = cudaMemsetAsync(probe, 0, 4 * sizeof(int), st) == cudaSuccess ? PMG_OK : PMG_ECUDA;
-            if (s == PMG_OK) {
-                const int ps__ = prof_begin("k_env_probe", st);
-                k_env_probe<<<kProbe / 256, 256, 0, st>>>(fin, C, 1.0f / (res * res), probe);
-                prof_end(ps__, 0.0, st);
-            }
-            if (s == PMG_OK) {
-                const float a = res * res;
-                const bool contiguous = C.ax == 2;
-                constexpr int kAhead = 5;
-                if (!contiguous && !(C.nb2 & 1) && !(C.b2lo & 1)) {
-                    // line pairs along the contiguous axis (float2 aligned);
-                    // the +-8 and +-12 kernels both launch, the probe runs one
-                    const int seg = tune_value(kTuneEdtPairSeg);
-                    const long long work = (nc >> 1) * ((n + seg - 1) / seg);
-                    const unsigned grid = (unsigned)grid_for(work, 256, 152LL * tune_value(kTuneEdtPairCtas));
-                    const int ps__ = prof_begin("k_env_pair", st);
-                    k_env_pair<8, kAhead><<<grid, 256, 0, st>>>(fin, fout, C, a, 1.0f / a, cfg.periodic ? 1 : 0, form,
-                                                                flag, seg, pr, slow, slow_cnt, (int)slow_cap);
-                    k_env_pair<12, kAhead><<<grid, 256, 0, st>>>(fin, fout, C, a, 1.0f / a, cfg.periodic ? 1 : 0,
-                                                                 form, flag, seg, pr, slow, slow_cnt, (int)slow_cap);
-                    if (pr.thr24 > 0)
-                        k_env_pair<24, kAhead><<<grid, 256, 0, st>>>(fin, fout, C, a, 1.0f / a,
-                                                                     cfg.periodic ? 1 : 0, form, flag, seg, pr, slow,
-                                                                     slow_cnt, (int)slow_cap);
-                    prof_end(ps__, (double)nc * n * 8, st);
-                } else if (contiguous && !(C.nb2 & 1) && !(C.b2lo & 1)) {
-                    // row pairs through shared-memory tiles
-                    const long long tiles = ((nc + 63) / 64) * ((n + kRowsTX - 1) / kRowsTX);
-                    const unsigned grid = (unsigned)std::min<long long>(tiles, 152LL * tune_value(kTuneEdtRowsCtas));
-                    const size_t sm8 = rows_smem_bytes<8>(), sm12 = rows_smem_bytes<12>();
-                    s = cudaFuncSetAttribute(k_env_pair_rows<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)sm8) == cudaSuccess &&
-                                cudaFuncSetAttribute(k_env_pair_rows<12>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)sm12) == cudaSuccess
-                            ? PMG_OK
-                            : PMG_ECUDA;
-                    const int ps__ = prof_begin("k_env_pair_rows", st);
-                    if (s == PMG_OK) {
-                        k_env_pair_rows<8><<<grid, 256, sm8, st>>>(fin, fout, C, a, 1.0f / a, cfg.periodic ? 1 : 0,
-                                                                  form, flag, pr, slow, slow_cnt, (int)slow_cap);
-                        k_env_pair_rows<12><<<grid, 256, sm12, st>>>(fin, fout, C, a, 1.0f / a,
-                                                                    cfg.periodic ? 1 : 0, form, flag, pr, slow,
-                                                                    slow_cnt, (int)slow_cap);
-                    }
-                    prof_end(ps__, (double)nc * n * 8, st);
-                } else {
-                    const int ps__ = prof_begin("k_env_window", st);
-                    k_env_window<<<grid_for(contiguous ? nc * 32 : nc * ((n + 63) / 64), 256, 152LL * 32), 256, 0,
-                                   st>>>(fin, fout, C, a, 1.0f / a, cfg.periodic ? 1 : 0, form, flag, pr);
-                    prof_end(ps__, (double)nc * n * 8, st);
-                }
-                if (s == PMG_OK)
-                    s = cudaGetLastError() == cudaSuccess ? PMG_OK : PMG_ECUDA;
-                if (s == PMG_OK && !(C.nb2 & 1) && !(C.b2lo & 1)) {
-                    // the voxels the line-pair kernels deferred
-                    const int ps__ = prof_begin("k_env_slow", st);
-                    k_env_slow<<<152 * 8, 256, 0, st>>>(fin, fout, C, a, 1.0f / a, cfg.periodic ? 1 : 0, form, flag,
-                                                        slow, slow_cnt, (int)slow_cap, pr);
-                    prof_end(ps__, 0.0, st);
-                    s = cudaGetLastError() == cudaSuccess ? PMG_OK : PMG_ECUDA;
-                }
-            }
-            if (s == PMG_OK) {
-                // the library's own flag buffer has room for the compacted list
-                // of flagged lines after the flags; a caller's buffer is used
-                // as it is (every line visited)
-                int *list = flag_buf ? nullptr : flag + nl, *cnt = flag_buf ? nullptr : flag + 2 * nl;
-                if (list) {
-                    s = cudaMemsetAsync(cnt, 0, sizeof(int), st) == cudaSuccess ? PMG_OK : PMG_ECUDA;
-                    const int ps__ = prof_begin("k_flag_list", st);
-                    if (s == PMG_OK)
-                        k_flag_list<<<grid_for(nc, 256, 152LL * 16), 256, 0, st>>>(flag, nc, list, cnt);
-                    prof_end(ps__, (double)nc * 4, st);
-                }
-                const int ps__ = prof_begin("k_envelope_ends", st);
-                if (s == PMG_OK)
-                    k_envelope_ends<<<grid_for(nc, block, 1LL << 30), block, smem, st>>>(
-                        fin, fout, C, res, cfg, num_hull, form, flag, list, cnt);
-                prof_end(ps__, 0.0, st);
-                if (s == PMG_OK)
-                    s = cudaGetLastError() == cudaSuccess ? PMG_OK : PMG_ECUDA;
-            }
-            if (s == PMG_OK) {
-                // the whole pass on the float envelope when the probe chose it
-                const int ps__ = prof_begin("k_envelope[probed]", st);
-                k_envelope<<<grid_for(nc, block, 1LL << 30), block, smem, st>>>(
-                    fin, fout, C, res, cfg, num_hull, form, MorphEpi{}, 0, pr);
-                prof_end(ps__, 0.0, st);
-                s = cudaGetLastError() == cudaSuccess ? PMG_OK : PMG_ECUDA;
-            }
-        }
+    // the outward scan; a caller's flag buffer that does not hold one byte per
+    // line (lines of a few voxels) leaves the pass to the float envelope
+    if (path == 0 && n <= kScanMaxLine && (!flag_buf || Ls.count() <= flag_cap * (long long)sizeof(int))) {
+        uint8_t *flag = (uint8_t *)flag_buf;
+        if (!flag_buf)
+            PMG_TRY(scratch_alloc((void **)&flag, (size_t)Ls.count(), st));
+        int s = launch_scan(fin, fout, Ls, res, cfg, form, me, vcap, flag, st);
+        if (s == PMG_OK)
+            s = launch_ends_float(fin, fout, Ls, res, cfg, num_hull, form, me, flag, st);
         const int s2 = flag_buf ? PMG_OK : scratch_free(flag, st);
         return s != PMG_OK ? s : s2;
     }
@@ -1666,7 +983,7 @@ int launch_envelope(const float *fin, float *fout, const Lines &Ls, float res,
     {
         const int ps__ = prof_begin(redo ? "k_envelope_redo" : "k_envelope", st);
         k_envelope<<<grid_for(Ls.count(), block, redo ? 152LL * 8 : 1LL << 30), block, smem, st>>>(
-            fin, fout, Ls, res, cfg, num_hull, form, me, redo, Probe{nullptr, 0, 0, 0});
+            fin, fout, Ls, res, cfg, num_hull, form, me, redo);
         prof_end(ps__, redo ? 0.0 : (double)Ls.count() * n * 4 + (form == PMG_EDT_MORPH ? (double)Ls.count() * me.o2 : (double)Ls.count() * n * 4), st);
     }
     PMG_CHECK_LAUNCH();
@@ -1689,6 +1006,16 @@ static int check_shape(const int64_t *shape, int nd)
     return PMG_OK;
 }
 
+// The linear pass of any voxel size: counts through the table of the running
+// sums, except where periodic correctors start the sums elsewhere.
+int launch_linear(const uint8_t *img, float *out, const int64_t *shape, float res, const pmg_axis_cfg &cfg,
+                  cudaStream_t st)
+{
+    if (tune_value(kTuneEdtPath) == 0 && !cfg.periodic && lin_ok((int)shape[0], cfg))
+        return launch_lin_float(img, out, shape, res, cfg, st);
+    return launch_pass0(img, out, all_lines(shape, 0), res, cfg, st);
+}
+
 // EDT with one ping-pong buffer: pass 0 -> out, envelope 1: out -> tmp,
 // envelope 2: tmp -> out.
 int edt3d_run(const uint8_t *img, float *out, float *tmp, const int64_t *shape, const float *res,
@@ -1696,7 +1023,17 @@ int edt3d_run(const uint8_t *img, float *out, float *tmp, const int64_t *shape, 
               long long flag_cap)
 {
     MorphEpi none{};
-    PMG_TRY(launch_pass0(img, out, all_lines(shape, 0), res[0], cfg[0], st));
+    const long long lines = (long long)shape[0] * std::max(shape[1], shape[2]);
+    if (tune_value(kTuneEdtPath) == 0 && lattice_ok(shape, res, cfg) &&
+        (!flag_buf || lines <= flag_cap * (long long)sizeof(int))) {
+        uint8_t *flag = (uint8_t *)flag_buf;
+        if (!flag_buf)
+            PMG_TRY(scratch_alloc((void **)&flag, (size_t)lines, st));
+        const int s = lattice_run(img, out, tmp, shape, res, cfg, num_hull, form, flag, st);
+        const int s2 = flag_buf ? PMG_OK : scratch_free(flag, st);
+        return s != PMG_OK ? s : s2;
+    }
+    PMG_TRY(launch_linear(img, out, shape, res[0], cfg[0], st));
     PMG_TRY(launch_envelope(out, tmp, all_lines(shape, 1), res[1], cfg[1], num_hull,
                             PMG_EDT_SQUARED, none, st, INT_MAX, flag_buf, flag_cap));
     PMG_TRY(launch_envelope(tmp, out, all_lines(shape, 2), res[2], cfg[2], num_hull, form, none,

@@ -161,11 +161,41 @@ int edt_cap_run(const uint8_t *E, uint16_t *KA, uint16_t *KB, uint16_t *KC, cons
 
 int launch_pass0(const uint8_t *img, float *out, const Lines &Ls, float res,
                  const pmg_axis_cfg &cfg, cudaStream_t st);
-// flag_buf (optional): per-line flags of the windowed path, flag_cap lines
-// long; without it the flags come from the stream-ordered scratch pool.
+// Longest line of k_lin, and of the envelope passes that hold a line on chip.
+constexpr int kLinMaxLine = 2048, kScanMaxLine = 1024;
+bool window_path_ok(float res, int n);
+// The linear pass along axis 0 (edt_lattice.cu): as counts (>= 0x4000: no
+// zero), or as squared distances (no periodic axis).
+bool lin_ok(int n, const pmg_axis_cfg &cfg);
+int launch_lin_counts(const uint8_t *img, uint16_t *out, const int64_t *shape, const pmg_axis_cfg &cfg,
+                      cudaStream_t st);
+int launch_lin_float(const uint8_t *img, float *out, const int64_t *shape, float res, const pmg_axis_cfg &cfg,
+                     cudaStream_t st);
+int launch_linear(const uint8_t *img, float *out, const int64_t *shape, float res, const pmg_axis_cfg &cfg,
+                  cudaStream_t st);
+// The whole transform on the integer lattice.
+bool lattice_ok(const int64_t *shape, const float *res, const pmg_axis_cfg *cfg);
+int lattice_run(const uint8_t *img, float *out, float *tmp, const int64_t *shape, const float *res,
+                const pmg_axis_cfg *cfg, int num_hull, int form, uint8_t *flags, cudaStream_t st);
+// Flagged lines: after a lattice pass over counts or heights (one byte per
+// line: 1 the low end, 4 the high end, 2 the whole line), and after a scan (1
+// the ends, 2 the whole line).
+int launch_ends_counts(const uint16_t *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
+                       int num_hull, const uint8_t *flag, cudaStream_t st);
+int launch_ends_heights(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
+                        int num_hull, int form, const uint8_t *flag, cudaStream_t st);
+int launch_ends_float(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
+                      int num_hull, int form, const MorphEpi &me, const uint8_t *flag, cudaStream_t st);
+// The outward scan (edt_scan.cu), lines of at most kScanMaxLine voxels; vcap:
+// values above it only matter as "above it".
+int launch_scan(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg, int form,
+                const MorphEpi &me, float vcap, uint8_t *flag, cudaStream_t st);
+// flag_buf (optional): flag_cap ints for the per-line flags; without it they
+// come from the stream-ordered scratch pool.
 int launch_envelope(const float *fin, float *fout, const Lines &Ls, float res,
                     const pmg_axis_cfg &cfg, int num_hull, int form, const MorphEpi &me,
-                    cudaStream_t st, int cap = INT_MAX, int *flag_buf = nullptr, long long flag_cap = 0);
+                    cudaStream_t st, int cap = INT_MAX, int *flag_buf = nullptr, long long flag_cap = 0,
+                    float vcap = INFINITY);
 int edt3d_run(const uint8_t *img, float *out, float *tmp, const int64_t *shape, const float *res,
               const pmg_axis_cfg *cfg, int num_hull, int form, cudaStream_t st, int *flag_buf = nullptr,
               long long flag_cap = 0);

@@ -1,0 +1,701 @@
+// Distance transform of isotropic power-of-two voxels on an integer lattice
+// (sm_103a), and the linear pass of every other voxel size.
+//
+// With one power-of-two voxel size res every height of the transform is
+// K * res^2 with an integer K, and the reference's float passes return the
+// exact minimum (edt_exact.cu has the rounding argument), so the passes run on
+// integers:
+//
+//  * k_lin       the linear pass (squared_edt_1d, _distance.hpp:135-182, with
+//                the correctors of _distance.pyx:240-279): counts of voxels to
+//                the nearest zero or restart, uint16, every position of a line
+//                by its own segment of threads;
+//  * k_par_cols  a strided envelope pass: min over v of K(v) + (x - v)^2;
+//  * k_par_rows  the same along the contiguous axis, out to float32.
+//
+// min over |d| <= k of K(x + d) + d^2 is built one distance at a time as
+//     g_k(x) = min(g_{k-1}(x), min(g_{k-1}(x - 1), g_{k-1}(x + 1)) + 2k - 1)
+// (d^2 = 1 + 3 + ... + (2d - 1); a path that turns back costs more), with the
+// line's heights in registers, two lines packed in the halves of 32-bit words.
+// It stops as soon as every value of the block (warp) is at most (k + 1)^2,
+// because a height farther away adds at least that much: the work follows
+// the medium's own distances, with no window to choose beforehand.
+//
+// Periodic lines: a voxel whose minimum exceeds the squared distance to a
+// line end may depend on the imported boundary hulls; that end of its line is
+// flagged (k_lattice_ends).  Heights of kBig and more
+// count as absent; a line left with such a value is flagged for the float
+// envelope, unless no height of the volume can reach kBig.
+#include <cfloat>
+#include <algorithm>
+
+#include "edt_internal.cuh"
+
+namespace pmg {
+
+// ---------------------------------------------------------------------------
+// linear pass
+// ---------------------------------------------------------------------------
+// "No zero so far": counts grow from here by at most the line length.
+constexpr int kLinInf = 0x4000;
+constexpr int kLinChunk = 16;      // positions a thread holds at once
+constexpr int kLinChunks = 8;      // chunks per thread
+constexpr int kLinWarps = 16;      // segments per line
+
+struct LinTab {
+    float v[kLinMaxLine + 1]; // squared distance of a count
+};
+struct NoTab {};
+template <class OUT>
+struct TabOf {
+    using T = NoTab;
+};
+template <>
+struct TabOf<float> {
+    using T = LinTab;
+};
+
+// bytes != 0 -> 0x01 per byte
+__device__ __forceinline__ uint32_t nz01(uint32_t v)
+{
+    return ((((v & 0x7f7f7f7fu) + 0x7f7f7f7fu) | v) >> 7) & 0x01010101u;
+}
+
+// two of the four 0/1 bytes as 16-bit masks (pair 0: bytes 0 and 1)
+template <int PAIR>
+__device__ __forceinline__ uint32_t mask2(uint32_t b)
+{
+    return __byte_perm(b, 0u, PAIR ? 0x4342 : 0x4140) * 0xFFFFu;
+}
+
+// Lines along axis 0 of [n][plane], VEC adjacent lines per lane (VEC = 4 where
+// plane and the pointers are multiples of 4, else 1), blockDim = (32, segments
+// of `seg` positions).  Each thread first runs its segment from "unknown" in
+// both directions (what it hands on to the neighbouring segments is the
+// smaller of its own count and the incoming one plus its length), then, with
+// the true incoming counts, computes both directions chunk by chunk in
+// registers and writes each output once.  An event is a zero (count 0) or a
+// change between nonzero values (count 1 on both sides).
+// Bound by HBM: 1 byte read (twice, the second time from cache) and 2 (4)
+// written per voxel.
+template <int VEC, class OUT>
+__global__ void __launch_bounds__(32 * kLinWarps) k_lin(const uint8_t *__restrict__ img, OUT *__restrict__ out,
+                                                        long long plane, int n, int seg, pmg_axis_cfg cfg,
+                                                        const __grid_constant__ typename TabOf<OUT>::T tab)
+{
+    constexpr int H = VEC == 4 ? 2 : 1; // 32-bit words of two counts
+    constexpr uint32_t kInf2 = (uint32_t)kLinInf * 0x10001u;
+    __shared__ uint32_t s_f[kLinWarps][H][32], s_b[kLinWarps][H][32];
+    __shared__ uint32_t s_corr[2][H][32];
+    extern __shared__ float s_tab[];
+    const int lane = threadIdx.x, w = threadIdx.y, nw = blockDim.y;
+    if constexpr (sizeof(OUT) == 4)
+        for (int q = w * 32 + lane; q <= n; q += nw * 32)
+            s_tab[q] = tab.v[q];
+    const long long line = ((long long)blockIdx.x * 32 + lane) * VEC;
+    const bool live = line < plane;
+    const uint8_t *in = img + (live ? line : 0);
+    auto row = [&](int i) -> uint32_t {
+        if constexpr (VEC == 4)
+            return __ldg(reinterpret_cast<const uint32_t *>(in + i * plane));
+        else
+            return __ldg(in + i * plane);
+    };
+    const int i0 = w * seg, i1 = min(n, i0 + seg);
+    // periodic correctors: counts at the first voxel from the last zero of the
+    // wrapped line and the other way round
+    if (cfg.periodic && (w == 0 || w == nw - 1)) {
+        int pos[VEC];
+#pragma unroll
+        for (int q = 0; q < VEC; q++)
+            pos[q] = -1;
+        for (int side = 0; side < 2; side++) {
+            if (side == 0 ? w != 0 : w != nw - 1)
+                continue;
+            const int lo = side == 0 ? cfg.f_lo : cfg.l_lo, hi = side == 0 ? n : n - cfg.l_hi;
+            for (int q = 0; q < VEC; q++)
+                pos[q] = -1;
+            for (int t = 0; t < hi - lo; t += 4) {
+                uint32_t r[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    r[u] = t + u < hi - lo ? row(side == 0 ? lo + t + u : hi - 1 - t - u) : 0xffffffffu;
+                bool open = false;
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+#pragma unroll
+                    for (int q = 0; q < VEC; q++)
+                        if (pos[q] < 0 && ((r[u] >> (8 * q)) & 0xffu) == 0)
+                            pos[q] = t + u;
+#pragma unroll
+                for (int q = 0; q < VEC; q++)
+                    open |= pos[q] < 0;
+                if (!__any_sync(0xffffffffu, open && live))
+                    break;
+            }
+            uint32_t c[VEC];
+#pragma unroll
+            for (int q = 0; q < VEC; q++) {
+                if (pos[q] < 0)
+                    c[q] = kLinInf;
+                else if (side == 0) // first zero F: the upper corrector F + a_u
+                    c[q] = (uint32_t)(lo + pos[q] + cfg.a_u);
+                else // last zero L: the lower corrector n - L + a_l
+                    c[q] = (uint32_t)(n - (hi - 1 - pos[q]) + cfg.a_l);
+            }
+#pragma unroll
+            for (int h = 0; h < H; h++)
+                s_corr[side][h][lane] = VEC == 4 ? c[2 * h % VEC] | (c[(2 * h + 1) % VEC] << 16) : c[0];
+        }
+    }
+    // counts handed on, from unknown incoming ones
+    uint32_t enl[kLinChunks][H]; // per chunk: the backward count just below it
+    uint32_t dn[H];
+#pragma unroll
+    for (int h = 0; h < H; h++)
+        dn[h] = kInf2;
+    uint32_t vp = i0 < n ? row(i0 > 0 ? i0 - 1 : 0) : 0u;
+#pragma unroll
+    for (int c = 0; c < kLinChunks; c++) {
+        const int a = i0 + c * kLinChunk;
+#pragma unroll
+        for (int h = 0; h < H; h++)
+            enl[c][h] = kInf2;
+        if (a >= i1)
+            continue;
+        uint32_t v[kLinChunk + 1];
+#pragma unroll
+        for (int u = 0; u <= kLinChunk; u++)
+            v[u] = row(min(a + u, n - 1));
+        const int len = min(kLinChunk, i1 - a);
+#pragma unroll
+        for (int u = 0; u < kLinChunk; u++)
+            if (u < len) {
+                const uint32_t nz = nz01(v[u]), df = nz01(v[u] ^ (u ? v[u ? u - 1 : 0] : vp));
+#pragma unroll
+                for (int h = 0; h < H; h++) {
+                    const uint32_t m = h ? mask2<1>(nz) : mask2<0>(nz), x = h ? mask2<1>(df) : mask2<0>(df);
+                    dn[h] = (((dn[h] & ~x) | (0x00010001u & x)) & m) + 0x00010001u;
+                }
+            }
+#pragma unroll
+        for (int u = kLinChunk - 1; u >= 0; u--)
+            if (u < len) {
+                const uint32_t nz = nz01(v[u]), df = nz01(v[u] ^ v[u + 1]);
+#pragma unroll
+                for (int h = 0; h < H; h++) {
+                    const uint32_t m = h ? mask2<1>(nz) : mask2<0>(nz), x = h ? mask2<1>(df) : mask2<0>(df);
+                    enl[c][h] = (((enl[c][h] & ~x) | (0x00010001u & x)) & m) + 0x00010001u;
+                }
+            }
+        vp = v[len == kLinChunk ? kLinChunk - 1 : 0]; // (a short chunk is the line's last)
+    }
+    {
+        // the segment's backward count: chunk by chunk from its high end
+        uint32_t e[H];
+#pragma unroll
+        for (int h = 0; h < H; h++)
+            e[h] = kInf2;
+#pragma unroll
+        for (int c = kLinChunks - 1; c >= 0; c--) {
+            const int a = i0 + c * kLinChunk;
+            if (a >= i1)
+                continue;
+            const uint32_t len = (uint32_t)min(kLinChunk, i1 - a) * 0x10001u;
+#pragma unroll
+            for (int h = 0; h < H; h++)
+                e[h] = __vminu2(enl[c][h], e[h] + len);
+        }
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            s_f[w][h][lane] = dn[h];
+            s_b[w][h][lane] = __vminu2(e[h], kInf2 + 0x20002000u);
+        }
+    }
+    __syncthreads();
+    if (i0 >= n || !live)
+        return;
+    // the true incoming counts of this segment
+    uint32_t en[H];
+#pragma unroll
+    for (int h = 0; h < H; h++) {
+        dn[h] = cfg.periodic ? s_corr[1][h][lane] : kInf2;
+        en[h] = cfg.periodic ? s_corr[0][h][lane] : kInf2;
+        const uint32_t cap = kInf2 + 0x20002000u; // keeps both halves below 2^16 over long lines
+        for (int q = 0; q < w; q++)
+            dn[h] = __vminu2(__vminu2(s_f[q][h][lane], dn[h] + (uint32_t)seg * 0x10001u), cap);
+        for (int q = (n - 1) / seg; q > w; q--) {
+            const uint32_t len = (uint32_t)(min(n, (q + 1) * seg) - q * seg) * 0x10001u;
+            en[h] = __vminu2(__vminu2(s_b[q][h][lane], en[h] + len), cap);
+        }
+    }
+    // the backward count above every chunk
+    uint32_t ea[kLinChunks][H];
+#pragma unroll
+    for (int c = kLinChunks - 1; c >= 0; c--) {
+        const int a = i0 + c * kLinChunk;
+        const uint32_t len = a < i1 ? (uint32_t)min(kLinChunk, i1 - a) * 0x10001u : 0u;
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            ea[c][h] = en[h];
+            if (a < i1)
+                en[h] = __vminu2(enl[c][h], en[h] + len);
+        }
+    }
+    vp = row(i0 > 0 ? i0 - 1 : 0);
+#pragma unroll
+    for (int c = 0; c < kLinChunks; c++) {
+        const int a = i0 + c * kLinChunk;
+        if (a >= i1)
+            break;
+        uint32_t v[kLinChunk + 1], d[kLinChunk][H];
+#pragma unroll
+        for (int u = 0; u <= kLinChunk; u++)
+            v[u] = row(min(a + u, n - 1));
+        const int len = min(kLinChunk, i1 - a);
+#pragma unroll
+        for (int u = 0; u < kLinChunk; u++) {
+            const uint32_t nz = nz01(v[u]), df = nz01(v[u] ^ (u ? v[u ? u - 1 : 0] : vp));
+#pragma unroll
+            for (int h = 0; h < H; h++) {
+                const uint32_t m = h ? mask2<1>(nz) : mask2<0>(nz), x = h ? mask2<1>(df) : mask2<0>(df);
+                d[u][h] = ((dn[h] & ~x) | (0x00010001u & x)) & m;
+                dn[h] = d[u][h] + 0x00010001u;
+            }
+        }
+        uint32_t e[H];
+#pragma unroll
+        for (int h = 0; h < H; h++)
+            e[h] = ea[c][h];
+#pragma unroll
+        for (int u = kLinChunk - 1; u >= 0; u--) {
+            if (u >= len)
+                continue;
+            const uint32_t nz = nz01(v[u]), df = nz01(v[u] ^ v[u + 1]);
+            uint32_t r[H];
+#pragma unroll
+            for (int h = 0; h < H; h++) {
+                const uint32_t m = h ? mask2<1>(nz) : mask2<0>(nz), x = h ? mask2<1>(df) : mask2<0>(df);
+                e[h] = ((e[h] & ~x) | (0x00010001u & x)) & m;
+                r[h] = __vminu2(d[u][h], e[h]);
+                e[h] += 0x00010001u;
+            }
+            OUT *o = out + (long long)(a + u) * plane + line;
+            if constexpr (sizeof(OUT) == 2) {
+                if constexpr (VEC == 4)
+                    *reinterpret_cast<uint2 *>(o) = make_uint2(r[0], r[H - 1]);
+                else
+                    *o = (OUT)r[0];
+            } else {
+                auto val = [&](uint32_t q) { return q <= (uint32_t)n ? s_tab[q] : FLT_MAX; };
+                if constexpr (VEC == 4)
+                    *reinterpret_cast<float4 *>(o) = make_float4(val(r[0] & 0xffffu), val(r[0] >> 16),
+                                                                 val(r[H - 1] & 0xffffu), val(r[H - 1] >> 16));
+                else
+                    *o = (OUT)val(r[0] & 0xffffu);
+            }
+        }
+        vp = v[kLinChunk - 1];
+    }
+}
+
+// The linear pass as counts needs correctors that are counts themselves.
+bool lin_ok(int n, const pmg_axis_cfg &c)
+{
+    if (n > kLinMaxLine)
+        return false;
+    if (!c.periodic)
+        return true;
+    // every index in range, and both correctors of every line in [0, kLinInf)
+    return c.f_lo >= 0 && c.l_lo >= 0 && c.l_hi >= 0 && c.l_lo + c.l_hi <= n && (long long)c.f_lo + c.a_u >= 0 &&
+           (long long)c.l_hi + 1 + c.a_l >= 0 && 2LL * n + std::max(c.a_u, c.a_l) < kLinInf;
+}
+
+template <class OUT>
+static int launch_lin_t(const uint8_t *img, OUT *out, const int64_t *shape, float res, const pmg_axis_cfg &cfg,
+                        cudaStream_t st)
+{
+    const int n = (int)shape[0];
+    const long long plane = (long long)shape[1] * shape[2];
+    // segments of whole chunks: 8 per line, 16 on lines beyond 1024
+    const int parts = n > 8 * kLinChunk * kLinChunks ? kLinWarps : 8;
+    const int seg = ((n + parts - 1) / parts + kLinChunk - 1) / kLinChunk * kLinChunk;
+    const dim3 block(32, (unsigned)((n + seg - 1) / seg));
+    typename TabOf<OUT>::T tab;
+    size_t smem = 0;
+    if constexpr (sizeof(OUT) == 4) {
+        // the reference's running sum of res, squared (_distance.hpp:135-182)
+        float d = 0.0f;
+        for (int k = 0; k <= n; k++) {
+            volatile float q = d * d;
+            tab.v[k] = q == INFINITY ? FLT_MAX : (float)q;
+            volatile float nd = d + res;
+            d = nd;
+        }
+        smem = sizeof(float) * (size_t)(n + 1);
+    }
+    const bool quads = !(plane & 3) && !(reinterpret_cast<uintptr_t>(img) & 3) &&
+                       !(reinterpret_cast<uintptr_t>(out) & (4 * sizeof(OUT) - 1));
+    const int ps__ = prof_begin("k_lin", st);
+    if (quads)
+        k_lin<4, OUT><<<(unsigned)((plane / 4 + 31) / 32), block, smem, st>>>(img, out, plane, n, seg, cfg, tab);
+    else
+        k_lin<1, OUT><<<(unsigned)((plane + 31) / 32), block, smem, st>>>(img, out, plane, n, seg, cfg, tab);
+    prof_end(ps__, (double)plane * n * (1 + sizeof(OUT)), st);
+    PMG_CHECK_LAUNCH();
+    return PMG_OK;
+}
+
+int launch_lin_counts(const uint8_t *img, uint16_t *out, const int64_t *shape, const pmg_axis_cfg &cfg,
+                      cudaStream_t st)
+{
+    return launch_lin_t<uint16_t>(img, out, shape, 1.0f, cfg, st);
+}
+
+int launch_lin_float(const uint8_t *img, float *out, const int64_t *shape, float res, const pmg_axis_cfg &cfg,
+                     cudaStream_t st)
+{
+    return launch_lin_t<float>(img, out, shape, res, cfg, st);
+}
+
+// ---------------------------------------------------------------------------
+// envelope passes
+// ---------------------------------------------------------------------------
+// Heights of kBig and more count as absent; kBig + 2 * kMaxStep stays below
+// 2^16, and (kMaxStep + 1)^2 is above every height below kBig.
+constexpr uint32_t kBig = 60000u, kMaxStep = 245u;
+constexpr uint32_t kBig2 = kBig * 0x10001u;
+
+// (count, count) -> (K, K), absent counts -> kBig
+__device__ __forceinline__ uint32_t square2(uint32_t c)
+{
+    const uint32_t a = min(c & 0xffffu, kMaxStep), b = min(c >> 16, kMaxStep);
+    return min(a * a, kBig) | (min(b * b, kBig) << 16);
+}
+
+// larger of the two halves
+__device__ __forceinline__ uint32_t hmax(uint32_t v) { return max(v & 0xffffu, v >> 16); }
+
+// flag bits of a voxel (see the file comment); el, er: squared distances to
+// the imports beyond the line's ends
+__device__ __forceinline__ unsigned line_need(uint32_t m, int x, int n, int periodic, int wide)
+{
+    if (m >= kBig)
+        return periodic || wide ? 2u : 0u;
+    if (!periodic)
+        return 0u;
+    const uint32_t lo = (uint32_t)(x + 1), hi = (uint32_t)(n - x);
+    return (m > lo * lo ? 1u : 0u) | (m > hi * hi ? 4u : 0u);
+}
+
+// Strided pass along axis 1 of [n0][n][s2]: one thread block per plane and
+// 32 * VEC adjacent lines (VEC = 2: two lines per lane, s2 even), warp w on
+// positions [w P, (w + 1) P) of its lines, heights in registers.  Warps hand
+// their end values on through shared memory, one barrier per step.
+template <int P, int VEC>
+__global__ void __launch_bounds__(32 * P) k_par_cols(const uint16_t *__restrict__ D, float *__restrict__ out, int n, int s2, float a,
+                           int periodic, int wide, uint8_t *__restrict__ flag)
+{
+    extern __shared__ uint32_t s_end[]; // [2][nw][2][32]
+    const int lane = threadIdx.x, w = threadIdx.y, nw = blockDim.y;
+    const int k0 = (blockIdx.x * 32 + lane) * VEC;
+    const bool live = k0 < s2;
+    const long long base = (long long)blockIdx.y * n * s2 + k0;
+    const int x0 = w * P;
+    uint32_t g[P];
+    const uint16_t *src = D + base + (long long)x0 * s2;
+#pragma unroll
+    for (int p = 0; p < P; p++) {
+        uint32_t c = 0xffffffffu;
+        if (live && x0 + p < n) {
+            if constexpr (VEC == 2)
+                c = __ldg(reinterpret_cast<const uint32_t *>(src + (long long)p * s2));
+            else
+                c = (uint32_t)__ldg(src + (long long)p * s2) | 0xffff0000u;
+        }
+        g[p] = c;
+    }
+    uint32_t mx = 0;
+#pragma unroll
+    for (int p = 0; p < P; p++) {
+        g[p] = square2(g[p]);
+        if (x0 + p < n)
+            mx = __vmaxu2(mx, g[p]);
+    }
+    if (!live)
+        mx = 0;
+    if (VEC == 1)
+        mx &= 0xffffu;
+    for (uint32_t k = 1; k <= kMaxStep; k++) {
+        uint32_t *e = s_end + (size_t)(k & 1) * nw * 64;
+        e[(w * 2) * 32 + lane] = g[0];
+        e[(w * 2 + 1) * 32 + lane] = g[P - 1];
+        const bool open = hmax(mx) > k * k;
+        if (!__syncthreads_or(open))
+            break;
+        if (!__any_sync(0xffffffffu, open))
+            continue; // this warp's values are final
+        uint32_t prev = w > 0 ? e[((w - 1) * 2 + 1) * 32 + lane] : kBig2;
+        const uint32_t right = w + 1 < nw ? e[((w + 1) * 2) * 32 + lane] : kBig2;
+        const uint32_t c = (2 * k - 1) * 0x10001u;
+        mx = 0;
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            const uint32_t cur = g[p];
+            const uint32_t t = __vminu2(prev, p + 1 < P ? g[p + 1 < P ? p + 1 : p] : right);
+            g[p] = __viaddmin_u16x2(t, c, cur);
+            if (x0 + p < n)
+                mx = __vmaxu2(mx, g[p]);
+            prev = cur;
+        }
+        if (!live)
+            mx = 0;
+        if (VEC == 1)
+            mx &= 0xffffu;
+    }
+    unsigned need0 = 0, need1 = 0;
+    if (live) {
+        float *dst = out + base + (long long)x0 * s2;
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            if (x0 + p >= n)
+                break;
+            const uint32_t lo = g[p] & 0xffffu, hi = g[p] >> 16;
+            const float f0 = lo >= kBig ? FLT_MAX : fmul((float)lo, a);
+            if constexpr (VEC == 2) {
+                const float f1 = hi >= kBig ? FLT_MAX : fmul((float)hi, a);
+                *reinterpret_cast<float2 *>(dst + (long long)p * s2) = make_float2(f0, f1);
+                need1 |= line_need(hi, x0 + p, n, periodic, wide);
+            } else {
+                dst[(long long)p * s2] = f0;
+            }
+            need0 |= line_need(lo, x0 + p, n, periodic, wide);
+        }
+    }
+    if (!flag)
+        return;
+    __syncthreads();
+    s_end[w * 32 + lane] = need0 | (need1 << 8);
+    __syncthreads();
+    if (w == 0 && live) {
+        unsigned need = 0;
+        for (int q = 0; q < nw; q++)
+            need |= s_end[q * 32 + lane];
+        uint8_t *fl = flag + (long long)blockIdx.y * s2 + k0;
+        fl[0] = (uint8_t)need;
+        if constexpr (VEC == 2)
+            fl[1] = (uint8_t)(need >> 8);
+    }
+}
+
+// Contiguous pass: one warp per pair of rows, lane l on positions [l P, (l +
+// 1) P), neighbouring values by shuffles; the rows pass through shared memory
+// (one word per position pair, padded by one word per P) so that global
+// loads and stores stay coalesced.
+constexpr int kRowWarps = 8;
+
+template <int P>
+__global__ void __launch_bounds__(32 * kRowWarps) k_par_rows(const float *__restrict__ fin, float *__restrict__ fout,
+                                                             long long nrows, int n, float a, float inv_a,
+                                                             int periodic, int wide, int form,
+                                                             uint8_t *__restrict__ flag)
+{
+    constexpr int kWords = 32 * P + 32;
+    extern __shared__ uint32_t s_rows[];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t *row = s_rows + w * kWords;
+    const long long pairs = (nrows + 1) >> 1;
+    const bool vec4 = !(n & 3) && !((reinterpret_cast<uintptr_t>(fin) | reinterpret_cast<uintptr_t>(fout)) & 15);
+    auto pack = [&](float f0, float f1) -> uint32_t {
+        const uint32_t u0 = (uint32_t)fminf(fmul(f0, inv_a), (float)kBig);
+        const uint32_t u1 = (uint32_t)fminf(fmul(f1, inv_a), (float)kBig);
+        return u0 | (u1 << 16);
+    };
+    auto slot = [](int c) { return c + c / P; };
+    for (long long r = blockIdx.x * (long long)kRowWarps + w; r < pairs; r += (long long)gridDim.x * kRowWarps) {
+        const bool two = 2 * r + 1 < nrows;
+        const float *in0 = fin + 2 * r * n, *in1 = in0 + (two ? n : 0);
+        if (vec4) {
+#pragma unroll
+            for (int t = 0; t < (P + 3) / 4; t++) {
+                const int c = (t * 32 + lane) * 4;
+                if (c < n) {
+                    const float4 f0 = __ldg(reinterpret_cast<const float4 *>(in0 + c));
+                    const float4 f1 = __ldg(reinterpret_cast<const float4 *>(in1 + c));
+                    row[slot(c)] = pack(f0.x, f1.x);
+                    row[slot(c + 1)] = pack(f0.y, f1.y);
+                    row[slot(c + 2)] = pack(f0.z, f1.z);
+                    row[slot(c + 3)] = pack(f0.w, f1.w);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int t = 0; t < P; t++) {
+                const int c = t * 32 + lane;
+                if (c < n)
+                    row[slot(c)] = pack(in0[c], in1[c]);
+            }
+        }
+        __syncwarp();
+        const int x0 = lane * P;
+        uint32_t g[P], mx = 0;
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            g[p] = x0 + p < n ? row[lane * (P + 1) + p] : kBig2;
+            if (x0 + p < n)
+                mx = __vmaxu2(mx, g[p]);
+        }
+        for (uint32_t k = 1; k <= kMaxStep; k++) {
+            if (!__any_sync(0xffffffffu, hmax(mx) > k * k))
+                break;
+            uint32_t prev = __shfl_up_sync(0xffffffffu, g[P - 1], 1);
+            uint32_t right = __shfl_down_sync(0xffffffffu, g[0], 1);
+            prev = lane > 0 ? prev : kBig2;
+            right = lane < 31 ? right : kBig2;
+            const uint32_t c = (2 * k - 1) * 0x10001u;
+            mx = 0;
+#pragma unroll
+            for (int p = 0; p < P; p++) {
+                const uint32_t cur = g[p];
+                const uint32_t t = __vminu2(prev, p + 1 < P ? g[p + 1 < P ? p + 1 : p] : right);
+                g[p] = __viaddmin_u16x2(t, c, cur);
+                if (x0 + p < n)
+                    mx = __vmaxu2(mx, g[p]);
+                prev = cur;
+            }
+        }
+        unsigned need = 0;
+#pragma unroll
+        for (int p = 0; p < P; p++)
+            if (x0 + p < n) {
+                row[lane * (P + 1) + p] = g[p];
+                need |= line_need(g[p] & 0xffffu, x0 + p, n, periodic, wide) |
+                        (line_need(g[p] >> 16, x0 + p, n, periodic, wide) << 8);
+            }
+        __syncwarp();
+        auto value = [&](uint32_t m) -> float {
+            const float f = m >= kBig ? FLT_MAX : fmul((float)m, a);
+            return form == PMG_EDT_DIST ? __fsqrt_rn(f) : f;
+        };
+        float *o0 = fout + 2 * r * n, *o1 = o0 + n;
+        if (vec4) {
+#pragma unroll
+            for (int t = 0; t < (P + 3) / 4; t++) {
+                const int c = (t * 32 + lane) * 4;
+                if (c < n) {
+                    const uint32_t q0 = row[slot(c)], q1 = row[slot(c + 1)], q2 = row[slot(c + 2)],
+                                   q3 = row[slot(c + 3)];
+                    *reinterpret_cast<float4 *>(o0 + c) = make_float4(value(q0 & 0xffffu), value(q1 & 0xffffu),
+                                                                      value(q2 & 0xffffu), value(q3 & 0xffffu));
+                    if (two)
+                        *reinterpret_cast<float4 *>(o1 + c) =
+                            make_float4(value(q0 >> 16), value(q1 >> 16), value(q2 >> 16), value(q3 >> 16));
+                }
+            }
+        } else {
+#pragma unroll
+            for (int t = 0; t < P; t++) {
+                const int c = t * 32 + lane;
+                if (c < n) {
+                    const uint32_t q = row[slot(c)];
+                    o0[c] = value(q & 0xffffu);
+                    if (two)
+                        o1[c] = value(q >> 16);
+                }
+            }
+        }
+        if (flag) {
+            need = __reduce_or_sync(0xffffffffu, need);
+            if (lane == 0) {
+                flag[2 * r] = (uint8_t)need;
+                if (two)
+                    flag[2 * r + 1] = (uint8_t)(need >> 8);
+            }
+        }
+        __syncwarp();
+    }
+}
+
+bool lattice_ok(const int64_t *shape, const float *res, const pmg_axis_cfg *cfg)
+{
+    if (!(res[0] == res[1] && res[1] == res[2]) || !lin_ok((int)shape[0], cfg[0]) || shape[0] > kScanMaxLine)
+        return false;
+    return window_path_ok(res[1], (int)shape[1]) && window_path_ok(res[2], (int)shape[2]);
+}
+
+template <int P>
+static void cols_p(const uint16_t *D, float *out, int n0, int n, int s2, float a, int periodic, int wide,
+                   uint8_t *flag, cudaStream_t st)
+{
+    const int nw = (n + P - 1) / P;
+    const size_t smem = (size_t)nw * 128 * sizeof(uint32_t);
+    if (!(s2 & 1))
+        k_par_cols<P, 2><<<dim3((unsigned)((s2 / 2 + 31) / 32), (unsigned)n0), dim3(32, (unsigned)nw), smem, st>>>(
+            D, out, n, s2, a, periodic, wide, flag);
+    else
+        k_par_cols<P, 1><<<dim3((unsigned)((s2 + 31) / 32), (unsigned)n0), dim3(32, (unsigned)nw), smem, st>>>(
+            D, out, n, s2, a, periodic, wide, flag);
+}
+
+template <int P>
+static void rows_p(const float *fin, float *fout, long long nrows, int n, float a, int periodic, int wide, int form,
+                   uint8_t *flag, cudaStream_t st)
+{
+    const size_t smem = sizeof(uint32_t) * (size_t)kRowWarps * (32 * P + 32);
+    const long long pairs = (nrows + 1) >> 1;
+    k_par_rows<P><<<grid_for(pairs, kRowWarps, 152LL * 64), 32 * kRowWarps, smem, st>>>(fin, fout, nrows, n, a, 1.0f / a,
+                                                                                    periodic, wide, form, flag);
+}
+
+// The three passes: counts in `out`, the first envelope in `tmp`, the result
+// in `out`.  flags: one byte per line of the larger envelope pass.
+int lattice_run(const uint8_t *img, float *out, float *tmp, const int64_t *shape, const float *res,
+                const pmg_axis_cfg *cfg, int num_hull, int form, uint8_t *flags, cudaStream_t st)
+{
+    const int n0 = (int)shape[0], n1 = (int)shape[1], n2 = (int)shape[2];
+    const float a = res[0] * res[0];
+    uint16_t *D = (uint16_t *)out;
+    PMG_TRY(launch_lin_counts(img, D, shape, cfg[0], st));
+    // whether a finite value of a pass can reach kBig (counts reach n0, plus
+    // the wrapped part on a periodic axis)
+    const long long m0 = (cfg[0].periodic ? 2LL : 1LL) * n0, m1 = m0 * m0 + (long long)n1 * n1;
+    const int wide1 = m1 >= (long long)kBig, wide2 = m1 + (long long)n2 * n2 >= (long long)kBig;
+    {
+        const int per = cfg[1].periodic ? 1 : 0;
+        uint8_t *fl = per || wide1 ? flags : nullptr;
+        const int ps__ = prof_begin("k_par_cols", st);
+        if (n1 <= 64)
+            cols_p<8>(D, tmp, n0, n1, n2, a, per, wide1, fl, st);
+        else if (n1 <= 256)
+            cols_p<16>(D, tmp, n0, n1, n2, a, per, wide1, fl, st);
+        else
+            cols_p<32>(D, tmp, n0, n1, n2, a, per, wide1, fl, st);
+        prof_end(ps__, (double)n0 * n1 * n2 * 6, st);
+        PMG_CHECK_LAUNCH();
+        if (fl)
+            PMG_TRY(launch_ends_counts(D, tmp, all_lines(shape, 1), res[1], cfg[1], num_hull, fl, st));
+    }
+    {
+        const int per = cfg[2].periodic ? 1 : 0;
+        uint8_t *fl = per || wide2 ? flags : nullptr;
+        const long long nrows = (long long)n0 * n1;
+        const int ps__ = prof_begin("k_par_rows", st);
+        if (n2 <= 64)
+            rows_p<2>(tmp, out, nrows, n2, a, per, wide2, form, fl, st);
+        else if (n2 <= 128)
+            rows_p<4>(tmp, out, nrows, n2, a, per, wide2, form, fl, st);
+        else if (n2 <= 256)
+            rows_p<8>(tmp, out, nrows, n2, a, per, wide2, form, fl, st);
+        else if (n2 <= 512)
+            rows_p<16>(tmp, out, nrows, n2, a, per, wide2, form, fl, st);
+        else
+            rows_p<32>(tmp, out, nrows, n2, a, per, wide2, form, fl, st);
+        prof_end(ps__, (double)n0 * n1 * n2 * 8, st);
+        PMG_CHECK_LAUNCH();
+        if (fl)
+            PMG_TRY(launch_ends_heights(tmp, out, all_lines(shape, 2), res[2], cfg[2], num_hull, form, fl, st));
+    }
+    return PMG_OK;
+}
+
+} // namespace pmg

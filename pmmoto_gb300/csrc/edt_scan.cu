@@ -1,0 +1,247 @@
+// Envelope passes of any voxel size as an outward scan (sm_103a).
+//
+// The reference's lower envelope (squared_edt_1d_parabolic, _distance.hpp:
+// 184-272) gives at every position x the float value a (x - v)^2 + f(v) of one
+// parabola v, chosen by float intersections.  Each intersection s(r, q) is off
+// by at most
+//     2^-24 (4 |f_r - f_q| / (2 a (r - q)) + 3 (r + q) / 2),
+// so the choice between two parabolas at x is the true one unless their values
+// there are closer than eta (scan_eta below): rounding can only swap
+// near-ties.  Hence, with m the smallest float value at x and "near" the
+// parabolas within eta of m:
+//  * near values all equal: the envelope's value is m;
+//  * otherwise, when no further value lies within a / 2 of m, the near
+//    parabolas keep their order on the envelope's stack whatever the others
+//    do (every intersection with another one lies clearly to one side of x),
+//    so replaying the reference's pushes and pops on them alone gives its
+//    choice;
+//  * otherwise (rare) the line is flagged for the whole float envelope.
+// m needs only the positions with a d^2 <= m + a / 2: the scan runs outward
+// from x, all lanes together, until that holds for every lane.  On a periodic
+// line a voxel whose m reaches the squared distance to a line end may depend
+// on the imported hulls: the line is flagged for its end segments.
+//
+// Lines are staged in shared memory (a thread's serial float envelope spends
+// its time waiting on dependent global loads; here every voxel is its own
+// thread and a candidate costs one shared-memory read and five
+// instructions).
+#include <cfloat>
+#include <algorithm>
+
+#include "edt_internal.cuh"
+
+namespace pmg {
+
+constexpr int kScanWarps = 8;
+
+// Values at x closer than this may be ordered either way by the reference's
+// float intersections (R: distance within which near parabolas lie).
+__device__ __forceinline__ float scan_eta(float a, float m, float R, float x)
+{
+    return a * (2.0f * R + 1.0f) * (7.0f * R + 3.0f * x + 8.0f) * 1.8e-7f + m * 4e-7f;
+}
+
+// The near parabolas of position x pushed in order as update_hull does
+// (_distance.hpp:89-112), then the reference's evaluation at x.  Returns false
+// when the line has to be replayed.
+template <class H>
+__device__ __noinline__ bool scan_resolve(const H &h, int n, int x, float a, float m, float R, float eta, float &out)
+{
+    if (0.25f < (3.0f * R + 1.0f) * (7.0f * R + 3.0f * (float)x + 8.0f) * 2.4e-7f)
+        return false;
+    constexpr int kNear = 8;
+    int v[kNear];
+    float f[kNear], r[kNear];
+    int cnt = 0, seen = 0;
+    const float top = m + 0.5f * a;
+    const int D = (int)__fsqrt_rn(top / a) + 1;
+    for (int q = max(0, x - D); q <= min(n - 1, x + D); q++) {
+        const float dx = (float)(q - x), fq = h(q);
+        const float val = fadd(fmul(a, fmul(dx, dx)), fq);
+        if (val <= m + eta) {
+            if (++seen > kNear)
+                return false;
+            float s = -INFINITY;
+            if (cnt > 0) {
+                s = isect(fq, (float)q, f[cnt - 1], (float)v[cnt - 1], a);
+                while (cnt > 1 && s <= r[cnt - 1]) {
+                    cnt--;
+                    s = isect(fq, (float)q, f[cnt - 1], (float)v[cnt - 1], a);
+                }
+            }
+            v[cnt] = q;
+            f[cnt] = fq;
+            r[cnt] = s;
+            cnt++;
+        } else if (val <= top) {
+            return false;
+        }
+    }
+    int k = 0;
+    while (k + 1 < cnt && r[k + 1] < (float)x)
+        k++;
+    const float dx = (float)(x - v[k]);
+    out = fadd(fmul(a, fmul(dx, dx)), f[k]);
+    return true;
+}
+
+// One voxel per lane (x < n on live lanes): the value and its line's flag bits.
+template <class H>
+__device__ __forceinline__ float scan_voxel(const H &h, int n, int x, bool live, float a, float inv_a, int periodic,
+                                            float vcap, unsigned &need)
+{
+    float m = live ? h(x) : 0.0f, m2 = INFINITY;
+    const float half = 0.5f * a;
+    for (int d = 1; d < n; d++) {
+        const float ad = fmul(a, (float)(d * d));
+        if (!__any_sync(0xffffffffu, live && ad <= m + half && ad <= vcap))
+            break;
+        if (live) {
+            // past a line end: the end position again, at a distance beyond its
+            // own, so more than a / 2 above the value it had there
+            const float v0 = fadd(ad, h(max(x - d, 0))), t0 = fmaxf(v0, m);
+            m = fminf(v0, m);
+            m2 = t0 != m ? fminf(m2, t0) : m2;
+            const float v1 = fadd(ad, h(min(x + d, n - 1))), t1 = fmaxf(v1, m);
+            m = fminf(v1, m);
+            m2 = t1 != m ? fminf(m2, t1) : m2;
+        }
+    }
+    if (!live || m > vcap)
+        return m;
+    if (m >= FLT_MAX) { // no solid voxel on the line
+        need |= periodic ? 1u : 0u;
+        return m;
+    }
+    const float R = __fsqrt_rn(m * inv_a);
+    const float eta = scan_eta(a, m, R, (float)x);
+    if (periodic) {
+        const int e = min(x + 1, n - x);
+        if (m + eta >= fmul(a, (float)e * (float)e)) {
+            need |= 1u;
+            return m;
+        }
+    }
+    if (m2 <= m + eta) {
+        float v = m;
+        if (scan_resolve(h, n, x, a, m, R, eta, v))
+            return v;
+        need |= 2u;
+    }
+    return m;
+}
+
+struct ColH {
+    const float *s; // position v of this lane's line at s[32 v]
+    __device__ __forceinline__ float operator()(int v) const { return s[v * 32]; }
+};
+struct RowH {
+    const float *s;
+    __device__ __forceinline__ float operator()(int v) const { return s[v]; }
+};
+
+// Strided lines (axis 0 or 1): one block per 32 adjacent lines, warp w on
+// positions w, w + 8, ...
+__global__ void __launch_bounds__(32 * kScanWarps) k_scan_cols(const float *__restrict__ fin, float *__restrict__ fout,
+                                                               Lines Ls, float a, float inv_a, int periodic, int form,
+                                                               MorphEpi me, float vcap, uint8_t *__restrict__ flag)
+{
+    extern __shared__ float s_line[]; // [n][32]
+    __shared__ unsigned s_need[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int tiles = (Ls.nb2 + 31) / 32;
+    const int ra = blockIdx.x / tiles, kb = (blockIdx.x - ra * tiles) * 32 + lane;
+    const bool live = kb < Ls.nb2;
+    const long long li = (long long)ra * Ls.nb2 + (live ? kb : 0);
+    const LineGeo g = line_addr(Ls, li);
+    const int n = g.n;
+    const float *src = fin + g.base;
+    if (threadIdx.x < 32)
+        s_need[threadIdx.x] = 0;
+#pragma unroll 8
+    for (int x = w; x < n; x += kScanWarps)
+        s_line[x * 32 + lane] = __ldg(src + x * g.stride);
+    __syncthreads();
+    const ColH h{s_line + lane};
+    unsigned need = 0;
+    for (int x = w; x < n; x += kScanWarps) {
+        const float v = scan_voxel(h, n, x, live, a, inv_a, periodic, vcap, need);
+        if (!live)
+            continue;
+        if (form == PMG_EDT_MORPH)
+            morph_store(me, g, x, v);
+        else
+            fout[g.base + x * g.stride] = form == PMG_EDT_DIST ? __fsqrt_rn(v) : v;
+    }
+    if (need)
+        atomicOr(s_need + lane, need);
+    __syncthreads();
+    if (w == 0 && live)
+        flag[li] = (uint8_t)s_need[lane];
+}
+
+// Contiguous lines: one warp per row, lanes on 32 consecutive positions.
+__global__ void __launch_bounds__(32 * kScanWarps) k_scan_rows(const float *__restrict__ fin, float *__restrict__ fout,
+                                                               Lines Ls, float a, float inv_a, int periodic, int form,
+                                                               MorphEpi me, float vcap, uint8_t *__restrict__ flag)
+{
+    extern __shared__ float s_line[]; // [kScanWarps][n]
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long long nlines = Ls.count();
+    const int n = (int)Ls.s2;
+    float *row = s_line + (long long)w * n;
+    for (long long li = blockIdx.x * (long long)kScanWarps + w; li < nlines;
+         li += (long long)gridDim.x * kScanWarps) {
+        const LineGeo g = line_addr(Ls, li);
+        const float *src = fin + g.base;
+#pragma unroll 8
+        for (int x = lane; x < n; x += 32)
+            row[x] = __ldg(src + x);
+        __syncwarp();
+        const RowH h{row};
+        unsigned need = 0;
+        for (int x0 = 0; x0 < n; x0 += 32) {
+            const int x = x0 + lane;
+            const bool live = x < n;
+            const float v = scan_voxel(h, n, x, live, a, inv_a, periodic, vcap, need);
+            if (!live)
+                continue;
+            if (form == PMG_EDT_MORPH)
+                morph_store(me, g, x, v);
+            else
+                fout[g.base + x] = form == PMG_EDT_DIST ? __fsqrt_rn(v) : v;
+        }
+        need = __reduce_or_sync(0xffffffffu, need);
+        if (lane == 0)
+            flag[li] = (uint8_t)need;
+        __syncwarp();
+    }
+}
+
+int launch_scan(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg, int form,
+                const MorphEpi &me, float vcap, uint8_t *flag, cudaStream_t st)
+{
+    const float a = res * res, inv_a = 1.0f / a;
+    const int per = cfg.periodic ? 1 : 0;
+    if (Ls.ax == 2) {
+        const size_t smem = sizeof(float) * (size_t)kScanWarps * (size_t)Ls.s2;
+        const int ps__ = prof_begin("k_scan_rows", st);
+        k_scan_rows<<<grid_for(Ls.count(), kScanWarps, 152LL * 64), 32 * kScanWarps, smem, st>>>(
+            fin, fout, Ls, a, inv_a, per, form, me, vcap, flag);
+        prof_end(ps__, (double)Ls.count() * Ls.s2 * (form == PMG_EDT_MORPH ? 5 : 8), st);
+    } else {
+        const int n = (int)(Ls.ax == 0 ? Ls.s0 : Ls.s1);
+        const size_t smem = sizeof(float) * 32 * (size_t)n;
+        if (smem > 47 * 1024)
+            PMG_CUDA(cudaFuncSetAttribute(k_scan_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const long long blocks = (long long)Ls.nb1 * ((Ls.nb2 + 31) / 32);
+        const int ps__ = prof_begin("k_scan_cols", st);
+        k_scan_cols<<<(unsigned)blocks, 32 * kScanWarps, smem, st>>>(fin, fout, Ls, a, inv_a, per, form, me, vcap,
+                                                                      flag);
+        prof_end(ps__, (double)Ls.count() * n * (form == PMG_EDT_MORPH ? 5 : 8), st);
+    }
+    PMG_CHECK_LAUNCH();
+    return PMG_OK;
+}
+
+} // namespace pmg

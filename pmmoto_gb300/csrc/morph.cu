@@ -228,11 +228,18 @@ int morph_run(const uint8_t *img, uint8_t *out, const int64_t *shape, const int3
             return morph_cap_run(E, (uint16_t *)A, (uint16_t *)B, X, T, me, st);
     }
 
-    PMG_TRY(launch_pass0(E, A, all_lines(X, 0), res[0], plain, st));
+    // squared distances above vcap are only ever "beyond the radius"; the two
+    // voxels of margin keep them out of every near-tie below it
+    const double amax = (double)res[0] * res[0] > (double)res[1] * res[1] ? (double)res[0] * res[0]
+                                                                          : (double)res[1] * res[1];
+    const double thr = thr_sq >= 0.0 ? thr_sq : radius * radius * 1.00001;
+    const float vcap = (float)(thr + 2.0 * (amax > (double)res[2] * res[2] ? amax : (double)res[2] * res[2]));
+    PMG_TRY(launch_linear(E, A, X, res[0], plain, st));
     Lines L1 = all_lines(X, 1); // lines over (i, k): keep i inside the unextended range
     L1.b1lo = me.e0;
     L1.nb1 = (int)shape[0];
-    PMG_TRY(launch_envelope(A, B, L1, res[1], plain, 4, PMG_EDT_SQUARED, me, st, T == INT_MIN ? INT_MAX : T));
+    PMG_TRY(launch_envelope(A, B, L1, res[1], plain, 4, PMG_EDT_SQUARED, me, st, T == INT_MIN ? INT_MAX : T, nullptr,
+                            0, vcap));
     Lines L2 = all_lines(X, 2); // lines over (i, j): both inside the unextended range
     L2.b1lo = me.e0;
     L2.nb1 = (int)shape[0];
@@ -240,7 +247,7 @@ int morph_run(const uint8_t *img, uint8_t *out, const int64_t *shape, const int3
     L2.nb2 = (int)shape[1];
     if (T != INT_MIN)
         return launch_env_thresh(B, L2, res[2], T, me, st);
-    PMG_TRY(launch_envelope(B, nullptr, L2, res[2], plain, 4, PMG_EDT_MORPH, me, st));
+    PMG_TRY(launch_envelope(B, nullptr, L2, res[2], plain, 4, PMG_EDT_MORPH, me, st, INT_MAX, nullptr, 0, vcap));
     return PMG_OK;
 }
 

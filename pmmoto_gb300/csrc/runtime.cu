@@ -79,17 +79,18 @@ struct TuneSpec {
     int def, lo, hi;
 };
 static const TuneSpec g_tune_spec[kTuneKnobs] = {
-    {"edt.pair_seg", 256, 32, 8192},    // positions per thread of the strided line-pair pass
-    {"edt.pair_ctas", 32, 1, 256},      // CTAs per SM of that pass (grid cap)
-    {"edt.rows_ctas", 16, 1, 256},      // CTAs per SM of the contiguous line-pair pass
+    // (accepted without effect: knobs of a former windowed pass)
+    {"edt.pair_seg", 256, 32, 8192},
+    {"edt.pair_ctas", 32, 1, 256},
+    {"edt.rows_ctas", 16, 1, 256},
     {"cc.cross_fused", 0, 0, 1},        // block labelling: one fused cross-tile pass (1) or two (0)
-    {"edt.path", 0, 0, 2},              // envelope passes: windowed (0), exact stream (1), float envelope (2)
-    {"edt.fallback", 96, 0, 8193},      // probe samples (of 8192) from which a strided windowed pass goes to the envelope
-    {"edt.fallback_rows", 2048, 0, 8193}, // the same for the contiguous (row) pass
-    {"edt.narrow", 64, 0, 8193},        // probe samples (of 8192) below which a strided pass takes the +-8 window
-    {"edt.narrow_rows", 32, 0, 8193},   // the same for the contiguous (row) pass
+    {"edt.path", 0, 0, 2},              // envelope passes: lattice / scan (0), exact stream (1), float envelope (2)
+    {"edt.fallback", 96, 0, 8193},      // (no effect)
+    {"edt.fallback_rows", 2048, 0, 8193}, // (no effect)
+    {"edt.narrow", 64, 0, 8193},        // (no effect)
+    {"edt.narrow_rows", 32, 0, 8193},   // (no effect)
     {"cc.seam_batched", 1, 0, 1},       // periodic merge: all features' seams in one sort (1) or one by one (0)
-    {"edt.wide", 1024, 0, 8193},        // probe samples (of 8192) below which a strided pass takes the +-24 window
+    {"edt.wide", 1024, 0, 8193},        // (no effect)
 };
 static std::atomic<int> g_tune[kTuneKnobs] = {{256}, {32}, {16}, {0}, {0}, {96}, {2048}, {64}, {32}, {1}, {1024}};
 
