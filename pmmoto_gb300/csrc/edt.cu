@@ -730,30 +730,30 @@ __global__ void __launch_bounds__(kEndBlock) k_envelope_ends(const float *__rest
     }
 }
 
-// Flagged lines of the lattice passes (flag bits 0 and 2: the low and the high
-// end, bit 1: the whole line).  Heights are integer multiples K of res^2, so a
-// voxel before the first zero (after the last one) is the smaller of the value
-// the pass left there and the imported parabolas, and only the imports have to
-// be found: the last (first) num_hull + 1 finite entries of the hull of the
-// far (near) segment.  They are wrapped one by one from the line's end -- the
-// entry next to e is the vertex whose intersection with e lies closest, of
-// equal ones the farthest (the reference pops on equality) -- by
-// cross-multiplied integer comparisons.  The reference compares rounded
-// quotients: a comparison closer than their rounding (kept in `hard`) leaves
-// the line to the float replay, and so do lines flagged as a whole, segments
-// too long for 32-bit products, and longer lines without a zero (there the
-// rounding of intersections across the whole line could reach the distance to
-// an integer).  A block takes 32 adjacent lines, warp 0 their low ends and
-// warp 1 their high ones, so that the two independent chains overlap.
-// Building the reference's hull stacks instead kept a warp in divergent
-// pops and divisions: 1024^3 field 1.8 ms over both passes, 128^3 pack 0.54 ms.
-constexpr int kWrapMax = 255;   // longest segment (products below 2^31)
-constexpr int kWrapLine = 320;  // longest line without a zero
+// Flagged lines of the lattice passes (line_reach: how many positions from the
+// low and the high end, or the whole line).  Heights are integer multiples K
+// of res^2, so a voxel there is the smaller of the value the pass left and the
+// imported parabolas, and only the imports have to be found: the last (first)
+// num_hull + 1 finite entries of the hull of the far (near) segment.  They
+// are wrapped one by one from the line's end -- the entry next to e is the
+// vertex whose intersection with e lies closest, of equal ones the farthest
+// (the reference pops on equality) -- by cross-multiplied integer
+// comparisons, up to the zero that ends the segment or the distance from
+// which no height could bring an intersection closer.  The reference compares
+// rounded quotients: a best one within their rounding of another leaves the
+// line to the float replay, and so do lines flagged as a whole and searches
+// too long for 32-bit products.  A block takes 32 adjacent lines, warp 0
+// their low ends and warp 1 their high ones, so that the two independent
+// chains overlap.
+// Bound by the latency of those chains.  Building the reference's hull stacks
+// instead kept a warp in divergent pops and divisions: 1024^3 field 1.8 ms
+// over both passes, 128^3 pack 0.54 ms.
+constexpr int kWrapMax = 255; // farthest entry (products below 2^31)
 
 template <class T>
 __global__ void __launch_bounds__(64) k_lattice_ends(const T *__restrict__ fin, float *__restrict__ fout, Lines Ls,
                                                      float res, pmg_axis_cfg cfg, int num_hull, int form,
-                                                     const uint8_t *__restrict__ flag)
+                                                     const uint16_t *__restrict__ flag)
 {
     extern __shared__ uint32_t smem_bm[]; // envelope bits of the replays: [nwords][32]
     __shared__ float s_ends[2 * kEndWin * 33];
@@ -771,22 +771,20 @@ __global__ void __launch_bounds__(64) k_lattice_ends(const T *__restrict__ fin, 
             continue;
         const LineGeo g = line_addr(Ls, l0 + min(lane, lines - 1));
         const int n = g.n;
+        const bool whole = (fl & 0xff) == 255;
         __syncthreads(); // (the previous tile's readers)
         if (w == 0)
-            s_hard[lane] = fl & 2;
+            s_hard[lane] = whole;
         stage_ends(s_ends, fin, Ls, l0, lines, g, res, w, 2);
         __syncthreads();
         const LineEnds<T> line{fin + g.base, g.stride, s_ends + lane, 33, n, 0, res};
-        if (!(fl & 2) && (fl & (w == 0 ? 1 : 4))) {
-            // positions of the segment from its end that faces the line: q = 0
-            // is that end, q = nv - 1 the zero that bounds it
+        const int reach = whole ? 0 : w == 0 ? fl & 0xff : fl >> 8;
+        if (reach > 0) {
+            // positions of the segment from its end that faces the line
             const int p0 = w == 0 ? n - cfg.hb_hi - 1 : cfg.hf_lo, dir = w == 0 ? -1 : 1;
             const int most = w == 0 ? n - cfg.hb_hi : n - cfg.hf_lo;
-            int nv = 0;
-            bool zero = false;
-            while (nv < most && !zero)
-                zero = line(p0 + dir * nv++) == 0.0f;
-            bool hard = nv < 1 || nv > kWrapMax || (!zero && (n > kWrapLine || nv < 2));
+            // (a segment of one voxel without a solid one: the reference's phantom import)
+            bool hard = most < 2;
             // entries (position q, height K); q = -1: none
             int eq[kMaxHull], ek[kMaxHull];
 #pragma unroll
@@ -800,41 +798,52 @@ __global__ void __launch_bounds__(64) k_lattice_ends(const T *__restrict__ fin, 
                     return f >= FLT_MAX ? -1 : (int)fmul(f, inv_a);
                 };
                 int e = 0, ke = height(0);
-                while (ke < 0 && ++e < nv)
+                while (ke < 0 && ++e < most)
                     ke = height(e);
-                if (e < nv) {
+                if (e < most) {
                     eq[0] = e;
                     ek[0] = ke;
                 }
 #pragma unroll
                 for (int c = 1; c < kMaxHull; c++) {
-                    if (c > num_hull || e >= nv)
-                        continue;
-                    // distance from e of the intersection with q: N / D, smallest
-                    int b = nv, kb2 = 0, nb = 0, db = 1;
+                    if (c > num_hull || e >= most || ke == 0)
+                        continue; // (a zero ends the segment)
+                    // distance from e of the intersection with q: N / (2 D), smallest
+                    int b = most, kb2 = 0, nb = 0, db = 1;
                     bool near = false; // another one within the rounding of the best
-                    for (int q = e + 1; q < nv; q++) {
+                    for (int q = e + 1; q < most; q++) {
+                        const int d = q - e;
+                        // no height from here on comes within 1 / 2 of the best
+                        if (b < most && (d * d - ke) * db - nb * d > d * db)
+                            break;
+                        if (d > kWrapMax) {
+                            hard = true;
+                            break;
+                        }
                         const int k = height(q);
                         if (k < 0)
                             continue;
-                        const int d = q - e, N = k - ke + d * d;
+                        const int N = k - ke + d * d;
                         const int diff = N * db - nb * d;
-                        const float tol = 2.4e-7f * (float)(2 * max(k, max(ke, kb2)) + 6 * nv) * (float)(d * db);
-                        if (b < nv && diff != 0 && (float)abs(diff) < tol)
+                        const float tol =
+                            2.4e-7f * (float)(2 * max(k, max(ke, kb2)) + 6 * (q + 1)) * (float)(d * db);
+                        if (b < most && diff != 0 && (float)abs(diff) < tol)
                             near = true;
-                        else if (b == nv || diff < 0)
+                        else if (b == most || diff < 0)
                             near = false;
-                        if (b == nv || diff <= 0) {
+                        if (b == most || diff <= 0) {
                             b = q;
                             kb2 = k;
                             nb = N;
                             db = d;
                         }
+                        if (k == 0)
+                            break;
                     }
                     hard = hard || near;
                     e = b;
                     ke = kb2;
-                    if (e < nv) {
+                    if (e < most) {
                         eq[c] = e;
                         ek[c] = ke;
                     }
@@ -844,38 +853,42 @@ __global__ void __launch_bounds__(64) k_lattice_ends(const T *__restrict__ fin, 
                 s_hard[lane] = 1;
             } else {
                 // import c lies eq[c] + 1 beyond the line's end
-                for (int i = 0; i < n; i++) {
-                    const int x = w == 0 ? i : n - 1 - i;
-                    if (line(x) == 0.0f)
-                        break;
-                    int best = 1 << 30;
+                float *o = fout + g.base + (w == 0 ? 0 : n - 1) * g.stride;
+                const long long step = w == 0 ? g.stride : -g.stride;
+                for (int i0 = 0; i0 < reach; i0 += 4) {
+                    float cur[4];
 #pragma unroll
-                    for (int c = 0; c < kMaxHull; c++)
-                        if (eq[c] >= 0) {
-                            const int d = i + 1 + eq[c];
-                            best = min(best, ek[c] + d * d);
-                        }
-                    if (best == 1 << 30)
-                        break;
-                    float val = fmul((float)best, aniso);
-                    if (form == PMG_EDT_DIST)
-                        val = __fsqrt_rn(val);
-                    // (both ends of a line without a zero meet here; values are >= 0)
-                    float *o = fout + g.base + x * g.stride;
-                    if (val < *o)
-                        atomicMin(reinterpret_cast<int *>(o), __float_as_int(val));
+                    for (int u = 0; u < 4; u++)
+                        cur[u] = i0 + u < reach ? o[(i0 + u) * step] : 0.0f;
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const int i = i0 + u;
+                        int best = 1 << 30;
+#pragma unroll
+                        for (int c = 0; c < kMaxHull; c++)
+                            if (eq[c] >= 0) {
+                                const int d = i + 1 + eq[c];
+                                best = min(best, ek[c] + d * d);
+                            }
+                        float val = best < 1 << 30 ? fmul((float)best, aniso) : FLT_MAX;
+                        if (form == PMG_EDT_DIST)
+                            val = __fsqrt_rn(val);
+                        // (the two ends may reach the same voxel; values are >= 0)
+                        if (val < cur[u])
+                            atomicMin(reinterpret_cast<int *>(o + i * step), __float_as_int(val));
+                    }
                 }
             }
         }
         __syncthreads();
         if (w == 0 && s_hard[lane])
-            replay_line(smem_bm + lane, 32, line, g, aniso, cfg, num_hull, (fl & 2) != 0, form, MorphEpi{}, fout);
+            replay_line(smem_bm + lane, 32, line, g, aniso, cfg, num_hull, whole, form, MorphEpi{}, fout);
     }
 }
 
 template <class T>
 static int launch_lattice_ends(const T *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
-                               int num_hull, int form, const uint8_t *flag, cudaStream_t st)
+                               int num_hull, int form, const uint16_t *flag, cudaStream_t st)
 {
     const int n = (int)(Ls.ax == 0 ? Ls.s0 : Ls.ax == 1 ? Ls.s1 : Ls.s2);
     const size_t smem = (size_t)((n + 31) / 32) * 32 * 4;
@@ -888,13 +901,13 @@ static int launch_lattice_ends(const T *fin, float *fout, const Lines &Ls, float
 }
 
 int launch_ends_counts(const uint16_t *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
-                       int num_hull, const uint8_t *flag, cudaStream_t st)
+                       int num_hull, const uint16_t *flag, cudaStream_t st)
 {
     return launch_lattice_ends(fin, fout, Ls, res, cfg, num_hull, PMG_EDT_SQUARED, flag, st);
 }
 
 int launch_ends_heights(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
-                        int num_hull, int form, const uint8_t *flag, cudaStream_t st)
+                        int num_hull, int form, const uint16_t *flag, cudaStream_t st)
 {
     return launch_lattice_ends(fin, fout, Ls, res, cfg, num_hull, form, flag, st);
 }
@@ -1025,10 +1038,10 @@ int edt3d_run(const uint8_t *img, float *out, float *tmp, const int64_t *shape, 
     MorphEpi none{};
     const long long lines = (long long)shape[0] * std::max(shape[1], shape[2]);
     if (tune_value(kTuneEdtPath) == 0 && lattice_ok(shape, res, cfg) &&
-        (!flag_buf || lines <= flag_cap * (long long)sizeof(int))) {
-        uint8_t *flag = (uint8_t *)flag_buf;
+        (!flag_buf || lines <= flag_cap * (long long)(sizeof(int) / sizeof(uint16_t)))) {
+        uint16_t *flag = (uint16_t *)flag_buf;
         if (!flag_buf)
-            PMG_TRY(scratch_alloc((void **)&flag, (size_t)lines, st));
+            PMG_TRY(scratch_alloc((void **)&flag, sizeof(uint16_t) * (size_t)lines, st));
         const int s = lattice_run(img, out, tmp, shape, res, cfg, num_hull, form, flag, st);
         const int s2 = flag_buf ? PMG_OK : scratch_free(flag, st);
         return s != PMG_OK ? s : s2;

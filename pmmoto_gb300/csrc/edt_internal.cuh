@@ -176,14 +176,13 @@ int launch_linear(const uint8_t *img, float *out, const int64_t *shape, float re
 // The whole transform on the integer lattice.
 bool lattice_ok(const int64_t *shape, const float *res, const pmg_axis_cfg *cfg);
 int lattice_run(const uint8_t *img, float *out, float *tmp, const int64_t *shape, const float *res,
-                const pmg_axis_cfg *cfg, int num_hull, int form, uint8_t *flags, cudaStream_t st);
-// Flagged lines: after a lattice pass over counts or heights (one byte per
-// line: 1 the low end, 4 the high end, 2 the whole line), and after a scan (1
-// the ends, 2 the whole line).
+                const pmg_axis_cfg *cfg, int num_hull, int form, uint16_t *flags, cudaStream_t st);
+// Flagged lines: after a lattice pass over counts or heights (line_reach), and
+// after a scan (1 the ends, 2 the whole line).
 int launch_ends_counts(const uint16_t *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
-                       int num_hull, const uint8_t *flag, cudaStream_t st);
+                       int num_hull, const uint16_t *flag, cudaStream_t st);
 int launch_ends_heights(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
-                        int num_hull, int form, const uint8_t *flag, cudaStream_t st);
+                        int num_hull, int form, const uint16_t *flag, cudaStream_t st);
 int launch_ends_float(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
                       int num_hull, int form, const MorphEpi &me, const uint8_t *flag, cudaStream_t st);
 // The outward scan (edt_scan.cu), lines of at most kScanMaxLine voxels; vcap:

@@ -33,13 +33,38 @@
 
 namespace pmg {
 
+// Packed 16-bit minima and maxima as single instructions (the vminu2 / vmaxu2
+// intrinsics are sequences here: the 512 x 512 x 1024 field's row pass ran 115
+// instructions per pair of voxels with them).
+__device__ __forceinline__ uint32_t min2(uint32_t a, uint32_t b)
+{
+    uint32_t r;
+    asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b)
+{
+    uint32_t r;
+    asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+
+// Integers below 2^16 to and from float by the exponent of 2^23 (exact; the
+// conversion instructions run at a fraction of the rate).
+__device__ __forceinline__ float lo_float(uint32_t v) { return __uint_as_float(0x4B000000u | (v & 0xffffu)) - 8388608.0f; }
+__device__ __forceinline__ float hi_float(uint32_t v) { return __uint_as_float(0x4B000000u | (v >> 16)) - 8388608.0f; }
+__device__ __forceinline__ uint32_t pack_float2(float a, float b) // integers in [0, 2^16)
+{
+    return __byte_perm(__float_as_uint(a + 8388608.0f), __float_as_uint(b + 8388608.0f), 0x5410);
+}
+
 // ---------------------------------------------------------------------------
 // linear pass
 // ---------------------------------------------------------------------------
 // "No zero so far": counts grow from here by at most the line length.
 constexpr int kLinInf = 0x4000;
-constexpr int kLinChunk = 16;      // positions a thread holds at once
-constexpr int kLinChunks = 8;      // chunks per thread
+constexpr int kLinChunk = 8;       // positions a thread holds at once
+constexpr int kLinChunks = 16;     // chunks per thread
 constexpr int kLinWarps = 16;      // segments per line
 
 struct LinTab {
@@ -68,6 +93,88 @@ __device__ __forceinline__ uint32_t mask2(uint32_t b)
     return __byte_perm(b, 0u, PAIR ? 0x4342 : 0x4140) * 0xFFFFu;
 }
 
+// One chunk's masks: m = voxel nonzero, x = its value differs from the
+// neighbour's (never needed for values 0 and 1, where a change is a zero on one
+// side and the count there restarts by itself).
+template <bool BIN, int H>
+__device__ __forceinline__ void lin_masks(uint32_t v, uint32_t nb, uint32_t (&m)[H], uint32_t (&x)[H])
+{
+    const uint32_t nz = BIN ? v : nz01(v);
+    m[0] = mask2<0>(nz);
+    if constexpr (H == 2)
+        m[1] = mask2<1>(nz);
+    if constexpr (!BIN) {
+        const uint32_t df = nz01(v ^ nb);
+        x[0] = mask2<0>(df);
+        if constexpr (H == 2)
+            x[1] = mask2<1>(df);
+    }
+}
+
+// count of a voxel from the count `c` it has without an event
+template <bool BIN>
+__device__ __forceinline__ uint32_t lin_count(uint32_t c, uint32_t m, uint32_t x)
+{
+    return BIN ? c & m : ((c & ~x) | (0x00010001u & x)) & m;
+}
+
+// The counts a chunk hands on: forward through dn (in: at its first voxel, out:
+// at the voxel after it), backward from "unknown" into en (at the voxel before).
+template <bool BIN, int H>
+__device__ __forceinline__ void lin_hand_on(const uint32_t (&v)[kLinChunk + 1], uint32_t vp, int len,
+                                            uint32_t (&dn)[H], uint32_t (&en)[H])
+{
+#pragma unroll
+    for (int u = 0; u < kLinChunk; u++)
+        if (u < len) {
+            uint32_t m[H], x[H] = {};
+            lin_masks<BIN, H>(v[u], u ? v[u ? u - 1 : 0] : vp, m, x);
+#pragma unroll
+            for (int h = 0; h < H; h++)
+                dn[h] = lin_count<BIN>(dn[h], m[h], x[h]) + 0x00010001u;
+        }
+#pragma unroll
+    for (int u = kLinChunk - 1; u >= 0; u--)
+        if (u < len) {
+            uint32_t m[H], x[H] = {};
+            lin_masks<BIN, H>(v[u], v[u + 1], m, x);
+#pragma unroll
+            for (int h = 0; h < H; h++)
+                en[h] = lin_count<BIN>(en[h], m[h], x[h]) + 0x00010001u;
+        }
+}
+
+// Both directions of a chunk with the true incoming counts: put(u, counts).
+template <bool BIN, int H, class Put>
+__device__ __forceinline__ void lin_chunk(const uint32_t (&v)[kLinChunk + 1], uint32_t vp, int len, uint32_t (&dn)[H],
+                                          uint32_t (&e)[H], Put &&put)
+{
+    uint32_t d[kLinChunk][H];
+#pragma unroll
+    for (int u = 0; u < kLinChunk; u++) {
+        uint32_t m[H], x[H] = {};
+        lin_masks<BIN, H>(v[u], u ? v[u ? u - 1 : 0] : vp, m, x);
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            d[u][h] = lin_count<BIN>(dn[h], m[h], x[h]);
+            dn[h] = d[u][h] + 0x00010001u;
+        }
+    }
+#pragma unroll
+    for (int u = kLinChunk - 1; u >= 0; u--)
+        if (u < len) {
+            uint32_t m[H], x[H] = {}, r[H];
+            lin_masks<BIN, H>(v[u], v[u + 1], m, x);
+#pragma unroll
+            for (int h = 0; h < H; h++) {
+                e[h] = lin_count<BIN>(e[h], m[h], x[h]);
+                r[h] = min2(d[u][h], e[h]);
+                e[h] += 0x00010001u;
+            }
+            put(u, r);
+        }
+}
+
 // Lines along axis 0 of [n][plane], VEC adjacent lines per lane (VEC = 4 where
 // plane and the pointers are multiples of 4, else 1), blockDim = (32, segments
 // of `seg` positions).  Each thread first runs its segment from "unknown" in
@@ -77,18 +184,22 @@ __device__ __forceinline__ uint32_t mask2(uint32_t b)
 // registers and writes each output once.  An event is a zero (count 0) or a
 // change between nonzero values (count 1 on both sides).
 // Bound by HBM: 1 byte read (twice, the second time from cache) and 2 (4)
-// written per voxel.
+// written per voxel; the chunk loops stay rolled, because unrolled they miss
+// the instruction cache.
 template <int VEC, class OUT>
-__global__ void __launch_bounds__(32 * kLinWarps) k_lin(const uint8_t *__restrict__ img, OUT *__restrict__ out,
+__global__ void __launch_bounds__(32 * kLinWarps, 2) k_lin(const uint8_t *__restrict__ img, OUT *__restrict__ out,
                                                         long long plane, int n, int seg, pmg_axis_cfg cfg,
                                                         const __grid_constant__ typename TabOf<OUT>::T tab)
 {
     constexpr int H = VEC == 4 ? 2 : 1; // 32-bit words of two counts
     constexpr uint32_t kInf2 = (uint32_t)kLinInf * 0x10001u;
+    constexpr uint32_t kCap2 = kInf2 + 0x20002000u; // keeps both halves below 2^16 over long lines
     __shared__ uint32_t s_f[kLinWarps][H][32], s_b[kLinWarps][H][32];
     __shared__ uint32_t s_corr[2][H][32];
-    extern __shared__ float s_tab[];
+    extern __shared__ uint32_t s_dyn[]; // backward counts of the chunks [nw][kLinChunks][H][32], then the table
     const int lane = threadIdx.x, w = threadIdx.y, nw = blockDim.y;
+    uint32_t *s_en = s_dyn + w * kLinChunks * H * 32 + lane;
+    float *s_tab = reinterpret_cast<float *>(s_dyn + nw * kLinChunks * H * 32);
     if constexpr (sizeof(OUT) == 4)
         for (int q = w * 32 + lane; q <= n; q += nw * 32)
             s_tab[q] = tab.v[q];
@@ -102,17 +213,16 @@ __global__ void __launch_bounds__(32 * kLinWarps) k_lin(const uint8_t *__restric
             return __ldg(in + i * plane);
     };
     const int i0 = w * seg, i1 = min(n, i0 + seg);
-    // periodic correctors: counts at the first voxel from the last zero of the
-    // wrapped line and the other way round
+    const int nc = (i1 - i0 + kLinChunk - 1) / kLinChunk;
+    // periodic correctors: the count at the last voxel from the first zero of
+    // the wrapped line, and at the first voxel from the last one
     if (cfg.periodic && (w == 0 || w == nw - 1)) {
-        int pos[VEC];
-#pragma unroll
-        for (int q = 0; q < VEC; q++)
-            pos[q] = -1;
         for (int side = 0; side < 2; side++) {
             if (side == 0 ? w != 0 : w != nw - 1)
                 continue;
+            int pos[VEC];
             const int lo = side == 0 ? cfg.f_lo : cfg.l_lo, hi = side == 0 ? n : n - cfg.l_hi;
+#pragma unroll
             for (int q = 0; q < VEC; q++)
                 pos[q] = -1;
             for (int t = 0; t < hi - lo; t += 4) {
@@ -148,153 +258,109 @@ __global__ void __launch_bounds__(32 * kLinWarps) k_lin(const uint8_t *__restric
                 s_corr[side][h][lane] = VEC == 4 ? c[2 * h % VEC] | (c[(2 * h + 1) % VEC] << 16) : c[0];
         }
     }
+    uint32_t v[kLinChunk + 1];
+    // a chunk's words and the next one (the last voxel again past the line's
+    // end); true when they all are 0 or 1
+    auto load = [&](int a, uint32_t vp) -> bool {
+        uint32_t big = vp;
+#pragma unroll
+        for (int u = 0; u <= kLinChunk; u++) {
+            v[u] = row(min(a + u, n - 1));
+            big |= v[u];
+        }
+        return !__any_sync(0xffffffffu, (big & 0xfefefefeu) != 0);
+    };
     // counts handed on, from unknown incoming ones
-    uint32_t enl[kLinChunks][H]; // per chunk: the backward count just below it
-    uint32_t dn[H];
+    uint32_t dn[H], en[H];
 #pragma unroll
     for (int h = 0; h < H; h++)
         dn[h] = kInf2;
-    uint32_t vp = i0 < n ? row(i0 > 0 ? i0 - 1 : 0) : 0u;
-#pragma unroll
-    for (int c = 0; c < kLinChunks; c++) {
-        const int a = i0 + c * kLinChunk;
+    uint32_t vp = row(i0 > 0 ? i0 - 1 : 0);
+#pragma unroll 1
+    for (int c = 0; c < nc; c++) {
+        const int a = i0 + c * kLinChunk, len = min(kLinChunk, i1 - a);
+        const bool bin = load(a, vp);
 #pragma unroll
         for (int h = 0; h < H; h++)
-            enl[c][h] = kInf2;
-        if (a >= i1)
-            continue;
-        uint32_t v[kLinChunk + 1];
+            en[h] = kInf2;
+        if (bin)
+            lin_hand_on<true, H>(v, vp, len, dn, en);
+        else
+            lin_hand_on<false, H>(v, vp, len, dn, en);
 #pragma unroll
-        for (int u = 0; u <= kLinChunk; u++)
-            v[u] = row(min(a + u, n - 1));
-        const int len = min(kLinChunk, i1 - a);
-#pragma unroll
-        for (int u = 0; u < kLinChunk; u++)
-            if (u < len) {
-                const uint32_t nz = nz01(v[u]), df = nz01(v[u] ^ (u ? v[u ? u - 1 : 0] : vp));
-#pragma unroll
-                for (int h = 0; h < H; h++) {
-                    const uint32_t m = h ? mask2<1>(nz) : mask2<0>(nz), x = h ? mask2<1>(df) : mask2<0>(df);
-                    dn[h] = (((dn[h] & ~x) | (0x00010001u & x)) & m) + 0x00010001u;
-                }
-            }
-#pragma unroll
-        for (int u = kLinChunk - 1; u >= 0; u--)
-            if (u < len) {
-                const uint32_t nz = nz01(v[u]), df = nz01(v[u] ^ v[u + 1]);
-#pragma unroll
-                for (int h = 0; h < H; h++) {
-                    const uint32_t m = h ? mask2<1>(nz) : mask2<0>(nz), x = h ? mask2<1>(df) : mask2<0>(df);
-                    enl[c][h] = (((enl[c][h] & ~x) | (0x00010001u & x)) & m) + 0x00010001u;
-                }
-            }
-        vp = v[len == kLinChunk ? kLinChunk - 1 : 0]; // (a short chunk is the line's last)
+        for (int h = 0; h < H; h++)
+            s_en[(c * H + h) * 32] = en[h];
+        vp = v[kLinChunk - 1]; // (a short chunk is the line's last)
     }
-    {
-        // the segment's backward count: chunk by chunk from its high end
-        uint32_t e[H];
+    // the segment's backward count: chunk by chunk from its high end
+#pragma unroll
+    for (int h = 0; h < H; h++)
+        en[h] = kInf2;
+    for (int c = nc - 1; c >= 0; c--) {
+        const uint32_t len = (uint32_t)min(kLinChunk, i1 - i0 - c * kLinChunk) * 0x10001u;
 #pragma unroll
         for (int h = 0; h < H; h++)
-            e[h] = kInf2;
+            en[h] = min2(s_en[(c * H + h) * 32], en[h] + len);
+    }
 #pragma unroll
-        for (int c = kLinChunks - 1; c >= 0; c--) {
-            const int a = i0 + c * kLinChunk;
-            if (a >= i1)
-                continue;
-            const uint32_t len = (uint32_t)min(kLinChunk, i1 - a) * 0x10001u;
-#pragma unroll
-            for (int h = 0; h < H; h++)
-                e[h] = __vminu2(enl[c][h], e[h] + len);
-        }
-#pragma unroll
-        for (int h = 0; h < H; h++) {
-            s_f[w][h][lane] = dn[h];
-            s_b[w][h][lane] = __vminu2(e[h], kInf2 + 0x20002000u);
-        }
+    for (int h = 0; h < H; h++) {
+        s_f[w][h][lane] = dn[h];
+        s_b[w][h][lane] = min2(en[h], kCap2);
     }
     __syncthreads();
-    if (i0 >= n || !live)
-        return;
     // the true incoming counts of this segment
-    uint32_t en[H];
 #pragma unroll
     for (int h = 0; h < H; h++) {
         dn[h] = cfg.periodic ? s_corr[1][h][lane] : kInf2;
         en[h] = cfg.periodic ? s_corr[0][h][lane] : kInf2;
-        const uint32_t cap = kInf2 + 0x20002000u; // keeps both halves below 2^16 over long lines
         for (int q = 0; q < w; q++)
-            dn[h] = __vminu2(__vminu2(s_f[q][h][lane], dn[h] + (uint32_t)seg * 0x10001u), cap);
-        for (int q = (n - 1) / seg; q > w; q--) {
+            dn[h] = min2(min2(s_f[q][h][lane], dn[h] + (uint32_t)seg * 0x10001u), kCap2);
+        for (int q = nw - 1; q > w; q--) {
             const uint32_t len = (uint32_t)(min(n, (q + 1) * seg) - q * seg) * 0x10001u;
-            en[h] = __vminu2(__vminu2(s_b[q][h][lane], en[h] + len), cap);
+            en[h] = min2(min2(s_b[q][h][lane], en[h] + len), kCap2);
         }
     }
     // the backward count above every chunk
-    uint32_t ea[kLinChunks][H];
-#pragma unroll
-    for (int c = kLinChunks - 1; c >= 0; c--) {
-        const int a = i0 + c * kLinChunk;
-        const uint32_t len = a < i1 ? (uint32_t)min(kLinChunk, i1 - a) * 0x10001u : 0u;
+    for (int c = nc - 1; c >= 0; c--) {
+        const uint32_t len = (uint32_t)min(kLinChunk, i1 - i0 - c * kLinChunk) * 0x10001u;
 #pragma unroll
         for (int h = 0; h < H; h++) {
-            ea[c][h] = en[h];
-            if (a < i1)
-                en[h] = __vminu2(enl[c][h], en[h] + len);
+            const uint32_t own = s_en[(c * H + h) * 32];
+            s_en[(c * H + h) * 32] = en[h];
+            en[h] = min2(own, en[h] + len);
         }
     }
     vp = row(i0 > 0 ? i0 - 1 : 0);
-#pragma unroll
-    for (int c = 0; c < kLinChunks; c++) {
-        const int a = i0 + c * kLinChunk;
-        if (a >= i1)
-            break;
-        uint32_t v[kLinChunk + 1], d[kLinChunk][H];
-#pragma unroll
-        for (int u = 0; u <= kLinChunk; u++)
-            v[u] = row(min(a + u, n - 1));
-        const int len = min(kLinChunk, i1 - a);
-#pragma unroll
-        for (int u = 0; u < kLinChunk; u++) {
-            const uint32_t nz = nz01(v[u]), df = nz01(v[u] ^ (u ? v[u ? u - 1 : 0] : vp));
-#pragma unroll
-            for (int h = 0; h < H; h++) {
-                const uint32_t m = h ? mask2<1>(nz) : mask2<0>(nz), x = h ? mask2<1>(df) : mask2<0>(df);
-                d[u][h] = ((dn[h] & ~x) | (0x00010001u & x)) & m;
-                dn[h] = d[u][h] + 0x00010001u;
-            }
-        }
-        uint32_t e[H];
+#pragma unroll 1
+    for (int c = 0; c < nc; c++) {
+        const int a = i0 + c * kLinChunk, len = min(kLinChunk, i1 - a);
+        const bool bin = load(a, vp);
 #pragma unroll
         for (int h = 0; h < H; h++)
-            e[h] = ea[c][h];
-#pragma unroll
-        for (int u = kLinChunk - 1; u >= 0; u--) {
-            if (u >= len)
-                continue;
-            const uint32_t nz = nz01(v[u]), df = nz01(v[u] ^ v[u + 1]);
-            uint32_t r[H];
-#pragma unroll
-            for (int h = 0; h < H; h++) {
-                const uint32_t m = h ? mask2<1>(nz) : mask2<0>(nz), x = h ? mask2<1>(df) : mask2<0>(df);
-                e[h] = ((e[h] & ~x) | (0x00010001u & x)) & m;
-                r[h] = __vminu2(d[u][h], e[h]);
-                e[h] += 0x00010001u;
-            }
-            OUT *o = out + (long long)(a + u) * plane + line;
+            en[h] = s_en[(c * H + h) * 32];
+        OUT *o = out + (long long)a * plane + line;
+        auto put = [&](int u, const uint32_t (&r)[H]) {
+            if (!live)
+                return;
+            OUT *q = o + u * plane;
             if constexpr (sizeof(OUT) == 2) {
                 if constexpr (VEC == 4)
-                    *reinterpret_cast<uint2 *>(o) = make_uint2(r[0], r[H - 1]);
+                    *reinterpret_cast<uint2 *>(q) = make_uint2(r[0], r[H - 1]);
                 else
-                    *o = (OUT)r[0];
+                    *q = (OUT)r[0];
             } else {
-                auto val = [&](uint32_t q) { return q <= (uint32_t)n ? s_tab[q] : FLT_MAX; };
+                auto val = [&](uint32_t k) { return k <= (uint32_t)n ? s_tab[k] : FLT_MAX; };
                 if constexpr (VEC == 4)
-                    *reinterpret_cast<float4 *>(o) = make_float4(val(r[0] & 0xffffu), val(r[0] >> 16),
+                    *reinterpret_cast<float4 *>(q) = make_float4(val(r[0] & 0xffffu), val(r[0] >> 16),
                                                                  val(r[H - 1] & 0xffffu), val(r[H - 1] >> 16));
                 else
-                    *o = (OUT)val(r[0] & 0xffffu);
+                    *q = (OUT)val(r[0] & 0xffffu);
             }
-        }
+        };
+        if (bin)
+            lin_chunk<true, H>(v, vp, len, dn, en, put);
+        else
+            lin_chunk<false, H>(v, vp, len, dn, en, put);
         vp = v[kLinChunk - 1];
     }
 }
@@ -322,7 +388,7 @@ static int launch_lin_t(const uint8_t *img, OUT *out, const int64_t *shape, floa
     const int seg = ((n + parts - 1) / parts + kLinChunk - 1) / kLinChunk * kLinChunk;
     const dim3 block(32, (unsigned)((n + seg - 1) / seg));
     typename TabOf<OUT>::T tab;
-    size_t smem = 0;
+    size_t smem = sizeof(uint32_t) * (size_t)block.y * kLinChunks * 2 * 32;
     if constexpr (sizeof(OUT) == 4) {
         // the reference's running sum of res, squared (_distance.hpp:135-182)
         float d = 0.0f;
@@ -332,10 +398,14 @@ static int launch_lin_t(const uint8_t *img, OUT *out, const int64_t *shape, floa
             volatile float nd = d + res;
             d = nd;
         }
-        smem = sizeof(float) * (size_t)(n + 1);
+        smem += sizeof(float) * (size_t)(n + 1);
     }
     const bool quads = !(plane & 3) && !(reinterpret_cast<uintptr_t>(img) & 3) &&
                        !(reinterpret_cast<uintptr_t>(out) & (4 * sizeof(OUT) - 1));
+    if (smem > 36 * 1024) { // (with the static arrays above the default limit)
+        PMG_CUDA(cudaFuncSetAttribute(k_lin<4, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PMG_CUDA(cudaFuncSetAttribute(k_lin<1, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    }
     const int ps__ = prof_begin("k_lin", st);
     if (quads)
         k_lin<4, OUT><<<(unsigned)((plane / 4 + 31) / 32), block, smem, st>>>(img, out, plane, n, seg, cfg, tab);
@@ -363,7 +433,7 @@ int launch_lin_float(const uint8_t *img, float *out, const int64_t *shape, float
 // ---------------------------------------------------------------------------
 // Heights of kBig and more count as absent; kBig + 2 * kMaxStep stays below
 // 2^16, and (kMaxStep + 1)^2 is above every height below kBig.
-constexpr uint32_t kBig = 60000u, kMaxStep = 245u;
+constexpr uint32_t kBig = 60000u, kMaxStep = 245u, kWholeLine = 255u;
 constexpr uint32_t kBig2 = kBig * 0x10001u;
 
 // (count, count) -> (K, K), absent counts -> kBig
@@ -373,35 +443,112 @@ __device__ __forceinline__ uint32_t square2(uint32_t c)
     return min(a * a, kBig) | (min(b * b, kBig) << 16);
 }
 
+// height of an integer minimum
+__device__ __forceinline__ float par_value(float k, float a) { return k >= (float)kBig ? FLT_MAX : fmul(k, a); }
+
 // larger of the two halves
 __device__ __forceinline__ uint32_t hmax(uint32_t v) { return max(v & 0xffffu, v >> 16); }
 
-// flag bits of a voxel (see the file comment); el, er: squared distances to
-// the imports beyond the line's ends
-__device__ __forceinline__ unsigned line_need(uint32_t m, int x, int n, int periodic, int wide)
+// Steps k and k + 1 on P positions in registers, given the two values on
+// either side before step k; returns the maxima of the first `valid` results.
+template <int P>
+__device__ __forceinline__ uint32_t par_steps(uint32_t (&g)[P], uint32_t l2, uint32_t l1, uint32_t r1, uint32_t r2,
+                                              uint32_t k, int valid)
 {
-    if (m >= kBig)
-        return periodic || wide ? 2u : 0u;
-    if (!periodic)
-        return 0u;
-    const uint32_t lo = (uint32_t)(x + 1), hi = (uint32_t)(n - x);
-    return (m > lo * lo ? 1u : 0u) | (m > hi * hi ? 4u : 0u);
+    const uint32_t c = (2 * k - 1) * 0x10001u, d = c + 0x00020002u;
+    // the neighbours' end values after step k
+    uint32_t prev = l1, left = __viaddmin_u16x2(min2(l2, g[0]), c, l1);
+    uint32_t right = __viaddmin_u16x2(min2(g[P - 1], r2), c, r1);
+#pragma unroll
+    for (int p = 0; p < P; p++) {
+        const uint32_t cur = g[p];
+        g[p] = __viaddmin_u16x2(prev, c, __viaddmin_u16x2(p + 1 < P ? g[p + 1 < P ? p + 1 : p] : r1, c, cur));
+        prev = cur;
+    }
+    prev = left;
+#pragma unroll
+    for (int p = 0; p < P; p++) {
+        const uint32_t cur = g[p];
+        g[p] = __viaddmin_u16x2(prev, d, __viaddmin_u16x2(p + 1 < P ? g[p + 1 < P ? p + 1 : p] : right, d, cur));
+        prev = cur;
+    }
+    uint32_t mx = 0;
+    if (valid >= P) {
+#pragma unroll
+        for (int p = 0; p < P; p += 2)
+            mx = __vimax3_u16x2(mx, g[p], g[p + 1]);
+    } else {
+#pragma unroll
+        for (int p = 0; p < P; p++)
+            if (p < valid)
+                mx = max2(mx, g[p]);
+    }
+    return mx;
+}
+
+// How far the imports beyond a periodic line's ends can reach into it, and
+// lines that need the float envelope: byte 0 (1) is one more than the last
+// position from the low (high) end whose minimum exceeds the squared distance
+// to the first import, byte 0 = kWholeLine the whole line.  g: the minima of
+// positions x0 ... of two lines, mx: their maxima (of valid positions); bytes
+// 0-1 for the line in the low halves, 2-3 for the other.
+template <int P>
+__device__ __forceinline__ uint32_t line_reach(const uint32_t (&g)[P], uint32_t mx, int x0, int n, int periodic,
+                                               int wide, bool second)
+{
+    const uint32_t big = hmax(mx);
+    const int last = min(x0 + P, n) - 1;
+    uint32_t lo0 = 0, lo1 = 0, hi0 = 0, hi1 = 0;
+    if (periodic && big > (uint32_t)((x0 + 1) * (x0 + 1)))
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            const uint32_t e = (uint32_t)(x0 + p + 1);
+            if (x0 + p < n && e <= kMaxStep) {
+                if ((g[p] & 0xffffu) > e * e)
+                    lo0 = e;
+                if ((g[p] >> 16) > e * e)
+                    lo1 = e;
+            }
+        }
+    if (periodic && big > (uint32_t)((n - last) * (n - last)))
+#pragma unroll
+        for (int p = P - 1; p >= 0; p--) {
+            const uint32_t e = (uint32_t)(n - x0 - p);
+            if (x0 + p < n && e <= kMaxStep) {
+                if ((g[p] & 0xffffu) > e * e)
+                    hi0 = e;
+                if ((g[p] >> 16) > e * e)
+                    hi1 = e;
+            }
+        }
+    if (big >= kBig && (periodic || wide)) {
+        if ((mx & 0xffffu) >= kBig)
+            lo0 = kWholeLine;
+        if ((mx >> 16) >= kBig)
+            lo1 = kWholeLine;
+    }
+    return lo0 | (hi0 << 8) | (second ? (lo1 << 16) | (hi1 << 24) : 0u);
 }
 
 // Strided pass along axis 1 of [n0][n][s2]: one thread block per plane and
-// 32 * VEC adjacent lines (VEC = 2: two lines per lane, s2 even), warp w on
-// positions [w P, (w + 1) P) of its lines, heights in registers.  Warps hand
-// their end values on through shared memory, one barrier per step.
-template <int P, int VEC>
-__global__ void __launch_bounds__(32 * P) k_par_cols(const uint16_t *__restrict__ D, float *__restrict__ out, int n, int s2, float a,
-                           int periodic, int wide, uint8_t *__restrict__ flag)
+// LN * VEC adjacent lines (VEC = 2: two lines per thread, s2 even), thread
+// group q of LN on positions [q P, (q + 1) P) of its lines, heights in
+// registers.  Groups hand their end values on through shared memory, one
+// barrier per step.  Lines beyond 512 voxels take LN = 16, so that two blocks
+// share an SM and one loads while the other computes.
+// Bound by the packed add-min pipe (two instructions per pair of voxels and
+// distance).
+template <int P, int VEC, int LN>
+__global__ void __launch_bounds__(P == 32 ? 512 : 32 * P, P == 32 ? 2 : 1)
+    k_par_cols(const uint16_t *__restrict__ D, float *__restrict__ out, int n, int s2, float a, int periodic, int wide,
+               uint16_t *__restrict__ flag)
 {
-    extern __shared__ uint32_t s_end[]; // [2][nw][2][32]
-    const int lane = threadIdx.x, w = threadIdx.y, nw = blockDim.y;
-    const int k0 = (blockIdx.x * 32 + lane) * VEC;
-    const bool live = k0 < s2;
-    const long long base = (long long)blockIdx.y * n * s2 + k0;
+    extern __shared__ uint32_t s_end[]; // [2][groups][4][LN]
+    const int l = threadIdx.x % LN, w = threadIdx.x / LN, nw = blockDim.x / LN;
+    const int k0 = (blockIdx.x * LN + l) * VEC;
     const int x0 = w * P;
+    const bool live = k0 < s2 && x0 < n;
+    const long long base = (long long)blockIdx.y * n * s2 + k0;
     uint32_t g[P];
     const uint16_t *src = D + base + (long long)x0 * s2;
 #pragma unroll
@@ -420,71 +567,68 @@ __global__ void __launch_bounds__(32 * P) k_par_cols(const uint16_t *__restrict_
     for (int p = 0; p < P; p++) {
         g[p] = square2(g[p]);
         if (x0 + p < n)
-            mx = __vmaxu2(mx, g[p]);
+            mx = max2(mx, g[p]);
     }
     if (!live)
         mx = 0;
     if (VEC == 1)
         mx &= 0xffffu;
-    for (uint32_t k = 1; k <= kMaxStep; k++) {
-        uint32_t *e = s_end + (size_t)(k & 1) * nw * 64;
-        e[(w * 2) * 32 + lane] = g[0];
-        e[(w * 2 + 1) * 32 + lane] = g[P - 1];
+    // two steps per round: the neighbours' two end values on either side
+    for (uint32_t k = 1; k <= kMaxStep; k += 2) {
+        uint32_t *e = s_end + (size_t)((k >> 1) & 1) * nw * 4 * LN + l;
+        e[(w * 4 + 0) * LN] = g[0];
+        e[(w * 4 + 1) * LN] = g[1];
+        e[(w * 4 + 2) * LN] = g[P - 2];
+        e[(w * 4 + 3) * LN] = g[P - 1];
         const bool open = hmax(mx) > k * k;
         if (!__syncthreads_or(open))
             break;
         if (!__any_sync(0xffffffffu, open))
             continue; // this warp's values are final
-        uint32_t prev = w > 0 ? e[((w - 1) * 2 + 1) * 32 + lane] : kBig2;
-        const uint32_t right = w + 1 < nw ? e[((w + 1) * 2) * 32 + lane] : kBig2;
-        const uint32_t c = (2 * k - 1) * 0x10001u;
-        mx = 0;
-#pragma unroll
-        for (int p = 0; p < P; p++) {
-            const uint32_t cur = g[p];
-            const uint32_t t = __vminu2(prev, p + 1 < P ? g[p + 1 < P ? p + 1 : p] : right);
-            g[p] = __viaddmin_u16x2(t, c, cur);
-            if (x0 + p < n)
-                mx = __vmaxu2(mx, g[p]);
-            prev = cur;
+        uint32_t l2 = kBig2, l1 = kBig2, r1 = kBig2, r2 = kBig2;
+        if (w > 0) {
+            l2 = e[(w * 4 - 2) * LN];
+            l1 = e[(w * 4 - 1) * LN];
         }
+        if (w + 1 < nw) {
+            r1 = e[(w * 4 + 4) * LN];
+            r2 = e[(w * 4 + 5) * LN];
+        }
+        mx = par_steps<P>(g, l2, l1, r1, r2, k, n - x0);
         if (!live)
             mx = 0;
         if (VEC == 1)
             mx &= 0xffffu;
     }
-    unsigned need0 = 0, need1 = 0;
     if (live) {
         float *dst = out + base + (long long)x0 * s2;
 #pragma unroll
         for (int p = 0; p < P; p++) {
             if (x0 + p >= n)
                 break;
-            const uint32_t lo = g[p] & 0xffffu, hi = g[p] >> 16;
-            const float f0 = lo >= kBig ? FLT_MAX : fmul((float)lo, a);
+            const float f0 = par_value(lo_float(g[p]), a);
             if constexpr (VEC == 2) {
-                const float f1 = hi >= kBig ? FLT_MAX : fmul((float)hi, a);
+                const float f1 = par_value(hi_float(g[p]), a);
                 *reinterpret_cast<float2 *>(dst + (long long)p * s2) = make_float2(f0, f1);
-                need1 |= line_need(hi, x0 + p, n, periodic, wide);
             } else {
                 dst[(long long)p * s2] = f0;
             }
-            need0 |= line_need(lo, x0 + p, n, periodic, wide);
         }
     }
     if (!flag)
         return;
     __syncthreads();
-    s_end[w * 32 + lane] = need0 | (need1 << 8);
+    s_end[w * LN + l] = live ? line_reach<P>(g, mx, x0, n, periodic, wide, VEC == 2) : 0u;
     __syncthreads();
     if (w == 0 && live) {
-        unsigned need = 0;
+        uint32_t need = 0;
         for (int q = 0; q < nw; q++)
-            need |= s_end[q * 32 + lane];
-        uint8_t *fl = flag + (long long)blockIdx.y * s2 + k0;
-        fl[0] = (uint8_t)need;
+            need = __vmaxu4(need, s_end[q * LN + l]);
+        uint16_t *fl = flag + (long long)blockIdx.y * s2 + k0;
         if constexpr (VEC == 2)
-            fl[1] = (uint8_t)(need >> 8);
+            *reinterpret_cast<uint32_t *>(fl) = need;
+        else
+            *fl = (uint16_t)need;
     }
 }
 
@@ -495,10 +639,10 @@ __global__ void __launch_bounds__(32 * P) k_par_cols(const uint16_t *__restrict_
 constexpr int kRowWarps = 8;
 
 template <int P>
-__global__ void __launch_bounds__(32 * kRowWarps) k_par_rows(const float *__restrict__ fin, float *__restrict__ fout,
+__global__ void __launch_bounds__(32 * kRowWarps, 4) k_par_rows(const float *__restrict__ fin, float *__restrict__ fout,
                                                              long long nrows, int n, float a, float inv_a,
                                                              int periodic, int wide, int form,
-                                                             uint8_t *__restrict__ flag)
+                                                             uint16_t *__restrict__ flag)
 {
     constexpr int kWords = 32 * P + 32;
     extern __shared__ uint32_t s_rows[];
@@ -507,16 +651,14 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_par_rows(const float *__rest
     const long long pairs = (nrows + 1) >> 1;
     const bool vec4 = !(n & 3) && !((reinterpret_cast<uintptr_t>(fin) | reinterpret_cast<uintptr_t>(fout)) & 15);
     auto pack = [&](float f0, float f1) -> uint32_t {
-        const uint32_t u0 = (uint32_t)fminf(fmul(f0, inv_a), (float)kBig);
-        const uint32_t u1 = (uint32_t)fminf(fmul(f1, inv_a), (float)kBig);
-        return u0 | (u1 << 16);
+        return pack_float2(fminf(fmul(f0, inv_a), (float)kBig), fminf(fmul(f1, inv_a), (float)kBig));
     };
     auto slot = [](int c) { return c + c / P; };
     for (long long r = blockIdx.x * (long long)kRowWarps + w; r < pairs; r += (long long)gridDim.x * kRowWarps) {
         const bool two = 2 * r + 1 < nrows;
         const float *in0 = fin + 2 * r * n, *in1 = in0 + (two ? n : 0);
         if (vec4) {
-#pragma unroll
+#pragma unroll 2
             for (int t = 0; t < (P + 3) / 4; t++) {
                 const int c = (t * 32 + lane) * 4;
                 if (c < n) {
@@ -529,7 +671,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_par_rows(const float *__rest
                 }
             }
         } else {
-#pragma unroll
+#pragma unroll 4
             for (int t = 0; t < P; t++) {
                 const int c = t * 32 + lane;
                 if (c < n)
@@ -543,73 +685,68 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_par_rows(const float *__rest
         for (int p = 0; p < P; p++) {
             g[p] = x0 + p < n ? row[lane * (P + 1) + p] : kBig2;
             if (x0 + p < n)
-                mx = __vmaxu2(mx, g[p]);
+                mx = max2(mx, g[p]);
         }
-        for (uint32_t k = 1; k <= kMaxStep; k++) {
+        for (uint32_t k = 1; k <= kMaxStep; k += 2) {
             if (!__any_sync(0xffffffffu, hmax(mx) > k * k))
                 break;
-            uint32_t prev = __shfl_up_sync(0xffffffffu, g[P - 1], 1);
-            uint32_t right = __shfl_down_sync(0xffffffffu, g[0], 1);
-            prev = lane > 0 ? prev : kBig2;
-            right = lane < 31 ? right : kBig2;
-            const uint32_t c = (2 * k - 1) * 0x10001u;
-            mx = 0;
-#pragma unroll
-            for (int p = 0; p < P; p++) {
-                const uint32_t cur = g[p];
-                const uint32_t t = __vminu2(prev, p + 1 < P ? g[p + 1 < P ? p + 1 : p] : right);
-                g[p] = __viaddmin_u16x2(t, c, cur);
-                if (x0 + p < n)
-                    mx = __vmaxu2(mx, g[p]);
-                prev = cur;
-            }
+            uint32_t l1 = __shfl_up_sync(0xffffffffu, g[P - 1], 1), l2 = __shfl_up_sync(0xffffffffu, g[P - 2], 1);
+            uint32_t r1 = __shfl_down_sync(0xffffffffu, g[0], 1), r2 = __shfl_down_sync(0xffffffffu, g[1], 1);
+            if (lane == 0)
+                l1 = l2 = kBig2;
+            if (lane == 31)
+                r1 = r2 = kBig2;
+            mx = par_steps<P>(g, l2, l1, r1, r2, k, n - x0);
         }
-        unsigned need = 0;
 #pragma unroll
         for (int p = 0; p < P; p++)
-            if (x0 + p < n) {
+            if (x0 + p < n)
                 row[lane * (P + 1) + p] = g[p];
-                need |= line_need(g[p] & 0xffffu, x0 + p, n, periodic, wide) |
-                        (line_need(g[p] >> 16, x0 + p, n, periodic, wide) << 8);
-            }
         __syncwarp();
-        auto value = [&](uint32_t m) -> float {
-            const float f = m >= kBig ? FLT_MAX : fmul((float)m, a);
+        auto value = [&](float k) -> float {
+            const float f = par_value(k, a);
             return form == PMG_EDT_DIST ? __fsqrt_rn(f) : f;
         };
         float *o0 = fout + 2 * r * n, *o1 = o0 + n;
         if (vec4) {
-#pragma unroll
+#pragma unroll 2
             for (int t = 0; t < (P + 3) / 4; t++) {
                 const int c = (t * 32 + lane) * 4;
                 if (c < n) {
                     const uint32_t q0 = row[slot(c)], q1 = row[slot(c + 1)], q2 = row[slot(c + 2)],
                                    q3 = row[slot(c + 3)];
-                    *reinterpret_cast<float4 *>(o0 + c) = make_float4(value(q0 & 0xffffu), value(q1 & 0xffffu),
-                                                                      value(q2 & 0xffffu), value(q3 & 0xffffu));
+                    *reinterpret_cast<float4 *>(o0 + c) = make_float4(value(lo_float(q0)), value(lo_float(q1)),
+                                                                      value(lo_float(q2)), value(lo_float(q3)));
                     if (two)
                         *reinterpret_cast<float4 *>(o1 + c) =
-                            make_float4(value(q0 >> 16), value(q1 >> 16), value(q2 >> 16), value(q3 >> 16));
+                            make_float4(value(hi_float(q0)), value(hi_float(q1)), value(hi_float(q2)), value(hi_float(q3)));
                 }
             }
         } else {
-#pragma unroll
+#pragma unroll 4
             for (int t = 0; t < P; t++) {
                 const int c = t * 32 + lane;
                 if (c < n) {
                     const uint32_t q = row[slot(c)];
-                    o0[c] = value(q & 0xffffu);
+                    o0[c] = value(lo_float(q));
                     if (two)
-                        o1[c] = value(q >> 16);
+                        o1[c] = value(hi_float(q));
                 }
             }
         }
         if (flag) {
-            need = __reduce_or_sync(0xffffffffu, need);
+            uint32_t need = x0 < n ? line_reach<P>(g, mx, x0, n, periodic, wide, two) : 0u;
+            if (__any_sync(0xffffffffu, need != 0)) {
+                uint32_t all = 0;
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    all |= __reduce_max_sync(0xffffffffu, (need >> (8 * q)) & 0xffu) << (8 * q);
+                need = all;
+            }
             if (lane == 0) {
-                flag[2 * r] = (uint8_t)need;
+                flag[2 * r] = (uint16_t)need;
                 if (two)
-                    flag[2 * r + 1] = (uint8_t)(need >> 8);
+                    flag[2 * r + 1] = (uint16_t)(need >> 16);
             }
         }
         __syncwarp();
@@ -623,23 +760,25 @@ bool lattice_ok(const int64_t *shape, const float *res, const pmg_axis_cfg *cfg)
     return window_path_ok(res[1], (int)shape[1]) && window_path_ok(res[2], (int)shape[2]);
 }
 
-template <int P>
+template <int P, int LN>
 static void cols_p(const uint16_t *D, float *out, int n0, int n, int s2, float a, int periodic, int wide,
-                   uint8_t *flag, cudaStream_t st)
+                   uint16_t *flag, cudaStream_t st)
 {
-    const int nw = (n + P - 1) / P;
-    const size_t smem = (size_t)nw * 128 * sizeof(uint32_t);
+    // whole warps (the last group may lie past the line's end)
+    const int groups = ((n + P - 1) / P + 32 / LN - 1) / (32 / LN) * (32 / LN);
+    const size_t smem = (size_t)groups * 8 * LN * sizeof(uint32_t);
+    const unsigned threads = (unsigned)(groups * LN);
     if (!(s2 & 1))
-        k_par_cols<P, 2><<<dim3((unsigned)((s2 / 2 + 31) / 32), (unsigned)n0), dim3(32, (unsigned)nw), smem, st>>>(
+        k_par_cols<P, 2, LN><<<dim3((unsigned)((s2 / 2 + LN - 1) / LN), (unsigned)n0), threads, smem, st>>>(
             D, out, n, s2, a, periodic, wide, flag);
     else
-        k_par_cols<P, 1><<<dim3((unsigned)((s2 + 31) / 32), (unsigned)n0), dim3(32, (unsigned)nw), smem, st>>>(
+        k_par_cols<P, 1, LN><<<dim3((unsigned)((s2 + LN - 1) / LN), (unsigned)n0), threads, smem, st>>>(
             D, out, n, s2, a, periodic, wide, flag);
 }
 
 template <int P>
 static void rows_p(const float *fin, float *fout, long long nrows, int n, float a, int periodic, int wide, int form,
-                   uint8_t *flag, cudaStream_t st)
+                   uint16_t *flag, cudaStream_t st)
 {
     const size_t smem = sizeof(uint32_t) * (size_t)kRowWarps * (32 * P + 32);
     const long long pairs = (nrows + 1) >> 1;
@@ -648,9 +787,9 @@ static void rows_p(const float *fin, float *fout, long long nrows, int n, float 
 }
 
 // The three passes: counts in `out`, the first envelope in `tmp`, the result
-// in `out`.  flags: one byte per line of the larger envelope pass.
+// in `out`.  flags: one entry per line of the larger envelope pass.
 int lattice_run(const uint8_t *img, float *out, float *tmp, const int64_t *shape, const float *res,
-                const pmg_axis_cfg *cfg, int num_hull, int form, uint8_t *flags, cudaStream_t st)
+                const pmg_axis_cfg *cfg, int num_hull, int form, uint16_t *flags, cudaStream_t st)
 {
     const int n0 = (int)shape[0], n1 = (int)shape[1], n2 = (int)shape[2];
     const float a = res[0] * res[0];
@@ -662,14 +801,16 @@ int lattice_run(const uint8_t *img, float *out, float *tmp, const int64_t *shape
     const int wide1 = m1 >= (long long)kBig, wide2 = m1 + (long long)n2 * n2 >= (long long)kBig;
     {
         const int per = cfg[1].periodic ? 1 : 0;
-        uint8_t *fl = per || wide1 ? flags : nullptr;
+        uint16_t *fl = per || wide1 ? flags : nullptr;
         const int ps__ = prof_begin("k_par_cols", st);
         if (n1 <= 64)
-            cols_p<8>(D, tmp, n0, n1, n2, a, per, wide1, fl, st);
+            cols_p<8, 32>(D, tmp, n0, n1, n2, a, per, wide1, fl, st);
         else if (n1 <= 256)
-            cols_p<16>(D, tmp, n0, n1, n2, a, per, wide1, fl, st);
+            cols_p<16, 32>(D, tmp, n0, n1, n2, a, per, wide1, fl, st);
+        else if (n1 <= 512)
+            cols_p<32, 32>(D, tmp, n0, n1, n2, a, per, wide1, fl, st);
         else
-            cols_p<32>(D, tmp, n0, n1, n2, a, per, wide1, fl, st);
+            cols_p<32, 16>(D, tmp, n0, n1, n2, a, per, wide1, fl, st);
         prof_end(ps__, (double)n0 * n1 * n2 * 6, st);
         PMG_CHECK_LAUNCH();
         if (fl)
@@ -677,7 +818,7 @@ int lattice_run(const uint8_t *img, float *out, float *tmp, const int64_t *shape
     }
     {
         const int per = cfg[2].periodic ? 1 : 0;
-        uint8_t *fl = per || wide2 ? flags : nullptr;
+        uint16_t *fl = per || wide2 ? flags : nullptr;
         const long long nrows = (long long)n0 * n1;
         const int ps__ = prof_begin("k_par_rows", st);
         if (n2 <= 64)

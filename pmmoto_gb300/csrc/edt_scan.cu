@@ -21,10 +21,10 @@
 // line a voxel whose m reaches the squared distance to a line end may depend
 // on the imported hulls: the line is flagged for its end segments.
 //
-// Lines are staged in shared memory (a thread's serial float envelope spends
-// its time waiting on dependent global loads; here every voxel is its own
-// thread and a candidate costs one shared-memory read and five
-// instructions).
+// Lines are staged in shared memory: a thread's serial float envelope spends
+// its time waiting on dependent loads, while here every voxel is its own
+// thread and bound by instruction issue (a shared-memory read and about five
+// instructions per candidate).
 #include <cfloat>
 #include <algorithm>
 
@@ -44,8 +44,9 @@ __device__ __forceinline__ float scan_eta(float a, float m, float R, float x)
 // The near parabolas of position x pushed in order as update_hull does
 // (_distance.hpp:89-112), then the reference's evaluation at x.  Returns false
 // when the line has to be replayed.
-template <class H>
-__device__ __noinline__ bool scan_resolve(const H &h, int n, int x, float a, float m, float R, float eta, float &out)
+template <int S>
+__device__ __noinline__ bool scan_resolve(const float *line, int n, int x, float a, float m, float R, float eta,
+                                          float &out)
 {
     if (0.25f < (3.0f * R + 1.0f) * (7.0f * R + 3.0f * (float)x + 8.0f) * 2.4e-7f)
         return false;
@@ -56,7 +57,7 @@ __device__ __noinline__ bool scan_resolve(const H &h, int n, int x, float a, flo
     const float top = m + 0.5f * a;
     const int D = (int)__fsqrt_rn(top / a) + 1;
     for (int q = max(0, x - D); q <= min(n - 1, x + D); q++) {
-        const float dx = (float)(q - x), fq = h(q);
+        const float dx = (float)(q - x), fq = line[S * q];
         const float val = fadd(fmul(a, fmul(dx, dx)), fq);
         if (val <= m + eta) {
             if (++seen > kNear)
@@ -85,27 +86,47 @@ __device__ __noinline__ bool scan_resolve(const H &h, int n, int x, float a, flo
     return true;
 }
 
-// One voxel per lane (x < n on live lanes): the value and its line's flag bits.
-template <class H>
-__device__ __forceinline__ float scan_voxel(const H &h, int n, int x, bool live, float a, float inv_a, int periodic,
-                                            float vcap, unsigned &need)
+// The smallest value m and the next larger one m2, updated with the values of
+// positions x - d and x + d.
+__device__ __forceinline__ void scan_pair(float v0, float v1, float &m, float &m2)
 {
-    float m = live ? h(x) : 0.0f, m2 = INFINITY;
+    const float lo = fminf(v0, v1), hi = fmaxf(v0, v1), t = fmaxf(lo, m);
+    m = fminf(lo, m);
+    m2 = fminf(m2, fminf(hi == m ? INFINITY : hi, t == m ? INFINITY : t));
+}
+
+// One voxel per lane: the value and its line's flag bits.  line: the staged
+// line (position v at line[S v]); a lane past the line's end (not live) reads
+// at the last position; safe: with safe > 0 every lane's x - safe and x + safe
+// lie inside the line.
+template <int S>
+__device__ __forceinline__ float scan_voxel(const float *line, int n, int x, int safe, bool live, float a, float inv_a,
+                                            int periodic, float vcap, unsigned &need)
+{
+    x = min(x, n - 1);
+    const float *c = line + S * x;
+    float m = *c, m2 = INFINITY;
     const float half = 0.5f * a;
-    for (int d = 1; d < n; d++) {
+    int d = 1;
+    bool open = true;
+    // two distances per step while both sides lie inside the line
+    for (const float *l = c - S, *r = c + S; d + 1 <= safe; d += 2, l -= 2 * S, r += 2 * S) {
         const float ad = fmul(a, (float)(d * d));
-        if (!__any_sync(0xffffffffu, live && ad <= m + half && ad <= vcap))
+        open = __any_sync(0xffffffffu, live && ad <= fminf(m + half, vcap));
+        if (!open)
             break;
-        if (live) {
-            // past a line end: the end position again, at a distance beyond its
-            // own, so more than a / 2 above the value it had there
-            const float v0 = fadd(ad, h(max(x - d, 0))), t0 = fmaxf(v0, m);
-            m = fminf(v0, m);
-            m2 = t0 != m ? fminf(m2, t0) : m2;
-            const float v1 = fadd(ad, h(min(x + d, n - 1))), t1 = fmaxf(v1, m);
-            m = fminf(v1, m);
-            m2 = t1 != m ? fminf(m2, t1) : m2;
-        }
+        const float ae = fmul(a, (float)((d + 1) * (d + 1)));
+        scan_pair(fadd(ad, l[0]), fadd(ad, r[0]), m, m2);
+        scan_pair(fadd(ae, l[-S]), fadd(ae, r[S]), m, m2);
+    }
+    // near a line end, one distance at a time
+    for (; open && d < n; d++) {
+        const float ad = fmul(a, (float)(d * d));
+        if (!__any_sync(0xffffffffu, live && ad <= fminf(m + half, vcap)))
+            break;
+        const float v0 = x - d >= 0 ? fadd(ad, line[S * (x - d)]) : INFINITY;
+        const float v1 = x + d < n ? fadd(ad, line[S * (x + d)]) : INFINITY;
+        scan_pair(v0, v1, m, m2);
     }
     if (!live || m > vcap)
         return m;
@@ -124,21 +145,12 @@ __device__ __forceinline__ float scan_voxel(const H &h, int n, int x, bool live,
     }
     if (m2 <= m + eta) {
         float v = m;
-        if (scan_resolve(h, n, x, a, m, R, eta, v))
+        if (scan_resolve<S>(line, n, x, a, m, R, eta, v))
             return v;
         need |= 2u;
     }
     return m;
 }
-
-struct ColH {
-    const float *s; // position v of this lane's line at s[32 v]
-    __device__ __forceinline__ float operator()(int v) const { return s[v * 32]; }
-};
-struct RowH {
-    const float *s;
-    __device__ __forceinline__ float operator()(int v) const { return s[v]; }
-};
 
 // Strided lines (axis 0 or 1): one block per 32 adjacent lines, warp w on
 // positions w, w + 8, ...
@@ -162,10 +174,9 @@ __global__ void __launch_bounds__(32 * kScanWarps) k_scan_cols(const float *__re
     for (int x = w; x < n; x += kScanWarps)
         s_line[x * 32 + lane] = __ldg(src + x * g.stride);
     __syncthreads();
-    const ColH h{s_line + lane};
     unsigned need = 0;
     for (int x = w; x < n; x += kScanWarps) {
-        const float v = scan_voxel(h, n, x, live, a, inv_a, periodic, vcap, need);
+        const float v = scan_voxel<32>(s_line + lane, n, x, min(x, n - 1 - x), live, a, inv_a, periodic, vcap, need);
         if (!live)
             continue;
         if (form == PMG_EDT_MORPH)
@@ -198,12 +209,11 @@ __global__ void __launch_bounds__(32 * kScanWarps) k_scan_rows(const float *__re
         for (int x = lane; x < n; x += 32)
             row[x] = __ldg(src + x);
         __syncwarp();
-        const RowH h{row};
         unsigned need = 0;
         for (int x0 = 0; x0 < n; x0 += 32) {
             const int x = x0 + lane;
             const bool live = x < n;
-            const float v = scan_voxel(h, n, x, live, a, inv_a, periodic, vcap, need);
+            const float v = scan_voxel<1>(row, n, x, min(x0, n - 32 - x0), live, a, inv_a, periodic, vcap, need);
             if (!live)
                 continue;
             if (form == PMG_EDT_MORPH)
