@@ -11,11 +11,11 @@
 // always links the larger root under the smaller, so a component's final root
 // is its smallest voxel index -- its first voxel in C-order raster scan.
 // Numbering components by the rank of their root therefore numbers them in
-// order of first appearance, the order cc3d issues labels.  Each voxel unites
-// with one representative of every 26-connected group of equal-valued
-// already-scanned neighbours (13 candidates), which removes most redundant
-// unions.  Periodic seams are united voxel-with-twin (the voxel its halo
-// copies), which is what the reference's pair matching does.
+// order of first appearance, the order cc3d issues labels.  Elements of a row
+// that touch form runs, and one union is made per pair of touching runs of
+// neighbouring rows, which removes most redundant unions.  Periodic seams are
+// united voxel-with-twin (the voxel its halo copies), which is what the
+// reference's pair matching does.
 //
 // Every data-dependent loop carries an iteration cap; hitting it sets a
 // device status word and the entry point returns PMG_EITER.
@@ -39,43 +39,16 @@ struct Vol3 {
     long long s0, s1, s2;
 };
 
-// The 13 already-scanned neighbours (C order) and their mutual 26-adjacency.
-__constant__ int c_nb[13][3];
-__constant__ unsigned short c_adj[13];
-
-static void host_tables(int nb[13][3], unsigned short adj[13])
-{
-    int n = 0;
-    for (int di = -1; di <= 0; di++)
-        for (int dj = -1; dj <= 1; dj++)
-            for (int dk = -1; dk <= 1; dk++) {
-                if (di == 0 && (dj > 0 || (dj == 0 && dk >= 0)))
-                    continue;
-                nb[n][0] = di;
-                nb[n][1] = dj;
-                nb[n][2] = dk;
-                n++;
-            }
-    for (int a = 0; a < 13; a++) {
-        adj[a] = 0;
-        for (int b = 0; b < 13; b++) {
-            if (a == b)
-                continue;
-            if (abs(nb[a][0] - nb[b][0]) <= 1 && abs(nb[a][1] - nb[b][1]) <= 1 &&
-                abs(nb[a][2] - nb[b][2]) <= 1)
-                adj[a] |= (unsigned short)(1u << b);
-        }
-    }
-}
-
 // ---- tiled labelling ------------------------------------------------------
-// Tiles of 4 x 8 x 32 voxels (C order, the last axis contiguous), one thread
-// per voxel.  Phase 1 unites equal neighbours inside the tile with a shared-
-// memory union-find whose roots are the smallest local index -- which is also
-// the smallest global index of that part of the component, because C order
-// inside a box follows the global C order.  Phase 2 unites neighbours that lie
-// in other tiles through the global parents.  Both phases use one
-// representative per 26-connected group of equal earlier neighbours.
+// Tiles of 4 x 8 x 32 elements (C order, the last axis contiguous; voxels here,
+// 2x2x2 blocks below), 32 rows of 32, one warp per row in the first phase.
+// Phase 1 unites the parts of a tile with a shared-memory union-find whose
+// roots are the smallest local index -- which is also the smallest global
+// index of that part of the component, because C order inside a box follows
+// the global C order.  Phase 2 unites across tile borders through the global
+// parents.  Both work on runs: touching neighbours of a row share the run's
+// first element (the head) as parent, and of the touching pairs of two
+// neighbouring rows one per pair of runs is united.
 constexpr int kT0 = 4, kT1 = 8, kT2 = 32, kTile = kT0 * kT1 * kT2;
 
 __device__ __forceinline__ int sfind(const int *L, int x)
@@ -126,132 +99,250 @@ __device__ __forceinline__ void sunite(int *L, int a, int b)
     }
 }
 
-// adj: shared-memory copy of c_adj (lanes index it with different values,
-// which constant memory would serialise)
-__device__ __forceinline__ unsigned cover_group(unsigned q_mask, unsigned same, const unsigned short *adj)
+// first element of the run of element c; cz: elements joined to the one before
+__device__ __forceinline__ int run_head(unsigned cz, int c) { return 31 - __clz(~cz & (0xffffffffu >> (31 - c))); }
+
+// neighbouring row q = 0..3: (-1, 0), (-1, -1), (-1, 1), (0, -1)
+__device__ __forceinline__ int row_d0(int q) { return q < 3 ? -1 : 0; }
+__device__ __forceinline__ int row_d1(int q) { return q == 0 ? 0 : q == 2 ? 1 : -1; }
+
+// Of the touching pairs of a row's elements with the ones before (em), beside
+// (e0) and after (ep) them in a neighbouring row, one per pair of runs: cz, bz
+// are the runs of the row and of its neighbour.  A straight pair is dropped
+// when the element before makes one between the same two runs, a slanted one
+// when a straight one does.
+__device__ __forceinline__ void row_reduce(unsigned cz, unsigned bz, unsigned &em, unsigned &e0, unsigned &ep)
 {
-    unsigned grp = q_mask, prev = 0;
-    while (grp != prev) {
-        prev = grp;
-        unsigned g = grp;
-        while (g) {
-            const int w = __ffs(g) - 1;
-            g &= g - 1;
-            grp |= adj[w] & same;
-        }
+    const unsigned s0 = e0;
+    e0 &= ~(cz & (s0 << 1) & bz);
+    em &= ~((s0 & bz) | (cz & (s0 << 1)));
+    ep &= ~((s0 & (bz >> 1)) | ((cz >> 1) & (s0 >> 1)));
+}
+
+// Row pairs across a tile's borders: the a = 0 plane's rows with the three rows
+// above, then the rows before b = 0, then the slanted ones of the other planes.
+constexpr int kCrossPairs = kT1 * 3 + kT0 + (kT0 - 1) * 2;
+
+__device__ __forceinline__ void cross_pair(int i, int &a, int &b, int &q)
+{
+    if (i < kT1 * 3) {
+        a = 0;
+        b = i / 3;
+        q = i % 3;
+    } else if (i < kT1 * 3 + kT0) {
+        a = i - kT1 * 3;
+        b = 0;
+        q = 3;
+    } else {
+        const int k = i - kT1 * 3 - kT0;
+        a = 1 + k / 2;
+        b = (k & 1) * (kT1 - 1);
+        q = 1 + (k & 1);
     }
-    return grp;
 }
 
-__device__ __forceinline__ void load_adj(unsigned short *s_adj)
-{
-    if (threadIdx.x < 13)
-        s_adj[threadIdx.x] = c_adj[threadIdx.x];
-}
+// Unions across a tile's borders.  Phase 1 left every element's tile-local root
+// in P, so two touching elements stand for a pair of tile-local components: a
+// shared-memory set of the pairs seen keeps all but the first of each pair
+// from the global union-find (a tile has a few components, and hundreds of
+// touching pairs).  Pairs are listed and then taken by all threads of the
+// block: a thread's own would run one after the other, each a chain of
+// dependent loads.
+constexpr int kPairSlots = 256, kPairProbes = 8, kPairList = 768;
 
+struct CrossSet {
+    unsigned long long set[kPairSlots];
+    int2 list[kPairList];
+    int count;
+
+    __device__ __forceinline__ void init()
+    {
+        for (int q = threadIdx.x; q < kPairSlots; q += blockDim.x)
+            set[q] = ~0ull;
+        if (threadIdx.x == 0)
+            count = 0;
+        __syncthreads();
+    }
+    // True when this pair has been seen in the block (its union is done by
+    // another thread); a full set lets pairs through.
+    __device__ __forceinline__ bool seen(int pa, int pb)
+    {
+        const unsigned long long key = ((unsigned long long)(unsigned)pa << 32) | (unsigned)pb;
+        unsigned h = ((unsigned)pa * 2654435761u) ^ ((unsigned)pb * 2246822519u);
+        h = (h ^ (h >> 15)) % kPairSlots;
+        for (int i = 0; i < kPairProbes; i++) {
+            const unsigned long long old = atomicCAS(set + h, ~0ull, key);
+            if (old == ~0ull)
+                return false;
+            if (old == key)
+                return true;
+            h = (h + 1) % kPairSlots;
+        }
+        return false;
+    }
+    __device__ __forceinline__ void join(int *P, int x, int y, int *err)
+    {
+        const int px = ld(P + x), py = ld(P + y);
+        if (px != py && !seen(px, py))
+            unite(P, px, py, err);
+    }
+    __device__ __forceinline__ void add(int *P, int x, int y, int *err)
+    {
+        const int k = atomicAdd(&count, 1);
+        if (k < kPairList)
+            list[k] = make_int2(x, y);
+        else
+            join(P, x, y, err);
+    }
+    // after every add of the block
+    __device__ __forceinline__ void finish(int *P, int *err)
+    {
+        __syncthreads();
+        const int total = min(count, kPairList);
+        for (int k = threadIdx.x; k < total; k += blockDim.x)
+            join(P, list[k].x, list[k].y, err);
+    }
+};
+
+// Grid of the tile kernels: tiles (x along the contiguous axis).
+struct TileId {
+    int ti, tj, tk, nt1, nt2;
+    __device__ __forceinline__ TileId()
+        : ti(blockIdx.z), tj(blockIdx.y), tk(blockIdx.x), nt1(gridDim.y), nt2(gridDim.x)
+    {
+    }
+    __device__ __forceinline__ int index() const { return (ti * nt1 + tj) * nt2 + tk; }
+};
+
+// Phase 1 on voxels (equal nonzero neighbours touch).  A voxel equal to the one
+// above it leaves its other earlier neighbours to that one: it is adjacent to
+// all of them.
 template <typename T>
 __global__ void __launch_bounds__(kTile) k_cc_tile(const T *__restrict__ img, int *__restrict__ P, Vol3 V)
 {
     __shared__ T sv[kTile];
     __shared__ int L[kTile];
-    __shared__ unsigned short s_adj[13];
-    load_adj(s_adj);
-    const int nt1 = (int)((V.s1 + kT1 - 1) / kT1), nt2 = (int)((V.s2 + kT2 - 1) / kT2);
-    const long long tile = blockIdx.x;
-    const long long ti = tile / ((long long)nt1 * nt2);
-    const int tj = (int)((tile / nt2) % nt1), tk = (int)(tile % nt2);
-    const int t = threadIdx.x;
-    const int a = t / (kT1 * kT2), b = (t / kT2) % kT1, c = t % kT2;
-    const long long i = ti * kT0 + a, j = (long long)tj * kT1 + b, k = (long long)tk * kT2 + c;
+    __shared__ unsigned s_cz[kT0 * kT1];
+    const TileId D;
+    const int t = threadIdx.x, r = t / kT2, lane = t % kT2, a = r / kT1, b = r % kT1;
+    const int i = D.ti * kT0 + a, j = D.tj * kT1 + b, k = D.tk * kT2 + lane;
     const bool inside = i < V.s0 && j < V.s1 && k < V.s2;
-    const long long g = (i * V.s1 + j) * V.s2 + k;
+    const long long g = ((long long)i * V.s1 + j) * V.s2 + k;
     const T v = inside ? img[g] : (T)0;
     sv[t] = v;
-    L[t] = v != 0 ? t : -1;
+    const T vp = __shfl_up_sync(0xffffffffu, v, 1);
+    const unsigned cz = __ballot_sync(0xffffffffu, lane > 0 && v != 0 && v == vp);
+    const int head = run_head(cz, lane);
+    L[t] = v != 0 ? r * kT2 + head : -1;
+    if (lane == 0)
+        s_cz[r] = cz;
     __syncthreads();
-    if (v != 0) {
-        unsigned same = 0;
+    if (__any_sync(0xffffffffu, v != 0)) {
+        // pairs as bits 3 q + dz + 1
+        unsigned todo = 0;
+        bool centre = false;
 #pragma unroll
-        for (int q = 0; q < 13; q++) {
-            const int aa = a + c_nb[q][0], bb = b + c_nb[q][1], cc = c + c_nb[q][2];
-            if (aa < 0 || bb < 0 || bb >= kT1 || cc < 0 || cc >= kT2)
+        for (int q = 0; q < 4; q++) {
+            if (a + row_d0(q) < 0 || b + row_d1(q) < 0 || b + row_d1(q) >= kT1)
                 continue;
-            if (sv[(aa * kT1 + bb) * kT2 + cc] == v)
-                same |= 1u << q;
+            const int rn = r + row_d0(q) * kT1 + row_d1(q);
+            const T n0 = sv[rn * kT2 + lane], nm = __shfl_up_sync(0xffffffffu, n0, 1),
+                    np = __shfl_down_sync(0xffffffffu, n0, 1);
+            const bool on = v != 0 && !centre;
+            unsigned E0 = __ballot_sync(0xffffffffu, on && n0 == v),
+                     Em = __ballot_sync(0xffffffffu, on && lane > 0 && nm == v),
+                     Ep = __ballot_sync(0xffffffffu, on && lane < 31 && np == v);
+            if (q == 0)
+                centre = (E0 >> lane) & 1u;
+            row_reduce(cz, s_cz[rn], Em, E0, Ep);
+            todo |= (((Em >> lane) & 1u) | (((E0 >> lane) & 1u) << 1) | (((Ep >> lane) & 1u) << 2)) << (3 * q);
         }
-        unsigned covered = 0;
-        while (same & ~covered) {
-            const int q = __ffs(same & ~covered) - 1;
-            sunite(L, t, ((a + c_nb[q][0]) * kT1 + b + c_nb[q][1]) * kT2 + c + c_nb[q][2]);
-            covered |= cover_group(1u << q, same, s_adj);
+        while (todo) {
+            const int e = __ffs(todo) - 1, q = e / 3, dz = e - 3 * q - 1;
+            todo &= todo - 1;
+            const int rn = r + row_d0(q) * kT1 + row_d1(q);
+            sunite(L, r * kT2 + head, rn * kT2 + run_head(s_cz[rn], lane + dz));
         }
     }
     __syncthreads();
-    if (v != 0)
-        L[t] = sfind(L, t);
-    __syncthreads();
+    int root = -1;
+    if (v != 0 && head == lane)
+        root = sfind(L, t);
+    root = __shfl_sync(0xffffffffu, root, head);
     if (inside) {
         int out = -1;
         if (v != 0) {
-            const int r = L[t];
-            const int ra = r / (kT1 * kT2), rb = (r / kT2) % kT1, rc = r % kT2;
-            out = (int)(((ti * kT0 + ra) * V.s1 + (long long)tj * kT1 + rb) * V.s2 + (long long)tk * kT2 + rc);
+            const int ra = root / (kT1 * kT2), rb = (root / kT2) % kT1, rc = root % kT2;
+            out = (int)(((long long)(D.ti * kT0 + ra) * V.s1 + D.tj * kT1 + rb) * V.s2 + D.tk * kT2 + rc);
         }
         P[g] = out;
     }
 }
 
-// Phase 2: unions with equal earlier neighbours in other tiles.  Neighbours in
-// the voxel's own tile (and everything 26-connected to them among the equal
-// neighbours) are already united by phase 1.
+// Phase 2 on voxels: a warp per row pair in different tiles, then a thread per
+// row end (slanted neighbours, and straight ones at the low end, lie in the
+// tiles beside).
+constexpr int kCcCrossThreads = 256;
+
 template <typename T>
-__global__ void k_cc_cross(const T *__restrict__ img, int *P, Vol3 V, int *err)
+__global__ void __launch_bounds__(kCcCrossThreads) k_cc_cross(const T *__restrict__ img, int *P, Vol3 V, int *err)
 {
-    __shared__ unsigned short s_adj[13];
-    load_adj(s_adj);
-    __syncthreads();
+    __shared__ CrossSet S;
+    const TileId D;
+    S.init();
     // volumes are below 2^31 voxels, so 32-bit index arithmetic suffices
-    const int n = (int)(V.s0 * V.s1 * V.s2);
-    const int S1 = (int)V.s1, S2 = (int)V.s2;
-    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
-        const int r = idx / S2;
-        const int k = idx - r * S2;
-        const int i = r / S1;
-        const int j = r - i * S1;
-        const int a = i & (kT0 - 1), b = j & (kT1 - 1), c = k & (kT2 - 1);
-        if (a > 0 && b > 0 && b < kT1 - 1 && c > 0 && c < kT2 - 1)
-            continue; // every earlier neighbour is inside the tile
-        const T v = img[idx];
-        if (v == 0)
+    const int S0 = (int)V.s0, S1 = (int)V.s1, S2 = (int)V.s2;
+    const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
+    for (int pi = w; pi < kCrossPairs; pi += kCcCrossThreads / 32) {
+        int a, b, q;
+        cross_pair(pi, a, b, q);
+        const int i = D.ti * kT0 + a, j = D.tj * kT1 + b, k = D.tk * kT2 + lane, ni = i + row_d0(q),
+                  nj = j + row_d1(q);
+        if (i >= S0 || j >= S1 || ni < 0 || nj < 0 || nj >= S1)
             continue;
-        unsigned same = 0, local = 0;
+        const int x = (i * S1 + j) * S2 + k, y = (ni * S1 + nj) * S2 + k;
+        const T v = k < S2 ? img[x] : (T)0, n0 = k < S2 ? img[y] : (T)0;
+        const T vp = __shfl_up_sync(0xffffffffu, v, 1);
+        T nm = __shfl_up_sync(0xffffffffu, n0, 1), np = __shfl_down_sync(0xffffffffu, n0, 1);
+        const unsigned cz = __ballot_sync(0xffffffffu, lane > 0 && v != 0 && v == vp),
+                       bz = __ballot_sync(0xffffffffu, lane > 0 && n0 != 0 && n0 == nm);
+        if (lane == 0)
+            nm = k > 0 ? img[y - 1] : (T)0;
+        if (lane == 31)
+            np = k + 1 < S2 ? img[y + 1] : (T)0;
+        unsigned E0 = __ballot_sync(0xffffffffu, v != 0 && n0 == v), Em = __ballot_sync(0xffffffffu, v != 0 && nm == v),
+                 Ep = __ballot_sync(0xffffffffu, v != 0 && np == v);
+        row_reduce(cz, bz, Em, E0, Ep);
+        if ((E0 >> lane) & 1u)
+            S.add(P, x, y, err);
+        if ((Em >> lane) & 1u)
+            S.add(P, x, y - 1, err);
+        if ((Ep >> lane) & 1u)
+            S.add(P, x, y + 1, err);
+    }
+    if (threadIdx.x < kT0 * kT1 * 2) {
+        const int r = threadIdx.x >> 1, a = r / kT1, b = r % kT1;
+        const bool low = !(threadIdx.x & 1);
+        const int dz = low ? -1 : 1;
+        const int i = D.ti * kT0 + a, j = D.tj * kT1 + b, k = D.tk * kT2 + (low ? 0 : kT2 - 1);
+        if (i < S0 && j < S1 && k < S2 && k + dz >= 0 && k + dz < S2) {
+            const int x = (i * S1 + j) * S2 + k;
+            const T v = img[x];
+            if (v != 0) {
+                if (low && img[x - 1] == v)
+                    S.add(P, x, x - 1, err);
 #pragma unroll
-        for (int q = 0; q < 13; q++) {
-            const int ai = i + c_nb[q][0], bj = j + c_nb[q][1], ck = k + c_nb[q][2];
-            if (ai < 0 || bj < 0 || ck < 0 || bj >= S1 || ck >= S2)
-                continue;
-            if (img[(ai * S1 + bj) * S2 + ck] != v)
-                continue;
-            same |= 1u << q;
-            const int aa = a + c_nb[q][0], bb = b + c_nb[q][1], cc = c + c_nb[q][2];
-            if (aa >= 0 && bb >= 0 && bb < kT1 && cc >= 0 && cc < kT2)
-                local |= 1u << q;
-        }
-        unsigned covered = 0;
-        unsigned lm = local;
-        while (lm) { // groups reached through in-tile neighbours are done
-            const int q = __ffs(lm) - 1;
-            const unsigned grp = cover_group(1u << q, same, s_adj);
-            covered |= grp;
-            lm &= ~grp;
-        }
-        while (same & ~covered) {
-            const int q = __ffs(same & ~covered) - 1;
-            const int ai = i + c_nb[q][0], bj = j + c_nb[q][1], ck = k + c_nb[q][2];
-            unite(P, idx, (ai * S1 + bj) * S2 + ck, err);
-            covered |= cover_group(1u << q, same, s_adj);
+                for (int q = 0; q < 4; q++) {
+                    if (a + row_d0(q) < 0 || b + row_d1(q) < 0 || b + row_d1(q) >= kT1 || j + row_d1(q) >= S1)
+                        continue; // (a row pair's, or outside)
+                    const int y = x + (row_d0(q) * S1 + row_d1(q)) * S2 + dz;
+                    if (img[y] == v)
+                        S.add(P, x, y, err);
+                }
+            }
         }
     }
+    S.finish(P, err);
 }
 
 // Seam twins of the voxel labelling (see Twins).
@@ -293,12 +384,25 @@ __global__ void k_cc_twins(const T *__restrict__ img, int *P, Twins W, int *err)
     }
 }
 
-__global__ void k_cc_flatten(int *P, long long n, int *err)
+// Four voxels per thread: their chains of dependent loads overlap.
+__global__ void __launch_bounds__(256) k_cc_flatten(int *P, long long n, int *err)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (int)n; i += gridDim.x * blockDim.x) {
-        const int p = P[i];
-        if (p >= 0 && p != i)
-            P[i] = find_root(P, p, err);
+    constexpr int NB = 4;
+    for (long long base = (long long)blockIdx.x * blockDim.x * NB; base < n;
+         base += (long long)gridDim.x * blockDim.x * NB) {
+        int p[NB], g[NB];
+#pragma unroll
+        for (int q = 0; q < NB; q++) {
+            const long long i = base + q * blockDim.x + threadIdx.x;
+            p[q] = i < n ? ld(P + i) : -1;
+        }
+#pragma unroll
+        for (int q = 0; q < NB; q++)
+            g[q] = p[q] >= 0 ? ld(P + p[q]) : -1;
+#pragma unroll
+        for (int q = 0; q < NB; q++)
+            if (g[q] != p[q])
+                P[base + q * blockDim.x + threadIdx.x] = find_root(P, g[q], err);
     }
 }
 
@@ -486,44 +590,25 @@ __global__ void k_select(const uint8_t *__restrict__ img, const int *__restrict_
 }
 
 // ---------------------------------------------------------------------------
-static bool g_tables_ready[64] = {false};
-
-static int ensure_tables()
-{
-    int dev = 0;
-    PMG_CUDA(cudaGetDevice(&dev));
-    if (dev >= 0 && dev < 64 && g_tables_ready[dev])
-        return PMG_OK;
-    int nb[13][3];
-    unsigned short adj[13];
-    host_tables(nb, adj);
-    PMG_CUDA(cudaMemcpyToSymbol(c_nb, nb, sizeof(nb)));
-    PMG_CUDA(cudaMemcpyToSymbol(c_adj, adj, sizeof(adj)));
-    if (dev >= 0 && dev < 64)
-        g_tables_ready[dev] = true;
-    return PMG_OK;
-}
-
 // Union-find of a volume into P (roots = smallest index); twins optional.
 template <typename T>
 static int uf_build(const T *img, int *P, const int64_t *shape, const int32_t *bc,
                     const int32_t *pad, bool twins, int *err, cudaStream_t st)
 {
-    PMG_TRY(ensure_tables());
     const long long n = shape[0] * shape[1] * shape[2];
     Vol3 V{shape[0], shape[1], shape[2]};
     const int block = 256;
-    const long long tiles = ((shape[0] + kT0 - 1) / kT0) * ((shape[1] + kT1 - 1) / kT1) *
-                            ((shape[2] + kT2 - 1) / kT2);
+    const dim3 tiles((unsigned)((shape[2] + kT2 - 1) / kT2), (unsigned)((shape[1] + kT1 - 1) / kT1),
+                     (unsigned)((shape[0] + kT0 - 1) / kT0));
     {
         const int ps__ = prof_begin("k_cc_tile", st);
-        k_cc_tile<T><<<(unsigned)tiles, kTile, 0, st>>>(img, P, V);
+        k_cc_tile<T><<<tiles, kTile, 0, st>>>(img, P, V);
         prof_end(ps__, (double)n * (sizeof(T) + 4), st);
     }
     PMG_CHECK_LAUNCH();
     {
         const int ps__ = prof_begin("k_cc_cross", st);
-        k_cc_cross<T><<<grid_for(n, block, 152LL * 32), block, 0, st>>>(img, P, V, err);
+        k_cc_cross<T><<<tiles, kCcCrossThreads, 0, st>>>(img, P, V, err);
         prof_end(ps__, 0.0, st);
     }
     PMG_CHECK_LAUNCH();
@@ -538,7 +623,7 @@ static int uf_build(const T *img, int *P, const int64_t *shape, const int32_t *b
     }
     {
         const int ps__ = prof_begin("k_cc_flatten", st);
-        k_cc_flatten<<<grid_for(n, block, 152LL * 32), block, 0, st>>>(P, n, err);
+        k_cc_flatten<<<grid_for((n + 3) / 4, block, 152LL * 32), block, 0, st>>>(P, n, err);
         prof_end(ps__, (double)n * 8, st);
     }
     PMG_CHECK_LAUNCH();
@@ -748,6 +833,9 @@ static int seam_keys_batched(const Src &src, const std::vector<SeamFeature> &fs,
         prof_end(ps__, (double)T * 28, st);
     }
     PMG_CHECK_LAUNCH();
+    // rows that repeat the key of the row before cannot be a first row: they go
+    // before the sort (labels change rarely along a seam; 12.6 M rows of a
+    // 1024^3 field took the sort 0.7 ms)
     const int nbits = 2 * lbits + 5;
     size_t tb = 0, tb2 = 0, tb3 = 0;
     PMG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, d_k, d_k2, d_i, d_i2, (int)T, 0, nbits, st));
@@ -756,22 +844,30 @@ static int seam_keys_batched(const Src &src, const std::vector<SeamFeature> &fs,
     size_t tbs = std::max(tb, std::max(tb2, tb3));
     void *d_t = nullptr;
     PMG_TRY(scratch_alloc(&d_t, tbs, st));
-    PMG_CUDA(cub::DeviceRadixSort::SortPairs(d_t, tbs, d_k, d_k2, d_i, d_i2, (int)T, 0, nbits, st));
-    {
+    auto heads = [&](const uint64_t *k, long long rows) -> int {
         const int ps__ = prof_begin("k_head_flags", st);
-        k_head_flags<<<grid_for(T, 256, 1LL << 30), 256, 0, st>>>(d_k2, T, d_f);
-        prof_end(ps__, (double)T * 9, st);
-    }
-    PMG_CHECK_LAUNCH();
-    PMG_CUDA(cub::DeviceSelect::Flagged(d_t, tbs, d_i2, d_f, d_i, d_nsel, (int)T, st));
-    PMG_CUDA(cub::DeviceSelect::Flagged(d_t, tbs, d_k2, d_f, d_k3, d_nsel + 1, (int)T, st));
+        k_head_flags<<<grid_for(rows, 256, 1LL << 30), 256, 0, st>>>(k, rows, d_f);
+        prof_end(ps__, (double)rows * 9, st);
+        PMG_CHECK_LAUNCH();
+        return PMG_OK;
+    };
+    int rows = 0;
+    PMG_TRY(heads(d_k, T));
+    PMG_CUDA(cub::DeviceSelect::Flagged(d_t, tbs, d_i, d_f, d_i2, d_nsel, (int)T, st));
+    PMG_CUDA(cub::DeviceSelect::Flagged(d_t, tbs, d_k, d_f, d_k3, d_nsel + 1, (int)T, st));
+    PMG_CUDA(cudaMemcpyAsync(&rows, d_nsel, sizeof(int), cudaMemcpyDeviceToHost, st));
+    PMG_CUDA(cudaStreamSynchronize(st));
+    PMG_CUDA(cub::DeviceRadixSort::SortPairs(d_t, tbs, d_k3, d_k2, d_i2, d_i, rows, 0, nbits, st));
+    PMG_TRY(heads(d_k2, rows));
+    PMG_CUDA(cub::DeviceSelect::Flagged(d_t, tbs, d_i, d_f, d_i2, d_nsel, rows, st));
+    PMG_CUDA(cub::DeviceSelect::Flagged(d_t, tbs, d_k2, d_f, d_k3, d_nsel + 1, rows, st));
     int nsel = 0;
     PMG_CUDA(cudaMemcpyAsync(&nsel, d_nsel, sizeof(int), cudaMemcpyDeviceToHost, st));
     PMG_CUDA(cudaStreamSynchronize(st));
     std::vector<uint32_t> first((size_t)nsel);
     std::vector<uint64_t> dkeys((size_t)nsel);
     if (nsel > 0) {
-        PMG_CUDA(cudaMemcpyAsync(first.data(), d_i, (size_t)nsel * 4, cudaMemcpyDeviceToHost, st));
+        PMG_CUDA(cudaMemcpyAsync(first.data(), d_i2, (size_t)nsel * 4, cudaMemcpyDeviceToHost, st));
         PMG_CUDA(cudaMemcpyAsync(dkeys.data(), d_k3, (size_t)nsel * 8, cudaMemcpyDeviceToHost, st));
     }
     PMG_CUDA(cudaStreamSynchronize(st));
@@ -1146,111 +1242,13 @@ struct BGrid {
     }
 };
 
-__device__ __forceinline__ bool fg_of(uint8_t v, int fgval) { return fgval >= 0 ? v == fgval : v != 0; }
-
-// touching voxels of a block for neighbour offset (d0, d1, d2): bit (x*2+y)*2+z
-__host__ __device__ inline unsigned touch_mask(int d0, int d1, int d2)
-{
-    unsigned m = 0;
-    for (int x = 0; x < 2; x++)
-        for (int y = 0; y < 2; y++)
-            for (int z = 0; z < 2; z++) {
-                if ((d0 == -1 && x != 0) || (d0 == 1 && x != 1))
-                    continue;
-                if ((d1 == -1 && y != 0) || (d1 == 1 && y != 1))
-                    continue;
-                if ((d2 == -1 && z != 0) || (d2 == 1 && z != 1))
-                    continue;
-                m |= 1u << ((x * 2 + y) * 2 + z);
-            }
-    return m;
-}
-
-// Touch masks of the 13 earlier neighbours: voxels of a block that touch
-// neighbour q, voxels of neighbour q that touch the block, and voxels of
-// neighbour r that touch neighbour q (0 when r and q are not adjacent).
-__constant__ uint8_t c_bt_self[13];
-__constant__ uint8_t c_bt_nb[13];
-__constant__ uint8_t c_bt_pair[13][13];
-// all 26 neighbours: offsets, voxels of a block touching neighbour q, voxels of
-// neighbour q touching the block
-__constant__ signed char c_g_d[26][3];
-__constant__ uint8_t c_g_self[26];
-__constant__ uint8_t c_g_nb[26];
-
-__device__ __forceinline__ unsigned bmask_of(int q, uint64_t mlo, uint64_t mhi)
-{
-    return (unsigned)((q < 8 ? mlo >> (8 * q) : mhi >> (8 * (q - 8))) & 0xffu);
-}
-
-struct BTabs {
-    unsigned short adj[13];
-    uint8_t pair[13][13];
-};
-
-__device__ __forceinline__ void load_btabs(BTabs &tb)
-{
-    if (threadIdx.x < 13)
-        tb.adj[threadIdx.x] = c_adj[threadIdx.x];
-    for (int q = threadIdx.x; q < 169; q += blockDim.x)
-        tb.pair[q / 13][q % 13] = c_bt_pair[q / 13][q % 13];
-}
-
-// Neighbours in `conn` that touch neighbour w (one step), w included: a union
-// with w links them too, because the union of each touching pair is done by
-// the later block of the pair.
-__device__ __forceinline__ unsigned bcover1(int w, unsigned conn, uint64_t mlo, uint64_t mhi, const BTabs &tb)
-{
-    unsigned grp = 1u << w;
-    const unsigned mw = bmask_of(w, mlo, mhi);
-    unsigned cand = tb.adj[w] & conn;
-    while (cand) {
-        const int u = __ffs(cand) - 1;
-        cand &= cand - 1;
-        if ((mw & tb.pair[w][u]) && (bmask_of(u, mlo, mhi) & tb.pair[u][w]))
-            grp |= 1u << u;
-    }
-    return grp;
-}
-
-// Everything in `conn` connected to neighbour w through chains of touching
-// neighbours (the closure of bcover1): worth its cost where a union is a
-// global-memory atomic.
-__device__ __forceinline__ unsigned bcover(int w, unsigned conn, uint64_t mlo, uint64_t mhi, const BTabs &tb)
-{
-    unsigned grp = 1u << w, frontier = 1u << w;
-    while (frontier) {
-        const int v = __ffs(frontier) - 1;
-        frontier &= frontier - 1;
-        const unsigned add = bcover1(v, conn & ~grp, mlo, mhi, tb) & ~grp;
-        grp |= add;
-        frontier |= add;
-    }
-    return grp;
-}
-
-// Neighbour (-1, 0, 0) (index 4 in c_nb order) is 26-adjacent to all twelve
-// other earlier neighbours, so it is taken first: in a dense region one union
-// with it covers every other one.
-constexpr int kCentre = 4;
-
-__device__ __forceinline__ int next_cover(unsigned rest)
-{
-    return ((rest >> kCentre) & 1u) ? kCentre : __ffs(rest) - 1;
-}
-
 // Foreground of the block selection: the voxels of one value (or nonzero)
 // of a uint8 image ...
 struct SrcImg {
     const uint8_t *img;
     int fgval;
-    __device__ __forceinline__ bool fg(long long idx, int, int, int) const { return fg_of(img[idx], fgval); }
-    // voxels idx and idx + 1 (idx even) with one 16-bit load: bit 0, bit 1
-    __device__ __forceinline__ unsigned fg2(long long idx, int, int, int) const
-    {
-        const unsigned v = *(const uint16_t *)(img + idx);
-        return (unsigned)fg_of((uint8_t)v, fgval) | ((unsigned)fg_of((uint8_t)(v >> 8), fgval) << 1);
-    }
+    // range (optional): OR and AND of the nonzero values seen by the tile pass
+    unsigned *range = nullptr;
 };
 
 // ... or an erosion read off a capped squared EDT: voxels with E > T stay,
@@ -1330,17 +1328,73 @@ __device__ __forceinline__ unsigned block_mask(const Src &src, const BGrid &G, i
     return m;
 }
 
+// bytes != 0 -> 0x01 per byte
+__device__ __forceinline__ unsigned nonzero01(unsigned v)
+{
+    return ((((v & 0x7f7f7f7fu) + 0x7f7f7f7fu) | v) >> 7) & 0x01010101u;
+}
+
+// The same of an image, its eight bytes in two words; they stay in w for the
+// caller (0 outside the volume).
+__device__ __forceinline__ unsigned block_mask(const SrcImg &src, const BGrid &G, int c0, int c1, int c2,
+                                               unsigned (&w)[2])
+{
+    const long long sy = G.s2, sx = (long long)G.s1 * G.s2;
+    const uint8_t *p = src.img + (2LL * c0 * G.s1 + 2 * c1) * sy + 2 * c2;
+    unsigned vol = 0xffu;
+    if (2 * c0 + 1 < G.s0 && 2 * c1 + 1 < G.s1 && 2 * c2 + 1 < G.s2 && !(G.s2 & 1)) {
+        // even rows: every voxel pair (z = 0, 1) starts on an even index
+#pragma unroll
+        for (int x = 0; x < 2; x++)
+            w[x] = (unsigned)*(const uint16_t *)(p + x * sx) | ((unsigned)*(const uint16_t *)(p + x * sx + sy) << 16);
+    } else {
+        vol = 0;
+        w[0] = w[1] = 0;
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            const int x = q >> 2, y = (q >> 1) & 1, z = q & 1;
+            if (2 * c0 + x < G.s0 && 2 * c1 + y < G.s1 && 2 * c2 + z < G.s2) {
+                w[x] |= (unsigned)p[x * sx + y * sy + z] << (8 * (q & 3));
+                vol |= 1u << q;
+            }
+        }
+    }
+    const unsigned pat = src.fgval >= 0 ? (unsigned)src.fgval * 0x01010101u : 0u;
+    unsigned a = nonzero01(w[0] ^ pat), b = nonzero01(w[1] ^ pat);
+    a = (a | (a >> 7) | (a >> 14) | (a >> 21)) & 0xfu;
+    b = (b | (b >> 7) | (b >> 14) | (b >> 21)) & 0xfu;
+    const unsigned m = a | (b << 4);
+    return (src.fgval >= 0 ? ~m : m) & vol;
+}
+
+__device__ __forceinline__ unsigned block_mask(const SrcImg &src, const BGrid &G, int c0, int c1, int c2)
+{
+    unsigned w[2];
+    return block_mask(src, G, c0, c1, c2, w);
+}
+
+// OR and AND of the nonzero bytes of w, over the warp, added to src.range.
+__device__ __forceinline__ void note_range(const SrcImg &src, const unsigned (&w)[2])
+{
+    const unsigned z0 = (nonzero01(w[0]) ^ 0x01010101u) * 0xffu, z1 = (nonzero01(w[1]) ^ 0x01010101u) * 0xffu;
+    unsigned o = w[0] | w[1], a = (w[0] | z0) & (w[1] | z1);
+    o |= o >> 16;
+    a &= a >> 16;
+    o = __reduce_or_sync(0xffffffffu, (o | (o >> 8)) & 0xffu);
+    a = __reduce_and_sync(0xffffffffu, (a & (a >> 8)) & 0xffu);
+    if ((threadIdx.x & 31) == 0 && o) {
+        // (values already seen cost a load)
+        if (o & ~*(volatile unsigned *)src.range)
+            atomicOr(src.range, o);
+        if (~a & 0xffu & *(volatile unsigned *)(src.range + 1))
+            atomicAnd(src.range + 1, a);
+    }
+}
+
 __device__ __forceinline__ unsigned block_mask(const SrcMask &src, const BGrid &G, int c0, int c1, int c2)
 {
     return src.M[((long long)c0 * G.b1 + c1) * G.b2 + c2];
 }
-
-// The 13 earlier neighbours in the order of c_nb, as arithmetic of the index
-// (constants once a loop over q is unrolled): (-1, q / 3 - 1, q % 3 - 1) for
-// q < 9, (0, -1, q - 10) for q < 12, (0, 0, -1) for q = 12.
-__device__ __forceinline__ int nb_d0(int q) { return q < 9 ? -1 : 0; }
-__device__ __forceinline__ int nb_d1(int q) { return q < 9 ? q / 3 - 1 : (q < 12 ? -1 : 0); }
-__device__ __forceinline__ int nb_d2(int q) { return q < 9 ? q % 3 - 1 : (q < 12 ? q - 10 : -1); }
 
 // Voxels of a block that touch its neighbour at offset (d0, d1, d2): bit
 // (x * 2 + y) * 2 + z, x on the d0 side and so on.
@@ -1352,410 +1406,240 @@ __device__ __forceinline__ unsigned touch_bits(int d0, int d1, int d2)
     return X & Y & Z;
 }
 
-// Phase 1 on tiles of 4 x 8 x 32 blocks (8 x 16 x 64 voxels), one thread per
-// block: block masks from the source, then a shared-memory union-find of the
+// ---- row runs -------------------------------------------------------------------
+// A tile of 4 x 8 x 32 blocks (8 x 16 x 64 voxels) has 32 rows of 32 blocks along
+// the contiguous axis.  A row's masks are kept as eight words, bit c of word i
+// the voxel i of block c (one ballot each): touching blocks of a row form
+// runs, whose blocks share the first one (the head) as parent, and the
+// touching pairs of two neighbouring rows are a few word operations by one
+// thread, reduced to one pair per pair of runs before any union.  With a
+// block per thread that tested its 13 earlier neighbours and united with a
+// cover of them, the two phases were bound by instruction issue (512^3 pack:
+// 0.50 and 0.28 ms).
+
+struct RowBits {
+    unsigned v[8];
+    __device__ __forceinline__ unsigned zlo() const { return v[0] | v[2] | v[4] | v[6]; }
+    __device__ __forceinline__ unsigned zhi() const { return v[1] | v[3] | v[5] | v[7]; }
+    // blocks that touch the block before them
+    __device__ __forceinline__ unsigned runs() const { return zlo() & (zhi() << 1); }
+    __device__ __forceinline__ unsigned full() const
+    {
+        return v[0] & v[1] & v[2] & v[3] & v[4] & v[5] & v[6] & v[7];
+    }
+    // blocks with one of the voxels `set` among those of even (odd) index
+    __device__ __forceinline__ unsigned even(unsigned set) const
+    {
+        return (set & 1u ? v[0] : 0u) | (set & 4u ? v[2] : 0u) | (set & 16u ? v[4] : 0u) | (set & 64u ? v[6] : 0u);
+    }
+    __device__ __forceinline__ unsigned odd(unsigned set) const
+    {
+        return (set & 2u ? v[1] : 0u) | (set & 8u ? v[3] : 0u) | (set & 32u ? v[5] : 0u) | (set & 128u ? v[7] : 0u);
+    }
+};
+
+__device__ __forceinline__ RowBits row_bits(const unsigned *p) // eight words, 16-byte aligned
+{
+    const uint4 a = *reinterpret_cast<const uint4 *>(p), b = *reinterpret_cast<const uint4 *>(p + 4);
+    return RowBits{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
+}
+
+// Touching pairs of a row's blocks with the blocks before (em), beside (e0) and
+// after (ep) them in neighbouring row q; before, after: the neighbouring
+// row's pieces in the tiles beside (their bits 31 and 0 count).
+__device__ __forceinline__ void row_pairs(int q, const RowBits &own, const RowBits &nb, const RowBits *before,
+                                          const RowBits *after, unsigned &em, unsigned &e0, unsigned &ep)
+{
+    const int d0 = row_d0(q), d1 = row_d1(q);
+    const unsigned a = touch_bits(d0, d1, 0), b = touch_bits(-d0, -d1, 0);
+    const unsigned o0 = own.even(a), o1 = own.odd(a), n0 = nb.even(b), n1 = nb.odd(b);
+    e0 = (o0 | o1) & (n0 | n1);
+    em = o0 & ((n1 << 1) | (before ? before->odd(b) >> 31 : 0u));
+    ep = o1 & ((n0 >> 1) | (after ? after->even(b) << 31 : 0u));
+}
+
+// words of a block row in the bit array: eight per tile column
+__device__ __forceinline__ long long row_word(const BGrid &G, int c0, int c1, int tk, int nt2)
+{
+    return (((long long)c0 * G.b1 + c1) * nt2 + tk) * 8;
+}
+
+// Phase 1: block masks from the source, then a shared-memory union-find of the
 // tile whose roots are the smallest block index of each tile-local part.
-// Every later step reads the block masks M, never the source again.
+// Every later step reads the block masks M and their row words V, never the
+// source again.  One warp per row, lane = block; thread 4 r + q makes the
+// pairs of row r with its neighbouring row q.
 //
 // With Pl, the tile-local parents are also kept in Pl; with dirty (per tile),
 // a tile whose flag is clear has not changed since Pl was written and only
 // copies Pl to P, and every recomputed tile clears its flag.
 template <class Src>
 __global__ void __launch_bounds__(kTile, 2) k_bcc_tile(Src src, int *__restrict__ P, uint8_t *__restrict__ M,
-                                                   BGrid G, int *__restrict__ Pl, int *__restrict__ dirty)
+                                                   unsigned *__restrict__ V, BGrid G, int *__restrict__ Pl,
+                                                   int *__restrict__ dirty)
 {
-    __shared__ uint8_t sm[kTile];
     __shared__ int L[kTile];
-    __shared__ BTabs tb;
-    const int nt1 = (G.b1 + kT1 - 1) / kT1, nt2 = (G.b2 + kT2 - 1) / kT2;
-    const int tile = blockIdx.x;
-    const int ti = tile / (nt1 * nt2), tj = (tile / nt2) % nt1, tk = tile % nt2;
-    const int t = threadIdx.x;
-    const int a = t / (kT1 * kT2), b = (t / kT2) % kT1, c = t % kT2;
-    const int c0 = ti * kT0 + a, c1 = tj * kT1 + b, c2 = tk * kT2 + c;
+    __shared__ __align__(16) unsigned s_v[kT0 * kT1 * 8];
+    const TileId T;
+    const int t = threadIdx.x, r = t / kT2, lane = t % kT2; // row r = a * kT1 + b
+    const int c0 = T.ti * kT0 + r / kT1, c1 = T.tj * kT1 + r % kT1, c2 = T.tk * kT2 + lane;
     const bool inside = c0 < G.b0 && c1 < G.b1 && c2 < G.b2;
-    if (dirty && !dirty[tile]) {
-        if (inside) {
-            const int bidx = (c0 * G.b1 + c1) * G.b2 + c2;
+    const int bidx = (c0 * G.b1 + c1) * G.b2 + c2;
+    if (dirty && !dirty[T.index()]) {
+        if (inside)
             P[bidx] = Pl[bidx];
-        }
         return;
     }
-    load_btabs(tb);
-    const unsigned m = inside ? block_mask(src, G, c0, c1, c2) : 0u;
-    sm[t] = (uint8_t)m;
-    L[t] = m ? t : -1;
-    __syncthreads();
-    if (m) {
-        unsigned conn = 0;
-        uint64_t mlo = 0, mhi = 0;
-        bool full = m == 0xffu; // this block and every connected neighbour full
+    unsigned m = 0;
+    if constexpr (std::is_same<Src, SrcImg>::value) {
+        unsigned w[2] = {0u, 0u};
+        if (inside)
+            m = block_mask(src, G, c0, c1, c2, w);
+        if (src.range)
+            note_range(src, w);
+    } else if (inside) {
+        m = block_mask(src, G, c0, c1, c2);
+    }
+    RowBits row;
 #pragma unroll
-        for (int q = 0; q < 13; q++) {
-            const int aa = a + nb_d0(q), bb = b + nb_d1(q), cc = c + nb_d2(q);
-            if (aa < 0 || bb < 0 || bb >= kT1 || cc < 0 || cc >= kT2)
-                continue;
-            if (!(m & touch_bits(nb_d0(q), nb_d1(q), nb_d2(q))))
-                continue;
-            const unsigned mn = sm[(aa * kT1 + bb) * kT2 + cc];
-            if (mn & touch_bits(-nb_d0(q), -nb_d1(q), -nb_d2(q))) {
-                conn |= 1u << q;
-                full = full && mn == 0xffu;
-                if (q < 8)
-                    mlo |= (uint64_t)mn << (8 * q);
-                else
-                    mhi |= (uint64_t)mn << (8 * (q - 8));
+    for (int i = 0; i < 8; i++)
+        row.v[i] = __ballot_sync(0xffffffffu, (m >> i) & 1u);
+    const unsigned cz = row.runs();
+    const int head = run_head(cz, lane);
+    L[t] = m ? r * kT2 + head : -1;
+    if (lane < 2) {
+        const uint4 w = lane ? make_uint4(row.v[4], row.v[5], row.v[6], row.v[7])
+                             : make_uint4(row.v[0], row.v[1], row.v[2], row.v[3]);
+        reinterpret_cast<uint4 *>(s_v)[r * 2 + lane] = w;
+        if (c0 < G.b0 && c1 < G.b1)
+            reinterpret_cast<uint4 *>(V + row_word(G, c0, c1, T.tk, T.nt2))[lane] = w;
+    }
+    __syncthreads();
+    if (t < kT0 * kT1 * 4) {
+        const int rr = t >> 2, q = t & 3, a = rr / kT1, b = rr % kT1, d0 = row_d0(q), d1 = row_d1(q);
+        if (a + d0 >= 0 && b + d1 >= 0 && b + d1 < kT1) {
+            const int rn = rr + d0 * kT1 + d1;
+            const RowBits own = row_bits(s_v + rr * 8), nb = row_bits(s_v + rn * 8);
+            unsigned em, e0, ep;
+            row_pairs(q, own, nb, nullptr, nullptr, em, e0, ep);
+            if (q > 0 && a > 0) {
+                // where the block above and a further neighbour are both full,
+                // they touch each other and that union is theirs
+                const RowBits up = row_bits(s_v + (rr - kT1) * 8);
+                const unsigned centre = (own.even(0x0Fu) | own.odd(0x0Fu)) & up.full(), f = nb.full();
+                e0 &= ~(centre & f);
+                em &= ~(centre & (f << 1));
+                ep &= ~(centre & (f >> 1));
             }
-        }
-        // dense fast path: full blocks touch whenever they are 26-adjacent, and
-        // the centre neighbour is adjacent to every other one
-        unsigned covered = (full && ((conn >> kCentre) & 1u)) ? conn & ~(1u << kCentre) : 0u;
-        while (conn & ~covered) {
-            const unsigned rest = conn & ~covered;
-            const int q = next_cover(rest);
-            sunite(L, t, ((a + nb_d0(q)) * kT1 + b + nb_d1(q)) * kT2 + c + nb_d2(q));
-            covered |= bcover1(q, rest, mlo, mhi, tb);
+            const unsigned ca = own.runs(), cb = nb.runs();
+            row_reduce(ca, cb, em, e0, ep);
+            while (em | e0 | ep) {
+                const int dz = e0 ? 0 : em ? -1 : 1;
+                const unsigned e = e0 ? e0 : em ? em : ep;
+                const int c = __ffs(e) - 1;
+                const unsigned bit = e & (0u - e);
+                e0 &= ~(dz == 0 ? bit : 0u);
+                em &= ~(dz < 0 ? bit : 0u);
+                ep &= ~(dz > 0 ? bit : 0u);
+                sunite(L, rr * kT2 + run_head(ca, c), rn * kT2 + run_head(cb, c + dz));
+            }
         }
     }
     __syncthreads();
-    if (m)
-        L[t] = sfind(L, t);
-    __syncthreads();
+    int root = -1;
+    if (m && head == lane)
+        root = sfind(L, t);
+    root = __shfl_sync(0xffffffffu, root, head);
     if (inside) {
-        const int bidx = (c0 * G.b1 + c1) * G.b2 + c2;
         if constexpr (!std::is_same<Src, SrcMask>::value)
             M[bidx] = (uint8_t)m;
         int out = -1;
         if (m) {
-            const int r = L[t];
-            const int ra = r / (kT1 * kT2), rb = (r / kT2) % kT1, rc = r % kT2;
-            out = ((ti * kT0 + ra) * G.b1 + tj * kT1 + rb) * G.b2 + tk * kT2 + rc;
+            const int ra = root / (kT1 * kT2), rb = (root / kT2) % kT1, rc = root % kT2;
+            out = ((T.ti * kT0 + ra) * G.b1 + T.tj * kT1 + rb) * G.b2 + T.tk * kT2 + rc;
         }
         P[bidx] = out;
         if (Pl)
             Pl[bidx] = out;
     }
     if (dirty && t == 0)
-        dirty[tile] = 0;
+        dirty[T.index()] = 0;
 }
 
-// Phase 2: blocks on a tile border unite with touching earlier neighbours in
-// other tiles; neighbours reached through an in-tile neighbour are skipped.
-// Border blocks of a tile (the only ones with earlier neighbours in other
-// tiles), numbered densely so that every lane of a warp has one: the a = 0
-// plane (kT1 x kT2), then the b = 0 and b = kT1 - 1 rows of the other planes,
-// then the c = 0 and c = kT2 - 1 ends of the remaining rows.
-constexpr int kBorderPlane = kT1 * kT2;
-constexpr int kBorderRows = (kT0 - 1) * 2 * kT2;
-constexpr int kBorderEnds = (kT0 - 1) * (kT1 - 2) * 2;
-constexpr int kBorder = kBorderPlane + kBorderRows + kBorderEnds;
-static_assert(kBorder <= 512, "a tile's border items fit one 512-thread block");
+// Phase 2: unions across tile borders, one thread block per tile and one thread
+// per pair of rows in different tiles or per row end, whose slanted (and, at
+// the low end, straight) neighbours lie in the tiles beside.
+constexpr int kCrossThreads = 128;
+static_assert(kCrossPairs + kT0 * kT1 * 2 <= kCrossThreads, "a thread per pair and per row end");
 
-__device__ __forceinline__ void border_block(int q, int &a, int &b, int &c)
+__global__ void __launch_bounds__(kCrossThreads) k_bcc_cross(int *P, const uint8_t *__restrict__ M,
+                                                             const unsigned *__restrict__ V, BGrid G, int *err)
 {
-    if (q < kBorderPlane) {
-        a = 0;
-        b = q / kT2;
-        c = q % kT2;
-    } else if (q < kBorderPlane + kBorderRows) {
-        const int r = q - kBorderPlane;
-        a = 1 + r / (2 * kT2);
-        b = ((r / kT2) & 1) ? kT1 - 1 : 0;
-        c = r % kT2;
-    } else {
-        const int r = q - kBorderPlane - kBorderRows;
-        a = 1 + r / (2 * (kT1 - 2));
-        b = 1 + (r % (2 * (kT1 - 2))) / 2;
-        c = (r & 1) ? kT2 - 1 : 0;
-    }
-}
-
-// Touching earlier neighbours of border block (c0, c1, c2) at tile offset
-// (a, b, c): conn, those inside the tile (local), the dense flag and their
-// masks (mlo: neighbours 0-7, mhi: 8-12).
-// Touching earlier neighbours of border block bi = (c0, c1, c2) at tile
-// offset (a, b, c): conn, those inside the tile (local), the dense flag and
-// their masks (MASKS: mlo for neighbours 0-7, mhi for 8-12).  INTERIOR: all
-// 13 neighbours lie inside the volume (no bounds checks).  LAZY: in-tile
-// neighbours are read only when the block is full (their only use in the
-// cross-tile test is the dense rule).
-template <bool INTERIOR, bool LAZY, bool MASKS>
-__device__ __forceinline__ void border_conn(const uint8_t *__restrict__ M, const BGrid &G, int bi, int c0, int c1,
-                                            int c2, int a, int b, int c, unsigned m, unsigned &conn,
-                                            unsigned &local, bool &full, uint64_t &mlo, uint64_t &mhi)
-{
-    conn = 0;
-    local = 0;
-    mlo = 0;
-    mhi = 0;
-    full = m == 0xffu;
-    const int plane = G.b1 * G.b2;
-#pragma unroll
-    for (int q = 0; q < 13; q++) {
-        const int d0 = nb_d0(q), d1 = nb_d1(q), d2 = nb_d2(q);
-        if (!INTERIOR) {
-            const int a0 = c0 + d0, a1 = c1 + d1, a2 = c2 + d2;
-            if (a0 < 0 || a1 < 0 || a2 < 0 || a1 >= G.b1 || a2 >= G.b2)
-                continue;
+    __shared__ CrossSet S;
+    const TileId T;
+    S.init();
+    // pairs of blocks: bit c of em, e0, ep is block x + c with y + c - 1, y + c
+    // and y + c + 1
+    unsigned em = 0, e0 = 0, ep = 0;
+    int x = 0, y = 0;
+    const int i = threadIdx.x;
+    if (i < kCrossPairs) {
+        int a, b, q;
+        cross_pair(i, a, b, q);
+        const int c0 = T.ti * kT0 + a, c1 = T.tj * kT1 + b, n0 = c0 + row_d0(q), n1 = c1 + row_d1(q);
+        if (c0 < G.b0 && c1 < G.b1 && n0 >= 0 && n1 >= 0 && n1 < G.b1) {
+            const unsigned *nv = V + row_word(G, n0, n1, T.tk, T.nt2);
+            const RowBits own = row_bits(V + row_word(G, c0, c1, T.tk, T.nt2)), nb = row_bits(nv);
+            RowBits before = {}, after = {};
+            if (T.tk > 0)
+                before = row_bits(nv - 8);
+            if (T.tk + 1 < T.nt2)
+                after = row_bits(nv + 8);
+            row_pairs(q, own, nb, &before, &after, em, e0, ep);
+            row_reduce(own.runs(), nb.runs(), em, e0, ep);
+            x = (c0 * G.b1 + c1) * G.b2 + T.tk * kT2;
+            y = (n0 * G.b1 + n1) * G.b2 + T.tk * kT2;
         }
-        if (!(m & touch_bits(d0, d1, d2)))
-            continue;
-        const bool in_tile = a + d0 >= 0 && b + d1 >= 0 && b + d1 < kT1 && c + d2 >= 0 && c + d2 < kT2;
-        if (LAZY && in_tile && m != 0xffu)
-            continue;
-        const unsigned mn = M[bi + d0 * plane + d1 * G.b2 + d2];
-        if (!(mn & touch_bits(-d0, -d1, -d2)))
-            continue;
-        conn |= 1u << q;
-        full = full && mn == 0xffu;
-        if (MASKS) {
-            if (q < 8)
-                mlo |= (uint64_t)mn << (8 * q);
-            else
-                mhi |= (uint64_t)mn << (8 * (q - 8));
-        }
-        if (in_tile)
-            local |= 1u << q;
-    }
-}
-
-// All 13 earlier neighbours of block (c0, c1, c2) inside the volume.
-__device__ __forceinline__ bool nb_interior(const BGrid &G, int c0, int c1, int c2)
-{
-    return c0 >= 1 && c1 >= 1 && c1 + 1 < G.b1 && c2 >= 1 && c2 + 1 < G.b2;
-}
-
-// Phase 2a: border blocks whose cross-tile links need no union (empty, no
-// touching neighbour outside the tile, or dense with an in-tile neighbour
-// that links them all) stop here; the others are listed for phase 2b (as
-// block indices), so that its warps run full.  One thread block per tile,
-// border item t on thread t.  The in-tile neighbours matter only for the
-// dense rule, so only full blocks read their masks.
-__global__ void __launch_bounds__(512) k_bcc_cross(const uint8_t *__restrict__ M, BGrid G, int *hard, int *nhard)
-{
-    const int nt1 = (G.b1 + kT1 - 1) / kT1, nt2 = (G.b2 + kT2 - 1) / kT2;
-    const int tile = blockIdx.x;
-    const int ti = tile / (nt1 * nt2), tj = (tile / nt2) % nt1, tk = tile % nt2;
-    const int t = threadIdx.x;
-    bool need = false;
-    int bi = -1;
-    if (t < kBorder) {
-        int a, b, c;
-        border_block(t, a, b, c);
-        const int c0 = ti * kT0 + a, c1 = tj * kT1 + b, c2 = tk * kT2 + c;
-        const unsigned m = c0 < G.b0 && c1 < G.b1 && c2 < G.b2 ? M[(c0 * G.b1 + c1) * G.b2 + c2] : 0u;
-        bi = (c0 * G.b1 + c1) * G.b2 + c2;
+    } else if (i >= kCrossThreads - kT0 * kT1 * 2) {
+        const int k = i - (kCrossThreads - kT0 * kT1 * 2), r = k >> 1, a = r / kT1, b = r % kT1;
+        const bool low = !(k & 1);
+        const int dz = low ? -1 : 1;
+        const int c0 = T.ti * kT0 + a, c1 = T.tj * kT1 + b, c2 = T.tk * kT2 + (low ? 0 : kT2 - 1);
+        const bool in = c0 < G.b0 && c1 < G.b1 && c2 < G.b2 && c2 + dz >= 0 && c2 + dz < G.b2;
+        x = (c0 * G.b1 + c1) * G.b2 + c2;
+        const unsigned m = in ? M[x] : 0u;
         if (m) {
-            unsigned conn, local;
-            bool full;
-            uint64_t mlo, mhi;
-            if (nb_interior(G, c0, c1, c2))
-                border_conn<true, true, false>(M, G, bi, c0, c1, c2, a, b, c, m, conn, local, full, mlo, mhi);
-            else
-                border_conn<false, true, false>(M, G, bi, c0, c1, c2, a, b, c, m, conn, local, full, mlo, mhi);
-            // in-tile neighbours were united in phase 1, and so was
-            // everything touching them
-            need = (conn & ~local) != 0 && !(full && ((conn >> kCentre) & 1u) && local);
-        }
-    }
-    if (t >= (kBorder + 31) / 32 * 32)
-        return; // warps without border items
-    const int lane = t & 31;
-    const unsigned bal = __ballot_sync(0xffffffffu, need);
-    if (bal) {
-        int pos = 0;
-        if (lane == 0)
-            pos = atomicAdd(nhard, __popc(bal));
-        pos = __shfl_sync(0xffffffffu, pos, 0);
-        if (need)
-            hard[pos + __popc(bal & ((1u << lane) - 1u))] = bi;
-    }
-}
-
-// Phase 2b: the listed border blocks unite with touching earlier neighbours in
-// other tiles; neighbours reached through an in-tile neighbour are skipped.
-// Each lane first collects its block's union targets, then the warp issues
-// them in rounds: lanes whose (block parent, neighbour parent) pairs are
-// equal would unite the same two components, so one lane per distinct pair
-// unites (parents only ever move towards roots, so equal parents read at
-// any time mean equal roots).  Consecutive listed blocks mostly come from one
-// tile and reach the same neighbouring components.
-__global__ void k_bcc_cross_unite(int *P, const uint8_t *__restrict__ M, BGrid G, int *err, const int *hard,
-                                  const int *nhard, unsigned long long *units)
-{
-    __shared__ BTabs tb;
-    load_btabs(tb);
-    __syncthreads();
-    const int cnt = *nhard;
-    if (units && blockIdx.x == 0 && threadIdx.x == 0 && cnt > 0)
-        atomicAdd(units, (unsigned long long)cnt);
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int h0 = warp * 32; h0 < cnt; h0 += nwarps * 32) {
-        // listed border blocks (block indices) and their offsets in their tile
-        const int h = h0 + lane;
-        unsigned todo = 0;
-        int bi = 0, pb = 0;
-        if (h < cnt) {
-            bi = hard[h];
-            int c2, c0, c1;
-            G.coords(bi, c0, c1, c2);
-            const int a = c0 % kT0, b = c1 % kT1, c = c2 % kT2;
-            const unsigned m = M[bi];
-            unsigned conn, local;
-            bool full;
-            uint64_t mlo, mhi;
-            if (nb_interior(G, c0, c1, c2))
-                border_conn<true, false, true>(M, G, bi, c0, c1, c2, a, b, c, m, conn, local, full, mlo, mhi);
-            else
-                border_conn<false, false, true>(M, G, bi, c0, c1, c2, a, b, c, m, conn, local, full, mlo, mhi);
-            unsigned covered = 0;
-            if (full && ((conn >> kCentre) & 1u))
-                covered = conn & ~(1u << kCentre); // the centre links all of them
-            while (local & ~covered) {
-                const int q = next_cover(local & ~covered);
-                covered |= bcover(q, conn & ~covered, mlo, mhi, tb);
+            // touching neighbours as bits 0-4 (0-3: row q, 4: the block before)
+            unsigned todo = 0;
+            if (low && (m & touch_bits(0, 0, -1)) && (M[x - 1] & touch_bits(0, 0, 1)))
+                todo = 16u;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int d0 = row_d0(q), d1 = row_d1(q);
+                if (a + d0 < 0 || b + d1 < 0 || b + d1 >= kT1 || c1 + d1 >= G.b1)
+                    continue; // (a row pair's, or outside)
+                if ((m & touch_bits(d0, d1, dz)) &&
+                    (M[x + (d0 * G.b1 + d1) * G.b2 + dz] & touch_bits(-d0, -d1, -dz)))
+                    todo |= 1u << q;
             }
-            while (conn & ~covered) {
-                const unsigned rest = conn & ~covered;
-                const int q = next_cover(rest);
-                todo |= 1u << q;
-                covered |= bcover(q, rest, mlo, mhi, tb);
-            }
-            pb = ld(P + bi);
-        }
-        while (__any_sync(0xffffffffu, todo != 0)) {
-            int o = -1;
-            unsigned long long key = ~0ull - (unsigned)lane; // unique for lanes without a target
-            if (todo) {
+            while (todo) {
                 const int q = __ffs(todo) - 1;
                 todo &= todo - 1;
-                o = bi + nb_d0(q) * G.b1 * G.b2 + nb_d1(q) * G.b2 + nb_d2(q);
-                key = ((unsigned long long)(unsigned)pb << 32) | (unsigned)ld(P + o);
-            }
-            const unsigned same = __match_any_sync(0xffffffffu, key);
-            if (o >= 0 && (__ffs(same) - 1) == lane)
-                unite(P, bi, o, err);
-        }
-    }
-}
-
-// Phases 2a and 2b in one pass: one thread block per tile, border item t on
-// thread t; a border block that needs cross-tile unions collects its targets
-// (as k_bcc_cross_unite does) and its warp unites in rounds, one lane per
-// distinct (block parent, neighbour parent) pair.  Each border block and its
-// neighbours' masks are read once, and no list is written.
-__global__ void __launch_bounds__(512) k_bcc_cross_fused(int *P, const uint8_t *__restrict__ M, BGrid G, int *err,
-                                                         unsigned long long *units)
-{
-    __shared__ BTabs tb;
-    load_btabs(tb);
-    __syncthreads();
-    const int nt1 = (G.b1 + kT1 - 1) / kT1, nt2 = (G.b2 + kT2 - 1) / kT2;
-    const int tile = blockIdx.x;
-    const int ti = tile / (nt1 * nt2), tj = (tile / nt2) % nt1, tk = tile % nt2;
-    const int t = threadIdx.x;
-    if (t >= (kBorder + 31) / 32 * 32)
-        return; // warps without border items
-    const int lane = t & 31;
-    unsigned todo = 0;
-    int bi = 0, pb = 0;
-    if (t < kBorder) {
-        int a, b, c;
-        border_block(t, a, b, c);
-        const int c0 = ti * kT0 + a, c1 = tj * kT1 + b, c2 = tk * kT2 + c;
-        const unsigned m = c0 < G.b0 && c1 < G.b1 && c2 < G.b2 ? M[(c0 * G.b1 + c1) * G.b2 + c2] : 0u;
-        bi = (c0 * G.b1 + c1) * G.b2 + c2;
-        if (m) {
-            unsigned conn, local;
-            bool full;
-            uint64_t mlo, mhi;
-            if (nb_interior(G, c0, c1, c2))
-                border_conn<true, false, true>(M, G, bi, c0, c1, c2, a, b, c, m, conn, local, full, mlo, mhi);
-            else
-                border_conn<false, false, true>(M, G, bi, c0, c1, c2, a, b, c, m, conn, local, full, mlo, mhi);
-            // in-tile neighbours were united in phase 1, and so was
-            // everything touching them
-            if ((conn & ~local) != 0 && !(full && ((conn >> kCentre) & 1u) && local)) {
-                unsigned covered = 0;
-                if (full && ((conn >> kCentre) & 1u))
-                    covered = conn & ~(1u << kCentre); // the centre links all of them
-                while (local & ~covered) {
-                    const int q = next_cover(local & ~covered);
-                    covered |= bcover(q, conn & ~covered, mlo, mhi, tb);
-                }
-                while (conn & ~covered) {
-                    const unsigned rest = conn & ~covered;
-                    const int q = next_cover(rest);
-                    todo |= 1u << q;
-                    covered |= bcover(q, rest, mlo, mhi, tb);
-                }
-                pb = ld(P + bi);
+                S.add(P, x, q == 4 ? x - 1 : x + (row_d0(q) * G.b1 + row_d1(q)) * G.b2 + dz, err);
             }
         }
     }
-    if (units && todo)
-        atomicAdd(units, 1ull);
-    while (__any_sync(0xffffffffu, todo != 0)) {
-        int o = -1;
-        unsigned long long key = ~0ull - (unsigned)lane; // unique for lanes without a target
-        if (todo) {
-            const int q = __ffs(todo) - 1;
-            todo &= todo - 1;
-            o = bi + nb_d0(q) * G.b1 * G.b2 + nb_d1(q) * G.b2 + nb_d2(q);
-            key = ((unsigned long long)(unsigned)pb << 32) | (unsigned)ld(P + o);
-        }
-        const unsigned same = __match_any_sync(0xffffffffu, key);
-        if (o >= 0 && (__ffs(same) - 1) == lane)
-            unite(P, bi, o, err);
+    while (em | e0 | ep) {
+        const int dz = e0 ? 0 : em ? -1 : 1;
+        const unsigned e = e0 ? e0 : em ? em : ep;
+        const int c = __ffs(e) - 1;
+        const unsigned bit = e & (0u - e);
+        e0 &= ~(dz == 0 ? bit : 0u);
+        em &= ~(dz < 0 ? bit : 0u);
+        ep &= ~(dz > 0 ? bit : 0u);
+        S.add(P, x + c, y + c + dz, err);
     }
-}
-
-static bool g_btables_ready[64] = {false};
-
-static int ensure_block_tables()
-{
-    int dev = 0;
-    PMG_CUDA(cudaGetDevice(&dev));
-    if (dev >= 0 && dev < 64 && g_btables_ready[dev])
-        return PMG_OK;
-    int nb[13][3];
-    unsigned short adj[13];
-    host_tables(nb, adj);
-    uint8_t self[13], other[13], pair[13][13];
-    for (int q = 0; q < 13; q++) {
-        self[q] = (uint8_t)touch_mask(nb[q][0], nb[q][1], nb[q][2]);
-        other[q] = (uint8_t)touch_mask(-nb[q][0], -nb[q][1], -nb[q][2]);
-        for (int r = 0; r < 13; r++)
-            pair[r][q] = (adj[r] >> q) & 1
-                             ? (uint8_t)touch_mask(nb[q][0] - nb[r][0], nb[q][1] - nb[r][1], nb[q][2] - nb[r][2])
-                             : (uint8_t)0;
-    }
-    PMG_CUDA(cudaMemcpyToSymbol(c_bt_self, self, sizeof(self)));
-    PMG_CUDA(cudaMemcpyToSymbol(c_bt_nb, other, sizeof(other)));
-    PMG_CUDA(cudaMemcpyToSymbol(c_bt_pair, pair, sizeof(pair)));
-    signed char gd[26][3];
-    uint8_t gself[26], gnb[26];
-    int q26 = 0;
-    for (int d0 = -1; d0 <= 1; d0++)
-        for (int d1 = -1; d1 <= 1; d1++)
-            for (int d2 = -1; d2 <= 1; d2++) {
-                if (!d0 && !d1 && !d2)
-                    continue;
-                gd[q26][0] = (signed char)d0;
-                gd[q26][1] = (signed char)d1;
-                gd[q26][2] = (signed char)d2;
-                gself[q26] = (uint8_t)touch_mask(d0, d1, d2);
-                gnb[q26] = (uint8_t)touch_mask(-d0, -d1, -d2);
-                q26++;
-            }
-    PMG_CUDA(cudaMemcpyToSymbol(c_g_d, gd, sizeof(gd)));
-    PMG_CUDA(cudaMemcpyToSymbol(c_g_self, gself, sizeof(gself)));
-    PMG_CUDA(cudaMemcpyToSymbol(c_g_nb, gnb, sizeof(gnb)));
-    if (dev >= 0 && dev < 64)
-        g_btables_ready[dev] = true;
-    return PMG_OK;
+    S.finish(P, err);
 }
 
 // periodic seams at block level: a foreground halo voxel joins the block of the
@@ -1799,15 +1683,6 @@ __global__ void k_bcc_twins(const uint8_t *__restrict__ M, int *P, BGrid G, Twin
         const int ba = (int)(((c[0] >> 1) * G.b1 + (c[1] >> 1)) * G.b2 + (c[2] >> 1));
         const int bb = (int)(((t[0] >> 1) * G.b1 + (t[1] >> 1)) * G.b2 + (t[2] >> 1));
         unite(P, ba, bb, err);
-    }
-}
-
-__global__ void k_bcc_flatten(int *P, int nb, int *err)
-{
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-        const int p = P[b];
-        if (p >= 0 && p != b)
-            P[b] = find_root(P, p, err);
     }
 }
 
@@ -1975,63 +1850,45 @@ static BGrid bgrid_of(const int64_t *shape)
     return G;
 }
 
-// Block union-find of the source: tiles, cross-tile unions, periodic seams
-// (twins), flattening.  P[b] = root block (the smallest block index of the
-// component), -1 for empty blocks; M[b] = block mask.
-template <class Src>
-static int bcc_build(const Src &src, const int64_t *shape, const int32_t *bc, const int32_t *pad, bool twins,
-                     int *P, uint8_t *M, int *err, cudaStream_t st, bool flatten = true, int *Pl = nullptr,
-                     int *dirty = nullptr, int *hard_buf = nullptr)
+// bytes of the row words of a block grid
+static size_t bcc_row_bytes(const BGrid &G)
 {
-    PMG_TRY(ensure_tables());
-    PMG_TRY(ensure_block_tables());
+    return (size_t)G.b0 * G.b1 * (size_t)((G.b2 + kT2 - 1) / kT2) * 8 * sizeof(unsigned);
+}
+
+static dim3 bcc_tiles(const BGrid &G)
+{
+    return dim3((unsigned)((G.b2 + kT2 - 1) / kT2), (unsigned)((G.b1 + kT1 - 1) / kT1),
+                (unsigned)((G.b0 + kT0 - 1) / kT0));
+}
+
+// Phase 1 of the block union-find (k_bcc_tile); V: bcc_row_bytes.
+template <class Src>
+static int bcc_tile_phase(const Src &src, const int64_t *shape, int *P, uint8_t *M, unsigned *V, cudaStream_t st,
+                          int *Pl = nullptr, int *dirty = nullptr)
+{
     const BGrid G = bgrid_of(shape);
     const int nb = G.b0 * G.b1 * G.b2;
-    const long long n = shape[0] * shape[1] * shape[2];
-    {
-        const int nt = ((G.b0 + kT0 - 1) / kT0) * ((G.b1 + kT1 - 1) / kT1) * ((G.b2 + kT2 - 1) / kT2);
-        const int ps__ = prof_begin("k_bcc_tile", st);
-        k_bcc_tile<Src><<<nt, kTile, 0, st>>>(src, P, M, G, Pl, dirty);
-        prof_end(ps__, src_bytes(src, n, nb) + (double)nb * 5, st);
-    }
+    const int ps__ = prof_begin("k_bcc_tile", st);
+    k_bcc_tile<Src><<<bcc_tiles(G), kTile, 0, st>>>(src, P, M, V, G, Pl, dirty);
+    prof_end(ps__, src_bytes(src, (long long)shape[0] * shape[1] * shape[2], nb) + (double)nb * 6, st);
     PMG_CHECK_LAUNCH();
-    if (tune_value(kTuneCcCrossFused)) {
-        const int nt = ((G.b0 + kT0 - 1) / kT0) * ((G.b1 + kT1 - 1) / kT1) * ((G.b2 + kT2 - 1) / kT2);
-        const int ps__ = prof_begin("k_bcc_cross_fused", st);
-        k_bcc_cross_fused<<<nt, 512, 0, st>>>(P, M, G, err, prof_units(kUnitsCrossUnite));
-        // per border block: its mask and the masks of its 13 earlier
-        // neighbours; two parents per union
-        prof_end(ps__, (double)nt * kBorder * 14, st);
+    return PMG_OK;
+}
+
+// Phase 2 and the periodic seams (twins).
+static int bcc_cross_phase(const int64_t *shape, const int32_t *bc, const int32_t *pad, bool twins, int *P,
+                           const uint8_t *M, const unsigned *V, int *err, cudaStream_t st)
+{
+    const BGrid G = bgrid_of(shape);
+    const long long n = shape[0] * shape[1] * shape[2];
+    const dim3 tiles = bcc_tiles(G);
+    {
+        const int ps__ = prof_begin("k_bcc_cross", st);
+        k_bcc_cross<<<tiles, kCrossThreads, 0, st>>>(P, M, V, G, err);
+        // the words of the rows of every pair
+        prof_end(ps__, (double)tiles.x * tiles.y * tiles.z * kCrossPairs * 2 * kT2, st);
         PMG_CHECK_LAUNCH();
-    } else {
-        const long long border = (long long)((G.b0 + kT0 - 1) / kT0) * ((G.b1 + kT1 - 1) / kT1) *
-                                 ((G.b2 + kT2 - 1) / kT2) * kBorder;
-        // list of the border blocks that need unions, and its length (in the
-        // caller's buffer of border + 64 ints, if given)
-        int *hard = hard_buf;
-        if (!hard)
-            PMG_TRY(scratch_alloc((void **)&hard, sizeof(int) * (size_t)(border + 64), st));
-        int *nhard = hard + border + 32;
-        PMG_CUDA(cudaMemsetAsync(nhard, 0, sizeof(int), st));
-        {
-            const int ps__ = prof_begin("k_bcc_cross", st);
-            const int nt = (int)(border / kBorder);
-            k_bcc_cross<<<nt, 512, 0, st>>>(M, G, hard, nhard);
-            // per border block: its mask, the mask facing it across the tile
-            // border
-            prof_end(ps__, (double)border * 2, st);
-        }
-        PMG_CHECK_LAUNCH();
-        {
-            const int ps__ = prof_begin("k_bcc_cross_unite", st);
-            k_bcc_cross_unite<<<152 * 16, 256, 0, st>>>(P, M, G, err, hard, nhard, prof_units(kUnitsCrossUnite));
-            // per listed border block: its entry and mask, the masks of its 13
-            // earlier neighbours, two parents per union
-            prof_end_units(ps__, kUnitsCrossUnite, 4 + 1 + 13 + 8, st);
-        }
-        PMG_CHECK_LAUNCH();
-        if (!hard_buf)
-            PMG_TRY(scratch_free(hard, st));
     }
     if (twins && any_periodic(bc)) {
         const int ps__ = prof_begin("k_bcc_twins", st);
@@ -2039,13 +1896,26 @@ static int bcc_build(const Src &src, const int64_t *shape, const int32_t *bc, co
         prof_end(ps__, 0.0, st);
         PMG_CHECK_LAUNCH();
     }
-    if (flatten) {
-        const int ps__ = prof_begin("k_bcc_flatten", st);
-        k_bcc_flatten<<<grid_for(nb, 256, 152LL * 64), 256, 0, st>>>(P, nb, err);
-        prof_end(ps__, (double)nb * 8, st);
-        PMG_CHECK_LAUNCH();
-    }
     return PMG_OK;
+}
+
+// Block union-find of the source: tiles, cross-tile unions, periodic seams
+// (twins).  P[b]: a parent on the way to the root block (the smallest block
+// index of the component), -1 for empty blocks; M[b] = block mask.
+template <class Src>
+static int bcc_build(const Src &src, const int64_t *shape, const int32_t *bc, const int32_t *pad, bool twins,
+                     int *P, uint8_t *M, int *err, cudaStream_t st, int *Pl = nullptr, int *dirty = nullptr,
+                     unsigned *Vkeep = nullptr)
+{
+    unsigned *V = Vkeep;
+    if (!V)
+        PMG_TRY(scratch_alloc((void **)&V, bcc_row_bytes(bgrid_of(shape)), st));
+    int s = bcc_tile_phase(src, shape, P, M, V, st, Pl, dirty);
+    if (s == PMG_OK)
+        s = bcc_cross_phase(shape, bc, pad, twins, P, M, V, err, st);
+    if (!Vkeep)
+        PMG_TRY(scratch_free(V, st));
+    return s;
 }
 
 // Inlet / outlet boxes (lo0, hi0, lo1, hi1, lo2, hi2; null or lo0 < 0 for
@@ -2133,7 +2003,7 @@ static int bcc_select_core(const Src &src, void *out, int out_bytes, const int64
                            unsigned long long *kept)
 {
     PMG_TRY(check_boxes(shape, inlet_box, outlet_box));
-    PMG_TRY(bcc_build(src, shape, bc, pad, true, P, M, err, st, false));
+    PMG_TRY(bcc_build(src, shape, bc, pad, true, P, M, err, st));
     return bcc_mark_select(out, out_bytes, shape, inlet_box, outlet_box, mode, val, P, M, mark, err, st, kept);
 }
 
@@ -2376,12 +2246,10 @@ static int grow_step(GrowSel &g, const Src &src, const int64_t *shape, const int
 {
     PMG_TRY(check_boxes(shape, inlet_box, outlet_box));
     if (!g.built) {
-        PMG_TRY(bcc_build(src, shape, bc, pad, true, g.P, g.M, err, st, false));
+        PMG_TRY(bcc_build(src, shape, bc, pad, true, g.P, g.M, err, st));
         g.built = true;
         return bcc_marks(shape, inlet_box, outlet_box, g.P, g.M, g.mark, err, st);
     }
-    PMG_TRY(ensure_tables());
-    PMG_TRY(ensure_block_tables());
     const BGrid G = bgrid_of(shape);
     const int nb = G.b0 * G.b1 * G.b2;
     const long long n = shape[0] * shape[1] * shape[2];
@@ -2764,8 +2632,6 @@ int grow_marks_pair(GrowSel &a, const uint8_t *S, int k, const uint16_t *E, int 
         return grow_marks_binary(b, img, fgval, shape, bc, pad, inlet_box, err, st);
     }
     PMG_TRY(check_boxes(shape, inlet_box, nullptr));
-    PMG_TRY(ensure_tables());
-    PMG_TRY(ensure_block_tables());
     const BGrid G = bgrid_of(shape);
     const int nb = G.b0 * G.b1 * G.b2;
     const long long n = shape[0] * shape[1] * shape[2];
@@ -2884,7 +2750,7 @@ int bcc_marks_binary(const uint8_t *img, int fgval, const int64_t *shape, const 
 {
     PMG_TRY(check_boxes(shape, inlet_box, outlet_box));
     SrcImg src{img, fgval};
-    PMG_TRY(bcc_build(src, shape, bc, pad, true, P, M, err, st, false));
+    PMG_TRY(bcc_build(src, shape, bc, pad, true, P, M, err, st));
     return bcc_marks(shape, inlet_box, outlet_box, P, M, mark, err, st);
 }
 
@@ -2901,9 +2767,8 @@ size_t shrink_sel_bytes(const int64_t *shape)
     const size_t nb = (size_t)G.b0 * G.b1 * G.b2;
     const size_t a = (nb + 255) & ~(size_t)255;
     const size_t nt = (size_t)((G.b0 + kT0 - 1) / kT0) * ((G.b1 + kT1 - 1) / kT1) * ((G.b2 + kT2 - 1) / kT2);
-    // P, Pl, M, mark, per-tile flags, the cross-tile list (kBorder per tile + 64)
-    return a * 4 * 2 + a * 2 + ((nt * 4 + 255) & ~(size_t)255) + (((nt * kBorder + 64) * 4 + 255) & ~(size_t)255) +
-           256;
+    // P, Pl, M, mark, per-tile flags, row words
+    return a * 4 * 2 + a * 2 + ((nt * 4 + 255) & ~(size_t)255) + bcc_row_bytes(G) + 256;
 }
 
 void shrink_sel_init(ShrinkSel &g, void *mem, const int64_t *shape)
@@ -2923,7 +2788,7 @@ void shrink_sel_init(ShrinkSel &g, void *mem, const int64_t *shape)
     p += a;
     g.dirty = (int *)p;
     p += (nt * 4 + 255) & ~(size_t)255;
-    g.hard = (int *)p;
+    g.V = (unsigned *)p;
     g.ntiles = (int)nt;
     g.built = false;
 }
@@ -2937,10 +2802,10 @@ int shrink_marks_binary(ShrinkSel &g, const uint8_t *img, int fgval, const int64
         PMG_CUDA(cudaMemsetAsync(g.dirty, 0, sizeof(int) * (size_t)g.ntiles, st));
     if (g.built) {
         // the producer of the changes kept the block masks current
-        PMG_TRY(bcc_build(SrcMask{g.M}, shape, bc, pad, true, g.P, g.M, err, st, false, g.Pl, g.dirty, g.hard));
+        PMG_TRY(bcc_build(SrcMask{g.M}, shape, bc, pad, true, g.P, g.M, err, st, g.Pl, g.dirty, g.V));
     } else {
         SrcImg src{img, fgval};
-        PMG_TRY(bcc_build(src, shape, bc, pad, true, g.P, g.M, err, st, false, g.Pl, nullptr, g.hard));
+        PMG_TRY(bcc_build(src, shape, bc, pad, true, g.P, g.M, err, st, g.Pl, nullptr, g.V));
     }
     g.built = true;
     return bcc_marks(shape, inlet_box, outlet_box, g.P, g.M, g.mark, err, st);
@@ -3184,58 +3049,6 @@ int drain_update_blocks(uint8_t *mp, const uint8_t *morph, const int64_t *shape,
 // component's first block plane (the plane of its root, the smallest block
 // index), so only blocks of that plane compete for it.
 
-// smallest and largest nonzero value: 16 bytes per load where the image is
-// 16-byte aligned (per-byte SIMD minima with zeros mapped to 255), bytes
-// otherwise and for the tail
-__global__ void k_nz_range(const uint8_t *__restrict__ img, long long n, unsigned *lohi)
-{
-    unsigned lo = 255, hi = 0;
-    const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x, nth = (long long)gridDim.x * blockDim.x;
-    long long head = 0;
-    if (!(reinterpret_cast<uintptr_t>(img) & 15)) {
-        const long long nv = n >> 4;
-        const uint4 *v4 = reinterpret_cast<const uint4 *>(img);
-        unsigned lo4 = 0xFFFFFFFFu, hi4 = 0u;
-        for (long long i = tid; i < nv; i += nth) {
-            const uint4 w = __ldg(v4 + i);
-            const unsigned ws[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                hi4 = __vmaxu4(hi4, ws[q]);
-                lo4 = __vminu4(lo4, ws[q] | __vcmpeq4(ws[q], 0u));
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            lo = min(lo, (lo4 >> (8 * q)) & 0xFFu);
-            hi = max(hi, (hi4 >> (8 * q)) & 0xFFu);
-        }
-        head = nv << 4;
-    }
-    for (long long i = head + tid; i < n; i += nth) {
-        const unsigned v = img[i];
-        if (v) {
-            lo = min(lo, v);
-            hi = max(hi, v);
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        lo = min(lo, __shfl_down_sync(0xffffffffu, lo, o));
-        hi = max(hi, __shfl_down_sync(0xffffffffu, hi, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(lohi, lo);
-        atomicMax(lohi + 1, hi);
-    }
-}
-
-__global__ void k_fill_i32(int *a, long long n, int v)
-{
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x)
-        a[i] = v;
-}
-
 __device__ __forceinline__ int block_first_voxel(const BGrid &G, int b, unsigned m)
 {
     int c0, c1, c2;
@@ -3245,33 +3058,71 @@ __device__ __forceinline__ int block_first_voxel(const BGrid &G, int b, unsigned
     return ((2 * c0 + x) * G.s1 + 2 * c1 + y) * G.s2 + 2 * c2 + z;
 }
 
-// F[root] = first voxel of the component
-__global__ void k_blk_first(const int *__restrict__ P, const uint8_t *__restrict__ M, BGrid G, int *F)
+// Parents flattened to the roots, the roots listed (roots[0 .. *nroots), in no
+// order) and F[root] lowered to the component's first voxel (unsigned, all ones
+// before).  Four blocks per thread, so that their chains of dependent loads
+// overlap: block by block this pass and a separate one for the first voxels
+// took 2.0 ms at 1024^3.
+__global__ void __launch_bounds__(256) k_blk_roots(int *__restrict__ P, const uint8_t *__restrict__ M, BGrid G,
+                                                   unsigned *F, int *__restrict__ roots, int *nroots, int *err)
 {
-    const int nb = G.b0 * G.b1 * G.b2;
-    const int plane = G.b1 * G.b2;
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-        const unsigned m = M[b];
-        if (!m)
-            continue;
-        const int r = P[b];
-        if (r < 0 || b / plane != r / plane)
-            continue;
-        const int f = block_first_voxel(G, b, m);
-        if (f < F[r])
-            atomicMin(F + r, f);
+    const int nb = G.b0 * G.b1 * G.b2, plane = G.b1 * G.b2;
+    const int lane = threadIdx.x & 31;
+    constexpr int NB = 4;
+    for (int base = blockIdx.x * blockDim.x * NB; base < nb; base += gridDim.x * blockDim.x * NB) {
+        int b[NB], p[NB], g[NB];
+        unsigned m[NB];
+#pragma unroll
+        for (int q = 0; q < NB; q++) {
+            b[q] = base + q * blockDim.x + threadIdx.x;
+            const bool in = b[q] < nb;
+            p[q] = in ? ld(P + b[q]) : -1;
+            m[q] = in ? M[b[q]] : 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < NB; q++)
+            g[q] = p[q] >= 0 && p[q] != b[q] ? ld(P + p[q]) : p[q];
+#pragma unroll
+        for (int q = 0; q < NB; q++) {
+            int r = p[q];
+            if (r >= 0 && r != b[q]) {
+                if (g[q] != r)
+                    r = find_root(P, g[q], err);
+                if (r != p[q])
+                    P[b[q]] = r;
+            }
+            const unsigned bal = __ballot_sync(0xffffffffu, r >= 0 && r == b[q]);
+            if (bal) {
+                int pos = 0;
+                if (lane == 0)
+                    pos = atomicAdd(nroots, __popc(bal));
+                pos = __shfl_sync(0xffffffffu, pos, 0);
+                if (r == b[q] && r >= 0)
+                    roots[pos + __popc(bal & ((1u << lane) - 1u))] = r;
+            }
+            // the first voxel lies in the root's block plane
+            if (r >= 0 && b[q] - r < plane) {
+                int c0, c1, c2;
+                G.coords(b[q], c0, c1, c2);
+                if (r >= c0 * plane) {
+                    const unsigned f = (unsigned)block_first_voxel(G, b[q], m[q]);
+                    if (f < *(volatile unsigned *)(F + r))
+                        atomicMin(F + r, f);
+                }
+            }
+        }
     }
 }
 
 // bit f of `bits` set for every component's first voxel f
-__global__ void k_blk_first_bits(const int *__restrict__ P, const uint8_t *__restrict__ M, const int *__restrict__ F,
-                                 int nb, unsigned *bits)
+__global__ void k_blk_first_bits(const int *__restrict__ roots, const int *__restrict__ nroots,
+                                 const unsigned *__restrict__ F, unsigned *bits)
 {
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
-        if (M[b] && P[b] == b) {
-            const int f = F[b];
-            atomicOr(bits + (f >> 5), 1u << (f & 31));
-        }
+    const int n = *nroots;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const unsigned f = F[roots[i]];
+        atomicOr(bits + (f >> 5), 1u << (f & 31));
+    }
 }
 
 // set bits per tile of 32 words (1024 voxels)
@@ -3289,23 +3140,22 @@ __global__ void k_bits_count(const unsigned *__restrict__ bits, long long nwords
 }
 
 // root blocks: F[root] <- 1 + rank of its first voxel among all first voxels
-__global__ void k_root_label(const int *__restrict__ P, const uint8_t *__restrict__ M, int *F, int nb,
+__global__ void k_root_label(const int *__restrict__ roots, const int *__restrict__ nroots, unsigned *F,
                              const unsigned *__restrict__ bits, const int *__restrict__ offs)
 {
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-        if (!M[b] || P[b] != b)
-            continue;
-        const int f = F[b];
-        const int w = f >> 5;
+    const int n = *nroots;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const unsigned f = F[roots[i]];
+        const unsigned w = f >> 5;
         int r = offs[f >> 10] + __popc(bits[w] & ((1u << (f & 31)) - 1u));
-        for (int u = (f >> 10) * 32; u < w; u++)
+        for (unsigned u = (f >> 10) * 32; u < w; u++)
             r += __popc(bits[u]);
-        F[b] = r + 1;
+        F[roots[i]] = (unsigned)r + 1u;
     }
 }
 
 // labels of every voxel: a block's label on its foreground voxels, 0 elsewhere
-__global__ void k_blk_label_out(const int *__restrict__ P, const uint8_t *__restrict__ M, const int *__restrict__ F,
+__global__ void k_blk_label_out(const int *__restrict__ P, const uint8_t *__restrict__ M, const unsigned *__restrict__ F,
                                 BGrid G, uint64_t *__restrict__ labels, const uint64_t *__restrict__ lut)
 {
     const int nb = G.b0 * G.b1 * G.b2;
@@ -3334,33 +3184,12 @@ __global__ void k_blk_label_out(const int *__restrict__ P, const uint8_t *__rest
     }
 }
 
-// 1: the image holds one nonzero value (or none), so blocks can label it
-static int single_value(const uint8_t *img, long long n, int *yes, cudaStream_t st)
-{
-    unsigned *lohi = nullptr;
-    PMG_TRY(scratch_alloc((void **)&lohi, 2 * sizeof(unsigned), st));
-    const unsigned init[2] = {255u, 0u};
-    PMG_CUDA(cudaMemcpyAsync(lohi, init, sizeof(init), cudaMemcpyHostToDevice, st));
-    {
-        const int ps__ = prof_begin("k_nz_range", st);
-        k_nz_range<<<grid_for(n, 256, 152LL * 16), 256, 0, st>>>(img, n, lohi);
-        prof_end(ps__, (double)n, st);
-    }
-    PMG_CHECK_LAUNCH();
-    unsigned h[2] = {0, 0};
-    PMG_CUDA(cudaMemcpyAsync(h, lohi, sizeof(h), cudaMemcpyDeviceToHost, st));
-    PMG_CUDA(cudaStreamSynchronize(st));
-    PMG_TRY(scratch_free(lohi, st));
-    *yes = h[1] == 0 || h[0] == h[1];
-    return PMG_OK;
-}
-
 // ... or computed from the block union-find: a voxel's label is its block's
 // root's number when the voxel is foreground.
 struct LabBlk {
     const int *P;
     const uint8_t *M;
-    const int *F;
+    const unsigned *F;
     BGrid G;
     __device__ __forceinline__ uint64_t at(long long i, long long j, long long k) const
     {
@@ -3370,84 +3199,100 @@ struct LabBlk {
     }
 };
 
-int cc_label_blocks(const uint8_t *img, uint64_t *labels, const int64_t *shape, const int32_t *bc,
-                    const int32_t *pad, int64_t *count, cudaStream_t st)
+// *single = 0 (and no labels) when the image holds two nonzero values, which
+// the tile phase finds on the way: the caller then labels voxel by voxel.
+static int cc_label_blocks(const uint8_t *img, uint64_t *labels, const int64_t *shape, const int32_t *bc,
+                           const int32_t *pad, int64_t *count, int *single, cudaStream_t st)
 {
     const BGrid G = bgrid_of(shape);
     const int nb = G.b0 * G.b1 * G.b2;
     const long long n = shape[0] * shape[1] * shape[2];
     const long long nwords = (n + 31) / 32, ntiles = (nwords + 31) / 32;
-    int *P = nullptr, *F = nullptr, *err = nullptr, *cnt = nullptr, *offs = nullptr;
-    uint8_t *M = nullptr;
-    unsigned *bits = nullptr;
-    PMG_TRY(scratch_alloc((void **)&P, (size_t)nb * 4, st));
-    PMG_TRY(scratch_alloc((void **)&F, (size_t)nb * 4, st));
-    PMG_TRY(scratch_alloc((void **)&M, (size_t)nb, st));
-    PMG_TRY(scratch_alloc((void **)&err, sizeof(int), st));
-    PMG_TRY(scratch_alloc((void **)&bits, (size_t)nwords * 4, st));
-    PMG_TRY(scratch_alloc((void **)&cnt, (size_t)ntiles * 4 + 4, st));
-    PMG_TRY(scratch_alloc((void **)&offs, (size_t)ntiles * 4 + 4, st));
-    PMG_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
-    PMG_CUDA(cudaMemsetAsync(bits, 0, (size_t)nwords * 4, st));
-    SrcImg src{img, -1};
-    PMG_TRY(bcc_build(src, shape, bc, pad, false, P, M, err, st));
-    {
-        const int ps__ = prof_begin("k_blk_first", st);
-        k_fill_i32<<<grid_for(nb, 256, 152LL * 32), 256, 0, st>>>(F, nb, INT_MAX);
-        k_blk_first<<<grid_for(nb, 256, 152LL * 32), 256, 0, st>>>(P, M, G, F);
-        k_blk_first_bits<<<grid_for(nb, 256, 152LL * 32), 256, 0, st>>>(P, M, F, nb, bits);
-        k_bits_count<<<grid_for(ntiles, 256, 152LL * 32), 256, 0, st>>>(bits, nwords, cnt);
-        prof_end(ps__, (double)nb * 13, st);
-    }
-    PMG_CHECK_LAUNCH();
+    // one allocation: parents, first voxels (then labels), roots, row words,
+    // masks, first-voxel bits, their counts and offsets, scalars, scan scratch
     size_t tb = 0;
-    PMG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, offs, (int)ntiles + 1, st));
-    void *tmp = nullptr;
-    PMG_TRY(scratch_alloc(&tmp, tb, st));
-    PMG_CUDA(cudaMemsetAsync(cnt + ntiles, 0, 4, st));
-    PMG_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, offs, (int)ntiles + 1, st));
-    k_root_label<<<grid_for(nb, 256, 152LL * 32), 256, 0, st>>>(P, M, F, nb, bits, offs);
-    PMG_CHECK_LAUNCH();
-    int total = 0;
-    PMG_CUDA(cudaMemcpyAsync(&total, offs + ntiles, sizeof(int), cudaMemcpyDeviceToHost, st));
-    int s = read_err(err, st);
-    // periodic seams: the relabelling table is built from the blocks' labels
-    // on the seam slabs and folded into the one pass that writes the labels
-    uint64_t *lut = nullptr;
-    int64_t merged = total;
-    if (s == PMG_OK && any_periodic(bc))
-        s = periodic_renumber(LabBlk{P, M, F, G}, labels, shape, bc, pad, total, &merged, st, &lut);
-    if (s == PMG_OK) {
-        const int ps__ = prof_begin("k_blk_label_out", st);
-        k_blk_label_out<<<grid_for(nb, 256, 152LL * 64), 256, 0, st>>>(P, M, F, G, labels, lut);
-        prof_end(ps__, (double)n * 8 + (double)nb * 9, st);
-        s = cudaGetLastError() == cudaSuccess ? PMG_OK : PMG_ECUDA;
-    }
-    if (lut)
-        PMG_TRY(scratch_free(lut, st));
-    PMG_TRY(scratch_free(tmp, st));
-    PMG_TRY(scratch_free(P, st));
-    PMG_TRY(scratch_free(F, st));
-    PMG_TRY(scratch_free(M, st));
-    PMG_TRY(scratch_free(err, st));
-    PMG_TRY(scratch_free(bits, st));
-    PMG_TRY(scratch_free(cnt, st));
-    PMG_TRY(scratch_free(offs, st));
-    if (s != PMG_OK)
-        return s;
-    *count = merged;
-    return PMG_OK;
+    PMG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, (int *)nullptr, (int *)nullptr, (int)ntiles + 1, st));
+    auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t ib = up((size_t)nb * 4), cb = up((size_t)ntiles * 4 + 4);
+    char *mem = nullptr;
+    PMG_TRY(scratch_alloc((void **)&mem, 3 * ib + bcc_row_bytes(G) + up((size_t)nb) + up((size_t)nwords * 4) + 2 * cb +
+                                            256 + tb,
+                          st));
+    char *p = mem;
+    auto take = [&](size_t b) {
+        char *q = p;
+        p += b;
+        return q;
+    };
+    int *P = (int *)take(ib);
+    unsigned *F = (unsigned *)take(ib);
+    int *roots = (int *)take(ib);
+    unsigned *V = (unsigned *)take(bcc_row_bytes(G));
+    uint8_t *M = (uint8_t *)take(up((size_t)nb));
+    unsigned *bits = (unsigned *)take(up((size_t)nwords * 4));
+    int *cnt = (int *)take(cb), *offs = (int *)take(cb);
+    int *err = (int *)take(256), *nroots = err + 1;
+    unsigned *range = (unsigned *)(err + 2); // OR, AND of the nonzero values
+    void *tmp = p;
+    auto run = [&]() -> int {
+        PMG_CUDA(cudaMemsetAsync(err, 0, 3 * sizeof(int), st));
+        PMG_CUDA(cudaMemsetAsync(range + 1, 0xff, sizeof(int), st));
+        SrcImg src{img, -1};
+        src.range = range;
+        PMG_TRY(bcc_tile_phase(src, shape, P, M, V, st));
+        unsigned h[2] = {0, 0};
+        PMG_CUDA(cudaMemcpyAsync(h, range, sizeof(h), cudaMemcpyDeviceToHost, st));
+        PMG_CUDA(cudaStreamSynchronize(st));
+        *single = h[0] == 0 || h[0] == (h[1] & 0xffu);
+        if (!*single)
+            return PMG_OK;
+        PMG_TRY(bcc_cross_phase(shape, bc, pad, false, P, M, V, err, st));
+        PMG_CUDA(cudaMemsetAsync(F, 0xff, (size_t)nb * 4, st));
+        PMG_CUDA(cudaMemsetAsync(bits, 0, (size_t)nwords * 4, st));
+        {
+            const int ps__ = prof_begin("k_blk_roots", st);
+            k_blk_roots<<<grid_for((nb + 3) / 4, 256, 152LL * 32), 256, 0, st>>>(P, M, G, F, roots, nroots, err);
+            k_blk_first_bits<<<152, 256, 0, st>>>(roots, nroots, F, bits);
+            k_bits_count<<<grid_for(ntiles, 256, 152LL * 32), 256, 0, st>>>(bits, nwords, cnt);
+            prof_end(ps__, (double)nb * 9 + (double)nwords * 4, st);
+        }
+        PMG_CHECK_LAUNCH();
+        PMG_CUDA(cudaMemsetAsync(cnt + ntiles, 0, 4, st));
+        size_t tb2 = tb;
+        PMG_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb2, cnt, offs, (int)ntiles + 1, st));
+        k_root_label<<<152, 256, 0, st>>>(roots, nroots, F, bits, offs);
+        PMG_CHECK_LAUNCH();
+        int total = 0;
+        PMG_CUDA(cudaMemcpyAsync(&total, offs + ntiles, sizeof(int), cudaMemcpyDeviceToHost, st));
+        PMG_TRY(read_err(err, st));
+        // periodic seams: the relabelling table is built from the blocks' labels
+        // on the seam slabs and folded into the one pass that writes the labels
+        uint64_t *lut = nullptr;
+        int64_t merged = total;
+        if (any_periodic(bc))
+            PMG_TRY(periodic_renumber(LabBlk{P, M, F, G}, labels, shape, bc, pad, total, &merged, st, &lut));
+        {
+            const int ps__ = prof_begin("k_blk_label_out", st);
+            k_blk_label_out<<<grid_for(nb, 256, 152LL * 64), 256, 0, st>>>(P, M, F, G, labels, lut);
+            prof_end(ps__, (double)n * 8 + (double)nb * 9, st);
+            PMG_CHECK_LAUNCH();
+        }
+        if (lut)
+            PMG_TRY(scratch_free(lut, st));
+        *count = merged;
+        return PMG_OK;
+    };
+    const int s = run();
+    PMG_TRY(scratch_free(mem, st));
+    return s;
 }
 
 int cc_label_u8(const uint8_t *img, uint64_t *labels, const int64_t *shape, const int32_t *bc, const int32_t *pad,
                 int64_t *count, cudaStream_t st)
 {
-    const long long n = shape[0] * shape[1] * shape[2];
-    int yes = 0;
-    PMG_TRY(single_value(img, n, &yes, st));
-    if (yes)
-        return cc_label_blocks(img, labels, shape, bc, pad, count, st);
-    return cc_label_t(img, labels, shape, bc, pad, count, st);
+    int single = 0;
+    PMG_TRY(cc_label_blocks(img, labels, shape, bc, pad, count, &single, st));
+    return single ? PMG_OK : cc_label_t(img, labels, shape, bc, pad, count, st);
 }
 
 // Selection with caller-provided scratch: P (n int32), mark (n bytes rounded
