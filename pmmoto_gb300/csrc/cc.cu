@@ -1232,6 +1232,7 @@ struct BGrid {
     int s0, s1, s2;    // voxel shape
     int b0, b1, b2;    // block shape
     FastDiv q2, q1;    // division by b2 and by b1
+    FastDiv qt;        // division by the pieces of a row (32 blocks)
     // block index -> (c0, c1, c2)
     __device__ __forceinline__ void coords(int b, int &c0, int &c1, int &c2) const
     {
@@ -1288,12 +1289,6 @@ struct SrcStep {
         const unsigned v = *(const uint16_t *)(S + idx);
         return (unsigned)((int)(v & 0xffu) <= k) | ((unsigned)((int)(v >> 8) <= k) << 1);
     }
-};
-
-// ... or the block masks themselves, kept current by the producer of the set
-// (the drainage update keeps the wetting phase's).
-struct SrcMask {
-    const uint8_t *M;
 };
 
 // Mask of block (c0, c1, c2): bit (x * 2 + y) * 2 + z for a foreground voxel
@@ -1373,28 +1368,30 @@ __device__ __forceinline__ unsigned block_mask(const SrcImg &src, const BGrid &G
     return block_mask(src, G, c0, c1, c2, w);
 }
 
-// OR and AND of the nonzero bytes of w, over the warp, added to src.range.
-__device__ __forceinline__ void note_range(const SrcImg &src, const unsigned (&w)[2])
-{
-    const unsigned z0 = (nonzero01(w[0]) ^ 0x01010101u) * 0xffu, z1 = (nonzero01(w[1]) ^ 0x01010101u) * 0xffu;
-    unsigned o = w[0] | w[1], a = (w[0] | z0) & (w[1] | z1);
-    o |= o >> 16;
-    a &= a >> 16;
-    o = __reduce_or_sync(0xffffffffu, (o | (o >> 8)) & 0xffu);
-    a = __reduce_and_sync(0xffffffffu, (a & (a >> 8)) & 0xffu);
-    if ((threadIdx.x & 31) == 0 && o) {
-        // (values already seen cost a load)
-        if (o & ~*(volatile unsigned *)src.range)
-            atomicOr(src.range, o);
-        if (~a & 0xffu & *(volatile unsigned *)(src.range + 1))
-            atomicAnd(src.range + 1, a);
+// OR and AND of the nonzero bytes of a source's voxels, added to its range.
+struct ByteRange {
+    unsigned o = 0u, a = ~0u;
+    __device__ __forceinline__ void add(const unsigned (&w)[2])
+    {
+        o |= w[0] | w[1];
+        a &= (w[0] | (nonzero01(w[0]) ^ 0x01010101u) * 0xffu) & (w[1] | (nonzero01(w[1]) ^ 0x01010101u) * 0xffu);
     }
-}
-
-__device__ __forceinline__ unsigned block_mask(const SrcMask &src, const BGrid &G, int c0, int c1, int c2)
-{
-    return src.M[((long long)c0 * G.b1 + c1) * G.b2 + c2];
-}
+    // by whole warps
+    __device__ __forceinline__ void flush(unsigned *range)
+    {
+        o |= o >> 16;
+        a &= a >> 16;
+        o = __reduce_or_sync(0xffffffffu, (o | (o >> 8)) & 0xffu);
+        a = __reduce_and_sync(0xffffffffu, (a & (a >> 8)) & 0xffu);
+        if ((threadIdx.x & 31) == 0 && o) {
+            // (values already seen cost a load)
+            if (o & ~*(volatile unsigned *)range)
+                atomicOr(range, o);
+            if (~a & 0xffu & *(volatile unsigned *)(range + 1))
+                atomicAnd(range + 1, a);
+        }
+    }
+};
 
 // Voxels of a block that touch its neighbour at offset (d0, d1, d2): bit
 // (x * 2 + y) * 2 + z, x on the d0 side and so on.
@@ -1464,103 +1461,158 @@ __device__ __forceinline__ long long row_word(const BGrid &G, int c0, int c1, in
     return (((long long)c0 * G.b1 + c1) * nt2 + tk) * 8;
 }
 
-// Phase 1: block masks from the source, then a shared-memory union-find of the
-// tile whose roots are the smallest block index of each tile-local part.
-// Every later step reads the block masks M and their row words V, never the
-// source again.  One warp per row, lane = block; thread 4 r + q makes the
-// pairs of row r with its neighbouring row q.
-//
-// With Pl, the tile-local parents are also kept in Pl; with dirty (per tile),
-// a tile whose flag is clear has not changed since Pl was written and only
-// copies Pl to P, and every recomputed tile clears its flag.
+// Block masks M and row words V of the source; every later step reads those,
+// never the source again.  One warp per piece of a row, lane = block, two pieces
+// at a time; bound by the source read.
 template <class Src>
-__global__ void __launch_bounds__(kTile, 2) k_bcc_tile(Src src, int *__restrict__ P, uint8_t *__restrict__ M,
-                                                   unsigned *__restrict__ V, BGrid G, int *__restrict__ Pl,
-                                                   int *__restrict__ dirty)
+__global__ void __launch_bounds__(256) k_block_words(Src src, uint8_t *__restrict__ M, unsigned *__restrict__ V, BGrid G,
+                                                     int nt2)
 {
-    __shared__ int L[kTile];
+    const int lane = threadIdx.x & 31, pieces = G.b0 * G.b1 * nt2;
+    constexpr int NP = 2;
+    [[maybe_unused]] ByteRange range;
+    for (int base = NP * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); base < pieces;
+         base += NP * ((gridDim.x * blockDim.x) >> 5)) {
+        unsigned m[NP];
+        int b[NP];
+#pragma unroll
+        for (int q = 0; q < NP; q++) {
+            const int row = (int)fdiv((unsigned)(base + q), G.qt), c0 = (int)fdiv((unsigned)row, G.q1), c1 = row - c0 * G.b1,
+                      c2 = (base + q - row * nt2) * kT2 + lane;
+            b[q] = base + q < pieces && c2 < G.b2 ? row * G.b2 + c2 : -1;
+            m[q] = 0;
+            if constexpr (std::is_same<Src, SrcImg>::value) {
+                unsigned w[2] = {0u, 0u};
+                if (b[q] >= 0)
+                    m[q] = block_mask(src, G, c0, c1, c2, w);
+                range.add(w);
+            } else if (b[q] >= 0) {
+                m[q] = block_mask(src, G, c0, c1, c2);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < NP; q++) {
+            if (b[q] >= 0)
+                M[b[q]] = (uint8_t)m[q];
+            unsigned mine = 0;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const unsigned w = __ballot_sync(0xffffffffu, (m[q] >> i) & 1u);
+                mine = lane == i ? w : mine;
+            }
+            if (lane < 8 && base + q < pieces)
+                V[(long long)(base + q) * 8 + lane] = mine;
+        }
+    }
+    if constexpr (std::is_same<Src, SrcImg>::value)
+        if (src.range)
+            range.flush(src.range);
+}
+
+// Phase 1: a shared-memory union-find of the tile's row words whose roots are
+// the smallest block index of each tile-local part.  Thread 4 r + q makes the
+// pairs of row r with its neighbouring row q, then looks up the parents of its
+// eight blocks of row r.
+// With R, the tile-local roots are also kept as bits (one word per 32 blocks of
+// a row): phase 2 only writes the parents of tile roots, so those bits restore
+// the parents of a tile that has not changed (dirty: per tile, cleared here).
+// A step is a few dependent loads of shared memory, so what counts is the
+// tiles in flight: 128 threads a tile keep a dozen of them on an SM.  With the
+// masks read and a thread per block (two tiles in flight) this took 2.85 ms at
+// 1024^3 (now 0.84 ms for k_block_words and 0.61 ms here), and restoring
+// unchanged tiles from a copy of the parents 0.14 ms a radius of the 512^3
+// drainage (now 0.03 ms).
+constexpr int kTileThreads = 4 * kT0 * kT1;
+
+__global__ void __launch_bounds__(kTileThreads) k_bcc_tile(const unsigned *__restrict__ V, int *__restrict__ P, BGrid G,
+                                                        unsigned *__restrict__ R, int *__restrict__ dirty)
+{
+    __shared__ __align__(16) int L[kTile];
     __shared__ __align__(16) unsigned s_v[kT0 * kT1 * 8];
     const TileId T;
-    const int t = threadIdx.x, r = t / kT2, lane = t % kT2; // row r = a * kT1 + b
-    const int c0 = T.ti * kT0 + r / kT1, c1 = T.tj * kT1 + r % kT1, c2 = T.tk * kT2 + lane;
-    const bool inside = c0 < G.b0 && c1 < G.b1 && c2 < G.b2;
-    const int bidx = (c0 * G.b1 + c1) * G.b2 + c2;
+    const int t = threadIdx.x, r = t >> 2, q = t & 3, a = r / kT1, b = r % kT1;
+    const int c0 = T.ti * kT0 + a, c1 = T.tj * kT1 + b;
+    const bool in_row = c0 < G.b0 && c1 < G.b1;
+    const int row = c0 * G.b1 + c1, piece = row * T.nt2 + T.tk, x0 = row * G.b2 + T.tk * kT2;
     if (dirty && !dirty[T.index()]) {
-        if (inside)
-            P[bidx] = Pl[bidx];
+        if (in_row)
+            for (unsigned w = R[piece] & (0xffu << (8 * q)); w; w &= w - 1) {
+                const int x = x0 + __ffs(w) - 1;
+                P[x] = x;
+            }
         return;
     }
-    unsigned m = 0;
-    if constexpr (std::is_same<Src, SrcImg>::value) {
-        unsigned w[2] = {0u, 0u};
-        if (inside)
-            m = block_mask(src, G, c0, c1, c2, w);
-        if (src.range)
-            note_range(src, w);
-    } else if (inside) {
-        m = block_mask(src, G, c0, c1, c2);
-    }
-    RowBits row;
+    reinterpret_cast<uint2 *>(s_v)[t] =
+        in_row ? *reinterpret_cast<const uint2 *>(V + (long long)piece * 8 + 2 * q) : make_uint2(0u, 0u);
 #pragma unroll
-    for (int i = 0; i < 8; i++)
-        row.v[i] = __ballot_sync(0xffffffffu, (m >> i) & 1u);
-    const unsigned cz = row.runs();
-    const int head = run_head(cz, lane);
-    L[t] = m ? r * kT2 + head : -1;
-    if (lane < 2) {
-        const uint4 w = lane ? make_uint4(row.v[4], row.v[5], row.v[6], row.v[7])
-                             : make_uint4(row.v[0], row.v[1], row.v[2], row.v[3]);
-        reinterpret_cast<uint4 *>(s_v)[r * 2 + lane] = w;
-        if (c0 < G.b0 && c1 < G.b1)
-            reinterpret_cast<uint4 *>(V + row_word(G, c0, c1, T.tk, T.nt2))[lane] = w;
+    for (int i = 0; i < kTile / (4 * kTileThreads); i++) {
+        const int e = 4 * (t + i * kTileThreads);
+        *reinterpret_cast<int4 *>(L + e) = make_int4(e, e + 1, e + 2, e + 3);
     }
     __syncthreads();
-    if (t < kT0 * kT1 * 4) {
-        const int rr = t >> 2, q = t & 3, a = rr / kT1, b = rr % kT1, d0 = row_d0(q), d1 = row_d1(q);
-        if (a + d0 >= 0 && b + d1 >= 0 && b + d1 < kT1) {
-            const int rn = rr + d0 * kT1 + d1;
-            const RowBits own = row_bits(s_v + rr * 8), nb = row_bits(s_v + rn * 8);
-            unsigned em, e0, ep;
-            row_pairs(q, own, nb, nullptr, nullptr, em, e0, ep);
-            if (q > 0 && a > 0) {
-                // where the block above and a further neighbour are both full,
-                // they touch each other and that union is theirs
-                const RowBits up = row_bits(s_v + (rr - kT1) * 8);
-                const unsigned centre = (own.even(0x0Fu) | own.odd(0x0Fu)) & up.full(), f = nb.full();
-                e0 &= ~(centre & f);
-                em &= ~(centre & (f << 1));
-                ep &= ~(centre & (f >> 1));
-            }
-            const unsigned ca = own.runs(), cb = nb.runs();
-            row_reduce(ca, cb, em, e0, ep);
-            while (em | e0 | ep) {
-                const int dz = e0 ? 0 : em ? -1 : 1;
-                const unsigned e = e0 ? e0 : em ? em : ep;
-                const int c = __ffs(e) - 1;
-                const unsigned bit = e & (0u - e);
-                e0 &= ~(dz == 0 ? bit : 0u);
-                em &= ~(dz < 0 ? bit : 0u);
-                ep &= ~(dz > 0 ? bit : 0u);
-                sunite(L, rr * kT2 + run_head(ca, c), rn * kT2 + run_head(cb, c + dz));
-            }
+    const RowBits own = row_bits(s_v + r * 8);
+    const unsigned ca = own.runs();
+    const int d0 = row_d0(q), d1 = row_d1(q);
+    if (a + d0 >= 0 && b + d1 >= 0 && b + d1 < kT1) {
+        const int rn = r + d0 * kT1 + d1;
+        const RowBits nb = row_bits(s_v + rn * 8);
+        unsigned em, e0, ep;
+        row_pairs(q, own, nb, nullptr, nullptr, em, e0, ep);
+        if (q > 0 && a > 0) {
+            // where the block above and a further neighbour are both full,
+            // they touch each other and that union is theirs
+            const RowBits up = row_bits(s_v + (r - kT1) * 8);
+            const unsigned centre = (own.even(0x0Fu) | own.odd(0x0Fu)) & up.full(), f = nb.full();
+            e0 &= ~(centre & f);
+            em &= ~(centre & (f << 1));
+            ep &= ~(centre & (f >> 1));
+        }
+        const unsigned cb = nb.runs();
+        row_reduce(ca, cb, em, e0, ep);
+        while (em | e0 | ep) {
+            const int dz = e0 ? 0 : em ? -1 : 1;
+            const unsigned e = e0 ? e0 : em ? em : ep;
+            const int c = __ffs(e) - 1;
+            const unsigned bit = e & (0u - e);
+            e0 &= ~(dz == 0 ? bit : 0u);
+            em &= ~(dz < 0 ? bit : 0u);
+            ep &= ~(dz > 0 ? bit : 0u);
+            sunite(L, r * kT2 + run_head(ca, c), rn * kT2 + run_head(cb, c + dz));
         }
     }
     __syncthreads();
-    int root = -1;
-    if (m && head == lane)
-        root = sfind(L, t);
-    root = __shfl_sync(0xffffffffu, root, head);
-    if (inside) {
-        if constexpr (!std::is_same<Src, SrcMask>::value)
-            M[bidx] = (uint8_t)m;
-        int out = -1;
-        if (m) {
-            const int ra = root / (kT1 * kT2), rb = (root / kT2) % kT1, rc = root % kT2;
-            out = ((T.ti * kT0 + ra) * G.b1 + T.tj * kT1 + rb) * G.b2 + T.tk * kT2 + rc;
+    if (in_row) {
+        const unsigned some = own.zlo() | own.zhi();
+        int out[8], head = -1, root = -1, roots = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int c = 8 * q + i;
+            out[i] = -1;
+            if ((some >> c) & 1u) {
+                const int h = run_head(ca, c);
+                if (h != head) {
+                    head = h;
+                    const int l = sfind(L, r * kT2 + h);
+                    roots |= (l == r * kT2 + c) << i;
+                    const int ra = l / (kT1 * kT2), rb = (l / kT2) % kT1, rc = l % kT2;
+                    root = ((T.ti * kT0 + ra) * G.b1 + T.tj * kT1 + rb) * G.b2 + T.tk * kT2 + rc;
+                }
+                out[i] = root;
+            }
         }
-        P[bidx] = out;
-        if (Pl)
-            Pl[bidx] = out;
+        const int left = G.b2 - T.tk * kT2 - 8 * q; // blocks of the row from here
+        int *dst = P + x0 + 8 * q;
+        if (left >= 8 && !(G.b2 & 3)) {
+            reinterpret_cast<int4 *>(dst)[0] = make_int4(out[0], out[1], out[2], out[3]);
+            reinterpret_cast<int4 *>(dst)[1] = make_int4(out[4], out[5], out[6], out[7]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                if (i < left)
+                    dst[i] = out[i];
+        }
+        if (R)
+            reinterpret_cast<uint8_t *>(R + piece)[q] = (uint8_t)roots;
     }
     if (dirty && t == 0)
         dirty[T.index()] = 0;
@@ -1682,7 +1734,10 @@ __global__ void k_bcc_twins(const uint8_t *__restrict__ M, int *P, BGrid G, Twin
             continue;
         const int ba = (int)(((c[0] >> 1) * G.b1 + (c[1] >> 1)) * G.b2 + (c[2] >> 1));
         const int bb = (int)(((t[0] >> 1) * G.b1 + (t[1] >> 1)) * G.b2 + (t[2] >> 1));
-        unite(P, ba, bb, err);
+        // from their parents: only the parents of tile roots are written
+        const int pa = ld(P + ba), pb = ld(P + bb);
+        if (pa != pb)
+            unite(P, pa, pb, err);
     }
 }
 
@@ -1708,38 +1763,6 @@ __device__ __forceinline__ unsigned eq2(unsigned pair, unsigned v)
 __global__ void k_bcc_mark(const uint8_t *__restrict__ M, const int *__restrict__ P, BGrid G, Box bx,
                            uint8_t *mark, uint8_t bit, int *err)
 {
-    long long lo[3], nbk[3];
-    for (int d = 0; d < 3; d++) {
-        lo[d] = bx.lo[d] >> 1;
-        nbk[d] = ((bx.hi[d] + 1) >> 1) - lo[d];
-    }
-    const long long n = nbk[0] * nbk[1] * nbk[2];
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
-         q += (long long)gridDim.x * blockDim.x) {
-        const int c2 = (int)(lo[2] + q % nbk[2]), c1 = (int)(lo[1] + (q / nbk[2]) % nbk[1]),
-                  c0 = (int)(lo[0] + q / (nbk[2] * nbk[1]));
-        const int b = (c0 * G.b1 + c1) * G.b2 + c2;
-        const unsigned inbox = spread_x(in2(2 * c0, bx.lo[0], bx.hi[0])) & spread_y(in2(2 * c1, bx.lo[1], bx.hi[1])) &
-                               spread_z(in2(2 * c2, bx.lo[2], bx.hi[2]));
-        if (!(M[b] & inbox))
-            continue;
-        int p = ld(P + b);
-        if (p >= 0)
-            p = find_root(P, p, err);
-        if (p >= 0 && !(mark[p] & bit))
-            atomicOr((unsigned int *)(mark + (p & ~3)), (unsigned int)bit << (8 * (p & 3)));
-    }
-}
-
-// k_bcc_mark for two block union-finds of the same grid at once
-// (blockIdx.y picks the set), marking the same face box.
-__global__ void k_bcc_mark2(const uint8_t *__restrict__ Ma, const int *__restrict__ Pa, uint8_t *mark_a,
-                            const uint8_t *__restrict__ Mb, const int *__restrict__ Pb, uint8_t *mark_b, BGrid G,
-                            Box bx, uint8_t bit, int *err)
-{
-    const uint8_t *M = blockIdx.y ? Mb : Ma;
-    const int *P = blockIdx.y ? Pb : Pa;
-    uint8_t *mark = blockIdx.y ? mark_b : mark_a;
     long long lo[3], nbk[3];
     for (int d = 0; d < 3; d++) {
         lo[d] = bx.lo[d] >> 1;
@@ -1832,9 +1855,8 @@ __host__ __device__ inline const uint8_t *src_elem(const SrcStep &s) { return s.
 template <class Src>
 static double src_bytes(const Src &src, long long n, long long nb)
 {
-    return std::is_same<Src, SrcMask>::value ? (double)nb : (double)n * sizeof(*src_elem(src));
+    return (double)n * sizeof(*src_elem(src));
 }
-__host__ __device__ inline const uint8_t *src_elem(const SrcMask &s) { return s.M; }
 
 static BGrid bgrid_of(const int64_t *shape)
 {
@@ -1847,6 +1869,7 @@ static BGrid bgrid_of(const int64_t *shape)
     G.b2 = (G.s2 + 1) / 2;
     G.q2 = fastdiv_of((unsigned)G.b2);
     G.q1 = fastdiv_of((unsigned)G.b1);
+    G.qt = fastdiv_of((unsigned)((G.b2 + kT2 - 1) / kT2));
     return G;
 }
 
@@ -1862,18 +1885,31 @@ static dim3 bcc_tiles(const BGrid &G)
                 (unsigned)((G.b0 + kT0 - 1) / kT0));
 }
 
-// Phase 1 of the block union-find (k_bcc_tile); V: bcc_row_bytes.
-template <class Src>
-static int bcc_tile_phase(const Src &src, const int64_t *shape, int *P, uint8_t *M, unsigned *V, cudaStream_t st,
-                          int *Pl = nullptr, int *dirty = nullptr)
+// Phase 1 from the row words; dirty: of the flagged tiles alone, the others'
+// parents being restored (R of an earlier call).
+static int bcc_tiles_run(const int64_t *shape, int *P, const unsigned *V, unsigned *R, int *dirty, cudaStream_t st)
 {
     const BGrid G = bgrid_of(shape);
-    const int nb = G.b0 * G.b1 * G.b2;
     const int ps__ = prof_begin("k_bcc_tile", st);
-    k_bcc_tile<Src><<<bcc_tiles(G), kTile, 0, st>>>(src, P, M, V, G, Pl, dirty);
-    prof_end(ps__, src_bytes(src, (long long)shape[0] * shape[1] * shape[2], nb) + (double)nb * 6, st);
+    k_bcc_tile<<<bcc_tiles(G), kTileThreads, 0, st>>>(V, P, G, R, dirty);
+    prof_end(ps__, (double)G.b0 * G.b1 * G.b2 * (dirty ? 1.0 / 8 : 5.0), st);
     PMG_CHECK_LAUNCH();
     return PMG_OK;
+}
+
+// Masks, row words (V: bcc_row_bytes) and phase 1 of the block union-find.
+template <class Src>
+static int bcc_tile_phase(const Src &src, const int64_t *shape, int *P, uint8_t *M, unsigned *V, cudaStream_t st,
+                          unsigned *R = nullptr)
+{
+    const BGrid G = bgrid_of(shape);
+    const int nb = G.b0 * G.b1 * G.b2, nt2 = (G.b2 + kT2 - 1) / kT2;
+    const long long pieces = (long long)G.b0 * G.b1 * nt2;
+    const int ps__ = prof_begin("k_block_words", st);
+    k_block_words<Src><<<grid_for((pieces + 1) / 2 * 32, 256, 152LL * 64), 256, 0, st>>>(src, M, V, G, nt2);
+    prof_end(ps__, src_bytes(src, (long long)shape[0] * shape[1] * shape[2], nb) + (double)nb * 2, st);
+    PMG_CHECK_LAUNCH();
+    return bcc_tiles_run(shape, P, V, R, nullptr, st);
 }
 
 // Phase 2 and the periodic seams (twins).
@@ -1904,13 +1940,13 @@ static int bcc_cross_phase(const int64_t *shape, const int32_t *bc, const int32_
 // index of the component), -1 for empty blocks; M[b] = block mask.
 template <class Src>
 static int bcc_build(const Src &src, const int64_t *shape, const int32_t *bc, const int32_t *pad, bool twins,
-                     int *P, uint8_t *M, int *err, cudaStream_t st, int *Pl = nullptr, int *dirty = nullptr,
-                     unsigned *Vkeep = nullptr)
+                     int *P, uint8_t *M, int *err, cudaStream_t st, unsigned *Vkeep = nullptr,
+                     unsigned *R = nullptr)
 {
     unsigned *V = Vkeep;
     if (!V)
         PMG_TRY(scratch_alloc((void **)&V, bcc_row_bytes(bgrid_of(shape)), st));
-    int s = bcc_tile_phase(src, shape, P, M, V, st, Pl, dirty);
+    int s = bcc_tile_phase(src, shape, P, M, V, st, R);
     if (s == PMG_OK)
         s = bcc_cross_phase(shape, bc, pad, twins, P, M, V, err, st);
     if (!Vkeep)
@@ -2042,158 +2078,214 @@ int select_run_erode(const uint16_t *E, int T, void *out, const int64_t *shape, 
 // Along a drainage curve two selected sets only ever grow: the eroded pore
 // space (its threshold falls with the radius) and the non-wetting phase (the
 // update turns wetting voxels non-wetting, never back).  Components of a
-// growing set only merge, so after one full block union-find a step re-reads
-// the block masks, lists the blocks whose mask grew, and unites each of them
-// with every touching neighbour; a pair of blocks that starts to touch always
-// has a grown member, and every other block keeps its parent.  The parents
-// keep pointing to smaller indices, so roots stay the smallest block of each
-// component and the flattened parents, marks and selection are those of a
-// full union-find of the same set.
+// growing set only merge, so after one full block union-find a step unites the
+// touching pairs with a block that changed (N, one bit per block); every other
+// pair is in one component already.  And a block once connected to the inlet
+// stays so: where the step's selection (k_pair_rows) takes the connected blocks
+// out of U (one bit per block), later steps neither look up their roots nor
+// unite two of them.  What a step keeps true of any two touching blocks is
+// "same component, or both connected": an equivalence, so pairs that the row
+// reduction leaves out follow from those that it keeps.
 
-// New masks; a block whose mask changed is listed (warp-aggregated append)
-// and, if it was empty, becomes its own root.  A mask that lost voxels is an
-// error (code 3): the set did not grow.
-template <class Src>
-__global__ void k_grow_masks(Src src, uint8_t *__restrict__ M, int *__restrict__ P, BGrid G, int *list,
-                             int *count, int *err)
-{
-    const int nb = G.b0 * G.b1 * G.b2;
-    const int lane = threadIdx.x & 31;
-    for (int base = blockIdx.x * blockDim.x; base < nb; base += gridDim.x * blockDim.x) {
-        const int b = base + threadIdx.x;
-        bool changed = false;
-        if (b < nb) {
-            // the old mask and the source are loaded independently
-            int c2, c0, c1;
-            G.coords(b, c0, c1, c2);
-            const unsigned old = M[b];
-            const unsigned m = block_mask(src, G, c0, c1, c2);
-            if (m != old) {
-                if (old & ~m)
-                    atomicExch(err, 3);
-                M[b] = (uint8_t)m;
-                if (!old)
-                    P[b] = b;
-                changed = true;
-            }
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, changed);
-        if (bal) {
-            int pos = 0;
-            if (lane == 0)
-                pos = atomicAdd(count, __popc(bal));
-            pos = __shfl_sync(0xffffffffu, pos, 0);
-            if (changed)
-                list[pos + __popc(bal & ((1u << lane) - 1u))] = b;
-        }
-    }
-}
-
-
-// One warp per listed block, one lane per neighbour (lanes 0-25): every lane
-// loads its neighbour's mask and parent at once.  The parents were flattened
-// after the previous step, so a touching neighbour whose parent equals the
-// block's starting parent is already in its component; of the others, one
-// lane per distinct parent unites (neighbours with one parent are in one
-// component already).
-// One listed block b of a growing set: its lane's neighbour (q, d) and, once
-// per distinct neighbour parent, the union.
-__device__ __forceinline__ void grow_unite_block(int *P, const uint8_t *__restrict__ M, const BGrid &G, int b,
-                                                 int lane, int d0, int d1, int d2, unsigned tself, unsigned tnb,
-                                                 int *err)
-{
-    int c2, c0, c1;
-    G.coords(b, c0, c1, c2);
-    const unsigned m = M[b];
-    const int pb = ld(P + b);
-    const int a0 = c0 + d0, a1 = c1 + d1, a2 = c2 + d2;
-    const bool valid = (m & tself) && a0 >= 0 && a1 >= 0 && a2 >= 0 && a0 < G.b0 && a1 < G.b1 && a2 < G.b2;
-    const int o = (a0 * G.b1 + a1) * G.b2 + a2;
-    unsigned mo = 0;
-    int po = -1;
-    if (valid) {
-        mo = M[o];
-        po = ld(P + o);
-    }
-    const bool need = (mo & tnb) && po != pb;
-    const unsigned needs = __ballot_sync(0xffffffffu, need);
-    if (!needs)
-        return;
-    const unsigned same = __match_any_sync(0xffffffffu, need ? po : -2 - lane);
-    if (need && (__ffs(same & needs) - 1) == lane)
-        unite(P, b, o, err);
-}
-
-// A set's listed blocks: step k's precomputed list (off) or the list a mask
-// pass (or the drainage update) filled (count).
-struct UniteList {
-    int *P;
-    const uint8_t *M;
-    const int *list, *count, *off;
-    __device__ __forceinline__ int size(const int *&l) const
-    {
-        if (off) {
-            l = list + off[0];
-            return off[1] - off[0];
-        }
-        l = list;
-        return *count;
-    }
+struct GrowWords {
+    unsigned *V, *N, *U;
 };
 
-// One warp per listed block of set A, then of set B (two growing sets of the
-// same grid in one launch: their dependent loads overlap), one lane per
-// neighbour (lanes 0-25): every lane loads its neighbour's mask and parent
-// at once.  The parents were flattened after the previous step, so a
-// touching neighbour whose parent equals the block's starting parent is
-// already in its component; of the others, one lane per distinct parent
-// unites (neighbours with one parent are in one component already).
-__global__ void k_grow_unite2(UniteList A, UniteList B, BGrid G, int *err, unsigned long long *units)
+// A block's new mask m: masks, row words, the changed and unconnected bits and,
+// for a block that was empty, its own root.  A mask that lost voxels is an
+// error (code 3): the set did not grow.
+__device__ __forceinline__ void grow_block(const BGrid &G, int b, int c0, int c1, int c2, unsigned old, unsigned m,
+                                           uint8_t *M, int *P, const GrowWords &W, int nt2, int *err)
 {
-    const int *la = nullptr, *lb = nullptr;
-    const int ca = A.P ? A.size(la) : 0, cb = B.P ? B.size(lb) : 0;
-    if (units && blockIdx.x == 0 && threadIdx.x == 0 && ca + cb > 0)
-        atomicAdd(units, (unsigned long long)(ca + cb));
-    const int lane = threadIdx.x & 31;
-    const int q = lane < 13 ? lane : lane + 1; // offset code (d0 + 1) * 9 + (d1 + 1) * 3 + d2 + 1, 13 skipped
-    const int d0 = q / 9 - 1, d1 = (q / 3) % 3 - 1, d2 = q % 3 - 1;
-    const unsigned tself = lane < 26 ? touch_bits(d0, d1, d2) : 0u, tnb = touch_bits(-d0, -d1, -d2);
-    const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long it = warp; it < (long long)ca + cb; it += nwarps) {
-        if (it < ca)
-            grow_unite_block(A.P, A.M, G, la[it], lane, d0, d1, d2, tself, tnb, err);
-        else
-            grow_unite_block(B.P, B.M, G, lb[it - ca], lane, d0, d1, d2, tself, tnb, err);
+    if (m == old)
+        return;
+    if (old & ~m)
+        atomicExch(err, 3);
+    M[b] = (uint8_t)m;
+    const long long piece = row_word(G, c0, c1, c2 / kT2, nt2) / 8;
+    const unsigned bit = 1u << (c2 % kT2);
+    if (!old) {
+        P[b] = b;
+        atomicOr(W.U + piece, bit);
+    }
+    atomicOr(W.N + piece, bit);
+    for (unsigned delta = m & ~old; delta; delta &= delta - 1)
+        atomicOr(W.V + piece * 8 + __ffs(delta) - 1, bit);
+}
+
+template <class Src>
+__global__ void k_grow_masks(Src src, uint8_t *M, int *P, GrowWords W, BGrid G, int nt2,
+                             int *err)
+{
+    const int nb = G.b0 * G.b1 * G.b2;
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
+        // the old mask and the source are loaded independently
+        int c2, c0, c1;
+        G.coords(b, c0, c1, c2);
+        const unsigned old = M[b];
+        grow_block(G, b, c0, c1, c2, old, block_mask(src, G, c0, c1, c2), M, P, W, nt2, err);
     }
 }
 
-// A single set: set B empty.
-__global__ void k_grow_unite(int *P, const uint8_t *__restrict__ M, BGrid G, const int *__restrict__ list,
-                             const int *__restrict__ count, const int *__restrict__ off, int *err,
+// Listed blocks (steps known in advance) take their masks from the source.
+template <class Src>
+__global__ void k_grow_apply(Src src, uint8_t *M, int *P, GrowWords W, BGrid G, int nt2,
+                             const int *__restrict__ list, const int *__restrict__ off, int *err,
                              unsigned long long *units)
 {
-    UniteList A{P, M, list, count, off};
-    const int *la = nullptr;
-    const int ca = A.size(la);
-    if (units && blockIdx.x == 0 && threadIdx.x == 0 && ca > 0)
-        atomicAdd(units, (unsigned long long)ca);
-    const int lane = threadIdx.x & 31;
-    const int q = lane < 13 ? lane : lane + 1;
-    const int d0 = q / 9 - 1, d1 = (q / 3) % 3 - 1, d2 = q % 3 - 1;
-    const unsigned tself = lane < 26 ? touch_bits(d0, d1, d2) : 0u, tnb = touch_bits(-d0, -d1, -d2);
-    const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long it = warp; it < ca; it += nwarps)
-        grow_unite_block(P, M, G, la[it], lane, d0, d1, d2, tself, tnb, err);
+    const int a = off[0], cnt = off[1] - a;
+    if (units && blockIdx.x == 0 && threadIdx.x == 0 && cnt > 0)
+        atomicAdd(units, (unsigned long long)cnt);
+    for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < cnt; it += gridDim.x * blockDim.x) {
+        const int b = list[a + it];
+        int c2, c0, c1;
+        G.coords(b, c0, c1, c2);
+        const unsigned old = M[b];
+        grow_block(G, b, c0, c1, c2, old, block_mask(src, G, c0, c1, c2), M, P, W, nt2, err);
+    }
 }
+
+// After the full union-find: every block unconnected, none changed.
+__global__ void k_grow_start(GrowWords W, int pieces)
+{
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < pieces; q += gridDim.x * blockDim.x) {
+        const RowBits r = row_bits(W.V + (long long)q * 8);
+        W.U[q] = r.zlo() | r.zhi();
+        W.N[q] = 0u;
+    }
+}
+
+// The unions of a step, of one or two sets of the same grid (blockIdx.y): the
+// touching pairs of a row piece (32 blocks) within the row and with the four
+// earlier neighbouring rows that have a changed block and an unconnected one.
+// A thread per piece and neighbouring row (and one for the pairs within the
+// row) lists them: the changed and unconnected words, 1/8 of the row words, tell
+// most of the threads that there are none.  k_grow_join then unites them, a
+// thread per pair: a union is a chain of dependent loads, so it is taken off
+// the threads that are mostly idle.
+// Bound by those chains.  A warp per grown block with a lane per neighbour spent
+// 0.28 ms a radius of the 512^3 drainage on three dependent loads per block and
+// on unions of blocks that were in one component already, a thread per piece and
+// row that united its own pairs 0.15 ms with half as many pairs (0.60 ms where
+// most pairs were new); now 0.09 ms for the list and 0.10 ms for the unions.
+struct RowSet {
+    int *P;
+    GrowWords W;
+    int2 *list;
+    int *count;
+    int cap; // pairs beyond it are united at once
+};
+constexpr int kGrowPieces = 32, kGrowThreads = 5 * kGrowPieces;
+
+__global__ void __launch_bounds__(kGrowThreads) k_grow_pairs(RowSet A, RowSet B, BGrid G, int nt2, int *err)
+{
+    const RowSet &R = blockIdx.y ? B : A;
+    const GrowWords W = R.W;
+    const int q = threadIdx.x / kGrowPieces, piece = blockIdx.x * kGrowPieces + threadIdx.x % kGrowPieces;
+    const int row = (int)fdiv((unsigned)piece, G.qt), tk = piece - row * nt2;
+    const int c0 = (int)fdiv((unsigned)row, G.q1), c1 = row - c0 * G.b1;
+    // q < 4: neighbouring row q; q == 4: the row itself (its blocks before)
+    const int d0 = q < 4 ? row_d0(q) : 0, d1 = q < 4 ? row_d1(q) : 0;
+    bool work = piece < G.b0 * G.b1 * nt2 && c0 + d0 >= 0 && c1 + d1 >= 0 && c1 + d1 < G.b1;
+    const int o = piece + (d0 * G.b1 + d1) * nt2;
+    unsigned n = 0, u = 0, nn = 0, un = 0, nm = 0, um = 0, n1 = 0, u1 = 0;
+    if (work) {
+        n = W.N[piece];
+        u = W.U[piece];
+        nn = W.N[o];
+        un = W.U[o];
+        if (tk > 0) {
+            nm = W.N[o - 1];
+            um = W.U[o - 1];
+        }
+        if (q < 4 && tk + 1 < nt2) {
+            n1 = W.N[o + 1];
+            u1 = W.U[o + 1];
+        }
+        work = (n | nn | nm | n1) && (u | un | um | u1);
+    }
+    if (!__any_sync(0xffffffffu, work))
+        return;
+    // bits of the pairs with the blocks before, beside and after
+    unsigned em = 0, e0 = 0, ep = 0;
+    if (work) {
+        const RowBits own = row_bits(W.V + (long long)piece * 8);
+        const unsigned cz = own.runs();
+        if (q == 4) {
+            em = cz;
+            if (tk > 0)
+                em |= own.zlo() & (row_bits(W.V + (long long)(piece - 1) * 8).zhi() >> 31);
+        } else {
+            const unsigned *nv = W.V + (long long)o * 8;
+            const RowBits nb = row_bits(nv);
+            RowBits before = {}, after = {};
+            if (tk > 0)
+                before = row_bits(nv - 8);
+            if (tk + 1 < nt2)
+                after = row_bits(nv + 8);
+            row_pairs(q, own, nb, &before, &after, em, e0, ep);
+            row_reduce(cz, nb.runs(), em, e0, ep);
+        }
+        em &= (n | nn << 1 | nm >> 31) & (u | un << 1 | um >> 31);
+        e0 &= (n | nn) & (u | un);
+        ep &= (n | nn >> 1 | n1 << 31) & (u | un >> 1 | u1 << 31);
+    }
+    // the warp's pairs take consecutive entries
+    const int lane = threadIdx.x & 31, mine = __popc(em) + __popc(e0) + __popc(ep);
+    int at = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, at, d);
+        at += lane >= d ? v : 0;
+    }
+    int first = 0;
+    if (lane == 31 && at)
+        first = atomicAdd(R.count, at);
+    at += __shfl_sync(0xffffffffu, first, 31) - mine;
+    const int x = row * G.b2 + tk * kT2, y = x + (d0 * G.b1 + d1) * G.b2;
+    while (em | e0 | ep) {
+        const int dz = e0 ? 0 : em ? -1 : 1;
+        const unsigned f = e0 ? e0 : em ? em : ep;
+        const int c = __ffs(f) - 1;
+        const unsigned bit = f & (0u - f);
+        e0 &= ~(dz == 0 ? bit : 0u);
+        em &= ~(dz < 0 ? bit : 0u);
+        ep &= ~(dz > 0 ? bit : 0u);
+        if (at < R.cap)
+            R.list[at] = make_int2(x + c, y + c + dz);
+        else
+            unite(R.P, x + c, y + c + dz, err);
+        at++;
+    }
+}
+
+// The listed pairs united; the roots that a block of threads joins are mostly
+// the same few (CrossSet).
+__global__ void __launch_bounds__(256) k_grow_join(RowSet A, RowSet B, int *err)
+{
+    __shared__ CrossSet S;
+    const RowSet &R = blockIdx.y ? B : A;
+    const int n = min(*R.count, R.cap);
+    if ((int)(blockIdx.x * blockDim.x) >= n)
+        return;
+    S.init();
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const int2 e = R.list[k];
+        S.join(R.P, e.x, e.y, err);
+    }
+}
+
+static int row_pieces(const BGrid &G) { return G.b0 * G.b1 * ((G.b2 + kT2 - 1) / kT2); }
+
+static size_t piece_bytes(const BGrid &G) { return ((size_t)row_pieces(G) * 4 + 255) & ~(size_t)255; }
 
 size_t grow_sel_bytes(const int64_t *shape)
 {
     const BGrid G = bgrid_of(shape);
     const size_t nb = (size_t)G.b0 * G.b1 * G.b2;
     const size_t a = (nb + 255) & ~(size_t)255;
-    return a * 4 + a + a + a * 4 + 256;
+    // parents, masks, marks, row words, changed and unconnected words, pairs
+    return a * 4 + a + a + bcc_row_bytes(G) + 2 * piece_bytes(G) + a * 4 + 256;
 }
 
 void grow_sel_init(GrowSel &g, void *mem, const int64_t *shape)
@@ -2208,85 +2300,109 @@ void grow_sel_init(GrowSel &g, void *mem, const int64_t *shape)
     p += a;
     g.mark = (uint8_t *)p;
     p += a;
-    g.list = (int *)p;
-    p += a * 4;
-    g.count = (int *)p;
+    g.V = (unsigned *)p;
+    p += bcc_row_bytes(G);
+    g.N = (unsigned *)p;
+    p += piece_bytes(G);
+    g.U = (unsigned *)p;
+    p += piece_bytes(G);
+    g.pairs = (int2 *)p;
+    g.npairs = (int *)(p + a * 4);
     g.built = false;
 }
 
-// One step of a growing selection up to the marks: the full block union-find
-// the first time, afterwards the grown blocks only.
-// Listed blocks take their masks from the source (steps known in advance).
+static GrowWords words(const GrowSel &g) { return GrowWords{g.V, g.N, g.U}; }
+
+// The set's first step: the full block union-find.
 template <class Src>
-__global__ void k_grow_apply(Src src, uint8_t *__restrict__ M, int *__restrict__ P, BGrid G,
-                             const int *__restrict__ list, const int *__restrict__ off, int *err,
-                             unsigned long long *units)
+static int grow_build(GrowSel &g, const Src &src, const int64_t *shape, const int32_t *bc, const int32_t *pad, int *err,
+                      cudaStream_t st)
 {
-    const int a = off[0], cnt = off[1] - a;
-    if (units && blockIdx.x == 0 && threadIdx.x == 0 && cnt > 0)
-        atomicAdd(units, (unsigned long long)cnt);
-    for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < cnt; it += gridDim.x * blockDim.x) {
-        const int b = list[a + it];
-        int c2, c0, c1;
-        G.coords(b, c0, c1, c2);
-        const unsigned old = M[b];
-        const unsigned m = block_mask(src, G, c0, c1, c2);
-        if (old & ~m)
-            atomicExch(err, 3);
-        M[b] = (uint8_t)m;
-        if (!old)
-            P[b] = b;
-    }
+    PMG_TRY(bcc_build(src, shape, bc, pad, true, g.P, g.M, err, st, g.V));
+    const int pieces = row_pieces(bgrid_of(shape));
+    const int ps__ = prof_begin("k_grow_start", st);
+    k_grow_start<<<grid_for(pieces, 256, 152LL * 16), 256, 0, st>>>(words(g), pieces);
+    prof_end(ps__, (double)pieces * 40, st);
+    PMG_CHECK_LAUNCH();
+    g.stamp = 0;
+    g.built = true;
+    g.pending = false;
+    return PMG_OK;
 }
 
+// The set's masks and row words brought up to date: from its list of step off,
+// or from the source, or (pending) by the producer already.
 template <class Src>
-static int grow_step(GrowSel &g, const Src &src, const int64_t *shape, const int32_t *bc, const int32_t *pad,
-                     const int64_t *inlet_box, const int64_t *outlet_box, int *err, cudaStream_t st,
-                     const int *off = nullptr)
+static int grow_masks(GrowSel &g, const Src &src, const int64_t *shape, const int *off, int *err, cudaStream_t st)
 {
-    PMG_TRY(check_boxes(shape, inlet_box, outlet_box));
-    if (!g.built) {
-        PMG_TRY(bcc_build(src, shape, bc, pad, true, g.P, g.M, err, st));
-        g.built = true;
-        return bcc_marks(shape, inlet_box, outlet_box, g.P, g.M, g.mark, err, st);
-    }
     const BGrid G = bgrid_of(shape);
-    const int nb = G.b0 * G.b1 * G.b2;
-    const long long n = shape[0] * shape[1] * shape[2];
+    const int nb = G.b0 * G.b1 * G.b2, nt2 = (G.b2 + kT2 - 1) / kT2;
     if (off) {
         const int ps__ = prof_begin("k_grow_apply", st);
-        k_grow_apply<Src><<<152 * 8, 256, 0, st>>>(src, g.M, g.P, G, g.ev, off, err, prof_units(kUnitsGrowApply));
+        k_grow_apply<Src><<<152 * 8, 256, 0, st>>>(src, g.M, g.P, words(g), G, nt2, g.ev, off, err,
+                                                   prof_units(kUnitsGrowApply));
         // per listed block: its list entry, eight source elements, mask read
         // and written, parent written
         prof_end_units(ps__, kUnitsGrowApply, 4 + 8 * sizeof(*src_elem(src)) + 2 + 4, st);
-        PMG_CHECK_LAUNCH();
-    } else if (g.pending) {
-        g.pending = false;
-    } else {
-        PMG_CUDA(cudaMemsetAsync(g.count, 0, sizeof(int), st));
+    } else if (!g.pending) {
         const int ps__ = prof_begin("k_grow_masks", st);
-        k_grow_masks<Src><<<grid_for(nb, 256, 152LL * 64), 256, 0, st>>>(src, g.M, g.P, G, g.list, g.count, err);
-        prof_end(ps__, (double)n * sizeof(*src_elem(src)) + (double)nb, st);
-        PMG_CHECK_LAUNCH();
-    }
-    {
-        const int ps__ = prof_begin(g.unite_label, st);
-        k_grow_unite<<<152 * 32, 256, 0, st>>>(g.P, g.M, G, off ? g.ev : g.list, g.count, off, err,
-                                               prof_units(g.unite_units));
-        // per listed block: its list entry, mask and parent, and the masks and
-        // parents of its 26 neighbours
-        if (g.unite_units >= 0)
-            prof_end_units(ps__, g.unite_units, 4 + 5 + 26 * 5, st);
-        else
-            prof_end(ps__, 0.0, st);
+        k_grow_masks<Src><<<grid_for(nb, 256, 152LL * 64), 256, 0, st>>>(src, g.M, g.P, words(g), G, nt2, err);
+        prof_end(ps__, (double)shape[0] * shape[1] * shape[2] * sizeof(*src_elem(src)) + (double)nb, st);
     }
     PMG_CHECK_LAUNCH();
-    if (any_periodic(bc)) {
-        const int ps__ = prof_begin("k_bcc_twins", st);
-        k_bcc_twins<<<grid_for(n, 256, 152LL * 32), 256, 0, st>>>(g.M, g.P, G, make_twins(shape, bc, pad), err);
-        prof_end(ps__, 0.0, st);
-        PMG_CHECK_LAUNCH();
+    g.pending = false;
+    return PMG_OK;
+}
+
+// Unions of one set, or of two in one launch.
+static int grow_rows(GrowSel &a, GrowSel *b, const int64_t *shape, int *err, cudaStream_t st)
+{
+    const BGrid G = bgrid_of(shape);
+    const int nt2 = (G.b2 + kT2 - 1) / kT2, pieces = row_pieces(G), cap = G.b0 * G.b1 * G.b2 / 2;
+    const RowSet A{a.P, words(a), a.pairs, a.npairs, cap}, B = b ? RowSet{b->P, words(*b), b->pairs, b->npairs, cap} : A;
+    const unsigned sets = b ? 2 : 1;
+    PMG_CUDA(cudaMemsetAsync(a.npairs, 0, sizeof(int), st));
+    if (b)
+        PMG_CUDA(cudaMemsetAsync(b->npairs, 0, sizeof(int), st));
+    {
+        const int ps__ = prof_begin("k_grow_pairs", st);
+        k_grow_pairs<<<dim3((unsigned)((pieces + kGrowPieces - 1) / kGrowPieces), sets), kGrowThreads, 0, st>>>(A, B, G,
+                                                                                                            nt2, err);
+        // the changed and the unconnected words (the words of pieces with pairs come on top)
+        prof_end(ps__, (double)pieces * 8 * sets, st);
     }
+    PMG_CHECK_LAUNCH();
+    {
+        const int ps__ = prof_begin("k_grow_join", st);
+        k_grow_join<<<dim3((unsigned)grid_for(cap, 256, 152LL * 4), sets), 256, 0, st>>>(A, B, err);
+        prof_end(ps__, 0.0, st);
+    }
+    PMG_CHECK_LAUNCH();
+    return PMG_OK;
+}
+
+// One step of a growing selection up to the marks.
+template <class Src>
+static int grow_step(GrowSel &g, const Src &src, const int64_t *shape, const int32_t *bc, const int32_t *pad,
+                     const int64_t *inlet_box, const int64_t *outlet_box, int *err, cudaStream_t st)
+{
+    PMG_TRY(check_boxes(shape, inlet_box, outlet_box));
+    if (!g.built) {
+        PMG_TRY(grow_build(g, src, shape, bc, pad, err, st));
+    } else {
+        PMG_TRY(grow_masks(g, src, shape, nullptr, err, st));
+        PMG_TRY(grow_rows(g, nullptr, shape, err, st));
+        PMG_CUDA(cudaMemsetAsync(g.N, 0, piece_bytes(bgrid_of(shape)), st));
+        if (any_periodic(bc)) {
+            const BGrid G = bgrid_of(shape);
+            const long long n = shape[0] * shape[1] * shape[2];
+            const int ps__ = prof_begin("k_bcc_twins", st);
+            k_bcc_twins<<<grid_for(n, 256, 152LL * 32), 256, 0, st>>>(g.M, g.P, G, make_twins(shape, bc, pad), err);
+            prof_end(ps__, 0.0, st);
+            PMG_CHECK_LAUNCH();
+        }
+    }
+    g.stamp = 0; // the marks below are no stamps
     return bcc_marks(shape, inlet_box, outlet_box, g.P, g.M, g.mark, err, st);
 }
 
@@ -2313,133 +2429,181 @@ static SrcErode erode_src(const uint16_t *E, int T, const int64_t *shape, const 
     return src;
 }
 
-constexpr int kPairBatch = 4;
+// Marks by stamp: the roots of the blocks of one or two sets (blockIdx.y) with
+// a voxel in the box get this step's stamp, so that the marks of earlier steps
+// need no clearing.
+struct StampSet {
+    const uint8_t *M;
+    int *P;
+    uint8_t *mark;
+    uint8_t stamp;
+};
 
-// Inlet selections of two growing sets A and B in one pass: out = 1 where A
-// is inlet-connected and, when *b_count > 0, B is inlet-connected too
-// (porosimetry.py:130-148: img_results kept where n_connected == 1 once the
-// phase exists); kept counts A's inlet-connected voxels before the
-// constraint.  Both parent arrays are flattened on the way.
-// BLK: out holds one mask per 2x2x2 block (bit (x * 2 + y) * 2 + z), else
-// one byte per voxel.
-template <bool BLK>
-__global__ void k_grow_pair_select(const uint8_t *__restrict__ MA, int *PA, const uint8_t *__restrict__ markA,
-                                   const uint8_t *__restrict__ MB, int *PB, const uint8_t *__restrict__ markB,
-                                   const unsigned long long *__restrict__ b_count, BGrid G,
-                                   uint8_t *__restrict__ out, unsigned long long *kept, int *err, int *xr)
+__global__ void k_face_stamp(StampSet A, StampSet B, BGrid G, Box bx, int *err)
 {
-    const int nb = G.b0 * G.b1 * G.b2;
+    const StampSet &R = blockIdx.y ? B : A;
+    int lo[3], nbk[3];
+    for (int d = 0; d < 3; d++) {
+        lo[d] = (int)(bx.lo[d] >> 1);
+        nbk[d] = (int)((bx.hi[d] + 1) >> 1) - lo[d];
+    }
+    const int n = nbk[0] * nbk[1] * nbk[2];
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+        const int c2 = lo[2] + q % nbk[2], c1 = lo[1] + (q / nbk[2]) % nbk[1], c0 = lo[0] + q / (nbk[2] * nbk[1]);
+        const int b = (c0 * G.b1 + c1) * G.b2 + c2;
+        const unsigned inbox = spread_x(in2(2 * c0, bx.lo[0], bx.hi[0])) & spread_y(in2(2 * c1, bx.lo[1], bx.hi[1])) &
+                               spread_z(in2(2 * c2, bx.lo[2], bx.hi[2]));
+        if (!(R.M[b] & inbox))
+            continue;
+        int p = ld(R.P + b);
+        if (p >= 0 && p != b)
+            p = find_root(R.P, p, err);
+        if (p >= 0 && R.mark[p] != R.stamp)
+            R.mark[p] = R.stamp;
+    }
+}
+
+// The next stamp of a mark array (cleared when the stamps run out).
+static int next_stamp(uint8_t *mark, int &stamp, size_t nb, cudaStream_t st)
+{
+    if (stamp == 0 || stamp == 255) {
+        PMG_CUDA(cudaMemsetAsync(mark, 0, nb, st));
+        stamp = 0;
+    }
+    stamp++;
+    return PMG_OK;
+}
+
+static int face_stamps(const int64_t *box, const int64_t *shape, StampSet A, const StampSet *B, int *err,
+                       cudaStream_t st)
+{
+    if (!box || box[0] < 0)
+        return PMG_OK;
+    Box b;
+    long long nbk = 1;
+    for (int d = 0; d < 3; d++) {
+        b.lo[d] = box[2 * d];
+        b.hi[d] = box[2 * d + 1];
+        nbk *= ((b.hi[d] + 1) >> 1) - (b.lo[d] >> 1);
+    }
+    if (b.size() <= 0)
+        return PMG_OK;
+    const int ps__ = prof_begin("k_face_stamp", st);
+    k_face_stamp<<<dim3((unsigned)grid_for(nbk, 128, 1LL << 30), B ? 2 : 1), 128, 0, st>>>(A, B ? *B : A,
+                                                                                         bgrid_of(shape), b, err);
+    // per block meeting the box: mask, parent, root parent
+    prof_end(ps__, (double)nbk * 9 * (B ? 2 : 1), st);
+    PMG_CHECK_LAUNCH();
+    return PMG_OK;
+}
+
+// Inlet selection of set A constrained by set B, as row words: the voxels of A
+// whose component has the inlet stamp and, when *b_count > 0, that are voxels
+// of B with the inlet stamp too (porosimetry.py:130-148: img_results kept
+// where n_connected == 1 once the phase exists); kept counts A's
+// inlet-connected voxels before the constraint, xr receives the block-plane
+// range of the output (kRangeBig encoding).  A warp takes four pieces of a row,
+// lane 8 q + i holding word i of piece q.  Only unconnected blocks' roots are
+// looked up (lane = block, the four pieces' loads of each level before any of
+// them is used, because they are chains of dependent loads), their parents
+// being flattened on the way; what is connected now leaves U, and the changed
+// bits are cleared.
+// Bound by the three row words read and written per piece where most blocks
+// are connected (0.08 ms a radius of the 512^3 drainage; with a root lookup for
+// every block 0.14 ms).
+struct SelectSet {
+    const uint8_t *mark;
+    int *P;
+    uint8_t stamp;
+    GrowWords W;
+};
+
+// The unconnected blocks of four pieces (u: each lane its piece's) looked up;
+// what stays unconnected.
+__device__ __forceinline__ unsigned still_unconnected(const SelectSet &A, unsigned u, int piece0, int nt2,
+                                                      const BGrid &G, int *err)
+{
+    constexpr int NB = 4;
+    const int lane = threadIdx.x & 31;
+    int x[NB], p[NB], g[NB];
+#pragma unroll
+    for (int q = 0; q < NB; q++) {
+        const int row = (int)fdiv((unsigned)(piece0 + q), G.qt);
+        x[q] = row * G.b2 + (piece0 + q - row * nt2) * kT2 + lane;
+        p[q] = (__shfl_sync(0xffffffffu, u, q * 8) >> lane) & 1u ? ld(A.P + x[q]) : -1;
+    }
+#pragma unroll
+    for (int q = 0; q < NB; q++)
+        g[q] = p[q] >= 0 && p[q] != x[q] ? ld(A.P + p[q]) : p[q];
+#pragma unroll
+    for (int q = 0; q < NB; q++)
+        if (g[q] != p[q]) {
+            p[q] = find_root(A.P, g[q], err);
+            A.P[x[q]] = p[q];
+        }
+    bool k[NB];
+#pragma unroll
+    for (int q = 0; q < NB; q++)
+        k[q] = p[q] >= 0 && A.mark[p[q]] == A.stamp;
+#pragma unroll
+    for (int q = 0; q < NB; q++) {
+        const unsigned got = __ballot_sync(0xffffffffu, k[q]);
+        if ((lane >> 3) == q)
+            u &= ~got;
+    }
+    return u;
+}
+
+__global__ void __launch_bounds__(256) k_pair_rows(SelectSet A, SelectSet B,
+                                                   const unsigned long long *__restrict__ b_count, BGrid G, int nt2,
+                                                   unsigned *__restrict__ out, unsigned long long *kept, int *err,
+                                                   int *xr)
+{
+    const int pieces = G.b0 * G.b1 * nt2, lane = threadIdx.x & 31;
     const bool constrain = *b_count > 0;
-    unsigned int cnt = 0;
-    int xmax = 0, xmin = 0; // block-plane range of the output's voxels, encoded as in XRange
-    // kPairBatch blocks per thread, each level of the root lookups (masks,
-    // parents, their parents, marks) loaded for all of them before any is
-    // used: the lookups are chains of dependent loads
-    constexpr int NB = kPairBatch;
-    for (int base = blockIdx.x * blockDim.x * NB + threadIdx.x; base < nb; base += gridDim.x * blockDim.x * NB) {
-        int bb[NB], pa[NB], pb[NB], ga[NB], gb[NB];
-        unsigned m[NB], mb[NB], ka[NB], kb[NB];
-#pragma unroll
-        for (int q = 0; q < NB; q++) {
-            bb[q] = base + q * blockDim.x;
-            const bool in = bb[q] < nb;
-            m[q] = in ? MA[bb[q]] : 0u;
-            mb[q] = in ? MB[bb[q]] : 0u;
+    unsigned cnt = 0;
+    int xmax = 0, xmin = 0;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (int base = warp * 4; base < pieces; base += nwarps * 4) {
+        const int piece = base + (lane >> 3);
+        const bool in = piece < pieces;
+        const long long word = (long long)base * 8 + lane;
+        const unsigned va = in ? A.W.V[word] : 0u, vb = in && constrain ? B.W.V[word] : 0u;
+        const unsigned ua0 = in ? A.W.U[piece] : 0u, ub0 = in ? B.W.U[piece] : 0u;
+        unsigned ua = ua0, ub = ub0;
+        if (__any_sync(0xffffffffu, ua0))
+            ua = still_unconnected(A, ua0, base, nt2, G, err);
+        if (__any_sync(0xffffffffu, ub0))
+            ub = still_unconnected(B, ub0, base, nt2, G, err);
+        if (in && (lane & 7) == 0) {
+            if (ua != ua0)
+                A.W.U[piece] = ua;
+            if (ub != ub0)
+                B.W.U[piece] = ub;
+            A.W.N[piece] = 0u;
+            B.W.N[piece] = 0u;
         }
-#pragma unroll
-        for (int q = 0; q < NB; q++) {
-            pa[q] = m[q] ? ld(PA + bb[q]) : -1;
-            pb[q] = mb[q] ? ld(PB + bb[q]) : -1;
-        }
-#pragma unroll
-        for (int q = 0; q < NB; q++) {
-            ga[q] = pa[q] >= 0 && pa[q] != bb[q] ? ld(PA + pa[q]) : pa[q];
-            gb[q] = pb[q] >= 0 && pb[q] != bb[q] ? ld(PB + pb[q]) : pb[q];
-        }
-#pragma unroll
-        for (int q = 0; q < NB; q++) {
-            // the root: the parent when it is its own parent, else further up
-            // (rare once the parents were flattened); parents flattened to it
-            int ra = pa[q], rb = pb[q];
-            if (ra >= 0 && ra != bb[q] && ga[q] != ra)
-                ra = find_root(PA, ga[q], err);
-            if (rb >= 0 && rb != bb[q] && gb[q] != rb)
-                rb = find_root(PB, gb[q], err);
-            if (ra != pa[q])
-                PA[bb[q]] = ra;
-            if (rb != pb[q])
-                PB[bb[q]] = rb;
-            pa[q] = ra;
-            pb[q] = rb;
-        }
-#pragma unroll
-        for (int q = 0; q < NB; q++) {
-            ka[q] = pa[q] >= 0 ? markA[pa[q]] : 0u;
-            kb[q] = pb[q] >= 0 ? markB[pb[q]] : 0u;
-        }
-#pragma unroll
-        for (int q = 0; q < NB; q++) {
-            const int b = bb[q];
-            if (b >= nb)
-                continue;
-            int c0, c1, c2;
-            G.coords(b, c0, c1, c2);
-            unsigned mm = ka[q] & 1u ? m[q] : 0u;
-            const unsigned keepB = kb[q] & 1u ? mb[q] : 0u;
-            cnt += __popc(mm);
-            if (constrain)
-                mm &= keepB;
-            if (mm) {
-                xmax = max(xmax, c0 + 1);
-                xmin = max(xmin, kRangeBig - c0);
-            }
-            if constexpr (BLK) {
-                out[b] = (uint8_t)mm;
-            } else {
-#pragma unroll
-                for (int x = 0; x < 2; x++)
-#pragma unroll
-                    for (int y = 0; y < 2; y++) {
-                        const int i = 2 * c0 + x, j = 2 * c1 + y;
-                        if (i >= G.s0 || j >= G.s1)
-                            continue;
-                        uint8_t *row = out + ((long long)i * G.s1 + j) * G.s2;
-#pragma unroll
-                        for (int z = 0; z < 2; z++) {
-                            const int k = 2 * c2 + z;
-                            if (k < G.s2)
-                                row[k] = (uint8_t)((mm >> ((x * 2 + y) * 2 + z)) & 1);
-                        }
-                    }
-            }
+        const unsigned wa = va & ~ua, o = constrain ? wa & vb & ~ub : wa;
+        cnt += __popc(wa);
+        if (in)
+            out[word] = o;
+        if (o) {
+            const int c0 = (int)fdiv(fdiv((unsigned)piece, G.qt), G.q1);
+            xmax = max(xmax, c0 + 1);
+            xmin = max(xmin, kRangeBig - c0);
         }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-        xmax = max(xmax, __shfl_down_sync(0xffffffffu, xmax, o));
-        xmin = max(xmin, __shfl_down_sync(0xffffffffu, xmin, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    xmax = __reduce_max_sync(0xffffffffu, xmax);
+    xmin = __reduce_max_sync(0xffffffffu, xmin);
+    if (lane == 0) {
         if (cnt)
             atomicAdd(kept, (unsigned long long)cnt);
-        if (xr && xmax) {
+        if (xmax) {
             atomicMax(xr, xmax);
             atomicMax(xr + 1, xmin);
         }
     }
-}
-
-int grow_marks_erode(GrowSel &g, const uint16_t *E, int T, const int64_t *shape, const int32_t *bc,
-                     const int32_t *pad, const int64_t *inlet_box, int *err, cudaStream_t st)
-{
-    return grow_step(g, erode_src(E, T, shape, bc), shape, bc, pad, inlet_box, nullptr, err, st);
-}
-
-int grow_marks_step(GrowSel &g, const uint8_t *S, int k, const int64_t *shape, const int32_t *bc,
-                    const int32_t *pad, const int64_t *inlet_box, int *err, cudaStream_t st)
-{
-    SrcStep src{S, k};
-    return grow_step(g, src, shape, bc, pad, inlet_box, nullptr, err, st, g.ev ? g.off + k : nullptr);
 }
 
 // Step values (255 outside the volume) of the eight voxels of a block, byte
@@ -2604,125 +2768,90 @@ int step_lists_build(GrowSel &g, const uint8_t *S, const int64_t *shape, int nst
     return PMG_OK;
 }
 
-int grow_marks_binary(GrowSel &g, const uint8_t *img, int fgval, const int64_t *shape, const int32_t *bc,
-                      const int32_t *pad, const int64_t *inlet_box, int *err, cudaStream_t st)
-{
-    SrcImg src{img, fgval};
-    return grow_step(g, src, shape, bc, pad, inlet_box, nullptr, err, st);
-}
-
-// The two growing selections of a drainage radius, up to their inlet marks,
-// in one union launch and one marks launch: the eroded space A (its step k
-// from the precomputed lists when S is given, else from the capped EDT E > T)
-// and the non-wetting phase B (fgval in img, or the list the last drainage
-// update left).  Taken once both are past their first full build and no axis
-// is periodic (no seam twins); otherwise the two steps run one after the
-// other.  Same parents and marks either way: each set's unions only involve
-// its own parents.
+// Both growing selections of a drainage radius up to their inlet stamps: the
+// eroded space A (its step k from the precomputed lists when S is given, else
+// from the capped EDT E > T) and the non-wetting phase B (fgval in img).
 int grow_marks_pair(GrowSel &a, const uint8_t *S, int k, const uint16_t *E, int T, GrowSel &b, const uint8_t *img,
                     int fgval, const int64_t *shape, const int32_t *bc, const int32_t *pad, const int64_t *inlet_box,
                     int *err, cudaStream_t st)
 {
-    const bool step_lists = S && a.ev;
-    if (!a.built || !b.built || any_periodic(bc) || (!S && !E)) {
-        if (S)
-            PMG_TRY(grow_marks_step(a, S, k, shape, bc, pad, inlet_box, err, st));
-        else
-            PMG_TRY(grow_marks_erode(a, E, T, shape, bc, pad, inlet_box, err, st));
-        return grow_marks_binary(b, img, fgval, shape, bc, pad, inlet_box, err, st);
-    }
     PMG_TRY(check_boxes(shape, inlet_box, nullptr));
+    const SrcStep step{S, k};
+    const SrcErode erode = erode_src(E, T, shape, bc);
+    const SrcImg phase{img, fgval};
+    const bool both = a.built && b.built;
+    const bool a_new = !a.built, b_new = !b.built;
+    if (a_new)
+        PMG_TRY(S ? grow_build(a, step, shape, bc, pad, err, st) : grow_build(a, erode, shape, bc, pad, err, st));
+    else
+        PMG_TRY(S ? grow_masks(a, step, shape, a.ev ? a.off + k : nullptr, err, st)
+                  : grow_masks(a, erode, shape, nullptr, err, st));
+    if (b_new)
+        PMG_TRY(grow_build(b, phase, shape, bc, pad, err, st));
+    else
+        PMG_TRY(grow_masks(b, phase, shape, nullptr, err, st));
+    if (both)
+        PMG_TRY(grow_rows(a, &b, shape, err, st));
+    else if (!a_new)
+        PMG_TRY(grow_rows(a, nullptr, shape, err, st));
+    else if (!b_new)
+        PMG_TRY(grow_rows(b, nullptr, shape, err, st));
     const BGrid G = bgrid_of(shape);
-    const int nb = G.b0 * G.b1 * G.b2;
-    const long long n = shape[0] * shape[1] * shape[2];
-    const int *a_off = step_lists ? a.off + k : nullptr;
-    // A's grown blocks
-    if (step_lists) {
-        const SrcStep src{S, k};
-        const int ps__ = prof_begin("k_grow_apply", st);
-        k_grow_apply<SrcStep><<<152 * 8, 256, 0, st>>>(src, a.M, a.P, G, a.ev, a_off, err,
-                                                       prof_units(kUnitsGrowApply));
-        prof_end_units(ps__, kUnitsGrowApply, 4 + 8 * sizeof(*src_elem(src)) + 2 + 4, st);
-        PMG_CHECK_LAUNCH();
-    } else if (S) {
-        const SrcStep src{S, k};
-        PMG_CUDA(cudaMemsetAsync(a.count, 0, sizeof(int), st));
-        const int ps__ = prof_begin("k_grow_masks", st);
-        k_grow_masks<SrcStep><<<grid_for(nb, 256, 152LL * 64), 256, 0, st>>>(src, a.M, a.P, G, a.list, a.count, err);
-        prof_end(ps__, (double)n + (double)nb, st);
-        PMG_CHECK_LAUNCH();
-    } else {
-        const SrcErode src = erode_src(E, T, shape, bc);
-        PMG_CUDA(cudaMemsetAsync(a.count, 0, sizeof(int), st));
-        const int ps__ = prof_begin("k_grow_masks", st);
-        k_grow_masks<SrcErode><<<grid_for(nb, 256, 152LL * 64), 256, 0, st>>>(src, a.M, a.P, G, a.list, a.count,
-                                                                            err);
-        prof_end(ps__, (double)n * 2 + (double)nb, st);
-        PMG_CHECK_LAUNCH();
-    }
-    // B's grown blocks: listed by the last update, or from its new masks
-    if (b.pending) {
-        b.pending = false;
-    } else {
-        const SrcImg src{img, fgval};
-        PMG_CUDA(cudaMemsetAsync(b.count, 0, sizeof(int), st));
-        const int ps__ = prof_begin("k_grow_masks", st);
-        k_grow_masks<SrcImg><<<grid_for(nb, 256, 152LL * 64), 256, 0, st>>>(src, b.M, b.P, G, b.list, b.count, err);
-        prof_end(ps__, (double)n + (double)nb, st);
-        PMG_CHECK_LAUNCH();
-    }
-    {
-        const int ps__ = prof_begin("k_grow_unite[pair]", st);
-        k_grow_unite2<<<152 * 32, 256, 0, st>>>(UniteList{a.P, a.M, step_lists ? a.ev : a.list, a.count, a_off},
-                                                UniteList{b.P, b.M, b.list, b.count, nullptr}, G, err,
-                                                prof_units(kUnitsGrowUnitePair));
-        // per listed block: its list entry, mask and parent, and the masks and
-        // parents of its 26 neighbours
-        prof_end_units(ps__, kUnitsGrowUnitePair, 4 + 5 + 26 * 5, st);
-        PMG_CHECK_LAUNCH();
-    }
-    // inlet marks of both
-    PMG_CUDA(cudaMemsetAsync(a.mark, 0, ((size_t)nb + 3) & ~(size_t)3, st));
-    PMG_CUDA(cudaMemsetAsync(b.mark, 0, ((size_t)nb + 3) & ~(size_t)3, st));
-    if (inlet_box && inlet_box[0] >= 0) {
-        Box bx;
-        for (int d = 0; d < 3; d++) {
-            bx.lo[d] = inlet_box[2 * d];
-            bx.hi[d] = inlet_box[2 * d + 1];
-        }
-        if (bx.size() > 0) {
-            long long nbk = 1;
-            for (int d = 0; d < 3; d++)
-                nbk *= ((bx.hi[d] + 1) >> 1) - (bx.lo[d] >> 1);
-            const int ps__ = prof_begin("k_bcc_mark", st);
-            k_bcc_mark2<<<dim3((unsigned)grid_for(nbk, 256, 1LL << 30), 2), 256, 0, st>>>(
-                a.M, a.P, a.mark, b.M, b.P, b.mark, G, bx, (uint8_t)1, err);
-            prof_end(ps__, (double)nbk * 18, st);
-            PMG_CHECK_LAUNCH();
-        }
-    }
+    const size_t nb = (size_t)G.b0 * G.b1 * G.b2;
+    PMG_TRY(next_stamp(a.mark, a.stamp, nb, st));
+    PMG_TRY(next_stamp(b.mark, b.stamp, nb, st));
+    const StampSet B{b.M, b.P, b.mark, (uint8_t)b.stamp};
+    return face_stamps(inlet_box, shape, StampSet{a.M, a.P, a.mark, (uint8_t)a.stamp}, &B, err, st);
+}
+
+int grow_pair_select(GrowSel &a, GrowSel &b, const unsigned long long *b_count, unsigned *out, const int64_t *shape,
+                     int *err, cudaStream_t st, unsigned long long *kept, int *xr)
+{
+    const BGrid G = bgrid_of(shape);
+    const int pieces = row_pieces(G);
+    PMG_CUDA(cudaMemsetAsync(xr, 0, 2 * sizeof(int), st));
+    const int ps__ = prof_begin("k_pair_rows", st);
+    k_pair_rows<<<grid_for((pieces + 3) / 4 * 32LL, 256, 152LL * 32), 256, 0, st>>>(
+        SelectSet{a.mark, a.P, (uint8_t)a.stamp, words(a)}, SelectSet{b.mark, b.P, (uint8_t)b.stamp, words(b)}, b_count, G,
+        (G.b2 + kT2 - 1) / kT2, out, kept, err, xr);
+    // words read and written, the unconnected and the changed words (the
+    // lookups come on top)
+    prof_end(ps__, (double)pieces * (96 + 8 + 8), st);
+    PMG_CHECK_LAUNCH();
     return PMG_OK;
 }
 
-int grow_pair_select(GrowSel &a, GrowSel &b, const unsigned long long *b_count, uint8_t *out,
-                     const int64_t *shape, int *err, cudaStream_t st, unsigned long long *kept, int *xr,
-                     bool blocks)
+size_t rows_bytes(const int64_t *shape) { return bcc_row_bytes(bgrid_of(shape)); }
+
+// Row words of the voxels equal to 1 of an image: one warp per piece of a row.
+__global__ void __launch_bounds__(256) k_bytes_to_rows(const uint8_t *__restrict__ img, unsigned *__restrict__ V,
+                                                       BGrid G, int nt2)
+{
+    const int lane = threadIdx.x & 31, pieces = G.b0 * G.b1 * nt2;
+    const SrcImg src{img, 1};
+    for (int piece = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; piece < pieces;
+         piece += (gridDim.x * blockDim.x) >> 5) {
+        const int row = (int)fdiv((unsigned)piece, G.qt), c0 = (int)fdiv((unsigned)row, G.q1), c1 = row - c0 * G.b1,
+                  c2 = (piece - row * nt2) * kT2 + lane;
+        const unsigned m = c2 < G.b2 ? block_mask(src, G, c0, c1, c2) : 0u;
+        unsigned mine = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const unsigned w = __ballot_sync(0xffffffffu, (m >> i) & 1u);
+            mine = lane == i ? w : mine;
+        }
+        if (lane < 8)
+            V[(long long)piece * 8 + lane] = mine;
+    }
+}
+
+int bytes_to_rows(const uint8_t *img, unsigned *V, const int64_t *shape, cudaStream_t st)
 {
     const BGrid G = bgrid_of(shape);
-    const int nb = G.b0 * G.b1 * G.b2;
-    const long long n = shape[0] * shape[1] * shape[2];
-    const int ps__ = prof_begin("k_grow_pair_select", st);
-    if (xr)
-        PMG_CUDA(cudaMemsetAsync(xr, 0, 2 * sizeof(int), st));
-    const unsigned grid = grid_for((nb + kPairBatch - 1) / kPairBatch, 256, 152LL * 64);
-    if (blocks)
-        k_grow_pair_select<true><<<grid, 256, 0, st>>>(a.M, a.P, a.mark, b.M, b.P, b.mark, b_count, G, out, kept,
-                                                        err, xr);
-    else
-        k_grow_pair_select<false><<<grid, 256, 0, st>>>(a.M, a.P, a.mark, b.M, b.P, b.mark, b_count, G, out, kept,
-                                                         err, xr);
-    // masks 2 B, parents and marks of the nonempty blocks about 8 B per block
-    prof_end(ps__, (blocks ? 0.0 : (double)n) + (double)nb * (blocks ? 11 : 10), st);
+    const int pieces = row_pieces(G);
+    const int ps__ = prof_begin("k_bytes_to_rows", st);
+    k_bytes_to_rows<<<grid_for(pieces * 32LL, 256, 152LL * 32), 256, 0, st>>>(img, V, G, (G.b2 + kT2 - 1) / kT2);
+    prof_end(ps__, (double)shape[0] * shape[1] * shape[2] + (double)pieces * 32, st);
     PMG_CHECK_LAUNCH();
     return PMG_OK;
 }
@@ -2736,30 +2865,12 @@ int select_grow_binary(GrowSel &g, const uint8_t *img, int fgval, void *out, con
                             st, kept);
 }
 
-int select_grow_erode(GrowSel &g, const uint16_t *E, int T, void *out, const int64_t *shape, const int32_t *bc,
-                      const int32_t *pad, const int64_t *inlet_box, const int64_t *outlet_box, int mode, int *err,
-                      cudaStream_t st, unsigned long long *kept)
-{
-    return grow_select_core(g, erode_src(E, T, shape, bc), out, shape, bc, pad, inlet_box, outlet_box, mode, 1, err,
-                            st, kept);
-}
-
-int bcc_marks_binary(const uint8_t *img, int fgval, const int64_t *shape, const int32_t *bc, const int32_t *pad,
-                     const int64_t *inlet_box, const int64_t *outlet_box, int *P, uint8_t *M, uint8_t *mark,
-                     int *err, cudaStream_t st)
-{
-    PMG_TRY(check_boxes(shape, inlet_box, outlet_box));
-    SrcImg src{img, fgval};
-    PMG_TRY(bcc_build(src, shape, bc, pad, true, P, M, err, st));
-    return bcc_marks(shape, inlet_box, outlet_box, P, M, mark, err, st);
-}
-
 // ---- selection of a shrinking set, tile by tile ---------------------------------
 // The wetting phase of a drainage curve only loses voxels; components can
 // split, so its union-find is rebuilt every step, but the tile phase is local:
 // a tile none of whose voxels changed gives the same tile-local parents as
-// before, kept in Pl.  The producer of the changes (the drainage update)
-// flags the tiles it touched and writes their new block masks.
+// before.  The producer of the changes (the drainage update) flags the tiles it
+// touched and keeps the block masks and row words current.
 
 size_t shrink_sel_bytes(const int64_t *shape)
 {
@@ -2767,8 +2878,8 @@ size_t shrink_sel_bytes(const int64_t *shape)
     const size_t nb = (size_t)G.b0 * G.b1 * G.b2;
     const size_t a = (nb + 255) & ~(size_t)255;
     const size_t nt = (size_t)((G.b0 + kT0 - 1) / kT0) * ((G.b1 + kT1 - 1) / kT1) * ((G.b2 + kT2 - 1) / kT2);
-    // P, Pl, M, mark, per-tile flags, row words
-    return a * 4 * 2 + a * 2 + ((nt * 4 + 255) & ~(size_t)255) + bcc_row_bytes(G) + 256;
+    // P, M, mark, per-tile flags, row words, tile roots, cut-off blocks
+    return a * 4 + a * 2 + ((nt * 4 + 255) & ~(size_t)255) + bcc_row_bytes(G) + 2 * piece_bytes(G) + 256;
 }
 
 void shrink_sel_init(ShrinkSel &g, void *mem, const int64_t *shape)
@@ -2780,8 +2891,6 @@ void shrink_sel_init(ShrinkSel &g, void *mem, const int64_t *shape)
     char *p = (char *)mem;
     g.P = (int *)p;
     p += a * 4;
-    g.Pl = (int *)p;
-    p += a * 4;
     g.M = (uint8_t *)p;
     p += a;
     g.mark = (uint8_t *)p;
@@ -2789,252 +2898,276 @@ void shrink_sel_init(ShrinkSel &g, void *mem, const int64_t *shape)
     g.dirty = (int *)p;
     p += (nt * 4 + 255) & ~(size_t)255;
     g.V = (unsigned *)p;
+    p += bcc_row_bytes(G);
+    g.R = (unsigned *)p;
+    p += piece_bytes(G);
+    g.T = (unsigned *)p;
     g.ntiles = (int)nt;
+    g.stamp = 0;
     g.built = false;
 }
 
 int shrink_marks_binary(ShrinkSel &g, const uint8_t *img, int fgval, const int64_t *shape, const int32_t *bc,
-                        const int32_t *pad, const int64_t *inlet_box, const int64_t *outlet_box, int *err,
-                        cudaStream_t st)
+                        const int32_t *pad, const int64_t *outlet_box, int *err, cudaStream_t st)
 {
-    PMG_TRY(check_boxes(shape, inlet_box, outlet_box));
-    if (!g.built)
-        PMG_CUDA(cudaMemsetAsync(g.dirty, 0, sizeof(int) * (size_t)g.ntiles, st));
+    PMG_TRY(check_boxes(shape, nullptr, outlet_box));
+    const BGrid G = bgrid_of(shape);
     if (g.built) {
-        // the producer of the changes kept the block masks current
-        PMG_TRY(bcc_build(SrcMask{g.M}, shape, bc, pad, true, g.P, g.M, err, st, g.Pl, g.dirty, g.V));
+        PMG_TRY(bcc_tiles_run(shape, g.P, g.V, g.R, g.dirty, st));
+        PMG_TRY(bcc_cross_phase(shape, bc, pad, true, g.P, g.M, g.V, err, st));
     } else {
-        SrcImg src{img, fgval};
-        PMG_TRY(bcc_build(src, shape, bc, pad, true, g.P, g.M, err, st, g.Pl, nullptr, g.V));
+        PMG_CUDA(cudaMemsetAsync(g.dirty, 0, sizeof(int) * (size_t)g.ntiles, st));
+        PMG_CUDA(cudaMemsetAsync(g.T, 0, piece_bytes(G), st));
+        const SrcImg src{img, fgval};
+        PMG_TRY(bcc_build(src, shape, bc, pad, true, g.P, g.M, err, st, g.V, g.R));
     }
     g.built = true;
-    return bcc_marks(shape, inlet_box, outlet_box, g.P, g.M, g.mark, err, st);
+    PMG_TRY(next_stamp(g.mark, g.stamp, (size_t)G.b0 * G.b1 * G.b2, st));
+    return face_stamps(outlet_box, shape, StampSet{g.M, g.P, g.mark, (uint8_t)g.stamp}, nullptr, err, st);
 }
 
-// ---- drainage update on blocks -------------------------------------------------
+// ---- drainage update on row words -------------------------------------------------
 // mp = 1 where morph == 1 on a wetting voxel (2) connected to the outlet,
 // reservoir slabs -> 1 (equilibrium_distribution.py:133-179,
 // subdomain_padded.py:285-307), fused with the saturation counts (value 2
-// inside the own box, multiphase.py:56-96; value 1 anywhere).  One thread per
-// 2x2x2 block: the wetting phase's outlet connection comes from its block
-// union-find (outlet mark bit 1), so no selected image is written.  With Mn,
-// the block masks of the non-wetting phase (value 1) are brought up to date
-// and grown blocks are listed for its next growing-selection step.
+// inside the own box, multiphase.py:56-96; value 1 anywhere).  Dilation, wetting
+// and non-wetting phase are row words, so the image itself is only written,
+// where it changes.  A thread per word finds the pieces of a row (32 blocks)
+// whose dilation meets wetting voxels not known to be cut off, which are then
+// taken by a warp each (lanes 0-7 its words, then lane = block).  The outlet
+// connection comes from the wetting phase's block union-find.  The masks and
+// words of both phases are kept current, and the wetting phase's changed tiles
+// flagged.
+// Bound by the words read where little changes, by the root searches elsewhere:
+// 0.08 ms a radius at 512^3; a thread per block that read image and dilation byte
+// by byte took 0.25 ms, four pieces to a warp one after the other 0.16 ms.
 
-constexpr int kUpdateBatch = 2;
-
-__global__ void __launch_bounds__(256, 5) k_drain_update_blocks(uint8_t *__restrict__ mp, const uint8_t *__restrict__ morph, int *Pw,
-                                      uint8_t *__restrict__ Mw, const uint8_t *__restrict__ markw, BGrid G,
-                                      Boxes B, uint8_t *__restrict__ Mn, int *__restrict__ Pn,
-                                      int *__restrict__ list, int *count, unsigned long long *cnt2,
-                                      unsigned long long *cnt1, int *err, int *__restrict__ wdirty,
-                                      const int *__restrict__ orange, int ranged, unsigned long long *units)
+// bit c: position 2 (32 tk + c) + z inside [lo, hi)
+__device__ __forceinline__ unsigned range_bits(int tk, int z, long long lo, long long hi)
 {
-    // orange: the x range [olo, ohi] (whole blocks) where the dilation result
-    // is defined; outside it the dilation is empty.  ranged: only blocks that
-    // can change are visited (the dilation range: the reservoir slabs were
-    // refilled by an earlier update), and cnt2 / cnt1 receive the changes
-    // (voxels leaving value 2 inside the own box, voxels newly 1) instead of
-    // the totals.
-    const int bxlo = orange ? orange[0] >> 1 : 0, bxhi = orange ? orange[1] >> 1 : G.b0 - 1;
-    // a ranged update walks the dilation's block planes only
-    const int plane = G.b1 * G.b2;
-    const int bstart = ranged ? max(0, bxlo) * plane : 0;
-    const int nb = G.b0 * G.b1 * G.b2;
-    const int bend = ranged ? min(nb, max(0, bxhi + 1) * plane) : nb;
-    if (units && blockIdx.x == 0 && threadIdx.x == 0 && bend > bstart)
-        atomicAdd(units, (unsigned long long)(bend - bstart) * 8ull);
-    const int lane = threadIdx.x & 31;
-    unsigned int c2 = 0, c1 = 0;
-    const bool pairs = !(G.s2 & 1);
-    const long long sx = (long long)G.s1 * G.s2, sy = G.s2;
-    // kUpdateBatch blocks per thread: every load of all of them is issued
-    // before any of them is updated
-    constexpr int NB = kUpdateBatch;
-    for (int base = bstart + blockIdx.x * blockDim.x * NB; base < bend; base += gridDim.x * blockDim.x * NB) {
-        int bq[NB];
-        bool act[NB], ind[NB];
-        unsigned vol[NB], wold[NB], oldn[NB], pv[NB][4], mv[NB][4];
-        long long base0[NB];
-#pragma unroll
-        for (int q = 0; q < NB; q++) {
-            const int b = base + q * blockDim.x + threadIdx.x;
-            bq[q] = b;
-            int c0, c1b, c2b;
-            G.coords(b, c0, c1b, c2b);
-            ind[q] = c0 >= bxlo && c0 <= bxhi;
-            act[q] = b < bend && (ind[q] || !ranged);
-            const int i0 = 2 * c0, j0 = 2 * c1b, k0 = 2 * c2b;
-            vol[q] = act[q] ? spread_x(in2(i0, 0, G.s0)) & spread_y(in2(j0, 0, G.s1)) & spread_z(in2(k0, 0, G.s2)) : 0u;
-            base0[q] = (long long)i0 * sx + (long long)j0 * sy + k0;
-            wold[q] = act[q] ? Mw[b] : 0u;
-            oldn[q] = act[q] && Mn ? Mn[b] : 0u;
-#pragma unroll
-            for (int t = 0; t < 4; t++) {
-                pv[q][t] = 0;
-                mv[q][t] = 0;
-                if ((vol[q] >> (2 * t)) & 3u) {
-                    const long long a = base0[q] + (t >> 1) * sx + (t & 1) * sy;
-                    if (pairs) {
-                        pv[q][t] = *(const uint16_t *)(mp + a);
-                        if (ind[q])
-                            mv[q][t] = *(const uint16_t *)(morph + a);
-                    } else {
-                        pv[q][t] = mp[a];
-                        if (ind[q])
-                            mv[q][t] = morph[a];
-                        if ((vol[q] >> (2 * t)) & 2u) {
-                            pv[q][t] |= (unsigned)mp[a + 1] << 8;
-                            if (ind[q])
-                                mv[q][t] |= (unsigned)morph[a + 1] << 8;
-                        }
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < NB; q++) {
-            const int b = bq[q];
-            bool changed = false;
-            if (act[q]) {
-                int c2b, c0, c1b;
-                G.coords(b, c0, c1b, c2b);
-                const int i0 = 2 * c0, j0 = 2 * c1b, k0 = 2 * c2b;
-                // voxels inside the own box and the reservoir slabs
-                const unsigned v = vol[q];
-                const unsigned own = spread_x(in2(i0, B.own[0], B.own[1])) & spread_y(in2(j0, B.own[2], B.own[3])) &
-                                     spread_z(in2(k0, B.own[4], B.own[5]));
-                const unsigned res = (spread_x(~in2(i0, B.rpad[0], (long long)G.s0 - B.rpad[1]) & 3u) |
-                                      spread_y(~in2(j0, B.rpad[2], (long long)G.s1 - B.rpad[3]) & 3u) |
-                                      spread_z(~in2(k0, B.rpad[4], (long long)G.s2 - B.rpad[5]) & 3u)) &
-                                     v;
-                unsigned wet = wold[q];
-                unsigned m1 = 0, is1 = 0, is2o = 0;
-#pragma unroll
-                for (int t = 0; t < 4; t++) {
-                    m1 |= eq2(mv[q][t], 1) << (2 * t);
-                    is1 |= eq2(pv[q][t], 1) << (2 * t);
-                    is2o |= eq2(pv[q][t], 2) << (2 * t);
-                }
-                // the wetting phase's outlet connection matters only where the
-                // dilation meets it
-                if (m1 & wet) {
-                    const int rw = find_root(Pw, ld(Pw + b), err);
-                    if (rw < 0 || !(markw[rw] & 2))
-                        wet = 0;
-                }
-                // voxels set to 1: invaded wetting voxels and reservoir slabs
-                const unsigned set1 = ((m1 & wet) | res) & v;
-                unsigned is2 = 0;
-#pragma unroll
-                for (int t = 0; t < 4; t++) {
-                    const unsigned bits = (set1 >> (2 * t)) & 3u;
-                    unsigned p = pv[q][t];
-                    if (bits) {
-                        const unsigned bm = (bits & 1u ? 0x00ffu : 0u) | (bits & 2u ? 0xff00u : 0u);
-                        p = (p & ~bm) | (0x0101u & bm);
-                        const long long a = base0[q] + (t >> 1) * sx + (t & 1) * sy;
-                        if (pairs) {
-                            *(uint16_t *)(mp + a) = (uint16_t)p;
-                        } else {
-                            if (bits & 1u)
-                                mp[a] = 1;
-                            if (bits & 2u)
-                                mp[a + 1] = 1;
-                        }
-                    }
-                    is2 |= eq2(p, 2) << (2 * t);
-                }
-                const unsigned nwm = (is1 | set1) & v;
-                if (wdirty && (is2 & v) != wold[q]) {
-                    // the wetting phase changed here: its tile is recomputed next step
-                    Mw[b] = (uint8_t)(is2 & v);
-                    const int nt1 = (G.b1 + kT1 - 1) / kT1, nt2 = (G.b2 + kT2 - 1) / kT2;
-                    const int tl = ((c0 / kT0) * nt1 + c1b / kT1) * nt2 + c2b / kT2;
-                    if (!wdirty[tl])
-                        wdirty[tl] = 1;
-                }
-                if (ranged) {
-                    c2 += __popc(set1 & is2o & own & v);
-                    c1 += __popc(set1 & ~is1 & v);
-                } else {
-                    c2 += __popc(is2 & own & v);
-                    c1 += __popc(nwm);
-                }
-                if (Mn && nwm != oldn[q]) {
-                    if (oldn[q] & ~nwm)
-                        atomicExch(err, 3);
-                    Mn[b] = (uint8_t)nwm;
-                    if (!oldn[q])
-                        Pn[b] = b;
-                    changed = true;
-                }
-            }
-            if (Mn) {
-                const unsigned bal = __ballot_sync(0xffffffffu, changed);
-                if (bal) {
-                    int pos = 0;
-                    if (lane == 0)
-                        pos = atomicAdd(count, __popc(bal));
-                    pos = __shfl_sync(0xffffffffu, pos, 0);
-                    if (changed)
-                        list[pos + __popc(bal & ((1u << lane) - 1u))] = b;
-                }
-            }
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        c2 += __shfl_down_sync(0xffffffffu, c2, o);
-        c1 += __shfl_down_sync(0xffffffffu, c1, o);
-    }
-    if (lane == 0 && c2)
-        atomicAdd(cnt2, (unsigned long long)c2);
-    if (lane == 0 && c1)
-        atomicAdd(cnt1, (unsigned long long)c1);
+    // positions v = base + 2 c
+    const long long base = 64LL * tk + z;
+    const long long a = lo > base ? (lo - base + 1) >> 1 : 0, b = hi > base ? (hi - base + 1) >> 1 : 0;
+    const unsigned ma = a >= 32 ? 0u : 0xffffffffu << a, mb = b >= 32 ? 0xffffffffu : (1u << b) - 1u;
+    return ma & mb;
 }
 
-// Running totals (count(own == 2), count(== 1)) from the update's full counts
-// or changes; the saturation numerator and the phase-1 count out.
-__global__ void k_drain_totals(int ranged, const unsigned long long *cnt2, const unsigned long long *cnt1,
-                               unsigned long long *tot, unsigned long long *sat_out, unsigned long long *ones_out)
+constexpr int kUpdatePieces = 64; // per block of 256 threads
+
+struct UpdateSets {
+    // wetting phase: row words, masks, parents, outlet stamps, tile flags
+    unsigned *Vw;
+    uint8_t *Mw;
+    int *Pw;
+    const uint8_t *markw;
+    uint8_t stamp;
+    int *wdirty;
+    // its blocks found cut off from the outlet (they stay so), one bit each
+    unsigned *Tw;
+    // non-wetting phase (Vn null: not kept)
+    unsigned *Vn, *Nn, *Un;
+    uint8_t *Mn;
+    int *Pn;
+};
+
+// D: the dilation (defined on the block planes of orange; null: none).  full:
+// every piece, with the reservoir slabs, the counts being all voxels of value
+// 2 in the own box and the voxels newly 1; otherwise only the dilation's planes
+// (the slabs were refilled before), and the changes of both counts.
+__global__ void __launch_bounds__(256) k_drain_update_rows(uint8_t *__restrict__ mp, const unsigned *__restrict__ D,
+                                                           UpdateSets U, BGrid G, int nt2, Boxes B,
+                                                           unsigned long long *cnt2, unsigned long long *cnt1, int *err,
+                                                           const int *__restrict__ orange, int full,
+                                                           unsigned long long *units)
+{
+    const int bxlo = orange ? orange[0] >> 1 : 0, bxhi = orange ? orange[1] >> 1 : G.b0 - 1;
+    const int plane = G.b1 * nt2;
+    const int first = full ? 0 : max(0, bxlo) * plane,
+              last = full ? G.b0 * plane : min(G.b0 * plane, max(0, bxhi + 1) * plane);
+    if (units && blockIdx.x == 0 && threadIdx.x == 0 && last > first)
+        atomicAdd(units, (unsigned long long)(last - first) * 256ull);
+    const int lane = threadIdx.x & 31, i = lane & 7;
+    const int X = i >> 2, Y = (i >> 1) & 1, Z = i & 1; // the voxel of this lane's word
+    const long long sx = (long long)G.s1 * G.s2, sy = G.s2;
+    unsigned c2n = 0, c1n = 0;
+    __shared__ int s_list[kUpdatePieces];
+    __shared__ int s_n;
+    for (int chunk = first + blockIdx.x * kUpdatePieces; chunk < last; chunk += gridDim.x * kUpdatePieces) {
+        if (threadIdx.x == 0)
+            s_n = 0;
+        __syncthreads();
+        for (int p = threadIdx.x >> 3; p < kUpdatePieces; p += blockDim.x >> 3) {
+            const int piece = chunk + p;
+            unsigned s = 0;
+            if (piece < last) {
+                const int c0 = (int)fdiv(fdiv((unsigned)piece, G.qt), G.q1);
+                if (D && c0 >= bxlo && c0 <= bxhi)
+                    s = U.Vw[(long long)piece * 8 + i] & D[(long long)piece * 8 + i] & ~U.Tw[piece];
+            }
+            const unsigned some = __ballot_sync(0xffffffffu, s != 0);
+            if (i == 0 && piece < last && (full || ((some >> (lane & 24)) & 0xffu)))
+                s_list[atomicAdd(&s_n, 1)] = piece;
+        }
+        __syncthreads();
+        for (int it = threadIdx.x >> 5; it < s_n; it += blockDim.x >> 5) {
+            const int piece = s_list[it];
+            const int row = (int)fdiv((unsigned)piece, G.qt), tk = piece - row * nt2;
+            const int c0 = (int)fdiv((unsigned)row, G.q1), c1 = row - c0 * G.b1;
+            const long long word = (long long)piece * 8 + i;
+            const bool in = lane < 8;
+            const unsigned w = in ? U.Vw[word] : 0u;
+            unsigned set1 = 0;
+            if (D && c0 >= bxlo && c0 <= bxhi) {
+                set1 = in ? w & D[word] & ~U.Tw[piece] : 0u;
+                const unsigned cand = __reduce_or_sync(0xffffffffu, set1);
+                int r = -1;
+                if ((cand >> lane) & 1u)
+                    r = find_root(U.Pw, row * G.b2 + tk * kT2 + lane, err);
+                const unsigned on = __ballot_sync(0xffffffffu, r >= 0 && U.markw[r] == U.stamp);
+                set1 &= on;
+                if (lane == 0 && (cand & ~on))
+                    U.Tw[piece] |= cand & ~on;
+            }
+            if (!full && !__any_sync(0xffffffffu, set1))
+                continue;
+            const int vi = 2 * c0 + X, vj = 2 * c1 + Y;
+            const bool row_in = vi < G.s0 && vj < G.s1;
+            const bool own_row = vi >= B.own[0] && vi < B.own[1] && vj >= B.own[2] && vj < B.own[3];
+            const unsigned own = in && own_row ? range_bits(tk, Z, B.own[4], B.own[5]) : 0u;
+            unsigned fresh = set1; // voxels that were not 1
+            if (full) {
+                // the reservoir slabs
+                const unsigned vol = in && row_in ? range_bits(tk, Z, 0, G.s2) : 0u;
+                const bool slab = vi < B.rpad[0] || vi >= G.s0 - B.rpad[1] || vj < B.rpad[2] || vj >= G.s1 - B.rpad[3];
+                const unsigned res = slab ? vol : vol & ~range_bits(tk, Z, B.rpad[4], (long long)G.s2 - B.rpad[5]);
+                unsigned was1 = 0;
+                for (unsigned q = res & ~set1; q; q &= q - 1) {
+                    const int c = __ffs(q) - 1;
+                    if (mp[vi * sx + vj * sy + 2 * (tk * kT2 + c) + Z] == 1)
+                        was1 |= 1u << c;
+                }
+                set1 |= res;
+                fresh = set1 & ~was1;
+                c2n += __popc(w & ~set1 & own);
+            } else {
+                c2n += __popc(set1 & own);
+            }
+            c1n += __popc(fresh);
+            const unsigned any = __reduce_or_sync(0xffffffffu, set1);
+            if (!any)
+                continue;
+            const unsigned nw = in && U.Vn ? U.Vn[word] : 0u;
+            const unsigned w2 = w & ~set1, nw2 = nw | set1;
+            if (in && set1) {
+                U.Vw[word] = w2;
+                if (U.Vn)
+                    U.Vn[word] = nw2;
+            }
+            // lane = block: the changed blocks' masks, and the image
+            unsigned mw = 0, mn = 0, ms = 0;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                mw |= ((__shfl_sync(0xffffffffu, w2, q) >> lane) & 1u) << q;
+                mn |= ((__shfl_sync(0xffffffffu, nw2, q) >> lane) & 1u) << q;
+                ms |= ((__shfl_sync(0xffffffffu, set1, q) >> lane) & 1u) << q;
+            }
+            // blocks of the non-wetting phase that grew and that are new
+            const unsigned grown = __reduce_or_sync(0xffffffffu, nw2 & ~nw),
+                           fresh_blocks = __reduce_or_sync(0xffffffffu, nw2) & ~__reduce_or_sync(0xffffffffu, nw);
+            const bool lost = __any_sync(0xffffffffu, w2 != w);
+            if (ms) {
+                const int c2 = tk * kT2 + lane, b = row * G.b2 + c2;
+                U.Mw[b] = (uint8_t)mw;
+                if (U.Vn) {
+                    U.Mn[b] = (uint8_t)mn;
+                    if ((fresh_blocks >> lane) & 1u)
+                        U.Pn[b] = b;
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const unsigned bits = (ms >> (2 * q)) & 3u;
+                    uint8_t *p = mp + (2 * c0 + (q >> 1)) * sx + (2 * c1 + (q & 1)) * sy + 2 * c2;
+                    if (bits == 3u && !(G.s2 & 1)) {
+                        *reinterpret_cast<uint16_t *>(p) = 0x0101u;
+                    } else {
+                        if (bits & 1u)
+                            p[0] = 1;
+                        if (bits & 2u)
+                            p[1] = 1;
+                    }
+                }
+            }
+            if (lane == 0) {
+                if (U.Vn) {
+                    U.Nn[piece] |= grown;
+                    U.Un[piece] |= fresh_blocks;
+                }
+                if (lost) {
+                    // the wetting phase changed here: its tile is recomputed next step
+                    const int nt1 = (G.b1 + kT1 - 1) / kT1;
+                    U.wdirty[((c0 / kT0) * nt1 + c1 / kT1) * nt2 + tk] = 1;
+                }
+            }
+        }
+        __syncthreads(); // s_n and the list are written again
+    }
+    c2n = __reduce_add_sync(0xffffffffu, c2n);
+    c1n = __reduce_add_sync(0xffffffffu, c1n);
+    if (lane == 0 && c2n)
+        atomicAdd(cnt2, (unsigned long long)c2n);
+    if (lane == 0 && c1n)
+        atomicAdd(cnt1, (unsigned long long)c1n);
+}
+
+// Running totals (count(own == 2), count(== 1)) from the update's counts; the
+// saturation numerator and the phase-1 count out.
+__global__ void k_drain_totals(int full, unsigned long long *cnt2, unsigned long long *cnt1, unsigned long long *tot,
+                               unsigned long long *sat_out, unsigned long long *ones)
 {
     if (threadIdx.x == 0 && blockIdx.x == 0) {
-        if (ranged) {
-            tot[0] -= *cnt2;
-            tot[1] += *cnt1;
-        } else {
-            tot[0] = *cnt2;
-            tot[1] = *cnt1;
-        }
+        tot[0] = full ? *cnt2 : tot[0] - *cnt2;
+        *ones += *cnt1;
         *sat_out = tot[0];
-        *ones_out = tot[1];
+        *cnt2 = 0;
+        *cnt1 = 0;
     }
 }
 
-int drain_totals(bool ranged, const unsigned long long *cnt2, const unsigned long long *cnt1, unsigned long long *tot,
-                 unsigned long long *sat_out, unsigned long long *ones_out, cudaStream_t st)
+int drain_totals(bool full, unsigned long long *cnt2, unsigned long long *cnt1, unsigned long long *tot,
+                 unsigned long long *sat_out, unsigned long long *ones, cudaStream_t st)
 {
-    k_drain_totals<<<1, 32, 0, st>>>(ranged ? 1 : 0, cnt2, cnt1, tot, sat_out, ones_out);
+    k_drain_totals<<<1, 32, 0, st>>>(full ? 1 : 0, cnt2, cnt1, tot, sat_out, ones);
     PMG_CHECK_LAUNCH();
     return PMG_OK;
 }
 
-int drain_update_blocks(uint8_t *mp, const uint8_t *morph, const int64_t *shape, int *P, uint8_t *M,
-                        const uint8_t *mark, const Boxes &B, GrowSel *g_nw, unsigned long long *cnt2_own,
-                        unsigned long long *cnt1, int *err, cudaStream_t st, int *wdirty, const int *orange,
-                        bool ranged)
+int drain_update_rows(uint8_t *mp, const unsigned *D, const int64_t *shape, ShrinkSel &w, const Boxes &B, GrowSel *g_nw,
+                      unsigned long long *cnt2, unsigned long long *cnt1, int *err, cudaStream_t st, const int *orange,
+                      bool full)
 {
     const BGrid G = bgrid_of(shape);
-    const int nb = G.b0 * G.b1 * G.b2;
-    const long long n = shape[0] * shape[1] * shape[2];
-    const int ps__ = prof_begin("k_drain_update_blocks", st);
-    k_drain_update_blocks<<<grid_for((nb + kUpdateBatch - 1) / kUpdateBatch, 256, 152LL * 64), 256, 0, st>>>(
-        mp, morph, P, M, mark, G, B, g_nw ? g_nw->M : nullptr, g_nw ? g_nw->P : nullptr,
-        g_nw ? g_nw->list : nullptr, g_nw ? g_nw->count : nullptr, cnt2_own, cnt1, err, wdirty, orange,
-        ranged ? 1 : 0, prof_units(kUnitsDrainUpdate));
-    // per voxel visited: multiphase read and written, dilation read
-    prof_end_units(ps__, kUnitsDrainUpdate, 3.0, st);
-    (void)n;
+    UpdateSets U{};
+    U.Vw = w.V;
+    U.Mw = w.M;
+    U.Pw = w.P;
+    U.markw = w.mark;
+    U.stamp = (uint8_t)w.stamp;
+    U.wdirty = w.dirty;
+    U.Tw = w.T;
+    if (g_nw) {
+        U.Vn = g_nw->V;
+        U.Nn = g_nw->N;
+        U.Un = g_nw->U;
+        U.Mn = g_nw->M;
+        U.Pn = g_nw->P;
+    }
+    const int ps__ = prof_begin("k_drain_update_rows", st);
+    k_drain_update_rows<<<grid_for((row_pieces(G) + kUpdatePieces - 1) / kUpdatePieces * 256LL, 256, 152LL * 64), 256, 0,
+                          st>>>(
+        mp, D, U, G, (G.b2 + kT2 - 1) / kT2, B, cnt2, cnt1, err, orange, full ? 1 : 0, prof_units(kUnitsDrainUpdate));
+    // per voxel visited: a bit of the dilation, of the wetting and of the
+    // non-wetting phase
+    prof_end_units(ps__, kUnitsDrainUpdate, 3.0 / 8.0, st);
     PMG_CHECK_LAUNCH();
     return PMG_OK;
 }

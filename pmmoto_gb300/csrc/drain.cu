@@ -92,6 +92,7 @@ struct Work {
     float *A, *B;
     int *P;
     uint8_t *M, *mark; // per-block masks and marks of the binary selection
+    unsigned *rows;    // row words (a drainage's selection)
     int *err;
     unsigned long long *cnt; // scalar counter
     void *base;
@@ -103,7 +104,8 @@ static int work_alloc(Work &w, const int64_t *shape, size_t morph_bytes, cudaStr
     const size_t a = (n + 255) & ~(size_t)255;
     const size_t nb = (size_t)((shape[0] + 1) / 2) * ((shape[1] + 1) / 2) * ((shape[2] + 1) / 2);
     const size_t bb = (nb + 255) & ~(size_t)255;
-    const size_t total = 3 * a + ((morph_bytes + 255) & ~(size_t)255) + a * 4 + 2 * bb + 512;
+    const size_t rb = rows_bytes(shape);
+    const size_t total = 3 * a + ((morph_bytes + 255) & ~(size_t)255) + a * 4 + 2 * bb + rb + 512;
     PMG_TRY(scratch_alloc(&w.base, total, st));
     char *p = (char *)w.base;
     w.t1 = (uint8_t *)p;
@@ -120,6 +122,8 @@ static int work_alloc(Work &w, const int64_t *shape, size_t morph_bytes, cudaStr
     p += bb;
     w.mark = (uint8_t *)p;
     p += bb;
+    w.rows = (unsigned *)p;
+    p += rb;
     w.err = (int *)p;
     w.cnt = (unsigned long long *)(p + 256);
     return PMG_OK;
@@ -184,8 +188,10 @@ static int porosimetry_run(const uint8_t *pm, uint8_t *out, const int64_t *shape
                            const Boxes &Bx, Work &w, cudaStream_t st, double ball_e, double ball_d,
                            const float *De = nullptr, const uint16_t *KC = nullptr, int Te = -1,
                            bool m1_counted = false, GrowSel *g_er = nullptr, GrowSel *g_nw = nullptr,
-                           const uint8_t *Sv = nullptr, int step = -1, int *orange = nullptr)
+                           const uint8_t *Sv = nullptr, int step = -1, int *orange = nullptr,
+                           unsigned *rows_out = nullptr)
 {
+    // rows_out (a drainage): the result as row words; out is then scratch
     // m1_counted: w.cnt[1] already holds count(mp == 1) (the drainage update
     // counts it); the inlet selection counts its kept voxels into w.cnt[0], and
     // both come back with one copy
@@ -203,15 +209,15 @@ static int porosimetry_run(const uint8_t *pm, uint8_t *out, const int64_t *shape
         PMG_TRY(grow_marks_pair(*g_er, Sv, step, KC, Te, *g_nw, mp, 1, shape, bc, pad, Bx.inlet, w.err, st));
         // the selection's x range (w.cnt[4]) limits the dilation to the planes
         // it can reach; the dilation's result range goes to orange
-        int *xr = orange ? (int *)(w.cnt + 4) : nullptr;
-        // the selection is written as per-block masks (w.M): the dilation's
-        // row pass reads them directly (w.t2 receives bytes on other paths)
-        PMG_TRY(grow_pair_select(*g_er, *g_nw, w.cnt + 1, w.M, shape, w.err, st, w.cnt, xr, true));
+        int *xr = (int *)(w.cnt + 4);
+        // the selection is written as row words (w.rows): the dilation's row
+        // pass reads them directly (w.t2 receives bytes on other paths)
+        PMG_TRY(grow_pair_select(*g_er, *g_nw, w.cnt + 1, w.rows, shape, w.err, st, w.cnt, xr));
         // the dilation reads the kept count (w.cnt[0]) on the device: no
         // dilation of an empty selection, and no host round trip per radius
         morph_split(w, shape, bc, ext_d, E, A, B);
         return morph_run(w.t2, out, shape, bc, pad, ext_d, res, r_d, cmp_d, 1, E, A, B, st, ball_d, w.cnt, xr,
-                         orange, w.M);
+                         orange, w.rows, rows_out);
     }
     if (orange) {
         // the paths below write the whole result
@@ -219,12 +225,8 @@ static int porosimetry_run(const uint8_t *pm, uint8_t *out, const int64_t *shape
         PMG_CHECK_LAUNCH();
     }
     if (KC && inlet) {
-        if (g_er)
-            PMG_TRY(select_grow_erode(*g_er, KC, Te, w.t2, shape, bc, pad, Bx.inlet, nullptr, PMG_SEL_INLET, w.err,
-                                      st, w.cnt));
-        else
-            PMG_TRY(select_run_erode(KC, Te, w.t2, shape, bc, pad, Bx.inlet, nullptr, PMG_SEL_INLET, w.P, w.M,
-                                     w.mark, w.err, st, w.cnt));
+        PMG_TRY(select_run_erode(KC, Te, w.t2, shape, bc, pad, Bx.inlet, nullptr, PMG_SEL_INLET, w.P, w.M, w.mark,
+                                 w.err, st, w.cnt));
         cur = w.t2;
     } else if (De) {
         ErodeThr T;
@@ -279,7 +281,10 @@ static int porosimetry_run(const uint8_t *pm, uint8_t *out, const int64_t *shape
             }
         }
         morph_split(w, shape, bc, ext_d, E, A, B);
-        PMG_TRY(morph_run(cur, out, shape, bc, pad, ext_d, res, r_d, cmp_d, 1, E, A, B, st, ball_d));
+        PMG_TRY(morph_run(cur, out, shape, bc, pad, ext_d, res, r_d, cmp_d, 1, E, A, B, st, ball_d, nullptr, nullptr,
+                          nullptr, nullptr, rows_out));
+    } else if (rows_out) {
+        PMG_TRY(bytes_to_rows(cur, rows_out, shape, st));
     } else if (cur != out) {
         PMG_CUDA(cudaMemcpyAsync(out, cur, (size_t)n, cudaMemcpyDeviceToDevice, st));
     }
@@ -517,20 +522,19 @@ extern "C" int pmg_drainage_ext(const uint8_t *pm_img, uint8_t *mp_img, const in
         shrink_sel_init(g_w, (char *)grow_mem + gb * (grow_er ? 2 : 1), shape);
     if (s == PMG_OK) {
         grow_sel_init(g_nw, grow_mem, shape);
-        g_nw.unite_label = "k_grow_unite[nonwetting]";
-        g_nw.unite_units = kUnitsGrowUniteB;
-        if (grow_er) {
+        if (grow_er)
             grow_sel_init(g_er, (char *)grow_mem + gb, shape);
-            g_er.unite_label = "k_grow_unite[eroded]";
-            g_er.unite_units = kUnitsGrowUniteA;
-        }
     }
     // the blocks of the eroded space that grow at each radius, listed once
     void *lists_mem = nullptr;
     if (s == PMG_OK && Sv)
         s = step_lists_build(g_er, Sv, shape, n_radii, &lists_mem, st);
+    // the dilation as bytes (paths that write them) and as row words
+    unsigned *drows = nullptr;
     if (s == PMG_OK)
-        s = scratch_alloc((void **)&morph, (size_t)n, st);
+        s = scratch_alloc((void **)&morph, (((size_t)n + 255) & ~(size_t)255) + rows_bytes(shape), st);
+    if (s == PMG_OK)
+        drows = (unsigned *)(morph + (((size_t)n + 255) & ~(size_t)255));
     if (s == PMG_OK)
         s = scratch_alloc((void **)&d_counts, sizeof(unsigned long long) * (size_t)(n_radii + 1), st);
     if (s == PMG_OK)
@@ -545,15 +549,16 @@ extern "C" int pmg_drainage_ext(const uint8_t *pm_img, uint8_t *mp_img, const in
         s = count_eq_async(mp_img, shape, whole, 1, w.cnt + 1, st);
     // After the first update (which refills the reservoir slabs), a radius can
     // change only voxels within the dilation's x range: the update visits that
-    // range alone and keeps the saturation counts as running totals
-    // (w.cnt[10], w.cnt[11]) from the changes it counts (w.cnt[8], w.cnt[9]).
+    // range alone and counts changes (w.cnt[8], w.cnt[9], cleared by
+    // drain_totals), the saturation count being a running total (w.cnt[10]).
     int *orange = (int *)(w.cnt + 5);
+    if (s == PMG_OK)
+        s = cudaMemsetAsync(w.cnt + 8, 0, 3 * sizeof(unsigned long long), st) == cudaSuccess ? PMG_OK : PMG_ECUDA;
     bool full_done = false;
     for (int k = 0; k < n_radii && s == PMG_OK; k++) {
         if (!active[k] && full_done) {
             // no dilation: nothing changes, the totals stand
-            PMG_CUDA(cudaMemsetAsync(w.cnt + 8, 0, 2 * sizeof(unsigned long long), st));
-            s = drain_totals(true, w.cnt + 8, w.cnt + 9, w.cnt + 10, d_counts + k, w.cnt + 1, st);
+            s = drain_totals(false, w.cnt + 8, w.cnt + 9, w.cnt + 10, d_counts + k, w.cnt + 1, st);
             continue;
         }
         if (active[k]) {
@@ -564,41 +569,28 @@ extern "C" int pmg_drainage_ext(const uint8_t *pm_img, uint8_t *mp_img, const in
             s = porosimetry_run(pm_img, morph, shape, bc, pad, ext, ext_d, res, radii[k], 1, radii_dilate[k], 1, 1,
                                 mp_img,
                                 Bx, w, st, ball_erode ? ball_erode[k] : -1.0, ball_dilate ? ball_dilate[k] : -1.0,
-                                De, KC, Te[(size_t)k], true, grow_er ? &g_er : nullptr, &g_nw, Sv, k, orange);
-        } else {
-            s = cudaMemsetAsync(morph, 0, (size_t)n, st) == cudaSuccess ? PMG_OK : PMG_ECUDA;
+                                De, KC, Te[(size_t)k], true, grow_er ? &g_er : nullptr, &g_nw, Sv, k, orange, drows);
         }
         if (s != PMG_OK)
             break;
-        // wetting phase connected to the outlet (its union-find and marks
+        // wetting phase connected to the outlet (its union-find and stamps
         // only; tiles the last update left alone keep their tile-local
-        // parents), then the
-        // update on blocks, which also brings the non-wetting phase's growing
-        // selection and the wetting phase's masks and tile flags up to date
-        s = shrink_marks_binary(g_w, mp_img, 2, shape, bc, pad, nullptr, Bx.outlet, w.err, st);
+        // parents), then the update on row words, which also brings the
+        // non-wetting phase's growing selection and the wetting phase's masks
+        // and tile flags up to date
+        s = shrink_marks_binary(g_w, mp_img, 2, shape, bc, pad, Bx.outlet, w.err, st);
         if (s != PMG_OK)
             break;
-        GrowSel *gn = nullptr;
-        if (g_nw.built) {
-            if (g_nw.pending) {
-                // the last update's list was never consumed: rebuild instead
-                g_nw.built = false;
-                g_nw.pending = false;
-            } else {
-                PMG_CUDA(cudaMemsetAsync(g_nw.count, 0, sizeof(int), st));
-                gn = &g_nw;
-            }
-        }
-        PMG_CUDA(cudaMemsetAsync(w.cnt + 8, 0, 2 * sizeof(unsigned long long), st));
-        s = drain_update_blocks(mp_img, morph, shape, g_w.P, g_w.M, g_w.mark, Bx, gn, w.cnt + 8, w.cnt + 9, w.err,
-                                st, g_w.dirty, active[k] ? orange : nullptr, full_done);
+        GrowSel *gn = g_nw.built ? &g_nw : nullptr;
+        s = drain_update_rows(mp_img, active[k] ? drows : nullptr, shape, g_w, Bx, gn, w.cnt + 8, w.cnt + 9, w.err, st,
+                              active[k] ? orange : nullptr, !full_done);
         if (s == PMG_OK)
-            s = drain_totals(full_done, w.cnt + 8, w.cnt + 9, w.cnt + 10, d_counts + k, w.cnt + 1, st);
+            s = drain_totals(!full_done, w.cnt + 8, w.cnt + 9, w.cnt + 10, d_counts + k, w.cnt + 1, st);
         if (s != PMG_OK)
             break;
         full_done = true;
         if (gn)
-            g_nw.pending = true;
+            gn->pending = true;
     }
     // union-find iteration caps are checked once per curve: the status word
     // is only ever set, never cleared, during the sweep

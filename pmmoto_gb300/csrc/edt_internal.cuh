@@ -150,12 +150,16 @@ bool cap_path_ok(const float *res, const int64_t *X, int T);
 // be empty), zero making the result all zeros without the envelope passes;
 // xr: a device x range of the seed blocks (kRangeBig encoding) -- the
 // result is then written only on the x range orange receives ([lo, hi] in
-// whole blocks, lo > hi for none) and is undefined elsewhere; blk (with
-// raw_dilate): the seeds as one mask per 2x2x2 block (bit (x * 2 + y) * 2 +
-// z, blocks in C order over the ceil-halved shape) instead of E
+// whole blocks, lo > hi for none) and is undefined elsewhere; rows (with
+// raw_dilate): the seeds as row words instead of E; rows_out: the result as row
+// words instead of bytes (only where cap_rows_out)
 int morph_cap_run(const uint8_t *E, uint16_t *KA, uint16_t *KB, const int64_t *X, int T, const MorphEpi &me,
                   cudaStream_t st, int raw_dilate = 0, const unsigned long long *gate = nullptr,
-                  const int *xr = nullptr, int *orange = nullptr, const uint8_t *blk = nullptr);
+                  const int *xr = nullptr, int *orange = nullptr, const unsigned *rows = nullptr,
+                  unsigned *rows_out = nullptr);
+// The last pass can write row words: no extension, line pairs (T small enough,
+// even contiguous extent).
+bool cap_rows_out(const int64_t *X, int T, const MorphEpi &me);
 int edt_cap_run(const uint8_t *E, uint16_t *KA, uint16_t *KB, uint16_t *KC, const int64_t *X, int T,
                 cudaStream_t st);
 

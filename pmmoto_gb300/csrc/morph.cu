@@ -11,6 +11,7 @@
 // and wall rule are fused into the last envelope pass, which writes the
 // uint8 result directly.
 #include "edt_internal.cuh"
+#include "pmg_internal.cuh"
 
 namespace pmg {
 
@@ -90,16 +91,16 @@ __global__ void k_extend(const uint8_t *__restrict__ img, uint8_t *__restrict__ 
     }
 }
 
-// One byte per voxel from per-block masks (bit (x * 2 + y) * 2 + z of the
-// block over the ceil-halved shape), one thread per block.
-__global__ void k_blocks_to_bytes(const uint8_t *__restrict__ blk, uint8_t *__restrict__ out, long long s0,
-                                  long long s1, long long s2)
+// One byte per voxel from row words: one thread per block.
+__global__ void k_rows_to_bytes(const unsigned *__restrict__ V, uint8_t *__restrict__ out, long long s0, long long s1,
+                                long long s2)
 {
-    const long long b1 = (s1 + 1) / 2, b2 = (s2 + 1) / 2, nb = (s0 + 1) / 2 * b1 * b2;
+    const long long b1 = (s1 + 1) / 2, b2 = (s2 + 1) / 2, nb = (s0 + 1) / 2 * b1 * b2, nt2 = (b2 + 31) / 32;
     for (long long b = blockIdx.x * (long long)blockDim.x + threadIdx.x; b < nb;
          b += (long long)gridDim.x * blockDim.x) {
         const long long r = b / b2, c2 = b - r * b2, c0 = r / b1, c1 = r - c0 * b1;
-        const unsigned m = blk[b];
+        const unsigned *w = V + (r * nt2 + (c2 >> 5)) * 8;
+        const int sh = (int)(c2 & 31);
         for (int x = 0; x < 2; x++)
             for (int y = 0; y < 2; y++) {
                 const long long i = 2 * c0 + x, j = 2 * c1 + y;
@@ -108,7 +109,7 @@ __global__ void k_blocks_to_bytes(const uint8_t *__restrict__ blk, uint8_t *__re
                 uint8_t *row = out + (i * s1 + j) * s2;
                 for (int z = 0; z < 2; z++)
                     if (2 * c2 + z < s2)
-                        row[2 * c2 + z] = (uint8_t)((m >> ((x * 2 + y) * 2 + z)) & 1);
+                        row[2 * c2 + z] = (uint8_t)((w[(x * 2 + y) * 2 + z] >> sh) & 1u);
             }
     }
 }
@@ -116,7 +117,8 @@ __global__ void k_blocks_to_bytes(const uint8_t *__restrict__ blk, uint8_t *__re
 int morph_run(const uint8_t *img, uint8_t *out, const int64_t *shape, const int32_t *bc,
               const int32_t *pad, const int32_t *ext, const float *res, double radius, int cmp64,
               int dilate, uint8_t *E, float *A, float *B, cudaStream_t st, double thr_sq,
-              const unsigned long long *gate, const int *xr, int *orange, const uint8_t *blk)
+              const unsigned long long *gate, const int *xr, int *orange, const unsigned *rows,
+              unsigned *rows_out)
 {
     // orange: on the paths below that ignore xr the whole result is written
     if (orange) {
@@ -183,14 +185,23 @@ int morph_run(const uint8_t *img, uint8_t *out, const int64_t *shape, const int3
 
     const bool cap = T != INT_MIN && cap_path_ok(res, X, T);
     const bool any_per = G.ax[0].periodic || G.ax[1].periodic || G.ax[2].periodic;
-    if (cap && dilate && !any_per) // the row pass reads the image (or its block masks) itself
-        return morph_cap_run(img, (uint16_t *)A, (uint16_t *)B, X, T, me, st, 1, gate, xr, orange, blk);
-    if (blk) {
+    if (cap && dilate && !any_per) { // the row pass reads the image (or its row words) itself
+        unsigned *direct = rows_out && cap_rows_out(X, T, me) ? rows_out : nullptr;
+        PMG_TRY(morph_cap_run(img, (uint16_t *)A, (uint16_t *)B, X, T, me, st, 1, gate, xr, orange, rows, direct));
+        return rows_out && !direct ? bytes_to_rows(out, rows_out, shape, st) : PMG_OK;
+    }
+    if (rows_out) {
+        // the paths below write bytes
+        PMG_TRY(morph_run(img, out, shape, bc, pad, ext, res, radius, cmp64, dilate, E, A, B, st, thr_sq, gate, xr,
+                          orange, rows));
+        return bytes_to_rows(out, rows_out, shape, st);
+    }
+    if (rows) {
         // the paths below read one byte per voxel: img is the caller's scratch
         const long long nb = (shape[0] + 1) / 2 * ((shape[1] + 1) / 2) * ((shape[2] + 1) / 2);
-        const int ps__ = prof_begin("k_blocks_to_bytes", st);
-        k_blocks_to_bytes<<<grid_for(nb, 256, 152LL * 32), 256, 0, st>>>(blk, const_cast<uint8_t *>(img), shape[0],
-                                                                          shape[1], shape[2]);
+        const int ps__ = prof_begin("k_rows_to_bytes", st);
+        k_rows_to_bytes<<<grid_for(nb, 256, 152LL * 32), 256, 0, st>>>(rows, const_cast<uint8_t *>(img), shape[0],
+                                                                        shape[1], shape[2]);
         prof_end(ps__, (double)nb * 9, st);
         PMG_CHECK_LAUNCH();
     }
@@ -375,8 +386,7 @@ extern "C" int pmg_morph(const uint8_t *img, uint8_t *out, const int64_t shape[3
     uint8_t *E = (uint8_t *)buf;
     float *A = (float *)((char *)buf + (((size_t)nvox + 255) & ~(size_t)255));
     float *B = A + nvox;
-    int s = morph_run(img, out, shape, bc, pad, ext, res, radius, cmp64, dilate, E, A, B, st, ball_sq, nullptr,
-                      nullptr, nullptr, nullptr);
+    int s = morph_run(img, out, shape, bc, pad, ext, res, radius, cmp64, dilate, E, A, B, st, ball_sq);
     int s2 = scratch_free(buf, st);
     return s != PMG_OK ? s : s2;
 }

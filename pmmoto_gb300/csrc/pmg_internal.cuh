@@ -5,14 +5,18 @@
 
 namespace pmg {
 
-// blk (dilation): the seeds as per-block masks (bit (x * 2 + y) * 2 + z over
-// the ceil-halved shape); img is then scratch of one byte per voxel, written
-// only on the paths that need the seeds as bytes.
+// rows (dilation): the seeds as row words (cc.cu: eight words per 32 2x2x2
+// blocks of a row, bit c of word (x * 2 + y) * 2 + z for that voxel of block c;
+// rows_bytes(shape)); img is then scratch of one byte per voxel, written only
+// on the paths that need the seeds as bytes.  rows_out: the result as row words
+// instead of bytes in out, which then is scratch too.
 int morph_run(const uint8_t *img, uint8_t *out, const int64_t *shape, const int32_t *bc,
               const int32_t *pad, const int32_t *ext, const float *res, double radius, int cmp64,
               int dilate, uint8_t *E, float *A, float *B, cudaStream_t st, double thr_sq = -1.0,
               const unsigned long long *gate = nullptr, const int *xr = nullptr, int *orange = nullptr,
-              const uint8_t *blk = nullptr);
+              const unsigned *rows = nullptr, unsigned *rows_out = nullptr);
+size_t rows_bytes(const int64_t *shape);
+int bytes_to_rows(const uint8_t *img, unsigned *V, const int64_t *shape, cudaStream_t st);
 size_t morph_scratch_bytes(const int64_t *shape, const int32_t *bc, const int32_t *ext);
 int erosion_edt_run(const uint8_t *img, float *D, const int64_t *shape, const int32_t *bc,
                     const int32_t *pad, const float *res, int unit_res, uint8_t *E, float *A,
@@ -48,19 +52,22 @@ struct GrowSel {
     int *P = nullptr;
     uint8_t *M = nullptr;
     uint8_t *mark = nullptr;
-    int *list = nullptr;
-    int *count = nullptr;
+    // row words; per 32 blocks of a row, the blocks that changed since the last
+    // step's unions and those not yet connected to the inlet
+    unsigned *V = nullptr;
+    unsigned *N = nullptr;
+    unsigned *U = nullptr;
+    int2 *pairs = nullptr; // blocks to unite (npairs of them)
+    int *npairs = nullptr;
+    int stamp = 0; // of the last step's inlet marks
     bool built = false;
-    // masks already brought up to date and grown blocks listed by the producer
-    // of the set (the drainage update); the next step skips its mask pass
+    // masks and words already brought up to date by the producer of the set
+    // (the drainage update); the next step skips its mask pass
     bool pending = false;
     // blocks that grow at each step, known in advance (step_lists_build):
     // step k's blocks are ev[off[k] .. off[k + 1])
     int *ev = nullptr;
     int *off = nullptr;
-    // profiler label of the union step, and its unit counter (-1: none)
-    const char *unite_label = "k_grow_unite";
-    int unite_units = -1;
 };
 // Per-step lists of the blocks of a step volume S (steps < nsteps; 255:
 // never) that grow at that step, in one allocation *mem (freed by the caller).
@@ -70,68 +77,48 @@ void grow_sel_init(GrowSel &g, void *mem, const int64_t *shape);
 int select_grow_binary(GrowSel &g, const uint8_t *img, int fgval, void *out, const int64_t *shape,
                        const int32_t *bc, const int32_t *pad, const int64_t *inlet_box, const int64_t *outlet_box,
                        int mode, int *err, cudaStream_t st, unsigned long long *kept = nullptr);
-int select_grow_erode(GrowSel &g, const uint16_t *E, int T, void *out, const int64_t *shape, const int32_t *bc,
-                      const int32_t *pad, const int64_t *inlet_box, const int64_t *outlet_box, int mode, int *err,
-                      cudaStream_t st, unsigned long long *kept = nullptr);
-// The step of a growing selection up to the inlet marks (no output) ...
-int grow_marks_erode(GrowSel &g, const uint16_t *E, int T, const int64_t *shape, const int32_t *bc,
-                     const int32_t *pad, const int64_t *inlet_box, int *err, cudaStream_t st);
-int grow_marks_binary(GrowSel &g, const uint8_t *img, int fgval, const int64_t *shape, const int32_t *bc,
-                      const int32_t *pad, const int64_t *inlet_box, int *err, cudaStream_t st);
-// (the set: voxels with step S <= k)
-int grow_marks_step(GrowSel &g, const uint8_t *S, int k, const int64_t *shape, const int32_t *bc,
-                    const int32_t *pad, const int64_t *inlet_box, int *err, cudaStream_t st);
-// Both growing selections of a drainage radius up to their inlet marks (the
+// Both growing selections of a drainage radius up to their inlet stamps (the
 // eroded space a: step k of S when S is given, else E > T; the non-wetting
-// phase b: fgval in img) in one union launch and one marks launch, once both
-// are built and no axis is periodic; the two steps above otherwise.
+// phase b: fgval in img), no axis being periodic.
 int grow_marks_pair(GrowSel &a, const uint8_t *S, int k, const uint16_t *E, int T, GrowSel &b, const uint8_t *img,
                     int fgval, const int64_t *shape, const int32_t *bc, const int32_t *pad, const int64_t *inlet_box,
                     int *err, cudaStream_t st);
-// ... and the inlet selection of a constrained by b (when *b_count > 0) in one
-// pass; kept counts a's inlet-connected voxels.
-// xr (optional): the x range of the output's set (kRangeBig encoding);
-// blocks: out holds one mask per 2x2x2 block (bit (x * 2 + y) * 2 + z)
-int grow_pair_select(GrowSel &a, GrowSel &b, const unsigned long long *b_count, uint8_t *out,
-                     const int64_t *shape, int *err, cudaStream_t st, unsigned long long *kept, int *xr = nullptr,
-                     bool blocks = false);
+// ... and the inlet selection of a constrained by b (when *b_count > 0) as row
+// words; kept counts a's inlet-connected voxels, xr receives the x range of the
+// output's set (kRangeBig encoding).
+int grow_pair_select(GrowSel &a, GrowSel &b, const unsigned long long *b_count, unsigned *out, const int64_t *shape,
+                     int *err, cudaStream_t st, unsigned long long *kept, int *xr);
 // Selection of a set that only shrinks (the drainage's wetting phase): full
-// block union-find every step, but tiles the producer did not flag reuse
-// their tile-local parents Pl.  Scratch of shrink_sel_bytes(shape) bytes.
+// block union-find every step, but tiles the producer did not flag keep their
+// tile-local parents.  Scratch of shrink_sel_bytes(shape) bytes.
 struct ShrinkSel {
     int *P = nullptr;
-    int *Pl = nullptr;
+    unsigned *R = nullptr; // tile roots, one bit per block
+    unsigned *T = nullptr; // blocks found cut off from the outlet, one bit per block
     uint8_t *M = nullptr;
     uint8_t *mark = nullptr;
     int *dirty = nullptr; // per tile: changed since the last step
     unsigned *V = nullptr; // row words of the masks
     int ntiles = 0;
+    int stamp = 0; // of the last step's outlet marks
     bool built = false;
 };
 size_t shrink_sel_bytes(const int64_t *shape);
 void shrink_sel_init(ShrinkSel &g, void *mem, const int64_t *shape);
 int shrink_marks_binary(ShrinkSel &g, const uint8_t *img, int fgval, const int64_t *shape, const int32_t *bc,
-                        const int32_t *pad, const int64_t *inlet_box, const int64_t *outlet_box, int *err,
-                        cudaStream_t st);
-// Block union-find of the voxels equal to fgval with inlet / outlet marks,
-// without a selected image (parents left unflattened).
-int bcc_marks_binary(const uint8_t *img, int fgval, const int64_t *shape, const int32_t *bc, const int32_t *pad,
-                     const int64_t *inlet_box, const int64_t *outlet_box, int *P, uint8_t *M, uint8_t *mark,
-                     int *err, cudaStream_t st);
-// The drainage update on blocks, reading the wetting phase's outlet
-// connection from its block union-find (P, M, mark from bcc_marks_binary with
-// the outlet box); maintains g_nw's masks when given.
-// With wdirty, M (the wetting phase's masks) is brought up to date and the
-// tiles whose masks changed are flagged.  orange (device, voxel x range
-// [lo, hi] in whole blocks, null: everything): the only blocks that can
-// change; ranged: the counts are changes since the last update rather than
-// totals (drain_totals keeps the running totals).
-int drain_update_blocks(uint8_t *mp, const uint8_t *morph, const int64_t *shape, int *P, uint8_t *M,
-                        const uint8_t *mark, const Boxes &B, GrowSel *g_nw, unsigned long long *cnt2_own,
-                        unsigned long long *cnt1, int *err, cudaStream_t st, int *wdirty = nullptr,
-                        const int *orange = nullptr, bool ranged = false);
-int drain_totals(bool ranged, const unsigned long long *cnt2, const unsigned long long *cnt1, unsigned long long *tot,
-                 unsigned long long *sat_out, unsigned long long *ones_out, cudaStream_t st);
+                        const int32_t *pad, const int64_t *outlet_box, int *err, cudaStream_t st);
+// The drainage update on row words: D the dilation (null: none), defined on
+// the voxel x range orange (device, [lo, hi] in whole blocks, null:
+// everything); full: every voxel and the reservoir slabs, the counts being all
+// voxels of value 2 in the own box and the voxels newly 1; otherwise only the
+// dilation's range, the counts being changes (drain_totals keeps the running
+// totals and clears them).  w's masks, words and tile flags are brought up to
+// date, and g_nw's when given.
+int drain_update_rows(uint8_t *mp, const unsigned *D, const int64_t *shape, ShrinkSel &w, const Boxes &B, GrowSel *g_nw,
+                      unsigned long long *cnt2, unsigned long long *cnt1, int *err, cudaStream_t st, const int *orange,
+                      bool full);
+int drain_totals(bool full, unsigned long long *cnt2, unsigned long long *cnt1, unsigned long long *tot,
+                 unsigned long long *sat_out, unsigned long long *ones, cudaStream_t st);
 int check_err(int *err, cudaStream_t st);
 int check_volume(const int64_t *shape);
 
