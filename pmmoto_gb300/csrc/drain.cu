@@ -158,6 +158,49 @@ __global__ void k_step_volume(const uint16_t *__restrict__ KC, uint8_t *__restri
     }
 }
 
+// ... of any voxel size, from the float distances: the first radius at which the
+// erosion (k_erode_from_edt's comparison) keeps the voxel.  The comparisons are
+// monotone (thr never rises), so a bisection finds it.  thr: of the squared
+// distance (sq), or of the distance; step: the radius index of each threshold.
+// Bound by the four bytes read and one written per voxel: 20 erosions written
+// and labelled again took 2.0 ms of the 167 x 133 x 150 drainage.
+__global__ void k_step_volume_f32(const float *__restrict__ D, uint8_t *__restrict__ S,
+                                  const double *__restrict__ thr, const uint8_t *__restrict__ step, int nthr, int sq,
+                                  long long s0, long long s1, long long s2, unsigned walls)
+{
+    __shared__ double s_thr[256];
+    __shared__ uint8_t s_step[256];
+    for (int v = threadIdx.x; v < nthr; v += blockDim.x) {
+        s_thr[v] = thr[v];
+        s_step[v] = step[v];
+    }
+    __syncthreads();
+    const long long rows = s0 * s1;
+    const int lane = threadIdx.x & 31;
+    const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long r = warp; r < rows; r += nwarps) {
+        const long long i = r / s1, j = r - (r / s1) * s1;
+        const bool wrow = ((walls & 1u) && i == 0) || ((walls & 2u) && i == s0 - 1) || ((walls & 4u) && j == 0) ||
+                          ((walls & 8u) && j == s1 - 1);
+        const long long base = r * s2;
+        for (long long k = lane; k < s2; k += 32) {
+            const float v = D[base + k];
+            const double d = sq ? (double)v : (double)__fsqrt_rn(v);
+            int lo = 0, hi = nthr; // the first threshold below d (none: nthr)
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (d <= s_thr[mid])
+                    lo = mid + 1;
+                else
+                    hi = mid;
+            }
+            const bool wall = wrow || ((walls & 16u) && k == 0) || ((walls & 32u) && k == s2 - 1);
+            S[base + k] = wall || lo == nthr ? (uint8_t)255 : s_step[lo];
+        }
+    }
+}
+
 static void morph_split(Work &w, const int64_t *shape, const int32_t *bc, const int32_t *ext,
                         uint8_t *&E, float *&A, float *&B)
 {
@@ -478,10 +521,52 @@ extern "C" int pmg_drainage_ext(const uint8_t *pm_img, uint8_t *mp_img, const in
                 last = Te[(size_t)k];
             }
     }
+    // the thresholds of the float distances (De), squared or not, likewise
+    std::vector<double> fthr;
+    std::vector<uint8_t> fstep;
+    bool fsq = false;
+    if (De && n_radii <= 254) {
+        bool ok = true;
+        for (int k = 0; k < n_radii && ok; k++)
+            if (active[k]) {
+                const bool sq = ball_erode && ball_erode[k] >= 0.0;
+                const double t = sq ? ball_erode[k] : radii[k];
+                ok = fthr.empty() || (sq == fsq && t <= fthr.back());
+                fsq = sq;
+                fthr.push_back(t);
+                fstep.push_back((uint8_t)k);
+            }
+        grow_er = ok && !fthr.empty();
+    }
     // the growing eroded space as one byte per voxel: the radius index at
     // which the voxel enters (the capped distances are not needed after it)
     uint8_t *Sv = nullptr;
-    if (s == PMG_OK && grow_er && n_radii <= 254) {
+    unsigned walls = 0;
+    for (int q = 0; q < 6; q++)
+        walls |= (bc[q] == PMG_BC_WALL ? 1u : 0u) << q;
+    if (s == PMG_OK && grow_er && De) {
+        const size_t m = fthr.size(), at = ((size_t)n + 255) & ~(size_t)255;
+        s = scratch_alloc((void **)&Sv, at + m * (sizeof(double) + 1), st);
+        double *dthr = (double *)(Sv + at);
+        uint8_t *dstep = (uint8_t *)(dthr + m);
+        // (a copy from pageable memory has read its source when it returns)
+        if (s == PMG_OK && (cudaMemcpyAsync(dthr, fthr.data(), m * sizeof(double), cudaMemcpyHostToDevice, st) !=
+                                cudaSuccess ||
+                            cudaMemcpyAsync(dstep, fstep.data(), m, cudaMemcpyHostToDevice, st) != cudaSuccess))
+            s = PMG_ECUDA;
+        if (s == PMG_OK) {
+            const int ps__ = prof_begin("k_step_volume", st);
+            k_step_volume_f32<<<grid_for(shape[0] * shape[1] * 32, 256, 152LL * 64), 256, 0, st>>>(
+                De, Sv, dthr, dstep, (int)m, fsq ? 1 : 0, shape[0], shape[1], shape[2], walls);
+            prof_end(ps__, (double)n * 5, st);
+            s = cudaGetLastError() == cudaSuccess ? PMG_OK : PMG_ECUDA;
+        }
+        if (s == PMG_OK) {
+            s = scratch_free(De, st);
+            De = nullptr;
+        }
+    }
+    if (s == PMG_OK && grow_er && KC && n_radii <= 254) {
         std::vector<uint8_t> tab((size_t)Tcap + 2, 255);
         for (int v = 0; v <= Tcap + 1; v++)
             for (int k = 0; k < n_radii; k++)
@@ -498,9 +583,6 @@ extern "C" int pmg_drainage_ext(const uint8_t *pm_img, uint8_t *mp_img, const in
                     : PMG_ECUDA;
         }
         if (s == PMG_OK) {
-            unsigned walls = 0;
-            for (int q = 0; q < 6; q++)
-                walls |= (bc[q] == PMG_BC_WALL ? 1u : 0u) << q;
             const int ps__ = prof_begin("k_step_volume", st);
             k_step_volume<<<grid_for(shape[0] * shape[1] * 32, 256, 152LL * 64), 256, 0, st>>>(
                 KC, Sv, dtab, Tcap + 1, shape[0], shape[1], shape[2], walls);

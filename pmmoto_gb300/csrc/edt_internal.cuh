@@ -157,8 +157,7 @@ int morph_cap_run(const uint8_t *E, uint16_t *KA, uint16_t *KB, const int64_t *X
                   cudaStream_t st, int raw_dilate = 0, const unsigned long long *gate = nullptr,
                   const int *xr = nullptr, int *orange = nullptr, const unsigned *rows = nullptr,
                   unsigned *rows_out = nullptr);
-// The last pass can write row words: no extension, line pairs (T small enough,
-// even contiguous extent).
+// The last pass can write row words: no extension, line pairs (T small enough).
 bool cap_rows_out(const int64_t *X, int T, const MorphEpi &me);
 int edt_cap_run(const uint8_t *E, uint16_t *KA, uint16_t *KB, uint16_t *KC, const int64_t *X, int T,
                 cudaStream_t st);

@@ -36,6 +36,10 @@ namespace pmg {
 struct CapGeo {
     int X0, X1, X2;       // extended shape
     int j0, nj, k0, nk;   // unextended ranges of axes 1 and 2
+    int P2, PO;           // row pitch of the heights: X2 made even; of k_cap_mid's output
+    // the voxel pairs that cover [k0, k0 + nk)
+    __host__ __device__ int kp0() const { return k0 >> 1; }
+    __host__ __device__ int np() const { return ((k0 + nk + 1) >> 1) - (k0 >> 1); }
 };
 
 // ---- x range of the seeds -------------------------------------------------------
@@ -90,7 +94,8 @@ __device__ __forceinline__ unsigned spread16(unsigned v)
 // even and odd positions interleaved, kept in shared memory with an empty word
 // on either side), then every lane finds the nearest seeds of two adjacent
 // voxels in the three words around them with one count of leading / trailing
-// zeros each way and stores both at once.
+// zeros each way and stores both at once (rows of even pitch; the column that
+// an odd row gains holds some height, read by no one).
 // Bound by the 2 bytes written per voxel and the bit counts; from per-block
 // mask bytes with a ballot per 32 voxels and one voxel a lane the drainage's
 // dilations took 0.16 ms at 512^3, now 0.11 ms.
@@ -117,7 +122,7 @@ __global__ void __launch_bounds__(256) k_cap_rows(const uint8_t *__restrict__ E,
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     const int big = T + 1;
-    const bool pairs = !(X2 & 1); // two voxels per store
+    const int P2 = (X2 + 1) & ~1;
     // with a seed range, only the rows of its planes
     const int r0 = xr ? max(sr.hlo, 0) * rs.X1 : 0;
     const int r1 = xr ? (int)min(rows, (long long)(sr.hhi + 1) * rs.X1) : (int)rows;
@@ -163,7 +168,7 @@ __global__ void __launch_bounds__(256) k_cap_rows(const uint8_t *__restrict__ E,
                 zw[(X2 - 1) >> 5] &= ~(1u << ((X2 - 1) & 31));
         }
         __syncwarp();
-        uint16_t *dst = KA + (long long)r * X2;
+        uint16_t *dst = KA + (long long)r * P2;
         // lane l on voxels 64 c + 2 l and the next one: word 2 c + l / 16
         const int hw = lane >> 4, sh = (2 * lane) & 31;
         for (int c = 0; 64 * c < X2; c++) {
@@ -174,15 +179,8 @@ __global__ void __launch_bounds__(256) k_cap_rows(const uint8_t *__restrict__ E,
             const uint32_t L0 = __funnelshift_l(wp, wc, 31 - sh), L1 = __funnelshift_l(wp, wc, 30 - sh);
             const int d0 = min(__clz(L0), __clz(__brev(R0))), d1 = min(__clz(L1), __clz(__brev(R1)));
             const uint32_t k0 = d0 <= W ? d0 * d0 : big, k1 = d1 <= W ? d1 * d1 : big;
-            if (pairs) {
-                if (x < X2)
-                    *reinterpret_cast<uint32_t *>(dst + x) = k0 | (k1 << 16);
-            } else {
-                if (x < X2)
-                    dst[x] = (uint16_t)k0;
-                if (x + 1 < X2)
-                    dst[x + 1] = (uint16_t)k1;
-            }
+            if (x < X2)
+                *reinterpret_cast<uint32_t *>(dst + x) = k0 | (k1 << 16);
         }
         __syncwarp();
     }
@@ -268,7 +266,8 @@ __global__ void __launch_bounds__(128) k_cap_mid(const uint16_t *__restrict__ KA
         sr.load(xr, G.X0, W);
     __shared__ int ring[RING * 128];
     const long long nlines = (long long)(AX == 1 ? G.X0 : G.nj) * G.nk;
-    const long long st = AX == 1 ? (long long)G.X2 : (long long)G.X1 * G.X2;
+    const long long st = AX == 1 ? (long long)G.P2 : (long long)G.X1 * G.P2;
+    const long long sto = AX == 1 ? (long long)G.PO : (long long)G.X1 * G.PO;
     const int n = AX == 1 ? G.X1 : G.X0;
     const int seglen = (n + nseg - 1) / nseg;
     const int big = T + 1;
@@ -287,9 +286,9 @@ __global__ void __launch_bounds__(128) k_cap_mid(const uint16_t *__restrict__ KA
         if (a >= b)
             continue;
         const int x2 = G.k0 + (int)(li - q * G.nk);
-        const long long base = AX == 1 ? q * G.X1 * G.X2 + x2 : (G.j0 + q) * G.X2 + x2;
-        const uint16_t *in = KA + base;
-        uint16_t *out = KB + base;
+        const long long lrow = AX == 1 ? q * G.X1 : G.j0 + q;
+        const uint16_t *in = KA + lrow * G.P2 + x2;
+        uint16_t *out = KB + lrow * G.PO + x2;
         CapLine<RING> L{ring + threadIdx.x, 0, -1, 0};
         const int i_first = max(0, a - W), i_last = b - 1 + W; // steps; step i emits x = i - W
         int cur[kCapChunk];
@@ -299,7 +298,7 @@ __global__ void __launch_bounds__(128) k_cap_mid(const uint16_t *__restrict__ KA
             cur[u] = i_first + u < n ? (int)*pin : big;
             pin += st;
         }
-        uint16_t *po = out + (long long)a * st; // output position x = i - W
+        uint16_t *po = out + (long long)a * sto; // output position x = i - W
         for (int i0 = i_first; i0 <= i_last; i0 += kCapChunk) {
             int nxt[kCapChunk];
 #pragma unroll
@@ -314,7 +313,7 @@ __global__ void __launch_bounds__(128) k_cap_mid(const uint16_t *__restrict__ KA
                 const int x = i - W;
                 if (x >= a && x < b) {
                     *po = (uint16_t)v;
-                    po += st;
+                    po += sto;
                 }
             }
 #pragma unroll
@@ -340,16 +339,14 @@ constexpr int kPairMaxW = 20;
 // heights loaded ahead: fewer for the wide windows, whose rings hold more
 __host__ __device__ constexpr int pair_ahead(int W) { return W <= 12 ? 8 : 4; }
 
-// Lines of a pass on pairs: AX = 1, pairs over (x0 in [0, X0), x2 / 2 in
-// [k0 / 2, (k0 + nk) / 2)) along axis 1; AX = 0, pairs over (x1 in [j0, j0 +
-// nj), x2 / 2 ...) along axis 0.  Word offset of line pair li and its stride.
+// Lines of a pass on pairs: AX = 1, np pairs over (x0 in [0, X0), x2 / 2 from
+// kp0) along axis 1; AX = 0, pairs over (x1 in [j0, j0 + nj), x2 / 2 ...) along
+// axis 0.  Word offset of line pair li.
 template <int AX>
 __device__ __forceinline__ long long pair_base(const CapGeo &G, long long li, int np)
 {
     const long long q = li / np;
-    const long long kp = li - q * np;
-    const long long v = AX == 1 ? q * G.X1 * G.X2 + G.k0 : (G.j0 + q) * G.X2 + G.k0;
-    return (v >> 1) + kp;
+    return (AX == 1 ? q * G.X1 : G.j0 + q) * (G.P2 >> 1) + G.kp0() + (li - q * np);
 }
 
 template <int AX, int W>
@@ -364,9 +361,9 @@ __global__ void __launch_bounds__(256) k_cap_mid_pair(const uint16_t *__restrict
     SeedRange sr{0, 0x7fffffff, 0, 0};
     if (xr)
         sr.load(xr, G.X0, W);
-    const int np = G.nk >> 1;
+    const int np = G.np();
     const long long nlines = (long long)(AX == 1 ? G.X0 : G.nj) * np;
-    const long long st = AX == 1 ? (long long)(G.X2 >> 1) : (long long)G.X1 * (G.X2 >> 1);
+    const long long st = AX == 1 ? (long long)(G.P2 >> 1) : (long long)G.X1 * (G.P2 >> 1);
     const int n = AX == 1 ? G.X1 : G.X0;
     const int nseg = (n + seglen - 1) / seglen;
     const long long l0 = AX == 1 && xr ? (long long)max(sr.hlo, 0) * np : 0;
@@ -456,7 +453,7 @@ __global__ void __launch_bounds__(128) k_cap_last(const uint16_t *__restrict__ K
         s_w[q] = (uint8_t)isqrt_small(T - q);
     __syncthreads();
     const long long nlines = (long long)G.nj * G.nk;
-    const long long st = (long long)G.X1 * G.X2;
+    const long long st = (long long)G.X1 * G.P2;
     const int n = G.X0;
     // positions x of the line that lie in the unextended volume (and in the
     // output range of the seeds)
@@ -476,7 +473,7 @@ __global__ void __launch_bounds__(128) k_cap_last(const uint16_t *__restrict__ K
         const int istart = max(0, ax - W), iend = bx - 1 + W;
         const int x1 = G.j0 + (int)(li / G.nk);
         const int x2 = G.k0 + (int)(li - (li / G.nk) * G.nk);
-        const uint16_t *in = KB + (long long)x1 * G.X2 + x2;
+        const uint16_t *in = KB + (long long)x1 * G.P2 + x2;
         const long long jo = x1 - me.e1, ko = x2 - me.e2;
         const bool wall_jk = (me.wall[2] && jo == 0) || (me.wall[3] && jo == me.o1 - 1) ||
                              (me.wall[4] && ko == 0) || (me.wall[5] && ko == me.o2 - 1);
@@ -536,7 +533,8 @@ __global__ void __launch_bounds__(128) k_cap_last(const uint16_t *__restrict__ K
 // Pass C for small W on line pairs (pairs over (x1 in [j0, j0 + nj), x2 / 2)
 // along axis 0): x is within iff min over |d| <= W of E_B(x + d) + d^2 <= T,
 // the same test as the intervals of k_cap_last, then the same epilogue; the
-// two outputs of a pair are stored as one 16-bit word (o2 and x2 - e2 even).
+// two outputs of a pair are stored as one 16-bit word where o2 and x2 - e2 are
+// even, else byte by byte.
 // ROWS: as row words instead (no extension) -- a warp holds 64 voxels of one
 // row, whose even and odd ones are two ballots, 1 bit written per voxel; each
 // row's pairs are padded to whole warps.
@@ -570,9 +568,9 @@ __global__ void __launch_bounds__(256) k_cap_last_pair(const uint16_t *__restric
         }
         return;
     }
-    const int np0 = G.nk >> 1, np = ROWS ? (np0 + 31) & ~31 : np0;
+    const int np0 = G.np(), np = ROWS ? (np0 + 31) & ~31 : np0;
     const long long nlines = (long long)G.nj * np;
-    const long long st = (long long)G.X1 * (G.X2 >> 1);
+    const long long st = (long long)G.X1 * (G.P2 >> 1);
     const int n = G.X0;
     const int xlo = max(max(0, me.e0), sr.olo), xhi = min(min(n, me.e0 + (int)me.o0), sr.ohi + 1);
     if (xhi <= xlo)
@@ -586,6 +584,7 @@ __global__ void __launch_bounds__(256) k_cap_last_pair(const uint16_t *__restric
     const long long ost = me.o1 * me.o2;
     const int xw0 = me.wall[0] ? me.e0 : -1, xw1 = me.wall[1] ? me.e0 + (int)me.o0 - 1 : -1;
     const uint32_t *in0 = (const uint32_t *)KB;
+    const bool odd = (me.o2 | me.e2) & 1; // pairs do not start on even output bytes
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < nlines * nseg;
          g += (long long)gridDim.x * blockDim.x) {
         const int seg = (int)(g / nlines);
@@ -595,18 +594,17 @@ __global__ void __launch_bounds__(256) k_cap_last_pair(const uint16_t *__restric
         const int x1 = G.j0 + (int)q;
         const int kp = (int)(li - q * np);
         const bool live = !ROWS || kp < np0;
-        const int x2 = G.k0 + 2 * kp;
+        const int x2 = 2 * (G.kp0() + kp);
         // (the padding lanes read the row's last pair and write no bit)
-        const uint32_t *in = in0 + (((G.j0 + q) * G.X2 + G.k0) >> 1) + (ROWS ? min(kp, np0 - 1) : kp);
+        const uint32_t *in = in0 + (G.j0 + q) * (G.P2 >> 1) + G.kp0() + (ROWS ? min(kp, np0 - 1) : kp);
         const long long jo = x1 - me.e1, ko = x2 - me.e2;
         const bool wall_j = (me.wall[2] && jo == 0) || (me.wall[3] && jo == me.o1 - 1);
-        // bytes of the pair kept off the wall lines
-        uint32_t keep = (wall_j || (me.wall[4] && ko == 0) ? 0u : 0x00ffu) |
-                        (wall_j || (me.wall[5] && ko + 1 == me.o2 - 1) ? 0u : 0xff00u);
-        if (!live)
-            keep = 0u;
-        uint16_t *dst = (uint16_t *)(me.out + jo * me.o2 + ko + (long long)(a - me.e0) * ost);
-        const long long ostw = ost >> 1;
+        // bytes of the pair inside the output and off the wall lines
+        const bool in0k = live && ko >= 0, in1k = live && ko + 1 < me.o2;
+        auto wall_k = [&](long long k) { return (me.wall[4] && k == 0) || (me.wall[5] && k == me.o2 - 1); };
+        const uint32_t keep = (!in0k || wall_j || wall_k(ko) ? 0u : 0x00ffu) |
+                              (!in1k || wall_j || wall_k(ko + 1) ? 0u : 0xff00u);
+        uint8_t *dst = me.out + jo * me.o2 + ko + (long long)(a - me.e0) * ost;
         uint32_t win[R];
 #pragma unroll
         for (int s = 0; s < R; s++) {
@@ -645,8 +643,15 @@ __global__ void __launch_bounds__(256) k_cap_last_pair(const uint16_t *__restric
                         v &= keep;
                         if (y == xw0 || y == xw1)
                             v = 0u;
-                        *dst = (uint16_t)v;
-                        dst += ostw;
+                        if (!odd) {
+                            *reinterpret_cast<uint16_t *>(dst) = (uint16_t)v;
+                        } else {
+                            if (in0k)
+                                dst[0] = (uint8_t)v;
+                            if (in1k)
+                                dst[1] = (uint8_t)(v >> 8);
+                        }
+                        dst += ost;
                     }
                 }
                 const int yn = y + W + 1 + pair_ahead(W);
@@ -688,7 +693,7 @@ static void launch_mid_pair_w(const uint16_t *in, uint16_t *out, const CapGeo &G
 {
     const int n = AX == 1 ? G.X1 : G.X0;
     const int seglen = pair_seglen(W);
-    const long long lines = (long long)(AX == 1 ? G.X0 : G.nj) * (G.nk >> 1);
+    const long long lines = (long long)(AX == 1 ? G.X0 : G.nj) * G.np();
     const long long work = lines * ((n + seglen - 1) / seglen);
     k_cap_mid_pair<AX, W><<<grid_for(work, 256, 1LL << 30), 256, 0, st>>>(in, out, G, T, gate, xr, seglen, units);
 }
@@ -706,7 +711,7 @@ static void launch_last_pair_w(const uint16_t *KB, const CapGeo &G, int T, const
                                unsigned long long *units)
 {
     const int seglen = pair_seglen(W);
-    const long long np = rows_out ? ((G.nk >> 1) + 31) & ~31 : G.nk >> 1;
+    const long long np = rows_out ? (G.np() + 31) & ~31 : G.np();
     const long long work = G.nj * np * ((G.X0 + seglen - 1) / seglen);
     const unsigned grid = grid_for(work, 256, 1LL << 30);
     if (rows_out)
@@ -724,9 +729,8 @@ static void launch_last_pair(const uint16_t *KB, const CapGeo &G, int T, int W, 
     });
 }
 
-// Line pairs need even x2 extents and starts (32-bit words of two heights,
-// 16-bit output words).
-static bool pair_ok(const CapGeo &G, int W) { return W <= kPairMaxW && !((G.X2 | G.k0 | G.nk) & 1); }
+// Line pairs: windows that fit the registers, output rows of the same pitch.
+static bool pair_ok(const CapGeo &G, int W) { return W <= kPairMaxW && G.PO == G.P2; }
 
 // the ring holds the live parabolas, at most 2W + 2
 template <int AX>
@@ -771,7 +775,7 @@ bool cap_rows_out(const int64_t *X, int T, const MorphEpi &me)
     while ((W + 1) * (W + 1) <= T)
         W++;
     const bool plain = me.e0 == 0 && me.e1 == 0 && me.e2 == 0 && me.o0 == X[0] && me.o1 == X[1] && me.o2 == X[2];
-    return plain && me.dilate && W <= kPairMaxW && !(X[2] & 1);
+    return plain && me.dilate && W <= kPairMaxW;
 }
 
 int morph_cap_run(const uint8_t *E, uint16_t *KA, uint16_t *KB, const int64_t *X, int T, const MorphEpi &me,
@@ -797,6 +801,7 @@ int morph_cap_run(const uint8_t *E, uint16_t *KA, uint16_t *KB, const int64_t *X
     G.nj = (int)me.o1;
     G.k0 = me.e2;
     G.nk = (int)me.o2;
+    G.P2 = G.PO = (G.X2 + 1) & ~1;
     const long long rows = (long long)G.X0 * G.X1;
     {
         const int block = 256;
@@ -848,6 +853,7 @@ int edt_cap_run(const uint8_t *E, uint16_t *KA, uint16_t *KB, uint16_t *KC, cons
     G.nj = G.X1;
     G.k0 = 0;
     G.nk = G.X2;
+    G.P2 = G.PO = (G.X2 + 1) & ~1;
     const long long rows = (long long)G.X0 * G.X1;
     const long long vox = rows * G.X2;
     {
@@ -870,6 +876,7 @@ int edt_cap_run(const uint8_t *E, uint16_t *KA, uint16_t *KB, uint16_t *KC, cons
     {
         const long long lines = (long long)G.nj * G.nk;
         const int ps__ = prof_begin("k_cap_mid0", st);
+        G.PO = G.X2; // the caller's volume
         PMG_TRY(launch_cap_mid<0>(KB, KC, G, T, W, lines, st));
         prof_end(ps__, (double)vox * 4, st);
     }
