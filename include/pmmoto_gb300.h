@@ -220,6 +220,19 @@ int pmg_porosimetry(const uint8_t *pm_img, const uint8_t *mp_img, uint8_t *out,
                     double ball_erode, double ball_dilate, void *stream);
 
 /*
+ * pore_size_distribution (filters/porosimetry.py:163-227): for the radii in the
+ * given order, out (float64, device) receives the first radius whose opening
+ * (pmg_porosimetry with equal radii and no multiphase constraint) covers a
+ * voxel of pm_img equal to 1, and 0 elsewhere.  radii, cmp64, ball_* (host
+ * arrays of n_radii) and ratios (3 per radius) as in pmg_porosimetry.
+ */
+int pmg_pore_sizes(const uint8_t *pm_img, double *out, const int64_t shape[3],
+                   const int32_t bc[6], const int32_t pad[6], const int64_t inlet_box[6],
+                   const float res[3], int32_t n_radii, const double *radii,
+                   const int32_t *cmp64, const int32_t *ratios, const double *ball_erode,
+                   const double *ball_dilate, int32_t inlet, void *stream);
+
+/*
  * drainage, standard method (filters/equilibrium_distribution.py:25-179)
  * with mode="distance", on the device.  For each of n_radii probe radii
  * (float64, host array, in capillary-pressure order): when active[k] the

@@ -10,6 +10,8 @@
 // All images stay on the device between steps; the host reads back only the
 // two phase-existence counts porosimetry branches on and, at the end, the
 // per-pressure counts.
+#include <algorithm>
+#include <cmath>
 #include <vector>
 
 #include "edt_internal.cuh"
@@ -57,8 +59,17 @@ struct ErodeThr {
     int wall[6];
 };
 
+// Rows of a volume inside an extended one: the first voxel at lo.
+struct ExtRows {
+    long long X1, X2, lo0, lo1, lo2;
+    __device__ __forceinline__ long long row(long long i, long long j) const
+    {
+        return ((i + lo0) * X1 + j + lo1) * X2 + lo2;
+    }
+};
+
 __global__ void k_erode_from_edt(const float *__restrict__ D, uint8_t *__restrict__ out, long long s0,
-                                 long long s1, long long s2, ErodeThr T)
+                                 long long s1, long long s2, ErodeThr T, ExtRows X)
 {
     const long long rows = s0 * s1;
     const int lane = threadIdx.x & 31;
@@ -69,8 +80,9 @@ __global__ void k_erode_from_edt(const float *__restrict__ D, uint8_t *__restric
         const bool wrow = (T.wall[0] && i == 0) || (T.wall[1] && i == s0 - 1) || (T.wall[2] && j == 0) ||
                           (T.wall[3] && j == s1 - 1);
         const long long base = r * s2;
+        const float *src = D + X.row(i, j);
         for (long long k = lane; k < s2; k += 32) {
-            const float v = D[base + k];
+            const float v = src[k];
             bool within;
             if (T.thr_sq >= 0.0) {
                 within = (double)v <= T.thr_sq;
@@ -163,7 +175,7 @@ __global__ void k_step_volume(const uint16_t *__restrict__ KC, uint8_t *__restri
 // monotone (thr never rises), so a bisection finds it.  thr: of the squared
 // distance (sq), or of the distance; step: the radius index of each threshold.
 // Bound by the four bytes read and one written per voxel: 20 erosions written
-// and labelled again took 2.0 ms of the 167 x 133 x 150 drainage.
+// and labelled again took 2.0 of 5.6 ms of a 150 x 121 x 99 drainage.
 __global__ void k_step_volume_f32(const float *__restrict__ D, uint8_t *__restrict__ S,
                                   const double *__restrict__ thr, const uint8_t *__restrict__ step, int nthr, int sq,
                                   long long s0, long long s1, long long s2, unsigned walls)
@@ -281,7 +293,7 @@ static int porosimetry_run(const uint8_t *pm, uint8_t *out, const int64_t *shape
             T.wall[q] = bc[q] == PMG_BC_WALL;
         const int ps__ = prof_begin("k_erode_from_edt", st);
         k_erode_from_edt<<<grid_for(shape[0] * shape[1] * 32, 256, 152LL * 64), 256, 0, st>>>(
-            De, w.t1, shape[0], shape[1], shape[2], T);
+            De, w.t1, shape[0], shape[1], shape[2], T, ExtRows{shape[1], shape[2], 0, 0, 0});
         prof_end(ps__, (double)n * 5, st);
         PMG_CHECK_LAUNCH();
     } else {
@@ -332,6 +344,59 @@ static int porosimetry_run(const uint8_t *pm, uint8_t *out, const int64_t *shape
         PMG_CUDA(cudaMemcpyAsync(out, cur, (size_t)n, cudaMemcpyDeviceToDevice, st));
     }
     return PMG_OK;
+}
+
+// ---- pore size distribution ---------------------------------------------------------
+// Voxels whose shared erosion distance lies too close to a radius's threshold
+// for its decision to be the one of that radius's own distances (pmg_pore_sizes
+// below): flag[k] of radius k.  thr: squared thresholds; top: clear of all of them; a1, a2, x1, x2: squared
+// spacings and extended lengths of the two envelope passes.
+__global__ void k_near_thresholds(const float *__restrict__ D, long long s0, long long s1, long long s2, ExtRows X,
+                                  const float *__restrict__ thr, int nthr, float top, float a1, float x1, float a2,
+                                  float x2, int *flag)
+{
+    const long long rows = s0 * s1;
+    const int lane = threadIdx.x & 31;
+    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; r < rows; r += nwarps) {
+        const float *src = D + X.row(r / s1, r % s1);
+        for (long long k = lane; k < s2; k += 32) {
+            const float v = src[k];
+            if (v > top)
+                continue;
+            const float R1 = sqrtf(v / a1), R2 = sqrtf(v / a2);
+            const float band = 3.6e-7f * (a1 * (2.0f * R1 + 1.0f) * (7.0f * R1 + 3.0f * x1 + 8.0f) +
+                                          a2 * (2.0f * R2 + 1.0f) * (7.0f * R2 + 3.0f * x2 + 8.0f)) +
+                               4e-6f * v;
+            for (int q = 0; q < nthr; q++)
+                if (fabsf(v - thr[q]) <= band)
+                    flag[q] = 1;
+        }
+    }
+}
+
+// The radius at the pore voxels that this opening is the first to cover.
+__global__ void k_first_cover(const uint8_t *__restrict__ pm, const uint8_t *__restrict__ cover,
+                              double *__restrict__ out, double radius, long long n)
+{
+    const long long step = (long long)gridDim.x * blockDim.x, n4 = n >> 2;
+    auto put = [&](long long i) {
+        if (out[i] == 0.0)
+            out[i] = radius;
+    };
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n4; q += step) {
+        const uchar4 c = reinterpret_cast<const uchar4 *>(cover)[q];
+        if (!(c.x | c.y | c.z | c.w))
+            continue;
+        for (int e = 0; e < 4; e++) {
+            const uint8_t v = e == 0 ? c.x : e == 1 ? c.y : e == 2 ? c.z : c.w;
+            if (v == 1 && pm[4 * q + e] == 1)
+                put(4 * q + e);
+        }
+    }
+    for (long long i = 4 * n4 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += step)
+        if (cover[i] == 1 && pm[i] == 1)
+            put(i);
 }
 
 static int ext_of(const int32_t *bc, const int32_t *pad, const int32_t *ratio, int32_t *ext)
@@ -389,6 +454,178 @@ extern "C" int pmg_porosimetry(const uint8_t *pm_img, const uint8_t *mp_img, uin
     if (s == PMG_OK)
         s = check_err(w.err, st);
     int s2 = scratch_free(w.base, st);
+    return s != PMG_OK ? s : s2;
+}
+
+// The openings of a pore size distribution (porosimetry.py:199-227) share one
+// erosion distance field where that gives every radius its own decisions.  A
+// radius's own field is that of the image extended by its own reach; the field
+// of the largest extension holds every seed of it and, beyond, only seeds
+// farther than the radius.  What may differ is which of two parabolas within
+// rounding (edt_scan.cu's eta, once per envelope pass) the reference takes, as
+// positions are counted from another origin: a radius with a voxel whose
+// distance lies within twice that of the threshold is eroded by itself
+// (k_near_thresholds).  Isotropic power-of-two voxels have exact fields.
+// 25 fields of a periodic 200^3 pack cost 11 of 13.5 ms of its kernels.
+extern "C" int pmg_pore_sizes(const uint8_t *pm_img, double *out, const int64_t shape[3], const int32_t bc[6],
+                              const int32_t pad[6], const int64_t inlet_box[6], const float res[3], int32_t n_radii,
+                              const double *radii, const int32_t *cmp64, const int32_t *ratios,
+                              const double *ball_erode, const double *ball_dilate, int32_t inlet, void *stream)
+{
+    PMG_TRY(check_common(shape, bc, pad));
+    if (!pm_img || !out || !res || n_radii < 0 ||
+        (n_radii > 0 && (!radii || !cmp64 || !ratios || !ball_erode || !ball_dilate))) {
+        set_error("pmg_pore_sizes: null argument");
+        return PMG_EINVAL;
+    }
+    cudaStream_t st = as_stream(stream);
+    const long long n = shape[0] * shape[1] * shape[2];
+    PMG_CUDA(cudaMemsetAsync(out, 0, (size_t)n * sizeof(double), st));
+    if (n_radii == 0)
+        return PMG_OK;
+    Boxes Bx{};
+    for (int q = 0; q < 6; q++) {
+        Bx.inlet[q] = inlet_box ? inlet_box[q] : -1;
+        Bx.outlet[q] = -1;
+    }
+    // the largest extension, and each radius's
+    std::vector<int32_t> ext((size_t)n_radii * 6);
+    int32_t big[6] = {0, 0, 0, 0, 0, 0};
+    size_t mb = 0;
+    for (int k = 0; k < n_radii; k++) {
+        int32_t *e = ext.data() + 6 * (size_t)k;
+        ext_of(bc, pad, ratios + 3 * k, e);
+        for (int q = 0; q < 6; q++)
+            big[q] = e[q] > big[q] ? e[q] : big[q];
+        const size_t b = morph_scratch_bytes(shape, bc, e);
+        mb = b > mb ? b : mb;
+    }
+    Work w{};
+    PMG_TRY(work_alloc(w, shape, mb, st));
+    PMG_CUDA(cudaMemsetAsync(w.err, 0, sizeof(int), st));
+    int s = PMG_OK;
+    const bool unit_res = ball_erode[0] >= 0.0;
+    const float unit[3] = {1.0f, 1.0f, 1.0f};
+    const float *r = unit_res ? unit : res;
+    // radii that may share: their reach lies inside their own extension
+    std::vector<char> shared((size_t)n_radii, 0);
+    int n_shared = 0;
+    for (int k = 0; k < n_radii; k++) {
+        bool ok = (ball_erode[k] >= 0.0) == unit_res;
+        const double reach = unit_res ? std::sqrt(ball_erode[k]) : radii[k];
+        for (int d = 0; d < 3 && ok; d++)
+            if (bc[2 * d] == PMG_BC_PERIODIC)
+                ok = reach <= (double)ext[6 * (size_t)k + 2 * d] * r[d] &&
+                     reach <= (double)ext[6 * (size_t)k + 2 * d + 1] * r[d];
+        shared[(size_t)k] = ok;
+        n_shared += ok;
+    }
+    float *D = nullptr;
+    void *mem = nullptr;
+    ExtRows XR{};
+    if (n_shared > 1) {
+        const size_t xb = morph_scratch_bytes(shape, bc, big);
+        long long nx = 1;
+        for (int d = 0; d < 3; d++)
+            nx *= shape[d] + (bc[2 * d] == PMG_BC_PERIODIC ? big[2 * d] + big[2 * d + 1] : 0);
+        const size_t tb = ((size_t)n_radii * 8 + 255) & ~(size_t)255;
+        bool fits = nx < INT_MAX;
+        for (int d = 0; d < 3; d++)
+            fits = fits && shape[d] + big[2 * d] + big[2 * d + 1] <= PMG_MAX_LINE;
+        if (fits && scratch_alloc(&mem, xb + 256 + tb, st) == PMG_OK) {
+            uint8_t *E = (uint8_t *)mem;
+            float *A = (float *)((char *)mem + (((size_t)nx + 255) & ~(size_t)255));
+            D = A + nx;
+            int64_t X[3], lo[3];
+            if (erosion_edt_ext_run(pm_img, D, shape, bc, pad, big, res, unit_res, E, A, X, lo, st) != PMG_OK) {
+                D = nullptr; // (no room for its scratch, say)
+                cudaGetLastError();
+            }
+            XR = ExtRows{X[1], X[2], lo[0], lo[1], lo[2]};
+            const pmg_axis_cfg plain = {0, 0, 0, 0, 1, 0, 0, 0};
+            bool exact = r[0] == r[1] && r[1] == r[2];
+            for (int d = 0; d < 3 && exact; d++)
+                exact = exact_path_ok(r[d], plain, (int)X[d]);
+            if (D && !exact) {
+                std::vector<float> thr((size_t)n_radii);
+                float top = 0.0f;
+                for (int k = 0; k < n_radii; k++)
+                    thr[(size_t)k] = (float)(unit_res ? ball_erode[k] : radii[k] * radii[k]);
+                for (float t : thr)
+                    top = t > top ? t : top;
+                top = 2.0f * top + 4.0f * std::max(r[1] * r[1], r[2] * r[2]);
+                float *dthr = (float *)((char *)mem + ((xb + 255) & ~(size_t)255));
+                int *dflag = (int *)(dthr + n_radii);
+                std::vector<int> flag((size_t)n_radii, 0);
+                s = cudaMemcpyAsync(dthr, thr.data(), sizeof(float) * (size_t)n_radii, cudaMemcpyHostToDevice, st) ==
+                                cudaSuccess &&
+                            cudaMemsetAsync(dflag, 0, sizeof(int) * (size_t)n_radii, st) == cudaSuccess
+                        ? PMG_OK
+                        : PMG_ECUDA;
+                if (s == PMG_OK) {
+                    const int ps__ = prof_begin("k_near_thresholds", st);
+                    k_near_thresholds<<<grid_for(shape[0] * shape[1] * 32, 256, 152LL * 32), 256, 0, st>>>(
+                        D, shape[0], shape[1], shape[2], XR, dthr, n_radii, top, r[1] * r[1], (float)X[1],
+                        r[2] * r[2], (float)X[2], dflag);
+                    prof_end(ps__, (double)n * 4, st);
+                    s = cudaGetLastError() == cudaSuccess &&
+                                cudaMemcpyAsync(flag.data(), dflag, sizeof(int) * (size_t)n_radii,
+                                                cudaMemcpyDeviceToHost, st) == cudaSuccess &&
+                                cudaStreamSynchronize(st) == cudaSuccess
+                            ? PMG_OK
+                            : PMG_ECUDA;
+                }
+                for (int k = 0; k < n_radii; k++)
+                    shared[(size_t)k] = shared[(size_t)k] && !flag[(size_t)k];
+            }
+        } else {
+            // no room for the field: every radius by itself
+            mem = nullptr;
+            cudaGetLastError();
+        }
+    }
+    uint8_t *E;
+    float *A, *B;
+    for (int k = 0; k < n_radii && s == PMG_OK; k++) {
+        const int32_t *e = ext.data() + 6 * (size_t)k;
+        morph_split(w, shape, bc, e, E, A, B);
+        uint8_t *cur = w.t1;
+        if (D && shared[(size_t)k]) {
+            ErodeThr T;
+            T.r32 = (float)radii[k];
+            T.r64 = radii[k];
+            T.cmp64 = cmp64[k];
+            T.thr_sq = ball_erode[k];
+            for (int q = 0; q < 6; q++)
+                T.wall[q] = bc[q] == PMG_BC_WALL;
+            const int ps__ = prof_begin("k_erode_from_edt", st);
+            k_erode_from_edt<<<grid_for(shape[0] * shape[1] * 32, 256, 152LL * 64), 256, 0, st>>>(
+                D, w.t1, shape[0], shape[1], shape[2], T, XR);
+            prof_end(ps__, (double)n * 5, st);
+            s = cudaGetLastError() == cudaSuccess ? PMG_OK : PMG_ECUDA;
+        } else {
+            s = morph_run(pm_img, w.t1, shape, bc, pad, e, res, radii[k], cmp64[k], 0, E, A, B, st, ball_erode[k]);
+        }
+        if (s == PMG_OK && inlet) {
+            s = select_run_binary(w.t1, w.t2, 1, shape, bc, pad, Bx.inlet, nullptr, PMG_SEL_INLET, -1, w.P, w.M, w.mark,
+                                  w.err, st, w.cnt);
+            cur = w.t2;
+        }
+        // (the dilation of nothing is nothing)
+        if (s == PMG_OK)
+            s = morph_run(cur, w.t3, shape, bc, pad, e, res, radii[k], cmp64[k], 1, E, A, B, st, ball_dilate[k]);
+        if (s == PMG_OK) {
+            const int ps__ = prof_begin("k_first_cover", st);
+            k_first_cover<<<grid_for(n / 4 + 1, 256, 152LL * 16), 256, 0, st>>>(pm_img, w.t3, out, radii[k], n);
+            prof_end(ps__, (double)n, st);
+            s = cudaGetLastError() == cudaSuccess ? PMG_OK : PMG_ECUDA;
+        }
+    }
+    if (s == PMG_OK && inlet)
+        s = check_err(w.err, st);
+    if (mem)
+        scratch_free(mem, st);
+    const int s2 = scratch_free(w.base, st);
     return s != PMG_OK ? s : s2;
 }
 

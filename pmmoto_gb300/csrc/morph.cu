@@ -262,6 +262,39 @@ int morph_run(const uint8_t *img, uint8_t *out, const int64_t *shape, const int3
     return PMG_OK;
 }
 
+// Squared EDT of the erosion image extended by ext on periodic axes, over the
+// whole extended volume (X, first unextended voxel at lo): D of scratch-sized
+// extended volumes as in morph_scratch_bytes (E, A scratch).  unit_res selects
+// the voxel-unit distances of the FFT-ball modes.
+int erosion_edt_ext_run(const uint8_t *img, float *D, const int64_t *shape, const int32_t *bc, const int32_t *pad,
+                        const int32_t *ext, const float *res, int unit_res, uint8_t *E, float *A, int64_t *X,
+                        int64_t *lo, cudaStream_t st)
+{
+    ExtGeo G;
+    for (int d = 0; d < 3; d++) {
+        ExtAxis &a = G.ax[d];
+        a.periodic = bc[2 * d] == PMG_BC_PERIODIC;
+        a.own_lo = pad[2 * d];
+        a.own_len = (int)(shape[d] - pad[2 * d] - pad[2 * d + 1]);
+        a.ext_lo = a.periodic ? ext[2 * d] : 0;
+        a.wall_lo = bc[2 * d] == PMG_BC_WALL;
+        a.wall_hi = bc[2 * d + 1] == PMG_BC_WALL;
+        a.S = shape[d];
+        a.X = shape[d] + (a.periodic ? ext[2 * d] + ext[2 * d + 1] : 0);
+        X[d] = a.X;
+        lo[d] = a.ext_lo;
+    }
+    {
+        const int ps__ = prof_begin("k_extend", st);
+        k_extend<<<grid_for(X[0] * X[1] * 32, 256, 152LL * 64), 256, 0, st>>>(img, E, G, 0, nullptr);
+        prof_end(ps__, (double)X[0] * X[1] * X[2] * 2, st);
+    }
+    PMG_CHECK_LAUNCH();
+    const float unit[3] = {1.0f, 1.0f, 1.0f};
+    pmg_axis_cfg plain[3] = {{0, 0, 0, 0, 1, 0, 0, 0}, {0, 0, 0, 0, 1, 0, 0, 0}, {0, 0, 0, 0, 1, 0, 0, 0}};
+    return edt3d_run(E, D, A, X, unit_res ? unit : res, plain, 4, PMG_EDT_SQUARED, st);
+}
+
 // Squared EDT of the unextended erosion image (wall planes zeroed), for
 // subdomains without periodic axes, where every radius sees this same image:
 // E is uint8 scratch of the volume, A float scratch, D receives the result.

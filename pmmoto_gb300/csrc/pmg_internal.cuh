@@ -21,6 +21,9 @@ size_t morph_scratch_bytes(const int64_t *shape, const int32_t *bc, const int32_
 int erosion_edt_run(const uint8_t *img, float *D, const int64_t *shape, const int32_t *bc,
                     const int32_t *pad, const float *res, int unit_res, uint8_t *E, float *A,
                     cudaStream_t st);
+int erosion_edt_ext_run(const uint8_t *img, float *D, const int64_t *shape, const int32_t *bc, const int32_t *pad,
+                        const int32_t *ext, const float *res, int unit_res, uint8_t *E, float *A, int64_t *X,
+                        int64_t *lo, cudaStream_t st);
 int erosion_cap_run(const uint8_t *img, uint16_t *KC, const int64_t *shape, const int32_t *bc,
                     const int32_t *pad, int Tcap, uint8_t *E, uint16_t *KA, uint16_t *KB, int *flag,
                     int *nonbinary, cudaStream_t st);

@@ -99,13 +99,22 @@ def pore_size_distribution(subdomain, porous_media, radii=None, num_radii=25, in
     morph.check_radii(subdomain, radii)
     g = geo_of(subdomain)
     pm, kind = morph.to_u8(porous_media.img)
-    out = torch.zeros(pm.shape, dtype=torch.float64, device=pm.device)
-    pore = pm == 1
-    for radius in radii:
-        tmp = porosimetry_device(g, pm, radius, radius, inlet, None, mode)
-        if bool(tmp.any()):
-            sel = pore & (out == 0) & (tmp == 1)
-            out = torch.where(sel, torch.as_tensor(float(radius), dtype=torch.float64, device=pm.device), out)
+    out = torch.empty(pm.shape, dtype=torch.float64, device=pm.device)
+    from .connected_components import _box
+
+    radii = [r for r in radii]
+    balls = [_balls(g, r, r, mode) for r in radii]
+    f64 = lambda v: np.ascontiguousarray(v, dtype=np.float64)  # noqa: E731
+    i32 = lambda v: np.ascontiguousarray(v, dtype=np.int32)  # noqa: E731
+    res32 = np.ascontiguousarray([np.float32(r) for r in g.res], dtype=np.float32)
+    st = lib().pmg_pore_sizes(_dev.ptr(pm), _dev.ptr(out), host_ptr(i64_array(pm.shape)), host_ptr(g.bc_codes()),
+                              host_ptr(g.pad_flat()), host_ptr(_box(g.face_slab("inlet"))), host_ptr(res32),
+                              len(radii), host_ptr(f64(radii)),
+                              host_ptr(i32([morph.compare_in_float64(r) for r in radii])),
+                              host_ptr(i32([morph.element_ratio(g.res, r) for r in radii])),
+                              host_ptr(f64([b[0] for b in balls])), host_ptr(f64([b[1] for b in balls])),
+                              int(bool(inlet)), _dev.stream_ptr(pm.device))
+    check(st, "pore_size_distribution")
     return _dev.give_back(out, kind)
 
 
