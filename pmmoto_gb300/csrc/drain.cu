@@ -52,10 +52,7 @@ __global__ void k_constrain(uint8_t *res, const uint8_t *__restrict__ nconn, lon
 // np.where(d <= r, 0, 1), unpad being the identity without extension), wall
 // planes forced to 0 (set_wall_bcs).  One warp per (i, j) row.
 struct ErodeThr {
-    float r32;
-    double r64;
-    int cmp64;
-    double thr_sq; // >= 0: FFT-ball mode, compare the voxel-unit squared distance
+    float lim; // within_limit of the radius
     int wall[6];
 };
 
@@ -81,16 +78,9 @@ __global__ void k_erode_from_edt(const float *__restrict__ D, uint8_t *__restric
                           (T.wall[3] && j == s1 - 1);
         const long long base = r * s2;
         const float *src = D + X.row(i, j);
+#pragma unroll 4
         for (long long k = lane; k < s2; k += 32) {
-            const float v = src[k];
-            bool within;
-            if (T.thr_sq >= 0.0) {
-                within = (double)v <= T.thr_sq;
-            } else {
-                const float dist = __fsqrt_rn(v);
-                within = T.cmp64 ? ((double)dist <= T.r64) : (dist <= T.r32);
-            }
-            uint8_t o = within ? 0 : 1;
+            uint8_t o = src[k] <= T.lim ? 0 : 1;
             if (wrow || (T.wall[4] && k == 0) || (T.wall[5] && k == s2 - 1))
                 o = 0;
             out[base + k] = o;
@@ -171,16 +161,15 @@ __global__ void k_step_volume(const uint16_t *__restrict__ KC, uint8_t *__restri
 }
 
 // ... of any voxel size, from the float distances: the first radius at which the
-// erosion (k_erode_from_edt's comparison) keeps the voxel.  The comparisons are
-// monotone (thr never rises), so a bisection finds it.  thr: of the squared
-// distance (sq), or of the distance; step: the radius index of each threshold.
+// erosion (k_erode_from_edt's comparison) keeps the voxel.  The limits never
+// rise, so a bisection finds it; step: the radius index of each limit.
 // Bound by the four bytes read and one written per voxel: 20 erosions written
 // and labelled again took 2.0 of 5.6 ms of a 150 x 121 x 99 drainage.
 __global__ void k_step_volume_f32(const float *__restrict__ D, uint8_t *__restrict__ S,
-                                  const double *__restrict__ thr, const uint8_t *__restrict__ step, int nthr, int sq,
+                                  const float *__restrict__ thr, const uint8_t *__restrict__ step, int nthr,
                                   long long s0, long long s1, long long s2, unsigned walls)
 {
-    __shared__ double s_thr[256];
+    __shared__ float s_thr[256];
     __shared__ uint8_t s_step[256];
     for (int v = threadIdx.x; v < nthr; v += blockDim.x) {
         s_thr[v] = thr[v];
@@ -197,9 +186,8 @@ __global__ void k_step_volume_f32(const float *__restrict__ D, uint8_t *__restri
                           ((walls & 8u) && j == s1 - 1);
         const long long base = r * s2;
         for (long long k = lane; k < s2; k += 32) {
-            const float v = D[base + k];
-            const double d = sq ? (double)v : (double)__fsqrt_rn(v);
-            int lo = 0, hi = nthr; // the first threshold below d (none: nthr)
+            const float d = D[base + k];
+            int lo = 0, hi = nthr; // the first limit below d (none: nthr)
             while (lo < hi) {
                 const int mid = (lo + hi) >> 1;
                 if (d <= s_thr[mid])
@@ -285,10 +273,7 @@ static int porosimetry_run(const uint8_t *pm, uint8_t *out, const int64_t *shape
         cur = w.t2;
     } else if (De) {
         ErodeThr T;
-        T.r32 = (float)r_e;
-        T.r64 = r_e;
-        T.cmp64 = cmp_e;
-        T.thr_sq = ball_e;
+        T.lim = within_limit(r_e, cmp_e, ball_e);
         for (int q = 0; q < 6; q++)
             T.wall[q] = bc[q] == PMG_BC_WALL;
         const int ps__ = prof_begin("k_erode_from_edt", st);
@@ -375,28 +360,32 @@ __global__ void k_near_thresholds(const float *__restrict__ D, long long s0, lon
     }
 }
 
-// The radius at the pore voxels that this opening is the first to cover.
+// The radius at the pore voxels that this opening is the first to cover; four
+// voxels per thread, the sizes read only where the opening covers one.
 __global__ void k_first_cover(const uint8_t *__restrict__ pm, const uint8_t *__restrict__ cover,
                               double *__restrict__ out, double radius, long long n)
 {
-    const long long step = (long long)gridDim.x * blockDim.x, n4 = n >> 2;
-    auto put = [&](long long i) {
-        if (out[i] == 0.0)
-            out[i] = radius;
-    };
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n4; q += step) {
-        const uchar4 c = reinterpret_cast<const uchar4 *>(cover)[q];
-        if (!(c.x | c.y | c.z | c.w))
-            continue;
-        for (int e = 0; e < 4; e++) {
-            const uint8_t v = e == 0 ? c.x : e == 1 ? c.y : e == 2 ? c.z : c.w;
-            if (v == 1 && pm[4 * q + e] == 1)
-                put(4 * q + e);
+    const long long step = (long long)gridDim.x * blockDim.x;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; 4 * q < n; q += step) {
+        if (4 * q + 4 <= n) {
+            const uchar4 c = reinterpret_cast<const uchar4 *>(cover)[q];
+            if (!(c.x | c.y | c.z | c.w))
+                continue;
+            double2 *o = reinterpret_cast<double2 *>(out) + 2 * q;
+            const double2 a = o[0], b = o[1];
+            const uint8_t *p = pm + 4 * q;
+            const bool s0 = c.x == 1 && p[0] == 1 && a.x == 0.0, s1 = c.y == 1 && p[1] == 1 && a.y == 0.0,
+                       s2 = c.z == 1 && p[2] == 1 && b.x == 0.0, s3 = c.w == 1 && p[3] == 1 && b.y == 0.0;
+            if (s0 | s1)
+                o[0] = make_double2(s0 ? radius : a.x, s1 ? radius : a.y);
+            if (s2 | s3)
+                o[1] = make_double2(s2 ? radius : b.x, s3 ? radius : b.y);
+        } else {
+            for (long long i = 4 * q; i < n; i++)
+                if (cover[i] == 1 && pm[i] == 1 && out[i] == 0.0)
+                    out[i] = radius;
         }
     }
-    for (long long i = 4 * n4 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += step)
-        if (cover[i] == 1 && pm[i] == 1)
-            put(i);
 }
 
 static int ext_of(const int32_t *bc, const int32_t *pad, const int32_t *ratio, int32_t *ext)
@@ -592,10 +581,7 @@ extern "C" int pmg_pore_sizes(const uint8_t *pm_img, double *out, const int64_t 
         uint8_t *cur = w.t1;
         if (D && shared[(size_t)k]) {
             ErodeThr T;
-            T.r32 = (float)radii[k];
-            T.r64 = radii[k];
-            T.cmp64 = cmp64[k];
-            T.thr_sq = ball_erode[k];
+            T.lim = within_limit(radii[k], cmp64[k], ball_erode[k]);
             for (int q = 0; q < 6; q++)
                 T.wall[q] = bc[q] == PMG_BC_WALL;
             const int ps__ = prof_begin("k_erode_from_edt", st);
@@ -710,10 +696,7 @@ extern "C" int pmg_drainage_ext(const uint8_t *pm_img, uint8_t *mp_img, const in
             if (!active[k])
                 continue;
             MorphEpi me{};
-            me.r32 = (float)radii[k];
-            me.r64 = radii[k];
-            me.cmp64 = 1;
-            me.thr_sq = ball_erode ? ball_erode[k] : -1.0;
+            me.lim = within_limit(radii[k], 1, ball_erode ? ball_erode[k] : -1.0);
             Te[(size_t)k] = morph_threshold(me, r[0] * r[0], kCapMaxT + 1);
             ok = Te[(size_t)k] >= 0 && Te[(size_t)k] <= kCapMaxT;
             Tcap = Te[(size_t)k] > Tcap ? Te[(size_t)k] : Tcap;
@@ -726,7 +709,7 @@ extern "C" int pmg_drainage_ext(const uint8_t *pm_img, uint8_t *mp_img, const in
                 float *A, *B;
                 const int32_t zero_ext[6] = {0, 0, 0, 0, 0, 0};
                 morph_split(w, shape, bc, zero_ext, E, A, B);
-                s = erosion_cap_run(pm_img, KC, shape, bc, pad, Tcap, E, (uint16_t *)A, (uint16_t *)B,
+                s = erosion_cap_run(pm_img, KC, shape, bc, pad, Tcap, (uint16_t *)A, (uint16_t *)B,
                                     (int *)((char *)w.err + 128), &nonbinary, st);
             }
             if (s == PMG_OK && nonbinary) {
@@ -758,18 +741,15 @@ extern "C" int pmg_drainage_ext(const uint8_t *pm_img, uint8_t *mp_img, const in
                 last = Te[(size_t)k];
             }
     }
-    // the thresholds of the float distances (De), squared or not, likewise
-    std::vector<double> fthr;
+    // the limits of the float distances (De) likewise
+    std::vector<float> fthr;
     std::vector<uint8_t> fstep;
-    bool fsq = false;
     if (De && n_radii <= 254) {
         bool ok = true;
         for (int k = 0; k < n_radii && ok; k++)
             if (active[k]) {
-                const bool sq = ball_erode && ball_erode[k] >= 0.0;
-                const double t = sq ? ball_erode[k] : radii[k];
-                ok = fthr.empty() || (sq == fsq && t <= fthr.back());
-                fsq = sq;
+                const float t = within_limit(radii[k], 1, ball_erode ? ball_erode[k] : -1.0);
+                ok = t == t && (fthr.empty() || t <= fthr.back());
                 fthr.push_back(t);
                 fstep.push_back((uint8_t)k);
             }
@@ -783,18 +763,18 @@ extern "C" int pmg_drainage_ext(const uint8_t *pm_img, uint8_t *mp_img, const in
         walls |= (bc[q] == PMG_BC_WALL ? 1u : 0u) << q;
     if (s == PMG_OK && grow_er && De) {
         const size_t m = fthr.size(), at = ((size_t)n + 255) & ~(size_t)255;
-        s = scratch_alloc((void **)&Sv, at + m * (sizeof(double) + 1), st);
-        double *dthr = (double *)(Sv + at);
+        s = scratch_alloc((void **)&Sv, at + m * (sizeof(float) + 1), st);
+        float *dthr = (float *)(Sv + at);
         uint8_t *dstep = (uint8_t *)(dthr + m);
         // (a copy from pageable memory has read its source when it returns)
-        if (s == PMG_OK && (cudaMemcpyAsync(dthr, fthr.data(), m * sizeof(double), cudaMemcpyHostToDevice, st) !=
+        if (s == PMG_OK && (cudaMemcpyAsync(dthr, fthr.data(), m * sizeof(float), cudaMemcpyHostToDevice, st) !=
                                 cudaSuccess ||
                             cudaMemcpyAsync(dstep, fstep.data(), m, cudaMemcpyHostToDevice, st) != cudaSuccess))
             s = PMG_ECUDA;
         if (s == PMG_OK) {
             const int ps__ = prof_begin("k_step_volume", st);
             k_step_volume_f32<<<grid_for(shape[0] * shape[1] * 32, 256, 152LL * 64), 256, 0, st>>>(
-                De, Sv, dthr, dstep, (int)m, fsq ? 1 : 0, shape[0], shape[1], shape[2], walls);
+                De, Sv, dthr, dstep, (int)m, shape[0], shape[1], shape[2], walls);
             prof_end(ps__, (double)n * 5, st);
             s = cudaGetLastError() == cudaSuccess ? PMG_OK : PMG_ECUDA;
         }

@@ -75,13 +75,16 @@ struct MorphEpi {
     long long o0, o1, o2; // unextended shape
     int e0, e1, e2;       // low-side extension per axis
     int wall[6];          // wall planes: axis0 lo/hi, axis1 lo/hi, axis2 lo/hi
-    float r32;            // radius rounded to float32
-    double r64;           // radius as float64
-    int cmp64;            // 1: compare in float64 (numpy float64 radius)
+    float lim;            // largest squared distance within the radius (within_limit)
     int dilate;           // 1: addition (1 where d <= r), 0: subtraction
-    double thr_sq;        // >= 0: compare the squared unit-resolution distance
-                          // with this integer bound instead (FFT-ball modes)
 };
+
+// The largest float v that the reference's comparison counts as within: thr_sq
+// >= 0 (FFT-ball modes): v <= thr_sq; else sqrt(v) <= r, the float root compared
+// in float64 (cmp64, a numpy float64 radius) or with r rounded to float.  The
+// root is monotone, so kernels compare the squared distance alone (the float64
+// comparison was 28 of 45 us of an erosion of 200^3 voxels).
+float within_limit(double r, int cmp64, double thr_sq);
 
 // Store of the fused morphology epilogue: "distance within the radius" at
 // position i of line g (extended coordinates) -> 0/1 of the unextended volume.
@@ -99,17 +102,7 @@ __device__ __forceinline__ void morph_put(const MorphEpi &me, const LineGeo &g, 
 }
 
 // The threshold of the epilogue on a squared distance `val`.
-__host__ __device__ __forceinline__ bool morph_within(const MorphEpi &me, float val)
-{
-    if (me.thr_sq >= 0.0)
-        return (double)val <= me.thr_sq;
-#ifdef __CUDA_ARCH__
-    const float dist = __fsqrt_rn(val);
-#else
-    const float dist = sqrtf(val); // IEEE correctly rounded, as __fsqrt_rn
-#endif
-    return me.cmp64 ? ((double)dist <= me.r64) : (dist <= me.r32);
-}
+__host__ __device__ __forceinline__ bool morph_within(const MorphEpi &me, float val) { return val <= me.lim; }
 
 __device__ __forceinline__ void morph_store(const MorphEpi &me, const LineGeo &g, int i, float val)
 {
@@ -140,27 +133,55 @@ int morph_threshold(const MorphEpi &me, float a, int lim);
 int launch_env_thresh(const float *fin, const Lines &Ls, float res, int T, const MorphEpi &me,
                       cudaStream_t st);
 
+// Geometry of an image extended on periodic axes.
+struct ExtAxis {
+    int periodic;
+    int own_lo, own_len; // own region of the padded axis
+    int ext_lo;          // low-side extension
+    int wall_lo, wall_hi;
+    long long S, X;      // padded and extended lengths
+};
+
+struct ExtGeo {
+    ExtAxis ax[3];
+};
+
+__device__ __forceinline__ long long src_index(const ExtAxis &a, long long x, bool &zero)
+{
+    const long long p = x - a.ext_lo; // coordinate in the padded image
+    if (a.periodic) {
+        long long q = (x - (a.own_lo + a.ext_lo)) % a.own_len;
+        if (q < 0)
+            q += a.own_len;
+        return q + a.own_lo;
+    }
+    if ((a.wall_lo && p == 0) || (a.wall_hi && p == a.S - 1))
+        zero = true;
+    return p;
+}
+
 // Capped integer morphology (morph_cap.cu): isotropic power-of-two voxels,
 // binary image, threshold T <= kCapMaxT; KA, KB: uint16 scratch of the
 // extended volume.
 constexpr int kCapMaxT = 1023;
 bool cap_path_ok(const float *res, const int64_t *X, int T);
-// raw_dilate: E is the unextended image of a dilation without periodic axes
-// (no k_extend copy); gate: a device count of the seeds (null: not known to
-// be empty), zero making the result all zeros without the envelope passes;
-// xr: a device x range of the seed blocks (kRangeBig encoding) -- the
-// result is then written only on the x range orange receives ([lo, hi] in
-// whole blocks, lo > hi for none) and is undefined elsewhere; rows (with
-// raw_dilate): the seeds as row words instead of E; rows_out: the result as row
-// words instead of bytes (only where cap_rows_out)
-int morph_cap_run(const uint8_t *E, uint16_t *KA, uint16_t *KB, const int64_t *X, int T, const MorphEpi &me,
-                  cudaStream_t st, int raw_dilate = 0, const unsigned long long *gate = nullptr,
-                  const int *xr = nullptr, int *orange = nullptr, const unsigned *rows = nullptr,
-                  unsigned *rows_out = nullptr);
+// img: the unextended image, read through G (erosions: flag, an int of device
+// scratch, tells whether it is binary; when not, *nonbinary is set and nothing
+// is written); gate: a device count of the seeds (null: not known to be empty),
+// zero making the result all zeros without the envelope passes; xr: a device x
+// range of the seed blocks (kRangeBig encoding) -- the result is then written
+// only on the x range orange receives ([lo, hi] in whole blocks, lo > hi for
+// none) and is undefined elsewhere; rows (dilations without periodic axes): the
+// seeds as row words instead of img; rows_out: the result as row words instead
+// of bytes (only where cap_rows_out)
+int morph_cap_run(const uint8_t *img, const ExtGeo &G, uint16_t *KA, uint16_t *KB, const int64_t *X, int T,
+                  const MorphEpi &me, cudaStream_t st, int *flag = nullptr, int *nonbinary = nullptr,
+                  const unsigned long long *gate = nullptr, const int *xr = nullptr, int *orange = nullptr,
+                  const unsigned *rows = nullptr, unsigned *rows_out = nullptr);
 // The last pass can write row words: no extension, line pairs (T small enough).
 bool cap_rows_out(const int64_t *X, int T, const MorphEpi &me);
-int edt_cap_run(const uint8_t *E, uint16_t *KA, uint16_t *KB, uint16_t *KC, const int64_t *X, int T,
-                cudaStream_t st);
+int edt_cap_run(const uint8_t *img, const ExtGeo &G, uint16_t *KA, uint16_t *KB, uint16_t *KC, const int64_t *X, int T,
+                int *flag, int *nonbinary, cudaStream_t st);
 
 int launch_pass0(const uint8_t *img, float *out, const Lines &Ls, float res,
                  const pmg_axis_cfg &cfg, cudaStream_t st);

@@ -10,42 +10,18 @@
 // the halo exchange becomes index arithmetic -- and the threshold, unpadding
 // and wall rule are fused into the last envelope pass, which writes the
 // uint8 result directly.
+#include <cmath>
+
 #include "edt_internal.cuh"
 #include "pmg_internal.cuh"
 
 namespace pmg {
 
-struct ExtAxis {
-    int periodic;
-    int own_lo, own_len; // own region of the padded axis
-    int ext_lo;          // low-side extension
-    int wall_lo, wall_hi;
-    long long S, X;      // padded and extended lengths
-};
-
-struct ExtGeo {
-    ExtAxis ax[3];
-};
-
-__device__ __forceinline__ long long src_index(const ExtAxis &a, long long x, bool &zero)
-{
-    const long long p = x - a.ext_lo; // coordinate in the padded image
-    if (a.periodic) {
-        long long q = (x - (a.own_lo + a.ext_lo)) % a.own_len;
-        if (q < 0)
-            q += a.own_len;
-        return q + a.own_lo;
-    }
-    if ((a.wall_lo && p == 0) || (a.wall_hi && p == a.S - 1))
-        zero = true;
-    return p;
-}
-
 // E[x] = img[wrap(x)] (0 on wall planes); logical_not for addition.  One warp
 // per (x0, x1) row of the extended volume: the row's source row and wall state
 // are resolved once, lanes walk x2.
 __global__ void k_extend(const uint8_t *__restrict__ img, uint8_t *__restrict__ ext, ExtGeo G,
-                         int logical_not, int *nonbinary)
+                         int logical_not)
 {
     const long long X1 = G.ax[1].X, X2 = G.ax[2].X;
     const long long rows = G.ax[0].X * X1;
@@ -84,11 +60,48 @@ __global__ void k_extend(const uint8_t *__restrict__ img, uint8_t *__restrict__ 
             uint8_t v = zero ? (uint8_t)0 : src[s2];
             if (logical_not)
                 v = v == 0 ? 1 : 0;
-            else if (v > 1 && nonbinary)
-                *nonbinary = 1;
             dst[x2] = v;
         }
     }
+}
+
+// largest float not above x
+static float float_floor(double x)
+{
+    const float f = (float)x;
+    return (double)f > x ? std::nextafter(f, -INFINITY) : f;
+}
+
+float within_limit(double r, int cmp64, double thr_sq)
+{
+    if (thr_sq >= 0.0)
+        return float_floor(thr_sq);
+    const float rf = cmp64 ? float_floor(r) : (float)r;
+    if (!(rf >= 0.0f))
+        return rf != rf ? rf : -1.0f; // no distance is within
+    float v = rf * rf;
+    while (std::sqrt(v) > rf) // (std::sqrt of a float rounds correctly)
+        v = std::nextafter(v, 0.0f);
+    while (v < INFINITY && std::sqrt(std::nextafter(v, INFINITY)) <= rf)
+        v = std::nextafter(v, INFINITY);
+    return v;
+}
+
+static ExtGeo ext_geo(const int64_t *shape, const int32_t *bc, const int32_t *pad, const int32_t *ext)
+{
+    ExtGeo G;
+    for (int d = 0; d < 3; d++) {
+        ExtAxis &a = G.ax[d];
+        a.periodic = bc[2 * d] == PMG_BC_PERIODIC;
+        a.own_lo = pad[2 * d];
+        a.own_len = (int)(shape[d] - pad[2 * d] - pad[2 * d + 1]);
+        a.ext_lo = a.periodic ? ext[2 * d] : 0;
+        a.wall_lo = bc[2 * d] == PMG_BC_WALL;
+        a.wall_hi = bc[2 * d + 1] == PMG_BC_WALL;
+        a.S = shape[d];
+        a.X = shape[d] + (a.periodic ? ext[2 * d] + ext[2 * d + 1] : 0);
+    }
+    return G;
 }
 
 // One byte per voxel from row words: one thread per block.
@@ -125,18 +138,10 @@ int morph_run(const uint8_t *img, uint8_t *out, const int64_t *shape, const int3
         k_set_int2<<<1, 32, 0, st>>>(orange, 0, (int)shape[0] - 1);
         PMG_CHECK_LAUNCH();
     }
-    ExtGeo G;
+    const ExtGeo G = ext_geo(shape, bc, pad, ext);
     int64_t X[3];
     for (int d = 0; d < 3; d++) {
-        ExtAxis &a = G.ax[d];
-        a.periodic = bc[2 * d] == PMG_BC_PERIODIC;
-        a.own_lo = pad[2 * d];
-        a.own_len = (int)(shape[d] - pad[2 * d] - pad[2 * d + 1]);
-        a.ext_lo = a.periodic ? ext[2 * d] : 0;
-        a.wall_lo = bc[2 * d] == PMG_BC_WALL;
-        a.wall_hi = bc[2 * d + 1] == PMG_BC_WALL;
-        a.S = shape[d];
-        a.X = shape[d] + (a.periodic ? ext[2 * d] + ext[2 * d + 1] : 0);
+        const ExtAxis &a = G.ax[d];
         X[d] = a.X;
         if (a.periodic && a.own_len <= 0) {
             set_error("morph: empty own region on periodic axis %d", d);
@@ -158,11 +163,8 @@ int morph_run(const uint8_t *img, uint8_t *out, const int64_t *shape, const int3
         me.wall[2 * d] = G.ax[d].wall_lo;
         me.wall[2 * d + 1] = G.ax[d].wall_hi;
     }
-    me.r32 = (float)radius;
-    me.r64 = radius;
-    me.cmp64 = cmp64;
+    me.lim = within_limit(radius, cmp64, thr_sq);
     me.dilate = dilate;
-    me.thr_sq = thr_sq;
     // the ball of the FFT modes is measured in voxels: unit resolution keeps
     // every squared distance an exact integer in float32
     const float unit[3] = {1.0f, 1.0f, 1.0f};
@@ -185,9 +187,12 @@ int morph_run(const uint8_t *img, uint8_t *out, const int64_t *shape, const int3
 
     const bool cap = T != INT_MIN && cap_path_ok(res, X, T);
     const bool any_per = G.ax[0].periodic || G.ax[1].periodic || G.ax[2].periodic;
-    if (cap && dilate && !any_per) { // the row pass reads the image (or its row words) itself
+    // The capped pipeline's row pass reads the image (or its row words) itself;
+    // it needs a binary image for an erosion (an int of B's end says so).
+    if (cap && dilate && !any_per) {
         unsigned *direct = rows_out && cap_rows_out(X, T, me) ? rows_out : nullptr;
-        PMG_TRY(morph_cap_run(img, (uint16_t *)A, (uint16_t *)B, X, T, me, st, 1, gate, xr, orange, rows, direct));
+        PMG_TRY(morph_cap_run(img, G, (uint16_t *)A, (uint16_t *)B, X, T, me, st, nullptr, nullptr, gate, xr, orange,
+                              rows, direct));
         return rows_out && !direct ? bytes_to_rows(out, rows_out, shape, st) : PMG_OK;
     }
     if (rows_out) {
@@ -217,27 +222,19 @@ int morph_run(const uint8_t *img, uint8_t *out, const int64_t *shape, const int3
         }
     }
 
-    // last int of B: "the image holds a value above 1" (erosion only; the
-    // capped pipeline needs a binary image)
-    int *flag = dilate ? nullptr : (int *)(B + total) - 1;
-    if (flag)
-        PMG_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
+    if (cap) {
+        int nonbin = 0;
+        int *flag = dilate ? nullptr : (int *)(B + total) - 1;
+        PMG_TRY(morph_cap_run(img, G, (uint16_t *)A, (uint16_t *)B, X, T, me, st, flag, &nonbin));
+        if (!nonbin)
+            return PMG_OK;
+    }
     {
         const int ps__ = prof_begin("k_extend", st);
-        k_extend<<<grid_for(X[0] * X[1] * 32, 256, 152LL * 64), 256, 0, st>>>(img, E, G, dilate, flag);
+        k_extend<<<grid_for(X[0] * X[1] * 32, 256, 152LL * 64), 256, 0, st>>>(img, E, G, dilate);
         prof_end(ps__, (double)total * 2, st);
     }
     PMG_CHECK_LAUNCH();
-
-    if (cap) {
-        int nonbin = 0;
-        if (flag) {
-            PMG_CUDA(cudaMemcpyAsync(&nonbin, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
-            PMG_CUDA(cudaStreamSynchronize(st));
-        }
-        if (!nonbin)
-            return morph_cap_run(E, (uint16_t *)A, (uint16_t *)B, X, T, me, st);
-    }
 
     // squared distances above vcap are only ever "beyond the radius"; the two
     // voxels of margin keep them out of every near-tie below it
@@ -270,23 +267,14 @@ int erosion_edt_ext_run(const uint8_t *img, float *D, const int64_t *shape, cons
                         const int32_t *ext, const float *res, int unit_res, uint8_t *E, float *A, int64_t *X,
                         int64_t *lo, cudaStream_t st)
 {
-    ExtGeo G;
+    const ExtGeo G = ext_geo(shape, bc, pad, ext);
     for (int d = 0; d < 3; d++) {
-        ExtAxis &a = G.ax[d];
-        a.periodic = bc[2 * d] == PMG_BC_PERIODIC;
-        a.own_lo = pad[2 * d];
-        a.own_len = (int)(shape[d] - pad[2 * d] - pad[2 * d + 1]);
-        a.ext_lo = a.periodic ? ext[2 * d] : 0;
-        a.wall_lo = bc[2 * d] == PMG_BC_WALL;
-        a.wall_hi = bc[2 * d + 1] == PMG_BC_WALL;
-        a.S = shape[d];
-        a.X = shape[d] + (a.periodic ? ext[2 * d] + ext[2 * d + 1] : 0);
-        X[d] = a.X;
-        lo[d] = a.ext_lo;
+        X[d] = G.ax[d].X;
+        lo[d] = G.ax[d].ext_lo;
     }
     {
         const int ps__ = prof_begin("k_extend", st);
-        k_extend<<<grid_for(X[0] * X[1] * 32, 256, 152LL * 64), 256, 0, st>>>(img, E, G, 0, nullptr);
+        k_extend<<<grid_for(X[0] * X[1] * 32, 256, 152LL * 64), 256, 0, st>>>(img, E, G, 0);
         prof_end(ps__, (double)X[0] * X[1] * X[2] * 2, st);
     }
     PMG_CHECK_LAUNCH();
@@ -303,25 +291,16 @@ int erosion_edt_run(const uint8_t *img, float *D, const int64_t *shape, const in
                     const int32_t *pad, const float *res, int unit_res, uint8_t *E, float *A,
                     cudaStream_t st)
 {
-    ExtGeo G;
-    for (int d = 0; d < 3; d++) {
-        ExtAxis &a = G.ax[d];
+    for (int d = 0; d < 3; d++)
         if (bc[2 * d] == PMG_BC_PERIODIC) {
             set_error("erosion EDT reuse needs a subdomain without periodic axes");
             return PMG_EINVAL;
         }
-        a.periodic = 0;
-        a.own_lo = pad[2 * d];
-        a.own_len = (int)(shape[d] - pad[2 * d] - pad[2 * d + 1]);
-        a.ext_lo = 0;
-        a.wall_lo = bc[2 * d] == PMG_BC_WALL;
-        a.wall_hi = bc[2 * d + 1] == PMG_BC_WALL;
-        a.S = shape[d];
-        a.X = shape[d];
-    }
+    const int32_t no_ext[6] = {0, 0, 0, 0, 0, 0};
+    const ExtGeo G = ext_geo(shape, bc, pad, no_ext);
     {
         const int ps__ = prof_begin("k_extend", st);
-        k_extend<<<grid_for(shape[0] * shape[1] * 32, 256, 152LL * 64), 256, 0, st>>>(img, E, G, 0, nullptr);
+        k_extend<<<grid_for(shape[0] * shape[1] * 32, 256, 152LL * 64), 256, 0, st>>>(img, E, G, 0);
         prof_end(ps__, (double)shape[0] * shape[1] * shape[2] * 2, st);
     }
     PMG_CHECK_LAUNCH();
@@ -336,39 +315,17 @@ int erosion_edt_run(const uint8_t *img, float *D, const int64_t *shape, const in
 // The pipeline needs a binary image; *nonbinary reports an image with values
 // above 1 (KC is then not written and the caller takes the float path).
 int erosion_cap_run(const uint8_t *img, uint16_t *KC, const int64_t *shape, const int32_t *bc,
-                    const int32_t *pad, int Tcap, uint8_t *E, uint16_t *KA, uint16_t *KB, int *flag,
-                    int *nonbinary, cudaStream_t st)
+                    const int32_t *pad, int Tcap, uint16_t *KA, uint16_t *KB, int *flag, int *nonbinary,
+                    cudaStream_t st)
 {
-    ExtGeo G;
-    for (int d = 0; d < 3; d++) {
-        ExtAxis &a = G.ax[d];
+    for (int d = 0; d < 3; d++)
         if (bc[2 * d] == PMG_BC_PERIODIC) {
             set_error("erosion EDT reuse needs a subdomain without periodic axes");
             return PMG_EINVAL;
         }
-        a.periodic = 0;
-        a.own_lo = pad[2 * d];
-        a.own_len = (int)(shape[d] - pad[2 * d] - pad[2 * d + 1]);
-        a.ext_lo = 0;
-        a.wall_lo = bc[2 * d] == PMG_BC_WALL;
-        a.wall_hi = bc[2 * d + 1] == PMG_BC_WALL;
-        a.S = shape[d];
-        a.X = shape[d];
-    }
-    PMG_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
-    {
-        const int ps__ = prof_begin("k_extend", st);
-        k_extend<<<grid_for(shape[0] * shape[1] * 32, 256, 152LL * 64), 256, 0, st>>>(img, E, G, 0, flag);
-        prof_end(ps__, (double)shape[0] * shape[1] * shape[2] * 2, st);
-    }
-    PMG_CHECK_LAUNCH();
-    int h = 0;
-    PMG_CUDA(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
-    PMG_CUDA(cudaStreamSynchronize(st));
-    *nonbinary = h;
-    if (h)
-        return PMG_OK;
-    return edt_cap_run(E, KA, KB, KC, shape, Tcap, st);
+    const int32_t no_ext[6] = {0, 0, 0, 0, 0, 0};
+    const ExtGeo G = ext_geo(shape, bc, pad, no_ext);
+    return edt_cap_run(img, G, KA, KB, KC, shape, Tcap, flag, nonbinary, st);
 }
 
 size_t morph_scratch_bytes(const int64_t *shape, const int32_t *bc, const int32_t *ext)

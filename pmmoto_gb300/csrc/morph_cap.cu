@@ -65,16 +65,16 @@ struct SeedRange {
 };
 
 // ---- pass A: rows -------------------------------------------------------------
-// raw == 0: E is the (extended) image whose zeros are the seeds.  raw == 1:
-// E is the unextended image of a dilation without periodic axes, read
-// directly -- the seeds are its nonzero voxels off the wall planes (the
-// logical_not of k_extend's image), so no extended copy is written.
-// With rows (raw only), the seeds come from row words (b1, nt2: block rows and
+// The seeds of a dilation are the nonzero voxels of the extended image off the
+// wall planes, those of an erosion its zeros and the wall planes.  Rows come
+// from the image, periodic axes reading the own region modulo its length, or
+// (dilations without periodic axes) from row words (b1, nt2: block rows and
 // pieces of a row).
 struct RowSrc {
-    int raw;
-    int X1;
-    int wall[6];
+    const uint8_t *img;
+    ExtGeo G;
+    int dilate;
+    int *nonbinary; // set when a voxel above 1 is met (null: not asked)
     const unsigned *rows;
     int b1, nt2;
 };
@@ -88,58 +88,83 @@ __device__ __forceinline__ unsigned spread16(unsigned v)
     return (v | (v << 1)) & 0x55555555u;
 }
 
+// Bytes k .. k + 3 of a row of n (k < n; zero past its end) at img + off, img
+// holding total bytes: two aligned words where those lie inside the image.
+__device__ __forceinline__ unsigned row_bytes(const uint8_t *img, long long off, int k, int n, long long total)
+{
+    const unsigned left = n - k >= 4 ? 0xffffffffu : (1u << (8 * (n - k))) - 1u;
+    const uint8_t *p = img + off + k;
+    const int mis = (int)((uintptr_t)p & 3u);
+    if (off + k >= mis && off + k - mis + 8 <= total) {
+        const unsigned *q = reinterpret_cast<const unsigned *>(p - mis);
+        return (mis ? __funnelshift_r(q[0], q[1], 8 * mis) : q[0]) & left;
+    }
+    unsigned v = 0;
+    for (int e = 0; e < 4 && k + e < n; e++)
+        v |= (unsigned)p[e] << (8 * e);
+    return v;
+}
+
+// Bits p .. p + 31 of a bit array.
+__device__ __forceinline__ unsigned bits_at(const uint32_t *w, int p)
+{
+    return __funnelshift_r(w[p >> 5], w[(p >> 5) + 1], p & 31);
+}
+
 // Only distances d <= W = floor(sqrt T) <= 31 give values below T + 1, so a
-// voxel needs the seeds within 31 positions on either side: the row's seeds
-// are first gathered as bit words (a ballot per 32 voxels, or row words with
-// even and odd positions interleaved, kept in shared memory with an empty word
-// on either side), then every lane finds the nearest seeds of two adjacent
-// voxels in the three words around them with one count of leading / trailing
-// zeros each way and stores both at once (rows of even pitch; the column that
-// an odd row gains holds some height, read by no one).
-// Bound by the 2 bytes written per voxel and the bit counts; from per-block
+// voxel needs the seeds within 31 positions on either side: the row's seeds are
+// first gathered as bit words in shared memory (from the image's bytes, four
+// per lane, wrapped on a periodic axis; or from row words with even and odd
+// positions interleaved), with an empty word on either side, then every lane
+// finds the nearest seeds of two adjacent voxels in the three words around them
+// with one count of leading / trailing zeros each way and stores both at once
+// (rows of even pitch; the column that an odd row gains holds some height, read
+// by no one).
+// Bound by the 2 bytes written per voxel and the bit counts.  From per-block
 // mask bytes with a ballot per 32 voxels and one voxel a lane the drainage's
-// dilations took 0.16 ms at 512^3, now 0.11 ms.
-__global__ void __launch_bounds__(256) k_cap_rows(const uint8_t *__restrict__ E, uint16_t *__restrict__ KA,
-                                                  long long rows, int X2, int T, int W, RowSrc rs,
-                                                  const unsigned long long *__restrict__ gate,
+// dilations took 0.16 ms at 512^3, now 0.11 ms; with a pass of its own for the
+// extended copy (60 us) 256 x 192 x 320 voxels took 98 us.
+template <bool WORDS>
+__global__ void __launch_bounds__(256) k_cap_rows(RowSrc rs, uint16_t *__restrict__ KA, long long rows, int X2, int T,
+                                                  int W, const unsigned long long *__restrict__ gate,
                                                   const int *__restrict__ xr, unsigned long long *units)
 {
     if (gate && *gate == 0)
         return; // empty seed set: the last pass writes the result alone
+    const ExtAxis &a2 = rs.G.ax[2];
+    const int X1 = (int)rs.G.ax[1].X, S2 = (int)a2.S;
     SeedRange sr{0, 0x7fffffff, 0, 0};
     if (xr)
-        sr.load(xr, (int)(rows / rs.X1), W);
-    extern __shared__ uint32_t s_zw[];
-    const unsigned FULL = 0xffffffffu;
+        sr.load(xr, (int)(rows / X1), W);
+    extern __shared__ uint32_t s_words[];
     const int lane = threadIdx.x & 31;
-    const int nw = (X2 + 31) >> 5;
-    uint32_t *zw = s_zw + (threadIdx.x >> 5) * (nw + 3) + 1; // zw[-1], zw[nw] and zw[nw + 1] stay 0
+    const int nw = (X2 + 31) >> 5, nown = WORDS ? 0 : ((S2 + 127) >> 7) * 4 + 1;
+    uint32_t *zw = s_words + (threadIdx.x >> 5) * (nw + 3 + nown) + 1; // zw[-1], zw[nw] and zw[nw + 1] stay 0
+    [[maybe_unused]] uint32_t *own = zw + nw + 2;                      // the unextended row, a zero word at its end
     if (lane == 0) {
         zw[-1] = 0u;
         zw[nw] = 0u;
         zw[nw + 1] = 0u;
+        if constexpr (!WORDS)
+            own[nown - 1] = 0u;
     }
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    const int big = T + 1;
-    const int P2 = (X2 + 1) & ~1;
+    const int big = T + 1, P2 = (X2 + 1) & ~1;
     // with a seed range, only the rows of its planes
-    const int r0 = xr ? max(sr.hlo, 0) * rs.X1 : 0;
-    const int r1 = xr ? (int)min(rows, (long long)(sr.hhi + 1) * rs.X1) : (int)rows;
+    const int r0 = xr ? max(sr.hlo, 0) * X1 : 0;
+    const int r1 = xr ? (int)min(rows, (long long)(sr.hhi + 1) * X1) : (int)rows;
     if (units && blockIdx.x == 0 && threadIdx.x == 0 && r1 > r0)
         atomicAdd(units, (unsigned long long)((long long)(r1 - r0) * X2));
     for (int r = r0 + warp; r < r1; r += nwarps) {
-        const uint8_t *src = E + (long long)r * X2;
+        const int i = r / X1, j = r - i * X1;
         bool wrow = false;
-        const int i = rs.raw ? r / rs.X1 : 0, j = r - i * rs.X1;
-        if (rs.raw)
-            wrow = (rs.wall[0] && i == 0) || (rs.wall[1] && i == rows / rs.X1 - 1) || (rs.wall[2] && j == 0) ||
-                   (rs.wall[3] && j == rs.X1 - 1);
+        const long long s0 = src_index(rs.G.ax[0], i, wrow), s1 = src_index(rs.G.ax[1], j, wrow);
         if (wrow) {
-            // a wall row holds no seeds
+            // a wall row: no voxel
             for (int c = lane; c < nw; c += 32)
                 zw[c] = 0u;
-        } else if (rs.rows) {
+        } else if constexpr (WORDS) {
             // 64 voxels per piece: even positions in one word, odd ones in the next
             const unsigned *p = rs.rows + ((long long)((i >> 1) * rs.b1 + (j >> 1)) * rs.nt2) * 8 +
                                 ((i & 1) * 2 + (j & 1)) * 2;
@@ -149,25 +174,59 @@ __global__ void __launch_bounds__(256) k_cap_rows(const uint8_t *__restrict__ E,
                 zw[c] = spread16((eo.x >> sh) & 0xffffu) | (spread16((eo.y >> sh) & 0xffffu) << 1);
             }
         } else {
-            const uint8_t want = rs.raw ? 0 : 1; // a seed is a voxel != want (raw) or == 0
-#pragma unroll 4
-            for (int c = 0; c < nw; c++) {
-                const int x = (c << 5) + lane;
-                const bool seed = x < X2 && ((src[x] == 0) != (want == 0));
-                const unsigned zm = __ballot_sync(FULL, seed);
-                if (lane == 0)
-                    zw[c] = zm;
+            const long long off = (s0 * rs.G.ax[1].S + s1) * S2, total = rs.G.ax[0].S * rs.G.ax[1].S * S2;
+            unsigned above = 0;
+            for (int b = 0; b < S2; b += 128) {
+                const int k = b + 4 * lane;
+                const unsigned v = k < S2 ? row_bytes(rs.img, off, k, S2, total) : 0u;
+                above |= v & 0xfefefefeu;
+                // bit e: byte e is not zero
+                const unsigned m = (((v & 0x7f7f7f7fu) + 0x7f7f7f7fu) | v) >> 7 & 0x01010101u;
+                unsigned w = ((m * 0x204081u) >> 21 & 0xfu) << (4 * (lane & 7));
+                w |= __shfl_xor_sync(0xffffffffu, w, 1);
+                w |= __shfl_xor_sync(0xffffffffu, w, 2);
+                w |= __shfl_xor_sync(0xffffffffu, w, 4);
+                if ((lane & 7) == 0)
+                    own[(b >> 5) + (lane >> 3)] = w;
+            }
+            if (above && rs.nonbinary)
+                *rs.nonbinary = 1;
+            __syncwarp();
+            for (int c = lane; c < nw; c += 32) {
+                unsigned w = 0;
+                if (!a2.periodic) {
+                    w = own[c];
+                } else {
+                    int q = (32 * c - (a2.own_lo + a2.ext_lo)) % a2.own_len;
+                    q += q < 0 ? a2.own_len : 0;
+                    for (int f = 0; f < 32;) {
+                        const int take = min(32 - f, a2.own_len - q);
+                        const unsigned v = bits_at(own, a2.own_lo + q) & (0xffffffffu >> (32 - take));
+                        w |= v << f;
+                        f += take;
+                        q = 0;
+                    }
+                }
+                zw[c] = w;
             }
         }
         __syncwarp();
-        if (!wrow && rs.raw && lane == 0) {
-            // wall planes at the row ends hold no seeds
-            if (rs.wall[4])
+        if (!wrow && lane == 0 && !a2.periodic) {
+            // the wall planes at the row's ends
+            if (a2.wall_lo)
                 zw[0] &= ~1u;
-            if (rs.wall[5])
+            if (a2.wall_hi)
                 zw[(X2 - 1) >> 5] &= ~(1u << ((X2 - 1) & 31));
         }
         __syncwarp();
+        if (!WORDS) {
+            // seeds: the row's voxels, or (erosion) the others
+            for (int c = lane; c < nw; c += 32) {
+                const unsigned in = X2 - 32 * c >= 32 ? 0xffffffffu : (1u << (X2 - 32 * c)) - 1u;
+                zw[c] = (rs.dilate ? zw[c] : ~zw[c]) & in;
+            }
+            __syncwarp();
+        }
         uint16_t *dst = KA + (long long)r * P2;
         // lane l on voxels 64 c + 2 l and the next one: word 2 c + l / 16
         const int hw = lane >> 4, sh = (2 * lane) & 31;
@@ -184,6 +243,33 @@ __global__ void __launch_bounds__(256) k_cap_rows(const uint8_t *__restrict__ E,
         }
         __syncwarp();
     }
+}
+
+// The row pass; *nonbinary (erosions) is read back from flag.
+static int launch_cap_rows(const uint8_t *img, const ExtGeo &EG, int dilate, const unsigned *seeds, uint16_t *KA,
+                           const CapGeo &G, int T, int W, int *flag, int *nonbinary, cudaStream_t st,
+                           const unsigned long long *gate, const int *xr)
+{
+    RowSrc rs{img, EG, dilate, flag, seeds, (int)((G.X1 + 1) / 2), (int)(((G.X2 + 1) / 2 + 31) / 32)};
+    const int block = 256, words = (G.X2 + 31) / 32 + 3 + (seeds ? 0 : ((int)EG.ax[2].S + 127) / 128 * 4 + 1);
+    const size_t smem = (size_t)(block / 32) * words * sizeof(uint32_t);
+    const long long rows = (long long)G.X0 * G.X1;
+    const unsigned grid = grid_for(rows * 32, block, 152LL * 16);
+    if (flag)
+        PMG_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
+    const int ps__ = prof_begin("k_cap_rows", st);
+    if (seeds)
+        k_cap_rows<true><<<grid, block, smem, st>>>(rs, KA, rows, G.X2, T, W, gate, xr, prof_units(kUnitsCapRows));
+    else
+        k_cap_rows<false><<<grid, block, smem, st>>>(rs, KA, rows, G.X2, T, W, gate, xr, prof_units(kUnitsCapRows));
+    // 1 B read (1/8 B from row words) + 2 B written per voxel
+    prof_end_units(ps__, kUnitsCapRows, seeds ? 2.125 : 3.0, st);
+    PMG_CHECK_LAUNCH();
+    if (flag) {
+        PMG_CUDA(cudaMemcpyAsync(nonbinary, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+        PMG_CUDA(cudaStreamSynchronize(st));
+    }
+    return PMG_OK;
 }
 
 // ---- pass B: capped envelope along axis 1 --------------------------------------
@@ -778,18 +864,10 @@ bool cap_rows_out(const int64_t *X, int T, const MorphEpi &me)
     return plain && me.dilate && W <= kPairMaxW;
 }
 
-int morph_cap_run(const uint8_t *E, uint16_t *KA, uint16_t *KB, const int64_t *X, int T, const MorphEpi &me,
-                  cudaStream_t st, int raw_dilate, const unsigned long long *gate, const int *xr, int *orange,
-                  const unsigned *seeds, unsigned *rows_out)
+int morph_cap_run(const uint8_t *img, const ExtGeo &EG, uint16_t *KA, uint16_t *KB, const int64_t *X, int T,
+                  const MorphEpi &me, cudaStream_t st, int *flag, int *nonbinary, const unsigned long long *gate,
+                  const int *xr, int *orange, const unsigned *seeds, unsigned *rows_out)
 {
-    RowSrc rs{};
-    rs.raw = raw_dilate;
-    rs.X1 = (int)X[1];
-    rs.rows = raw_dilate ? seeds : nullptr;
-    rs.b1 = (int)((X[1] + 1) / 2);
-    rs.nt2 = (int)(((X[2] + 1) / 2 + 31) / 32);
-    for (int q = 0; q < 6; q++)
-        rs.wall[q] = me.wall[q];
     int W = 0;
     while ((W + 1) * (W + 1) <= T)
         W++;
@@ -802,17 +880,9 @@ int morph_cap_run(const uint8_t *E, uint16_t *KA, uint16_t *KB, const int64_t *X
     G.k0 = me.e2;
     G.nk = (int)me.o2;
     G.P2 = G.PO = (G.X2 + 1) & ~1;
-    const long long rows = (long long)G.X0 * G.X1;
-    {
-        const int block = 256;
-        const size_t smem = (size_t)(block / 32) * ((G.X2 + 31) / 32 + 3) * sizeof(uint32_t);
-        const int ps__ = prof_begin("k_cap_rows", st);
-        k_cap_rows<<<grid_for(rows * 32, block, 152LL * 16), block, smem, st>>>(
-            E, KA, rows, G.X2, T, W, rs, gate, xr, prof_units(kUnitsCapRows));
-        // 1 B read (1/8 B from row words) + 2 B written per voxel
-        prof_end_units(ps__, kUnitsCapRows, rs.rows ? 2.125 : 3.0, st);
-    }
-    PMG_CHECK_LAUNCH();
+    PMG_TRY(launch_cap_rows(img, EG, me.dilate, seeds, KA, G, T, W, flag, nonbinary, st, gate, xr));
+    if (flag && *nonbinary)
+        return PMG_OK;
     {
         const long long lines = (long long)G.X0 * G.nk;
         const int ps__ = prof_begin("k_cap_mid", st);
@@ -837,10 +907,11 @@ int morph_cap_run(const uint8_t *E, uint16_t *KA, uint16_t *KB, const int64_t *X
     return PMG_OK;
 }
 
-// Capped squared EDT of a binary image without extension: E = min(exact d^2
+// Capped squared EDT of a binary image (nothing is written when it is not):
+// E = min(exact d^2
 // in units of res^2, T + 1) as uint16, all three passes on the same volume.
-int edt_cap_run(const uint8_t *E, uint16_t *KA, uint16_t *KB, uint16_t *KC, const int64_t *X, int T,
-                cudaStream_t st)
+int edt_cap_run(const uint8_t *img, const ExtGeo &EG, uint16_t *KA, uint16_t *KB, uint16_t *KC, const int64_t *X, int T,
+                int *flag, int *nonbinary, cudaStream_t st)
 {
     int W = 0;
     while ((W + 1) * (W + 1) <= T)
@@ -854,18 +925,10 @@ int edt_cap_run(const uint8_t *E, uint16_t *KA, uint16_t *KB, uint16_t *KC, cons
     G.k0 = 0;
     G.nk = G.X2;
     G.P2 = G.PO = (G.X2 + 1) & ~1;
-    const long long rows = (long long)G.X0 * G.X1;
-    const long long vox = rows * G.X2;
-    {
-        const int block = 256;
-        const size_t smem = (size_t)(block / 32) * ((G.X2 + 31) / 32 + 3) * sizeof(uint32_t);
-        const int ps__ = prof_begin("k_cap_rows", st);
-        k_cap_rows<<<grid_for(rows * 32, block, 152LL * 16), block, smem, st>>>(E, KA, rows, G.X2, T, W,
-                                                                                RowSrc{}, nullptr, nullptr,
-                                                                                prof_units(kUnitsCapRows));
-        prof_end_units(ps__, kUnitsCapRows, 3.0, st);
-    }
-    PMG_CHECK_LAUNCH();
+    const long long vox = (long long)G.X0 * G.X1 * G.X2;
+    PMG_TRY(launch_cap_rows(img, EG, 0, nullptr, KA, G, T, W, flag, nonbinary, st, nullptr, nullptr));
+    if (*nonbinary)
+        return PMG_OK;
     {
         const long long lines = (long long)G.X0 * G.nk;
         const int ps__ = prof_begin("k_cap_mid", st);

@@ -25,8 +25,8 @@ int erosion_edt_ext_run(const uint8_t *img, float *D, const int64_t *shape, cons
                         const int32_t *ext, const float *res, int unit_res, uint8_t *E, float *A, int64_t *X,
                         int64_t *lo, cudaStream_t st);
 int erosion_cap_run(const uint8_t *img, uint16_t *KC, const int64_t *shape, const int32_t *bc,
-                    const int32_t *pad, int Tcap, uint8_t *E, uint16_t *KA, uint16_t *KB, int *flag,
-                    int *nonbinary, cudaStream_t st);
+                    const int32_t *pad, int Tcap, uint16_t *KA, uint16_t *KB, int *flag, int *nonbinary,
+                    cudaStream_t st);
 
 int select_run(const uint8_t *img, void *out, int out_bytes, const int64_t *shape,
                const int32_t *bc, const int32_t *pad, const int64_t *inlet_box,
