@@ -432,48 +432,40 @@ __device__ int boundary_hull(Stack &S, const L &line, int start, int nv, float a
 
 // The imported boundary hulls of a periodic line (return_boundary_hull on the
 // segment before the first zero and after the last zero, the far end's hull
-// becoming the lower imports): lower imports into S, upper ones into up_*.
+// becoming the lower imports).  A zero height is exactly a zero voxel of the
+// original image: pass 0 gives 0 only there and every later pass keeps it, all
+// other values being >= res^2 > 0.
+
+// near end (forward) -> upper imports
 template <class L>
-__device__ __forceinline__ void load_imports(Stack &S, const L &line, int n, float aniso, const pmg_axis_cfg &cfg,
-                                             int num_hull, int *up_v, float *up_h, float *up_r, int &n_up)
+__device__ __forceinline__ void load_upper(Stack &S, const L &line, int n, float aniso, const pmg_axis_cfg &cfg,
+                                           int num_hull, int *up_v, float *up_h, float *up_r, int &n_up)
 {
-    // first / last zero (a zero height is exactly a zero voxel of the
-    // original image: pass 0 gives 0 only there and every later pass keeps
-    // it, all other values being >= res^2 > 0)
-    int bf = -1, bb = -1;
+    int bf = -1;
     for (int i = cfg.hf_lo; i < n; i++)
         if (line(i) == 0.0f) {
             bf = i;
             break;
         }
+    const int nv = bf == -1 ? n - cfg.hf_lo : bf - cfg.hf_lo + 1;
+    n_up = boundary_hull(S, line, cfg.hf_lo, nv, aniso, num_hull, 0, true, up_v, up_h, up_r);
+}
+
+// far end (backward) -> lower imports into S, given in top-down order
+template <class L>
+__device__ __forceinline__ void load_lower(Stack &S, const L &line, int n, float aniso, const pmg_axis_cfg &cfg,
+                                           int num_hull)
+{
+    int bb = -1;
     for (int i = n - cfg.hb_hi - 1; i >= 0; i--)
         if (line(i) == 0.0f) {
             bb = i;
             break;
         }
-    // near end (forward) -> upper imports
-    int start, nv, corr;
-    if (bf == -1) {
-        start = cfg.hf_lo;
-        nv = n - cfg.hf_lo;
-    } else {
-        start = cfg.hf_lo;
-        nv = bf - cfg.hf_lo + 1;
-    }
-    corr = 0;
-    n_up = boundary_hull(S, line, start, nv, aniso, num_hull, corr, true, up_v, up_h, up_r);
-    // far end (backward) -> lower imports, given in top-down order
     int lo_v[kMaxHull];
     float lo_h[kMaxHull], lo_r[kMaxHull];
-    if (bb == -1) {
-        start = 0;
-        nv = n - cfg.hb_hi;
-    } else {
-        start = bb;
-        nv = n - bb - cfg.hb_hi;
-    }
-    corr = -nv;
-    const int n_lo = boundary_hull(S, line, start, nv, aniso, num_hull, corr, false, lo_v, lo_h, lo_r);
+    const int start = bb == -1 ? 0 : bb, nv = n - start - cfg.hb_hi;
+    const int n_lo = boundary_hull(S, line, start, nv, aniso, num_hull, -nv, false, lo_v, lo_h, lo_r);
     // the reference pushes the lower list in reverse (rbegin..rend)
     for (int j = 0; j < n_lo; j++) {
         S.lv[j] = lo_v[n_lo - 1 - j];
@@ -481,6 +473,14 @@ __device__ __forceinline__ void load_imports(Stack &S, const L &line, int n, flo
         S.lr[j] = lo_r[n_lo - 1 - j];
     }
     S.nl = n_lo;
+}
+
+template <class L>
+__device__ __forceinline__ void load_imports(Stack &S, const L &line, int n, float aniso, const pmg_axis_cfg &cfg,
+                                             int num_hull, int *up_v, float *up_h, float *up_r, int &n_up)
+{
+    load_upper(S, line, n, aniso, cfg, num_hull, up_v, up_h, up_r, n_up);
+    load_lower(S, line, n, aniso, cfg, num_hull);
 }
 
 // Evaluation sweep over the final stack (bottom to top), written for
@@ -580,11 +580,13 @@ __global__ void k_envelope(const float *__restrict__ fin, float *__restrict__ fo
 // the voxels up to the first zero, and the voxels from the last zero with the
 // upper imports.  No parabola can pop a zero off the stack, so these partial
 // stacks and sweeps make the same float decisions as the whole line's.
-// bm: this thread's envelope bits, nthr threads apart.
+// part: 3 for both ends, 1 for the low end or the whole line, 2 for the high end
+// (nothing where the whole line is replayed), so that two threads can share a
+// line.  bm: this thread's envelope bits, nthr threads apart.
 template <class L>
 __device__ __noinline__ void replay_line(uint32_t *bm, int nthr, const L &line, const LineGeo &g, float aniso,
                                          const pmg_axis_cfg &cfg, int num_hull, bool whole, int form,
-                                         const MorphEpi &me, float *fout)
+                                         const MorphEpi &me, float *fout, int part = 3)
 {
     Stack S;
     S.bm = bm;
@@ -608,12 +610,16 @@ __device__ __noinline__ void replay_line(uint32_t *bm, int nthr, const L &line, 
     int up_v[kMaxHull];
     float up_h[kMaxHull], up_r[kMaxHull];
     int n_up = 0;
-    if (cfg.periodic)
-        load_imports(S, line, n, aniso, cfg, num_hull, up_v, up_h, up_r, n_up);
     whole = whole || z1 < 0;
+    if (whole && part == 2)
+        return;
+    if (cfg.periodic && (whole || (part & 2)))
+        load_upper(S, line, n, aniso, cfg, num_hull, up_v, up_h, up_r, n_up);
+    if (cfg.periodic && (whole || (part & 1)))
+        load_lower(S, line, n, aniso, cfg, num_hull);
     const int lo_end = whole ? n - 1 : z1; // last native of the lower stack
     // lower part: the imports below, natives up to lo_end
-    if (whole || z1 > 0) {
+    if (whole || ((part & 1) && z1 > 0)) {
         int loop_start;
         if (S.nl > 0) {
             loop_start = 0;
@@ -644,7 +650,7 @@ __device__ __noinline__ void replay_line(uint32_t *bm, int nthr, const L &line, 
     }
     // upper part: the zero at z2 at the bottom, natives above it, the upper
     // imports on top
-    if (z2 < n - 1) {
+    if ((part & 2) && z2 < n - 1) {
         S.nl = 0;
         S.nu = 0;
         S.setbit(z2);
@@ -693,10 +699,14 @@ __device__ __forceinline__ void stage_ends(float *se, const T *__restrict__ fin,
     }
 }
 
-// Flagged lines of any voxel size (flag bit 1: the whole line): one lane per
-// line, 32 adjacent lines per warp (unflagged ones idle); both ends of the
-// lines are staged in shared memory first, because the zero searches, hulls,
-// pushes and the sweep read them again and again in dependent steps.
+// Flagged lines of any voxel size (flag bit 1: the whole line): a block takes 32
+// adjacent lines (unflagged ones idle), the lanes of warp 0 their low ends or
+// the whole line and those of warp 1 their high ends, two chains that overlap.
+// Both ends of the lines are staged in shared memory first, because the zero
+// searches, hulls, pushes and the sweep read them again and again in dependent
+// steps.
+// Bound by the latency of those steps: with one lane for both ends a periodic
+// 341 x 298 x 125 field took 0.80 ms here.
 constexpr int kEndBlock = 64;
 
 __global__ void __launch_bounds__(kEndBlock) k_envelope_ends(const float *__restrict__ fin, float *__restrict__ fout,
@@ -704,29 +714,27 @@ __global__ void __launch_bounds__(kEndBlock) k_envelope_ends(const float *__rest
                                                              int form, MorphEpi me, const uint8_t *__restrict__ flag)
 {
     extern __shared__ uint32_t smem_bm[];
-    __shared__ float s_ends[kEndBlock / 32][2 * kEndWin * 33];
+    __shared__ float s_ends[2 * kEndWin * 33];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    float *se = s_ends[w];
     // tiles of 32 lines that are adjacent in memory (along the second axis)
     const int tiles = (Ls.nb2 + 31) / 32;
     const long long ntiles = (long long)Ls.nb1 * tiles;
-    for (long long t = blockIdx.x * (long long)(kEndBlock / 32) + w; t < ntiles;
-         t += (long long)gridDim.x * (kEndBlock / 32)) {
+    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int ra = (int)(t / tiles), kb = (int)(t - (long long)ra * tiles) * 32;
         const int lines = min(32, Ls.nb2 - kb);
         const long long l0 = (long long)ra * Ls.nb2 + kb;
         const int fl = lane < lines ? flag[l0 + lane] : 0;
-        if (!__any_sync(0xffffffffu, fl))
+        if (!__any_sync(0xffffffffu, fl)) // the same for both warps
             continue;
         const LineGeo g = line_addr(Ls, l0 + min(lane, lines - 1));
-        __syncwarp();
-        stage_ends(se, fin, Ls, l0, lines, g, res, 0, 1);
-        __syncwarp();
+        __syncthreads(); // (the previous tile's readers)
+        stage_ends(s_ends, fin, Ls, l0, lines, g, res, w, 2);
+        __syncthreads();
         if (!fl)
             continue;
-        const LineEnds<float> line{fin + g.base, g.stride, se + lane, 33, g.n, 0, res};
+        const LineEnds<float> line{fin + g.base, g.stride, s_ends + lane, 33, g.n, 0, res};
         replay_line(smem_bm + threadIdx.x, kEndBlock, line, g, fmul(res, res), cfg, num_hull, (fl & 2) != 0, form, me,
-                    fout);
+                    fout, 1 << w);
     }
 }
 
@@ -919,7 +927,7 @@ int launch_ends_float(const float *fin, float *fout, const Lines &Ls, float res,
     const size_t smem = (size_t)((n + 31) / 32) * kEndBlock * 4;
     const long long tiles = (long long)Ls.nb1 * ((Ls.nb2 + 31) / 32);
     const int ps__ = prof_begin("k_envelope_ends", st);
-    k_envelope_ends<<<grid_for(tiles, kEndBlock / 32, 152LL * 64), kEndBlock, smem, st>>>(
+    k_envelope_ends<<<grid_for(tiles, 1, 152LL * 64), kEndBlock, smem, st>>>(
         fin, fout, Ls, res, cfg, num_hull, form, me, flag);
     prof_end(ps__, 0.0, st);
     PMG_CHECK_LAUNCH();
