@@ -11,17 +11,26 @@
 //   dgrad     D[pos_in, c_in]   = sum_{tap, c_out} dZ[pos_out(pos_in, tap), c_out] W[c_out, tap, c_in]
 //   wgrad     D[(tap, c_in), c_out] = sum_{pos_out} X[pos_in(pos_out, tap), c_in] dZ[pos_out, c_out]
 //
-// One CTA of 128 threads computes a 128 x N tile (N = 16, 32 or 64 output
+// One CTA of 128 threads computes 128 x N tiles (N = 16, 32 or 64 output
 // columns) with the fp32 accumulator in tensor memory.  The K loop runs in
-// chunks of 64 bf16 (one 128-byte row per tile row): all threads gather the
-// chunk's operands from global memory (the im2col gather, zero outside the
-// volume) into shared memory in the 128-byte-swizzled K-major layout, one
-// elected thread issues four tcgen05.mma (K = 16 each) and commits them to
-// the stage's mbarrier, and the next chunk is gathered into another of
-// three stages meanwhile.  The epilogue reads the accumulator with
-// tcgen05.ld (thread t owns row t) and applies bias + ReLU (forward), the
-// ReLU mask of the layer below (dgrad) or an fp32 atomic add into the
-// weight gradient (wgrad, split over K across CTAs).
+// chunks of 64 bf16: all threads gather the chunk's operands with 16-byte
+// cp.async (the im2col gather, zero-filled outside the volume) into one of
+// three shared-memory stages, two chunks ahead of the one elected thread that
+// issues four tcgen05.mma (K = 16 each) and commits them to the stage's
+// mbarrier.  The epilogue reads the accumulator with tcgen05.ld (thread t owns
+// row t) and applies bias + ReLU (forward), the ReLU mask of the layer below
+// (dgrad) or an fp32 atomic add into the weight gradient (wgrad, split over K
+// across CTAs).  CTAs are persistent, so tensor memory is allocated once.
+//
+// * dgrad: an input position takes a tap only where its parity matches, so the
+//   input positions of one parity class share their 1, 2, 4 or 8 taps: one GEMM
+//   per class (27 / 8 taps a position instead of 27, 7/8 of them zeros).
+// * wgrad: both operands run along K in memory (positions), so they are
+//   MN-major tiles, copied as they lie.  Transposed into K-major tiles two
+//   bytes at a time, a chunk took ten times its loads in stores.
+// * The first layer (one input channel: K = 27) gathers from a patch of the input
+//   in shared memory; its weight gradient, 27 x N with the positions along K, is
+//   fp32 FMAs (a lane per tap) on such a patch.
 //
 // Every mbarrier wait has a time limit (about 1 s of %globaltimer); a wait
 // that runs out records an error code, the CTA waits (again bounded) for its
@@ -134,6 +143,22 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar)
                  : "memory");
 }
 
+// 16 bytes global -> shared, zeros where !valid (src is then not read).
+__device__ __forceinline__ void cp16(uint8_t *dst, const void *src, bool valid)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)),
+                 "l"(__cvta_generic_to_global(src)), "r"(valid ? 16 : 0)
+                 : "memory");
+}
+
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+template <int N>
+__device__ __forceinline__ void cp_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // 16 consecutive fp32 columns of this thread's TMEM lane.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v)
 {
@@ -170,16 +195,28 @@ __device__ __forceinline__ uint64_t sdesc_sw128(uint32_t addr)
     return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 
-// Instruction descriptor of kind::f16: fp32 accumulator, bf16 A and B, both
-// K-major, M = 128, N = n.
-__host__ __device__ constexpr uint32_t idesc_bf16(int n)
+// Byte offset of 16-byte chunk g (8 of the M or N index) of K index k in an
+// MN-major tile of 64 K with the 128-byte swizzle: per 64 of M (N) one column
+// of 8192 bytes, in it rows of 128 bytes (one k each), groups of 8 rows 1024
+// bytes apart.
+__device__ __forceinline__ uint32_t swmn(int k, int g)
 {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+    return (uint32_t)((g >> 3) * 8192 + (k >> 3) * 1024 + (k & 7) * 128 + (((g & 7) ^ (k & 7)) << 4));
 }
 
-__device__ __forceinline__ void st_shared16(uint8_t *base, uint32_t off, uint4 v)
+// Descriptor of such a tile: leading byte offset 8192 (next 64 of M or N),
+// stride byte offset 1024 (next 8 of K).
+__device__ __forceinline__ uint64_t sdesc_mn128(uint32_t addr)
 {
-    *reinterpret_cast<uint4 *>(base + off) = v;
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | (512ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+
+// Instruction descriptor of kind::f16: fp32 accumulator, bf16 A and B, both
+// K-major or (mn, the transpose bits) both MN-major, M = 128, N = n.
+__host__ __device__ constexpr uint32_t idesc_bf16(int n, bool mn)
+{
+    return (1u << 4) | (1u << 7) | (1u << 10) | (mn ? 3u << 15 : 0u) | ((uint32_t)(n >> 3) << 17) |
+           ((uint32_t)(kBM >> 4) << 24);
 }
 
 // ---- convolution geometry -----------------------------------------------------
@@ -191,269 +228,241 @@ struct Geo {
     __device__ __forceinline__ long long npos_out() const { return (long long)batch * dout * dout * dout; }
 };
 
-// Zero-filled 8 x bf16.
-__device__ __forceinline__ uint4 zero4() { return make_uint4(0u, 0u, 0u, 0u); }
-
 // ---- the three convolution operators as GEMM operand gatherers ---------------------
+// (input channels >= 16; lg*: log2 of the channel counts)
+
+// valid taps along an axis of d positions from i0 = first tap's position: bit k
+__device__ __forceinline__ unsigned taps_in(int i0, int d)
+{
+    unsigned v = 0;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        v |= (unsigned)(i0 + k >= 0 && i0 + k < d) << k;
+    return v;
+}
 
 // forward: rows = output positions, K = 27 * cin (tap-major), N = cout.
 // B operand: Wk [cout][kp] bf16, k = tap * cin + c, zero-padded to kp.
 struct OpFwd {
+    static constexpr bool kMN = false;
     Geo g;
     const __nv_bfloat16 *x;  // [npos_in][cin]
     const __nv_bfloat16 *wk; // [cout][kp]
     const float *bias;       // [cout]
     __nv_bfloat16 *y;        // [npos_out][cout]
-    int kp;
-    __device__ __forceinline__ long long rows() const { return g.npos_out(); }
-    __device__ __forceinline__ int kchunks() const { return kp / kBK; }
-
-    __device__ __forceinline__ void load_a(uint8_t *sa, long long m0, int kc, int tid) const
+    int kp, lgc;
+    FastDiv qo;
+    struct Row {
+        long long m, base; // base: first tap's input position
+        unsigned vz, vy, vx;
+    };
+    __device__ __forceinline__ void chunks(int, int, int, int &kc0, int &kc1) const
     {
-        const long long m = m0 + tid;
-        const bool live = m < rows();
-        int n = 0, z = 0, yy = 0, xx = 0;
-        if (live) {
-            long long q = m;
-            xx = (int)(q % g.dout);
-            q /= g.dout;
-            yy = (int)(q % g.dout);
-            q /= g.dout;
-            z = (int)(q % g.dout);
-            n = (int)(q / g.dout);
-        }
+        kc0 = 0;
+        kc1 = kp / kBK;
+    }
+    __device__ __forceinline__ Row row(int tile, int tid) const
+    {
+        Row r;
+        r.m = (long long)tile * kBM + tid;
+        const bool live = r.m < g.npos_out();
+        const unsigned m = live ? (unsigned)r.m : 0u, q1 = fdiv(m, qo), q2 = fdiv(q1, qo), n = fdiv(q2, qo);
+        const int xx = (int)(m - q1 * g.dout), yy = (int)(q1 - q2 * g.dout), z = (int)(q2 - n * g.dout), d = g.di;
+        r.base = (((long long)n * d + 2 * z - 1) * d + 2 * yy - 1) * d + 2 * xx - 1;
+        r.vz = live ? taps_in(2 * z - 1, d) : 0u;
+        r.vy = taps_in(2 * yy - 1, d);
+        r.vx = taps_in(2 * xx - 1, d);
+        return r;
+    }
+    __device__ __forceinline__ void load(uint8_t *sa, uint8_t *sb, const Row &r, int kc, int tid, int bn) const
+    {
         const int d = g.di;
 #pragma unroll
         for (int j = 0; j < 8; j++) {
-            const int k0 = kc * kBK + j * 8;
-            uint4 v = zero4();
-            if (live) {
-                if (g.cin >= 8) {
-                    const int t = k0 / g.cin, c0 = k0 - t * g.cin;
-                    if (t < 27) {
-                        const int iz = 2 * z + t / 9 - 1, iy = 2 * yy + (t / 3) % 3 - 1, ix = 2 * xx + t % 3 - 1;
-                        if (iz >= 0 && iz < d && iy >= 0 && iy < d && ix >= 0 && ix < d)
-                            v = *reinterpret_cast<const uint4 *>(
-                                x + ((((long long)n * d + iz) * d + iy) * d + ix) * g.cin + c0);
-                    }
-                } else { // cin == 1: eight taps
-                    __nv_bfloat16 e[8];
-#pragma unroll
-                    for (int u = 0; u < 8; u++) {
-                        const int t = k0 + u;
-                        e[u] = __float2bfloat16(0.0f);
-                        if (t < 27) {
-                            const int iz = 2 * z + t / 9 - 1, iy = 2 * yy + (t / 3) % 3 - 1, ix = 2 * xx + t % 3 - 1;
-                            if (iz >= 0 && iz < d && iy >= 0 && iy < d && ix >= 0 && ix < d)
-                                e[u] = x[(((long long)n * d + iz) * d + iy) * d + ix];
-                        }
-                    }
-                    v = *reinterpret_cast<const uint4 *>(e);
-                }
-            }
-            st_shared16(sa, sw128(tid, j), v);
+            const int k0 = kc * kBK + j * 8, t = k0 >> lgc, c0 = k0 & (g.cin - 1);
+            const int kz = t / 9, ky = t / 3 - 3 * kz, kx = t - 3 * (t / 3);
+            const bool in = t < 27 && ((r.vz >> kz) & (r.vy >> ky) & (r.vx >> kx) & 1u);
+            cp16(sa + sw128(tid, j), in ? x + (r.base + (kz * d + ky) * d + kx) * g.cin + c0 : x, in);
         }
-    }
-
-    __device__ __forceinline__ void load_b(uint8_t *sb, int kc, int tid, int bn) const
-    {
         for (int it = tid; it < bn * 8; it += kThreads) {
-            const int r = it >> 3, j = it & 7;
-            const uint4 v = *reinterpret_cast<const uint4 *>(wk + (long long)r * kp + kc * kBK + j * 8);
-            st_shared16(sb, sw128(r, j), v);
+            const int o = it >> 3, j = it & 7;
+            cp16(sb + sw128(o, j), wk + (long long)o * kp + kc * kBK + j * 8, true);
         }
     }
-
-    __device__ __forceinline__ void store(long long m, int c0, const float *v, int) const
+    __device__ __forceinline__ void store(const Row &r, int c0, const float *v) const
     {
-        if (m >= rows())
+        if (r.m >= g.npos_out())
             return;
         __align__(16) __nv_bfloat16 o[16];
 #pragma unroll
         for (int i = 0; i < 16; i++)
             o[i] = __float2bfloat16(fmaxf(v[i] + bias[c0 + i], 0.0f));
-        uint4 *dst = reinterpret_cast<uint4 *>(y + m * g.cout + c0);
+        uint4 *dst = reinterpret_cast<uint4 *>(y + r.m * g.cout + c0);
         dst[0] = reinterpret_cast<const uint4 *>(o)[0];
         dst[1] = reinterpret_cast<const uint4 *>(o)[1];
     }
 };
 
-// dgrad: rows = input positions, K = 27 * cout (tap-major), N = cin.
-// B operand: WkT [cin][kp] bf16, k = tap * cout + o.  The result is masked by
-// ReLU' of the layer below (its output xact > 0) -- the gradient of that
-// layer's pre-activation.
+// dgrad: rows = input positions of one parity class, K = its taps * cout, N =
+// cin.  Input iz takes tap kz from output oz when iz = 2 oz + kz - 1: an even
+// one tap 1 from iz / 2, an odd one tap 0 from (iz + 1) / 2 and tap 2 from
+// (iz - 1) / 2.  B operand: WkT [cin][kp] bf16, k = tap * cout + o.  The result
+// is masked by ReLU' of the layer below (its output xact > 0) -- the gradient of
+// that layer's pre-activation.
 struct OpDgrad {
+    static constexpr bool kMN = false;
     Geo g;
     const __nv_bfloat16 *dz;   // [npos_out][cout]
     const __nv_bfloat16 *wkt;  // [cin][kp]
     const __nv_bfloat16 *xact; // [npos_in][cin]
     __nv_bfloat16 *dx;         // [npos_in][cin]
-    int kp;
-    __device__ __forceinline__ long long rows() const { return g.npos_in(); }
-    __device__ __forceinline__ int kchunks() const { return kp / kBK; }
-
-    __device__ __forceinline__ void load_a(uint8_t *sa, long long m0, int kc, int tid) const
+    int kp, lgc;
+    int first[9];         // first tile of each class, the most taps first
+    FastDiv qh[2];        // division by the even and the odd positions of an axis
+    int nh[2];
+    struct Row {
+        long long pos;     // input position, -1: none
+        long long base;    // output position (n, a, b, c)
+        int cls;           // odd axes: bits 2 (z), 1 (y), 0 (x)
+        unsigned hz, hy, hx; // the next output of an odd axis exists
+    };
+    __device__ __forceinline__ int cls_of(int tile) const
     {
-        const long long m = m0 + tid;
-        const bool live = m < rows();
-        int n = 0, iz = 0, iy = 0, ix = 0;
-        if (live) {
-            long long q = m;
-            ix = (int)(q % g.di);
-            q /= g.di;
-            iy = (int)(q % g.di);
-            q /= g.di;
-            iz = (int)(q % g.di);
-            n = (int)(q / g.di);
-        }
-        const int d = g.dout;
+        int c = 0;
+#pragma unroll
+        for (int k = 1; k < 8; k++)
+            c += tile >= first[k];
+        return 7 - c;
+    }
+    __device__ __forceinline__ void chunks(int tile, int, int, int &kc0, int &kc1) const
+    {
+        kc0 = 0;
+        kc1 = ((g.cout << __popc(cls_of(tile))) + kBK - 1) / kBK;
+    }
+    __device__ __forceinline__ Row row(int tile, int tid) const
+    {
+        Row r;
+        r.cls = cls_of(tile);
+        const int pz = r.cls >> 2, py = (r.cls >> 1) & 1, px = r.cls & 1;
+        const unsigned nz = nh[pz], ny = nh[py], nx = nh[px];
+        const unsigned m = (unsigned)((tile - first[7 - r.cls]) * kBM + tid), rows = g.batch * nz * ny * nx;
+        const unsigned q1 = fdiv(m, qh[px]), q2 = fdiv(q1, qh[py]), n = fdiv(q2, qh[pz]);
+        const int c = (int)(m - q1 * nx), b = (int)(q1 - q2 * ny), a = (int)(q2 - n * nz);
+        r.pos = m < rows ? (((long long)n * g.di + 2 * a + pz) * g.di + 2 * b + py) * g.di + 2 * c + px : -1;
+        r.base = (((long long)n * g.dout + a) * g.dout + b) * g.dout + c;
+        r.hz = a + 1 < g.dout;
+        r.hy = b + 1 < g.dout;
+        r.hx = c + 1 < g.dout;
+        return r;
+    }
+    __device__ __forceinline__ void load(uint8_t *sa, uint8_t *sb, const Row &r, int kc, int tid, int bn) const
+    {
+        const int pz = r.cls >> 2, py = (r.cls >> 1) & 1, px = r.cls & 1, ntaps = 1 << __popc(r.cls), d = g.dout;
+        // local tap t: one bit per odd axis, 0: tap 0 (the next output), 1: tap 2
+        auto bits = [&](int t, int &bz, int &by, int &bx) {
+            bx = px ? t & 1 : 1;
+            t >>= px;
+            by = py ? t & 1 : 1;
+            t >>= py;
+            bz = pz ? t & 1 : 1;
+        };
 #pragma unroll
         for (int j = 0; j < 8; j++) {
-            const int k0 = kc * kBK + j * 8;
-            uint4 v = zero4();
-            const int t = k0 / g.cout, o0 = k0 - t * g.cout;
-            if (live && t < 27) {
-                // input iz takes tap kz from output oz when iz = 2 oz + kz - 1
-                const int sz = iz + 1 - t / 9, sy = iy + 1 - (t / 3) % 3, sx = ix + 1 - t % 3;
-                if (sz >= 0 && sy >= 0 && sx >= 0 && !(sz & 1) && !(sy & 1) && !(sx & 1)) {
-                    const int oz = sz >> 1, oy = sy >> 1, ox = sx >> 1;
-                    if (oz < d && oy < d && ox < d)
-                        v = *reinterpret_cast<const uint4 *>(
-                            dz + ((((long long)n * d + oz) * d + oy) * d + ox) * g.cout + o0);
-                }
-            }
-            st_shared16(sa, sw128(tid, j), v);
+            const int k0 = kc * kBK + j * 8, t = k0 >> lgc, o0 = k0 & (g.cout - 1);
+            int bz, by, bx;
+            bits(t, bz, by, bx);
+            const bool in = t < ntaps && r.pos >= 0 && (bz || r.hz) && (by || r.hy) && (bx || r.hx);
+            cp16(sa + sw128(tid, j), in ? dz + (r.base + ((1 - bz) * d + 1 - by) * d + 1 - bx) * g.cout + o0 : dz, in);
         }
-    }
-
-    __device__ __forceinline__ void load_b(uint8_t *sb, int kc, int tid, int bn) const
-    {
         for (int it = tid; it < bn * 8; it += kThreads) {
-            const int r = it >> 3, j = it & 7;
-            const uint4 v = *reinterpret_cast<const uint4 *>(wkt + (long long)r * kp + kc * kBK + j * 8);
-            st_shared16(sb, sw128(r, j), v);
+            const int c = it >> 3, j = it & 7, k0 = kc * kBK + j * 8, t = k0 >> lgc, o0 = k0 & (g.cout - 1);
+            int bz, by, bx;
+            bits(t, bz, by, bx);
+            const int tap = ((pz ? 2 * bz : 1) * 3 + (py ? 2 * by : 1)) * 3 + (px ? 2 * bx : 1);
+            cp16(sb + sw128(c, j), t < ntaps ? wkt + (long long)c * kp + tap * g.cout + o0 : wkt, t < ntaps);
         }
     }
-
-    __device__ __forceinline__ void store(long long m, int c0, const float *v, int) const
+    __device__ __forceinline__ void store(const Row &r, int c0, const float *v) const
     {
-        if (m >= rows())
+        if (r.pos < 0)
             return;
-        const __nv_bfloat16 *xa = xact + m * g.cin + c0;
-        __align__(16) __nv_bfloat16 o[16];
+        const uint4 *xa = reinterpret_cast<const uint4 *>(xact + r.pos * g.cin + c0);
+        __align__(16) __nv_bfloat16 x[16], o[16];
+        reinterpret_cast<uint4 *>(x)[0] = xa[0];
+        reinterpret_cast<uint4 *>(x)[1] = xa[1];
 #pragma unroll
         for (int i = 0; i < 16; i++)
-            o[i] = __float2bfloat16(__bfloat162float(xa[i]) > 0.0f ? v[i] : 0.0f);
-        uint4 *dst = reinterpret_cast<uint4 *>(dx + m * g.cin + c0);
+            o[i] = __float2bfloat16(__bfloat162float(x[i]) > 0.0f ? v[i] : 0.0f);
+        uint4 *dst = reinterpret_cast<uint4 *>(dx + r.pos * g.cin + c0);
         dst[0] = reinterpret_cast<const uint4 *>(o)[0];
         dst[1] = reinterpret_cast<const uint4 *>(o)[1];
     }
 };
 
-// wgrad: rows = (tap, c_in) pairs (27 * cin, tile rows beyond are zero),
-// K = output positions (split over CTAs), N = cout.  Both operands are
-// gathered transposed (positions along K).  The result is added into dw
-// [27 * cin][cout] fp32 with atomics.
+// wgrad: rows = (tap, c_in) pairs (27 * cin, tile rows beyond are zero), K =
+// output positions (split over CTAs), N = 64 (columns beyond cout are zero).
+// The result is added into dw [27 * cin][cout] fp32 with atomics.
 struct OpWgrad {
+    static constexpr bool kMN = true;
     Geo g;
     const __nv_bfloat16 *x;  // [npos_in][cin]
     const __nv_bfloat16 *dz; // [npos_out][cout]
     float *dw;               // [27 * cin][cout]
     int kchunks_total;       // ceil(npos_out / 64)
-    __device__ __forceinline__ long long rows() const { return 27LL * g.cin; }
-    __device__ __forceinline__ int kchunks() const { return kchunks_total; }
-
-    // element (row r, K column j) of a tile: byte offset in the swizzled layout
-    static __device__ __forceinline__ uint32_t el(int r, int j) { return sw128(r, j >> 3) + ((j & 7) << 1); }
-
-    __device__ __forceinline__ void load_a(uint8_t *sa, long long m0, int kc, int tid) const
+    int lgc;
+    FastDiv qo;
+    struct Row {
+        int m;                // this thread's accumulator row
+        int kz, ky, kx, c0;   // of the eight rows that it gathers (kz < 0: none)
+    };
+    __device__ __forceinline__ void chunks(int, int split, int nsplit, int &kc0, int &kc1) const
     {
-        // zero the tile, then scatter the live (position, tap, channel) values
-        for (int it = tid; it < kBM * 8; it += kThreads)
-            st_shared16(sa, sw128(it >> 3, it & 7), zero4());
-        __syncthreads();
-        const long long p0 = (long long)kc * kBK;
-        const long long np = g.npos_out();
+        const int per = (kchunks_total + nsplit - 1) / nsplit;
+        kc0 = split * per;
+        kc1 = min(kchunks_total, kc0 + per);
+    }
+    __device__ __forceinline__ Row row(int tile, int tid) const
+    {
+        Row r;
+        r.m = tile * kBM + tid;
+        const int r0 = tile * kBM + (tid & 15) * 8, t = r0 >> lgc;
+        r.c0 = r0 & (g.cin - 1);
+        r.kz = t < 27 ? t / 9 : -1;
+        r.ky = t / 3 % 3;
+        r.kx = t % 3;
+        return r;
+    }
+    __device__ __forceinline__ void load(uint8_t *sa, uint8_t *sb, const Row &r, int kc, int tid, int) const
+    {
+        const unsigned np = (unsigned)g.npos_out();
         const int d = g.di, dd = g.dout;
-        if (g.cin >= 8) {
-            const int groups = kBM / 8; // 8 channels per group
-            for (int it = tid; it < kBK * groups; it += kThreads) {
-                const int j = it % kBK, gr = it / kBK;
-                const long long r0 = m0 + (long long)gr * 8;
-                const long long p = p0 + j;
-                if (r0 >= rows() || p >= np)
-                    continue;
-                const int t = (int)(r0 / g.cin), c0 = (int)(r0 - (long long)t * g.cin);
-                long long q = p;
-                const int ox = (int)(q % dd);
-                q /= dd;
-                const int oy = (int)(q % dd);
-                q /= dd;
-                const int oz = (int)(q % dd);
-                const int n = (int)(q / dd);
-                const int iz = 2 * oz + t / 9 - 1, iy = 2 * oy + (t / 3) % 3 - 1, ix = 2 * ox + t % 3 - 1;
-                if (iz < 0 || iz >= d || iy < 0 || iy >= d || ix < 0 || ix >= d)
-                    continue;
-                const uint4 v = *reinterpret_cast<const uint4 *>(
-                    x + ((((long long)n * d + iz) * d + iy) * d + ix) * g.cin + c0);
-                const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&v);
-                const int rl = gr * 8;
+        // A: 64 positions x 16 groups of 8 rows; this thread group tid % 16
 #pragma unroll
-                for (int u = 0; u < 8; u++)
-                    *reinterpret_cast<__nv_bfloat16 *>(sa + el(rl + u, j)) = e[u];
-            }
-        } else { // cin == 1: rows are the 27 taps
-            for (int it = tid; it < kBK * 27; it += kThreads) {
-                const int j = it % kBK, t = it / kBK;
-                const long long p = p0 + j;
-                if (m0 != 0 || p >= np)
-                    continue;
-                long long q = p;
-                const int ox = (int)(q % dd);
-                q /= dd;
-                const int oy = (int)(q % dd);
-                q /= dd;
-                const int oz = (int)(q % dd);
-                const int n = (int)(q / dd);
-                const int iz = 2 * oz + t / 9 - 1, iy = 2 * oy + (t / 3) % 3 - 1, ix = 2 * ox + t % 3 - 1;
-                if (iz < 0 || iz >= d || iy < 0 || iy >= d || ix < 0 || ix >= d)
-                    continue;
-                *reinterpret_cast<__nv_bfloat16 *>(sa + el(t, j)) = x[(((long long)n * d + iz) * d + iy) * d + ix];
-            }
+        for (int u = 0; u < 8; u++) {
+            const int j = (tid >> 4) + 8 * u;
+            const unsigned p = (unsigned)kc * kBK + j, q1 = fdiv(p, qo), q2 = fdiv(q1, qo), n = fdiv(q2, qo);
+            const int iz = 2 * (int)(q2 - n * dd) + r.kz - 1, iy = 2 * (int)(q1 - q2 * dd) + r.ky - 1,
+                      ix = 2 * (int)(p - q1 * dd) + r.kx - 1;
+            const bool in = r.kz >= 0 && p < np && iz >= 0 && iz < d && iy >= 0 && iy < d && ix >= 0 && ix < d;
+            cp16(sa + swmn(j, tid & 15), in ? x + ((((long long)n * d + iz) * d + iy) * d + ix) * g.cin + r.c0 : x, in);
+        }
+        // B: 64 positions x 8 groups of 8 columns
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int j = (tid >> 3) + 16 * u, c0 = (tid & 7) * 8;
+            const unsigned p = (unsigned)kc * kBK + j;
+            const bool in = p < np && c0 < g.cout;
+            cp16(sb + swmn(j, tid & 7), in ? dz + (long long)p * g.cout + c0 : dz, in);
         }
     }
-
-    __device__ __forceinline__ void load_b(uint8_t *sb, int kc, int tid, int bn) const
+    __device__ __forceinline__ void store(const Row &r, int c0, const float *v) const
     {
-        for (int it = tid; it < bn * 8; it += kThreads)
-            st_shared16(sb, sw128(it >> 3, it & 7), zero4());
-        __syncthreads();
-        const long long p0 = (long long)kc * kBK;
-        const long long np = g.npos_out();
-        const int groups = bn / 8;
-        for (int it = tid; it < kBK * groups; it += kThreads) {
-            const int j = it % kBK, gr = it / kBK;
-            const long long p = p0 + j;
-            if (p >= np)
-                continue;
-            const uint4 v = *reinterpret_cast<const uint4 *>(dz + p * g.cout + gr * 8);
-            const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&v);
-#pragma unroll
-            for (int u = 0; u < 8; u++)
-                *reinterpret_cast<__nv_bfloat16 *>(sb + el(gr * 8 + u, j)) = e[u];
-        }
-    }
-
-    __device__ __forceinline__ void store(long long m, int c0, const float *v, int bn) const
-    {
-        if (m >= rows())
+        if (r.m >= 27 * g.cin || c0 >= g.cout)
             return;
-        float *dst = dw + m * g.cout + c0;
+        float4 *dst = reinterpret_cast<float4 *>(dw + (long long)r.m * g.cout + c0);
 #pragma unroll
-        for (int i = 0; i < 16; i++)
-            if (v[i] != 0.0f)
-                atomicAdd(dst + i, v[i]);
-        (void)bn;
+        for (int i = 0; i < 4; i++)
+            atomicAdd(dst + i, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
     }
 };
 
@@ -468,12 +477,17 @@ struct TileSmem {
 };
 
 // Error codes written to *err: 1 = an mbarrier wait ran out of time.
+// Bound by the gather's latency and L2 traffic (a chunk's 16 to 24 KB are a few
+// hundred cycles of tensor core work), hence two chunks in flight per CTA and
+// three to four CTAs on an SM.  At batch 64, three layers: forward 0.15, dgrad
+// 0.21, wgrad 0.13 ms; with loads that each chunk waited for, K-major wgrad tiles
+// and all 27 taps in dgrad, four layers took 0.67, 1.51 and 1.14 ms.
 template <class Op, int BN>
-__global__ void __launch_bounds__(kThreads) k_umma_conv(Op op, int ksplit, int *err)
+__global__ void __launch_bounds__(kThreads) k_umma_conv(Op op, int ntiles, int ksplit, int *err)
 {
     static_assert(BN == 16 || BN == 32 || BN == 64, "tile width");
     constexpr int kCols = BN < 32 ? 32 : BN; // TMEM allocation: a power of two >= 32
-    constexpr uint32_t kIdesc = idesc_bf16(BN);
+    constexpr uint32_t kIdesc = idesc_bf16(BN, Op::kMN);
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bar[kStages];
     __shared__ __align__(8) uint64_t done_bar;
@@ -497,58 +511,83 @@ __global__ void __launch_bounds__(kThreads) k_umma_conv(Op op, int ksplit, int *
     tc_fence_after();
     const uint32_t tmem = tmem_base;
 
-    const long long m0 = (long long)blockIdx.x * kBM;
-    const int nk_all = op.kchunks();
-    const int per = (nk_all + ksplit - 1) / ksplit;
-    const int kc0 = blockIdx.y * per;
-    const int kc1 = min(nk_all, kc0 + per);
     bool ok = true;
-    int issued = 0;
-    for (int kc = kc0; kc < kc1; kc++) {
-        const int i = kc - kc0;
-        const int s = i % kStages;
-        uint8_t *sa = smem + s * TileSmem<BN>::kStage;
-        uint8_t *sb = sa + TileSmem<BN>::kA;
-        if (i >= kStages) // the MMAs that read this stage (chunk i - kStages) are done
-            ok = mbar_wait(&bar[s], (unsigned)((i / kStages) - 1) & 1u);
-        if (!__syncthreads_and(ok)) {
-            ok = false;
+    int gi = 0; // chunks of the earlier items: chunk i of this one is use (gi + i) / kStages of its stage
+    const int items = ntiles * ksplit;
+    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+        const int tile = item / ksplit;
+        int kc0, kc1;
+        op.chunks(tile, item - tile * ksplit, ksplit, kc0, kc1);
+        const int n = kc1 - kc0;
+        if (n <= 0)
+            continue;
+        const typename Op::Row row = op.row(tile, tid);
+        // chunk i into its stage, once the MMAs of the stage's last use are done
+        auto fetch = [&](int i) {
+            if (i < n) {
+                const int use = gi + i, s = use % kStages;
+                if (use >= kStages)
+                    ok = mbar_wait(&bar[s], (unsigned)(use / kStages - 1) & 1u) && ok;
+                uint8_t *sa = smem + s * TileSmem<BN>::kStage;
+                if (ok)
+                    op.load(sa, sa + TileSmem<BN>::kA, row, kc0 + i, tid, BN);
+            }
+            cp_commit(); // (a group per chunk, empty past the last)
+        };
+        fetch(0);
+        fetch(1);
+        int i = 0;
+        for (; i < n; i++) {
+            cp_wait<1>(); // chunk i has landed
+            fence_async_smem();
+            if (!__syncthreads_and(ok)) {
+                ok = false;
+                break;
+            }
+            if (tid == 0) {
+                tc_fence_after();
+                const int s = (gi + i) % kStages;
+                const uint32_t a0 = smem_u32(smem + s * TileSmem<BN>::kStage), b0 = a0 + TileSmem<BN>::kA;
+#pragma unroll
+                for (int kk = 0; kk < kBK / 16; kk++)
+                    umma_bf16(tmem, Op::kMN ? sdesc_mn128(a0 + kk * 2048) : sdesc_sw128(a0 + kk * 32),
+                              Op::kMN ? sdesc_mn128(b0 + kk * 2048) : sdesc_sw128(b0 + kk * 32), kIdesc,
+                              (i > 0 || kk > 0) ? 1u : 0u);
+                umma_commit(&bar[s]);
+            }
+            fetch(i + 2);
+        }
+        if (!ok)
             break;
+        gi += n;
+        // the item's last MMA (and so all of them)
+        ok = mbar_wait(&bar[(gi - 1) % kStages], (unsigned)((gi - 1) / kStages) & 1u);
+        tc_fence_after();
+        // one decision for the whole CTA: tcgen05.ld below is warp-collective
+        ok = __syncthreads_and(ok) != 0;
+        if (ok) {
+            const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
+#pragma unroll
+            for (int c0 = 0; c0 < BN; c0 += 16) {
+                float v[16];
+                tmem_ld16(lane_addr + (uint32_t)c0, v);
+                op.store(row, c0, v);
+            }
         }
-        op.load_a(sa, m0, kc, tid);
-        op.load_b(sb, kc, tid, BN);
-        fence_async_smem();
+        // the next item's MMAs overwrite the accumulator
+        tc_fence_before();
         __syncthreads();
-        if (tid == 0) {
-            tc_fence_after();
-            const uint32_t a0 = smem_u32(sa), b0 = smem_u32(sb);
-#pragma unroll
-            for (int kk = 0; kk < kBK / 16; kk++)
-                umma_bf16(tmem, sdesc_sw128(a0 + kk * 32), sdesc_sw128(b0 + kk * 32), kIdesc,
-                          (i > 0 || kk > 0) ? 1u : 0u);
-            umma_commit(&bar[s]);
-        }
-        issued++;
+        tc_fence_after();
     }
-    // all MMAs of this CTA done (or none issued)
-    if (tid == 0)
-        umma_commit(&done_bar);
-    const bool done = mbar_wait(&done_bar, 0);
-    tc_fence_after();
-    // one decision for the whole CTA: tcgen05.ld below is warp-collective
-    const bool good = __syncthreads_and(done && ok) != 0;
-    if (!good) {
-        if (tid == 0)
+    cp_wait<0>();
+    if (!__syncthreads_and(ok)) {
+        // own MMAs in flight, for a bounded time
+        if (tid == 0) {
             atomicExch(err, 1);
-    } else if (issued > 0) {
-        const long long m = m0 + tid;
-        const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-#pragma unroll
-        for (int c0 = 0; c0 < BN; c0 += 16) {
-            float v[16];
-            tmem_ld16(lane_addr + (uint32_t)c0, v);
-            op.store(m, c0, v, BN);
+            umma_commit(&done_bar);
         }
+        mbar_wait(&done_bar, 0);
+        tc_fence_after();
     }
     tc_fence_before();
     __syncthreads();
@@ -557,33 +596,267 @@ __global__ void __launch_bounds__(kThreads) k_umma_conv(Op op, int ksplit, int *
 }
 
 template <class Op, int BN>
-static int launch_tiles(const Op &op, long long rows, int ksplit, int *err, cudaStream_t st, const char *name,
+static int launch_tiles(const Op &op, int ntiles, int ksplit, int *err, cudaStream_t st, const char *name,
                         double flops)
 {
     const int smem = TileSmem<BN>::kBytes;
     PMG_CUDA(cudaFuncSetAttribute(k_umma_conv<Op, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    const dim3 grid((unsigned)((rows + kBM - 1) / kBM), (unsigned)ksplit);
+    // resident CTAs: shared memory (227 KB of an SM) allows three or four
+    const long long items = (long long)ntiles * ksplit;
+    const unsigned grid = (unsigned)std::min<long long>(items, 152LL * (227 * 1024 / (smem + 1024)));
     const int ps__ = prof_begin(name, st);
-    k_umma_conv<Op, BN><<<grid, kThreads, smem, st>>>(op, ksplit, err);
+    k_umma_conv<Op, BN><<<grid, kThreads, smem, st>>>(op, ntiles, ksplit, err);
     prof_end(ps__, flops, st);
     PMG_CHECK_LAUNCH();
     return PMG_OK;
 }
 
 template <class Op>
-static int launch_bn(const Op &op, int bn, long long rows, int ksplit, int *err, cudaStream_t st, const char *name,
+static int launch_bn(const Op &op, int bn, int ntiles, int ksplit, int *err, cudaStream_t st, const char *name,
                      double flops)
 {
     switch (bn) {
     case 16:
-        return launch_tiles<Op, 16>(op, rows, ksplit, err, st, name, flops);
+        return launch_tiles<Op, 16>(op, ntiles, ksplit, err, st, name, flops);
     case 32:
-        return launch_tiles<Op, 32>(op, rows, ksplit, err, st, name, flops);
+        return launch_tiles<Op, 32>(op, ntiles, ksplit, err, st, name, flops);
     case 64:
-        return launch_tiles<Op, 64>(op, rows, ksplit, err, st, name, flops);
+        return launch_tiles<Op, 64>(op, ntiles, ksplit, err, st, name, flops);
     default:
         set_error("cnn: output channels %d not in {16, 32, 64}", bn);
         return PMG_EINVAL;
+    }
+}
+
+// ---- the first layer: one input channel ---------------------------------------------
+constexpr int kPatchX = 32, kPatchY = 4; // output positions of a tile: 128
+
+// Forward: the tile kernel's GEMM with the A rows built from the patch of the
+// input that the 4 x 32 positions read (even and odd columns apart, so that a
+// warp's reads are consecutive).  K is 27 padded to 32; a GEMM over the 64 that
+// the weights are padded to adds zeros.  Bound by the patch's loads and the 32
+// bytes written per position; taps gathered one by one from global memory were
+// most of the forward's 0.67 ms at batch 64, this is 0.08 ms.
+template <int BN>
+__global__ void __launch_bounds__(kThreads) k_conv1_fwd(const __nv_bfloat16 *__restrict__ x,
+                                                        const __nv_bfloat16 *__restrict__ wk, int kp,
+                                                        const float *__restrict__ bias, __nv_bfloat16 *__restrict__ y,
+                                                        int d, int dd, int ty, int tx, int ntiles, int *err)
+{
+    constexpr int kCols = BN < 32 ? 32 : BN, kRows = 2 * kPatchY + 1;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __nv_bfloat16 s_e[3][kRows][kPatchX + 2], s_o[3][kRows][kPatchX];
+    __shared__ __align__(8) uint64_t bar, done_bar;
+    __shared__ uint32_t tmem_base;
+    uint8_t *sa = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t *sb = sa + kBM * 128;
+    const int tid = threadIdx.x, warp = tid >> 5, xl = tid & 31, yl = tid >> 5;
+    if (warp == 0) {
+        tmem_alloc(&tmem_base, kCols);
+        tmem_relinquish();
+    }
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        mbar_init(&done_bar, 1);
+        fence_barrier_init();
+    }
+    for (int it = tid; it < BN * 4; it += kThreads) {
+        const int r = it >> 2, j = it & 3;
+        *reinterpret_cast<uint4 *>(sb + sw128(r, j)) =
+            *reinterpret_cast<const uint4 *>(wk + (long long)r * kp + j * 8);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base;
+    bool ok = true;
+    unsigned phase = 0;
+    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+        int t = tile;
+        const int xb = t % tx;
+        t /= tx;
+        const int yb = t % ty;
+        t /= ty;
+        const int z = t % dd, n = t / dd;
+        // patch column c is input column ix0 - 1 + c: pairs (2 q + 1, 2 q + 2) from input column ix0 + 2 q
+        const int ix0 = 2 * xb * kPatchX, iy0 = 2 * yb * kPatchY - 1;
+        for (int it = tid; it < 3 * kRows * (kPatchX + 1); it += kThreads) {
+            const int row = it / (kPatchX + 1), q = it - row * (kPatchX + 1) - 1;
+            const int kz = row / kRows, yy = row - kz * kRows;
+            const int iz = 2 * z - 1 + kz, iy = iy0 + yy, ix = ix0 + 2 * q;
+            __nv_bfloat16 a = __float2bfloat16(0.0f), b = a;
+            if (iz >= 0 && iz < d && iy >= 0 && iy < d) {
+                const __nv_bfloat16 *src = x + (((long long)n * d + iz) * d + iy) * d;
+                if (ix >= 0 && ix < d)
+                    a = src[ix];
+                if (ix + 1 >= 0 && ix + 1 < d)
+                    b = src[ix + 1];
+            }
+            if (q >= 0)
+                s_o[kz][yy][q] = a;
+            s_e[kz][yy][q + 1] = b;
+        }
+        __syncthreads();
+        __align__(16) __nv_bfloat16 k[32];
+#pragma unroll
+        for (int tap = 0; tap < 32; tap++) {
+            const int kz = tap / 9, ky = tap / 3 % 3, kx = tap % 3;
+            if (tap < 27)
+                k[tap] = kx == 1 ? s_o[kz][2 * yl + ky][xl] : s_e[kz][2 * yl + ky][xl + (kx >> 1)];
+            else
+                k[tap] = __float2bfloat16(0.0f);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            *reinterpret_cast<uint4 *>(sa + sw128(tid, j)) = reinterpret_cast<const uint4 *>(k)[j];
+        fence_async_smem();
+        __syncthreads();
+        if (tid == 0) {
+            tc_fence_after();
+            const uint32_t a0 = smem_u32(sa), b0 = smem_u32(sb);
+#pragma unroll
+            for (int kk = 0; kk < 2; kk++)
+                umma_bf16(tmem, sdesc_sw128(a0 + kk * 32), sdesc_sw128(b0 + kk * 32), idesc_bf16(BN, false), kk > 0);
+            umma_commit(&bar);
+        }
+        ok = mbar_wait(&bar, phase);
+        phase ^= 1u;
+        tc_fence_after();
+        ok = __syncthreads_and(ok) != 0; // tcgen05.ld is warp-collective
+        if (ok) {
+            const int ox = xb * kPatchX + xl, oy = yb * kPatchY + yl;
+            const bool in = ox < dd && oy < dd;
+            __nv_bfloat16 *dst = y + ((((long long)n * dd + z) * dd + oy) * dd + ox) * BN;
+#pragma unroll
+            for (int c0 = 0; c0 < BN; c0 += 16) {
+                float v[16];
+                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+                __align__(16) __nv_bfloat16 o[16];
+#pragma unroll
+                for (int c = 0; c < 16; c++)
+                    o[c] = __float2bfloat16(fmaxf(v[c] + bias[c0 + c], 0.0f));
+                if (in) {
+                    reinterpret_cast<uint4 *>(dst + c0)[0] = reinterpret_cast<const uint4 *>(o)[0];
+                    reinterpret_cast<uint4 *>(dst + c0)[1] = reinterpret_cast<const uint4 *>(o)[1];
+                }
+            }
+        }
+        tc_fence_before(); // (the next MMA overwrites the accumulator, after two barriers)
+    }
+    if (!__syncthreads_and(ok)) {
+        if (tid == 0) {
+            atomicExch(err, 1);
+            umma_commit(&done_bar);
+        }
+        mbar_wait(&done_bar, 0);
+        tc_fence_after();
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0)
+        tmem_dealloc(tmem, kCols);
+}
+
+static int kpad(int k) { return (k + kBK - 1) / kBK * kBK; }
+
+template <int BN>
+static int launch_conv1_fwd(const __nv_bfloat16 *x, const __nv_bfloat16 *wk, const float *bias, __nv_bfloat16 *y,
+                            const Geo &g, int *err, cudaStream_t st)
+{
+    const int smem = kBM * 128 + BN * 128 + 1024;
+    PMG_CUDA(cudaFuncSetAttribute(k_conv1_fwd<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const int ty = (g.dout + kPatchY - 1) / kPatchY, tx = (g.dout + kPatchX - 1) / kPatchX;
+    const long long tiles = (long long)g.batch * g.dout * ty * tx;
+    const int ps__ = prof_begin("k_conv1_fwd", st);
+    k_conv1_fwd<BN><<<(unsigned)std::min<long long>(tiles, 152 * 8), kThreads, smem, st>>>(
+        x, wk, kpad(27), bias, y, g.di, g.dout, ty, tx, (int)tiles, err);
+    prof_end(ps__, 2.0 * g.batch * g.dout * g.dout * g.dout * g.cout * 27.0, st);
+    PMG_CHECK_LAUNCH();
+    return PMG_OK;
+}
+
+// Weight gradient: a warp takes 32 output positions of a row one after the
+// other, lane = tap (lane 27: the constant 1, whose row is the bias gradient),
+// 16 output channels (blockIdx.y) in registers.  128 threads on 4 x 32 positions,
+// blocks stride over the tiles.  Bound by the shared-memory reads that feed the
+// FMAs and by the patch's loads: 0.15 ms at batch 64.
+constexpr int kWgY = 4;
+
+__global__ void __launch_bounds__(128) k_conv1_wgrad(const __nv_bfloat16 *__restrict__ x,
+                                                     const __nv_bfloat16 *__restrict__ dz, float *__restrict__ dw,
+                                                     float *__restrict__ db, int d, int dd, int cout, int ty, int tx,
+                                                     int ntiles)
+{
+    // banks of the 27 taps of one position: row stride 67 = 3, plane stride 617 = 9 (mod 32)
+    constexpr int kRows = 2 * kWgY + 1, kCols = 2 * kPatchX + 1, kRS = 67, kPS = 617;
+    static_assert(kRows * kRS <= kPS, "planes do not overlap");
+    __shared__ float s_x[3 * kPS];
+    __shared__ __align__(16) float s_d[128][16];
+    const int c0 = blockIdx.y * 16, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int kz = lane / 9, ky = lane / 3 % 3, kx = lane % 3;
+    const float fixed = lane == 27 ? 1.0f : 0.0f;
+    float acc[16];
+#pragma unroll
+    for (int c = 0; c < 16; c++)
+        acc[c] = 0.0f;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        int t = tile;
+        const int xb = t % tx;
+        t /= tx;
+        const int yb = t % ty;
+        t /= ty;
+        const int z = t % dd, n = t / dd;
+        __syncthreads(); // (the last tile's readers)
+        for (int it = threadIdx.x; it < 3 * kRows * kCols; it += blockDim.x) {
+            const int row = it / kCols, c = it - row * kCols, pz = row / kRows, yy = row - pz * kRows;
+            const int iz = 2 * z - 1 + pz, iy = 2 * yb * kWgY - 1 + yy, ix = 2 * xb * kPatchX - 1 + c;
+            const bool in = iz >= 0 && iz < d && iy >= 0 && iy < d && ix >= 0 && ix < d;
+            s_x[pz * kPS + yy * kRS + c] =
+                in ? __bfloat162float(x[(((long long)n * d + iz) * d + iy) * d + ix]) : 0.0f;
+        }
+        {
+            const int oy = yb * kWgY + w, ox = xb * kPatchX + lane;
+            uint4 q[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+            if (oy < dd && ox < dd) {
+                const uint4 *src =
+                    reinterpret_cast<const uint4 *>(dz + ((((long long)n * dd + z) * dd + oy) * dd + ox) * cout + c0);
+                q[0] = src[0];
+                q[1] = src[1];
+            }
+            const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(q);
+            float4 *dst = reinterpret_cast<float4 *>(s_d[threadIdx.x]);
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                dst[c] = make_float4(__bfloat162float(e[4 * c]), __bfloat162float(e[4 * c + 1]),
+                                     __bfloat162float(e[4 * c + 2]), __bfloat162float(e[4 * c + 3]));
+        }
+        __syncthreads();
+        const float *sx = s_x + (lane < 27 ? kz * kPS + (2 * w + ky) * kRS + kx : 0);
+#pragma unroll 4
+        for (int p = 0; p < 32; p++) {
+            const float v = lane < 27 ? sx[2 * p] : fixed;
+            const float4 *q = reinterpret_cast<const float4 *>(s_d[w * 32 + p]);
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const float4 f = q[c];
+                acc[4 * c] = __fmaf_rn(v, f.x, acc[4 * c]);
+                acc[4 * c + 1] = __fmaf_rn(v, f.y, acc[4 * c + 1]);
+                acc[4 * c + 2] = __fmaf_rn(v, f.z, acc[4 * c + 2]);
+                acc[4 * c + 3] = __fmaf_rn(v, f.w, acc[4 * c + 3]);
+            }
+        }
+    }
+    // the four warps' sums, then one add per block
+    __syncthreads();
+    float4 *mine = reinterpret_cast<float4 *>(s_d[threadIdx.x]);
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+        mine[c] = make_float4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
+    __syncthreads();
+    for (int it = threadIdx.x; it < 28 * 16; it += blockDim.x) {
+        const int tap = it >> 4, c = it & 15;
+        const float v = s_d[tap][c] + s_d[32 + tap][c] + s_d[64 + tap][c] + s_d[96 + tap][c];
+        atomicAdd(tap < 27 ? dw + tap * cout + c0 + c : db + c0 + c, v);
     }
 }
 
@@ -600,7 +873,8 @@ static int check_geo(int batch, int di, int cin, int cout)
     return PMG_OK;
 }
 
-static int kpad(int k) { return (k + kBK - 1) / kBK * kBK; }
+
+static int log2_of(int c) { return c == 16 ? 4 : c == 32 ? 5 : 6; }
 
 // ---- weight packing (fp32 master [cout][cin][27] -> bf16 GEMM operands) -------------
 
@@ -632,19 +906,27 @@ __global__ void k_unpack_dw(const float *__restrict__ dw, int cin, int cout, flo
     }
 }
 
-// bias gradient: db[o] = sum over positions of dz[p][o]
-__global__ void k_bias_grad(const __nv_bfloat16 *__restrict__ dz, long long np, int cout, float *__restrict__ db)
+// bias gradient: db[o] = sum over positions of dz[p][o]; eight channels per
+// thread.
+__global__ void __launch_bounds__(256) k_bias_grad(const __nv_bfloat16 *__restrict__ dz, long long np, int cout,
+                                                   float *__restrict__ db)
 {
     __shared__ float acc[64];
     if (threadIdx.x < 64)
         acc[threadIdx.x] = 0.0f;
     __syncthreads();
-    const int o = threadIdx.x % cout;
-    const int lanes = blockDim.x / cout;
-    float s = 0.0f;
-    for (long long p = (long long)blockIdx.x * lanes + threadIdx.x / cout; p < np; p += (long long)gridDim.x * lanes)
-        s += __bfloat162float(dz[p * cout + o]);
-    atomicAdd(&acc[o], s);
+    const int groups = cout >> 3, gr = threadIdx.x % groups, lanes = blockDim.x / groups;
+    float s[8] = {};
+    for (long long p = (long long)blockIdx.x * lanes + threadIdx.x / groups; p < np; p += (long long)gridDim.x * lanes) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(dz + p * cout + gr * 8);
+        const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&v);
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            s[i] += __bfloat162float(e[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+        atomicAdd(&acc[gr * 8 + i], s[i]);
     __syncthreads();
     if (threadIdx.x < cout)
         atomicAdd(db + threadIdx.x, acc[threadIdx.x]);
@@ -792,15 +1074,26 @@ extern "C" int pmg_cnn_conv_fwd(const void *x, const void *wk, const float *bias
         return PMG_EINVAL;
     }
     PMG_TRY(check_geo(batch, di, cin, cout));
+    cudaStream_t st = as_stream(stream);
+    const Geo g{batch, di, (di + 1) / 2, cin, cout};
+    const long long rows = (long long)batch * g.dout * g.dout * g.dout;
+    if (cin == 1) {
+        const auto *px = (const __nv_bfloat16 *)x, *pw = (const __nv_bfloat16 *)wk;
+        auto *py = (__nv_bfloat16 *)y;
+        return cout == 16   ? launch_conv1_fwd<16>(px, pw, bias, py, g, err, st)
+               : cout == 32 ? launch_conv1_fwd<32>(px, pw, bias, py, g, err, st)
+                            : launch_conv1_fwd<64>(px, pw, bias, py, g, err, st);
+    }
     OpFwd op;
-    op.g = Geo{batch, di, (di + 1) / 2, cin, cout};
+    op.g = g;
     op.x = (const __nv_bfloat16 *)x;
     op.wk = (const __nv_bfloat16 *)wk;
     op.bias = bias;
     op.y = (__nv_bfloat16 *)y;
     op.kp = kpad(27 * cin);
-    const long long rows = (long long)batch * op.g.dout * op.g.dout * op.g.dout;
-    return launch_bn(op, cout, rows, 1, err, as_stream(stream), "k_umma_conv_fwd",
+    op.lgc = log2_of(cin);
+    op.qo = fastdiv_of((unsigned)g.dout);
+    return launch_bn(op, cout, (int)((rows + kBM - 1) / kBM), 1, err, st, "k_umma_conv_fwd",
                      2.0 * rows * cout * 27.0 * cin);
 }
 
@@ -823,8 +1116,20 @@ extern "C" int pmg_cnn_conv_dgrad(const void *dz, const void *wkt, const void *x
     op.xact = (const __nv_bfloat16 *)xact;
     op.dx = (__nv_bfloat16 *)dx;
     op.kp = kpad(27 * cout);
+    op.lgc = log2_of(cout);
+    op.nh[0] = (di + 1) / 2;
+    op.nh[1] = di / 2;
+    for (int p = 0; p < 2; p++)
+        op.qh[p] = fastdiv_of((unsigned)op.nh[p]);
+    long long tiles = 0;
+    for (int k = 0; k < 8; k++) {
+        const int c = 7 - k;
+        op.first[k] = (int)tiles;
+        tiles += ((long long)batch * op.nh[c >> 2] * op.nh[(c >> 1) & 1] * op.nh[c & 1] + kBM - 1) / kBM;
+    }
+    op.first[8] = (int)tiles;
     const long long rows = (long long)batch * di * di * di;
-    return launch_bn(op, cin, rows, 1, err, as_stream(stream), "k_umma_conv_dgrad",
+    return launch_bn(op, cin, (int)tiles, 1, err, as_stream(stream), "k_umma_conv_dgrad",
                      2.0 * rows * cin * 27.0 * cout / 8.0);
 }
 
@@ -838,29 +1143,42 @@ extern "C" int pmg_cnn_conv_wgrad(const void *x, const void *dz, float *dw, floa
     }
     PMG_TRY(check_geo(batch, di, cin, cout));
     cudaStream_t st = as_stream(stream);
-    OpWgrad op;
-    op.g = Geo{batch, di, (di + 1) / 2, cin, cout};
-    op.x = (const __nv_bfloat16 *)x;
-    op.dz = (const __nv_bfloat16 *)dz;
-    op.dw = dw;
-    const long long np = (long long)batch * op.g.dout * op.g.dout * op.g.dout;
-    op.kchunks_total = (int)((np + kBK - 1) / kBK);
+    const Geo g{batch, di, (di + 1) / 2, cin, cout};
+    const long long np = (long long)batch * g.dout * g.dout * g.dout;
     const long long rows = 27LL * cin;
-    const int mt = (int)((rows + kBM - 1) / kBM);
-    // split K so that about four CTAs run per SM
-    int ksplit = (4 * 152 + mt - 1) / mt;
-    ksplit = std::max(1, std::min(ksplit, op.kchunks_total));
     PMG_CUDA(cudaMemsetAsync(dw, 0, sizeof(float) * (size_t)rows * cout, st));
     PMG_CUDA(cudaMemsetAsync(dbias, 0, sizeof(float) * (size_t)cout, st));
-    PMG_TRY(launch_bn(op, cout, rows, ksplit, err, st, "k_umma_conv_wgrad", 2.0 * np * cout * 27.0 * cin));
+    if (cin == 1) {
+        const int ty = (g.dout + kWgY - 1) / kWgY, tx = (g.dout + kPatchX - 1) / kPatchX;
+        const long long tiles = (long long)batch * g.dout * ty * tx;
+        const int ps__ = prof_begin("k_conv1_wgrad", st);
+        k_conv1_wgrad<<<dim3((unsigned)std::min<long long>(tiles, 152 * 8), cout / 16), 128, 0, st>>>(
+            (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)dz, dw, dbias, di, g.dout, cout, ty, tx, (int)tiles);
+        prof_end(ps__, 2.0 * np * cout * 27.0, st);
+        PMG_CHECK_LAUNCH();
+    } else {
+        OpWgrad op;
+        op.g = g;
+        op.x = (const __nv_bfloat16 *)x;
+        op.dz = (const __nv_bfloat16 *)dz;
+        op.dw = dw;
+        op.kchunks_total = (int)((np + kBK - 1) / kBK);
+        op.lgc = log2_of(cin);
+        op.qo = fastdiv_of((unsigned)g.dout);
+        const int mt = (int)((rows + kBM - 1) / kBM);
+        // split K over about three CTAs per SM, but not below eight chunks
+        // each: every split adds its whole tile with atomics
+        const int ksplit = std::max(1, std::min(3 * 152 / mt, op.kchunks_total / 8));
+        PMG_TRY((launch_tiles<OpWgrad, 64>(op, mt, ksplit, err, st, "k_umma_conv_wgrad", 2.0 * np * cout * 27.0 * cin)));
+    }
     {
         const int ps__ = prof_begin("k_unpack_dw", st);
         k_unpack_dw<<<64, 256, 0, st>>>(dw, cin, cout, grad);
         prof_end(ps__, 0.0, st);
     }
-    {
+    if (cin > 1) {
         const int ps__ = prof_begin("k_bias_grad", st);
-        k_bias_grad<<<152, 256, 0, st>>>((const __nv_bfloat16 *)dz, np, cout, dbias);
+        k_bias_grad<<<grid_for(np * (cout / 8), 256, 152LL * 4), 256, 0, st>>>((const __nv_bfloat16 *)dz, np, cout, dbias);
         prof_end(ps__, 0.0, st);
     }
     PMG_CHECK_LAUNCH();

@@ -152,4 +152,31 @@ __global__ void k_set_int2(int *p, int a, int b);
 // [1] = kRangeBig - the smallest (so a zeroed pair is the empty range).
 constexpr int kRangeBig = 1 << 30;
 
+// floor(n / d) of a 32-bit n by one multiplication (Granlund and Montgomery,
+// "Division by invariant integers using multiplication", 1994: the
+// round-up multiplier m = floor(2^32 (2^l - d) / d) + 1, l = ceil(log2 d),
+// with the add-and-halve fix-up), exact for every n and d >= 1
+struct FastDiv {
+    unsigned m;
+    int s1, s2;
+};
+
+static inline FastDiv fastdiv_of(unsigned d)
+{
+    int l = 0;
+    while (l < 32 && (1ull << l) < d)
+        l++;
+    FastDiv f;
+    f.m = (unsigned)(((1ull << 32) * ((1ull << l) - d)) / d + 1ull);
+    f.s1 = l < 1 ? l : 1;
+    f.s2 = l > 1 ? l - 1 : 0;
+    return f;
+}
+
+__device__ __forceinline__ unsigned fdiv(unsigned n, const FastDiv &f)
+{
+    const unsigned t = __umulhi(f.m, n);
+    return (t + ((n - t) >> f.s1)) >> f.s2;
+}
+
 } // namespace pmg
