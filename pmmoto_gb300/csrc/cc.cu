@@ -2297,6 +2297,7 @@ static int grow_build(GrowSel &g, const Src &src, const int64_t *shape, const in
     k_grow_start<<<grid_for(pieces, 256, 152LL * 16), 256, 0, st>>>(words(g), pieces);
     prof_end(ps__, (double)pieces * 40, st);
     PMG_CHECK_LAUNCH();
+    PMG_CUDA(cudaMemsetAsync(g.npairs, 0, sizeof(int), st));
     g.stamp = 0;
     g.built = true;
     g.pending = false;
@@ -2327,16 +2328,14 @@ static int grow_masks(GrowSel &g, const Src &src, const int64_t *shape, const in
     return PMG_OK;
 }
 
-// Unions of one set, or of two in one launch.
+// Unions of one set, or of two in one launch (their pair counts are zero: the
+// selection of the last step or the build cleared them).
 static int grow_rows(GrowSel &a, GrowSel *b, const int64_t *shape, int *err, cudaStream_t st)
 {
     const BGrid G = bgrid_of(shape);
     const int nt2 = (G.b2 + kT2 - 1) / kT2, pieces = row_pieces(G), cap = G.b0 * G.b1 * G.b2 / 2;
     const RowSet A{a.P, words(a), a.pairs, a.npairs, cap}, B = b ? RowSet{b->P, words(*b), b->pairs, b->npairs, cap} : A;
     const unsigned sets = b ? 2 : 1;
-    PMG_CUDA(cudaMemsetAsync(a.npairs, 0, sizeof(int), st));
-    if (b)
-        PMG_CUDA(cudaMemsetAsync(b->npairs, 0, sizeof(int), st));
     {
         const int ps__ = prof_begin("k_grow_pairs", st);
         k_grow_pairs<<<dim3((unsigned)((pieces + kGrowPieces - 1) / kGrowPieces), sets), kGrowThreads, 0, st>>>(A, B, G,
@@ -2366,6 +2365,7 @@ static int grow_step(GrowSel &g, const Src &src, const int64_t *shape, const int
         PMG_TRY(grow_masks(g, src, shape, nullptr, err, st));
         PMG_TRY(grow_rows(g, nullptr, shape, err, st));
         PMG_CUDA(cudaMemsetAsync(g.N, 0, piece_bytes(bgrid_of(shape)), st));
+        PMG_CUDA(cudaMemsetAsync(g.npairs, 0, sizeof(int), st));
         if (any_periodic(bc)) {
             const BGrid G = bgrid_of(shape);
             const long long n = shape[0] * shape[1] * shape[2];
@@ -2489,6 +2489,7 @@ struct SelectSet {
     int *P;
     uint8_t stamp;
     GrowWords W;
+    int *npairs; // cleared for the next step
 };
 
 // The unconnected blocks of four pieces (u: each lane its piece's) looked up;
@@ -2537,6 +2538,8 @@ __global__ void __launch_bounds__(256) k_pair_rows(SelectSet A, SelectSet B,
     unsigned cnt = 0;
     int xmax = 0, xmin = 0;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        *A.npairs = *B.npairs = 0;
     for (int base = warp * 4; base < pieces; base += nwarps * 4) {
         const int piece = base + (lane >> 3);
         const bool in = piece < pieces;
@@ -2782,10 +2785,10 @@ int grow_pair_select(GrowSel &a, GrowSel &b, const unsigned long long *b_count, 
 {
     const BGrid G = bgrid_of(shape);
     const int pieces = row_pieces(G);
-    PMG_CUDA(cudaMemsetAsync(xr, 0, 2 * sizeof(int), st));
     const int ps__ = prof_begin("k_pair_rows", st);
     k_pair_rows<<<grid_for((pieces + 3) / 4 * 32LL, 256, 152LL * 32), 256, 0, st>>>(
-        SelectSet{a.mark, a.P, (uint8_t)a.stamp, words(a)}, SelectSet{b.mark, b.P, (uint8_t)b.stamp, words(b)}, b_count, G,
+        SelectSet{a.mark, a.P, (uint8_t)a.stamp, words(a), a.npairs},
+        SelectSet{b.mark, b.P, (uint8_t)b.stamp, words(b), b.npairs}, b_count, G,
         (G.b2 + kT2 - 1) / kT2, out, kept, err, xr);
     // words read and written, the unconnected and the changed words (the
     // lookups come on top)
@@ -2927,6 +2930,23 @@ __device__ __forceinline__ unsigned range_bits(int tk, int z, long long lo, long
 
 constexpr int kUpdatePieces = 64; // per block of 256 threads
 
+// The running totals (own voxels of value 2, voxels of value 1) from the counts
+// of one update, which are cleared, and the saturation numerator.
+__device__ __forceinline__ void drain_totals(const DrainCounts &C, int full)
+{
+    // (atomics: the counts are the other blocks' atomic adds)
+    const unsigned long long c2 = atomicExch(C.cnt2, 0ull), c1 = atomicExch(C.cnt1, 0ull);
+    *C.tot = full ? c2 : *C.tot - c2;
+    *C.ones += c1;
+    *C.sat = *C.tot;
+}
+
+__global__ void k_drain_same(DrainCounts C) // a radius that changes nothing
+{
+    *C.sat = *C.tot;
+}
+
+
 struct UpdateSets {
     // wetting phase: row words, masks, parents, outlet stamps, tile flags
     unsigned *Vw;
@@ -2949,9 +2969,8 @@ struct UpdateSets {
 // (the slabs were refilled before), and the changes of both counts.
 __global__ void __launch_bounds__(256) k_drain_update_rows(uint8_t *__restrict__ mp, const unsigned *__restrict__ D,
                                                            UpdateSets U, BGrid G, int nt2, Boxes B,
-                                                           unsigned long long *cnt2, unsigned long long *cnt1, int *err,
-                                                           const int *__restrict__ orange, int full,
-                                                           unsigned long long *units)
+                                                           DrainCounts C, int *err, const int *__restrict__ orange,
+                                                           int full, unsigned long long *units)
 {
     const int bxlo = orange ? orange[0] >> 1 : 0, bxhi = orange ? orange[1] >> 1 : G.b0 - 1;
     const int plane = G.b1 * nt2;
@@ -3087,36 +3106,30 @@ __global__ void __launch_bounds__(256) k_drain_update_rows(uint8_t *__restrict__
     c2n = __reduce_add_sync(0xffffffffu, c2n);
     c1n = __reduce_add_sync(0xffffffffu, c1n);
     if (lane == 0 && c2n)
-        atomicAdd(cnt2, (unsigned long long)c2n);
+        atomicAdd(C.cnt2, (unsigned long long)c2n);
     if (lane == 0 && c1n)
-        atomicAdd(cnt1, (unsigned long long)c1n);
-}
-
-// Running totals (count(own == 2), count(== 1)) from the update's counts; the
-// saturation numerator and the phase-1 count out.
-__global__ void k_drain_totals(int full, unsigned long long *cnt2, unsigned long long *cnt1, unsigned long long *tot,
-                               unsigned long long *sat_out, unsigned long long *ones)
-{
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        tot[0] = full ? *cnt2 : tot[0] - *cnt2;
-        *ones += *cnt1;
-        *sat_out = tot[0];
-        *cnt2 = 0;
-        *cnt1 = 0;
+        atomicAdd(C.cnt1, (unsigned long long)c1n);
+    // the last block to finish: totals, and clean counters for the next radius
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(C.ticket, 1u) == gridDim.x - 1) {
+        __threadfence();
+        drain_totals(C, full);
+        *C.kept = 0;
+        C.xr[0] = C.xr[1] = 0;
+        *C.ticket = 0u;
     }
 }
 
-int drain_totals(bool full, unsigned long long *cnt2, unsigned long long *cnt1, unsigned long long *tot,
-                 unsigned long long *sat_out, unsigned long long *ones, cudaStream_t st)
+int drain_same(const DrainCounts &C, cudaStream_t st)
 {
-    k_drain_totals<<<1, 32, 0, st>>>(full ? 1 : 0, cnt2, cnt1, tot, sat_out, ones);
+    k_drain_same<<<1, 1, 0, st>>>(C);
     PMG_CHECK_LAUNCH();
     return PMG_OK;
 }
 
 int drain_update_rows(uint8_t *mp, const unsigned *D, const int64_t *shape, ShrinkSel &w, const Boxes &B, GrowSel *g_nw,
-                      unsigned long long *cnt2, unsigned long long *cnt1, int *err, cudaStream_t st, const int *orange,
-                      bool full)
+                      const DrainCounts &C, int *err, cudaStream_t st, const int *orange, bool full)
 {
     const BGrid G = bgrid_of(shape);
     UpdateSets U{};
@@ -3137,7 +3150,7 @@ int drain_update_rows(uint8_t *mp, const unsigned *D, const int64_t *shape, Shri
     const int ps__ = prof_begin("k_drain_update_rows", st);
     k_drain_update_rows<<<grid_for((row_pieces(G) + kUpdatePieces - 1) / kUpdatePieces * 256LL, 256, 152LL * 64), 256, 0,
                           st>>>(
-        mp, D, U, G, (G.b2 + kT2 - 1) / kT2, B, cnt2, cnt1, err, orange, full ? 1 : 0, prof_units(kUnitsDrainUpdate));
+        mp, D, U, G, (G.b2 + kT2 - 1) / kT2, B, C, err, orange, full ? 1 : 0, prof_units(kUnitsDrainUpdate));
     // per voxel visited: a bit of the dilation, of the wetting and of the
     // non-wetting phase
     prof_end_units(ps__, kUnitsDrainUpdate, 3.0 / 8.0, st);

@@ -244,14 +244,14 @@ static int porosimetry_run(const uint8_t *pm, uint8_t *out, const int64_t *shape
     float *A, *B;
     morph_split(w, shape, bc, ext_e, E, A, B);
     uint8_t *cur = w.t1;
-    PMG_CUDA(cudaMemsetAsync(w.cnt, 0, sizeof(unsigned long long), st));
     if (g_er && g_nw && (KC || Sv) && inlet && mp && m1_counted) {
         // both selections grow along the curve: one pass writes the eroded
         // inlet-connected space constrained by the inlet-connected
         // non-wetting phase (when that phase exists, counted in w.cnt[1])
         PMG_TRY(grow_marks_pair(*g_er, Sv, step, KC, Te, *g_nw, mp, 1, shape, bc, pad, Bx.inlet, w.err, st));
         // the selection's x range (w.cnt[4]) limits the dilation to the planes
-        // it can reach; the dilation's result range goes to orange
+        // it can reach; the dilation's result range goes to orange.  Like the
+        // kept count (w.cnt[0]) it is zero here (DrainCounts)
         int *xr = (int *)(w.cnt + 4);
         // the selection is written as row words (w.rows): the dilation's row
         // pass reads them directly (w.t2 receives bytes on other paths)
@@ -262,6 +262,7 @@ static int porosimetry_run(const uint8_t *pm, uint8_t *out, const int64_t *shape
         return morph_run(w.t2, out, shape, bc, pad, ext_d, res, r_d, cmp_d, 1, E, A, B, st, ball_d, w.cnt, xr,
                          orange, w.rows, rows_out);
     }
+    PMG_CUDA(cudaMemsetAsync(w.cnt, 0, sizeof(unsigned long long), st));
     if (orange) {
         // the paths below write the whole result
         k_set_int2<<<1, 32, 0, st>>>(orange, 0, (int)shape[0] - 1);
@@ -387,6 +388,54 @@ __global__ void k_first_cover(const uint8_t *__restrict__ pm, const uint8_t *__r
         }
     }
 }
+
+// A second stream that takes work between begin (after what the first stream
+// holds) and end, which join makes the first stream wait for.
+struct Fork {
+    cudaStream_t side = nullptr;
+    cudaEvent_t from = nullptr, to = nullptr;
+    bool pending = false;
+    int open()
+    {
+        PMG_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+        PMG_CUDA(cudaEventCreateWithFlags(&from, cudaEventDisableTiming));
+        PMG_CUDA(cudaEventCreateWithFlags(&to, cudaEventDisableTiming));
+        return PMG_OK;
+    }
+    int begin(cudaStream_t st)
+    {
+        PMG_CUDA(cudaEventRecord(from, st));
+        PMG_CUDA(cudaStreamWaitEvent(side, from, 0));
+        return PMG_OK;
+    }
+    int end()
+    {
+        if (cudaEventRecord(to, side) != cudaSuccess) {
+            cudaStreamSynchronize(side); // (what it holds must not outlive its scratch)
+            set_error("drainage: event record failed");
+            return PMG_ECUDA;
+        }
+        pending = true;
+        return PMG_OK;
+    }
+    int join(cudaStream_t st)
+    {
+        if (pending)
+            PMG_CUDA(cudaStreamWaitEvent(st, to, 0));
+        pending = false;
+        return PMG_OK;
+    }
+    ~Fork()
+    {
+        // (work still queued is finished before the stream goes)
+        if (to)
+            cudaEventDestroy(to);
+        if (from)
+            cudaEventDestroy(from);
+        if (side)
+            cudaStreamDestroy(side);
+    }
+};
 
 static int ext_of(const int32_t *bc, const int32_t *pad, const int32_t *ratio, int32_t *ext)
 {
@@ -848,19 +897,39 @@ extern "C" int pmg_drainage_ext(const uint8_t *pm_img, uint8_t *mp_img, const in
         s = count_eq_async(mp_img, shape, whole, 1, w.cnt + 1, st);
     // After the first update (which refills the reservoir slabs), a radius can
     // change only voxels within the dilation's x range: the update visits that
-    // range alone and counts changes (w.cnt[8], w.cnt[9], cleared by
-    // drain_totals), the saturation count being a running total (w.cnt[10]).
+    // range alone and counts changes (w.cnt[8], w.cnt[9]), the saturation count
+    // being a running total (w.cnt[10]).
     int *orange = (int *)(w.cnt + 5);
+    DrainCounts C{w.cnt + 8, w.cnt + 9, w.cnt + 10, w.cnt + 1, nullptr, w.cnt, (int *)(w.cnt + 4),
+                  (unsigned *)(w.cnt + 11)};
     if (s == PMG_OK)
-        s = cudaMemsetAsync(w.cnt + 8, 0, 3 * sizeof(unsigned long long), st) == cudaSuccess ? PMG_OK : PMG_ECUDA;
+        s = cudaMemsetAsync(w.cnt, 0, sizeof(unsigned long long), st) == cudaSuccess &&
+                    cudaMemsetAsync(w.cnt + 4, 0, 8 * sizeof(unsigned long long), st) == cudaSuccess
+                ? PMG_OK
+                : PMG_ECUDA;
+    // The wetting phase's union-find depends on the last update alone: it runs on
+    // a stream of its own beside the selection and the dilation, whose kernels
+    // leave much of the chip waiting on dependent loads.
+    Fork fork;
+    if (s == PMG_OK)
+        s = fork.open();
     bool full_done = false;
     for (int k = 0; k < n_radii && s == PMG_OK; k++) {
+        C.sat = d_counts + k;
         if (!active[k] && full_done) {
             // no dilation: nothing changes, the totals stand
-            s = drain_totals(false, w.cnt + 8, w.cnt + 9, w.cnt + 10, d_counts + k, w.cnt + 1, st);
+            s = drain_same(C, st);
             continue;
         }
-        if (active[k]) {
+        // wetting phase connected to the outlet (its union-find and stamps
+        // only; tiles the last update left alone keep their tile-local parents)
+        s = fork.begin(st);
+        if (s == PMG_OK) {
+            s = shrink_marks_binary(g_w, mp_img, 2, shape, bc, pad, Bx.outlet, w.err, fork.side);
+            const int s1 = fork.end();
+            s = s == PMG_OK ? s1 : s;
+        }
+        if (active[k] && s == PMG_OK) {
             int32_t ext[6], ext_d[6];
             ext_of(bc, pad, ratios + 3 * k, ext);
             ext_of(bc, pad, ratios_dilate + 3 * k, ext_d);
@@ -870,21 +939,18 @@ extern "C" int pmg_drainage_ext(const uint8_t *pm_img, uint8_t *mp_img, const in
                                 Bx, w, st, ball_erode ? ball_erode[k] : -1.0, ball_dilate ? ball_dilate[k] : -1.0,
                                 De, KC, Te[(size_t)k], true, grow_er ? &g_er : nullptr, &g_nw, Sv, k, orange, drows);
         }
+        {
+            // (also after an error: the scratch below is freed in st's order)
+            const int s1 = fork.join(st);
+            s = s == PMG_OK ? s1 : s;
+        }
         if (s != PMG_OK)
             break;
-        // wetting phase connected to the outlet (its union-find and stamps
-        // only; tiles the last update left alone keep their tile-local
-        // parents), then the update on row words, which also brings the
-        // non-wetting phase's growing selection and the wetting phase's masks
-        // and tile flags up to date
-        s = shrink_marks_binary(g_w, mp_img, 2, shape, bc, pad, Bx.outlet, w.err, st);
-        if (s != PMG_OK)
-            break;
+        // the update on row words, which also brings the non-wetting phase's
+        // growing selection and the wetting phase's masks and tile flags up to date
         GrowSel *gn = g_nw.built ? &g_nw : nullptr;
-        s = drain_update_rows(mp_img, active[k] ? drows : nullptr, shape, g_w, Bx, gn, w.cnt + 8, w.cnt + 9, w.err, st,
+        s = drain_update_rows(mp_img, active[k] ? drows : nullptr, shape, g_w, Bx, gn, C, w.err, st,
                               active[k] ? orange : nullptr, !full_done);
-        if (s == PMG_OK)
-            s = drain_totals(!full_done, w.cnt + 8, w.cnt + 9, w.cnt + 10, d_counts + k, w.cnt + 1, st);
         if (s != PMG_OK)
             break;
         full_done = true;

@@ -88,7 +88,7 @@ int grow_marks_pair(GrowSel &a, const uint8_t *S, int k, const uint16_t *E, int 
                     int *err, cudaStream_t st);
 // ... and the inlet selection of a constrained by b (when *b_count > 0) as row
 // words; kept counts a's inlet-connected voxels, xr receives the x range of the
-// output's set (kRangeBig encoding).
+// output's set (kRangeBig encoding); both are zero before.
 int grow_pair_select(GrowSel &a, GrowSel &b, const unsigned long long *b_count, unsigned *out, const int64_t *shape,
                      int *err, cudaStream_t st, unsigned long long *kept, int *xr);
 // Selection of a set that only shrinks (the drainage's wetting phase): full
@@ -110,18 +110,24 @@ size_t shrink_sel_bytes(const int64_t *shape);
 void shrink_sel_init(ShrinkSel &g, void *mem, const int64_t *shape);
 int shrink_marks_binary(ShrinkSel &g, const uint8_t *img, int fgval, const int64_t *shape, const int32_t *bc,
                         const int32_t *pad, const int64_t *outlet_box, int *err, cudaStream_t st);
+// The counts of a drainage curve (device): cnt2 and cnt1 of one update, their
+// running totals tot and ones, the saturation numerator of the radius (sat), and
+// what the next radius's selection counts into (kept, xr), cleared with them by
+// the update's last block (ticket: its blocks done).
+struct DrainCounts {
+    unsigned long long *cnt2, *cnt1, *tot, *ones, *sat, *kept;
+    int *xr;
+    unsigned *ticket;
+};
 // The drainage update on row words: D the dilation (null: none), defined on
 // the voxel x range orange (device, [lo, hi] in whole blocks, null:
 // everything); full: every voxel and the reservoir slabs, the counts being all
 // voxels of value 2 in the own box and the voxels newly 1; otherwise only the
-// dilation's range, the counts being changes (drain_totals keeps the running
-// totals and clears them).  w's masks, words and tile flags are brought up to
-// date, and g_nw's when given.
+// dilation's range, the counts being changes.  w's masks, words and tile flags
+// are brought up to date, and g_nw's when given.
 int drain_update_rows(uint8_t *mp, const unsigned *D, const int64_t *shape, ShrinkSel &w, const Boxes &B, GrowSel *g_nw,
-                      unsigned long long *cnt2, unsigned long long *cnt1, int *err, cudaStream_t st, const int *orange,
-                      bool full);
-int drain_totals(bool full, unsigned long long *cnt2, unsigned long long *cnt1, unsigned long long *tot,
-                 unsigned long long *sat_out, unsigned long long *ones, cudaStream_t st);
+                      const DrainCounts &C, int *err, cudaStream_t st, const int *orange, bool full);
+int drain_same(const DrainCounts &C, cudaStream_t st); // a radius without change
 int check_err(int *err, cudaStream_t st);
 int check_volume(const int64_t *shape);
 
