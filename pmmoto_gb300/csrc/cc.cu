@@ -2128,7 +2128,7 @@ __global__ void k_grow_start(GrowWords W, int pieces)
     }
 }
 
-// The unions of a step, of one or two sets of the same grid (blockIdx.y): the
+// The unions of a step: the
 // touching pairs of a row piece (32 blocks) within the row and with the four
 // earlier neighbouring rows that have a changed block and an unconnected one.
 // A thread per piece and neighbouring row (and one for the pairs within the
@@ -2150,9 +2150,8 @@ struct RowSet {
 };
 constexpr int kGrowPieces = 32, kGrowThreads = 5 * kGrowPieces;
 
-__global__ void __launch_bounds__(kGrowThreads) k_grow_pairs(RowSet A, RowSet B, BGrid G, int nt2, int *err)
+__global__ void __launch_bounds__(kGrowThreads) k_grow_pairs(RowSet R, BGrid G, int nt2, int *err)
 {
-    const RowSet &R = blockIdx.y ? B : A;
     const GrowWords W = R.W;
     const int q = threadIdx.x / kGrowPieces, piece = blockIdx.x * kGrowPieces + threadIdx.x % kGrowPieces;
     const int row = (int)fdiv((unsigned)piece, G.qt), tk = piece - row * nt2;
@@ -2234,10 +2233,9 @@ __global__ void __launch_bounds__(kGrowThreads) k_grow_pairs(RowSet A, RowSet B,
 
 // The listed pairs united; the roots that a block of threads joins are mostly
 // the same few (CrossSet).
-__global__ void __launch_bounds__(256) k_grow_join(RowSet A, RowSet B, int *err)
+__global__ void __launch_bounds__(256) k_grow_join(RowSet R, int *err)
 {
     __shared__ CrossSet S;
-    const RowSet &R = blockIdx.y ? B : A;
     const int n = min(*R.count, R.cap);
     if ((int)(blockIdx.x * blockDim.x) >= n)
         return;
@@ -2328,25 +2326,23 @@ static int grow_masks(GrowSel &g, const Src &src, const int64_t *shape, const in
     return PMG_OK;
 }
 
-// Unions of one set, or of two in one launch (their pair counts are zero: the
-// selection of the last step or the build cleared them).
-static int grow_rows(GrowSel &a, GrowSel *b, const int64_t *shape, int *err, cudaStream_t st)
+// The step's unions (the pair count is zero: the selection of the last step or
+// the build cleared it).
+static int grow_rows(GrowSel &g, const int64_t *shape, int *err, cudaStream_t st)
 {
     const BGrid G = bgrid_of(shape);
     const int nt2 = (G.b2 + kT2 - 1) / kT2, pieces = row_pieces(G), cap = G.b0 * G.b1 * G.b2 / 2;
-    const RowSet A{a.P, words(a), a.pairs, a.npairs, cap}, B = b ? RowSet{b->P, words(*b), b->pairs, b->npairs, cap} : A;
-    const unsigned sets = b ? 2 : 1;
+    const RowSet R{g.P, words(g), g.pairs, g.npairs, cap};
     {
         const int ps__ = prof_begin("k_grow_pairs", st);
-        k_grow_pairs<<<dim3((unsigned)((pieces + kGrowPieces - 1) / kGrowPieces), sets), kGrowThreads, 0, st>>>(A, B, G,
-                                                                                                            nt2, err);
+        k_grow_pairs<<<(unsigned)((pieces + kGrowPieces - 1) / kGrowPieces), kGrowThreads, 0, st>>>(R, G, nt2, err);
         // the changed and the unconnected words (the words of pieces with pairs come on top)
-        prof_end(ps__, (double)pieces * 8 * sets, st);
+        prof_end(ps__, (double)pieces * 8, st);
     }
     PMG_CHECK_LAUNCH();
     {
         const int ps__ = prof_begin("k_grow_join", st);
-        k_grow_join<<<dim3((unsigned)grid_for(cap, 256, 152LL * 4), sets), 256, 0, st>>>(A, B, err);
+        k_grow_join<<<(unsigned)grid_for(cap, 256, 152LL * 4), 256, 0, st>>>(R, err);
         prof_end(ps__, 0.0, st);
     }
     PMG_CHECK_LAUNCH();
@@ -2363,7 +2359,7 @@ static int grow_step(GrowSel &g, const Src &src, const int64_t *shape, const int
         PMG_TRY(grow_build(g, src, shape, bc, pad, err, st));
     } else {
         PMG_TRY(grow_masks(g, src, shape, nullptr, err, st));
-        PMG_TRY(grow_rows(g, nullptr, shape, err, st));
+        PMG_TRY(grow_rows(g, shape, err, st));
         PMG_CUDA(cudaMemsetAsync(g.N, 0, piece_bytes(bgrid_of(shape)), st));
         PMG_CUDA(cudaMemsetAsync(g.npairs, 0, sizeof(int), st));
         if (any_periodic(bc)) {
@@ -2402,8 +2398,8 @@ static SrcErode erode_src(const uint16_t *E, int T, const int64_t *shape, const 
     return src;
 }
 
-// Marks by stamp: the roots of the blocks of one or two sets (blockIdx.y) with
-// a voxel in the box get this step's stamp, so that the marks of earlier steps
+// Marks by stamp: the roots of the set's blocks with a voxel in the box get this
+// step's stamp, so that the marks of earlier steps
 // need no clearing.
 struct StampSet {
     const uint8_t *M;
@@ -2412,9 +2408,8 @@ struct StampSet {
     uint8_t stamp;
 };
 
-__global__ void k_face_stamp(StampSet A, StampSet B, BGrid G, Box bx, int *err)
+__global__ void k_face_stamp(StampSet R, BGrid G, Box bx, int *err)
 {
-    const StampSet &R = blockIdx.y ? B : A;
     int lo[3], nbk[3];
     for (int d = 0; d < 3; d++) {
         lo[d] = (int)(bx.lo[d] >> 1);
@@ -2447,8 +2442,7 @@ static int next_stamp(uint8_t *mark, int &stamp, size_t nb, cudaStream_t st)
     return PMG_OK;
 }
 
-static int face_stamps(const int64_t *box, const int64_t *shape, StampSet A, const StampSet *B, int *err,
-                       cudaStream_t st)
+static int face_stamps(const int64_t *box, const int64_t *shape, StampSet R, int *err, cudaStream_t st)
 {
     if (!box || box[0] < 0)
         return PMG_OK;
@@ -2462,10 +2456,9 @@ static int face_stamps(const int64_t *box, const int64_t *shape, StampSet A, con
     if (b.size() <= 0)
         return PMG_OK;
     const int ps__ = prof_begin("k_face_stamp", st);
-    k_face_stamp<<<dim3((unsigned)grid_for(nbk, 128, 1LL << 30), B ? 2 : 1), 128, 0, st>>>(A, B ? *B : A,
-                                                                                         bgrid_of(shape), b, err);
+    k_face_stamp<<<(unsigned)grid_for(nbk, 128, 1LL << 30), 128, 0, st>>>(R, bgrid_of(shape), b, err);
     // per block meeting the box: mask, parent, root parent
-    prof_end(ps__, (double)nbk * 9 * (B ? 2 : 1), st);
+    prof_end(ps__, (double)nbk * 9, st);
     PMG_CHECK_LAUNCH();
     return PMG_OK;
 }
@@ -2744,40 +2737,33 @@ int step_lists_build(GrowSel &g, const uint8_t *S, const int64_t *shape, int nst
     return PMG_OK;
 }
 
-// Both growing selections of a drainage radius up to their inlet stamps: the
-// eroded space A (its step k from the precomputed lists when S is given, else
-// from the capped EDT E > T) and the non-wetting phase B (fgval in img).
-int grow_marks_pair(GrowSel &a, const uint8_t *S, int k, const uint16_t *E, int T, GrowSel &b, const uint8_t *img,
-                    int fgval, const int64_t *shape, const int32_t *bc, const int32_t *pad, const int64_t *inlet_box,
-                    int *err, cudaStream_t st)
+template <class Src>
+static int grow_marks(GrowSel &g, const Src &src, const int64_t *shape, const int32_t *bc, const int32_t *pad,
+                      const int *off, const int64_t *inlet_box, int *err, cudaStream_t st)
 {
     PMG_TRY(check_boxes(shape, inlet_box, nullptr));
-    const SrcStep step{S, k};
-    const SrcErode erode = erode_src(E, T, shape, bc);
-    const SrcImg phase{img, fgval};
-    const bool both = a.built && b.built;
-    const bool a_new = !a.built, b_new = !b.built;
-    if (a_new)
-        PMG_TRY(S ? grow_build(a, step, shape, bc, pad, err, st) : grow_build(a, erode, shape, bc, pad, err, st));
-    else
-        PMG_TRY(S ? grow_masks(a, step, shape, a.ev ? a.off + k : nullptr, err, st)
-                  : grow_masks(a, erode, shape, nullptr, err, st));
-    if (b_new)
-        PMG_TRY(grow_build(b, phase, shape, bc, pad, err, st));
-    else
-        PMG_TRY(grow_masks(b, phase, shape, nullptr, err, st));
-    if (both)
-        PMG_TRY(grow_rows(a, &b, shape, err, st));
-    else if (!a_new)
-        PMG_TRY(grow_rows(a, nullptr, shape, err, st));
-    else if (!b_new)
-        PMG_TRY(grow_rows(b, nullptr, shape, err, st));
+    if (!g.built) {
+        PMG_TRY(grow_build(g, src, shape, bc, pad, err, st));
+    } else {
+        PMG_TRY(grow_masks(g, src, shape, off, err, st));
+        PMG_TRY(grow_rows(g, shape, err, st));
+    }
     const BGrid G = bgrid_of(shape);
-    const size_t nb = (size_t)G.b0 * G.b1 * G.b2;
-    PMG_TRY(next_stamp(a.mark, a.stamp, nb, st));
-    PMG_TRY(next_stamp(b.mark, b.stamp, nb, st));
-    const StampSet B{b.M, b.P, b.mark, (uint8_t)b.stamp};
-    return face_stamps(inlet_box, shape, StampSet{a.M, a.P, a.mark, (uint8_t)a.stamp}, &B, err, st);
+    PMG_TRY(next_stamp(g.mark, g.stamp, (size_t)G.b0 * G.b1 * G.b2, st));
+    return face_stamps(inlet_box, shape, StampSet{g.M, g.P, g.mark, (uint8_t)g.stamp}, err, st);
+}
+
+int grow_marks_eroded(GrowSel &g, const uint8_t *S, int k, const uint16_t *E, int T, const int64_t *shape,
+                      const int32_t *bc, const int32_t *pad, const int64_t *inlet_box, int *err, cudaStream_t st)
+{
+    return S ? grow_marks(g, SrcStep{S, k}, shape, bc, pad, g.ev ? g.off + k : nullptr, inlet_box, err, st)
+             : grow_marks(g, erode_src(E, T, shape, bc), shape, bc, pad, nullptr, inlet_box, err, st);
+}
+
+int grow_marks_phase(GrowSel &g, const uint8_t *img, int fgval, const int64_t *shape, const int32_t *bc,
+                     const int32_t *pad, const int64_t *inlet_box, int *err, cudaStream_t st)
+{
+    return grow_marks(g, SrcImg{img, fgval}, shape, bc, pad, nullptr, inlet_box, err, st);
 }
 
 int grow_pair_select(GrowSel &a, GrowSel &b, const unsigned long long *b_count, unsigned *out, const int64_t *shape,
@@ -2899,7 +2885,7 @@ int shrink_marks_binary(ShrinkSel &g, const uint8_t *img, int fgval, const int64
     }
     g.built = true;
     PMG_TRY(next_stamp(g.mark, g.stamp, (size_t)G.b0 * G.b1 * G.b2, st));
-    return face_stamps(outlet_box, shape, StampSet{g.M, g.P, g.mark, (uint8_t)g.stamp}, nullptr, err, st);
+    return face_stamps(outlet_box, shape, StampSet{g.M, g.P, g.mark, (uint8_t)g.stamp}, err, st);
 }
 
 // ---- drainage update on row words -------------------------------------------------

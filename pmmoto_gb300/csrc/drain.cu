@@ -224,6 +224,54 @@ static int count_sync(const uint8_t *img, const int64_t *shape, const int64_t *b
     return PMG_OK;
 }
 
+// A second stream that takes work between begin (after what the first stream
+// holds) and end, which join makes the first stream wait for.
+struct Fork {
+    cudaStream_t side = nullptr;
+    cudaEvent_t from = nullptr, to = nullptr;
+    bool pending = false;
+    int open()
+    {
+        PMG_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+        PMG_CUDA(cudaEventCreateWithFlags(&from, cudaEventDisableTiming));
+        PMG_CUDA(cudaEventCreateWithFlags(&to, cudaEventDisableTiming));
+        return PMG_OK;
+    }
+    int begin(cudaStream_t st)
+    {
+        PMG_CUDA(cudaEventRecord(from, st));
+        PMG_CUDA(cudaStreamWaitEvent(side, from, 0));
+        return PMG_OK;
+    }
+    int end()
+    {
+        if (cudaEventRecord(to, side) != cudaSuccess) {
+            cudaStreamSynchronize(side); // (what it holds must not outlive its scratch)
+            set_error("drainage: event record failed");
+            return PMG_ECUDA;
+        }
+        pending = true;
+        return PMG_OK;
+    }
+    int join(cudaStream_t st)
+    {
+        if (pending)
+            PMG_CUDA(cudaStreamWaitEvent(st, to, 0));
+        pending = false;
+        return PMG_OK;
+    }
+    ~Fork()
+    {
+        // (work still queued is finished before the stream goes)
+        if (to)
+            cudaEventDestroy(to);
+        if (from)
+            cudaEventDestroy(from);
+        if (side)
+            cudaStreamDestroy(side);
+    }
+};
+
 // porosimetry.py:84-160 (mode="distance") into `out`.
 static int porosimetry_run(const uint8_t *pm, uint8_t *out, const int64_t *shape, const int32_t *bc,
                            const int32_t *pad, const int32_t *ext_e, const int32_t *ext_d, const float *res,
@@ -232,9 +280,10 @@ static int porosimetry_run(const uint8_t *pm, uint8_t *out, const int64_t *shape
                            const float *De = nullptr, const uint16_t *KC = nullptr, int Te = -1,
                            bool m1_counted = false, GrowSel *g_er = nullptr, GrowSel *g_nw = nullptr,
                            const uint8_t *Sv = nullptr, int step = -1, int *orange = nullptr,
-                           unsigned *rows_out = nullptr)
+                           unsigned *rows_out = nullptr, Fork *eroded = nullptr)
 {
-    // rows_out (a drainage): the result as row words; out is then scratch
+    // a drainage: rows_out, the result as row words (out is then scratch); eroded,
+    // where the eroded space's marks of this radius were made
     // m1_counted: w.cnt[1] already holds count(mp == 1) (the drainage update
     // counts it); the inlet selection counts its kept voxels into w.cnt[0], and
     // both come back with one copy
@@ -244,11 +293,12 @@ static int porosimetry_run(const uint8_t *pm, uint8_t *out, const int64_t *shape
     float *A, *B;
     morph_split(w, shape, bc, ext_e, E, A, B);
     uint8_t *cur = w.t1;
-    if (g_er && g_nw && (KC || Sv) && inlet && mp && m1_counted) {
+    if (eroded) {
         // both selections grow along the curve: one pass writes the eroded
         // inlet-connected space constrained by the inlet-connected
         // non-wetting phase (when that phase exists, counted in w.cnt[1])
-        PMG_TRY(grow_marks_pair(*g_er, Sv, step, KC, Te, *g_nw, mp, 1, shape, bc, pad, Bx.inlet, w.err, st));
+        PMG_TRY(grow_marks_phase(*g_nw, mp, 1, shape, bc, pad, Bx.inlet, w.err, st));
+        PMG_TRY(eroded->join(st));
         // the selection's x range (w.cnt[4]) limits the dilation to the planes
         // it can reach; the dilation's result range goes to orange.  Like the
         // kept count (w.cnt[0]) it is zero here (DrainCounts)
@@ -256,6 +306,7 @@ static int porosimetry_run(const uint8_t *pm, uint8_t *out, const int64_t *shape
         // the selection is written as row words (w.rows): the dilation's row
         // pass reads them directly (w.t2 receives bytes on other paths)
         PMG_TRY(grow_pair_select(*g_er, *g_nw, w.cnt + 1, w.rows, shape, w.err, st, w.cnt, xr));
+        PMG_TRY(eroded->begin(st)); // the next radius's marks may follow
         // the dilation reads the kept count (w.cnt[0]) on the device: no
         // dilation of an empty selection, and no host round trip per radius
         morph_split(w, shape, bc, ext_d, E, A, B);
@@ -388,54 +439,6 @@ __global__ void k_first_cover(const uint8_t *__restrict__ pm, const uint8_t *__r
         }
     }
 }
-
-// A second stream that takes work between begin (after what the first stream
-// holds) and end, which join makes the first stream wait for.
-struct Fork {
-    cudaStream_t side = nullptr;
-    cudaEvent_t from = nullptr, to = nullptr;
-    bool pending = false;
-    int open()
-    {
-        PMG_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-        PMG_CUDA(cudaEventCreateWithFlags(&from, cudaEventDisableTiming));
-        PMG_CUDA(cudaEventCreateWithFlags(&to, cudaEventDisableTiming));
-        return PMG_OK;
-    }
-    int begin(cudaStream_t st)
-    {
-        PMG_CUDA(cudaEventRecord(from, st));
-        PMG_CUDA(cudaStreamWaitEvent(side, from, 0));
-        return PMG_OK;
-    }
-    int end()
-    {
-        if (cudaEventRecord(to, side) != cudaSuccess) {
-            cudaStreamSynchronize(side); // (what it holds must not outlive its scratch)
-            set_error("drainage: event record failed");
-            return PMG_ECUDA;
-        }
-        pending = true;
-        return PMG_OK;
-    }
-    int join(cudaStream_t st)
-    {
-        if (pending)
-            PMG_CUDA(cudaStreamWaitEvent(st, to, 0));
-        pending = false;
-        return PMG_OK;
-    }
-    ~Fork()
-    {
-        // (work still queued is finished before the stream goes)
-        if (to)
-            cudaEventDestroy(to);
-        if (from)
-            cudaEventDestroy(from);
-        if (side)
-            cudaStreamDestroy(side);
-    }
-};
 
 static int ext_of(const int32_t *bc, const int32_t *pad, const int32_t *ratio, int32_t *ext)
 {
@@ -909,10 +912,27 @@ extern "C" int pmg_drainage_ext(const uint8_t *pm_img, uint8_t *mp_img, const in
                 : PMG_ECUDA;
     // The wetting phase's union-find depends on the last update alone: it runs on
     // a stream of its own beside the selection and the dilation, whose kernels
-    // leave much of the chip waiting on dependent loads.
-    Fork fork;
+    // leave much of the chip waiting on dependent loads.  The eroded space does
+    // not depend on the phases at all: a third stream prepares the next radius's
+    // while this one's selection is dilated.
+    Fork fork, eroded;
     if (s == PMG_OK)
         s = fork.open();
+    if (s == PMG_OK && grow_er)
+        s = eroded.open();
+    auto next_eroded = [&](int k) -> int {
+        while (k < n_radii && !active[k])
+            k++;
+        if (!grow_er || k == n_radii)
+            return PMG_OK;
+        const int s1 = grow_marks_eroded(g_er, Sv, k, KC, Te[(size_t)k], shape, bc, pad, Bx.inlet, w.err, eroded.side);
+        const int s2 = eroded.end();
+        return s1 != PMG_OK ? s1 : s2;
+    };
+    if (s == PMG_OK && grow_er)
+        s = eroded.begin(st);
+    if (s == PMG_OK)
+        s = next_eroded(0);
     bool full_done = false;
     for (int k = 0; k < n_radii && s == PMG_OK; k++) {
         C.sat = d_counts + k;
@@ -937,7 +957,10 @@ extern "C" int pmg_drainage_ext(const uint8_t *pm_img, uint8_t *mp_img, const in
             s = porosimetry_run(pm_img, morph, shape, bc, pad, ext, ext_d, res, radii[k], 1, radii_dilate[k], 1, 1,
                                 mp_img,
                                 Bx, w, st, ball_erode ? ball_erode[k] : -1.0, ball_dilate ? ball_dilate[k] : -1.0,
-                                De, KC, Te[(size_t)k], true, grow_er ? &g_er : nullptr, &g_nw, Sv, k, orange, drows);
+                                De, KC, Te[(size_t)k], true, grow_er ? &g_er : nullptr, &g_nw, Sv, k, orange, drows,
+                                grow_er ? &eroded : nullptr);
+            if (s == PMG_OK)
+                s = next_eroded(k + 1);
         }
         {
             // (also after an error: the scratch below is freed in st's order)
@@ -956,6 +979,11 @@ extern "C" int pmg_drainage_ext(const uint8_t *pm_img, uint8_t *mp_img, const in
         full_done = true;
         if (gn)
             gn->pending = true;
+    }
+    {
+        // (scratch is freed in st's order)
+        const int s1 = eroded.join(st);
+        s = s == PMG_OK ? s1 : s;
     }
     // union-find iteration caps are checked once per curve: the status word
     // is only ever set, never cleared, during the sweep

@@ -150,9 +150,14 @@ __device__ __forceinline__ long long src_index(const ExtAxis &a, long long x, bo
 {
     const long long p = x - a.ext_lo; // coordinate in the padded image
     if (a.periodic) {
-        long long q = (x - (a.own_lo + a.ext_lo)) % a.own_len;
+        long long q = x - (a.own_lo + a.ext_lo);
+        // (mostly within a period on either side: a 64-bit division otherwise)
+        if (q < -a.own_len || q >= 2LL * a.own_len)
+            q %= a.own_len;
         if (q < 0)
             q += a.own_len;
+        else if (q >= a.own_len)
+            q -= a.own_len;
         return q + a.own_lo;
     }
     if ((a.wall_lo && p == 0) || (a.wall_hi && p == a.S - 1))

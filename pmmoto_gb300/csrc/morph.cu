@@ -133,11 +133,6 @@ int morph_run(const uint8_t *img, uint8_t *out, const int64_t *shape, const int3
               const unsigned long long *gate, const int *xr, int *orange, const unsigned *rows,
               unsigned *rows_out)
 {
-    // orange: on the paths below that ignore xr the whole result is written
-    if (orange) {
-        k_set_int2<<<1, 32, 0, st>>>(orange, 0, (int)shape[0] - 1);
-        PMG_CHECK_LAUNCH();
-    }
     const ExtGeo G = ext_geo(shape, bc, pad, ext);
     int64_t X[3];
     for (int d = 0; d < 3; d++) {
@@ -188,12 +183,17 @@ int morph_run(const uint8_t *img, uint8_t *out, const int64_t *shape, const int3
     const bool cap = T != INT_MIN && cap_path_ok(res, X, T);
     const bool any_per = G.ax[0].periodic || G.ax[1].periodic || G.ax[2].periodic;
     // The capped pipeline's row pass reads the image (or its row words) itself;
-    // it needs a binary image for an erosion (an int of B's end says so).
+    // it needs a binary image for an erosion (an int of E, unused there, says so).
     if (cap && dilate && !any_per) {
         unsigned *direct = rows_out && cap_rows_out(X, T, me) ? rows_out : nullptr;
         PMG_TRY(morph_cap_run(img, G, (uint16_t *)A, (uint16_t *)B, X, T, me, st, nullptr, nullptr, gate, xr, orange,
                               rows, direct));
         return rows_out && !direct ? bytes_to_rows(out, rows_out, shape, st) : PMG_OK;
+    }
+    // orange: the paths below ignore xr and write the whole result
+    if (orange) {
+        k_set_int2<<<1, 32, 0, st>>>(orange, 0, (int)shape[0] - 1);
+        PMG_CHECK_LAUNCH();
     }
     if (rows_out) {
         // the paths below write bytes
@@ -224,7 +224,7 @@ int morph_run(const uint8_t *img, uint8_t *out, const int64_t *shape, const int3
 
     if (cap) {
         int nonbin = 0;
-        int *flag = dilate ? nullptr : (int *)(B + total) - 1;
+        int *flag = dilate ? nullptr : (int *)E;
         PMG_TRY(morph_cap_run(img, G, (uint16_t *)A, (uint16_t *)B, X, T, me, st, flag, &nonbin));
         if (!nonbin)
             return PMG_OK;

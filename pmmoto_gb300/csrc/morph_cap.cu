@@ -67,17 +67,27 @@ struct SeedRange {
 // ---- pass A: rows -------------------------------------------------------------
 // The seeds of a dilation are the nonzero voxels of the extended image off the
 // wall planes, those of an erosion its zeros and the wall planes.  Rows come
-// from the image, periodic axes reading the own region modulo its length, or
-// (dilations without periodic axes) from row words (b1, nt2: block rows and
-// pieces of a row).
+// from the image's nonzero voxels as bits (in memory order; periodic axes read
+// the own region modulo its length), or (dilations without periodic axes) from
+// row words (b1, nt2: block rows and pieces of a row).
 struct RowSrc {
-    const uint8_t *img;
     ExtGeo G;
     int dilate;
-    int *nonbinary; // set when a voxel above 1 is met (null: not asked)
+    const unsigned *bits;
+    long long last; // last word of bits
     const unsigned *rows;
     int b1, nt2;
+    FastDiv q1; // division by the extended rows of a plane
+    FastDiv qp; // and by the words of a row of k_seed_bits
 };
+
+// minimum of both 16-bit halves
+__device__ __forceinline__ uint32_t pair_min(uint32_t a, uint32_t b)
+{
+    uint32_t r;
+    asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
 
 // bits 0-15 of v at the even positions
 __device__ __forceinline__ unsigned spread16(unsigned v)
@@ -88,182 +98,219 @@ __device__ __forceinline__ unsigned spread16(unsigned v)
     return (v | (v << 1)) & 0x55555555u;
 }
 
-// Bytes k .. k + 3 of a row of n (k < n; zero past its end) at img + off, img
-// holding total bytes: two aligned words where those lie inside the image.
-__device__ __forceinline__ unsigned row_bytes(const uint8_t *img, long long off, int k, int n, long long total)
+// bits of the nonzero bytes of v
+__device__ __forceinline__ unsigned nonzero4(unsigned v)
 {
-    const unsigned left = n - k >= 4 ? 0xffffffffu : (1u << (8 * (n - k))) - 1u;
-    const uint8_t *p = img + off + k;
-    const int mis = (int)((uintptr_t)p & 3u);
-    if (off + k >= mis && off + k - mis + 8 <= total) {
-        const unsigned *q = reinterpret_cast<const unsigned *>(p - mis);
-        return (mis ? __funnelshift_r(q[0], q[1], 8 * mis) : q[0]) & left;
-    }
-    unsigned v = 0;
-    for (int e = 0; e < 4 && k + e < n; e++)
-        v |= (unsigned)p[e] << (8 * e);
-    return v;
+    const unsigned m = (((v & 0x7f7f7f7fu) + 0x7f7f7f7fu) | v) >> 7 & 0x01010101u;
+    return (m * 0x204081u) >> 21 & 0xfu;
 }
 
-// Bits p .. p + 31 of a bit array.
-__device__ __forceinline__ unsigned bits_at(const uint32_t *w, int p)
+// Nonzero voxels of an image as bits in memory order; *nonbinary is set when a
+// voxel above 1 is met (null: not asked).  A lane takes 16 bytes; bound by the
+// image read.
+__global__ void __launch_bounds__(256) k_image_bits(const uint8_t *__restrict__ img, unsigned *__restrict__ bits,
+                                                    long long n, int *nonbinary)
 {
-    return __funnelshift_r(w[p >> 5], w[(p >> 5) + 1], p & 31);
+    const int lane = threadIdx.x & 31;
+    const bool aligned = !((uintptr_t)img & 15);
+    unsigned above = 0;
+    for (long long base = (blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31)) * 16; base < n;
+         base += (long long)gridDim.x * blockDim.x * 16) {
+        const long long at = base + 16 * lane;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (aligned && at + 16 <= n) {
+            v = *reinterpret_cast<const uint4 *>(img + at);
+        } else {
+            unsigned w[4] = {0u, 0u, 0u, 0u};
+            for (int e = 0; e < 16 && at + e < n; e++)
+                w[e >> 2] |= (unsigned)img[at + e] << (8 * (e & 3));
+            v = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        above |= (v.x | v.y | v.z | v.w) & 0xfefefefeu;
+        unsigned w = nonzero4(v.x) | nonzero4(v.y) << 4 | nonzero4(v.z) << 8 | nonzero4(v.w) << 12;
+        w |= __shfl_down_sync(0xffffffffu, w, 1) << 16;
+        if (!(lane & 1) && at < n)
+            bits[at >> 5] = w;
+    }
+    if (nonbinary && __any_sync(0xffffffffu, above) && lane == 0)
+        *nonbinary = 1;
+}
+
+// Word c of the seeds of row r of the extended volume.
+template <bool WORDS>
+__device__ __forceinline__ unsigned seed_word(const RowSrc &rs, int r, int c, int X1, int X2)
+{
+    const int i = (int)fdiv((unsigned)r, rs.q1), j = r - i * X1;
+    const ExtAxis &a2 = rs.G.ax[2];
+    bool wrow = false;
+    const int s0 = (int)src_index(rs.G.ax[0], i, wrow), s1 = (int)src_index(rs.G.ax[1], j, wrow);
+    unsigned w = 0; // a wall row: no voxel
+    if (!wrow) {
+        if constexpr (WORDS) {
+            // 64 voxels per piece: even positions in one word, odd ones in the next
+            const uint2 eo = *reinterpret_cast<const uint2 *>(
+                rs.rows + ((long long)((i >> 1) * rs.b1 + (j >> 1)) * rs.nt2 + (c >> 1)) * 8 + ((i & 1) * 2 + (j & 1)) * 2);
+            const int sh = (c & 1) * 16;
+            w = spread16((eo.x >> sh) & 0xffffu) | (spread16((eo.y >> sh) & 0xffffu) << 1);
+        } else {
+            const long long row = ((long long)s0 * rs.G.ax[1].S + s1) * a2.S;
+            // bits from position p of the row (past its end: the next rows')
+            auto bits_at = [&](int p) {
+                const long long b = row + p;
+                return __funnelshift_r(rs.bits[b >> 5], rs.bits[min((b >> 5) + 1, rs.last)], (unsigned)b & 31u);
+            };
+            if (!a2.periodic) {
+                w = bits_at(32 * c);
+            } else {
+                int q = 32 * c - (a2.own_lo + a2.ext_lo);
+                if (q < -a2.own_len || q >= a2.own_len)
+                    q %= a2.own_len;
+                q += q < 0 ? a2.own_len : 0;
+                for (int f = 0; f < 32;) {
+                    const int take = min(32 - f, a2.own_len - q);
+                    w |= (bits_at(a2.own_lo + q) & (0xffffffffu >> (32 - take))) << f;
+                    f += take;
+                    q = 0;
+                }
+            }
+        }
+        if (!a2.periodic) {
+            // the wall planes at the row's ends
+            if (a2.wall_lo && c == 0)
+                w &= ~1u;
+            if (a2.wall_hi && c == (X2 - 1) >> 5)
+                w &= ~(1u << ((X2 - 1) & 31));
+        }
+    }
+    // seeds: the voxels, or (erosion) the others
+    const unsigned in = X2 - 32 * c >= 32 ? 0xffffffffu : (1u << (X2 - 32 * c)) - 1u;
+    return (rs.dilate ? w : ~w) & in;
+}
+
+// Squared distances, at most big, of two adjacent positions (the first at bit sh
+// of wc, sh even) to the nearest set bits of their row's words wp, wc, wn: bit
+// 31 - t of l holds the positions x - t and x + t.
+__device__ __forceinline__ uint32_t pair_heights(uint32_t wp, uint32_t wc, uint32_t wn, int sh, uint32_t bigp)
+{
+    const uint32_t l0 = __funnelshift_l(wp, wc, 31 - sh) | __brev(__funnelshift_r(wc, wn, sh)),
+                   l1 = __funnelshift_l(wp, wc, 30 - sh) | __brev(__funnelshift_r(wc, wn, sh + 1));
+    const uint32_t d0 = __clz(l0), d1 = __clz(l1); // 32: none near, above every W
+    return pair_min(d0 * d0 + d1 * d1 * 65536u, bigp);
+}
+
+// The seeds of the extended volume as bits: nw words per row between a zero word
+// before and two behind (pitch nw + 3).  One thread per word.
+template <bool WORDS>
+__global__ void __launch_bounds__(256) k_seed_bits(RowSrc rs, unsigned *__restrict__ eb, int rows, int X2, int W,
+                                                   const unsigned long long *__restrict__ gate,
+                                                   const int *__restrict__ xr)
+{
+    if (gate && *gate == 0)
+        return;
+    const int X1 = (int)rs.G.ax[1].X, nw = (X2 + 31) >> 5, pitch = nw + 3;
+    SeedRange sr{0, 0x7fffffff, 0, 0};
+    if (xr)
+        sr.load(xr, rows / X1, W);
+    const int r0 = xr ? max(sr.hlo, 0) * X1 : 0, r1 = xr ? (int)min((long long)rows, (long long)(sr.hhi + 1) * X1) : rows;
+    // (words of a volume: below 2^32)
+    const long long n = (long long)max(r1 - r0, 0) * pitch;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+        const int rr = (int)fdiv((unsigned)q, rs.qp), c = (int)((unsigned)q - (unsigned)rr * pitch) - 1, r = r0 + rr;
+        eb[(long long)r * pitch + c + 1] = c >= 0 && c < nw ? seed_word<WORDS>(rs, r, c, X1, X2) : 0u;
+    }
 }
 
 // Only distances d <= W = floor(sqrt T) <= 31 give values below T + 1, so a
-// voxel needs the seeds within 31 positions on either side: the row's seeds are
-// first gathered as bit words in shared memory (from the image's bytes, four
-// per lane, wrapped on a periodic axis; or from row words with even and odd
-// positions interleaved), with an empty word on either side, then every lane
-// finds the nearest seeds of two adjacent voxels in the three words around them
-// with one count of leading / trailing zeros each way and stores both at once
-// (rows of even pitch; the column that an odd row gains holds some height, read
-// by no one).
-// Bound by the 2 bytes written per voxel and the bit counts.  From per-block
-// mask bytes with a ballot per 32 voxels and one voxel a lane the drainage's
-// dilations took 0.16 ms at 512^3, now 0.11 ms; with a pass of its own for the
-// extended copy (60 us) 256 x 192 x 320 voxels took 98 us.
+// voxel needs the seeds within 31 positions on either side: the row's seed words
+// are gathered in shared memory, with an empty word on either side, then every
+// lane finds the nearest seeds of two adjacent voxels in the three words around
+// them and stores both at once (rows of even pitch; the column that an odd row
+// gains holds some height, read by no one).  For the wide probes only: the
+// others' next pass takes the heights from the words itself.
 template <bool WORDS>
-__global__ void __launch_bounds__(256) k_cap_rows(RowSrc rs, uint16_t *__restrict__ KA, long long rows, int X2, int T,
+__global__ void __launch_bounds__(256) k_cap_rows(RowSrc rs, uint16_t *__restrict__ KA, int rows, int X2, int T,
                                                   int W, const unsigned long long *__restrict__ gate,
                                                   const int *__restrict__ xr, unsigned long long *units)
 {
     if (gate && *gate == 0)
         return; // empty seed set: the last pass writes the result alone
-    const ExtAxis &a2 = rs.G.ax[2];
-    const int X1 = (int)rs.G.ax[1].X, S2 = (int)a2.S;
+    const int X1 = (int)rs.G.ax[1].X;
     SeedRange sr{0, 0x7fffffff, 0, 0};
     if (xr)
-        sr.load(xr, (int)(rows / X1), W);
+        sr.load(xr, rows / X1, W);
     extern __shared__ uint32_t s_words[];
-    const int lane = threadIdx.x & 31;
-    const int nw = (X2 + 31) >> 5, nown = WORDS ? 0 : ((S2 + 127) >> 7) * 4 + 1;
-    uint32_t *zw = s_words + (threadIdx.x >> 5) * (nw + 3 + nown) + 1; // zw[-1], zw[nw] and zw[nw + 1] stay 0
-    [[maybe_unused]] uint32_t *own = zw + nw + 2;                      // the unextended row, a zero word at its end
+    const int lane = threadIdx.x & 31, nw = (X2 + 31) >> 5;
+    uint32_t *zw = s_words + (threadIdx.x >> 5) * (nw + 3) + 1; // zw[-1], zw[nw] and zw[nw + 1] stay 0
     if (lane == 0) {
         zw[-1] = 0u;
         zw[nw] = 0u;
         zw[nw + 1] = 0u;
-        if constexpr (!WORDS)
-            own[nown - 1] = 0u;
     }
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    const int big = T + 1, P2 = (X2 + 1) & ~1;
+    const int P2 = (X2 + 1) & ~1;
+    const uint32_t bigp = (uint32_t)(T + 1) * 0x10001u;
     // with a seed range, only the rows of its planes
     const int r0 = xr ? max(sr.hlo, 0) * X1 : 0;
-    const int r1 = xr ? (int)min(rows, (long long)(sr.hhi + 1) * X1) : (int)rows;
+    const int r1 = xr ? (int)min((long long)rows, (long long)(sr.hhi + 1) * X1) : rows;
     if (units && blockIdx.x == 0 && threadIdx.x == 0 && r1 > r0)
         atomicAdd(units, (unsigned long long)((long long)(r1 - r0) * X2));
     for (int r = r0 + warp; r < r1; r += nwarps) {
-        const int i = r / X1, j = r - i * X1;
-        bool wrow = false;
-        const long long s0 = src_index(rs.G.ax[0], i, wrow), s1 = src_index(rs.G.ax[1], j, wrow);
-        if (wrow) {
-            // a wall row: no voxel
-            for (int c = lane; c < nw; c += 32)
-                zw[c] = 0u;
-        } else if constexpr (WORDS) {
-            // 64 voxels per piece: even positions in one word, odd ones in the next
-            const unsigned *p = rs.rows + ((long long)((i >> 1) * rs.b1 + (j >> 1)) * rs.nt2) * 8 +
-                                ((i & 1) * 2 + (j & 1)) * 2;
-            for (int c = lane; c < nw; c += 32) {
-                const uint2 eo = *reinterpret_cast<const uint2 *>(p + (c >> 1) * 8);
-                const int sh = (c & 1) * 16;
-                zw[c] = spread16((eo.x >> sh) & 0xffffu) | (spread16((eo.y >> sh) & 0xffffu) << 1);
-            }
-        } else {
-            const long long off = (s0 * rs.G.ax[1].S + s1) * S2, total = rs.G.ax[0].S * rs.G.ax[1].S * S2;
-            unsigned above = 0;
-            for (int b = 0; b < S2; b += 128) {
-                const int k = b + 4 * lane;
-                const unsigned v = k < S2 ? row_bytes(rs.img, off, k, S2, total) : 0u;
-                above |= v & 0xfefefefeu;
-                // bit e: byte e is not zero
-                const unsigned m = (((v & 0x7f7f7f7fu) + 0x7f7f7f7fu) | v) >> 7 & 0x01010101u;
-                unsigned w = ((m * 0x204081u) >> 21 & 0xfu) << (4 * (lane & 7));
-                w |= __shfl_xor_sync(0xffffffffu, w, 1);
-                w |= __shfl_xor_sync(0xffffffffu, w, 2);
-                w |= __shfl_xor_sync(0xffffffffu, w, 4);
-                if ((lane & 7) == 0)
-                    own[(b >> 5) + (lane >> 3)] = w;
-            }
-            if (above && rs.nonbinary)
-                *rs.nonbinary = 1;
-            __syncwarp();
-            for (int c = lane; c < nw; c += 32) {
-                unsigned w = 0;
-                if (!a2.periodic) {
-                    w = own[c];
-                } else {
-                    int q = (32 * c - (a2.own_lo + a2.ext_lo)) % a2.own_len;
-                    q += q < 0 ? a2.own_len : 0;
-                    for (int f = 0; f < 32;) {
-                        const int take = min(32 - f, a2.own_len - q);
-                        const unsigned v = bits_at(own, a2.own_lo + q) & (0xffffffffu >> (32 - take));
-                        w |= v << f;
-                        f += take;
-                        q = 0;
-                    }
-                }
-                zw[c] = w;
-            }
-        }
+        for (int c = lane; c < nw; c += 32)
+            zw[c] = seed_word<WORDS>(rs, r, c, X1, X2);
         __syncwarp();
-        if (!wrow && lane == 0 && !a2.periodic) {
-            // the wall planes at the row's ends
-            if (a2.wall_lo)
-                zw[0] &= ~1u;
-            if (a2.wall_hi)
-                zw[(X2 - 1) >> 5] &= ~(1u << ((X2 - 1) & 31));
-        }
-        __syncwarp();
-        if (!WORDS) {
-            // seeds: the row's voxels, or (erosion) the others
-            for (int c = lane; c < nw; c += 32) {
-                const unsigned in = X2 - 32 * c >= 32 ? 0xffffffffu : (1u << (X2 - 32 * c)) - 1u;
-                zw[c] = (rs.dilate ? zw[c] : ~zw[c]) & in;
-            }
-            __syncwarp();
-        }
         uint16_t *dst = KA + (long long)r * P2;
         // lane l on voxels 64 c + 2 l and the next one: word 2 c + l / 16
         const int hw = lane >> 4, sh = (2 * lane) & 31;
         for (int c = 0; 64 * c < X2; c++) {
             const int x = 64 * c + 2 * lane;
-            const uint32_t wp = zw[2 * c + hw - 1], wc = zw[2 * c + hw], wn = zw[2 * c + hw + 1];
-            // bit t of R: position x + t; bit 31 - t of L: position x - t
-            const uint32_t R0 = __funnelshift_r(wc, wn, sh), R1 = __funnelshift_r(wc, wn, sh + 1);
-            const uint32_t L0 = __funnelshift_l(wp, wc, 31 - sh), L1 = __funnelshift_l(wp, wc, 30 - sh);
-            const int d0 = min(__clz(L0), __clz(__brev(R0))), d1 = min(__clz(L1), __clz(__brev(R1)));
-            const uint32_t k0 = d0 <= W ? d0 * d0 : big, k1 = d1 <= W ? d1 * d1 : big;
+            const uint32_t v = pair_heights(zw[2 * c + hw - 1], zw[2 * c + hw], zw[2 * c + hw + 1], sh, bigp);
             if (x < X2)
-                *reinterpret_cast<uint32_t *>(dst + x) = k0 | (k1 << 16);
+                *reinterpret_cast<uint32_t *>(dst + x) = v;
         }
         __syncwarp();
     }
 }
 
-// The row pass; *nonbinary (erosions) is read back from flag.
-static int launch_cap_rows(const uint8_t *img, const ExtGeo &EG, int dilate, const unsigned *seeds, uint16_t *KA,
-                           const CapGeo &G, int T, int W, int *flag, int *nonbinary, cudaStream_t st,
-                           const unsigned long long *gate, const int *xr)
+// The row pass: heights to KA, or (eb) the seeds' words there.  bits: scratch of a
+// word per 32 voxels of the image; *nonbinary (erosions) is read back
+// from flag.
+static int launch_cap_rows(const uint8_t *img, const ExtGeo &EG, int dilate, const unsigned *seeds, unsigned *bits,
+                           uint16_t *KA, bool eb, const CapGeo &G, int T, int W, int *flag, int *nonbinary,
+                           cudaStream_t st, const unsigned long long *gate, const int *xr)
 {
-    RowSrc rs{img, EG, dilate, flag, seeds, (int)((G.X1 + 1) / 2), (int)(((G.X2 + 1) / 2 + 31) / 32)};
-    const int block = 256, words = (G.X2 + 31) / 32 + 3 + (seeds ? 0 : ((int)EG.ax[2].S + 127) / 128 * 4 + 1);
-    const size_t smem = (size_t)(block / 32) * words * sizeof(uint32_t);
-    const long long rows = (long long)G.X0 * G.X1;
-    const unsigned grid = grid_for(rows * 32, block, 152LL * 16);
+    const long long n = EG.ax[0].S * EG.ax[1].S * EG.ax[2].S;
+    RowSrc rs{EG, dilate, bits, (n - 1) >> 5, seeds, (G.X1 + 1) / 2, ((G.X2 + 1) / 2 + 31) / 32,
+              fastdiv_of((unsigned)G.X1), fastdiv_of((unsigned)((G.X2 + 31) / 32 + 3))};
+    const int block = 256, rows = G.X0 * G.X1;
     if (flag)
         PMG_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
-    const int ps__ = prof_begin("k_cap_rows", st);
-    if (seeds)
-        k_cap_rows<true><<<grid, block, smem, st>>>(rs, KA, rows, G.X2, T, W, gate, xr, prof_units(kUnitsCapRows));
-    else
-        k_cap_rows<false><<<grid, block, smem, st>>>(rs, KA, rows, G.X2, T, W, gate, xr, prof_units(kUnitsCapRows));
-    // 1 B read (1/8 B from row words) + 2 B written per voxel
-    prof_end_units(ps__, kUnitsCapRows, seeds ? 2.125 : 3.0, st);
+    if (!seeds) {
+        const int ps__ = prof_begin("k_image_bits", st);
+        k_image_bits<<<grid_for((n + 15) / 16, block, 152LL * 32), block, 0, st>>>(img, bits, n, flag);
+        prof_end(ps__, (double)n * 1.125, st);
+        PMG_CHECK_LAUNCH();
+    }
+    if (eb) {
+        const int pitch = (G.X2 + 31) / 32 + 3;
+        const unsigned grid = grid_for((long long)rows * pitch, block, 152LL * 32);
+        const int ps__ = prof_begin("k_seed_bits", st);
+        if (seeds)
+            k_seed_bits<true><<<grid, block, 0, st>>>(rs, (unsigned *)KA, rows, G.X2, W, gate, xr);
+        else
+            k_seed_bits<false><<<grid, block, 0, st>>>(rs, (unsigned *)KA, rows, G.X2, W, gate, xr);
+        prof_end(ps__, (double)rows * pitch * 8, st);
+    } else {
+        const size_t smem = (size_t)(block / 32) * ((G.X2 + 31) / 32 + 3) * sizeof(uint32_t);
+        const unsigned grid = grid_for((long long)rows * 32, block, 152LL * 16);
+        const int ps__ = prof_begin("k_cap_rows", st);
+        if (seeds)
+            k_cap_rows<true><<<grid, block, smem, st>>>(rs, KA, rows, G.X2, T, W, gate, xr, prof_units(kUnitsCapRows));
+        else
+            k_cap_rows<false><<<grid, block, smem, st>>>(rs, KA, rows, G.X2, T, W, gate, xr, prof_units(kUnitsCapRows));
+        // 1/8 B read + 2 B written per voxel
+        prof_end_units(ps__, kUnitsCapRows, 2.125, st);
+    }
     PMG_CHECK_LAUNCH();
     if (flag) {
         PMG_CUDA(cudaMemcpyAsync(nonbinary, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -425,37 +472,16 @@ constexpr int kPairMaxW = 20;
 // heights loaded ahead: fewer for the wide windows, whose rings hold more
 __host__ __device__ constexpr int pair_ahead(int W) { return W <= 12 ? 8 : 4; }
 
-// Lines of a pass on pairs: AX = 1, np pairs over (x0 in [0, X0), x2 / 2 from
-// kp0) along axis 1; AX = 0, pairs over (x1 in [j0, j0 + nj), x2 / 2 ...) along
-// axis 0.  Word offset of line pair li.
-template <int AX>
-__device__ __forceinline__ long long pair_base(const CapGeo &G, long long li, int np)
-{
-    const long long q = li / np;
-    return (AX == 1 ? q * G.X1 : G.j0 + q) * (G.P2 >> 1) + G.kp0() + (li - q * np);
-}
-
-template <int AX, int W>
+// Along axis 0 (pairs over x1 in [j0, j0 + nj), x2 / 2 from kp0).
+template <int W>
 __global__ void __launch_bounds__(256) k_cap_mid_pair(const uint16_t *__restrict__ KA, uint16_t *__restrict__ KB,
-                                                      CapGeo G, int T, const unsigned long long *__restrict__ gate,
-                                                      const int *__restrict__ xr, int seglen,
-                                                      unsigned long long *units)
+                                                      CapGeo G, int T, int seglen, unsigned long long *units)
 {
     constexpr int R = 2 * W + 1 + pair_ahead(W);
-    if (gate && *gate == 0)
-        return;
-    SeedRange sr{0, 0x7fffffff, 0, 0};
-    if (xr)
-        sr.load(xr, G.X0, W);
-    const int np = G.np();
-    const long long nlines = (long long)(AX == 1 ? G.X0 : G.nj) * np;
-    const long long st = AX == 1 ? (long long)(G.P2 >> 1) : (long long)G.X1 * (G.P2 >> 1);
-    const int n = AX == 1 ? G.X1 : G.X0;
+    const int np = G.np(), n = G.X0;
+    const long long span = (long long)G.nj * np, st = (long long)G.X1 * (G.P2 >> 1);
     const int nseg = (n + seglen - 1) / seglen;
-    const long long l0 = AX == 1 && xr ? (long long)max(sr.hlo, 0) * np : 0;
-    const long long l1 = AX == 1 && xr ? min(nlines, (long long)(sr.hhi + 1) * np) : nlines;
-    const long long span = l1 > l0 ? l1 - l0 : 0;
-    if (units && blockIdx.x == 0 && threadIdx.x == 0 && span)
+    if (units && blockIdx.x == 0 && threadIdx.x == 0)
         atomicAdd(units, (unsigned long long)(span * 2 * n));
     const uint32_t bigp = (uint32_t)(T + 1) * 0x10001u;
     const uint32_t *in0 = (const uint32_t *)KA;
@@ -463,7 +489,8 @@ __global__ void __launch_bounds__(256) k_cap_mid_pair(const uint16_t *__restrict
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < span * nseg;
          g += (long long)gridDim.x * blockDim.x) {
         const int seg = (int)(g / span);
-        const long long base = pair_base<AX>(G, l0 + (g - (long long)seg * span), np);
+        const long long li = g - (long long)seg * span, q = li / np;
+        const long long base = (G.j0 + q) * (G.P2 >> 1) + G.kp0() + (li - q * np);
         const uint32_t *in = in0 + base;
         uint32_t *out = out0 + base;
         const int a = seg * seglen, b = min(n, a + seglen);
@@ -488,6 +515,78 @@ __global__ void __launch_bounds__(256) k_cap_mid_pair(const uint16_t *__restrict
                     out[y * st] = m;
                 const int yn = y + W + 1 + pair_ahead(W);
                 win[u] = y < b && yn < n ? __ldg(in + yn * st) : bigp;
+            }
+        }
+    }
+}
+
+// Passes A and B in one for small W: the heights of a position are taken from
+// the three seed words around it (k_seed_bits) where the ring needs them, so
+// neither written nor read.  The words of the next height are loaded a step
+// ahead; a warp's 64 voxels share two to three words of a row.
+// Bound by instruction issue.  As two passes (heights written, then read) this
+// took 108 + 105 us a radius of the 512^3 drainage, and 55 + 23 us on 256 x 192 x
+// 320 voxels.
+template <int W>
+__global__ void __launch_bounds__(256) k_cap_rows_mid(const unsigned *__restrict__ eb, uint16_t *__restrict__ KB,
+                                                      CapGeo G, int T, const unsigned long long *__restrict__ gate,
+                                                      const int *__restrict__ xr, int seglen,
+                                                      unsigned long long *units)
+{
+    constexpr int R = 2 * W + 1;
+    if (gate && *gate == 0)
+        return;
+    SeedRange sr{0, 0x7fffffff, 0, 0};
+    if (xr)
+        sr.load(xr, G.X0, W);
+    const int np = G.np(), n = G.X1, pitch = ((G.X2 + 31) >> 5) + 3;
+    const long long nlines = (long long)G.X0 * np, st = G.P2 >> 1;
+    const int nseg = (n + seglen - 1) / seglen;
+    const long long l0 = xr ? (long long)max(sr.hlo, 0) * np : 0;
+    const long long l1 = xr ? min(nlines, (long long)(sr.hhi + 1) * np) : nlines;
+    const long long span = l1 > l0 ? l1 - l0 : 0;
+    if (units && blockIdx.x == 0 && threadIdx.x == 0 && span)
+        atomicAdd(units, (unsigned long long)(span * 2 * n));
+    const uint32_t bigp = (uint32_t)(T + 1) * 0x10001u;
+    for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < span * nseg;
+         g += (long long)gridDim.x * blockDim.x) {
+        const int seg = (int)(g / span);
+        const long long li = l0 + (g - (long long)seg * span), q = li / np;
+        const int kp = G.kp0() + (int)(li - q * np), x = 2 * kp, sh = x & 31;
+        const unsigned *in = eb + q * n * pitch + (x >> 5);
+        uint32_t *out = (uint32_t *)KB + q * n * st + kp;
+        const int a = seg * seglen, b = min(n, a + seglen);
+        uint32_t w[3];
+        auto fetch = [&](int y) {
+            const bool ok = y >= 0 && y < n;
+            const unsigned *p = in + (long long)y * pitch;
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+                w[c] = ok ? __ldg(p + c) : 0u;
+        };
+        uint32_t win[R];
+#pragma unroll
+        for (int s = 0; s < R; s++) {
+            fetch(a - W + s);
+            win[s] = pair_heights(w[0], w[1], w[2], sh, bigp);
+        }
+        fetch(a + W + 1);
+        for (int y0 = a; y0 < b; y0 += R) {
+#pragma unroll
+            for (int u = 0; u < R; u++) {
+                const int y = y0 + u;
+                uint32_t m = win[(u + W) % R];
+#pragma unroll
+                for (int d = 1; d <= W; d++) {
+                    const uint32_t dd = (uint32_t)(d * d) * 0x10001u;
+                    m = __viaddmin_u16x2(win[(u + W - d) % R], dd, m);
+                    m = __viaddmin_u16x2(win[(u + W + d) % R], dd, m);
+                }
+                if (y < b)
+                    out[y * st] = m;
+                // the slot of y - W takes y + W + 1
+                win[u] = pair_heights(w[0], w[1], w[2], sh, bigp);
+                fetch(y < b ? y + W + 2 : n);
             }
         }
     }
@@ -756,9 +855,17 @@ __global__ void __launch_bounds__(256) k_cap_last_pair(const uint16_t *__restric
     }
 }
 
-// Segment length of the pair kernels: whole groups of the register ring,
-// about four per segment.
-static int pair_seglen(int W) { return 4 * (2 * W + 1 + pair_ahead(W)); }
+// Segment length of the pair kernels on `lines` lines of n: whole groups of the
+// register ring of R, four per segment, as each starts with a ring to fill, and
+// fewer (two at least) where that leaves less than about six warps per scheduler
+// (200^3 voxels: 29 + 26 us for the two passes with four, 24 + 21 us with two).
+static int pair_seglen(int R, int n, long long lines)
+{
+    int g = 4;
+    while (g > 2 && lines * ((n + g * R - 1) / (g * R)) < 152LL * 768)
+        g--;
+    return g * R;
+}
 
 // Calls f with std::integral_constant<int, w> for 0 <= w <= kPairMaxW.
 template <int W, class F>
@@ -773,22 +880,35 @@ static void with_w(int w, F &&f)
     f(std::integral_constant<int, W>{});
 }
 
-template <int AX, int W>
-static void launch_mid_pair_w(const uint16_t *in, uint16_t *out, const CapGeo &G, int T, cudaStream_t st,
-                              const unsigned long long *gate, const int *xr, unsigned long long *units)
+static void launch_mid_pair(const uint16_t *in, uint16_t *out, const CapGeo &G, int T, int W, cudaStream_t st,
+                            unsigned long long *units)
 {
-    const int n = AX == 1 ? G.X1 : G.X0;
-    const int seglen = pair_seglen(W);
-    const long long lines = (long long)(AX == 1 ? G.X0 : G.nj) * G.np();
-    const long long work = lines * ((n + seglen - 1) / seglen);
-    k_cap_mid_pair<AX, W><<<grid_for(work, 256, 1LL << 30), 256, 0, st>>>(in, out, G, T, gate, xr, seglen, units);
+    with_w<0>(W, [&](auto c) {
+        constexpr int w = decltype(c)::value;
+        const int seglen = pair_seglen(2 * w + 1 + pair_ahead(w), G.X0, (long long)G.nj * G.np());
+        const long long work = (long long)G.nj * G.np() * ((G.X0 + seglen - 1) / seglen);
+        k_cap_mid_pair<w><<<grid_for(work, 256, 1LL << 30), 256, 0, st>>>(in, out, G, T, seglen, units);
+    });
 }
 
-template <int AX>
-static void launch_mid_pair(const uint16_t *in, uint16_t *out, const CapGeo &G, int T, int W, cudaStream_t st,
-                            const unsigned long long *gate, const int *xr, unsigned long long *units)
+// The two passes in one (words: the seeds' words in KA) where the window fits the
+// registers and the words fit the heights' scratch.
+static bool rows_mid_ok(const CapGeo &G, int W) { return W <= kPairMaxW && G.X2 >= 4; }
+
+static int launch_rows_mid(const uint16_t *KA, uint16_t *KB, const CapGeo &G, int T, int W, cudaStream_t st,
+                           const unsigned long long *gate, const int *xr)
 {
-    with_w<0>(W, [&](auto c) { launch_mid_pair_w<AX, decltype(c)::value>(in, out, G, T, st, gate, xr, units); });
+    const int ps__ = prof_begin("k_cap_rows_mid", st);
+    with_w<0>(W, [&](auto c) {
+        constexpr int w = decltype(c)::value;
+        const int seglen = pair_seglen(2 * w + 1, G.X1, (long long)G.X0 * G.np());
+        const long long work = (long long)G.X0 * G.np() * ((G.X1 + seglen - 1) / seglen);
+        k_cap_rows_mid<w><<<grid_for(work, 256, 1LL << 30), 256, 0, st>>>((const unsigned *)KA, KB, G, T, gate, xr, seglen,
+                                                                         prof_units(kUnitsCapMid));
+    });
+    prof_end_units(ps__, kUnitsCapMid, 2.125, st); // 1/8 B read + 2 B written per voxel
+    PMG_CHECK_LAUNCH();
+    return PMG_OK;
 }
 
 template <int W>
@@ -796,8 +916,8 @@ static void launch_last_pair_w(const uint16_t *KB, const CapGeo &G, int T, const
                                const unsigned long long *gate, const int *xr, int *orange, unsigned *rows_out,
                                unsigned long long *units)
 {
-    const int seglen = pair_seglen(W);
     const long long np = rows_out ? (G.np() + 31) & ~31 : G.np();
+    const int seglen = pair_seglen(2 * W + 1 + pair_ahead(W), G.X0, G.nj * np);
     const long long work = G.nj * np * ((G.X0 + seglen - 1) / seglen);
     const unsigned grid = grid_for(work, 256, 1LL << 30);
     if (rows_out)
@@ -831,10 +951,11 @@ static int launch_cap_mid(const uint16_t *in, uint16_t *out, const CapGeo &G, in
     // axis-1 passes count their voxels (k_cap_mid); the axis-0 pass of the
     // erosion EDT (k_cap_mid0) is booked from the host
     unsigned long long *units = AX == 1 ? prof_units(kUnitsCapMid) : nullptr;
-    if (pair_ok(G, W)) {
-        launch_mid_pair<AX>(in, out, G, T, W, st, gate, xr, units);
-        return PMG_OK;
-    }
+    if constexpr (AX == 0) // (along axis 1: k_cap_rows_mid)
+        if (pair_ok(G, W)) {
+            launch_mid_pair(in, out, G, T, W, st, units);
+            return PMG_OK;
+        }
     if (2 * W + 2 <= 16)
         k_cap_mid<AX, 16><<<grid, 128, 0, st>>>(in, out, G, T, W, gate, xr, nseg, units);
     else if (2 * W + 2 <= 32)
@@ -880,10 +1001,13 @@ int morph_cap_run(const uint8_t *img, const ExtGeo &EG, uint16_t *KA, uint16_t *
     G.k0 = me.e2;
     G.nk = (int)me.o2;
     G.P2 = G.PO = (G.X2 + 1) & ~1;
-    PMG_TRY(launch_cap_rows(img, EG, me.dilate, seeds, KA, G, T, W, flag, nonbinary, st, gate, xr));
+    const bool fused = rows_mid_ok(G, W);
+    PMG_TRY(launch_cap_rows(img, EG, me.dilate, seeds, (unsigned *)KB, KA, fused, G, T, W, flag, nonbinary, st, gate, xr));
     if (flag && *nonbinary)
         return PMG_OK;
-    {
+    if (fused) {
+        PMG_TRY(launch_rows_mid(KA, KB, G, T, W, st, gate, xr));
+    } else {
         const long long lines = (long long)G.X0 * G.nk;
         const int ps__ = prof_begin("k_cap_mid", st);
         PMG_TRY(launch_cap_mid<1>(KA, KB, G, T, W, lines, st, gate, xr));
@@ -926,10 +1050,14 @@ int edt_cap_run(const uint8_t *img, const ExtGeo &EG, uint16_t *KA, uint16_t *KB
     G.nk = G.X2;
     G.P2 = G.PO = (G.X2 + 1) & ~1;
     const long long vox = (long long)G.X0 * G.X1 * G.X2;
-    PMG_TRY(launch_cap_rows(img, EG, 0, nullptr, KA, G, T, W, flag, nonbinary, st, nullptr, nullptr));
+    const bool fused = rows_mid_ok(G, W);
+    PMG_TRY(launch_cap_rows(img, EG, 0, nullptr, (unsigned *)KB, KA, fused, G, T, W, flag, nonbinary, st, nullptr,
+                            nullptr));
     if (*nonbinary)
         return PMG_OK;
-    {
+    if (fused) {
+        PMG_TRY(launch_rows_mid(KA, KB, G, T, W, st, nullptr, nullptr));
+    } else {
         const long long lines = (long long)G.X0 * G.nk;
         const int ps__ = prof_begin("k_cap_mid", st);
         PMG_TRY(launch_cap_mid<1>(KA, KB, G, T, W, lines, st));

@@ -80,13 +80,14 @@ void grow_sel_init(GrowSel &g, void *mem, const int64_t *shape);
 int select_grow_binary(GrowSel &g, const uint8_t *img, int fgval, void *out, const int64_t *shape,
                        const int32_t *bc, const int32_t *pad, const int64_t *inlet_box, const int64_t *outlet_box,
                        int mode, int *err, cudaStream_t st, unsigned long long *kept = nullptr);
-// Both growing selections of a drainage radius up to their inlet stamps (the
-// eroded space a: step k of S when S is given, else E > T; the non-wetting
-// phase b: fgval in img), no axis being periodic.
-int grow_marks_pair(GrowSel &a, const uint8_t *S, int k, const uint16_t *E, int T, GrowSel &b, const uint8_t *img,
-                    int fgval, const int64_t *shape, const int32_t *bc, const int32_t *pad, const int64_t *inlet_box,
-                    int *err, cudaStream_t st);
-// ... and the inlet selection of a constrained by b (when *b_count > 0) as row
+// A growing selection of a drainage radius up to its inlet stamps, no axis being
+// periodic: the eroded space (step k of S when S is given, else E > T), the
+// non-wetting phase (fgval in img).
+int grow_marks_eroded(GrowSel &g, const uint8_t *S, int k, const uint16_t *E, int T, const int64_t *shape,
+                      const int32_t *bc, const int32_t *pad, const int64_t *inlet_box, int *err, cudaStream_t st);
+int grow_marks_phase(GrowSel &g, const uint8_t *img, int fgval, const int64_t *shape, const int32_t *bc,
+                     const int32_t *pad, const int64_t *inlet_box, int *err, cudaStream_t st);
+// The inlet selection of a constrained by b (when *b_count > 0) as row
 // words; kept counts a's inlet-connected voxels, xr receives the x range of the
 // output's set (kRangeBig encoding); both are zero before.
 int grow_pair_select(GrowSel &a, GrowSel &b, const unsigned long long *b_count, unsigned *out, const int64_t *shape,
