@@ -216,30 +216,49 @@ struct TileId {
 
 // Phase 1 on voxels (equal nonzero neighbours touch).  A voxel equal to the one
 // above it leaves its other earlier neighbours to that one: it is adjacent to
-// all of them.
+// all of them.  A warp takes four rows, whose loads overlap; the pairs of a row
+// with one of its neighbouring rows are then united by one lane (lane 4 u + q:
+// row u, neighbour q).
+// A tile is a chain of dependent steps between barriers: with a thread per voxel
+// (1024 of them, two tiles in flight on an SM) this took 244 us on 257 x 200 x 323
+// voxels, now 174 us.
+constexpr int kCcTileThreads = 256, kCcRows = kTile / kCcTileThreads;
+
 template <typename T>
-__global__ void __launch_bounds__(kTile) k_cc_tile(const T *__restrict__ img, int *__restrict__ P, Vol3 V)
+__global__ void __launch_bounds__(kCcTileThreads) k_cc_tile(const T *__restrict__ img, int *__restrict__ P, Vol3 V)
 {
     __shared__ T sv[kTile];
     __shared__ int L[kTile];
     __shared__ unsigned s_cz[kT0 * kT1];
     const TileId D;
-    const int t = threadIdx.x, r = t / kT2, lane = t % kT2, a = r / kT1, b = r % kT1;
-    const int i = D.ti * kT0 + a, j = D.tj * kT1 + b, k = D.tk * kT2 + lane;
-    const bool inside = i < V.s0 && j < V.s1 && k < V.s2;
-    const long long g = ((long long)i * V.s1 + j) * V.s2 + k;
-    const T v = inside ? img[g] : (T)0;
-    sv[t] = v;
-    const T vp = __shfl_up_sync(0xffffffffu, v, 1);
-    const unsigned cz = __ballot_sync(0xffffffffu, lane > 0 && v != 0 && v == vp);
-    const int head = run_head(cz, lane);
-    L[t] = v != 0 ? r * kT2 + head : -1;
-    if (lane == 0)
-        s_cz[r] = cz;
+    const int w = threadIdx.x / kT2, lane = threadIdx.x % kT2, k = D.tk * kT2 + lane;
+    T v[kCcRows];
+    unsigned cz[kCcRows];
+    long long g[kCcRows]; // -1: outside
+#pragma unroll
+    for (int u = 0; u < kCcRows; u++) {
+        const int r = w * kCcRows + u, i = D.ti * kT0 + r / kT1, j = D.tj * kT1 + r % kT1;
+        const bool inside = i < V.s0 && j < V.s1 && k < V.s2;
+        g[u] = inside ? ((long long)i * V.s1 + j) * V.s2 + k : -1;
+        v[u] = inside ? img[g[u]] : (T)0;
+    }
+#pragma unroll
+    for (int u = 0; u < kCcRows; u++) {
+        const int r = w * kCcRows + u;
+        sv[r * kT2 + lane] = v[u];
+        const T vp = __shfl_up_sync(0xffffffffu, v[u], 1);
+        cz[u] = __ballot_sync(0xffffffffu, lane > 0 && v[u] != 0 && v[u] == vp);
+        L[r * kT2 + lane] = v[u] != 0 ? r * kT2 + run_head(cz[u], lane) : -1;
+        if (lane == 0)
+            s_cz[r] = cz[u];
+    }
     __syncthreads();
-    if (__any_sync(0xffffffffu, v != 0)) {
-        // pairs as bits 3 q + dz + 1
-        unsigned todo = 0;
+    unsigned em = 0, e0 = 0, ep = 0; // of this lane's pair of rows
+#pragma unroll
+    for (int u = 0; u < kCcRows; u++) {
+        const int r = w * kCcRows + u, a = r / kT1, b = r % kT1;
+        if (!__any_sync(0xffffffffu, v[u] != 0))
+            continue;
         bool centre = false;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
@@ -248,34 +267,50 @@ __global__ void __launch_bounds__(kTile) k_cc_tile(const T *__restrict__ img, in
             const int rn = r + row_d0(q) * kT1 + row_d1(q);
             const T n0 = sv[rn * kT2 + lane], nm = __shfl_up_sync(0xffffffffu, n0, 1),
                     np = __shfl_down_sync(0xffffffffu, n0, 1);
-            const bool on = v != 0 && !centre;
-            unsigned E0 = __ballot_sync(0xffffffffu, on && n0 == v),
-                     Em = __ballot_sync(0xffffffffu, on && lane > 0 && nm == v),
-                     Ep = __ballot_sync(0xffffffffu, on && lane < 31 && np == v);
+            const bool on = v[u] != 0 && !centre;
+            const unsigned E0 = __ballot_sync(0xffffffffu, on && n0 == v[u]),
+                           Em = __ballot_sync(0xffffffffu, on && lane > 0 && nm == v[u]),
+                           Ep = __ballot_sync(0xffffffffu, on && lane < 31 && np == v[u]);
             if (q == 0)
                 centre = (E0 >> lane) & 1u;
-            row_reduce(cz, s_cz[rn], Em, E0, Ep);
-            todo |= (((Em >> lane) & 1u) | (((E0 >> lane) & 1u) << 1) | (((Ep >> lane) & 1u) << 2)) << (3 * q);
+            if (lane == 4 * u + q) {
+                em = Em;
+                e0 = E0;
+                ep = Ep;
+            }
         }
-        while (todo) {
-            const int e = __ffs(todo) - 1, q = e / 3, dz = e - 3 * q - 1;
-            todo &= todo - 1;
-            const int rn = r + row_d0(q) * kT1 + row_d1(q);
-            sunite(L, r * kT2 + head, rn * kT2 + run_head(s_cz[rn], lane + dz));
+    }
+    if (em | e0 | ep) {
+        const int q = lane & 3, r = w * kCcRows + (lane >> 2), rn = r + row_d0(q) * kT1 + row_d1(q);
+        const unsigned ca = s_cz[r], cb = s_cz[rn];
+        row_reduce(ca, cb, em, e0, ep);
+        while (em | e0 | ep) {
+            const int dz = e0 ? 0 : em ? -1 : 1;
+            const unsigned e = e0 ? e0 : em ? em : ep;
+            const int c = __ffs(e) - 1;
+            const unsigned bit = e & (0u - e);
+            e0 &= ~(dz == 0 ? bit : 0u);
+            em &= ~(dz < 0 ? bit : 0u);
+            ep &= ~(dz > 0 ? bit : 0u);
+            sunite(L, r * kT2 + run_head(ca, c), rn * kT2 + run_head(cb, c + dz));
         }
     }
     __syncthreads();
-    int root = -1;
-    if (v != 0 && head == lane)
-        root = sfind(L, t);
-    root = __shfl_sync(0xffffffffu, root, head);
-    if (inside) {
-        int out = -1;
-        if (v != 0) {
-            const int ra = root / (kT1 * kT2), rb = (root / kT2) % kT1, rc = root % kT2;
-            out = (int)(((long long)(D.ti * kT0 + ra) * V.s1 + D.tj * kT1 + rb) * V.s2 + D.tk * kT2 + rc);
+#pragma unroll
+    for (int u = 0; u < kCcRows; u++) {
+        const int r = w * kCcRows + u, head = run_head(cz[u], lane);
+        int root = -1;
+        if (v[u] != 0 && head == lane)
+            root = sfind(L, r * kT2 + lane);
+        root = __shfl_sync(0xffffffffu, root, head);
+        if (g[u] >= 0) {
+            int out = -1;
+            if (v[u] != 0) {
+                const int ra = root / (kT1 * kT2), rb = (root / kT2) % kT1, rc = root % kT2;
+                out = (int)(((long long)(D.ti * kT0 + ra) * V.s1 + D.tj * kT1 + rb) * V.s2 + D.tk * kT2 + rc);
+            }
+            P[g[u]] = out;
         }
-        P[g] = out;
     }
 }
 
@@ -602,7 +637,7 @@ static int uf_build(const T *img, int *P, const int64_t *shape, const int32_t *b
                      (unsigned)((shape[0] + kT0 - 1) / kT0));
     {
         const int ps__ = prof_begin("k_cc_tile", st);
-        k_cc_tile<T><<<tiles, kTile, 0, st>>>(img, P, V);
+        k_cc_tile<T><<<tiles, kCcTileThreads, 0, st>>>(img, P, V);
         prof_end(ps__, (double)n * (sizeof(T) + 4), st);
     }
     PMG_CHECK_LAUNCH();
