@@ -2268,10 +2268,12 @@ __global__ void __launch_bounds__(kGrowThreads) k_grow_pairs(RowSet R, BGrid G, 
 
 // The listed pairs united; the roots that a block of threads joins are mostly
 // the same few (CrossSet).
-__global__ void __launch_bounds__(256) k_grow_join(RowSet R, int *err)
+__global__ void __launch_bounds__(256) k_grow_join(RowSet R, int *err, unsigned long long *units)
 {
     __shared__ CrossSet S;
     const int n = min(*R.count, R.cap);
+    if (units && blockIdx.x == 0 && threadIdx.x == 0)
+        atomicAdd(units, (unsigned long long)n);
     if ((int)(blockIdx.x * blockDim.x) >= n)
         return;
     S.init();
@@ -2377,8 +2379,9 @@ static int grow_rows(GrowSel &g, const int64_t *shape, int *err, cudaStream_t st
     PMG_CHECK_LAUNCH();
     {
         const int ps__ = prof_begin("k_grow_join", st);
-        k_grow_join<<<(unsigned)grid_for(cap, 256, 152LL * 4), 256, 0, st>>>(R, err);
-        prof_end(ps__, 0.0, st);
+        k_grow_join<<<(unsigned)grid_for(cap, 256, 152LL * 4), 256, 0, st>>>(R, err, prof_units(kUnitsGrowJoin));
+        // per pair: its entry, both blocks' parents and a root's
+        prof_end_units(ps__, kUnitsGrowJoin, 8 + 3 * 4, st);
     }
     PMG_CHECK_LAUNCH();
     return PMG_OK;

@@ -53,7 +53,7 @@ void prof_end(int slot, double bytes, cudaStream_t st);
 // bytes per unit for the profile.
 constexpr int kUnitSlots = 16;
 constexpr int kUnitsCapRows = 0, kUnitsCapMid = 1, kUnitsCapLast = 2, kUnitsDrainUpdate = 3;
-constexpr int kUnitsGrowApply = 7;
+constexpr int kUnitsGrowApply = 7, kUnitsGrowJoin = 4;
 unsigned long long *prof_units(int id);
 void prof_end_units(int slot, int id, double bytes_per_unit, cudaStream_t st);
 

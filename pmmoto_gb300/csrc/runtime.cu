@@ -83,7 +83,7 @@ static const TuneSpec g_tune_spec[kTuneKnobs] = {
     {"edt.pair_seg", 256, 32, 8192},
     {"edt.pair_ctas", 32, 1, 256},
     {"edt.rows_ctas", 16, 1, 256},
-    {"cc.cross_fused", 0, 0, 1},        // block labelling: one fused cross-tile pass (1) or two (0)
+    {"cc.cross_fused", 0, 0, 1},        // (no effect: knob of a former cross-tile phase)
     {"edt.path", 0, 0, 2},              // envelope passes: lattice / scan (0), exact stream (1), float envelope (2)
     {"edt.fallback", 96, 0, 8193},      // (no effect)
     {"edt.fallback_rows", 2048, 0, 8193}, // (no effect)
