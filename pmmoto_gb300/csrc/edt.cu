@@ -517,8 +517,11 @@ __device__ __forceinline__ void evaluate(Stack &S, const L &line, int nwords, fl
 }
 
 __global__ void k_envelope(const float *__restrict__ fin, float *__restrict__ fout, Lines Ls, float res,
-                           pmg_axis_cfg cfg, int num_hull, int form, MorphEpi me, int redo)
+                           pmg_axis_cfg cfg, int num_hull, int form, MorphEpi me, int redo,
+                           const int *__restrict__ wide)
 {
+    if (wide && *wide < kWideSamples)
+        return; // (the scan has the pass)
     const long long nlines = Ls.count();
     extern __shared__ uint32_t smem_bm[];
     const float aniso = fmul(res, res);
@@ -699,29 +702,35 @@ __device__ __forceinline__ void stage_ends(float *se, const T *__restrict__ fin,
     }
 }
 
-// Flagged lines of any voxel size (flag bit 1: the whole line): a block takes 32
-// adjacent lines (unflagged ones idle), the lanes of warp 0 their low ends or
+// Flagged lines of any voxel size (flag bit 1: the whole line): a block takes
+// `width` adjacent lines (unflagged ones idle), the lanes of warp 0 their low ends or
 // the whole line and those of warp 1 their high ends, two chains that overlap.
 // Both ends of the lines are staged in shared memory first, because the zero
 // searches, hulls, pushes and the sweep read them again and again in dependent
 // steps.
-// Bound by the latency of those steps: with one lane for both ends a periodic
-// 341 x 298 x 125 field took 0.80 ms here.
+// Bound by the latency of those steps, and by the lanes of a warp popping
+// different numbers of parabolas: with one lane for both ends a periodic 341 x
+// 298 x 125 field took 0.80 ms here, now 0.57 ms.  A warp of 32 lines waits for
+// the slowest at every push, so few lines are spread over more warps: eight
+// to a warp where that leaves each scheduler a handful of warps at most.
 constexpr int kEndBlock = 64;
 
 __global__ void __launch_bounds__(kEndBlock) k_envelope_ends(const float *__restrict__ fin, float *__restrict__ fout,
                                                              Lines Ls, float res, pmg_axis_cfg cfg, int num_hull,
-                                                             int form, MorphEpi me, const uint8_t *__restrict__ flag)
+                                                             int form, MorphEpi me, const uint8_t *__restrict__ flag,
+                                                             int width, const int *__restrict__ wide)
 {
+    if (wide && *wide >= kWideSamples)
+        return;
     extern __shared__ uint32_t smem_bm[];
     __shared__ float s_ends[2 * kEndWin * 33];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    // tiles of 32 lines that are adjacent in memory (along the second axis)
-    const int tiles = (Ls.nb2 + 31) / 32;
+    // tiles of lines that are adjacent in memory (along the second axis)
+    const int tiles = (Ls.nb2 + width - 1) / width;
     const long long ntiles = (long long)Ls.nb1 * tiles;
     for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const int ra = (int)(t / tiles), kb = (int)(t - (long long)ra * tiles) * 32;
-        const int lines = min(32, Ls.nb2 - kb);
+        const int ra = (int)(t / tiles), kb = (int)(t - (long long)ra * tiles) * width;
+        const int lines = min(width, Ls.nb2 - kb);
         const long long l0 = (long long)ra * Ls.nb2 + kb;
         const int fl = lane < lines ? flag[l0 + lane] : 0;
         if (!__any_sync(0xffffffffu, fl)) // the same for both warps
@@ -921,14 +930,15 @@ int launch_ends_heights(const float *fin, float *fout, const Lines &Ls, float re
 }
 
 int launch_ends_float(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
-                      int num_hull, int form, const MorphEpi &me, const uint8_t *flag, cudaStream_t st)
+                      int num_hull, int form, const MorphEpi &me, const uint8_t *flag, const int *wide, cudaStream_t st)
 {
     const int n = (int)(Ls.ax == 0 ? Ls.s0 : Ls.ax == 1 ? Ls.s1 : Ls.s2);
     const size_t smem = (size_t)((n + 31) / 32) * kEndBlock * 4;
-    const long long tiles = (long long)Ls.nb1 * ((Ls.nb2 + 31) / 32);
+    const int width = (long long)Ls.nb1 * ((Ls.nb2 + 31) / 32) * 2 <= 152LL * 4 * 4 ? 8 : 32;
+    const long long tiles = (long long)Ls.nb1 * ((Ls.nb2 + width - 1) / width);
     const int ps__ = prof_begin("k_envelope_ends", st);
     k_envelope_ends<<<grid_for(tiles, 1, 152LL * 64), kEndBlock, smem, st>>>(
-        fin, fout, Ls, res, cfg, num_hull, form, me, flag);
+        fin, fout, Ls, res, cfg, num_hull, form, me, flag, width, wide);
     prof_end(ps__, 0.0, st);
     PMG_CHECK_LAUNCH();
     return PMG_OK;
@@ -983,15 +993,33 @@ int launch_envelope(const float *fin, float *fout, const Lines &Ls, float res,
         PMG_CUDA(cudaFuncSetAttribute(k_envelope, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
     const int path = tune_value(kTuneEdtPath);
-    // the outward scan; a caller's flag buffer that does not hold one byte per
-    // line (lines of a few voxels) leaves the pass to the float envelope
-    if (path == 0 && n <= kScanMaxLine && (!flag_buf || Ls.count() <= flag_cap * (long long)sizeof(int))) {
+    // The outward scan; a caller's flag buffer that does not hold one byte per
+    // line (and the probe's count; lines of a few voxels) leaves the pass to the
+    // float envelope.  Periodic lines of wide pores are mostly replayed at their
+    // ends after the scan, which the envelope alone does faster: voxel sizes
+    // that are no power of two, whose near-ties are many, take it at once
+    // (400 x 300 x 300 pack, voxels of 2.25: 6.4 ms, the envelope 4.0 ms), the
+    // others by a probe on the device (pack, voxels 2 x 1 x 1: 6.5 and 3.9 ms;
+    // 300 x 400 x 425 field of narrow pores: 2.3 and 3.0 ms).
+    const size_t flag_bytes = ((size_t)Ls.count() + 7) / 4 * 4; // (then the count)
+    if (path == 0 && n <= kScanMaxLine && (!cfg.periodic || window_path_ok(res, n)) &&
+        (!flag_buf || flag_bytes + sizeof(int) <= (size_t)flag_cap * sizeof(int))) {
         uint8_t *flag = (uint8_t *)flag_buf;
         if (!flag_buf)
-            PMG_TRY(scratch_alloc((void **)&flag, (size_t)Ls.count(), st));
-        int s = launch_scan(fin, fout, Ls, res, cfg, form, me, vcap, flag, st);
+            PMG_TRY(scratch_alloc((void **)&flag, flag_bytes + sizeof(int), st));
+        int *wide = cfg.periodic ? (int *)(flag + flag_bytes) : nullptr;
+        int s = wide ? launch_pore_probe(fin, Ls, res, wide, st) : PMG_OK;
         if (s == PMG_OK)
-            s = launch_ends_float(fin, fout, Ls, res, cfg, num_hull, form, me, flag, st);
+            s = launch_scan(fin, fout, Ls, res, cfg, form, me, vcap, flag, wide, st);
+        if (s == PMG_OK)
+            s = launch_ends_float(fin, fout, Ls, res, cfg, num_hull, form, me, flag, wide, st);
+        if (s == PMG_OK && wide) {
+            const int ps__ = prof_begin("k_envelope[wide]", st);
+            k_envelope<<<grid_for(Ls.count(), block, 1LL << 30), block, smem, st>>>(fin, fout, Ls, res, cfg, num_hull, form,
+                                                                                   me, 0, wide);
+            prof_end(ps__, 0.0, st);
+            s = cudaGetLastError() == cudaSuccess ? PMG_OK : PMG_ECUDA;
+        }
         const int s2 = flag_buf ? PMG_OK : scratch_free(flag, st);
         return s != PMG_OK ? s : s2;
     }
@@ -1004,7 +1032,7 @@ int launch_envelope(const float *fin, float *fout, const Lines &Ls, float res,
     {
         const int ps__ = prof_begin(redo ? "k_envelope_redo" : "k_envelope", st);
         k_envelope<<<grid_for(Ls.count(), block, redo ? 152LL * 8 : 1LL << 30), block, smem, st>>>(
-            fin, fout, Ls, res, cfg, num_hull, form, me, redo);
+            fin, fout, Ls, res, cfg, num_hull, form, me, redo, nullptr);
         prof_end(ps__, redo ? 0.0 : (double)Ls.count() * n * 4 + (form == PMG_EDT_MORPH ? (double)Ls.count() * me.o2 : (double)Ls.count() * n * 4), st);
     }
     PMG_CHECK_LAUNCH();

@@ -213,11 +213,15 @@ int launch_ends_counts(const uint16_t *fin, float *fout, const Lines &Ls, float 
 int launch_ends_heights(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
                         int num_hull, int form, const uint16_t *flag, cudaStream_t st);
 int launch_ends_float(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
-                      int num_hull, int form, const MorphEpi &me, const uint8_t *flag, cudaStream_t st);
+                      int num_hull, int form, const MorphEpi &me, const uint8_t *flag, const int *wide,
+                      cudaStream_t st);
 // The outward scan (edt_scan.cu), lines of at most kScanMaxLine voxels; vcap:
 // values above it only matter as "above it".
 int launch_scan(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg, int form,
-                const MorphEpi &me, float vcap, uint8_t *flag, cudaStream_t st);
+                const MorphEpi &me, float vcap, uint8_t *flag, const int *wide, cudaStream_t st);
+// Wide pores: at least kWideSamples of the probe's samples (device count *wide).
+constexpr int kWideSamples = 256;
+int launch_pore_probe(const float *fin, const Lines &Ls, float res, int *wide, cudaStream_t st);
 // flag_buf (optional): flag_cap ints for the per-line flags; without it they
 // come from the stream-ordered scratch pool.
 int launch_envelope(const float *fin, float *fout, const Lines &Ls, float res,

@@ -156,8 +156,11 @@ __device__ __forceinline__ float scan_voxel(const float *line, int n, int x, int
 // positions w, w + 8, ...
 __global__ void __launch_bounds__(32 * kScanWarps) k_scan_cols(const float *__restrict__ fin, float *__restrict__ fout,
                                                                Lines Ls, float a, float inv_a, int periodic, int form,
-                                                               MorphEpi me, float vcap, uint8_t *__restrict__ flag)
+                                                               MorphEpi me, float vcap, uint8_t *__restrict__ flag,
+                                                               const int *__restrict__ wide)
 {
+    if (wide && *wide >= kWideSamples)
+        return; // (the float envelope takes every line)
     extern __shared__ float s_line[]; // [n][32]
     __shared__ unsigned s_need[32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -194,8 +197,11 @@ __global__ void __launch_bounds__(32 * kScanWarps) k_scan_cols(const float *__re
 // Contiguous lines: one warp per row, lanes on 32 consecutive positions.
 __global__ void __launch_bounds__(32 * kScanWarps) k_scan_rows(const float *__restrict__ fin, float *__restrict__ fout,
                                                                Lines Ls, float a, float inv_a, int periodic, int form,
-                                                               MorphEpi me, float vcap, uint8_t *__restrict__ flag)
+                                                               MorphEpi me, float vcap, uint8_t *__restrict__ flag,
+                                                               const int *__restrict__ wide)
 {
+    if (wide && *wide >= kWideSamples)
+        return;
     extern __shared__ float s_line[]; // [kScanWarps][n]
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long nlines = Ls.count();
@@ -228,8 +234,37 @@ __global__ void __launch_bounds__(32 * kScanWarps) k_scan_rows(const float *__re
     }
 }
 
+// Samples of a pass whose value lies beyond 12 positions along the line, counted
+// in *wide (zero before): kWideSamplesOf positions spread over the lines.
+constexpr int kWideSamplesOf = 8192;
+
+__global__ void k_pore_probe(const float *__restrict__ fin, Lines Ls, float a, int *wide)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const LineGeo g = line_addr(Ls, (long long)t * Ls.count() / kWideSamplesOf);
+    const int n = g.n, x = (int)((t * 2654435761u >> 8) % (unsigned)n);
+    float m = INFINITY;
+#pragma unroll 5
+    for (int d = -12; d <= 12; d++)
+        if (x + d >= 0 && x + d < n)
+            m = fminf(m, fin[g.base + (x + d) * g.stride] + a * (float)(d * d));
+    const unsigned far = __ballot_sync(0xffffffffu, m > 144.0f * a);
+    if ((threadIdx.x & 31) == 0 && far)
+        atomicAdd(wide, __popc(far));
+}
+
+int launch_pore_probe(const float *fin, const Lines &Ls, float res, int *wide, cudaStream_t st)
+{
+    PMG_CUDA(cudaMemsetAsync(wide, 0, sizeof(int), st));
+    const int ps__ = prof_begin("k_pore_probe", st);
+    k_pore_probe<<<kWideSamplesOf / 128, 128, 0, st>>>(fin, Ls, res * res, wide);
+    prof_end(ps__, 0.0, st);
+    PMG_CHECK_LAUNCH();
+    return PMG_OK;
+}
+
 int launch_scan(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg, int form,
-                const MorphEpi &me, float vcap, uint8_t *flag, cudaStream_t st)
+                const MorphEpi &me, float vcap, uint8_t *flag, const int *wide, cudaStream_t st)
 {
     const float a = res * res, inv_a = 1.0f / a;
     const int per = cfg.periodic ? 1 : 0;
@@ -237,7 +272,7 @@ int launch_scan(const float *fin, float *fout, const Lines &Ls, float res, const
         const size_t smem = sizeof(float) * (size_t)kScanWarps * (size_t)Ls.s2;
         const int ps__ = prof_begin("k_scan_rows", st);
         k_scan_rows<<<grid_for(Ls.count(), kScanWarps, 152LL * 64), 32 * kScanWarps, smem, st>>>(
-            fin, fout, Ls, a, inv_a, per, form, me, vcap, flag);
+            fin, fout, Ls, a, inv_a, per, form, me, vcap, flag, wide);
         prof_end(ps__, (double)Ls.count() * Ls.s2 * (form == PMG_EDT_MORPH ? 5 : 8), st);
     } else {
         const int n = (int)(Ls.ax == 0 ? Ls.s0 : Ls.s1);
@@ -247,7 +282,7 @@ int launch_scan(const float *fin, float *fout, const Lines &Ls, float res, const
         const long long blocks = (long long)Ls.nb1 * ((Ls.nb2 + 31) / 32);
         const int ps__ = prof_begin("k_scan_cols", st);
         k_scan_cols<<<(unsigned)blocks, 32 * kScanWarps, smem, st>>>(fin, fout, Ls, a, inv_a, per, form, me, vcap,
-                                                                      flag);
+                                                                      flag, wide);
         prof_end(ps__, (double)Ls.count() * n * (form == PMG_EDT_MORPH ? 5 : 8), st);
     }
     PMG_CHECK_LAUNCH();
