@@ -1,9 +1,10 @@
 """Autotuner of launch parameters (no counterpart in the reference).
 
-Some launch parameters change only speed, never results: the line-pair
-envelope passes' segment length and CTA counts (library knobs set through
-``pmg_tune_set``) and the number of CUDA streams the batched configuration
-spreads its media over (a host-side knob).  The tuner times every candidate
+Some launch parameters change only speed, never results: library knobs set
+through ``pmg_tune_set`` (those of the former line-pair envelope passes and
+cross-tile phase are still accepted and timed, without effect) and the number
+of CUDA streams the batched configuration spreads its media over (a host-side
+knob).  The tuner times every candidate
 of one knob at a time (coordinate descent, the others held at their current
 best) on a synthetic medium of the caller's shape class, with CUDA events
 after a warm-up, and keeps the fastest.
