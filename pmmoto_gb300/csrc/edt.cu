@@ -516,12 +516,54 @@ __device__ __forceinline__ void evaluate(Stack &S, const L &line, int nwords, fl
     }
 }
 
-__global__ void k_envelope(const float *__restrict__ fin, float *__restrict__ fout, Lines Ls, float res,
-                           pmg_axis_cfg cfg, int num_hull, int form, MorphEpi me, int redo,
-                           const int *__restrict__ wide)
+// The stack before the natives: the lower imports, or native 0; the first native
+// to push.
+template <class L>
+__device__ __forceinline__ int stack_base(Stack &S, const L &line)
 {
-    if (wide && *wide < kWideSamples)
-        return; // (the scan has the pass)
+    if (S.nl > 0) {
+        S.nn = 0;
+        S.ntv = -1;
+        S.tv = S.lv[S.nl - 1];
+        S.th = S.lh[S.nl - 1];
+        S.tr = S.lr[S.nl - 1];
+        return 0;
+    }
+    S.setbit(0);
+    S.nn = 1;
+    S.ntv = 0;
+    S.tv = 0;
+    S.th = line(0);
+    S.tr = -INFINITY;
+    return 1;
+}
+
+// The reference's envelope of a whole line.
+template <class L>
+__device__ __forceinline__ void envelope_line(Stack &S, const L &line, const LineGeo &g, float aniso,
+                                              const pmg_axis_cfg &cfg, int num_hull, int form, const MorphEpi &me,
+                                              float *fout)
+{
+    const int n = g.n;
+    const int nwords = (n + 31) >> 5;
+    S.clear(nwords);
+    S.nl = 0;
+    S.nu = 0;
+    int up_v[kMaxHull];
+    float up_h[kMaxHull], up_r[kMaxHull];
+    int n_up = 0;
+    if (cfg.periodic)
+        load_imports(S, line, n, aniso, cfg, num_hull, up_v, up_h, up_r, n_up);
+    for (int i = stack_base(S, line); i < n; i++)
+        insert(S, line, i, line(i), aniso, 0);
+    for (int j = 0; j < n_up; j++)
+        insert(S, line, up_v[j] + n, up_h[j], aniso, 1);
+    evaluate(S, line, nwords, aniso, form, me, g, fout + g.base, 0, n);
+}
+
+__global__ void k_envelope(const float *__restrict__ fin, float *__restrict__ fout, Lines Ls, float res,
+                           pmg_axis_cfg cfg, int num_hull, int form, MorphEpi me, int redo)
+{
     const long long nlines = Ls.count();
     extern __shared__ uint32_t smem_bm[];
     const float aniso = fmul(res, res);
@@ -534,40 +576,28 @@ __global__ void k_envelope(const float *__restrict__ fin, float *__restrict__ fo
         // second chance for lines the exact streaming kernel handed back
         if (redo && !line_marked(fout, me, g, form))
             continue;
-        const LineGlobal line{fin + g.base, g.stride};
-        const int n = g.n;
-        const int nwords = (n + 31) >> 5;
-        S.clear(nwords);
-        S.nl = 0;
-        S.nu = 0;
-        int up_v[kMaxHull];
-        float up_h[kMaxHull], up_r[kMaxHull];
-        int n_up = 0;
-        if (cfg.periodic)
-            load_imports(S, line, n, aniso, cfg, num_hull, up_v, up_h, up_r, n_up);
-        // main build
-        int loop_start;
-        if (S.nl > 0) {
-            loop_start = 0;
-            S.nn = 0;
-            S.ntv = -1;
-            S.tv = S.lv[S.nl - 1];
-            S.th = S.lh[S.nl - 1];
-            S.tr = S.lr[S.nl - 1];
-        } else {
-            loop_start = 1;
-            S.setbit(0);
-            S.nn = 1;
-            S.ntv = 0;
-            S.tv = 0;
-            S.th = line(0);
-            S.tr = -INFINITY;
-        }
-        for (int i = loop_start; i < n; i++)
-            insert(S, line, i, line(i), aniso, 0);
-        for (int j = 0; j < n_up; j++)
-            insert(S, line, up_v[j] + n, up_h[j], aniso, 1);
-        evaluate(S, line, nwords, aniso, form, me, g, fout + g.base, 0, n);
+        envelope_line(S, LineGlobal{fin + g.base, g.stride}, g, aniso, cfg, num_hull, form, me, fout);
+    }
+}
+
+// Lines that a scan handed over (flag kScanWhole).
+__global__ void k_envelope_whole(const float *__restrict__ fin, float *__restrict__ fout, Lines Ls, float res,
+                                 pmg_axis_cfg cfg, int num_hull, int form, MorphEpi me,
+                                 const uint8_t *__restrict__ flag, const int *__restrict__ wide)
+{
+    const bool all = wide && *wide;
+    const long long nlines = Ls.count();
+    extern __shared__ uint32_t smem_bm[];
+    const float aniso = fmul(res, res);
+    Stack S;
+    S.bm = smem_bm + threadIdx.x;
+    S.nthr = blockDim.x;
+    for (long long li = blockIdx.x * (long long)blockDim.x + threadIdx.x; li < nlines;
+         li += (long long)gridDim.x * blockDim.x) {
+        if (!all && !(flag[li] & kScanWhole))
+            continue;
+        const LineGeo g = line_addr(Ls, li);
+        envelope_line(S, LineGlobal{fin + g.base, g.stride}, g, aniso, cfg, num_hull, form, me, fout);
     }
 }
 
@@ -623,24 +653,7 @@ __device__ __noinline__ void replay_line(uint32_t *bm, int nthr, const L &line, 
     const int lo_end = whole ? n - 1 : z1; // last native of the lower stack
     // lower part: the imports below, natives up to lo_end
     if (whole || ((part & 1) && z1 > 0)) {
-        int loop_start;
-        if (S.nl > 0) {
-            loop_start = 0;
-            S.nn = 0;
-            S.ntv = -1;
-            S.tv = S.lv[S.nl - 1];
-            S.th = S.lh[S.nl - 1];
-            S.tr = S.lr[S.nl - 1];
-        } else {
-            loop_start = 1;
-            S.setbit(0);
-            S.nn = 1;
-            S.ntv = 0;
-            S.tv = 0;
-            S.th = line(0);
-            S.tr = -INFINITY;
-        }
-        for (int i = loop_start; i <= lo_end; i++)
+        for (int i = stack_base(S, line); i <= lo_end; i++)
             insert(S, line, i, line(i), aniso, 0);
         if (whole) {
             for (int j = 0; j < n_up; j++)
@@ -702,9 +715,10 @@ __device__ __forceinline__ void stage_ends(float *se, const T *__restrict__ fin,
     }
 }
 
-// Flagged lines of any voxel size (flag bit 1: the whole line): a block takes
-// `width` adjacent lines (unflagged ones idle), the lanes of warp 0 their low ends or
-// the whole line and those of warp 1 their high ends, two chains that overlap.
+// Lines whose ends a scan flagged (kScanEnds alone: k_envelope_whole has the
+// others), of any voxel size: a block takes `width` adjacent lines (unflagged ones
+// idle), the lanes of warp 0 their low ends, or the line when it has no zero, and
+// those of warp 1 their high ends, two chains that overlap.
 // Both ends of the lines are staged in shared memory first, because the zero
 // searches, hulls, pushes and the sweep read them again and again in dependent
 // steps.
@@ -720,7 +734,7 @@ __global__ void __launch_bounds__(kEndBlock) k_envelope_ends(const float *__rest
                                                              int form, MorphEpi me, const uint8_t *__restrict__ flag,
                                                              int width, const int *__restrict__ wide)
 {
-    if (wide && *wide >= kWideSamples)
+    if (wide && *wide)
         return;
     extern __shared__ uint32_t smem_bm[];
     __shared__ float s_ends[2 * kEndWin * 33];
@@ -732,18 +746,18 @@ __global__ void __launch_bounds__(kEndBlock) k_envelope_ends(const float *__rest
         const int ra = (int)(t / tiles), kb = (int)(t - (long long)ra * tiles) * width;
         const int lines = min(width, Ls.nb2 - kb);
         const long long l0 = (long long)ra * Ls.nb2 + kb;
-        const int fl = lane < lines ? flag[l0 + lane] : 0;
-        if (!__any_sync(0xffffffffu, fl)) // the same for both warps
+        const bool ends = lane < lines && flag[l0 + lane] == kScanEnds;
+        if (!__any_sync(0xffffffffu, ends)) // the same for both warps
             continue;
         const LineGeo g = line_addr(Ls, l0 + min(lane, lines - 1));
         __syncthreads(); // (the previous tile's readers)
         stage_ends(s_ends, fin, Ls, l0, lines, g, res, w, 2);
         __syncthreads();
-        if (!fl)
+        if (!ends)
             continue;
         const LineEnds<float> line{fin + g.base, g.stride, s_ends + lane, 33, g.n, 0, res};
-        replay_line(smem_bm + threadIdx.x, kEndBlock, line, g, fmul(res, res), cfg, num_hull, (fl & 2) != 0, form, me,
-                    fout, 1 << w);
+        replay_line(smem_bm + threadIdx.x, kEndBlock, line, g, fmul(res, res), cfg, num_hull, false, form, me, fout,
+                    1 << w);
     }
 }
 
@@ -989,34 +1003,33 @@ int launch_envelope(const float *fin, float *fout, const Lines &Ls, float res,
     const int n = (int)(Ls.ax == 0 ? Ls.s0 : Ls.ax == 1 ? Ls.s1 : Ls.s2);
     int block = envelope_block(n);
     size_t smem = (size_t)((n + 31) / 32) * block * 4;
-    if (smem > 48 * 1024)
+    if (smem > 48 * 1024) // (lines far beyond a scan's)
         PMG_CUDA(cudaFuncSetAttribute(k_envelope, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
     const int path = tune_value(kTuneEdtPath);
-    // The outward scan; a caller's flag buffer that does not hold one byte per
-    // line (and the probe's count; lines of a few voxels) leaves the pass to the
-    // float envelope.  Periodic lines of wide pores are mostly replayed at their
-    // ends after the scan, which the envelope alone does faster: voxel sizes
-    // that are no power of two, whose near-ties are many, take it at once
-    // (400 x 300 x 300 pack, voxels of 2.25: 6.4 ms, the envelope 4.0 ms), the
-    // others by a probe on the device (pack, voxels 2 x 1 x 1: 6.5 and 3.9 ms;
-    // 300 x 400 x 425 field of narrow pores: 2.3 and 3.0 ms).
-    const size_t flag_bytes = ((size_t)Ls.count() + 7) / 4 * 4; // (then the count)
+    // The outward scan, the float envelope on the lines that it hands over (wide
+    // pores, unresolved near-ties), and their ends replayed on periodic lines.
+    // A caller's flag buffer that does not hold one byte per line (lines of a few
+    // voxels) leaves the pass to the float envelope, and so do periodic lines of
+    // voxel sizes that are no power of two, whose near-ties are many (400 x 300 x
+    // 300 pack, voxels of 2.25: 6.4 ms, the envelope 4.0 ms).
+    const long long nl = Ls.count();
+    const size_t flag_bytes = ((size_t)nl + 3) / 4 * 4; // (then the probe's choice)
     if (path == 0 && n <= kScanMaxLine && (!cfg.periodic || window_path_ok(res, n)) &&
         (!flag_buf || flag_bytes + sizeof(int) <= (size_t)flag_cap * sizeof(int))) {
         uint8_t *flag = (uint8_t *)flag_buf;
         if (!flag_buf)
             PMG_TRY(scratch_alloc((void **)&flag, flag_bytes + sizeof(int), st));
-        int *wide = cfg.periodic ? (int *)(flag + flag_bytes) : nullptr;
-        int s = wide ? launch_pore_probe(fin, Ls, res, wide, st) : PMG_OK;
+        const int *wide = nullptr;
+        int s = launch_pore_probe(fin, Ls, res, vcap, cfg.periodic, (int *)(flag + flag_bytes), &wide, st);
         if (s == PMG_OK)
             s = launch_scan(fin, fout, Ls, res, cfg, form, me, vcap, flag, wide, st);
-        if (s == PMG_OK)
+        if (s == PMG_OK && cfg.periodic)
             s = launch_ends_float(fin, fout, Ls, res, cfg, num_hull, form, me, flag, wide, st);
-        if (s == PMG_OK && wide) {
-            const int ps__ = prof_begin("k_envelope[wide]", st);
-            k_envelope<<<grid_for(Ls.count(), block, 1LL << 30), block, smem, st>>>(fin, fout, Ls, res, cfg, num_hull, form,
-                                                                                   me, 0, wide);
+        if (s == PMG_OK) {
+            const int ps__ = prof_begin("k_envelope_whole", st);
+            k_envelope_whole<<<grid_for(nl, block, 1LL << 30), block, smem, st>>>(fin, fout, Ls, res, cfg, num_hull,
+                                                                                 form, me, flag, wide);
             prof_end(ps__, 0.0, st);
             s = cudaGetLastError() == cudaSuccess ? PMG_OK : PMG_ECUDA;
         }
@@ -1032,7 +1045,7 @@ int launch_envelope(const float *fin, float *fout, const Lines &Ls, float res,
     {
         const int ps__ = prof_begin(redo ? "k_envelope_redo" : "k_envelope", st);
         k_envelope<<<grid_for(Ls.count(), block, redo ? 152LL * 8 : 1LL << 30), block, smem, st>>>(
-            fin, fout, Ls, res, cfg, num_hull, form, me, redo, nullptr);
+            fin, fout, Ls, res, cfg, num_hull, form, me, redo);
         prof_end(ps__, redo ? 0.0 : (double)Ls.count() * n * 4 + (form == PMG_EDT_MORPH ? (double)Ls.count() * me.o2 : (double)Ls.count() * n * 4), st);
     }
     PMG_CHECK_LAUNCH();

@@ -207,7 +207,7 @@ bool lattice_ok(const int64_t *shape, const float *res, const pmg_axis_cfg *cfg)
 int lattice_run(const uint8_t *img, float *out, float *tmp, const int64_t *shape, const float *res,
                 const pmg_axis_cfg *cfg, int num_hull, int form, uint16_t *flags, cudaStream_t st);
 // Flagged lines: after a lattice pass over counts or heights (line_reach), and
-// after a scan (1 the ends, 2 the whole line).
+// after a scan (kScanEnds).
 int launch_ends_counts(const uint16_t *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
                        int num_hull, const uint16_t *flag, cudaStream_t st);
 int launch_ends_heights(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
@@ -216,12 +216,15 @@ int launch_ends_float(const float *fin, float *fout, const Lines &Ls, float res,
                       int num_hull, int form, const MorphEpi &me, const uint8_t *flag, const int *wide,
                       cudaStream_t st);
 // The outward scan (edt_scan.cu), lines of at most kScanMaxLine voxels; vcap:
-// values above it only matter as "above it".
+// values above it only matter as "above it".  Line flags: the ends depend on
+// imported hulls; the whole line is left to the float envelope.  wide (device,
+// null: never): set by the probe when the envelope is to take every line, and
+// the scan then does nothing.
+constexpr int kScanEnds = 1, kScanWhole = 2;
+int launch_pore_probe(const float *fin, const Lines &Ls, float res, float vcap, int periodic, int *wide,
+                      const int **choice, cudaStream_t st);
 int launch_scan(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg, int form,
                 const MorphEpi &me, float vcap, uint8_t *flag, const int *wide, cudaStream_t st);
-// Wide pores: at least kWideSamples of the probe's samples (device count *wide).
-constexpr int kWideSamples = 256;
-int launch_pore_probe(const float *fin, const Lines &Ls, float res, int *wide, cudaStream_t st);
 // flag_buf (optional): flag_cap ints for the per-line flags; without it they
 // come from the stream-ordered scratch pool.
 int launch_envelope(const float *fin, float *fout, const Lines &Ls, float res,

@@ -27,6 +27,9 @@
 // instructions per candidate).
 #include <cfloat>
 #include <algorithm>
+#include <cmath>
+
+#include <cooperative_groups.h>
 
 #include "edt_internal.cuh"
 
@@ -131,7 +134,7 @@ __device__ __forceinline__ float scan_voxel(const float *line, int n, int x, int
     if (!live || m > vcap)
         return m;
     if (m >= FLT_MAX) { // no solid voxel on the line
-        need |= periodic ? 1u : 0u;
+        need |= periodic ? kScanEnds : 0u;
         return m;
     }
     const float R = __fsqrt_rn(m * inv_a);
@@ -139,7 +142,7 @@ __device__ __forceinline__ float scan_voxel(const float *line, int n, int x, int
     if (periodic) {
         const int e = min(x + 1, n - x);
         if (m + eta >= fmul(a, (float)e * (float)e)) {
-            need |= 1u;
+            need |= kScanEnds;
             return m;
         }
     }
@@ -147,9 +150,20 @@ __device__ __forceinline__ float scan_voxel(const float *line, int n, int x, int
         float v = m;
         if (scan_resolve<S>(line, n, x, a, m, R, eta, v))
             return v;
-        need |= 2u;
+        need |= kScanWhole;
     }
     return m;
+}
+
+// A scan starts while the probe in front of it still runs (launch_after_probe):
+// its first blocks load their lines before they wait for the choice, which hides
+// the probe (2 x 8 of 305 us of a 256^3 field); the others find it made.
+constexpr unsigned kFirstBlocks = 152 * 4;
+
+__device__ __forceinline__ bool left_to_envelope(const int *wide)
+{
+    cudaGridDependencySynchronize();
+    return wide && *(const volatile int *)wide;
 }
 
 // Strided lines (axis 0 or 1): one block per 32 adjacent lines, warp w on
@@ -159,8 +173,8 @@ __global__ void __launch_bounds__(32 * kScanWarps) k_scan_cols(const float *__re
                                                                MorphEpi me, float vcap, uint8_t *__restrict__ flag,
                                                                const int *__restrict__ wide)
 {
-    if (wide && *wide >= kWideSamples)
-        return; // (the float envelope takes every line)
+    if (blockIdx.x >= kFirstBlocks && left_to_envelope(wide))
+        return;
     extern __shared__ float s_line[]; // [n][32]
     __shared__ unsigned s_need[32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -173,13 +187,21 @@ __global__ void __launch_bounds__(32 * kScanWarps) k_scan_cols(const float *__re
     const float *src = fin + g.base;
     if (threadIdx.x < 32)
         s_need[threadIdx.x] = 0;
+    bool some = false;
 #pragma unroll 8
-    for (int x = w; x < n; x += kScanWarps)
-        s_line[x * 32 + lane] = __ldg(src + x * g.stride);
-    __syncthreads();
+    for (int x = w; x < n; x += kScanWarps) {
+        const float v = __ldg(src + x * g.stride);
+        some |= v < FLT_MAX;
+        s_line[x * 32 + lane] = v;
+    }
+    // without a solid on any of the lines, nothing to scan
+    const bool scan = __syncthreads_or(some) || periodic;
+    if (blockIdx.x < kFirstBlocks && left_to_envelope(wide))
+        return;
     unsigned need = 0;
     for (int x = w; x < n; x += kScanWarps) {
-        const float v = scan_voxel<32>(s_line + lane, n, x, min(x, n - 1 - x), live, a, inv_a, periodic, vcap, need);
+        const float v = scan ? scan_voxel<32>(s_line + lane, n, x, min(x, n - 1 - x), live, a, inv_a, periodic, vcap, need)
+                             : FLT_MAX;
         if (!live)
             continue;
         if (form == PMG_EDT_MORPH)
@@ -200,8 +222,9 @@ __global__ void __launch_bounds__(32 * kScanWarps) k_scan_rows(const float *__re
                                                                MorphEpi me, float vcap, uint8_t *__restrict__ flag,
                                                                const int *__restrict__ wide)
 {
-    if (wide && *wide >= kWideSamples)
+    if (blockIdx.x >= kFirstBlocks && left_to_envelope(wide))
         return;
+    bool early = blockIdx.x < kFirstBlocks;
     extern __shared__ float s_line[]; // [kScanWarps][n]
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long nlines = Ls.count();
@@ -211,15 +234,24 @@ __global__ void __launch_bounds__(32 * kScanWarps) k_scan_rows(const float *__re
          li += (long long)gridDim.x * kScanWarps) {
         const LineGeo g = line_addr(Ls, li);
         const float *src = fin + g.base;
+        bool some = false;
 #pragma unroll 8
-        for (int x = lane; x < n; x += 32)
-            row[x] = __ldg(src + x);
+        for (int x = lane; x < n; x += 32) {
+            const float v = __ldg(src + x);
+            some |= v < FLT_MAX;
+            row[x] = v;
+        }
+        const bool scan = __any_sync(0xffffffffu, some) || periodic;
         __syncwarp();
+        if (early && left_to_envelope(wide))
+            return;
+        early = false;
         unsigned need = 0;
         for (int x0 = 0; x0 < n; x0 += 32) {
             const int x = x0 + lane;
             const bool live = x < n;
-            const float v = scan_voxel<1>(row, n, x, min(x0, n - 32 - x0), live, a, inv_a, periodic, vcap, need);
+            const float v = scan ? scan_voxel<1>(row, n, x, min(x0, n - 32 - x0), live, a, inv_a, periodic, vcap, need)
+                                 : FLT_MAX;
             if (!live)
                 continue;
             if (form == PMG_EDT_MORPH)
@@ -234,33 +266,111 @@ __global__ void __launch_bounds__(32 * kScanWarps) k_scan_rows(const float *__re
     }
 }
 
-// Samples of a pass whose value lies beyond 12 positions along the line, counted
-// in *wide (zero before): kWideSamplesOf positions spread over the lines.
-constexpr int kWideSamplesOf = 8192;
+// Wide pores.  A scan's cost grows with the distances of its voxels, the float
+// envelope's hardly does, so a probe in front of the pass estimates the steps of
+// a scan from kProbeGroups of its warps (32 adjacent lines, or 32 consecutive
+// positions of a row) and sets *wide when the envelope is the cheaper one.
+// A sample's steps come from the heights at offsets that grow with the distance:
+// heights' roots change by at most a voxel from one position to the next, so a
+// solid between two offsets shows.  One cluster, so that the sum needs no
+// clearing.
+constexpr int kProbeBlocks = 8, kProbeThreads = 512, kProbeGroups = kProbeBlocks * kProbeThreads / 32;
 
-__global__ void k_pore_probe(const float *__restrict__ fin, Lines Ls, float a, int *wide)
+__global__ void __cluster_dims__(kProbeBlocks, 1, 1) __launch_bounds__(kProbeThreads)
+    k_pore_probe(const float *__restrict__ fin, Lines Ls, float a, float inv_a, float most, float budget, int *wide)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const LineGeo g = line_addr(Ls, (long long)t * Ls.count() / kWideSamplesOf);
-    const int n = g.n, x = (int)((t * 2654435761u >> 8) % (unsigned)n);
-    float m = INFINITY;
-#pragma unroll 5
-    for (int d = -12; d <= 12; d++)
-        if (x + d >= 0 && x + d < n)
-            m = fminf(m, fin[g.base + (x + d) * g.stride] + a * (float)(d * d));
-    const unsigned far = __ballot_sync(0xffffffffu, m > 144.0f * a);
-    if ((threadIdx.x & 31) == 0 && far)
-        atomicAdd(wide, __popc(far));
+    cudaTriggerProgrammaticLaunchCompletion(); // (the scan may start: its first blocks wait)
+    __shared__ unsigned s_sum;
+    const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x == 0)
+        s_sum = 0;
+    __syncthreads();
+    // group q of equal shares of the lines; where in its share and along the
+    // lines by multiplicative hashes (a regular pattern could follow the axes)
+    const unsigned q = blockIdx.x * (kProbeThreads / 32) + (threadIdx.x >> 5);
+    const long long nl = Ls.count(), li = (q * nl + (long long)(q * 2246822519u >> 4) % nl) / kProbeGroups;
+    LineGeo g = line_addr(Ls, Ls.ax == 2 ? li : min(li + lane, nl - 1));
+    const int n = g.n;
+    int x = (int)((q * 2654435761u >> 8) % (unsigned)n);
+    if (Ls.ax == 2)
+        x = min(x / 32 * 32 + lane, n - 1);
+    const float *c = fin + g.base;
+    constexpr int kOff[12] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64};
+    float m = c[x * g.stride];
+#pragma unroll
+    for (int k = 0; k < 12; k++)
+        m = fminf(m, fminf(c[max(x - kOff[k], 0) * g.stride], c[min(x + kOff[k], n - 1) * g.stride]) +
+                         a * (float)(kOff[k] * kOff[k]));
+    // (a warp scans as far as its farthest lane)
+    const unsigned far = __reduce_max_sync(0xffffffffu, (unsigned)fminf(__fsqrt_rn(m * inv_a), most));
+    if (lane == 0)
+        atomicAdd(&s_sum, far);
+    cluster.sync();
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        unsigned sum = 0;
+        for (int k = 0; k < kProbeBlocks; k++)
+            sum += *cluster.map_shared_rank(&s_sum, k);
+        *wide = (float)sum > budget * (float)kProbeGroups;
+    }
+    cluster.sync(); // (the other blocks' sums are read until here)
 }
 
-int launch_pore_probe(const float *fin, const Lines &Ls, float res, int *wide, cudaStream_t st)
+// Steps a voxel from which the envelope is the faster one.  A step costs about 1 ps a
+// voxel (512^3: 0.14 ms a pass), the envelope 15 to 50 ps (1.9 to 7 ms), and on few
+// lines one chain of n pushes (1 to 2 us each) whatever their number, hence the
+// term in the lines.  Scan alone, envelope alone, chosen, in ms, both passes,
+// voxels of 2.25: 512^3 field of sigma 4: 2.0, 5.1, 2.0; cavity of radius 230: 7.2, 5.1,
+// 5.1; points 10 voxels apart on average: 14.4, 7.6, 5.8; 20: 51, 10.6, 10.6; 200 x 180 x
+// 220 cavity of radius 81: 0.32, 0.82, 0.32; points 20 voxels apart: 2.0, 1.5, 1.5;
+// 96^3: 0.25, 0.51, 0.25.  On periodic lines the ends are replayed after a scan, so
+// the crossing lies lower (voxels 1 x 1 x 2, 512^3 field of sigma 4: 3.5, 5.5, 3.5;
+// sigma 20: 12.7, 8.6, 8.6).
+static float scan_budget(const Lines &Ls, int periodic)
 {
-    PMG_CUDA(cudaMemsetAsync(wide, 0, sizeof(int), st));
+    const float nl = (float)Ls.count();
+    const int k = tune_value(kTuneEdtWide); // 1024: as it is; 0: always the envelope, 8193: never
+    if (k == 0 || k > 8192)
+        return k == 0 ? -1.0f : INFINITY;
+    return (periodic ? std::max(5.0f, 0.22e6f / nl) : std::max(36.0f, 3.6e6f / nl)) * ((float)k / 1024.0f);
+}
+
+// *choice = wide once the probe has set it, null where no scan of the pass can
+// take more steps than the budget (short lines, a small cap).
+int launch_pore_probe(const float *fin, const Lines &Ls, float res, float vcap, int periodic, int *wide,
+                      const int **choice, cudaStream_t st)
+{
+    const float a = res * res, inv_a = 1.0f / a;
+    const int n = (int)(Ls.ax == 0 ? Ls.s0 : Ls.ax == 1 ? Ls.s1 : Ls.s2);
+    // the most steps of a voxel: to the line's end, or to the cap
+    const float most = std::fmin((float)n, std::sqrt(vcap * inv_a) + 1.0f), budget = scan_budget(Ls, periodic);
+    *choice = nullptr;
+    if (most <= budget)
+        return PMG_OK;
     const int ps__ = prof_begin("k_pore_probe", st);
-    k_pore_probe<<<kWideSamplesOf / 128, 128, 0, st>>>(fin, Ls, res * res, wide);
+    k_pore_probe<<<kProbeBlocks, kProbeThreads, 0, st>>>(fin, Ls, a, inv_a, most, budget, wide);
     prof_end(ps__, 0.0, st);
     PMG_CHECK_LAUNCH();
+    *choice = wide;
     return PMG_OK;
+}
+
+// A launch that need not wait for the end of the kernel before it.
+template <class... Args>
+static cudaError_t launch_after_probe(void (*kernel)(Args...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+                                      Args... args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 int launch_scan(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg, int form,
@@ -271,8 +381,12 @@ int launch_scan(const float *fin, float *fout, const Lines &Ls, float res, const
     if (Ls.ax == 2) {
         const size_t smem = sizeof(float) * (size_t)kScanWarps * (size_t)Ls.s2;
         const int ps__ = prof_begin("k_scan_rows", st);
-        k_scan_rows<<<grid_for(Ls.count(), kScanWarps, 152LL * 64), 32 * kScanWarps, smem, st>>>(
-            fin, fout, Ls, a, inv_a, per, form, me, vcap, flag, wide);
+        const unsigned grid = grid_for(Ls.count(), kScanWarps, 152LL * 64);
+        if (wide)
+            PMG_CUDA(launch_after_probe(k_scan_rows, grid, 32 * kScanWarps, smem, st, fin, fout, Ls, a, inv_a, per, form, me,
+                                        vcap, flag, wide));
+        else
+            k_scan_rows<<<grid, 32 * kScanWarps, smem, st>>>(fin, fout, Ls, a, inv_a, per, form, me, vcap, flag, wide);
         prof_end(ps__, (double)Ls.count() * Ls.s2 * (form == PMG_EDT_MORPH ? 5 : 8), st);
     } else {
         const int n = (int)(Ls.ax == 0 ? Ls.s0 : Ls.s1);
@@ -281,8 +395,12 @@ int launch_scan(const float *fin, float *fout, const Lines &Ls, float res, const
             PMG_CUDA(cudaFuncSetAttribute(k_scan_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         const long long blocks = (long long)Ls.nb1 * ((Ls.nb2 + 31) / 32);
         const int ps__ = prof_begin("k_scan_cols", st);
-        k_scan_cols<<<(unsigned)blocks, 32 * kScanWarps, smem, st>>>(fin, fout, Ls, a, inv_a, per, form, me, vcap,
-                                                                      flag, wide);
+        if (wide)
+            PMG_CUDA(launch_after_probe(k_scan_cols, (unsigned)blocks, 32 * kScanWarps, smem, st, fin, fout, Ls, a, inv_a, per,
+                                        form, me, vcap, flag, wide));
+        else
+            k_scan_cols<<<(unsigned)blocks, 32 * kScanWarps, smem, st>>>(fin, fout, Ls, a, inv_a, per, form, me, vcap, flag,
+                                                                        wide);
         prof_end(ps__, (double)Ls.count() * n * (form == PMG_EDT_MORPH ? 5 : 8), st);
     }
     PMG_CHECK_LAUNCH();

@@ -90,7 +90,7 @@ static const TuneSpec g_tune_spec[kTuneKnobs] = {
     {"edt.narrow", 64, 0, 8193},        // (no effect)
     {"edt.narrow_rows", 32, 0, 8193},   // (no effect)
     {"cc.seam_batched", 1, 0, 1},       // periodic merge: all features' seams in one sort (1) or one by one (0)
-    {"edt.wide", 1024, 0, 8193},        // (no effect)
+    {"edt.wide", 1024, 0, 8193},        // scanned passes: steps (in 1/1024 of the measured crossing) that the envelope takes over from
 };
 static std::atomic<int> g_tune[kTuneKnobs] = {{256}, {32}, {16}, {0}, {0}, {96}, {2048}, {64}, {32}, {1}, {1024}};
 
