@@ -17,7 +17,8 @@
 //    choice;
 //  * otherwise (rare) the line is flagged for the whole float envelope.
 // m needs only the positions with a d^2 <= m + a / 2: the scan runs outward
-// from x, all lanes together, until that holds for every lane.  On a periodic
+// from x, all lanes together, until that holds for every lane.  Where eta is the
+// larger one the line is flagged as well.  On a periodic
 // line a voxel whose m reaches the squared distance to a line end may depend
 // on the imported hulls: the line is flagged for its end segments.
 //
@@ -145,6 +146,12 @@ __device__ __forceinline__ float scan_voxel(const float *line, int n, int x, int
             need |= kScanEnds;
             return m;
         }
+    }
+    // (the scan ends at m + a / 2: from about 300 voxels on long lines a parabola
+    // between there and m + eta may not have been looked at)
+    if (eta > half) {
+        need |= kScanWhole;
+        return m;
     }
     if (m2 <= m + eta) {
         float v = m;

@@ -92,3 +92,25 @@ def test_both_choices_vs_oracle(shape, per):
     finally:
         L.pmg_prof_enable(0)
         tune._set_lib("edt.wide", -1)
+
+
+@pytest.mark.parametrize("res", [(2.25,) * 3, (1.0, 1.0, 2.0), (30.0, 0.75, 0.75)])
+def test_far_near_ties_on_long_lines_vs_oracle(res):
+    """Scans of distances where the envelope's rounding may order values more than
+    half a step apart: solids hundreds of voxels away, in pairs that nearly tie."""
+    from pmmoto_gb300 import tune
+    from pmmoto_gb300.filters import distance as D
+
+    rng = np.random.default_rng(12)
+    img = np.ones((40, 3, 1024), np.uint8)
+    for i in range(40):
+        lo, hi = rng.integers(0, 200), rng.integers(824, 1024)
+        img[i, rng.integers(0, 3), lo] = img[i, rng.integers(0, 3), hi] = 0
+    want = O.edt3d(img, resolution=res, squared=True)
+    try:
+        tune._set_lib("edt.wide", 8193)
+        np.testing.assert_array_equal(D.edt3d(img, resolution=res, squared=True), want)
+        np.testing.assert_array_equal(D.edt3d(img.transpose(0, 2, 1).copy(), resolution=(res[0], res[2], res[1]), squared=True),
+                                      O.edt3d(img.transpose(0, 2, 1).copy(), resolution=(res[0], res[2], res[1]), squared=True))
+    finally:
+        tune._set_lib("edt.wide", -1)
