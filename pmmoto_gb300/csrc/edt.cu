@@ -779,11 +779,12 @@ __global__ void __launch_bounds__(kEndBlock) k_envelope_ends(const float *__rest
 // Bound by the latency of those chains.  Building the reference's hull stacks
 // instead kept a warp in divergent pops and divisions: 1024^3 field 1.8 ms
 // over both passes, 128^3 pack 0.54 ms.
-constexpr int kWrapMax = 255; // farthest entry (products below 2^31)
+constexpr int kWrapMax = 255;        // farthest entry
+constexpr float kTall = 2097152.0f;  // tallest height (their products' differences stay below 2^31)
 
 template <class T>
 __global__ void __launch_bounds__(64) k_lattice_ends(const T *__restrict__ fin, float *__restrict__ fout, Lines Ls,
-                                                     float res, pmg_axis_cfg cfg, int num_hull, int form,
+                                                     float res, float resh, pmg_axis_cfg cfg, int num_hull, int form,
                                                      const uint16_t *__restrict__ flag)
 {
     extern __shared__ uint32_t smem_bm[]; // envelope bits of the replays: [nwords][32]
@@ -806,9 +807,9 @@ __global__ void __launch_bounds__(64) k_lattice_ends(const T *__restrict__ fin, 
         __syncthreads(); // (the previous tile's readers)
         if (w == 0)
             s_hard[lane] = whole;
-        stage_ends(s_ends, fin, Ls, l0, lines, g, res, w, 2);
+        stage_ends(s_ends, fin, Ls, l0, lines, g, resh, w, 2);
         __syncthreads();
-        const LineEnds<T> line{fin + g.base, g.stride, s_ends + lane, 33, n, 0, res};
+        const LineEnds<T> line{fin + g.base, g.stride, s_ends + lane, 33, n, 0, resh};
         const int reach = whole ? 0 : w == 0 ? fl & 0xff : fl >> 8;
         if (reach > 0) {
             // positions of the segment from its end that faces the line
@@ -824,9 +825,11 @@ __global__ void __launch_bounds__(64) k_lattice_ends(const T *__restrict__ fin, 
                 ek[c] = 0;
             }
             if (!hard) {
+                // (a height beyond kTall leaves the line to the float replay: 32-bit products)
                 auto height = [&](int q) -> int {
-                    const float f = line(p0 + dir * q);
-                    return f >= FLT_MAX ? -1 : (int)fmul(f, inv_a);
+                    const float f = line(p0 + dir * q), k = fmul(f, inv_a);
+                    hard = hard || (f < FLT_MAX && k > kTall);
+                    return f >= FLT_MAX || k > kTall ? -1 : (int)k;
                 };
                 int e = 0, ke = height(0);
                 while (ke < 0 && ++e < most)
@@ -918,29 +921,30 @@ __global__ void __launch_bounds__(64) k_lattice_ends(const T *__restrict__ fin, 
 }
 
 template <class T>
-static int launch_lattice_ends(const T *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
-                               int num_hull, int form, const uint16_t *flag, cudaStream_t st)
+static int launch_lattice_ends(const T *fin, float *fout, const Lines &Ls, float res, float resh,
+                               const pmg_axis_cfg &cfg, int num_hull, int form, const uint16_t *flag, cudaStream_t st)
 {
     const int n = (int)(Ls.ax == 0 ? Ls.s0 : Ls.ax == 1 ? Ls.s1 : Ls.s2);
     const size_t smem = (size_t)((n + 31) / 32) * 32 * 4;
     const long long tiles = (long long)Ls.nb1 * ((Ls.nb2 + 31) / 32);
     const int ps__ = prof_begin("k_lattice_ends", st);
-    k_lattice_ends<T><<<grid_for(tiles, 1, 152LL * 64), 64, smem, st>>>(fin, fout, Ls, res, cfg, num_hull, form, flag);
+    k_lattice_ends<T><<<grid_for(tiles, 1, 152LL * 64), 64, smem, st>>>(fin, fout, Ls, res, resh, cfg, num_hull, form,
+                                                                          flag);
     prof_end(ps__, 0.0, st);
     PMG_CHECK_LAUNCH();
     return PMG_OK;
 }
 
-int launch_ends_counts(const uint16_t *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
-                       int num_hull, const uint16_t *flag, cudaStream_t st)
+int launch_ends_counts(const uint16_t *fin, float *fout, const Lines &Ls, float res, float res_count,
+                       const pmg_axis_cfg &cfg, int num_hull, const uint16_t *flag, cudaStream_t st)
 {
-    return launch_lattice_ends(fin, fout, Ls, res, cfg, num_hull, PMG_EDT_SQUARED, flag, st);
+    return launch_lattice_ends(fin, fout, Ls, res, res_count, cfg, num_hull, PMG_EDT_SQUARED, flag, st);
 }
 
 int launch_ends_heights(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
                         int num_hull, int form, const uint16_t *flag, cudaStream_t st)
 {
-    return launch_lattice_ends(fin, fout, Ls, res, cfg, num_hull, form, flag, st);
+    return launch_lattice_ends(fin, fout, Ls, res, res, cfg, num_hull, form, flag, st);
 }
 
 int launch_ends_float(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
@@ -1085,22 +1089,28 @@ int edt3d_run(const uint8_t *img, float *out, float *tmp, const int64_t *shape, 
               long long flag_cap)
 {
     MorphEpi none{};
-    const long long lines = (long long)shape[0] * std::max(shape[1], shape[2]);
-    if (tune_value(kTuneEdtPath) == 0 && lattice_ok(shape, res, cfg) &&
-        (!flag_buf || lines <= flag_cap * (long long)(sizeof(int) / sizeof(uint16_t)))) {
-        uint16_t *flag = (uint16_t *)flag_buf;
-        if (!flag_buf)
-            PMG_TRY(scratch_alloc((void **)&flag, sizeof(uint16_t) * (size_t)lines, st));
-        const int s = lattice_run(img, out, tmp, shape, res, cfg, num_hull, form, flag, st);
-        const int s2 = flag_buf ? PMG_OK : scratch_free(flag, st);
-        return s != PMG_OK ? s : s2;
-    }
-    PMG_TRY(launch_linear(img, out, shape, res[0], cfg[0], st));
-    PMG_TRY(launch_envelope(out, tmp, all_lines(shape, 1), res[1], cfg[1], num_hull,
-                            PMG_EDT_SQUARED, none, st, INT_MAX, flag_buf, flag_cap));
-    PMG_TRY(launch_envelope(tmp, out, all_lines(shape, 2), res[2], cfg[2], num_hull, form, none,
-                            st, INT_MAX, flag_buf, flag_cap));
-    return PMG_OK;
+    LatticePlan P{};
+    if (tune_value(kTuneEdtPath) == 0)
+        P = lattice_plan(shape, res, cfg);
+    // a 16-bit flag per line of the larger lattice pass
+    const long long lines = (long long)shape[0] * std::max(P.cols ? shape[2] : 0, P.rows ? shape[1] : 0);
+    if (flag_buf && lines > flag_cap * (long long)(sizeof(int) / sizeof(uint16_t)))
+        P = LatticePlan{};
+    uint16_t *flag = (uint16_t *)flag_buf;
+    if (!flag_buf && (P.cols || P.rows))
+        PMG_TRY(scratch_alloc((void **)&flag, sizeof(uint16_t) * (size_t)lines, st));
+    int s = P.counts ? launch_lin_counts(img, (uint16_t *)out, shape, cfg[0], st)
+                     : launch_linear(img, out, shape, res[0], cfg[0], st);
+    if (s == PMG_OK)
+        s = P.cols ? lattice_cols(P, out, tmp, shape, res, cfg, num_hull, flag, st)
+                   : launch_envelope(out, tmp, all_lines(shape, 1), res[1], cfg[1], num_hull, PMG_EDT_SQUARED, none, st,
+                                     INT_MAX, flag_buf, flag_cap);
+    if (s == PMG_OK)
+        s = P.rows ? lattice_rows(P, tmp, out, shape, res, cfg, num_hull, form, flag, st)
+                   : launch_envelope(tmp, out, all_lines(shape, 2), res[2], cfg[2], num_hull, form, none, st, INT_MAX,
+                                     flag_buf, flag_cap);
+    const int s2 = flag_buf ? PMG_OK : scratch_free(flag, st);
+    return s != PMG_OK ? s : s2;
 }
 
 } // namespace pmg

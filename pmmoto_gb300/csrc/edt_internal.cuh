@@ -202,14 +202,22 @@ int launch_lin_float(const uint8_t *img, float *out, const int64_t *shape, float
                      cudaStream_t st);
 int launch_linear(const uint8_t *img, float *out, const int64_t *shape, float res, const pmg_axis_cfg &cfg,
                   cudaStream_t st);
-// The whole transform on the integer lattice.
-bool lattice_ok(const int64_t *shape, const float *res, const pmg_axis_cfg *cfg);
-int lattice_run(const uint8_t *img, float *out, float *tmp, const int64_t *shape, const float *res,
-                const pmg_axis_cfg *cfg, int num_hull, int form, uint16_t *flags, cudaStream_t st);
-// Flagged lines: after a lattice pass over counts or heights (line_reach), and
-// after a scan (kScanEnds).
-int launch_ends_counts(const uint16_t *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
-                       int num_hull, const uint16_t *flag, cudaStream_t st);
+// The passes of a transform that run on the integer lattice: cols along axis 1
+// (counts: from the counts of the linear pass, whose voxels are 2^shift of its
+// own), rows along axis 2; wide1, wide2: finite heights may exceed its range.
+struct LatticePlan {
+    bool cols, counts, rows, wide1, wide2;
+    int shift;
+};
+LatticePlan lattice_plan(const int64_t *shape, const float *res, const pmg_axis_cfg *cfg);
+int lattice_cols(const LatticePlan &P, const void *in, float *out, const int64_t *shape, const float *res,
+                 const pmg_axis_cfg *cfg, int num_hull, uint16_t *flags, cudaStream_t st);
+int lattice_rows(const LatticePlan &P, const float *in, float *out, const int64_t *shape, const float *res,
+                 const pmg_axis_cfg *cfg, int num_hull, int form, uint16_t *flags, cudaStream_t st);
+// Flagged lines: after a lattice pass over counts (of voxels of res_count) or
+// heights (line_reach), and after a scan (kScanEnds).
+int launch_ends_counts(const uint16_t *fin, float *fout, const Lines &Ls, float res, float res_count,
+                       const pmg_axis_cfg &cfg, int num_hull, const uint16_t *flag, cudaStream_t st);
 int launch_ends_heights(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
                         int num_hull, int form, const uint16_t *flag, cudaStream_t st);
 int launch_ends_float(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,

@@ -1,16 +1,20 @@
-// Distance transform of isotropic power-of-two voxels on an integer lattice
-// (sm_103a), and the linear pass of every other voxel size.
+// Distance transform of power-of-two voxels on an integer lattice (sm_103a), and
+// the linear pass of every other voxel size.
 //
-// With one power-of-two voxel size res every height of the transform is
-// K * res^2 with an integer K, and the reference's float passes return the
-// exact minimum (edt_exact.cu has the rounding argument), so the passes run on
-// integers:
+// Where the voxel sizes are powers of two and a pass's own is the smallest of the
+// axes so far, every height that it reads is K * res^2 with an integer K, and the
+// reference's float passes return the exact minimum at every position where it is
+// below kBig (edt_exact.cu has the rounding argument for heights below 2^24;
+// taller ones meet such a parabola thousands of positions away, far beyond their
+// rounding).  So the passes run on integers, pass by pass:
 //
 //  * k_lin       the linear pass (squared_edt_1d, _distance.hpp:135-182, with
 //                the correctors of _distance.pyx:240-279): counts of voxels to
 //                the nearest zero or restart, uint16, every position of a line
 //                by its own segment of threads;
-//  * k_par_cols  a strided envelope pass: min over v of K(v) + (x - v)^2;
+//  * k_par_cols  a strided envelope pass: min over v of K(v) + (x - v)^2, from
+//                counts (K = count^2 times the squared ratio of the sizes) or
+//                from heights;
 //  * k_par_rows  the same along the contiguous axis, out to float32.
 //
 // min over |d| <= k of K(x + d) + d^2 is built one distance at a time as
@@ -28,6 +32,7 @@
 // envelope, unless no height of the volume can reach kBig.
 #include <cfloat>
 #include <algorithm>
+#include <cmath>
 
 #include "edt_internal.cuh"
 
@@ -436,11 +441,20 @@ int launch_lin_float(const uint8_t *img, float *out, const int64_t *shape, float
 constexpr uint32_t kBig = 60000u, kMaxStep = 245u, kWholeLine = 255u;
 constexpr uint32_t kBig2 = kBig * 0x10001u;
 
-// (count, count) -> (K, K), absent counts -> kBig
-__device__ __forceinline__ uint32_t square2(uint32_t c)
+// (count, count) -> (K, K), absent counts -> kBig; the counted voxels are 2^shift
+// of the pass's own (shift <= kMaxShift)
+constexpr int kMaxShift = 16;
+
+__device__ __forceinline__ uint32_t square2(uint32_t c, int shift)
 {
-    const uint32_t a = min(c & 0xffffu, kMaxStep), b = min(c >> 16, kMaxStep);
+    const uint32_t a = min(min(c & 0xffffu, 255u) << shift, kMaxStep), b = min(min(c >> 16, 255u) << shift, kMaxStep);
     return min(a * a, kBig) | (min(b * b, kBig) << 16);
+}
+
+// heights -> (K, K)
+__device__ __forceinline__ uint32_t pack_heights(float f0, float f1, float inv_a)
+{
+    return pack_float2(fminf(fmul(f0, inv_a), (float)kBig), fminf(fmul(f1, inv_a), (float)kBig));
 }
 
 // height of an integer minimum
@@ -530,7 +544,7 @@ __device__ __forceinline__ uint32_t line_reach(const uint32_t (&g)[P], uint32_t 
     return lo0 | (hi0 << 8) | (second ? (lo1 << 16) | (hi1 << 24) : 0u);
 }
 
-// Strided pass along axis 1 of [n0][n][s2]: one thread block per plane and
+// Strided pass along axis 1 of [n0][n][s2] in at most `last` steps: one thread block per plane and
 // LN * VEC adjacent lines (VEC = 2: two lines per thread, s2 even), thread
 // group q of LN on positions [q P, (q + 1) P) of its lines, heights in
 // registers.  Groups hand their end values on through shared memory, one
@@ -538,10 +552,10 @@ __device__ __forceinline__ uint32_t line_reach(const uint32_t (&g)[P], uint32_t 
 // share an SM and one loads while the other computes.
 // Bound by the packed add-min pipe (two instructions per pair of voxels and
 // distance).
-template <int P, int VEC, int LN>
+template <class T, int P, int VEC, int LN>
 __global__ void __launch_bounds__(P == 32 ? 512 : 32 * P, P == 32 ? 2 : 1)
-    k_par_cols(const uint16_t *__restrict__ D, float *__restrict__ out, int n, int s2, float a, int periodic, int wide,
-               uint16_t *__restrict__ flag)
+    k_par_cols(const T *__restrict__ D, float *__restrict__ out, int n, int s2, float a, float inv_a, int shift, int last,
+               int periodic, int wide, uint16_t *__restrict__ flag)
 {
     extern __shared__ uint32_t s_end[]; // [2][groups][4][LN]
     const int l = threadIdx.x % LN, w = threadIdx.x / LN, nw = blockDim.x / LN;
@@ -550,31 +564,44 @@ __global__ void __launch_bounds__(P == 32 ? 512 : 32 * P, P == 32 ? 2 : 1)
     const bool live = k0 < s2 && x0 < n;
     const long long base = (long long)blockIdx.y * n * s2 + k0;
     uint32_t g[P];
-    const uint16_t *src = D + base + (long long)x0 * s2;
+    const T *src = D + base + (long long)x0 * s2;
+    if constexpr (sizeof(T) == 2) {
 #pragma unroll
-    for (int p = 0; p < P; p++) {
-        uint32_t c = 0xffffffffu;
-        if (live && x0 + p < n) {
-            if constexpr (VEC == 2)
-                c = __ldg(reinterpret_cast<const uint32_t *>(src + (long long)p * s2));
-            else
-                c = (uint32_t)__ldg(src + (long long)p * s2) | 0xffff0000u;
+        for (int p = 0; p < P; p++) {
+            uint32_t c = 0xffffffffu;
+            if (live && x0 + p < n) {
+                if constexpr (VEC == 2)
+                    c = __ldg(reinterpret_cast<const uint32_t *>(src + (long long)p * s2));
+                else
+                    c = (uint32_t)__ldg(src + (long long)p * s2) | 0xffff0000u;
+            }
+            g[p] = c;
         }
-        g[p] = c;
+#pragma unroll
+        for (int p = 0; p < P; p++)
+            g[p] = square2(g[p], shift);
+    } else {
+        float f[P][VEC];
+#pragma unroll
+        for (int p = 0; p < P; p++)
+#pragma unroll
+            for (int v = 0; v < VEC; v++)
+                f[p][v] = live && x0 + p < n ? __ldg(src + (long long)p * s2 + v) : FLT_MAX;
+#pragma unroll
+        for (int p = 0; p < P; p++)
+            g[p] = pack_heights(f[p][0], VEC == 2 ? f[p][VEC - 1] : FLT_MAX, inv_a);
     }
     uint32_t mx = 0;
 #pragma unroll
-    for (int p = 0; p < P; p++) {
-        g[p] = square2(g[p]);
+    for (int p = 0; p < P; p++)
         if (x0 + p < n)
             mx = max2(mx, g[p]);
-    }
     if (!live)
         mx = 0;
     if (VEC == 1)
         mx &= 0xffffu;
     // two steps per round: the neighbours' two end values on either side
-    for (uint32_t k = 1; k <= kMaxStep; k += 2) {
+    for (uint32_t k = 1; k <= (uint32_t)last; k += 2) {
         uint32_t *e = s_end + (size_t)((k >> 1) & 1) * nw * 4 * LN + l;
         e[(w * 4 + 0) * LN] = g[0];
         e[(w * 4 + 1) * LN] = g[1];
@@ -650,9 +677,8 @@ __global__ void __launch_bounds__(32 * kRowWarps, 4) k_par_rows(const float *__r
     uint32_t *row = s_rows + w * kWords;
     const long long pairs = (nrows + 1) >> 1;
     const bool vec4 = !(n & 3) && !((reinterpret_cast<uintptr_t>(fin) | reinterpret_cast<uintptr_t>(fout)) & 15);
-    auto pack = [&](float f0, float f1) -> uint32_t {
-        return pack_float2(fminf(fmul(f0, inv_a), (float)kBig), fminf(fmul(f1, inv_a), (float)kBig));
-    };
+    const uint32_t last = min(kMaxStep, (uint32_t)n - 1);
+    auto pack = [&](float f0, float f1) -> uint32_t { return pack_heights(f0, f1, inv_a); };
     auto slot = [](int c) { return c + c / P; };
     for (long long r = blockIdx.x * (long long)kRowWarps + w; r < pairs; r += (long long)gridDim.x * kRowWarps) {
         const bool two = 2 * r + 1 < nrows;
@@ -687,7 +713,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 4) k_par_rows(const float *__r
             if (x0 + p < n)
                 mx = max2(mx, g[p]);
         }
-        for (uint32_t k = 1; k <= kMaxStep; k += 2) {
+        for (uint32_t k = 1; k <= last; k += 2) {
             if (!__any_sync(0xffffffffu, hmax(mx) > k * k))
                 break;
             uint32_t l1 = __shfl_up_sync(0xffffffffu, g[P - 1], 1), l2 = __shfl_up_sync(0xffffffffu, g[P - 2], 1);
@@ -753,15 +779,38 @@ __global__ void __launch_bounds__(32 * kRowWarps, 4) k_par_rows(const float *__r
     }
 }
 
-bool lattice_ok(const int64_t *shape, const float *res, const pmg_axis_cfg *cfg)
+// log2 of the ratio of two power-of-two voxel sizes, -1 when a < b or it is too large
+static int size_shift(float a, float b)
 {
-    if (!(res[0] == res[1] && res[1] == res[2]) || !lin_ok((int)shape[0], cfg[0]) || shape[0] > kScanMaxLine)
-        return false;
-    return window_path_ok(res[1], (int)shape[1]) && window_path_ok(res[2], (int)shape[2]);
+    int ea = 0, eb = 0;
+    frexpf(a, &ea);
+    frexpf(b, &eb);
+    return ea < eb || ea - eb > kMaxShift ? -1 : ea - eb;
 }
 
-template <int P, int LN>
-static void cols_p(const uint16_t *D, float *out, int n0, int n, int s2, float a, int periodic, int wide,
+// Which passes run on the lattice, and from what (edt_internal.cuh).
+LatticePlan lattice_plan(const int64_t *shape, const float *res, const pmg_axis_cfg *cfg)
+{
+    LatticePlan P{};
+    const int n1 = (int)shape[1], n2 = (int)shape[2];
+    // (window_path_ok of one voxel: a power of two)
+    if (!window_path_ok(res[0], 1) || !window_path_ok(res[1], 1) || !window_path_ok(res[2], 1))
+        return P;
+    P.shift = size_shift(res[0], res[1]);
+    P.cols = n1 <= kScanMaxLine && P.shift >= 0;
+    P.counts = P.cols && lin_ok((int)shape[0], cfg[0]);
+    P.rows = n2 <= kScanMaxLine && size_shift(res[0], res[2]) >= 0 && size_shift(res[1], res[2]) >= 0;
+    // whether a finite value of a pass can reach kBig (counts reach n0, plus the
+    // wrapped part on a periodic axis)
+    const double m0 = (cfg[0].periodic ? 2.0 : 1.0) * (double)shape[0] * res[0];
+    const double m1 = m0 * m0 + (double)n1 * n1 * res[1] * res[1], m2 = m1 + (double)n2 * n2 * res[2] * res[2];
+    P.wide1 = m1 >= (double)kBig * res[1] * res[1];
+    P.wide2 = m2 >= (double)kBig * res[2] * res[2];
+    return P;
+}
+
+template <class T, int P, int LN>
+static void cols_p(const T *D, float *out, int n0, int n, int s2, float a, int shift, int last, int periodic, int wide,
                    uint16_t *flag, cudaStream_t st)
 {
     // whole warps (the last group may lie past the line's end)
@@ -769,11 +818,29 @@ static void cols_p(const uint16_t *D, float *out, int n0, int n, int s2, float a
     const size_t smem = (size_t)groups * 8 * LN * sizeof(uint32_t);
     const unsigned threads = (unsigned)(groups * LN);
     if (!(s2 & 1))
-        k_par_cols<P, 2, LN><<<dim3((unsigned)((s2 / 2 + LN - 1) / LN), (unsigned)n0), threads, smem, st>>>(
-            D, out, n, s2, a, periodic, wide, flag);
+        k_par_cols<T, P, 2, LN><<<dim3((unsigned)((s2 / 2 + LN - 1) / LN), (unsigned)n0), threads, smem, st>>>(
+            D, out, n, s2, a, 1.0f / a, shift, last, periodic, wide, flag);
     else
-        k_par_cols<P, 1, LN><<<dim3((unsigned)((s2 + LN - 1) / LN), (unsigned)n0), threads, smem, st>>>(
-            D, out, n, s2, a, periodic, wide, flag);
+        k_par_cols<T, P, 1, LN><<<dim3((unsigned)((s2 + LN - 1) / LN), (unsigned)n0), threads, smem, st>>>(
+            D, out, n, s2, a, 1.0f / a, shift, last, periodic, wide, flag);
+}
+
+template <class T>
+static int cols_run(const T *D, float *out, int n0, int n, int s2, float a, int shift, int last, int periodic, int wide,
+                    uint16_t *flag, cudaStream_t st)
+{
+    const int ps__ = prof_begin("k_par_cols", st);
+    if (n <= 64)
+        cols_p<T, 8, 32>(D, out, n0, n, s2, a, shift, last, periodic, wide, flag, st);
+    else if (n <= 256)
+        cols_p<T, 16, 32>(D, out, n0, n, s2, a, shift, last, periodic, wide, flag, st);
+    else if (n <= 512)
+        cols_p<T, 32, 32>(D, out, n0, n, s2, a, shift, last, periodic, wide, flag, st);
+    else
+        cols_p<T, 32, 16>(D, out, n0, n, s2, a, shift, last, periodic, wide, flag, st);
+    prof_end(ps__, (double)n0 * n * s2 * (sizeof(T) + 4), st);
+    PMG_CHECK_LAUNCH();
+    return PMG_OK;
 }
 
 template <int P>
@@ -786,57 +853,49 @@ static void rows_p(const float *fin, float *fout, long long nrows, int n, float 
                                                                                     periodic, wide, form, flag);
 }
 
-// The three passes: counts in `out`, the first envelope in `tmp`, the result
-// in `out`.  flags: one entry per line of the larger envelope pass.
-int lattice_run(const uint8_t *img, float *out, float *tmp, const int64_t *shape, const float *res,
-                const pmg_axis_cfg *cfg, int num_hull, int form, uint16_t *flags, cudaStream_t st)
+// Pass along axis 1 from counts or heights to `out`; flags: one entry per line.
+int lattice_cols(const LatticePlan &P, const void *in, float *out, const int64_t *shape, const float *res,
+                 const pmg_axis_cfg *cfg, int num_hull, uint16_t *flags, cudaStream_t st)
 {
     const int n0 = (int)shape[0], n1 = (int)shape[1], n2 = (int)shape[2];
-    const float a = res[0] * res[0];
-    uint16_t *D = (uint16_t *)out;
-    PMG_TRY(launch_lin_counts(img, D, shape, cfg[0], st));
-    // whether a finite value of a pass can reach kBig (counts reach n0, plus
-    // the wrapped part on a periodic axis)
-    const long long m0 = (cfg[0].periodic ? 2LL : 1LL) * n0, m1 = m0 * m0 + (long long)n1 * n1;
-    const int wide1 = m1 >= (long long)kBig, wide2 = m1 + (long long)n2 * n2 >= (long long)kBig;
-    {
-        const int per = cfg[1].periodic ? 1 : 0;
-        uint16_t *fl = per || wide1 ? flags : nullptr;
-        const int ps__ = prof_begin("k_par_cols", st);
-        if (n1 <= 64)
-            cols_p<8, 32>(D, tmp, n0, n1, n2, a, per, wide1, fl, st);
-        else if (n1 <= 256)
-            cols_p<16, 32>(D, tmp, n0, n1, n2, a, per, wide1, fl, st);
-        else if (n1 <= 512)
-            cols_p<32, 32>(D, tmp, n0, n1, n2, a, per, wide1, fl, st);
-        else
-            cols_p<32, 16>(D, tmp, n0, n1, n2, a, per, wide1, fl, st);
-        prof_end(ps__, (double)n0 * n1 * n2 * 6, st);
-        PMG_CHECK_LAUNCH();
-        if (fl)
-            PMG_TRY(launch_ends_counts(D, tmp, all_lines(shape, 1), res[1], cfg[1], num_hull, fl, st));
+    const float a = res[1] * res[1];
+    const int per = cfg[1].periodic ? 1 : 0, last = std::min((int)kMaxStep, n1 - 1);
+    uint16_t *fl = per || P.wide1 ? flags : nullptr;
+    if (P.counts) {
+        PMG_TRY(cols_run((const uint16_t *)in, out, n0, n1, n2, a, P.shift, last, per, P.wide1, fl, st));
+        return fl ? launch_ends_counts((const uint16_t *)in, out, all_lines(shape, 1), res[1], res[0], cfg[1], num_hull, fl,
+                                       st)
+                  : PMG_OK;
     }
-    {
-        const int per = cfg[2].periodic ? 1 : 0;
-        uint16_t *fl = per || wide2 ? flags : nullptr;
-        const long long nrows = (long long)n0 * n1;
-        const int ps__ = prof_begin("k_par_rows", st);
-        if (n2 <= 64)
-            rows_p<2>(tmp, out, nrows, n2, a, per, wide2, form, fl, st);
-        else if (n2 <= 128)
-            rows_p<4>(tmp, out, nrows, n2, a, per, wide2, form, fl, st);
-        else if (n2 <= 256)
-            rows_p<8>(tmp, out, nrows, n2, a, per, wide2, form, fl, st);
-        else if (n2 <= 512)
-            rows_p<16>(tmp, out, nrows, n2, a, per, wide2, form, fl, st);
-        else
-            rows_p<32>(tmp, out, nrows, n2, a, per, wide2, form, fl, st);
-        prof_end(ps__, (double)n0 * n1 * n2 * 8, st);
-        PMG_CHECK_LAUNCH();
-        if (fl)
-            PMG_TRY(launch_ends_heights(tmp, out, all_lines(shape, 2), res[2], cfg[2], num_hull, form, fl, st));
-    }
-    return PMG_OK;
+    PMG_TRY(cols_run((const float *)in, out, n0, n1, n2, a, 0, last, per, P.wide1, fl, st));
+    return fl ? launch_ends_heights((const float *)in, out, all_lines(shape, 1), res[1], cfg[1], num_hull, PMG_EDT_SQUARED,
+                                    fl, st)
+              : PMG_OK;
+}
+
+// Pass along axis 2.
+int lattice_rows(const LatticePlan &P, const float *in, float *out, const int64_t *shape, const float *res,
+                 const pmg_axis_cfg *cfg, int num_hull, int form, uint16_t *flags, cudaStream_t st)
+{
+    const int n2 = (int)shape[2];
+    const float a = res[2] * res[2];
+    const int per = cfg[2].periodic ? 1 : 0;
+    uint16_t *fl = per || P.wide2 ? flags : nullptr;
+    const long long nrows = (long long)shape[0] * shape[1];
+    const int ps__ = prof_begin("k_par_rows", st);
+    if (n2 <= 64)
+        rows_p<2>(in, out, nrows, n2, a, per, P.wide2, form, fl, st);
+    else if (n2 <= 128)
+        rows_p<4>(in, out, nrows, n2, a, per, P.wide2, form, fl, st);
+    else if (n2 <= 256)
+        rows_p<8>(in, out, nrows, n2, a, per, P.wide2, form, fl, st);
+    else if (n2 <= 512)
+        rows_p<16>(in, out, nrows, n2, a, per, P.wide2, form, fl, st);
+    else
+        rows_p<32>(in, out, nrows, n2, a, per, P.wide2, form, fl, st);
+    prof_end(ps__, (double)nrows * n2 * 8, st);
+    PMG_CHECK_LAUNCH();
+    return fl ? launch_ends_heights(in, out, all_lines(shape, 2), res[2], cfg[2], num_hull, form, fl, st) : PMG_OK;
 }
 
 } // namespace pmg
