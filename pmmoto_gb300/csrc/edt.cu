@@ -181,14 +181,6 @@ struct LineGlobal {
 // memory in between, as floats or as counts of voxels).
 constexpr int kEndWin = 32;
 
-__device__ __forceinline__ float height_of(const float *p, float) { return __ldg(p); }
-__device__ __forceinline__ float height_of(const uint16_t *p, float res)
-{
-    const uint32_t c = __ldg(p);
-    const float d = fmul((float)c, res);
-    return c >= 0x4000u ? FLT_MAX : fmul(d, d);
-}
-
 template <class T>
 struct LineEnds {
     const T *p;
@@ -580,12 +572,41 @@ __global__ void k_envelope(const float *__restrict__ fin, float *__restrict__ fo
     }
 }
 
-// Lines that a scan handed over (flag kScanWhole).
-__global__ void k_envelope_whole(const float *__restrict__ fin, float *__restrict__ fout, Lines Ls, float res,
-                                 pmg_axis_cfg cfg, int num_hull, int form, MorphEpi me,
-                                 const uint8_t *__restrict__ flag, const int *__restrict__ wide)
+// Lines that a scan or a lattice pass left to the envelope, or (wide) all of them.
+template <class T>
+struct LineOf {
+    const T *p;
+    long long st;
+    float res;
+    __device__ __forceinline__ float operator()(int v) const { return height_of(p + v * st, res); }
+    __device__ __forceinline__ LineOf from(int v) const { return {p + v * st, st, res}; }
+};
+
+// A solid on the line at all (a lattice pass flags every line with a voxel out of
+// its range).
+template <class L>
+__device__ __forceinline__ bool some_height(const L &line, int n)
+{
+    bool some = false;
+    for (int i = 0; i < n && !some; i += 8) {
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            some |= i + u < n && line(min(i + u, n - 1)) < FLT_MAX;
+    }
+    return some;
+}
+
+__device__ __forceinline__ bool whole_flag(uint8_t f) { return f & kScanWhole; }
+__device__ __forceinline__ bool whole_flag(uint16_t f) { return (f & 0xff) == kWholeLine; }
+
+template <class T, class F>
+__global__ void k_envelope_whole(const T *__restrict__ fin, float *__restrict__ fout, Lines Ls, float res, float resh,
+                                 pmg_axis_cfg cfg, int num_hull, int form, MorphEpi me, const F *__restrict__ flag,
+                                 const int *__restrict__ wide)
 {
     const bool all = wide && *wide;
+    if (!all && !flag)
+        return;
     const long long nlines = Ls.count();
     extern __shared__ uint32_t smem_bm[];
     const float aniso = fmul(res, res);
@@ -594,10 +615,19 @@ __global__ void k_envelope_whole(const float *__restrict__ fin, float *__restric
     S.nthr = blockDim.x;
     for (long long li = blockIdx.x * (long long)blockDim.x + threadIdx.x; li < nlines;
          li += (long long)gridDim.x * blockDim.x) {
-        if (!all && !(flag[li] & kScanWhole))
+        if (!all && !whole_flag(flag[li]))
             continue;
         const LineGeo g = line_addr(Ls, li);
-        envelope_line(S, LineGlobal{fin + g.base, g.stride}, g, aniso, cfg, num_hull, form, me, fout);
+        const LineOf<T> line{fin + g.base, g.stride, resh};
+        // (a scan flags no line without a height, and has no such outputs to write)
+        if (all || sizeof(F) == 1 || (cfg.periodic && (g.n - cfg.hf_lo < 2 || g.n - cfg.hb_hi < 2)) || some_height(line, g.n)) {
+            envelope_line(S, line, g, aniso, cfg, num_hull, form, me, fout);
+        } else {
+            const float none = form == PMG_EDT_DIST ? __fsqrt_rn(FLT_MAX) : FLT_MAX;
+#pragma unroll 8
+            for (int i = 0; i < g.n; i++)
+                fout[g.base + i * g.stride] = none;
+        }
     }
 }
 
@@ -618,8 +648,8 @@ __global__ void k_envelope_whole(const float *__restrict__ fin, float *__restric
 // line.  bm: this thread's envelope bits, nthr threads apart.
 template <class L>
 __device__ __noinline__ void replay_line(uint32_t *bm, int nthr, const L &line, const LineGeo &g, float aniso,
-                                         const pmg_axis_cfg &cfg, int num_hull, bool whole, int form,
-                                         const MorphEpi &me, float *fout, int part = 3)
+                                         const pmg_axis_cfg &cfg, int num_hull, int form, const MorphEpi &me,
+                                         float *fout, int part = 3)
 {
     Stack S;
     S.bm = bm;
@@ -643,7 +673,7 @@ __device__ __noinline__ void replay_line(uint32_t *bm, int nthr, const L &line, 
     int up_v[kMaxHull];
     float up_h[kMaxHull], up_r[kMaxHull];
     int n_up = 0;
-    whole = whole || z1 < 0;
+    const bool whole = z1 < 0;
     if (whole && part == 2)
         return;
     if (cfg.periodic && (whole || (part & 2)))
@@ -756,8 +786,7 @@ __global__ void __launch_bounds__(kEndBlock) k_envelope_ends(const float *__rest
         if (!ends)
             continue;
         const LineEnds<float> line{fin + g.base, g.stride, s_ends + lane, 33, g.n, 0, res};
-        replay_line(smem_bm + threadIdx.x, kEndBlock, line, g, fmul(res, res), cfg, num_hull, false, form, me, fout,
-                    1 << w);
+        replay_line(smem_bm + threadIdx.x, kEndBlock, line, g, fmul(res, res), cfg, num_hull, form, me, fout, 1 << w);
     }
 }
 
@@ -785,7 +814,7 @@ constexpr float kTall = 2097152.0f;  // tallest height (their products' differen
 template <class T>
 __global__ void __launch_bounds__(64) k_lattice_ends(const T *__restrict__ fin, float *__restrict__ fout, Lines Ls,
                                                      float res, float resh, pmg_axis_cfg cfg, int num_hull, int form,
-                                                     const uint16_t *__restrict__ flag)
+                                                     uint16_t *__restrict__ flag, int defer)
 {
     extern __shared__ uint32_t smem_bm[]; // envelope bits of the replays: [nwords][32]
     __shared__ float s_ends[2 * kEndWin * 33];
@@ -798,25 +827,24 @@ __global__ void __launch_bounds__(64) k_lattice_ends(const T *__restrict__ fin, 
         const int ra = (int)(t / tiles), kb = (int)(t - (long long)ra * tiles) * 32;
         const int lines = min(32, Ls.nb2 - kb);
         const long long l0 = (long long)ra * Ls.nb2 + kb;
-        const int fl = lane < lines ? flag[l0 + lane] : 0;
+        const int all = lane < lines ? flag[l0 + lane] : 0, fl = whole_flag((uint16_t)all) ? 0 : all;
         if (!__any_sync(0xffffffffu, fl)) // the same for both warps
             continue;
         const LineGeo g = line_addr(Ls, l0 + min(lane, lines - 1));
         const int n = g.n;
-        const bool whole = (fl & 0xff) == 255;
         __syncthreads(); // (the previous tile's readers)
         if (w == 0)
-            s_hard[lane] = whole;
+            s_hard[lane] = 0;
         stage_ends(s_ends, fin, Ls, l0, lines, g, resh, w, 2);
         __syncthreads();
         const LineEnds<T> line{fin + g.base, g.stride, s_ends + lane, 33, n, 0, resh};
-        const int reach = whole ? 0 : w == 0 ? fl & 0xff : fl >> 8;
+        const int reach = w == 0 ? fl & 0xff : fl >> 8;
         if (reach > 0) {
             // positions of the segment from its end that faces the line
             const int p0 = w == 0 ? n - cfg.hb_hi - 1 : cfg.hf_lo, dir = w == 0 ? -1 : 1;
             const int most = w == 0 ? n - cfg.hb_hi : n - cfg.hf_lo;
             // (a segment of one voxel without a solid one: the reference's phantom import)
-            bool hard = most < 2;
+            bool hard = most < 2, far = false; // far: out of this search's range
             // entries (position q, height K); q = -1: none
             int eq[kMaxHull], ek[kMaxHull];
 #pragma unroll
@@ -828,7 +856,7 @@ __global__ void __launch_bounds__(64) k_lattice_ends(const T *__restrict__ fin, 
                 // (a height beyond kTall leaves the line to the float replay: 32-bit products)
                 auto height = [&](int q) -> int {
                     const float f = line(p0 + dir * q), k = fmul(f, inv_a);
-                    hard = hard || (f < FLT_MAX && k > kTall);
+                    far = far || (f < FLT_MAX && k > kTall);
                     return f >= FLT_MAX || k > kTall ? -1 : (int)k;
                 };
                 int e = 0, ke = height(0);
@@ -851,7 +879,7 @@ __global__ void __launch_bounds__(64) k_lattice_ends(const T *__restrict__ fin, 
                         if (b < most && (d * d - ke) * db - nb * d > d * db)
                             break;
                         if (d > kWrapMax) {
-                            hard = true;
+                            far = true;
                             break;
                         }
                         const int k = height(q);
@@ -883,8 +911,8 @@ __global__ void __launch_bounds__(64) k_lattice_ends(const T *__restrict__ fin, 
                     }
                 }
             }
-            if (hard) {
-                s_hard[lane] = 1;
+            if (far || hard) {
+                atomicMax(&s_hard[lane], far ? 2 : 1);
             } else {
                 // import c lies eq[c] + 1 beyond the line's end
                 float *o = fout + g.base + (w == 0 ? 0 : n - 1) * g.stride;
@@ -915,37 +943,37 @@ __global__ void __launch_bounds__(64) k_lattice_ends(const T *__restrict__ fin, 
             }
         }
         __syncthreads();
-        if (w == 0 && s_hard[lane])
-            replay_line(smem_bm + lane, 32, line, g, aniso, cfg, num_hull, whole, form, MorphEpi{}, fout);
+        if (w > 0)
+            continue;
+        // many such lines: as a whole, by the kernel that follows
+        const int hard = s_hard[lane];
+        const bool many = defer && __popc(__ballot_sync(0xffffffffu, hard == 2)) >= 16;
+        if (many && hard == 2)
+            flag[l0 + lane] = kWholeLine;
+        else if (hard)
+            replay_line(smem_bm + lane, 32, line, g, aniso, cfg, num_hull, form, MorphEpi{}, fout);
     }
 }
 
 template <class T>
-static int launch_lattice_ends(const T *fin, float *fout, const Lines &Ls, float res, float resh,
-                               const pmg_axis_cfg &cfg, int num_hull, int form, const uint16_t *flag, cudaStream_t st)
+int launch_lattice_ends(const T *fin, float *fout, const Lines &Ls, float res, float res_height, const pmg_axis_cfg &cfg,
+                        int num_hull, int form, uint16_t *flag, int defer, cudaStream_t st)
 {
     const int n = (int)(Ls.ax == 0 ? Ls.s0 : Ls.ax == 1 ? Ls.s1 : Ls.s2);
     const size_t smem = (size_t)((n + 31) / 32) * 32 * 4;
     const long long tiles = (long long)Ls.nb1 * ((Ls.nb2 + 31) / 32);
     const int ps__ = prof_begin("k_lattice_ends", st);
-    k_lattice_ends<T><<<grid_for(tiles, 1, 152LL * 64), 64, smem, st>>>(fin, fout, Ls, res, resh, cfg, num_hull, form,
-                                                                          flag);
+    k_lattice_ends<T><<<grid_for(tiles, 1, 152LL * 64), 64, smem, st>>>(fin, fout, Ls, res, res_height, cfg, num_hull, form,
+                                                                          flag, defer);
     prof_end(ps__, 0.0, st);
     PMG_CHECK_LAUNCH();
     return PMG_OK;
 }
 
-int launch_ends_counts(const uint16_t *fin, float *fout, const Lines &Ls, float res, float res_count,
-                       const pmg_axis_cfg &cfg, int num_hull, const uint16_t *flag, cudaStream_t st)
-{
-    return launch_lattice_ends(fin, fout, Ls, res, res_count, cfg, num_hull, PMG_EDT_SQUARED, flag, st);
-}
-
-int launch_ends_heights(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
-                        int num_hull, int form, const uint16_t *flag, cudaStream_t st)
-{
-    return launch_lattice_ends(fin, fout, Ls, res, res, cfg, num_hull, form, flag, st);
-}
+template int launch_lattice_ends(const float *, float *, const Lines &, float, float, const pmg_axis_cfg &, int, int,
+                                 uint16_t *, int, cudaStream_t);
+template int launch_lattice_ends(const uint16_t *, float *, const Lines &, float, float, const pmg_axis_cfg &, int, int,
+                                 uint16_t *, int, cudaStream_t);
 
 int launch_ends_float(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
                       int num_hull, int form, const MorphEpi &me, const uint8_t *flag, const int *wide, cudaStream_t st)
@@ -987,6 +1015,25 @@ static int envelope_block(int n)
         block >>= 1;
     return block;
 }
+
+template <class T, class F>
+int launch_whole(const T *fin, float *fout, const Lines &Ls, float res, float res_height, const pmg_axis_cfg &cfg,
+                 int num_hull, int form, const MorphEpi &me, const F *flag, const int *wide, cudaStream_t st)
+{
+    const int n = (int)(Ls.ax == 0 ? Ls.s0 : Ls.ax == 1 ? Ls.s1 : Ls.s2), block = envelope_block(n);
+    const size_t smem = (size_t)((n + 31) / 32) * block * 4; // (48 KB at most)
+    const int ps__ = prof_begin("k_envelope_whole", st);
+    k_envelope_whole<<<grid_for(Ls.count(), block, 1LL << 30), block, smem, st>>>(fin, fout, Ls, res, res_height, cfg, num_hull,
+                                                                                 form, me, flag, wide);
+    prof_end(ps__, 0.0, st);
+    PMG_CHECK_LAUNCH();
+    return PMG_OK;
+}
+
+template int launch_whole(const float *, float *, const Lines &, float, float, const pmg_axis_cfg &, int, int,
+                          const MorphEpi &, const uint16_t *, const int *, cudaStream_t);
+template int launch_whole(const uint16_t *, float *, const Lines &, float, float, const pmg_axis_cfg &, int, int,
+                          const MorphEpi &, const uint16_t *, const int *, cudaStream_t);
 
 // power-of-two voxel size and lines of at most 1024 voxels (imported hull
 // vertices then stay within the exact float range of the reference's
@@ -1030,13 +1077,8 @@ int launch_envelope(const float *fin, float *fout, const Lines &Ls, float res,
             s = launch_scan(fin, fout, Ls, res, cfg, form, me, vcap, flag, wide, st);
         if (s == PMG_OK && cfg.periodic)
             s = launch_ends_float(fin, fout, Ls, res, cfg, num_hull, form, me, flag, wide, st);
-        if (s == PMG_OK) {
-            const int ps__ = prof_begin("k_envelope_whole", st);
-            k_envelope_whole<<<grid_for(nl, block, 1LL << 30), block, smem, st>>>(fin, fout, Ls, res, cfg, num_hull,
-                                                                                 form, me, flag, wide);
-            prof_end(ps__, 0.0, st);
-            s = cudaGetLastError() == cudaSuccess ? PMG_OK : PMG_ECUDA;
-        }
+        if (s == PMG_OK)
+            s = launch_whole(fin, fout, Ls, res, res, cfg, num_hull, form, me, flag, wide, st);
         const int s2 = flag_buf ? PMG_OK : scratch_free(flag, st);
         return s != PMG_OK ? s : s2;
     }

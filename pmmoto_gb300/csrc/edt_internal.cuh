@@ -1,6 +1,7 @@
 // Internal interface between the EDT kernels and their users (morphology).
 #pragma once
 
+#include <cfloat>
 #include <climits>
 #include <cmath>
 
@@ -49,6 +50,16 @@ __device__ __forceinline__ LineGeo line_addr(const Lines &L, long long li)
     }
     return g;
 }
+
+// Heights as they are, or as counts of voxels (0x4000 and more: none).
+__device__ __forceinline__ float height_of(const float *p, float) { return __ldg(p); }
+__device__ __forceinline__ float height_of(const uint16_t *p, float res)
+{
+    const uint32_t c = __ldg(p);
+    const float d = fmul((float)c, res);
+    return c >= 0x4000u ? FLT_MAX : fmul(d, d);
+}
+
 
 __host__ inline Lines all_lines(const int64_t *shape, int ax)
 {
@@ -210,19 +221,55 @@ struct LatticePlan {
     int shift;
 };
 LatticePlan lattice_plan(const int64_t *shape, const float *res, const pmg_axis_cfg *cfg);
+// (flags: one entry per line)
 int lattice_cols(const LatticePlan &P, const void *in, float *out, const int64_t *shape, const float *res,
                  const pmg_axis_cfg *cfg, int num_hull, uint16_t *flags, cudaStream_t st);
 int lattice_rows(const LatticePlan &P, const float *in, float *out, const int64_t *shape, const float *res,
                  const pmg_axis_cfg *cfg, int num_hull, int form, uint16_t *flags, cudaStream_t st);
-// Flagged lines: after a lattice pass over counts (of voxels of res_count) or
-// heights (line_reach), and after a scan (kScanEnds).
-int launch_ends_counts(const uint16_t *fin, float *fout, const Lines &Ls, float res, float res_count,
-                       const pmg_axis_cfg &cfg, int num_hull, const uint16_t *flag, cudaStream_t st);
-int launch_ends_heights(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
-                        int num_hull, int form, const uint16_t *flag, cudaStream_t st);
+// Flagged lines: after a lattice pass over heights or counts (of voxels of
+// res_height; line_reach), and after a scan (kScanEnds); the whole ones and, when
+// the probe chose so, all.
+template <class T>
+int launch_lattice_ends(const T *fin, float *fout, const Lines &Ls, float res, float res_height, const pmg_axis_cfg &cfg,
+                        int num_hull, int form, uint16_t *flag, int defer, cudaStream_t st);
+template <class T, class F>
+int launch_whole(const T *fin, float *fout, const Lines &Ls, float res, float res_height, const pmg_axis_cfg &cfg,
+                 int num_hull, int form, const MorphEpi &me, const F *flag, const int *wide, cudaStream_t st);
+constexpr int kWholeLine = 255; // (low byte of a lattice flag)
 int launch_ends_float(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg,
                       int num_hull, int form, const MorphEpi &me, const uint8_t *flag, const int *wide,
                       cudaStream_t st);
+// Passes whose kernel a probe in front of them chooses (device int, null: no
+// probe; nonzero: the float envelope takes every line) start while the probe
+// still runs: their first blocks load their lines before they wait for the
+// choice, which hides the probe (2 x 8 of 305 us of a 256^3 scan); the others find
+// it made.
+constexpr unsigned kFirstBlocks = 152 * 4;
+
+__device__ __forceinline__ bool left_to_envelope(const int *wide)
+{
+    cudaGridDependencySynchronize();
+    return wide && *(const volatile int *)wide;
+}
+
+// A launch that need not wait for the end of the probe before it.
+template <class... Args, class... Given>
+cudaError_t launch_after_probe(void (*kernel)(Args...), dim3 grid, unsigned block, size_t smem, cudaStream_t st,
+                               Given... args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Args>(args)...);
+}
+
 // The outward scan (edt_scan.cu), lines of at most kScanMaxLine voxels; vcap:
 // values above it only matter as "above it".  Line flags: the ends depend on
 // imported hulls; the whole line is left to the float envelope.  wide (device,

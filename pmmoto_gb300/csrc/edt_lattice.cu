@@ -438,8 +438,23 @@ int launch_lin_float(const uint8_t *img, float *out, const int64_t *shape, float
 // ---------------------------------------------------------------------------
 // Heights of kBig and more count as absent; kBig + 2 * kMaxStep stays below
 // 2^16, and (kMaxStep + 1)^2 is above every height below kBig.
-constexpr uint32_t kBig = 60000u, kMaxStep = 245u, kWholeLine = 255u;
+constexpr uint32_t kBig = 60000u, kMaxStep = 245u;
 constexpr uint32_t kBig2 = kBig * 0x10001u;
+
+// Wide pores: all steps take up to 17 ps a voxel (512^3: 2.3 ms a pass), and lines
+// with a voxel left out of range go to the float envelope (15 to 50 ps) all the
+// same.  So where most threads of a block (warp) still hold positions without any
+// height in range after 32 steps, or a quarter of them after 64, its lines are left
+// to the envelope at once (only where heights may exceed the range at all and the
+// line reaches beyond it).  512^3, both passes, ms, all steps and whole lines
+// afterwards, envelope alone, now: no solid 13.2, 3.8, 2.1; ball of radius 51 in the
+// middle 18.0, 9.8, 8.5; points 160 voxels apart 13.2, 6.0, 6.1, 40 apart 23.6, 14.1,
+// 14.0, 10 apart 2.6, 7.3, 2.6; cavity of radius 230 1.4, 4.8, 1.4.
+__device__ __forceinline__ bool bail_step(uint32_t k) { return k == 33 || k == 65; }
+__device__ __forceinline__ bool bail(uint32_t k, int lost, int threads)
+{
+    return k == 33 ? 4 * lost > 3 * threads : 4 * lost > threads;
+}
 
 // (count, count) -> (K, K), absent counts -> kBig; the counted voxels are 2^shift
 // of the pass's own (shift <= kMaxShift)
@@ -462,6 +477,17 @@ __device__ __forceinline__ float par_value(float k, float a) { return k >= (floa
 
 // larger of the two halves
 __device__ __forceinline__ uint32_t hmax(uint32_t v) { return max(v & 0xffffu, v >> 16); }
+
+// smallest value of P positions
+template <int P>
+__device__ __forceinline__ uint32_t hmin(const uint32_t (&g)[P])
+{
+    uint32_t m = g[0];
+#pragma unroll
+    for (int p = 1; p < P; p++)
+        m = min2(m, g[p]);
+    return min(m & 0xffffu, m >> 16);
+}
 
 // Steps k and k + 1 on P positions in registers, given the two values on
 // either side before step k; returns the maxima of the first `valid` results.
@@ -535,7 +561,7 @@ __device__ __forceinline__ uint32_t line_reach(const uint32_t (&g)[P], uint32_t 
                     hi1 = e;
             }
         }
-    if (big >= kBig && (periodic || wide)) {
+    if (big >= kBig && wide) {
         if ((mx & 0xffffu) >= kBig)
             lo0 = kWholeLine;
         if ((mx >> 16) >= kBig)
@@ -607,10 +633,21 @@ __global__ void __launch_bounds__(P == 32 ? 512 : 32 * P, P == 32 ? 2 : 1)
         e[(w * 4 + 1) * LN] = g[1];
         e[(w * 4 + 2) * LN] = g[P - 2];
         e[(w * 4 + 3) * LN] = g[P - 1];
-        const bool open = hmax(mx) > k * k;
+        if (wide && n > (int)kMaxStep && bail_step(k) && bail(k, __syncthreads_count(hmax(mx) >= kBig), (n + P - 1) / P * LN)) {
+            if (w == 0 && live) {
+                uint16_t *fl = flag + (long long)blockIdx.y * s2 + k0;
+                if constexpr (VEC == 2)
+                    *reinterpret_cast<uint32_t *>(fl) = kWholeLine * 0x10001u;
+                else
+                    *fl = kWholeLine;
+            }
+            return;
+        }
+        // (without any height in range on the lines, further steps change nothing)
+        const bool open = k == 33 ? hmin<P>(g) < kBig : hmax(mx) > k * k;
         if (!__syncthreads_or(open))
             break;
-        if (!__any_sync(0xffffffffu, open))
+        if (k != 33 && !__any_sync(0xffffffffu, open))
             continue; // this warp's values are final
         uint32_t l2 = kBig2, l1 = kBig2, r1 = kBig2, r2 = kBig2;
         if (w > 0) {
@@ -713,8 +750,12 @@ __global__ void __launch_bounds__(32 * kRowWarps, 4) k_par_rows(const float *__r
             if (x0 + p < n)
                 mx = max2(mx, g[p]);
         }
+        bool left = false; // to the envelope
         for (uint32_t k = 1; k <= last; k += 2) {
-            if (!__any_sync(0xffffffffu, hmax(mx) > k * k))
+            if (!__any_sync(0xffffffffu, k == 33 ? hmin<P>(g) < kBig : hmax(mx) > k * k))
+                break;
+            left = wide && n > (int)kMaxStep && bail_step(k) && bail(k, __popc(__ballot_sync(0xffffffffu, hmax(mx) >= kBig)), (n + P - 1) / P);
+            if (left)
                 break;
             uint32_t l1 = __shfl_up_sync(0xffffffffu, g[P - 1], 1), l2 = __shfl_up_sync(0xffffffffu, g[P - 2], 1);
             uint32_t r1 = __shfl_down_sync(0xffffffffu, g[0], 1), r2 = __shfl_down_sync(0xffffffffu, g[1], 1);
@@ -723,6 +764,12 @@ __global__ void __launch_bounds__(32 * kRowWarps, 4) k_par_rows(const float *__r
             if (lane == 31)
                 r1 = r2 = kBig2;
             mx = par_steps<P>(g, l2, l1, r1, r2, k, n - x0);
+        }
+        if (left) {
+            if (lane < (two ? 2 : 1))
+                flag[2 * r + lane] = kWholeLine;
+            __syncwarp();
+            continue;
         }
 #pragma unroll
         for (int p = 0; p < P; p++)
@@ -800,9 +847,9 @@ LatticePlan lattice_plan(const int64_t *shape, const float *res, const pmg_axis_
     P.cols = n1 <= kScanMaxLine && P.shift >= 0;
     P.counts = P.cols && lin_ok((int)shape[0], cfg[0]);
     P.rows = n2 <= kScanMaxLine && size_shift(res[0], res[2]) >= 0 && size_shift(res[1], res[2]) >= 0;
-    // whether a finite value of a pass can reach kBig (counts reach n0, plus the
-    // wrapped part on a periodic axis)
-    const double m0 = (cfg[0].periodic ? 2.0 : 1.0) * (double)shape[0] * res[0];
+    // whether a finite value of a pass can reach kBig (counts reach n0, or the
+    // correctors of a wrapped line, which are distances to one of its zeros)
+    const double m0 = ((double)shape[0] + (cfg[0].periodic ? std::max(0, std::max(cfg[0].a_u, cfg[0].a_l)) : 0)) * res[0];
     const double m1 = m0 * m0 + (double)n1 * n1 * res[1] * res[1], m2 = m1 + (double)n2 * n2 * res[2] * res[2];
     P.wide1 = m1 >= (double)kBig * res[1] * res[1];
     P.wide2 = m2 >= (double)kBig * res[2] * res[2];
@@ -853,24 +900,38 @@ static void rows_p(const float *fin, float *fout, long long nrows, int n, float 
                                                                                     periodic, wide, form, flag);
 }
 
-// Pass along axis 1 from counts or heights to `out`; flags: one entry per line.
+// What a lattice pass left over: the ends of periodic lines, and whole lines.
+template <class T>
+static int rest(const T *in, float *out, const Lines &Ls, float res, float resh, const pmg_axis_cfg &cfg, int num_hull,
+                int form, uint16_t *flag, int whole, cudaStream_t st)
+{
+    if (cfg.periodic)
+        PMG_TRY(launch_lattice_ends(in, out, Ls, res, resh, cfg, num_hull, form, flag, whole, st));
+    return whole ? launch_whole(in, out, Ls, res, resh, cfg, num_hull, form, MorphEpi{}, flag, nullptr, st) : PMG_OK;
+}
+
+// (a hull segment of one voxel without a solid gives the reference's phantom
+// import: its lines are whole ones)
+static bool phantom(const pmg_axis_cfg &c, int n) { return c.periodic && (n - c.hf_lo < 2 || n - c.hb_hi < 2); }
+
+// Pass along axis 1 from counts or heights to `out`.
 int lattice_cols(const LatticePlan &P, const void *in, float *out, const int64_t *shape, const float *res,
                  const pmg_axis_cfg *cfg, int num_hull, uint16_t *flags, cudaStream_t st)
 {
     const int n0 = (int)shape[0], n1 = (int)shape[1], n2 = (int)shape[2];
     const float a = res[1] * res[1];
     const int per = cfg[1].periodic ? 1 : 0, last = std::min((int)kMaxStep, n1 - 1);
-    uint16_t *fl = per || P.wide1 ? flags : nullptr;
+    const int whole = P.wide1 || phantom(cfg[1], n1);
+    uint16_t *fl = per || whole ? flags : nullptr;
+    const Lines Ls = all_lines(shape, 1);
     if (P.counts) {
-        PMG_TRY(cols_run((const uint16_t *)in, out, n0, n1, n2, a, P.shift, last, per, P.wide1, fl, st));
-        return fl ? launch_ends_counts((const uint16_t *)in, out, all_lines(shape, 1), res[1], res[0], cfg[1], num_hull, fl,
-                                       st)
-                  : PMG_OK;
+        const uint16_t *D = (const uint16_t *)in;
+        PMG_TRY(cols_run(D, out, n0, n1, n2, a, P.shift, last, per, whole, fl, st));
+        return rest(D, out, Ls, res[1], res[0], cfg[1], num_hull, PMG_EDT_SQUARED, fl, whole, st);
     }
-    PMG_TRY(cols_run((const float *)in, out, n0, n1, n2, a, 0, last, per, P.wide1, fl, st));
-    return fl ? launch_ends_heights((const float *)in, out, all_lines(shape, 1), res[1], cfg[1], num_hull, PMG_EDT_SQUARED,
-                                    fl, st)
-              : PMG_OK;
+    const float *D = (const float *)in;
+    PMG_TRY(cols_run(D, out, n0, n1, n2, a, 0, last, per, whole, fl, st));
+    return rest(D, out, Ls, res[1], res[1], cfg[1], num_hull, PMG_EDT_SQUARED, fl, whole, st);
 }
 
 // Pass along axis 2.
@@ -879,23 +940,23 @@ int lattice_rows(const LatticePlan &P, const float *in, float *out, const int64_
 {
     const int n2 = (int)shape[2];
     const float a = res[2] * res[2];
-    const int per = cfg[2].periodic ? 1 : 0;
-    uint16_t *fl = per || P.wide2 ? flags : nullptr;
+    const int per = cfg[2].periodic ? 1 : 0, whole = P.wide2 || phantom(cfg[2], n2);
+    uint16_t *fl = per || whole ? flags : nullptr;
     const long long nrows = (long long)shape[0] * shape[1];
     const int ps__ = prof_begin("k_par_rows", st);
     if (n2 <= 64)
-        rows_p<2>(in, out, nrows, n2, a, per, P.wide2, form, fl, st);
+        rows_p<2>(in, out, nrows, n2, a, per, whole, form, fl, st);
     else if (n2 <= 128)
-        rows_p<4>(in, out, nrows, n2, a, per, P.wide2, form, fl, st);
+        rows_p<4>(in, out, nrows, n2, a, per, whole, form, fl, st);
     else if (n2 <= 256)
-        rows_p<8>(in, out, nrows, n2, a, per, P.wide2, form, fl, st);
+        rows_p<8>(in, out, nrows, n2, a, per, whole, form, fl, st);
     else if (n2 <= 512)
-        rows_p<16>(in, out, nrows, n2, a, per, P.wide2, form, fl, st);
+        rows_p<16>(in, out, nrows, n2, a, per, whole, form, fl, st);
     else
-        rows_p<32>(in, out, nrows, n2, a, per, P.wide2, form, fl, st);
+        rows_p<32>(in, out, nrows, n2, a, per, whole, form, fl, st);
     prof_end(ps__, (double)nrows * n2 * 8, st);
     PMG_CHECK_LAUNCH();
-    return fl ? launch_ends_heights(in, out, all_lines(shape, 2), res[2], cfg[2], num_hull, form, fl, st) : PMG_OK;
+    return rest(in, out, all_lines(shape, 2), res[2], res[2], cfg[2], num_hull, form, fl, whole, st);
 }
 
 } // namespace pmg

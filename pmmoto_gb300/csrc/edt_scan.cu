@@ -162,17 +162,6 @@ __device__ __forceinline__ float scan_voxel(const float *line, int n, int x, int
     return m;
 }
 
-// A scan starts while the probe in front of it still runs (launch_after_probe):
-// its first blocks load their lines before they wait for the choice, which hides
-// the probe (2 x 8 of 305 us of a 256^3 field); the others find it made.
-constexpr unsigned kFirstBlocks = 152 * 4;
-
-__device__ __forceinline__ bool left_to_envelope(const int *wide)
-{
-    cudaGridDependencySynchronize();
-    return wide && *(const volatile int *)wide;
-}
-
 // Strided lines (axis 0 or 1): one block per 32 adjacent lines, warp w on
 // positions w, w + 8, ...
 __global__ void __launch_bounds__(32 * kScanWarps) k_scan_cols(const float *__restrict__ fin, float *__restrict__ fout,
@@ -286,7 +275,7 @@ constexpr int kProbeBlocks = 8, kProbeThreads = 512, kProbeGroups = kProbeBlocks
 __global__ void __cluster_dims__(kProbeBlocks, 1, 1) __launch_bounds__(kProbeThreads)
     k_pore_probe(const float *__restrict__ fin, Lines Ls, float a, float inv_a, float most, float budget, int *wide)
 {
-    cudaTriggerProgrammaticLaunchCompletion(); // (the scan may start: its first blocks wait)
+    cudaTriggerProgrammaticLaunchCompletion(); // (the pass may start: its first blocks wait)
     __shared__ unsigned s_sum;
     const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     const int lane = threadIdx.x & 31;
@@ -362,24 +351,6 @@ int launch_pore_probe(const float *fin, const Lines &Ls, float res, float vcap, 
     return PMG_OK;
 }
 
-// A launch that need not wait for the end of the kernel before it.
-template <class... Args>
-static cudaError_t launch_after_probe(void (*kernel)(Args...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
-                                      Args... args)
-{
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 int launch_scan(const float *fin, float *fout, const Lines &Ls, float res, const pmg_axis_cfg &cfg, int form,
                 const MorphEpi &me, float vcap, uint8_t *flag, const int *wide, cudaStream_t st)
 {
@@ -390,7 +361,7 @@ int launch_scan(const float *fin, float *fout, const Lines &Ls, float res, const
         const int ps__ = prof_begin("k_scan_rows", st);
         const unsigned grid = grid_for(Ls.count(), kScanWarps, 152LL * 64);
         if (wide)
-            PMG_CUDA(launch_after_probe(k_scan_rows, grid, 32 * kScanWarps, smem, st, fin, fout, Ls, a, inv_a, per, form, me,
+            PMG_CUDA(launch_after_probe(k_scan_rows, dim3(grid), 32 * kScanWarps, smem, st, fin, fout, Ls, a, inv_a, per, form, me,
                                         vcap, flag, wide));
         else
             k_scan_rows<<<grid, 32 * kScanWarps, smem, st>>>(fin, fout, Ls, a, inv_a, per, form, me, vcap, flag, wide);
@@ -403,7 +374,7 @@ int launch_scan(const float *fin, float *fout, const Lines &Ls, float res, const
         const long long blocks = (long long)Ls.nb1 * ((Ls.nb2 + 31) / 32);
         const int ps__ = prof_begin("k_scan_cols", st);
         if (wide)
-            PMG_CUDA(launch_after_probe(k_scan_cols, (unsigned)blocks, 32 * kScanWarps, smem, st, fin, fout, Ls, a, inv_a, per,
+            PMG_CUDA(launch_after_probe(k_scan_cols, dim3((unsigned)blocks), 32 * kScanWarps, smem, st, fin, fout, Ls, a, inv_a, per,
                                         form, me, vcap, flag, wide));
         else
             k_scan_cols<<<(unsigned)blocks, 32 * kScanWarps, smem, st>>>(fin, fout, Ls, a, inv_a, per, form, me, vcap, flag,

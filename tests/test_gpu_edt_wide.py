@@ -36,15 +36,16 @@ def _kernels():
 
 
 @pytest.mark.parametrize("medium", sorted(MEDIA))
-@pytest.mark.parametrize("res", [(2.25,) * 3, (1.0, 1.0, 2.0)])
-def test_wide_pores_cost_no_more_than_the_float_envelope(medium, res):
-    """No more than twice its time (a scan of this size takes 5 to 30 times)."""
+@pytest.mark.parametrize("res,n", [((2.25,) * 3, 256), ((1.0, 1.0, 2.0), 256), ((1.0,) * 3, 512)])
+def test_wide_pores_cost_no_more_than_the_float_envelope(medium, res, n):
+    """No more than twice its time (scans of this size alone take 5 to 30 times as
+    long, all steps of the lattice up to 3 times)."""
     import torch
 
     from pmmoto_gb300 import tune
     from pmmoto_gb300.filters import distance as D
 
-    img = torch.as_tensor(MEDIA[medium]((256, 256, 256)), device="cuda")
+    img = torch.as_tensor(MEDIA[medium]((n, n, n)), device="cuda")
     best, got = {}, {}
     try:
         for path in (0, 2):
@@ -114,3 +115,23 @@ def test_far_near_ties_on_long_lines_vs_oracle(res):
                                       O.edt3d(img.transpose(0, 2, 1).copy(), resolution=(res[0], res[2], res[1]), squared=True))
     finally:
         tune._set_lib("edt.wide", -1)
+
+
+@pytest.mark.parametrize("shape", [(5, 300, 520), (7, 520, 299), (300, 260, 12)])
+@pytest.mark.parametrize("per", [(False,) * 3, (True,) * 3, (False, True, False)])
+def test_lattice_lines_left_to_the_envelope_vs_oracle(shape, per):
+    """Power-of-two voxels: lines longer than a lattice pass reaches with few solids
+    or none, beside lines with many, so that blocks give up their lines early, late
+    or not at all."""
+    from pmmoto_gb300.filters import distance as D
+
+    rng = np.random.default_rng(sum(shape))
+    media = [_points(shape, 1e-4, 7), _points(shape, 3e-6, 8), np.ones(shape, np.uint8)]
+    half = np.ones(shape, np.uint8)  # dense in one corner, a single solid in the far half
+    half[:, : shape[1] // 4, : shape[2] // 3] = rng.random((shape[0], shape[1] // 4, shape[2] // 3)) >= 0.1
+    half[shape[0] // 2, -2, -3] = 0
+    for img in media + [half]:
+        for res in ((1.0,) * 3, (2.0, 1.0, 1.0)):
+            for squared in (True, False):
+                np.testing.assert_array_equal(D.edt3d(img, periodic=per, resolution=res, squared=squared),
+                                              O.edt3d(img, periodic=per, resolution=res, squared=squared))
