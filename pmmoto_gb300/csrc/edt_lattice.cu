@@ -450,10 +450,11 @@ constexpr uint32_t kBig2 = kBig * 0x10001u;
 // afterwards, envelope alone, now: no solid 13.2, 3.8, 2.1; ball of radius 51 in the
 // middle 18.0, 9.8, 8.5; points 160 voxels apart 13.2, 6.0, 6.1, 40 apart 23.6, 14.1,
 // 14.0, 10 apart 2.6, 7.3, 2.6; cavity of radius 230 1.4, 4.8, 1.4.
-__device__ __forceinline__ bool bail_step(uint32_t k) { return k == 33 || k == 65; }
-__device__ __forceinline__ bool bail(uint32_t k, int lost, int threads)
+__device__ __forceinline__ uint32_t first_stop(uint32_t last) { return min(last, 31u); }
+__device__ __forceinline__ uint32_t next_stop(uint32_t stop, uint32_t last) { return stop < 32 ? min(last, 63u) : last; }
+__device__ __forceinline__ bool give_up(uint32_t stop, int lost, int threads)
 {
-    return k == 33 ? 4 * lost > 3 * threads : 4 * lost > threads;
+    return stop < 32 ? 4 * lost > 3 * threads : 4 * lost > threads;
 }
 
 // (count, count) -> (K, K), absent counts -> kBig; the counted voxels are 2^shift
@@ -633,21 +634,23 @@ __global__ void __launch_bounds__(P == 32 ? 512 : 32 * P, P == 32 ? 2 : 1)
         e[(w * 4 + 1) * LN] = g[1];
         e[(w * 4 + 2) * LN] = g[P - 2];
         e[(w * 4 + 3) * LN] = g[P - 1];
-        if (wide && n > (int)kMaxStep && bail_step(k) && bail(k, __syncthreads_count(hmax(mx) >= kBig), (n + P - 1) / P * LN)) {
-            if (w == 0 && live) {
-                uint16_t *fl = flag + (long long)blockIdx.y * s2 + k0;
-                if constexpr (VEC == 2)
-                    *reinterpret_cast<uint32_t *>(fl) = kWholeLine * 0x10001u;
-                else
-                    *fl = kWholeLine;
-            }
-            return;
-        }
-        // (without any height in range on the lines, further steps change nothing)
-        const bool open = k == 33 ? hmin<P>(g) < kBig : hmax(mx) > k * k;
+        const bool open = hmax(mx) > k * k;
         if (!__syncthreads_or(open))
             break;
-        if (k != 33 && !__any_sync(0xffffffffu, open))
+        if (wide && n > (int)kMaxStep && (k == 33 || k == 65)) {
+            const int lost = __syncthreads_count(hmax(mx) >= kBig);
+            if (give_up(k - 2, lost, (n + P - 1) / P * LN)) {
+                if (w == 0 && live) {
+                    uint16_t *fl = flag + (long long)blockIdx.y * s2 + k0;
+                    if constexpr (VEC == 2)
+                        *reinterpret_cast<uint32_t *>(fl) = kWholeLine * 0x10001u;
+                    else
+                        *fl = kWholeLine;
+                }
+                return;
+            }
+        }
+        if (!__any_sync(0xffffffffu, open))
             continue; // this warp's values are final
         uint32_t l2 = kBig2, l1 = kBig2, r1 = kBig2, r2 = kBig2;
         if (w > 0) {
@@ -751,19 +754,27 @@ __global__ void __launch_bounds__(32 * kRowWarps, 4) k_par_rows(const float *__r
                 mx = max2(mx, g[p]);
         }
         bool left = false; // to the envelope
-        for (uint32_t k = 1; k <= last; k += 2) {
-            if (!__any_sync(0xffffffffu, k == 33 ? hmin<P>(g) < kBig : hmax(mx) > k * k))
+        uint32_t k = 1;
+        for (uint32_t stop = first_stop(last);; stop = next_stop(stop, last)) {
+            bool done = false;
+            for (; k <= stop; k += 2) {
+                done = !__any_sync(0xffffffffu, hmax(mx) > k * k);
+                if (done)
+                    break;
+                uint32_t l1 = __shfl_up_sync(0xffffffffu, g[P - 1], 1), l2 = __shfl_up_sync(0xffffffffu, g[P - 2], 1);
+                uint32_t r1 = __shfl_down_sync(0xffffffffu, g[0], 1), r2 = __shfl_down_sync(0xffffffffu, g[1], 1);
+                if (lane == 0)
+                    l1 = l2 = kBig2;
+                if (lane == 31)
+                    r1 = r2 = kBig2;
+                mx = par_steps<P>(g, l2, l1, r1, r2, k, n - x0);
+            }
+            if (done || k > last)
                 break;
-            left = wide && n > (int)kMaxStep && bail_step(k) && bail(k, __popc(__ballot_sync(0xffffffffu, hmax(mx) >= kBig)), (n + P - 1) / P);
-            if (left)
+            left = wide && n > (int)kMaxStep &&
+                   give_up(stop, __popc(__ballot_sync(0xffffffffu, hmax(mx) >= kBig)), (n + P - 1) / P);
+            if (left || !__any_sync(0xffffffffu, hmin<P>(g) < kBig))
                 break;
-            uint32_t l1 = __shfl_up_sync(0xffffffffu, g[P - 1], 1), l2 = __shfl_up_sync(0xffffffffu, g[P - 2], 1);
-            uint32_t r1 = __shfl_down_sync(0xffffffffu, g[0], 1), r2 = __shfl_down_sync(0xffffffffu, g[1], 1);
-            if (lane == 0)
-                l1 = l2 = kBig2;
-            if (lane == 31)
-                r1 = r2 = kBig2;
-            mx = par_steps<P>(g, l2, l1, r1, r2, k, n - x0);
         }
         if (left) {
             if (lane < (two ? 2 : 1))

@@ -322,12 +322,16 @@ __global__ void __cluster_dims__(kProbeBlocks, 1, 1) __launch_bounds__(kProbeThr
 // 96^3: 0.25, 0.51, 0.25.  On periodic lines the ends are replayed after a scan, so
 // the crossing lies lower (voxels 1 x 1 x 2, 512^3 field of sigma 4: 3.5, 5.5, 3.5;
 // sigma 20: 12.7, 8.6, 8.6).
-static float scan_budget(const Lines &Ls, int periodic)
+// Below five million voxels the two lie close together whatever the distances, and
+// the probes would cost more (2 x 2 us of 70 at four million).
+static float scan_budget(const Lines &Ls, int n, int periodic)
 {
     const float nl = (float)Ls.count();
     const int k = tune_value(kTuneEdtWide); // 1024: as it is; 0: always the envelope, 8193: never
-    if (k == 0 || k > 8192)
-        return k == 0 ? -1.0f : INFINITY;
+    if (k == 0)
+        return -1.0f;
+    if (k > 8192 || (!periodic && nl * (float)n < 5e6f))
+        return INFINITY;
     return (periodic ? std::max(5.0f, 0.22e6f / nl) : std::max(36.0f, 3.6e6f / nl)) * ((float)k / 1024.0f);
 }
 
@@ -339,7 +343,7 @@ int launch_pore_probe(const float *fin, const Lines &Ls, float res, float vcap, 
     const float a = res * res, inv_a = 1.0f / a;
     const int n = (int)(Ls.ax == 0 ? Ls.s0 : Ls.ax == 1 ? Ls.s1 : Ls.s2);
     // the most steps of a voxel: to the line's end, or to the cap
-    const float most = std::fmin((float)n, std::sqrt(vcap * inv_a) + 1.0f), budget = scan_budget(Ls, periodic);
+    const float most = std::fmin((float)n, std::sqrt(vcap * inv_a) + 1.0f), budget = scan_budget(Ls, n, periodic);
     *choice = nullptr;
     if (most <= budget)
         return PMG_OK;
