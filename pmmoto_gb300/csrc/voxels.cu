@@ -15,6 +15,7 @@
 //  * pmg_count_eq / pmg_max_f32 -- the scalar reductions behind porosity,
 //    saturation, phase_exists and PorousMedia.max_distance.
 #include <cfloat>
+#include <climits>
 #include <cstring>
 
 #include "pmg_common.cuh"
@@ -78,16 +79,38 @@ struct Halo {
     int wall_lo[3], wall_hi[3];
 };
 
-// One warp per row: rows of a halo or wall plane are written whole, of the others
-// only the columns outside the own region and on wall planes.
+// Rows by groups of 2^shift lanes: a warp, or a part of one where rows are short
+// (halo update of 4000 x 2000 rows of six voxels: 1.86 ms with a warp and a 64-bit
+// division each, now 0.22 ms).
+struct Rows {
+    int shift;
+    FastDiv q1; // division by the rows of a plane, of row numbers below 2^32
+    long long n1;
+    __device__ __forceinline__ void split(long long r, long long &i, long long &j) const
+    {
+        i = r >> 32 ? r / n1 : (long long)fdiv((unsigned)r, q1);
+        j = r - i * n1;
+    }
+};
+
+static Rows rows_of(long long n1, long long len)
+{
+    int shift = 5;
+    while (shift > 2 && len <= 1 << (shift - 1))
+        shift--;
+    return Rows{shift, fastdiv_of((unsigned)(n1 < INT_MAX ? n1 : INT_MAX)), n1};
+}
+
+// Rows of a halo or wall plane are written whole, of the others only the columns
+// outside the own region and on wall planes.
 // Bound by the rows' bookkeeping: a thread per voxel spent 0.64 ms at 512^3 on
 // three divisions each.
 template <typename T>
-__global__ void __launch_bounds__(256) k_update_buffer(T *img, Halo H)
+__global__ void __launch_bounds__(256) k_update_buffer(T *img, Halo H, Rows R)
 {
     const long long S1 = H.s[1], S2 = H.s[2], rows = H.s[0] * S1;
-    const int lane = threadIdx.x & 31;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+    const int lanes = 1 << R.shift, lane = threadIdx.x & (lanes - 1);
+    const long long ngroups = ((long long)gridDim.x * blockDim.x) >> R.shift;
     // coordinate c of axis d: t the own one it copies; false when there is none
     auto source = [&](int d, long long c, long long &t, bool &halo) {
         t = c;
@@ -95,15 +118,21 @@ __global__ void __launch_bounds__(256) k_update_buffer(T *img, Halo H)
             return true;
         if (!H.periodic[d] || H.own_len[d] <= 0)
             return false; // reservoir or end/wall halo: no neighbour copy
-        long long q = (c - H.own_lo[d]) % H.own_len[d];
+        // (mostly within a period on either side: a 64-bit division otherwise)
+        long long q = c - H.own_lo[d];
+        if (q < -H.own_len[d] || q >= 2LL * H.own_len[d])
+            q %= H.own_len[d];
         if (q < 0)
             q += H.own_len[d];
+        else if (q >= H.own_len[d])
+            q -= H.own_len[d];
         t = q + H.own_lo[d];
         halo = true;
         return true;
     };
-    for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; r < rows; r += nwarps) {
-        const long long c0 = r / S1, c1 = r - c0 * S1;
+    for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> R.shift; r < rows; r += ngroups) {
+        long long c0, c1;
+        R.split(r, c0, c1);
         const bool wall_row = (H.wall_lo[0] && c0 == 0) || (H.wall_hi[0] && c0 == H.s[0] - 1) ||
                               (H.wall_lo[1] && c1 == 0) || (H.wall_hi[1] && c1 == S1 - 1);
         long long t0, t1;
@@ -122,13 +151,13 @@ __global__ void __launch_bounds__(256) k_update_buffer(T *img, Halo H)
                 row[k] = src[t2];
         };
         if (wall_row || (halo && ok)) {
-            for (long long k = lane; k < S2; k += 32)
+            for (long long k = lane; k < S2; k += lanes)
                 put(k);
         } else {
             const long long lo = H.own_lo[2], hi = lo + H.own_len[2];
-            for (long long k = lane; k < lo; k += 32)
+            for (long long k = lane; k < lo; k += lanes)
                 put(k);
-            for (long long k = hi + lane; k < S2; k += 32)
+            for (long long k = hi + lane; k < S2; k += lanes)
                 put(k);
             // wall planes inside the own region
             if (lane == 0 && H.wall_lo[2] && lo == 0)
@@ -162,19 +191,23 @@ __global__ void k_count_eq(const uint8_t *__restrict__ img, long long s1, long l
         atomicAdd(cnt, (unsigned long long)c);
 }
 
-// One warp per row of the box (a thread per voxel was bound by its divisions:
-// 0.70 ms at 512^3).
+// By the rows of the box (a thread per voxel was bound by its divisions: 0.70 ms at
+// 512^3).
+template <bool WARP>
 __global__ void __launch_bounds__(256) k_max_f32(const float *__restrict__ x, long long s1, long long s2, long long lo0,
                                                  long long n0, long long lo1, long long n1, long long lo2,
-                                                 long long n2, unsigned int *best)
+                                                 long long n2, Rows R, unsigned int *best)
 {
-    const long long rows = n0 * n1, nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+    const int shift = WARP ? 5 : R.shift;
+    const long long rows = n0 * n1, ngroups = ((long long)gridDim.x * blockDim.x) >> shift;
+    const int lanes = WARP ? 32 : 1 << R.shift;
     float m = -FLT_MAX;
-    for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; r < rows; r += nwarps) {
-        const long long i = r / n1, j = r - i * n1;
+    for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> shift; r < rows; r += ngroups) {
+        long long i, j;
+        R.split(r, i, j);
         const float *row = x + ((lo0 + i) * s1 + lo1 + j) * s2 + lo2;
 #pragma unroll 8
-        for (long long k = threadIdx.x & 31; k < n2; k += 32)
+        for (long long k = threadIdx.x & (lanes - 1); k < n2; k += lanes)
             m = fmaxf(m, row[k]);
     }
     for (int o = 16; o > 0; o >>= 1)
@@ -205,23 +238,25 @@ int update_buffer_run(void *img, int elem_bytes, const int64_t *shape, const int
                       const int32_t *pad, cudaStream_t st)
 {
     const Halo H = make_halo(shape, bc, pad);
-    const unsigned g = grid_for(shape[0] * shape[1] * 32, 256, 152LL * 64);
+    // (most rows only have a column or two to write)
+    const Rows R = rows_of(shape[1], shape[2] > 64 ? 32 : 4);
+    const unsigned g = grid_for((shape[0] * shape[1]) << R.shift, 256, 152LL * 64);
     if (elem_bytes == 1)
         {
             const int ps__ = prof_begin("k_update_buffer", st);
-            k_update_buffer<uint8_t><<<g, 256, 0, st>>>((uint8_t *)img, H);
+            k_update_buffer<uint8_t><<<g, 256, 0, st>>>((uint8_t *)img, H, R);
             prof_end(ps__, 0.0, st);
         }
     else if (elem_bytes == 4)
         {
             const int ps__ = prof_begin("k_update_buffer", st);
-            k_update_buffer<float><<<g, 256, 0, st>>>((float *)img, H);
+            k_update_buffer<float><<<g, 256, 0, st>>>((float *)img, H, R);
             prof_end(ps__, 0.0, st);
         }
     else if (elem_bytes == 8)
         {
             const int ps__ = prof_begin("k_update_buffer", st);
-            k_update_buffer<uint64_t><<<g, 256, 0, st>>>((uint64_t *)img, H);
+            k_update_buffer<uint64_t><<<g, 256, 0, st>>>((uint64_t *)img, H, R);
             prof_end(ps__, 0.0, st);
         }
     else {
@@ -341,9 +376,11 @@ extern "C" int pmg_max_f32(const float *x, const int64_t shape[3], const int64_t
     const long long n0 = box[1] - box[0], n1 = box[3] - box[2], n2 = box[5] - box[4];
     if (n0 > 0 && n1 > 0 && n2 > 0) {
         {
+            const Rows R = rows_of(n1, n2);
             const int ps__ = prof_begin("k_max_f32", st);
-            k_max_f32<<<grid_for(n0 * n1 * 32, 256, 152LL * 16), 256, 0, st>>>(x, shape[1], shape[2], box[0], n0,
-                                                                         box[2], n1, box[4], n2, d);
+            auto *kernel = R.shift == 5 ? k_max_f32<true> : k_max_f32<false>;
+            kernel<<<grid_for((n0 * n1) << R.shift, 256, 152LL * 16), 256, 0, st>>>(x, shape[1], shape[2], box[0], n0, box[2],
+                                                                                 n1, box[4], n2, R, d);
             prof_end(ps__, (double)(n0 * n1 * n2) * 4, st);
         }
         PMG_CHECK_LAUNCH();
