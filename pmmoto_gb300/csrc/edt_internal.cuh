@@ -226,6 +226,9 @@ int lattice_cols(const LatticePlan &P, const void *in, float *out, const int64_t
                  const pmg_axis_cfg *cfg, int num_hull, uint16_t *flags, cudaStream_t st);
 int lattice_rows(const LatticePlan &P, const float *in, float *out, const int64_t *shape, const float *res,
                  const pmg_axis_cfg *cfg, int num_hull, int form, uint16_t *flags, cudaStream_t st);
+bool cols_capped_ok(const int64_t *X, float res, int T);
+int launch_cols_capped(const float *fin, float *fout, const int64_t *X, int lo, int planes, float res, int T,
+                       cudaStream_t st);
 // Flagged lines: after a lattice pass over heights or counts (of voxels of
 // res_height; line_reach), and after a scan (kScanEnds); the whole ones and, when
 // the probe chose so, all.

@@ -911,6 +911,25 @@ static void rows_p(const float *fin, float *fout, long long nrows, int n, float 
                                                                                     periodic, wide, form, flag);
 }
 
+// Pass along axis 1 of planes [lo, lo + planes) of a volume X of power-of-two voxels,
+// from heights; only values up to T (times the squared size) matter, larger ones
+// come out as anything above.
+bool cols_capped_ok(const int64_t *X, float res, int T)
+{
+    return tune_value(kTuneEdtPath) == 0 && window_path_ok(res, (int)X[1]) && T >= 0 && T < (int)kBig;
+}
+
+int launch_cols_capped(const float *fin, float *fout, const int64_t *X, int lo, int planes, float res, int T,
+                       cudaStream_t st)
+{
+    int W = 0;
+    while ((W + 1) * (W + 1) <= T)
+        W++;
+    const long long at = (long long)lo * X[1] * X[2];
+    return cols_run(fin + at, fout + at, planes, (int)X[1], (int)X[2], res * res, 0, std::min(W + 1, (int)X[1] - 1), 0, 0,
+                    nullptr, st);
+}
+
 // What a lattice pass left over: the ends of periodic lines, and whole lines.
 template <class T>
 static int rest(const T *in, float *out, const Lines &Ls, float res, float resh, const pmg_axis_cfg &cfg, int num_hull,

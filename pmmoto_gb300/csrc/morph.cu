@@ -246,8 +246,11 @@ int morph_run(const uint8_t *img, uint8_t *out, const int64_t *shape, const int3
     Lines L1 = all_lines(X, 1); // lines over (i, k): keep i inside the unextended range
     L1.b1lo = me.e0;
     L1.nb1 = (int)shape[0];
-    PMG_TRY(launch_envelope(A, B, L1, res[1], plain, 4, PMG_EDT_SQUARED, me, st, T == INT_MIN ? INT_MAX : T, nullptr,
-                            0, vcap));
+    if (T != INT_MIN && cols_capped_ok(X, res[1], T))
+        PMG_TRY(launch_cols_capped(A, B, X, me.e0, (int)shape[0], res[1], T, st));
+    else
+        PMG_TRY(launch_envelope(A, B, L1, res[1], plain, 4, PMG_EDT_SQUARED, me, st, T == INT_MIN ? INT_MAX : T, nullptr,
+                                0, vcap));
     Lines L2 = all_lines(X, 2); // lines over (i, j): both inside the unextended range
     L2.b1lo = me.e0;
     L2.nb1 = (int)shape[0];
