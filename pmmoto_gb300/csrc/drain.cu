@@ -467,6 +467,15 @@ static size_t max_morph_bytes(const int64_t *shape, const int32_t *bc, const int
     return a > b ? a : b;
 }
 
+// A failed allocation alone, whose error is then taken back.
+static bool no_room(int status)
+{
+    if (status != PMG_ECUDA || cudaPeekAtLastError() != cudaErrorMemoryAllocation)
+        return false;
+    cudaGetLastError();
+    return true;
+}
+
 static int check_common(const int64_t *shape, const int32_t *bc, const int32_t *pad)
 {
     PMG_TRY(check_geometry(shape, bc, pad));
@@ -584,14 +593,20 @@ extern "C" int pmg_pore_sizes(const uint8_t *pm_img, double *out, const int64_t 
         bool fits = nx < INT_MAX;
         for (int d = 0; d < 3; d++)
             fits = fits && shape[d] + big[2 * d] + big[2 * d + 1] <= PMG_MAX_LINE;
-        if (fits && scratch_alloc(&mem, xb + 256 + tb, st) == PMG_OK) {
+        const int got = fits ? scratch_alloc(&mem, xb + 256 + tb, st) : PMG_OK;
+        if (got != PMG_OK) {
+            // no room for the field: every radius by itself
+            mem = nullptr;
+            s = no_room(got) ? PMG_OK : got;
+        } else if (fits) {
             uint8_t *E = (uint8_t *)mem;
             float *A = (float *)((char *)mem + (((size_t)nx + 255) & ~(size_t)255));
             D = A + nx;
             int64_t X[3], lo[3];
-            if (erosion_edt_ext_run(pm_img, D, shape, bc, pad, big, res, unit_res, E, A, X, lo, st) != PMG_OK) {
-                D = nullptr; // (no room for its scratch, say)
-                cudaGetLastError();
+            const int ran = erosion_edt_ext_run(pm_img, D, shape, bc, pad, big, res, unit_res, E, A, X, lo, st);
+            if (ran != PMG_OK) {
+                D = nullptr; // (no room for its scratch)
+                s = no_room(ran) ? PMG_OK : ran;
             }
             XR = ExtRows{X[1], X[2], lo[0], lo[1], lo[2]};
             const pmg_axis_cfg plain = {0, 0, 0, 0, 1, 0, 0, 0};
@@ -641,10 +656,6 @@ extern "C" int pmg_pore_sizes(const uint8_t *pm_img, double *out, const int64_t 
                     if (flag[(size_t)k])
                         shared[(size_t)at[(size_t)k]] = 0;
             }
-        } else {
-            // no room for the field: every radius by itself
-            mem = nullptr;
-            cudaGetLastError();
         }
     }
     uint8_t *todo = nullptr; // the pore voxels that no opening has covered yet
