@@ -410,6 +410,7 @@ struct OpWgrad {
     float *dw;               // [27 * cin][cout]
     int kchunks_total;       // ceil(npos_out / 64)
     int lgc;
+    int vec;                 // dw is 16-byte aligned
     FastDiv qo;
     struct Row {
         int m;                // this thread's accumulator row
@@ -459,10 +460,16 @@ struct OpWgrad {
     {
         if (r.m >= 27 * g.cin || c0 >= g.cout)
             return;
-        float4 *dst = reinterpret_cast<float4 *>(dw + (long long)r.m * g.cout + c0);
+        float *dst = dw + (long long)r.m * g.cout + c0;
+        if (vec) {
 #pragma unroll
-        for (int i = 0; i < 4; i++)
-            atomicAdd(dst + i, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
+            for (int i = 0; i < 4; i++)
+                atomicAdd(reinterpret_cast<float4 *>(dst) + i, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; i++)
+                atomicAdd(dst + i, v[i]);
+        }
     }
 };
 
@@ -1162,6 +1169,7 @@ extern "C" int pmg_cnn_conv_wgrad(const void *x, const void *dz, float *dw, floa
         op.x = (const __nv_bfloat16 *)x;
         op.dz = (const __nv_bfloat16 *)dz;
         op.dw = dw;
+        op.vec = !(reinterpret_cast<uintptr_t>(dw) & 15);
         op.kchunks_total = (int)((np + kBK - 1) / kBK);
         op.lgc = log2_of(cin);
         op.qo = fastdiv_of((unsigned)g.dout);
