@@ -839,8 +839,11 @@ __global__ void __launch_bounds__(128) k_conv1_wgrad(const __nv_bfloat16 *__rest
         }
         __syncthreads();
         const float *sx = s_x + (lane < 27 ? kz * kPS + (2 * w + ky) * kRS + kx : 0);
+        // (only the positions inside: beyond them an input may still be read, and a
+        // zero gradient times one that is not finite is not zero)
+        const int np = yb * kWgY + w < dd ? min(32, dd - xb * kPatchX) : 0;
 #pragma unroll 4
-        for (int p = 0; p < 32; p++) {
+        for (int p = 0; p < np; p++) {
             const float v = lane < 27 ? sx[2 * p] : fixed;
             const float4 *q = reinterpret_cast<const float4 *>(s_d[w * 32 + p]);
 #pragma unroll
