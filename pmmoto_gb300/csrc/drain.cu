@@ -279,8 +279,7 @@ static int porosimetry_run(const uint8_t *pm, uint8_t *out, const int64_t *shape
                            const Boxes &Bx, Work &w, cudaStream_t st, double ball_e, double ball_d,
                            const float *De = nullptr, const uint16_t *KC = nullptr, int Te = -1,
                            bool m1_counted = false, GrowSel *g_er = nullptr, GrowSel *g_nw = nullptr,
-                           const uint8_t *Sv = nullptr, int step = -1, int *orange = nullptr,
-                           unsigned *rows_out = nullptr, Fork *eroded = nullptr)
+                           int *orange = nullptr, unsigned *rows_out = nullptr, Fork *eroded = nullptr)
 {
     // a drainage: rows_out, the result as row words (out is then scratch); eroded,
     // where the eroded space's marks of this radius were made
@@ -997,7 +996,7 @@ extern "C" int pmg_drainage_ext(const uint8_t *pm_img, uint8_t *mp_img, const in
             s = porosimetry_run(pm_img, morph, shape, bc, pad, ext, ext_d, res, radii[k], 1, radii_dilate[k], 1, 1,
                                 mp_img,
                                 Bx, w, st, ball_erode ? ball_erode[k] : -1.0, ball_dilate ? ball_dilate[k] : -1.0,
-                                De, KC, Te[(size_t)k], true, grow_er ? &g_er : nullptr, &g_nw, Sv, k, orange, drows,
+                                De, KC, Te[(size_t)k], true, grow_er ? &g_er : nullptr, &g_nw, orange, drows,
                                 grow_er ? &eroded : nullptr);
             if (s == PMG_OK)
                 s = next_eroded(k + 1);
