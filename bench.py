@@ -451,9 +451,6 @@ def measure_large(args, local, peak, peak_kind):
     from pmmoto_gb300.filters import distance as D
 
     n = 1024
-    from pmmoto_gb300 import tune
-
-    tuned = tune.tune_edt((n, n, n))  # launch parameters of this shape class (cached)
     own = grf.gen_grf_medium(n)
     idx = torch.arange(-1, n + 1, device="cuda") % n
     img = own[idx][:, idx][:, :, idx].contiguous()
@@ -468,7 +465,6 @@ def measure_large(args, local, peak, peak_kind):
            "cc": (lambda: CC.connect_components_device(img, geo), img.numel(), 17.0)}
     res_out = {"workload": "1024^3 GRF medium (sigma 4, porosity 0.35, periodic); edt3d squared on the own "
                            "1024^3 volume, connected components on the padded 1026^3 image",
-               "edt_tuned": tuned,
                "l2": "inputs larger than L2 (1 GB image, 4 GB distances, 8.6 GB labels)"}
     steps = max(3, min(args.steps, 10))
     for name, (op, vox, bpv) in ops.items():

@@ -362,21 +362,25 @@ int pmg_set_iteration_cap(int32_t cap);
 
 /*
  * Tunable launch parameters (no counterpart in the reference): results never
- * depend on them, only speed.  Names: "edt.path" (envelope passes: the integer
- * lattice and the outward scan, 0, the exact integer stream, 1, or the float
- * envelope, 2; default 0), "edt.wide" (outward scans: sampled steps a voxel, in
- * 1/1024 of the measured crossing point, from which the float envelope takes
- * the pass; 0 always, 8193 never; default 1024), "cc.seam_batched" (periodic merge: the seams of all periodic
- * features deduplicated in one sort, 1, or one feature at a time, 0; default
- * 1; one at a time is also taken when labels need more than 29 bits).
+ * depend on them, only speed.  Names:
+ *   "edt.path"        envelope passes: the integer lattice and the outward scan
+ *                     (0), the exact integer stream (1) or the float envelope
+ *                     (2); default 0
+ *   "edt.wide"        outward scans: sampled steps a voxel, in 1/1024 of the
+ *                     measured crossing point, from which the float envelope
+ *                     takes the pass; 0 always, 8193 never; default 1024
+ *   "cc.seam_batched" periodic merge: the seams of all periodic features
+ *                     deduplicated in one sort (1) or one feature at a time (0);
+ *                     default 1; one at a time is also taken when labels need
+ *                     more than 29 bits
  * "edt.pair_seg", "edt.pair_ctas", "edt.rows_ctas", "edt.fallback",
- * "edt.fallback_rows", "edt.narrow" and "edt.narrow_rows" belonged
- * to a windowed pass that the lattice passes replaced, "cc.cross_fused" (0 or 1)
- * to a cross-tile phase that the row words replaced; they are still accepted, in
- * the same ranges, so that saved settings keep loading, and have no effect.  A negative value restores the default, and so does 0 for the
- * knobs whose smallest value is 1; values are process-wide and apply to
- * launches that follow.  pmmoto_gb300.tune sets them from its cached
- * measurements.
+ * "edt.fallback_rows", "edt.narrow" and "edt.narrow_rows" belonged to a windowed
+ * pass that the lattice passes replaced, "cc.cross_fused" (0 or 1) to a
+ * cross-tile phase that the row words replaced; they are still accepted, in the
+ * same ranges, so that saved settings keep loading, and have no effect.
+ * A negative value restores the default, and so does 0 for the knobs whose
+ * smallest value is 1; values are process-wide and apply to launches that
+ * follow.  pmmoto_gb300.tune sets them from its cached measurements.
  */
 int pmg_tune_set(const char *name, int32_t value);
 int pmg_tune_get(const char *name, int32_t *value);

@@ -79,13 +79,14 @@ struct TuneSpec {
     int def, lo, hi;
 };
 static const TuneSpec g_tune_spec[kTuneKnobs] = {
-    // (accepted without effect: knobs of a former windowed pass)
+    // No effect: knobs of a former windowed pass (edt.*) and cross-tile phase,
+    // accepted, kept and given back so that saved settings load.
     {"edt.pair_seg", 256, 32, 8192},
     {"edt.pair_ctas", 32, 1, 256},
     {"edt.rows_ctas", 16, 1, 256},
-    {"cc.cross_fused", 0, 0, 1},        // (no effect: knob of a former cross-tile phase)
+    {"cc.cross_fused", 0, 0, 1},
     {"edt.path", 0, 0, 2},              // envelope passes: lattice / scan (0), exact stream (1), float envelope (2)
-    {"edt.fallback", 96, 0, 8193},      // (no effect)
+    {"edt.fallback", 96, 0, 8193},      // (no effect, as above)
     {"edt.fallback_rows", 2048, 0, 8193}, // (no effect)
     {"edt.narrow", 64, 0, 8193},        // (no effect)
     {"edt.narrow_rows", 32, 0, 8193},   // (no effect)

@@ -1,13 +1,14 @@
 """Autotuner of launch parameters (no counterpart in the reference).
 
 Some launch parameters change only speed, never results: library knobs set
-through ``pmg_tune_set`` (those of the former line-pair envelope passes and
-cross-tile phase are still accepted and timed, without effect) and the number
-of CUDA streams the batched configuration spreads its media over (a host-side
-knob).  The tuner times every candidate
-of one knob at a time (coordinate descent, the others held at their current
-best) on a synthetic medium of the caller's shape class, with CUDA events
-after a warm-up, and keeps the fastest.
+through ``pmg_tune_set`` and the number of CUDA streams the batched
+configuration spreads its media over (a host-side knob).  The tuner times
+every candidate of one knob at a time (coordinate descent, the others held at
+their current best) with CUDA events after a warm-up, and keeps the fastest.
+The library's present distance transform and labelling choose their launches by
+rules on sizes and types; the knobs of their former passes (``INERT``) are
+still read from caches and ``PMG_TUNE`` and accepted by the library, so that
+saved settings keep loading, but have no effect and are not timed.
 
 Results are cached as JSON (``$PMG_TUNE_CACHE``, default
 ``~/.cache/pmmoto_gb300/autotune.json``) under the key
@@ -33,6 +34,7 @@ KNOBS = {
     "batch": {"batch.workers": [2, 4, 8, 16]},
 }
 HOST_KNOBS = {"batch.workers": 8}
+INERT = {"edt.pair_seg", "edt.pair_ctas", "edt.rows_ctas", "cc.cross_fused"}
 _lock = threading.Lock()
 _applied: dict[str, dict] = {}
 
@@ -155,9 +157,14 @@ def _time(fn, steps: int) -> float:
     return e0.elapsed_time(e1) / steps
 
 
-def _descend(kernel: str, shape, run, steps: int, set_knob) -> tuple[dict, dict]:
+def _live(kernel: str) -> dict:
+    """The knobs of `kernel` that still change its launches."""
+    return {name: cands for name, cands in KNOBS[kernel].items() if name not in INERT}
+
+
+def _descend(kernel: str, run, steps: int, set_knob) -> tuple[dict, dict]:
     best, timings = {}, {}
-    for name, cands in KNOBS[kernel].items():
+    for name, cands in _live(kernel).items():
         res = {}
         for c in cands:
             set_knob(name, c)
@@ -169,54 +176,61 @@ def _descend(kernel: str, shape, run, steps: int, set_knob) -> tuple[dict, dict]
     return best, timings
 
 
-def tune_edt(shape, periodic=(True, True, True), steps: int = 3, force: bool = False) -> dict:
-    """Tune the EDT's line-pair passes for `shape` on a GRF medium of that
-    shape (porosity 0.35, sigma 4 voxels); cached per shape class."""
-    import torch
-
-    from .domain_generation import grf
-    from .filters import distance as D
-
-    k = key("edt", shape)
-    if not force:
-        cached = load_cache().get(k)
-        if cached:
-            _applied.pop(k, None)
-            return apply("edt", shape)
-    img = grf.gen_grf_medium(tuple(int(s) for s in shape))
-    out = torch.empty(img.shape, dtype=torch.float32, device=img.device)
-    cfg = D.edt3d_cfg(periodic)
-    res = np.ones(3, np.float32)
-    best, timings = _descend("edt", shape, lambda: D.edt3d_device(img, res, cfg, True, out), steps, _set_lib)
+def _tune_lib(kernel: str, shape, medium, steps: int, force: bool) -> dict:
+    """Tune the library knobs of `kernel` on the call that `medium` makes for
+    `shape`; {} without any timing when the kernel has no live knob."""
+    k = key(kernel, shape)
+    if not force and load_cache().get(k):
+        _applied.pop(k, None)
+        return apply(kernel, shape)
+    best, timings = _descend(kernel, medium(), steps, _set_lib) if _live(kernel) else ({}, {})
     save_entry(k, best, timings)
     _applied[k] = best
     return best
+
+
+def tune_edt(shape, periodic=(True, True, True), steps: int = 3, force: bool = False) -> dict:
+    """Tune the EDT's live knobs (none at present: {}) for `shape` on a GRF
+    medium of that shape (porosity 0.35, sigma 4 voxels); cached per shape
+    class."""
+
+    def medium():
+        import torch
+
+        from .domain_generation import grf
+        from .filters import distance as D
+
+        img = grf.gen_grf_medium(tuple(int(s) for s in shape))
+        out = torch.empty(img.shape, dtype=torch.float32, device=img.device)
+        cfg = D.edt3d_cfg(periodic)
+        res = np.ones(3, np.float32)
+        return lambda: D.edt3d_device(img, res, cfg, True, out)
+
+    return _tune_lib("edt", shape, medium, steps, force)
 
 
 def tune_cc(shape, steps: int = 3, force: bool = False) -> dict:
-    """Tune the block labelling for padded periodic volumes of `shape` on a GRF
-    medium (porosity 0.35, sigma 4 voxels); cached per shape class."""
-    import pmmoto_gb300 as P
+    """Tune the labelling's live knobs (none at present: {}) for padded
+    periodic volumes of `shape` on a GRF medium (porosity 0.35, sigma 4
+    voxels); cached per shape class."""
 
-    from .core.geometry import geo_of
-    from .domain_generation import grf
-    from .filters import connected_components as CC
+    def medium():
+        import torch
 
-    k = key("cc", shape)
-    if not force and load_cache().get(k):
-        _applied.pop(k, None)
-        return apply("cc", shape)
-    own = grf.gen_grf_medium(tuple(int(s) - 2 for s in shape))
-    import torch
+        import pmmoto_gb300 as P
 
-    idx = [torch.arange(-1, n + 1, device=own.device) % n for n in own.shape]
-    img = own[idx[0]][:, idx[1]][:, :, idx[2]].contiguous()
-    sd = P.initialize(tuple(own.shape), boundary_types=(("periodic", "periodic"),) * 3)
-    geo = geo_of(sd)
-    best, timings = _descend("cc", shape, lambda: CC.connect_components_device(img, geo), steps, _set_lib)
-    save_entry(k, best, timings)
-    _applied[k] = best
-    return best
+        from .core.geometry import geo_of
+        from .domain_generation import grf
+        from .filters import connected_components as CC
+
+        own = grf.gen_grf_medium(tuple(int(s) - 2 for s in shape))
+        idx = [torch.arange(-1, n + 1, device=own.device) % n for n in own.shape]
+        img = own[idx[0]][:, idx[1]][:, :, idx[2]].contiguous()
+        sd = P.initialize(tuple(own.shape), boundary_types=(("periodic", "periodic"),) * 3)
+        geo = geo_of(sd)
+        return lambda: CC.connect_components_device(img, geo)
+
+    return _tune_lib("cc", shape, medium, steps, force)
 
 
 def tune_batch(items, fn, steps: int = 1, force: bool = False) -> dict:
@@ -233,6 +247,6 @@ def tune_batch(items, fn, steps: int = 1, force: bool = False) -> dict:
     def run():
         batch.map_streams(fn, items, workers=cur["batch.workers"])
 
-    best, timings = _descend("batch", shape, run, steps, lambda n, v: cur.__setitem__(n, v))
+    best, timings = _descend("batch", run, steps, lambda n, v: cur.__setitem__(n, v))
     save_entry(k, best, timings)
     return best
