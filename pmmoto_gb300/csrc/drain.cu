@@ -7,9 +7,10 @@
 //   25-179): per capillary pressure, porosimetry with the inlet and multiphase
 //   constraints, outlet-connected wetting phase, update, reservoir refill,
 //   wetting-phase count in the own region (the saturation numerator).
-// All images stay on the device between steps; the host reads back only the
-// two phase-existence counts porosimetry branches on and, at the end, the
-// per-pressure counts.
+// All images stay on the device between steps.  A drainage reads back its
+// per-pressure counts at the end; per pressure it waits only where a branch on the
+// host depends on the data (porosimetry's phase counts without a growing
+// selection, the seed count of a dilation by scan).
 #include <algorithm>
 #include <cmath>
 #include <vector>

@@ -1,7 +1,25 @@
 // Exact Euclidean distance transform on GB300 (sm_103a).
 //
-// Three kernels, one thread per 1-D line, lanes of a warp on neighbouring
-// lines so that the strided axes are read and written coalesced:
+// A transform is a linear pass along axis 0 and two envelope passes; edt3d_run
+// gives each the first of these that takes its sizes:
+//
+//  * the linear pass: k_lin (edt_lattice.cu), counts for a lattice pass behind
+//    it or squared distances; k_pass0 here for periodic lines of voxel sizes that
+//    are no power of two and for lines beyond 2048;
+//  * an envelope pass of power-of-two voxels, lines of at most 1024: the integer
+//    lattice (edt_lattice.cu);
+//  * an envelope pass of other voxel sizes, or of a voxel size that is larger than
+//    an earlier axis's (or less than 2^-16 of it), lines of at most 1024: the
+//    outward scan (edt_scan.cu), or the float envelope where a probe finds its
+//    pores wide;
+//  * longer lines: the exact integer stream (edt_exact.cu) where the sizes allow
+//    it, the float envelope otherwise.
+//
+// Lines that the lattice and the scan cannot finish are handed back to the float
+// envelope here: whole (k_envelope_whole), or their periodic ends alone
+// (k_lattice_ends, k_envelope_ends).  The float kernels run one thread per 1-D
+// line, lanes of a warp on neighbouring lines so that the strided axes are read
+// and written coalesced:
 //
 //  * k_pass0     -- the linear two-sweep pass of squared_edt_1d
 //                   (src/pmmoto/filters/distance/_distance.hpp:135-182) with
@@ -31,7 +49,6 @@
 #include "edt_internal.cuh"
 
 namespace pmg {
-
 
 // ---------------------------------------------------------------------------
 // pass 0: squared_edt_1d along axis `ax`
@@ -638,8 +655,8 @@ __global__ void k_envelope_whole(const T *__restrict__ fin, float *__restrict__ 
 // on the imported hulls at their ends, or need the reference's float envelope
 // as a whole.
 
-// One line replayed with the float envelope: the whole line (`whole`, or a line
-// without a zero height), or its end segments only -- the lower imports with
+// One line replayed with the float envelope: a line without a zero height as a
+// whole, any other by its end segments only -- the lower imports with
 // the voxels up to the first zero, and the voxels from the last zero with the
 // upper imports.  No parabola can pop a zero off the stack, so these partial
 // stacks and sweeps make the same float decisions as the whole line's.

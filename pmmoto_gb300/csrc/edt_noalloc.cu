@@ -10,9 +10,8 @@
 // of allocating; the caller still passes the input and output buffers.
 //
 // The arrays are file-scope __device__ variables: every GPU that loads this
-// library holds them (64 MiB for the intermediate volume, 4 MiB for the
-// per-line flags and the deferred voxels of the windowed envelope path) until
-// the process exits.
+// library holds them (64 MiB for the intermediate volume, 4 MiB for the flags
+// that the lattice and scan passes set per line) until the process exits.
 // Host code may not use an array's name as a device address, so the first
 // call on each device resolves both addresses with cudaGetSymbolAddress
 // while that device is current and caches them.  The cache is not
@@ -27,15 +26,15 @@ namespace pmg {
 // 16 Mi float32 = 64 MiB: volumes of up to 16,777,216 voxels (e.g. 256^3).
 constexpr long long kNoAllocMaxVoxels = 16LL * 1024 * 1024;
 
-// 1 Mi int32 = 4 MiB: the first half per-line flags (an envelope pass with
-// more lines runs in blocks of rows that fit; one row is at most PMG_MAX_LINE
-// lines), the second half the voxels the line-pair kernels defer (about 262 K;
-// beyond that a line takes the whole float envelope).
-constexpr long long kNoAllocMaxFlagLines = 1LL << 20;
-static_assert(kNoAllocMaxFlagLines / 2 >= PMG_MAX_LINE, "a row of lines must fit the flag half");
+// 1 Mi int32 = 4 MiB: 16 bits per line of a lattice pass (2 Mi lines), a byte per
+// line of a scan and the choice of its probe.  Volumes with more lines than that
+// (lines of eight, four voxels and fewer) do not take these passes: a transform
+// whose lattice flags do not fit runs no pass on the lattice, and a scan whose
+// flags do not fit is left to the float envelope.
+constexpr long long kNoAllocFlagInts = 1LL << 20;
 
 static __device__ __align__(256) float g_edt_noalloc_scratch[kNoAllocMaxVoxels];
-static __device__ __align__(256) int g_edt_noalloc_flags[kNoAllocMaxFlagLines];
+static __device__ __align__(256) int g_edt_noalloc_flags[kNoAllocFlagInts];
 
 static std::mutex g_noalloc_mu;
 static float *g_noalloc_ptr[64] = {nullptr};
@@ -115,8 +114,9 @@ extern "C" int pmg_edt3d_noalloc(const uint8_t *img, float *out, const int64_t s
     int *flags = nullptr;
     PMG_TRY(noalloc_scratch(&tmp, &flags));
     // every scratch element read by the second envelope pass is written by the
-    // first one, and the envelope clears the flags of each block of lines
-    // before it uses them, so nothing left by an earlier call leaks through
+    // first one, and a pass that flags lines writes every line's flag (its probe
+    // the choice) before the kernels that read them, so nothing left by an earlier
+    // call leaks through
     return edt3d_run(img, out, tmp, shape, res, cfg, num_hull, form, as_stream(stream), flags,
-                     kNoAllocMaxFlagLines);
+                     kNoAllocFlagInts);
 }
