@@ -138,7 +138,7 @@ __device__ __forceinline__ float scan_voxel(const float *line, int n, int x, int
         need |= periodic ? kScanEnds : 0u;
         return m;
     }
-    const float R = __fsqrt_rn(m * inv_a);
+    const float R = fminf(__fsqrt_rn(m * inv_a), (float)n); // (no parabola is farther)
     const float eta = scan_eta(a, m, R, (float)x);
     if (periodic) {
         const int e = min(x + 1, n - x);
@@ -266,14 +266,12 @@ __global__ void __launch_bounds__(32 * kScanWarps) k_scan_rows(const float *__re
 // envelope's hardly does, so a probe in front of the pass estimates the steps of
 // a scan from kProbeGroups of its warps (32 adjacent lines, or 32 consecutive
 // positions of a row) and sets *wide when the envelope is the cheaper one.
-// A sample's steps come from the heights at offsets that grow with the distance:
-// heights' roots change by at most a voxel from one position to the next, so a
-// solid between two offsets shows.  One cluster, so that the sum needs no
-// clearing.
+// One cluster, so that the sum needs no clearing.
 constexpr int kProbeBlocks = 8, kProbeThreads = 512, kProbeGroups = kProbeBlocks * kProbeThreads / 32;
 
 __global__ void __cluster_dims__(kProbeBlocks, 1, 1) __launch_bounds__(kProbeThreads)
-    k_pore_probe(const float *__restrict__ fin, Lines Ls, float a, float inv_a, float most, float budget, int *wide)
+    k_pore_probe(const float *__restrict__ fin, Lines Ls, float a, float inv_a, float vcap, float most, float budget,
+                 int *wide)
 {
     cudaTriggerProgrammaticLaunchCompletion(); // (the pass may start: its first blocks wait)
     __shared__ unsigned s_sum;
@@ -292,14 +290,31 @@ __global__ void __cluster_dims__(kProbeBlocks, 1, 1) __launch_bounds__(kProbeThr
     if (Ls.ax == 2)
         x = min(x / 32 * 32 + lane, n - 1);
     const float *c = fin + g.base;
-    constexpr int kOff[12] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64};
     float m = c[x * g.stride];
+    const auto at = [&](int d) {
+        m = fminf(m, fminf(c[max(x - d, 0) * g.stride], c[min(x + d, n - 1) * g.stride]) + a * (float)(d * d));
+    };
+    // every distance up to 128 (lines of a volume that is thin along the earlier axes
+    // hold solids at single positions), then some
+    int d = 0;
+    bool open = true;
+    for (; d < 128 && open; d += 16) {
 #pragma unroll
-    for (int k = 0; k < 12; k++)
-        m = fminf(m, fminf(c[max(x - kOff[k], 0) * g.stride], c[min(x + kOff[k], n - 1) * g.stride]) +
-                         a * (float)(kOff[k] * kOff[k]));
-    // (a warp scans as far as its farthest lane)
-    const unsigned far = __reduce_max_sync(0xffffffffu, (unsigned)fminf(__fsqrt_rn(m * inv_a), most));
+        for (int u = 1; u <= 16; u++)
+            at(d + u);
+        open = __any_sync(0xffffffffu, m > a * (float)((d + 16) * (d + 16)));
+    }
+    for (; open && d < n; d += d / 2) {
+#pragma unroll
+        for (int u = 1; u <= 4; u++)
+            at(d + d * u / 8);
+        open = __any_sync(0xffffffffu, m > a * (float)(d * d / 4 * 9));
+    }
+    // (a warp scans as far as its farthest lane; lines that a scan would leave to the
+    // envelope after all count as far)
+    const float R = fminf(__fsqrt_rn(m * inv_a), (float)n);
+    const bool whole = m <= vcap && scan_eta(a, m, R, (float)x) > 0.5f * a;
+    const unsigned far = __reduce_max_sync(0xffffffffu, (unsigned)(whole ? most : fminf(R, most)));
     if (lane == 0)
         atomicAdd(&s_sum, far);
     cluster.sync();
@@ -313,26 +328,28 @@ __global__ void __cluster_dims__(kProbeBlocks, 1, 1) __launch_bounds__(kProbeThr
 }
 
 // Steps a voxel from which the envelope is the faster one.  A step costs about 1 ps a
-// voxel (512^3: 0.14 ms a pass), the envelope 15 to 50 ps (1.9 to 7 ms), and on few
-// lines one chain of n pushes (1 to 2 us each) whatever their number, hence the
-// term in the lines.  Scan alone, envelope alone, chosen, in ms, both passes,
-// voxels of 2.25: 512^3 field of sigma 4: 2.0, 5.1, 2.0; cavity of radius 230: 7.2, 5.1,
-// 5.1; points 10 voxels apart on average: 14.4, 7.6, 5.8; 20: 51, 10.6, 10.6; 200 x 180 x
-// 220 cavity of radius 81: 0.32, 0.82, 0.32; points 20 voxels apart: 2.0, 1.5, 1.5;
-// 96^3: 0.25, 0.51, 0.25.  On periodic lines the ends are replayed after a scan, so
-// the crossing lies lower (voxels 1 x 1 x 2, 512^3 field of sigma 4: 3.5, 5.5, 3.5;
-// sigma 20: 12.7, 8.6, 8.6).
-// Below five million voxels the two lie close together whatever the distances, and
-// the probes would cost more (2 x 2 us of 70 at four million).
-static float scan_budget(const Lines &Ls, int n, int periodic)
+// voxel (512^3: 0.14 ms a pass), the envelope 15 to 50 ps (1.9 to 7 ms) and at least
+// one chain of n pushes (1 to 2 us each), hence the term in the lines.  With few lines
+// a scan is a chain too: of columns n / 8 rounds of as many steps as their
+// distances (65 ns each), of rows n / 32, hence the upper ends.  Scan alone,
+// envelope alone, chosen, in ms, voxels of 2.25: 512^3 field of sigma 4: 2.0, 5.1, 2.0;
+// cavity of radius 230: 7.2, 5.1, 5.1; points 20 voxels apart on average: 51, 10.6, 10.6;
+// 256^3 points 10 voxels apart: 1.97, 1.39, 1.1; one pass of 1000 x 1000, points 40, 80
+// voxels apart: 0.46, 0.91, 0.46 and 2.15, 1.01, 1.01; 1024 x 100, points 20: 0.25, 0.95, 0.25.
+// On periodic lines the ends are replayed after a scan, so the crossing lies lower
+// (voxels 1 x 1 x 2, 512^3 field of sigma 4: 3.5, 5.5, 3.5; sigma 20: 12.7, 8.6, 8.6; 1000 x
+// 1000, points 4 and 20 voxels apart: 0.90, 2.3, 0.90 and 3.9, 3.8, 3.8).
+static float scan_budget(const Lines &Ls, int periodic)
 {
     const float nl = (float)Ls.count();
     const int k = tune_value(kTuneEdtWide); // 1024: as it is; 0: always the envelope, 8193: never
     if (k == 0)
         return -1.0f;
-    if (k > 8192 || (!periodic && nl * (float)n < 5e6f))
+    if (k > 8192)
         return INFINITY;
-    return (periodic ? std::max(5.0f, 0.22e6f / nl) : std::max(36.0f, 3.6e6f / nl)) * ((float)k / 1024.0f);
+    const float steps = periodic ? std::min(12.0f, std::max(5.0f, 0.11e6f / nl))
+                                 : std::min(Ls.ax == 2 ? 190.0f : 95.0f, std::max(36.0f, 1.3e6f / nl));
+    return steps * ((float)k / 1024.0f);
 }
 
 // *choice = wide once the probe has set it, null where no scan of the pass can
@@ -343,12 +360,15 @@ int launch_pore_probe(const float *fin, const Lines &Ls, float res, float vcap, 
     const float a = res * res, inv_a = 1.0f / a;
     const int n = (int)(Ls.ax == 0 ? Ls.s0 : Ls.ax == 1 ? Ls.s1 : Ls.s2);
     // the most steps of a voxel: to the line's end, or to the cap
-    const float most = std::fmin((float)n, std::sqrt(vcap * inv_a) + 1.0f), budget = scan_budget(Ls, n, periodic);
+    const float most = std::fmin((float)n, std::sqrt(vcap * inv_a) + 1.0f), budget = scan_budget(Ls, periodic);
     *choice = nullptr;
-    if (most <= budget)
+    // (on a small volume with short lines the two lie close together whatever the
+    // distances: 100 x 300 x 100, rows without a solid nearby, 0.40 and 0.11 ms, where
+    // the probe is 2 to 5 us of calls from 70)
+    if (most <= budget || (!periodic && budget >= 0.0f && n <= 128 && (float)Ls.count() * (float)n < 5e6f))
         return PMG_OK;
     const int ps__ = prof_begin("k_pore_probe", st);
-    k_pore_probe<<<kProbeBlocks, kProbeThreads, 0, st>>>(fin, Ls, a, inv_a, most, budget, wide);
+    k_pore_probe<<<kProbeBlocks, kProbeThreads, 0, st>>>(fin, Ls, a, inv_a, vcap, most, budget, wide);
     prof_end(ps__, 0.0, st);
     PMG_CHECK_LAUNCH();
     *choice = wide;
